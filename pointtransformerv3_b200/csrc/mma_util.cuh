@@ -94,6 +94,12 @@ __device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b)
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b)
+{
+    uint64_t d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
 
 // a pair from two 32-bit words (low word = first of the pair)
 __device__ __forceinline__ uint64_t pack2u(uint32_t lo, uint32_t hi)
@@ -155,6 +161,26 @@ __device__ __forceinline__ uint32_t exp2_poly2_bf16(uint64_t x2, const Exp2Const
     px = __int_as_float(__float_as_int(px) + (__float_as_int(tx) << 23));
     py = __int_as_float(__float_as_int(py) + (__float_as_int(ty) << 23));
     return pack_bf16(px, py);
+}
+
+// acc + the squares of a bf16 pair
+__device__ __forceinline__ float sq_norm_bf16x2(uint32_t v, float acc)
+{
+    const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v));
+    return fmaf(f.x, f.x, fmaf(f.y, f.y, acc));
+}
+// squared norm of 16 bf16 values
+__device__ __forceinline__ float sq_norm16(const uint4& a, const uint4& b)
+{
+    float v = sq_norm_bf16x2(a.x, sq_norm_bf16x2(a.y, sq_norm_bf16x2(a.z, sq_norm_bf16x2(a.w, 0.f))));
+    return sq_norm_bf16x2(b.x, sq_norm_bf16x2(b.y, sq_norm_bf16x2(b.z, sq_norm_bf16x2(b.w, v))));
+}
+// maximum that keeps a NaN
+__device__ __forceinline__ float max_nan(float a, float b)
+{
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
 }
 
 }  // namespace ptv3

@@ -260,6 +260,26 @@ def test_attention_tcgen05_large_scores():
     assert rel_l2(b, a) < 1e-2
 
 
+@pytest.mark.parametrize("n", [63, 64, 65, 1000, 2100])
+@pytest.mark.parametrize("gain", [1.0, 3.0, 12.0])
+def test_attention_with_and_without_reference_value(n, gain):
+    """The mma.sync kernel takes tiles whose scores are bounded by their norms without a running
+    maximum: all tiles (gain 1), some (one patch half has large queries) or none; full key groups
+    and ragged ends."""
+    C, H, K = 32, 2, 1024
+    g = torch.Generator().manual_seed(n)
+    qkv = torch.randn(n, 3 * C, generator=g)
+    qkv[:, C:2 * C] *= gain
+    qkv[n // 2:, :C] *= gain
+    qkv = qkv.bfloat16().cuda()
+    order = torch.randperm(n, generator=g).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    a = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25, algo=1)
+    b = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25, algo=2)
+    assert bool(torch.isfinite(b.float()).all())
+    assert rel_l2(b, a) < (5e-3 if gain < 10 else 1e-2)
+
+
 @pytest.mark.parametrize("algo,dtype", [(0, torch.bfloat16), (1, torch.bfloat16), (1, torch.float32),
                                         (4, torch.bfloat16)])
 def test_attention_reports_a_patch_longer_than_max_seqlen(algo, dtype):
