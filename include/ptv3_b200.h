@@ -535,6 +535,75 @@ int ptv3_unpool_stage_fwd(const void* skip_feat, const void* child_feat, const v
                           const float* child_scale, const float* child_shift, void* out, void* skip_act, int dtype,
                           uint32_t* status, void* workspace, size_t workspace_bytes, void* stream);
 
+/*
+ * The whole bf16 backbone in one call (model.py:884-982, PointTransformerV3.forward of a
+ * segmentation network, inference): serialization, kernel maps, pooling plans, stem, encoder and
+ * decoder, queued on two streams from C++.  The kernels are the ones behind the entry points
+ * above; what the call saves is host time (a pass over a small room is bounded by it) and the
+ * waits between a plan's result and the next plan's launch.
+ *
+ * Memory comes from the caller: alloc(ctx, bytes, pool) returns device memory that stays valid
+ * until the work queued by the call has run (pool 0: memory ordered by main_stream, pool 1: by
+ * plan_stream and afterwards used on both), 256-byte aligned, or NULL to give up.
+ */
+typedef void* (*ptv3_alloc_fn)(void* ctx, size_t bytes, int pool);
+
+typedef struct ptv3_stage_args {
+    int n_blocks;
+    const ptv3_block_args* blocks;  /* HOST array; parameters, widths, scale and algo filled in */
+    const int* order_index;         /* HOST, per block: row of the serialized orders */
+    const int* patch;               /* HOST, per block: patch size; negative: min(-patch, smallest scene),
+                                       the rule without flash attention (model.py:441-444) */
+    /* the transition into the stage, absent on encoder stage 0: SerializedPooling (encoder) or
+       SerializedUnpooling (decoder: w / b / scale / shift project the coarse level, *_skip the fine one) */
+    int c_in, c_skip, c_out;
+    int pooling_depth, reduce;
+    const void *w, *b, *w_skip, *b_skip;
+    const float *scale, *shift, *scale_skip, *shift_skip;   /* BatchNorm(eval) as fp32 scale and shift */
+} ptv3_stage_args;
+
+typedef struct ptv3_backbone_args {
+    /* network */
+    int n_enc, n_dec;               /* n_dec == n_enc - 1, decoder stages from coarse to fine */
+    const ptv3_stage_args *enc, *dec;
+    int stem_c_in, stem_c_out, stem_ksize;
+    const void* stem_weight;
+    const float *stem_scale, *stem_shift;
+    int k;                          /* orders */
+    /* one pass */
+    int64_t n;
+    int n_scenes, depth;
+    const int64_t* counts;          /* HOST, n_scenes: points of every scene */
+    const int* order_ids;           /* HOST, k (as for ptv3_encode, already shuffled) */
+    const int* row_perm;            /* HOST, (n_enc - 1) x k or NULL: shuffle of every pooling */
+    const void* feat;               /* n x stem_c_in bf16 */
+    const int32_t* grid_coord;      /* n x 3 */
+    const int64_t *offset, *batch;  /* n_scenes, n */
+    /* outputs of the finest level */
+    int64_t *code, *order, *inverse;    /* k x n */
+    int32_t *indices, *nbr;             /* n x 4, 27 x n (columns in the order of row 0) */
+    int64_t *pad, *unpad;               /* plan for the patch size of the first block of enc[0] */
+    int32_t* cu_seqlens;
+    void* out;                          /* n x width of the last decoder stage */
+    int64_t* level_counts;          /* HOST, n_enc x n_scenes: points of every scene on every level */
+    /* page-locked HOST memory the device can address, (n_enc - 1) x (3 + n_scenes) int64 */
+    int64_t* meta_host;
+    uint32_t* status;
+    ptv3_alloc_fn alloc;
+    void* alloc_ctx;
+    void *main_stream, *plan_stream;
+} ptv3_backbone_args;
+
+int ptv3_backbone_fwd(const ptv3_backbone_args* args);
+
+/*
+ * Largest grid coordinate per axis and the scene offsets of a batch, stored by the kernel in
+ * page-locked host memory: out_host = {max x, max y, max z, offset[0 .. n_scenes), 1}.  The caller
+ * zeroes the last word and polls it.  scratch: 16 bytes of device memory.
+ */
+int ptv3_batch_stats(const int32_t* grid_coord, int64_t n, const int64_t* offset, int n_scenes,
+                     int64_t* out_host, void* scratch, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

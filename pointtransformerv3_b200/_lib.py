@@ -32,6 +32,32 @@ class BlockArgs(ctypes.Structure):
         + [("workspace_bytes", c_sz)])
 
 
+ALLOC_FN = ctypes.CFUNCTYPE(c_ptr, c_ptr, c_sz, c_int)
+
+
+class StageArgs(ctypes.Structure):
+    """ptv3_stage_args of include/ptv3_b200.h (same field order)."""
+    _fields_ = ([("n_blocks", c_int), ("blocks", ctypes.POINTER(BlockArgs)), ("order_index", ctypes.POINTER(c_int)),
+                 ("patch", ctypes.POINTER(c_int)), ("c_in", c_int), ("c_skip", c_int), ("c_out", c_int),
+                 ("pooling_depth", c_int), ("reduce", c_int)]
+                + [(name, c_ptr) for name in ("w", "b", "w_skip", "b_skip", "scale", "shift", "scale_skip",
+                                              "shift_skip")])
+
+
+class BackboneArgs(ctypes.Structure):
+    """ptv3_backbone_args of include/ptv3_b200.h (same field order)."""
+    _fields_ = (
+        [("n_enc", c_int), ("n_dec", c_int), ("enc", ctypes.POINTER(StageArgs)), ("dec", ctypes.POINTER(StageArgs)),
+         ("stem_c_in", c_int), ("stem_c_out", c_int), ("stem_ksize", c_int), ("stem_weight", c_ptr),
+         ("stem_scale", c_ptr), ("stem_shift", c_ptr), ("k", c_int), ("n", c_i64), ("n_scenes", c_int),
+         ("depth", c_int), ("counts", ctypes.POINTER(c_i64)), ("order_ids", ctypes.POINTER(c_int)),
+         ("row_perm", ctypes.POINTER(c_int))]
+        + [(name, c_ptr) for name in ("feat", "grid_coord", "offset", "batch", "code", "order", "inverse", "indices",
+                                      "nbr", "pad", "unpad", "cu_seqlens", "out")]
+        + [("level_counts", ctypes.POINTER(c_i64)), ("meta_host", c_ptr), ("status", c_ptr), ("alloc", ALLOC_FN),
+           ("alloc_ctx", c_ptr), ("main_stream", c_ptr), ("plan_stream", c_ptr)])
+
+
 # name -> (restype, argtypes); must list every symbol of include/ptv3_b200.h
 SIGNATURES = {
     "ptv3_last_error": (ctypes.c_char_p, []),
@@ -93,6 +119,8 @@ SIGNATURES = {
     "ptv3_block_supported": (c_int, [c_int, c_int, c_int, c_int]),
     "ptv3_block_workspace_bytes": (c_sz, [ctypes.POINTER(BlockArgs)]),
     "ptv3_block_fwd": (c_int, [ctypes.POINTER(BlockArgs), c_ptr]),
+    "ptv3_backbone_fwd": (c_int, [ctypes.POINTER(BackboneArgs)]),
+    "ptv3_batch_stats": (c_int, [c_ptr, c_i64, c_ptr, c_int, c_ptr, c_ptr, c_ptr]),
     "ptv3_unpool_fwd": (c_int, [c_ptr, c_ptr, c_ptr, c_i64, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr,
                                 c_ptr, c_int, c_ptr]),
 }

@@ -25,6 +25,7 @@
 #include "kmap.cuh"
 #include "mma_util.cuh"
 #include "voxel_index.cuh"
+#include "plan.cuh"
 #include "vec.cuh"
 
 namespace ptv3 {
@@ -430,9 +431,18 @@ static int launch_conv_direct(const void* feat, const int32_t* indices, const vo
     return check_launch("ptv3_subm_conv_direct_fwd");
 }
 
-static size_t conv_direct_weight_bytes(int ksize) { return align_up((size_t)ksize * ksize * ksize * 8 * 64 * 4, 256); }
+size_t conv_direct_weight_bytes(int ksize) { return align_up((size_t)ksize * ksize * ksize * 8 * 64 * 4, 256); }
 // hash table of blocks (sized for one block per voxel), block counter, one 64-entry table per block
 static size_t conv_direct_index_bytes(int64_t n) { return voxel_index_bytes(n); }
+
+int conv_direct_from_index(const VoxelIndex& vi, const void* feat, const int32_t* indices, const void* weight,
+                           const float* bn_scale, const float* bn_shift, void* out, const int64_t* row_order,
+                           int64_t n, int c_in, int c_out, int ksize, uint32_t* status, void* weight_scratch,
+                           cudaStream_t stream)
+{
+    return launch_conv_direct_mma(feat, indices, weight, nullptr, bn_scale, bn_shift, 1, out, row_order, n, c_in, c_out,
+                                  ksize, vi.keys, vi.vals, vi.cap_mask, vi.cells, status, weight_scratch, stream);
+}
 
 }  // namespace ptv3
 

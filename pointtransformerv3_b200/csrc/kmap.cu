@@ -12,6 +12,7 @@
 #include "common.cuh"
 #include "kmap.cuh"
 #include "voxel_index.cuh"
+#include "plan.cuh"
 
 namespace ptv3 {
 
@@ -153,6 +154,15 @@ int km_build_table(const int32_t* indices, int64_t n, void* workspace, uint32_t*
     return check_launch("voxel hash table");
 }
 
+int kmap_from_index(const VoxelIndex& vi, const int32_t* indices, int64_t n, int ksize, const int64_t* row_order,
+                    int32_t* nbr, uint32_t* status, cudaStream_t stream)
+{
+    km_block_probe_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(indices, n, ksize, vi, nbr, row_order,
+                                                                           status);
+    count_launches(1);
+    return check_launch("ptv3_kmap_build");
+}
+
 }  // namespace ptv3
 
 extern "C" size_t ptv3_kmap_workspace_bytes(int64_t n)
@@ -190,9 +200,7 @@ extern "C" int ptv3_kmap_build_ordered(const int32_t* indices, int64_t n, int ks
         VoxelIndex vi;
         const int rc = build_voxel_index(indices, n, workspace, status, stream, &vi);
         if (rc != PTV3_OK) return rc;
-        km_block_probe_kernel<<<blocks, 256, 0, stream>>>(indices, n, ksize, vi, nbr, row_order, status);
-        count_launches(1);
-        return check_launch("ptv3_kmap_build");
+        return kmap_from_index(vi, indices, n, ksize, row_order, nbr, status, stream);
     }
     const uint64_t cap = km_capacity(n);
     Carver cv(workspace);

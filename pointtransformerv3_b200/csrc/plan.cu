@@ -7,6 +7,7 @@
 // cell are contiguous in every order, so the pooled order of row r is the
 // cluster id sequence along the fine order of row r with repeats removed.
 #include "common.cuh"
+#include "plan.cuh"
 #include "scan.cuh"
 #include "../../include/ptv3_b200.h"
 
@@ -158,7 +159,8 @@ struct OrderSink {
 __global__ void pool_meta_kernel(const uint32_t* __restrict__ totals, int k, int64_t n, int B,
                                  const unsigned long long* __restrict__ scene_count,
                                  int64_t* __restrict__ idx_ptr, int64_t* __restrict__ meta,
-                                 int64_t* __restrict__ meta_host, uint32_t* __restrict__ status)
+                                 int64_t* __restrict__ meta_host, int64_t* __restrict__ offset,
+                                 uint32_t* __restrict__ status)
 {
     if (threadIdx.x == 0 && blockIdx.x == 0) {
         const int64_t m = totals[0];
@@ -166,7 +168,13 @@ __global__ void pool_meta_kernel(const uint32_t* __restrict__ totals, int k, int
         meta[0] = m;
         for (int r = 1; r <= k; ++r)
             if ((int64_t)totals[r] != m) atomicOr(status, PTV3_STATUS_BAD_INDEX);
-        for (int b = 0; b < B; ++b) meta[1 + b] = (int64_t)scene_count[b];
+        int64_t end = 0;
+        for (int b = 0; b < B; ++b) {
+            const int64_t c = (int64_t)scene_count[b];
+            meta[1 + b] = c;
+            end += c;
+            if (offset) offset[b] = end;
+        }
         if (meta_host) {
             // the same numbers and the status word, stored straight into the caller's mapped host
             // memory: the host reads them after waiting for the stream, with no copy in between
@@ -222,7 +230,56 @@ __global__ void __launch_bounds__(256) batch_indices_kernel(const int64_t* __res
     }
 }
 
+// largest coordinate per axis; the block that finishes last stores it, with the offsets, in host memory
+__global__ void __launch_bounds__(256) batch_stats_kernel(const int32_t* __restrict__ grid_coord, int64_t n,
+                                                          const int64_t* __restrict__ offset, int B,
+                                                          int32_t* __restrict__ scratch, int64_t* out_host)
+{
+    int32_t mx[3] = {0, 0, 0};
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride)
+#pragma unroll
+        for (int a = 0; a < 3; ++a) mx[a] = max(mx[a], grid_coord[3 * i + a]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        mx[a] = __reduce_max_sync(0xffffffffu, mx[a]);
+        if ((threadIdx.x & 31) == 0 && mx[a] > 0) atomicMax(&scratch[a], mx[a]);
+    }
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&scratch[3], 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    for (int b = threadIdx.x; b < B; b += blockDim.x) out_host[3 + b] = offset[b];
+    if (threadIdx.x < 3) out_host[threadIdx.x] = atomicMax(&scratch[threadIdx.x], 0);
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        *reinterpret_cast<volatile int64_t*>(&out_host[3 + B]) = 1;
+        __threadfence_system();
+    }
+}
+
 }  // namespace ptv3
+
+extern "C" int ptv3_batch_stats(const int32_t* grid_coord, int64_t n, const int64_t* offset, int n_scenes,
+                                int64_t* out_host, void* scratch, void* stream_)
+{
+    using namespace ptv3;
+    PTV3_REQUIRE(n >= 0 && n_scenes >= 1, PTV3_ERR_INVALID_ARGUMENT, "ptv3_batch_stats: bad sizes");
+    PTV3_REQUIRE((grid_coord || n == 0) && offset && out_host && scratch, PTV3_ERR_INVALID_ARGUMENT,
+                 "ptv3_batch_stats: null pointer");
+    cudaStream_t stream = (cudaStream_t)stream_;
+    if (cudaMemsetAsync(scratch, 0, 16, stream) != cudaSuccess) return check_launch("ptv3_batch_stats");
+    int64_t blocks = (n + 1023) / 1024;         // four points per thread
+    if (blocks < 1) blocks = 1;
+    if (blocks > 148 * 4) blocks = 148 * 4;
+    batch_stats_kernel<<<(unsigned)blocks, 256, 0, stream>>>(grid_coord, n, offset, n_scenes, (int32_t*)scratch,
+                                                             out_host);
+    count_launches(1);
+    return check_launch("ptv3_batch_stats");
+}
 
 extern "C" int ptv3_batch_indices(const int64_t* offset, int n_scenes, const int32_t* grid_coord, int64_t n,
                                   int64_t* batch, int32_t* indices, void* stream)
@@ -271,16 +328,13 @@ extern "C" size_t ptv3_pool_plan_workspace_bytes(int k, int64_t n, int n_scenes)
     return ptv3::pool_ws(k, n, n_scenes).bytes;
 }
 
-extern "C" int ptv3_pool_plan(const int64_t* code, const int64_t* order, const int32_t* grid_coord,
-                              const int64_t* batch, int k, int64_t n, int n_scenes,
-                              int pooling_depth, const int* row_perm, int64_t* cluster,
-                              int64_t* idx_ptr, int64_t* head, int64_t* pooled_code,
-                              int64_t* pooled_order, int64_t* pooled_inverse,
-                              int32_t* pooled_grid_coord, int64_t* pooled_batch, int64_t* meta,
-                              int64_t* meta_host, uint32_t* status, void* workspace,
-                              size_t workspace_bytes, void* stream_)
+int ptv3::pool_plan(const int64_t* code, const int64_t* order, const int32_t* grid_coord, const int64_t* batch, int k,
+                    int64_t n, int n_scenes, int pooling_depth, const int* row_perm, int64_t* cluster,
+                    int64_t* idx_ptr, int64_t* head, int64_t* pooled_code, int64_t* pooled_order,
+                    int64_t* pooled_inverse, int32_t* pooled_grid_coord, int64_t* pooled_batch, int64_t* meta,
+                    int64_t* meta_host, int64_t* pooled_offset, uint32_t* status, void* workspace,
+                    size_t workspace_bytes, cudaStream_t stream)
 {
-    using namespace ptv3;
     PTV3_REQUIRE(k >= 1 && k <= PTV3_MAX_ORDERS && n >= 1 && n_scenes >= 1,
                  PTV3_ERR_INVALID_ARGUMENT, "ptv3_pool_plan: bad k/n/n_scenes");
     PTV3_REQUIRE(pooling_depth >= 0 && pooling_depth <= 16, PTV3_ERR_INVALID_ARGUMENT,
@@ -293,7 +347,6 @@ extern "C" int ptv3_pool_plan(const int64_t* code, const int64_t* order, const i
     const PoolWs w = pool_ws(k, n, n_scenes);
     PTV3_REQUIRE(workspace_bytes >= w.bytes, PTV3_ERR_WORKSPACE,
                  "ptv3_pool_plan: workspace %zu < %zu bytes", workspace_bytes, w.bytes);
-    cudaStream_t stream = (cudaStream_t)stream_;
     Carver cv(workspace);
     uint32_t* tile_sums = cv.take<uint32_t>((size_t)(k + 1) * w.ntiles);
     uint32_t* totals = cv.take<uint32_t>(k + 1);
@@ -321,7 +374,22 @@ extern "C" int ptv3_pool_plan(const int64_t* code, const int64_t* order, const i
     scan_tile_sums_kernel<<<dim3(w.ntiles, k), SC_THREADS, 0, stream>>>(of, n, w.ntiles, ts2);
     scan_sums_kernel<<<k, SC_THREADS, 0, stream>>>(ts2, w.ntiles, totals + 1);
     scan_apply_kernel<<<dim3(w.ntiles, k), SC_THREADS, 0, stream>>>(of, os, n, w.ntiles, ts2);
-    pool_meta_kernel<<<1, 32, 0, stream>>>(totals, k, n, n_scenes, scene_count, idx_ptr, meta, meta_host, status);
+    pool_meta_kernel<<<1, 32, 0, stream>>>(totals, k, n, n_scenes, scene_count, idx_ptr, meta, meta_host,
+                                         pooled_offset, status);
     count_launches(7);
     return check_launch("ptv3_pool_plan");
+}
+
+extern "C" int ptv3_pool_plan(const int64_t* code, const int64_t* order, const int32_t* grid_coord,
+                              const int64_t* batch, int k, int64_t n, int n_scenes,
+                              int pooling_depth, const int* row_perm, int64_t* cluster,
+                              int64_t* idx_ptr, int64_t* head, int64_t* pooled_code,
+                              int64_t* pooled_order, int64_t* pooled_inverse,
+                              int32_t* pooled_grid_coord, int64_t* pooled_batch, int64_t* meta,
+                              int64_t* meta_host, uint32_t* status, void* workspace,
+                              size_t workspace_bytes, void* stream)
+{
+    return ptv3::pool_plan(code, order, grid_coord, batch, k, n, n_scenes, pooling_depth, row_perm, cluster, idx_ptr,
+                           head, pooled_code, pooled_order, pooled_inverse, pooled_grid_coord, pooled_batch, meta,
+                           meta_host, nullptr, status, workspace, workspace_bytes, (cudaStream_t)stream);
 }

@@ -1,0 +1,27 @@
+// Index-side launches that the one-call backbone queues itself.
+#pragma once
+#include "common.cuh"
+#include "voxel_index.cuh"
+
+namespace ptv3 {
+
+// ptv3_pool_plan that also writes the cumulative scene sizes of the pooled level (n_scenes int64)
+int pool_plan(const int64_t* code, const int64_t* order, const int32_t* grid_coord, const int64_t* batch, int k,
+              int64_t n, int n_scenes, int pooling_depth, const int* row_perm, int64_t* cluster, int64_t* idx_ptr,
+              int64_t* head, int64_t* pooled_code, int64_t* pooled_order, int64_t* pooled_inverse,
+              int32_t* pooled_grid_coord, int64_t* pooled_batch, int64_t* meta, int64_t* meta_host,
+              int64_t* pooled_offset, uint32_t* status, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+
+// kernel map of a voxel set whose index exists already
+int kmap_from_index(const VoxelIndex& vi, const int32_t* indices, int64_t n, int ksize, const int64_t* row_order,
+                    int32_t* nbr, uint32_t* status, cudaStream_t stream);
+
+// bf16 stem convolution (+ BatchNorm + GELU) on an existing voxel index; `weight_scratch` holds
+// conv_direct_weight_bytes(ksize) bytes
+size_t conv_direct_weight_bytes(int ksize);
+int conv_direct_from_index(const VoxelIndex& vi, const void* feat, const int32_t* indices, const void* weight,
+                           const float* bn_scale, const float* bn_shift, void* out, const int64_t* row_order,
+                           int64_t n, int c_in, int c_out, int ksize, uint32_t* status, void* weight_scratch,
+                           cudaStream_t stream);
+
+}  // namespace ptv3

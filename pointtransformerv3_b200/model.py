@@ -10,7 +10,7 @@ from functools import partial
 import torch
 import torch.nn as nn
 
-from . import _lib, ops
+from . import _lib, backbone, ops
 from . import sparse as spconv
 from .point import AttrDict, Point, offset2bincount
 
@@ -286,9 +286,9 @@ class Block(PointModule):
         self.drop_path_rate = drop_path
         self.drop_path = PointSequential(nn.Identity())
 
-    def _fusable(self, point):
+    def _fusable_form(self):
         """The fused path covers the reference configuration: pre-norm, plain
-        affine LayerNorms, exact GELU, fp32 or bf16 features."""
+        affine LayerNorms, exact GELU."""
         def plain_ln(m):
             return type(m) is nn.LayerNorm and m.elementwise_affine and m.bias is not None
         mlp = self.mlp[0] if len(self.mlp) == 1 else None
@@ -297,8 +297,11 @@ class Block(PointModule):
                 and len(self.norm1) == 1 and plain_ln(self.norm1[0])
                 and len(self.norm2) == 1 and plain_ln(self.norm2[0])
                 and type(mlp) is MLP and type(mlp.act) is nn.GELU
-                and getattr(mlp.act, "approximate", "none") == "none"
-                and point.feat.dtype in (torch.float32, torch.bfloat16)
+                and getattr(mlp.act, "approximate", "none") == "none")
+
+    def _fusable(self, point):
+        """... on fp32 or bf16 features."""
+        return (self._fusable_form() and point.feat.dtype in (torch.float32, torch.bfloat16)
                 and "sparse_conv_feat" in point.keys())
 
     def _native_args(self, dt, device):
@@ -467,12 +470,15 @@ class SerializedPooling(PointModule):
         self.norm = PointSequential(norm_layer(out_channels)) if norm_layer is not None else None
         self.act = PointSequential(act_layer()) if act_layer is not None else None
 
+    def pooling_depth(self):
+        return (math.ceil(self.stride) - 1).bit_length()
+
     def plan(self, point):
         """Index side of the pooling (model.py:640-680, 690-695): clusters, pooled
         codes/orders/inverses, grid coordinates and scene ids of the coarse level,
         returned as a Point without features.  Draws the order shuffle.  One host
         read (the size of the coarse level)."""
-        pooling_depth = (math.ceil(self.stride) - 1).bit_length()
+        pooling_depth = self.pooling_depth()
         if pooling_depth > point.serialized_depth:
             pooling_depth = 0
         assert {"serialized_code", "serialized_order", "serialized_inverse", "serialized_depth"}.issubset(
@@ -560,11 +566,14 @@ class SerializedUnpooling(PointModule):
             self.proj_skip.add(act_layer())
         self.traceable = traceable
 
-    def _fusable(self):
+    def _fusable_form(self):
         def ok(seq):
-            return (len(seq) == 3 and type(seq[1]) is nn.BatchNorm1d and not seq[1].training
+            return (len(seq) == 3 and type(seq[1]) is nn.BatchNorm1d
                     and type(seq[2]) is nn.GELU and getattr(seq[2], "approximate", "none") == "none")
         return ok(self.proj) and ok(self.proj_skip)
+
+    def _fusable(self):
+        return self._fusable_form() and not self.proj[1].training and not self.proj_skip[1].training
 
     def forward(self, point):
         assert not self.training, "inference only"
@@ -634,6 +643,9 @@ class Embedding(PointModule):
             point.feat = point.sparse_conv_feat.features
             return point
         return self.stem(point)
+
+
+_PLAN_STREAMS = {}      # (device, stream) -> planning stream
 
 
 class PointTransformerV3(PointModule):
@@ -728,12 +740,45 @@ class PointTransformerV3(PointModule):
                 self.dec.add(module=dec, name=f"dec{s}")
 
     def _side_stream(self, device):
-        streams = self.__dict__.setdefault("_ptv3_side_streams", {})
-        if device not in streams:
+        """The planning stream that goes with the current stream (shared by the networks that run there, so
+        that the memory its plans used serves the next network too)."""
+        key = (device, torch.cuda.current_stream(device).cuda_stream)
+        if key not in _PLAN_STREAMS:
             # high priority: the plan kernels are tiny and must not queue behind the blocks of a
             # feature kernel that fills the GPU
-            streams[device] = torch.cuda.Stream(device=device, priority=-1)
-        return streams[device]
+            _PLAN_STREAMS[key] = torch.cuda.Stream(device=device, priority=-1)
+        return _PLAN_STREAMS[key]
+
+    def _native(self, point):
+        """The one-call form of this forward, where it covers the network and the input: bf16 on the GPU,
+        standard modules, nobody hooked onto a single module, no per-operator timing."""
+        feat = point.feat
+        if (feat.dtype != torch.bfloat16 or not feat.is_cuda or feat.dim() != 2 or feat.shape[0] == 0
+                or ops.TIMERS is not None or feat.requires_grad):
+            return None
+        native = backbone.of(self)
+        if native is None or feat.shape[1] != native.width_in or native.observed():
+            return None
+        return native
+
+    def _forward_native(self, native, point, depth):
+        point._ensure_grid_coord()
+        if "sparse_shape" not in point.keys() or depth is None or "_counts" not in point.keys():
+            top, ends = ops.batch_stats(point.grid_coord, point.offset)
+            if depth is None:
+                depth = max(top).bit_length()
+            if "sparse_shape" not in point.keys():
+                point["sparse_shape"] = [v + 96 for v in top]
+            point["_counts"] = [b - a for a, b in zip([0] + ends, ends)]
+        point["_shape_pad"] = point.get("_shape_pad", 96)
+        depth = max(int(depth), 1)
+        assert depth * 3 + len(point["_counts"]).bit_length() <= 63
+        assert depth <= 16
+        point = native.run(self, point, depth, self._side_stream(point.feat.device))
+        point["_defer_status"] = False
+        if not self.defer_status_check:
+            _lib.raise_on_status(point["_status"], "PointTransformerV3.forward")
+        return point
 
     def forward(self, data_dict):
         """data_dict: ``feat``, ``grid_coord`` (or ``coord`` + ``grid_size``) and
@@ -764,6 +809,9 @@ class PointTransformerV3(PointModule):
         status = point.device_status()
         point["_defer_status"] = True
         feat_dtype = point.feat.dtype
+        native = self._native(point)
+        if native is not None:
+            return self._forward_native(native, point, depth)
         # -- Schedule.  Serialization and the pooling plans need only coordinates.  They run on a
         #    second, high-priority stream: a plan has one host read (its size) and a few dozen small
         #    launches, and is made two stages ahead of the features (level 1 while the stem runs,

@@ -344,6 +344,23 @@ def pool_plan(code, order, grid_coord, batch, n_scenes, pooling_depth, row_perm=
                 batch=pbatch[:m], counts=host[1:], m=m, offset=_offsets_to_device(host[1:], dev))
 
 
+def batch_stats(grid_coord, offset):
+    """(largest grid coordinate per axis, offsets) of a batch as Python ints: one kernel that stores
+    them in mapped host memory, which the host polls."""
+    _lib.require_cuda(grid_coord, offset)
+    grid_coord = grid_coord.to(torch.int32).contiguous()
+    offset = offset.to(torch.int64).contiguous()
+    n_scenes = offset.shape[0]
+    host = _pinned(4 + n_scenes, torch.int64, "batch_stats")
+    host[-1] = 0
+    scratch = torch.empty(4, dtype=torch.int32, device=offset.device)
+    _lib.check(_lib.load().ptv3_batch_stats(_lib.ptr(grid_coord), grid_coord.shape[0], _lib.ptr(offset), n_scenes,
+                                            host.data_ptr(), _lib.ptr(scratch), _lib.stream()), "ptv3_batch_stats")
+    _wait_flag(host)
+    got = host.tolist()
+    return got[:3], got[3:-1]
+
+
 POLL_SECONDS = 2.0      # how long a host thread polls a "done" word before it asks the driver
 
 
