@@ -66,6 +66,9 @@ int ptv3_version(void);
 long long ptv3_launch_count(void);
 /* clears a device status word in stream order (a memset, not a kernel) */
 int ptv3_status_reset(uint32_t* status, void* stream);
+/* stores the status word, then 1, in page-locked HOST memory the device can address (2 int64) once the
+   work queued before it has run; the caller zeroes the second word and polls it */
+int ptv3_status_report(const uint32_t* status, int64_t* host, void* stream);
 
 /*
  * Space-filling-curve codes.
@@ -497,6 +500,26 @@ size_t ptv3_voxel_dedup_workspace_bytes(int64_t n);
 int ptv3_voxel_dedup(const int32_t* indices, int64_t n, const int64_t* offset, int n_scenes, int64_t* keep,
                      int64_t* point2voxel, int64_t* new_offset, int64_t* count, uint32_t* status,
                      void* workspace, size_t workspace_bytes, void* stream);
+
+/*
+ * Raw points to one point per voxel in one call (what ptv3_grid_coord, the scene index of every point
+ * and ptv3_voxel_dedup give together), and the rows of the kept points.
+ *   coord        n x 3 fp32; offset: n_scenes cumulative counts
+ *   origin       3 fp32 out: the smallest coordinate per axis
+ *   keep         n int64 (m used): the first point of every occupied voxel, in input order
+ *   point2voxel  n int64: row of every point's voxel among the kept ones; new_offset: n_scenes int64
+ *   count_host   3 int64 of page-locked HOST memory the device can address: m, the status word, 1, stored
+ *                as soon as they are known; the caller zeroes the last word and polls it; count: m on the device
+ * ptv3_voxelize_rows writes coordinates, grid coordinates and features (rows of feat_row_bytes bytes,
+ * any type) of the m kept points.
+ */
+size_t ptv3_voxelize_workspace_bytes(int64_t n);
+int ptv3_voxelize(const float* coord, int64_t n, float grid_size, const int64_t* offset, int n_scenes, float* origin,
+                  int64_t* keep, int64_t* point2voxel, int64_t* new_offset, int64_t* count_host, int64_t* count,
+                  uint32_t* status, void* workspace, size_t workspace_bytes, void* stream);
+int ptv3_voxelize_rows(const int64_t* keep, int64_t m, const float* coord, const float* origin, float grid_size,
+                       const void* feat, int64_t feat_row_bytes, float* out_coord, int32_t* out_grid, void* out_feat,
+                       void* stream);
 
 /*
  * Segmentation head (the step after the backbone; the reference file ends with the

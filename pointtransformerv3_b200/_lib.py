@@ -74,6 +74,7 @@ SIGNATURES = {
                                        c_int, c_int, c_int, c_f32, c_int, c_ptr]),
     "ptv3_kmap_workspace_bytes": (c_sz, [c_i64]),
     "ptv3_status_reset": (c_int, [c_ptr, c_ptr]),
+    "ptv3_status_report": (c_int, [c_ptr, c_ptr, c_ptr]),
     "ptv3_batch_indices": (c_int, [c_ptr, c_int, c_ptr, c_i64, c_ptr, c_ptr, c_ptr]),
     "ptv3_kmap_build": (c_int, [c_ptr, c_i64, c_int, c_ptr, c_ptr, c_ptr, c_sz, c_ptr]),
     "ptv3_kmap_build_ordered": (c_int, [c_ptr, c_i64, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_sz, c_ptr]),
@@ -108,6 +109,10 @@ SIGNATURES = {
     "ptv3_grid_coord": (c_int, [c_ptr, c_i64, c_f32, c_ptr, c_ptr, c_ptr]),
     "ptv3_voxel_dedup_workspace_bytes": (c_sz, [c_i64]),
     "ptv3_voxel_dedup": (c_int, [c_ptr, c_i64, c_ptr, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_sz, c_ptr]),
+    "ptv3_voxelize_workspace_bytes": (c_sz, [c_i64]),
+    "ptv3_voxelize": (c_int, [c_ptr, c_i64, c_f32, c_ptr, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr,
+                              c_sz, c_ptr]),
+    "ptv3_voxelize_rows": (c_int, [c_ptr, c_i64, c_ptr, c_ptr, c_f32, c_ptr, c_i64, c_ptr, c_ptr, c_ptr, c_ptr]),
     "ptv3_seg_head_fwd": (c_int, [c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_i64, c_int, c_int, c_int, c_ptr]),
     "ptv3_pool_stage_supported": (c_int, [c_int, c_int, c_int]),
     "ptv3_pool_stage_workspace_bytes": (c_sz, [c_i64, c_int]),
@@ -194,8 +199,12 @@ STATUS_BITS = {1: "index or size out of range", 2: "hash probe limit reached", 4
 
 
 def raise_on_status(status, what):
-    """Reads the device status word (one host sync) and raises if a bit is set."""
-    v = int(status.item())
+    """Reads the device status word (the host waits for the current stream) and raises if a bit is set."""
+    if status.is_cuda:
+        from . import ops
+        v = ops.read_status(status)
+    else:
+        v = int(status.item())
     if v:
         msg = ", ".join(m for b, m in STATUS_BITS.items() if v & b)
         raise Ptv3Error("%s: device status 0x%x (%s)" % (what, v, msg))

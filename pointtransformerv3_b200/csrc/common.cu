@@ -8,6 +8,14 @@ namespace ptv3 {
 static thread_local char g_err[512] = "";
 static std::atomic<long long> g_launches{0};
 
+static __global__ void status_report_kernel(const uint32_t* status, int64_t* host)
+{
+    host[0] = *status;
+    __threadfence_system();
+    *reinterpret_cast<volatile int64_t*>(&host[1]) = 1;
+    __threadfence_system();
+}
+
 void count_launches(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long long launches() { return g_launches.load(std::memory_order_relaxed); }
 
@@ -34,6 +42,13 @@ int check_launch(const char* what)
 extern "C" const char* ptv3_last_error(void) { return ptv3::g_err; }
 extern "C" int ptv3_version(void) { return 1; }
 extern "C" long long ptv3_launch_count(void) { return ptv3::launches(); }
+extern "C" int ptv3_status_report(const uint32_t* status, int64_t* host, void* stream)
+{
+    PTV3_REQUIRE(status && host, PTV3_ERR_INVALID_ARGUMENT, "ptv3_status_report: null pointer");
+    ptv3::status_report_kernel<<<1, 1, 0, (cudaStream_t)stream>>>(status, host);
+    ptv3::count_launches(1);
+    return ptv3::check_launch("ptv3_status_report");
+}
 extern "C" int ptv3_status_reset(uint32_t* status, void* stream)
 {
     PTV3_REQUIRE(status != nullptr, PTV3_ERR_INVALID_ARGUMENT, "ptv3_status_reset: null pointer");

@@ -6,6 +6,8 @@
 // SerializedPooling.forward).  Pooled orders need no sort: children of a parent
 // cell are contiguous in every order, so the pooled order of row r is the
 // cluster id sequence along the fine order of row r with repeats removed.
+#include <limits.h>
+
 #include "common.cuh"
 #include "plan.cuh"
 #include "scan.cuh"
@@ -230,12 +232,14 @@ __global__ void __launch_bounds__(256) batch_indices_kernel(const int64_t* __res
     }
 }
 
+constexpr int BS_CLEARED = (int)0x80808080;       // scratch words before the kernel: below every coordinate
+
 // largest coordinate per axis; the block that finishes last stores it, with the offsets, in host memory
 __global__ void __launch_bounds__(256) batch_stats_kernel(const int32_t* __restrict__ grid_coord, int64_t n,
                                                           const int64_t* __restrict__ offset, int B,
                                                           int32_t* __restrict__ scratch, int64_t* out_host)
 {
-    int32_t mx[3] = {0, 0, 0};
+    int32_t mx[3] = {INT_MIN, INT_MIN, INT_MIN};
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride)
 #pragma unroll
@@ -243,16 +247,16 @@ __global__ void __launch_bounds__(256) batch_stats_kernel(const int32_t* __restr
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         mx[a] = __reduce_max_sync(0xffffffffu, mx[a]);
-        if ((threadIdx.x & 31) == 0 && mx[a] > 0) atomicMax(&scratch[a], mx[a]);
+        if ((threadIdx.x & 31) == 0) atomicMax(&scratch[a], mx[a]);
     }
     __shared__ bool last;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(&scratch[3], 1) == (int)gridDim.x - 1;
+    if (threadIdx.x == 0) last = atomicAdd(&scratch[3], 1) == BS_CLEARED + (int)gridDim.x - 1;
     __syncthreads();
     if (!last) return;
     for (int b = threadIdx.x; b < B; b += blockDim.x) out_host[3 + b] = offset[b];
-    if (threadIdx.x < 3) out_host[threadIdx.x] = atomicMax(&scratch[threadIdx.x], 0);
+    if (threadIdx.x < 3) out_host[threadIdx.x] = atomicMax(&scratch[threadIdx.x], INT_MIN);
     __threadfence_system();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -271,7 +275,7 @@ extern "C" int ptv3_batch_stats(const int32_t* grid_coord, int64_t n, const int6
     PTV3_REQUIRE((grid_coord || n == 0) && offset && out_host && scratch, PTV3_ERR_INVALID_ARGUMENT,
                  "ptv3_batch_stats: null pointer");
     cudaStream_t stream = (cudaStream_t)stream_;
-    if (cudaMemsetAsync(scratch, 0, 16, stream) != cudaSuccess) return check_launch("ptv3_batch_stats");
+    if (cudaMemsetAsync(scratch, 0x80, 16, stream) != cudaSuccess) return check_launch("ptv3_batch_stats");
     int64_t blocks = (n + 1023) / 1024;         // four points per thread
     if (blocks < 1) blocks = 1;
     if (blocks > 148 * 4) blocks = 148 * 4;

@@ -118,6 +118,16 @@ def new_status(device):
     return status
 
 
+def read_status(status):
+    """The device status word, once the work queued on the current stream has run: stored in mapped
+    host memory by a kernel and polled, which takes a third of the time of a copy and a stream wait."""
+    host = _pinned(2, torch.int64, "status")
+    host[1] = 0
+    _lib.check(_lib.load().ptv3_status_report(_lib.ptr(status), host.data_ptr(), _lib.stream()), "ptv3_status_report")
+    _wait_flag(host)
+    return int(host[0])
+
+
 def pad_layout(counts, patch):
     """Host arithmetic of model.py:392-404: (n_pad, n_seq) from per-scene counts."""
     n_pad = n_seq = 0
@@ -717,6 +727,46 @@ def voxel_dedup(indices, offset=None, status=None):
         raise _lib.Ptv3Error("ptv3_voxel_dedup: device status 0x%x" % host[1])
     m = host[0]
     return dict(keep=keep[:m], point2voxel=p2v, offset=new_offset, m=m)
+
+
+def voxelize(coord, feat, offset, grid_size):
+    """Raw points to one point per voxel: coord (N, 3) float32, feat (N, ...), offset (B,) ->
+    dict(keep, point2voxel, offset, coord, grid_coord, feat).  One host wait (the number of voxels)."""
+    _lib.require_cuda(coord, feat, offset)
+    lib = _lib.load()
+    coord, feat = coord.contiguous(), feat.contiguous()
+    offset = offset.to(torch.int64).contiguous()
+    n, dev, n_scenes = coord.shape[0], coord.device, offset.shape[0]
+    if coord.dtype != torch.float32 or feat.shape[0] != n:
+        raise ValueError("coord must be float32 (N, 3), feat (N, ...)")
+    p2v = torch.empty(n, dtype=torch.int64, device=dev)
+    keep = torch.empty(n, dtype=torch.int64, device=dev)
+    new_offset = torch.empty(n_scenes, dtype=torch.int64, device=dev)
+    small = torch.empty(8, dtype=torch.int32, device=dev)      # origin (3 floats), status, count (int64)
+    status = small[3:4]
+    _lib.check(lib.ptv3_status_reset(_lib.ptr(status), _lib.stream()), "ptv3_status_reset")
+    nbytes = lib.ptv3_voxelize_workspace_bytes(n)
+    ws = _lib.workspace(nbytes, dev)
+    host = _pinned(3, torch.int64, "voxelize")
+    host[-1] = 0
+    with timed("voxelize", 64.0 * n):
+        _lib.check(lib.ptv3_voxelize(_lib.ptr(coord), n, float(grid_size), _lib.ptr(offset), n_scenes, _lib.ptr(small),
+                                     _lib.ptr(keep), _lib.ptr(p2v), _lib.ptr(new_offset), host.data_ptr(),
+                                     _lib.ptr(small[4:]), _lib.ptr(status), _lib.ptr(ws), nbytes, _lib.stream()),
+                   "ptv3_voxelize")
+    _wait_flag(host)
+    m, bits, _ = host.tolist()
+    if bits:
+        raise _lib.Ptv3Error("ptv3_voxelize: device status 0x%x" % bits)
+    out = dict(keep=keep[:m], point2voxel=p2v, offset=new_offset,
+               coord=torch.empty((m, 3), dtype=torch.float32, device=dev),
+               grid_coord=torch.empty((m, 3), dtype=torch.int32, device=dev),
+               feat=torch.empty((m,) + feat.shape[1:], dtype=feat.dtype, device=dev))
+    row_bytes = feat.numel() // n * feat.element_size()
+    _lib.check(lib.ptv3_voxelize_rows(_lib.ptr(keep), m, _lib.ptr(coord), _lib.ptr(small), float(grid_size),
+                                      _lib.ptr(feat), row_bytes, _lib.ptr(out["coord"]), _lib.ptr(out["grid_coord"]),
+                                      _lib.ptr(out["feat"]), _lib.stream()), "ptv3_voxelize_rows")
+    return out
 
 
 def seg_head(feat, weight, bias=None, want_logits=True, want_labels=True):

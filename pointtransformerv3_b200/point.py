@@ -119,6 +119,15 @@ class Point(AttrDict):
             self["grid_coord"] = torch.div(
                 self.coord - self.coord.min(0)[0], self.grid_size, rounding_mode="trunc").int()
 
+    def _bounds(self):
+        """Largest grid coordinate per axis as Python ints (the host waits once; the scene sizes come along)."""
+        if self.grid_coord.is_cuda and "offset" in self.keys() and self.grid_coord.shape[0] > 0:
+            top, ends = ops.batch_stats(self.grid_coord, self.offset)
+            if "_counts" not in self.keys():
+                self["_counts"] = [b - a for a, b in zip([0] + ends, ends)]
+            return top
+        return torch.max(self.grid_coord, dim=0).values.tolist()
+
     def serialization(self, order="z", depth=None, shuffle_orders=False):
         """model.py:81-136: codes of every requested order, their stable argsort
         and inverse; rows optionally shuffled with ``torch.randperm`` on the
@@ -127,7 +136,7 @@ class Point(AttrDict):
         self._ensure_grid_coord()
         order = [order] if isinstance(order, str) else list(order)
         if depth is None:
-            depth = int(self.grid_coord.max()).bit_length()
+            depth = max(self._bounds()).bit_length()
         depth = max(int(depth), 1)
         self["serialized_depth"] = depth
         n_scene_bits = len(self.offset).bit_length()
@@ -164,7 +173,7 @@ class Point(AttrDict):
         if "sparse_shape" in self.keys():
             sparse_shape = self.sparse_shape
         else:
-            sparse_shape = torch.add(torch.max(self.grid_coord, dim=0).values, pad).tolist()
+            sparse_shape = [v + pad for v in self._bounds()]
             self["_shape_pad"] = pad
         self["sparse_shape"] = sparse_shape
         self["sparse_conv_feat"] = SparseConvTensor(

@@ -53,9 +53,10 @@ class SparseConvTensor:
         return SparseConvTensor(feature, self.indices, self.spatial_shape, self.batch_size, self.indice_dict,
                                 self.row_order, self.status, self.defer_status, self.prebuilt)
 
-    def kernel_map(self, kernel_size, indice_key=None):
+    def kernel_map(self, kernel_size, indice_key=None, check=True):
         """(nbr, row_order): the offset-major neighbour table with its columns in
-        ``row_order`` (natural order when that is None)."""
+        ``row_order`` (natural order when that is None).  ``check=False``: the caller reads
+        the tensor's status word itself."""
         key = (indice_key, kernel_size)
         if indice_key is not None and key in self.indice_dict:
             return self.indice_dict[key]
@@ -65,7 +66,7 @@ class SparseConvTensor:
                 self.indice_dict[key] = entry
             return entry
         nbr = ops.kmap_build(self.indices, kernel_size, self.status, self.row_order)
-        if self.status is not None and not self.defer_status:
+        if check and self.status is not None and not self.defer_status:
             from . import _lib
             _lib.raise_on_status(self.status, "ptv3_kmap_build")
         entry = (nbr, self.row_order)
@@ -138,21 +139,26 @@ class SubMConv3d(SparseModule):
                 _lib.raise_on_status(x.status, "ptv3_subm_conv_direct_fwd")
             return x.replace_feature(out)
         assert bn_scale is None and not gelu
-        geo = self.geometry(x)
+        geo = self.geometry(x, check=False)
         if "pair_in" in geo:
-            return x.replace_feature(ops.subm_conv_pairs(x.features, geo, self.weight, self.bias))
-        out = ops.subm_conv(x.features, geo["nbr"], self.weight, self.bias, row_order=geo["row_order"],
-                            status=x.status if x.defer_status else None)
+            out = ops.subm_conv_pairs(x.features, geo, self.weight, self.bias)
+        else:
+            out = ops.subm_conv(x.features, geo["nbr"], self.weight, self.bias, row_order=geo["row_order"],
+                                status=x.status)
+        # one look at the status word covers the kernel map and the convolution
+        if x.status is not None and not x.defer_status:
+            from . import _lib
+            _lib.raise_on_status(x.status, "SubMConv3d")
         return x.replace_feature(out)
 
-    def geometry(self, x):
+    def geometry(self, x, check=True):
         """The index structure this convolution runs on for the sparse tensor ``x``:
         the pair list on the coarsest levels (few voxels, very wide channels: only the
         pairs that exist are multiplied), else dict(nbr, row_order) of the kernel map."""
         if uses_pair_path(x.features.shape[0], self.in_channels, self.out_channels, x.features.dtype,
                           self.kernel_size):
             return x.pair_list(self.kernel_size, self.indice_key)
-        nbr, row_order = x.kernel_map(self.kernel_size, self.indice_key)
+        nbr, row_order = x.kernel_map(self.kernel_size, self.indice_key, check)
         return {"nbr": nbr, "row_order": row_order}
 
 

@@ -20,14 +20,20 @@ def voxelize(coord, feat, offset, grid_size, extra=None):
     backbone; ``point2voxel`` (N,) maps every input point to its row there, for
     scattering per-voxel results back to points.  ``extra``: optional dict of
     further per-point tensors to carry along.  One host read (the voxel count)."""
-    offset = offset.to(torch.int64)
-    batch = offset2batch(offset, coord.shape[0])
-    grid, _ = ops.grid_coord(coord, grid_size)
-    indices = torch.cat([batch.unsqueeze(-1).int(), grid], dim=1).contiguous()
-    d = ops.voxel_dedup(indices, offset)
-    keep = d["keep"]
-    out = {"coord": coord.index_select(0, keep), "grid_coord": grid.index_select(0, keep),
-           "feat": feat.index_select(0, keep), "offset": d["offset"], "grid_size": grid_size}
+    n = coord.shape[0]
+    if coord.dtype == torch.float32 and n and len(offset) <= min(n, 4096):
+        d = ops.voxelize(coord, feat, offset, grid_size)
+        out = {"coord": d["coord"], "grid_coord": d["grid_coord"], "feat": d["feat"]}
+    else:
+        # other coordinate types (the grid is computed in 32 bits), empty input, very many scenes
+        offset = offset.to(torch.int64)
+        grid, _ = ops.grid_coord(coord, grid_size)
+        indices = torch.cat([offset2batch(offset, n).unsqueeze(-1).int(), grid], dim=1).contiguous()
+        d = ops.voxel_dedup(indices, offset)
+        keep = d["keep"]
+        out = {"coord": coord.index_select(0, keep), "grid_coord": grid.index_select(0, keep),
+               "feat": feat.index_select(0, keep)}
+    out["offset"], out["grid_size"] = d["offset"], grid_size
     for k, v in (extra or {}).items():
-        out[k] = v.index_select(0, keep)
+        out[k] = v.index_select(0, d["keep"])
     return out, d["point2voxel"]

@@ -153,3 +153,25 @@ def test_voxelize_feeds_the_backbone():
     assert torch.equal(a, b)
     # per-point results: scatter the voxel features back
     assert a[p2v].shape == (n, a.shape[1])
+
+
+@pytest.mark.parametrize("sizes", [[1], [255], [2048, 1], [2049, 3, 4096], [40000, 1, 17, 9000]])
+@pytest.mark.parametrize("width,dtype", [(6, torch.float32), (3, torch.bfloat16), (8, torch.bfloat16), (5, torch.uint8)])
+def test_voxelize_in_one_call(sizes, width, dtype):
+    """The fused front end against its single operators: scan tiles and their edges, scenes of one point,
+    feature rows of every alignment."""
+    import pointtransformerv3_b200 as P
+    from pointtransformerv3_b200 import ops
+    n = sum(sizes)
+    g = torch.Generator().manual_seed(n)
+    coord = (torch.rand(n, 3, generator=g) * 1.5 - 0.4).cuda()
+    feat = (torch.rand(n, width, generator=g) * 200).to(dtype).cuda()
+    offset = torch.tensor(sizes).cumsum(0).cuda()
+    data, p2v = P.voxelize(coord, feat, offset, 0.05, extra={"row": torch.arange(n).cuda()})
+    grid, _ = ops.grid_coord(coord, 0.05)
+    indices = torch.cat([P.offset2batch(offset, n).unsqueeze(-1).int(), grid], 1).contiguous()
+    want = ops.voxel_dedup(indices, offset)
+    assert torch.equal(p2v, want["point2voxel"]) and torch.equal(data["offset"], want["offset"])
+    assert torch.equal(data["row"], want["keep"])
+    for key, full in (("coord", coord), ("grid_coord", grid), ("feat", feat)):
+        assert torch.equal(data[key], full[want["keep"]]), key
