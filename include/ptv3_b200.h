@@ -69,6 +69,9 @@ int ptv3_status_reset(uint32_t* status, void* stream);
 /* stores the status word, then 1, in page-locked HOST memory the device can address (2 int64) once the
    work queued before it has run; the caller zeroes the second word and polls it */
 int ptv3_status_report(const uint32_t* status, int64_t* host, void* stream);
+/* polls a word of such memory until it is not zero; after two seconds it waits for the stream instead, and
+   fails if the word is still zero then */
+int ptv3_host_wait(const int64_t* word, void* stream);
 
 /*
  * Space-filling-curve codes.
@@ -622,7 +625,8 @@ int ptv3_backbone_fwd(const ptv3_backbone_args* args);
 /*
  * Largest grid coordinate per axis and the scene offsets of a batch, stored by the kernel in
  * page-locked host memory: out_host = {max x, max y, max z, offset[0 .. n_scenes), 1}.  The caller
- * zeroes the last word and polls it.  scratch: 16 bytes of device memory.
+ * zeroes the last word and polls it.  scratch: 16 bytes of device memory, every byte 0x80 before the
+ * first call; each call leaves them so.
  */
 int ptv3_batch_stats(const int32_t* grid_coord, int64_t n, const int64_t* offset, int n_scenes,
                      int64_t* out_host, void* scratch, void* stream);

@@ -74,6 +74,7 @@ SIGNATURES = {
                                        c_int, c_int, c_int, c_f32, c_int, c_ptr]),
     "ptv3_kmap_workspace_bytes": (c_sz, [c_i64]),
     "ptv3_status_reset": (c_int, [c_ptr, c_ptr]),
+    "ptv3_host_wait": (c_int, [c_ptr, c_ptr]),
     "ptv3_status_report": (c_int, [c_ptr, c_ptr, c_ptr]),
     "ptv3_batch_indices": (c_int, [c_ptr, c_int, c_ptr, c_i64, c_ptr, c_ptr, c_ptr]),
     "ptv3_kmap_build": (c_int, [c_ptr, c_i64, c_int, c_ptr, c_ptr, c_ptr, c_sz, c_ptr]),

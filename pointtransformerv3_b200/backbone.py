@@ -199,8 +199,8 @@ class NativeBackbone:
         host_counts = (ctypes.c_int64 * n_scenes)(*counts)
         level_counts = (ctypes.c_int64 * (a.n_enc * n_scenes))()
         ids = (ctypes.c_int * k)(*[ops.ORDER_IDS[o] for o in order])
-        meta = ops._pinned((a.n_enc - 1) * (3 + n_scenes), torch.int64, "backbone.meta")
         main = torch.cuda.current_stream()
+        meta = ops._host_words((a.n_enc - 1) * (3 + n_scenes), "backbone.meta", main.cuda_stream)
         chunks, failed = ([], []), []
 
         def alloc(_, nbytes, pool):
@@ -223,7 +223,7 @@ class NativeBackbone:
         a.indices, a.nbr, a.out = indices.data_ptr(), nbr.data_ptr(), out.data_ptr()
         if pad is not None:
             a.pad, a.unpad, a.cu_seqlens = pad.data_ptr(), unpad.data_ptr(), cu.data_ptr()
-        a.level_counts, a.meta_host, a.status = level_counts, meta.data_ptr(), status.data_ptr()
+        a.level_counts, a.meta_host, a.status = level_counts, meta.address, status.data_ptr()
         a.alloc = _lib.ALLOC_FN(alloc)
         a.main_stream, a.plan_stream = main.cuda_stream, side.cuda_stream
         rc = _lib.load().ptv3_backbone_fwd(ctypes.byref(a))

@@ -9,14 +9,12 @@
 // instead of when its stage comes up.
 #include "common.cuh"
 #include "plan.cuh"
-#include <chrono>
 #include <string.h>
 
 namespace ptv3 {
 
 constexpr int BB_MAX_STAGES = 12;
 constexpr size_t BB_CHUNK = (size_t)16 << 20;       // smallest piece of memory asked for at a time
-constexpr double BB_POLL_SECONDS = 2.0;             // polling before the driver is asked
 
 #define BB_STEP(call)                    \
     do {                                 \
@@ -263,15 +261,7 @@ int Pass::take_plan(bool block)
     volatile int64_t* host = flag(made_ - 1);
     if (!host[2 + a_.n_scenes]) {
         if (!block) return PTV3_OK;
-        const auto began = std::chrono::steady_clock::now();
-        for (uint32_t i = 0; !host[2 + a_.n_scenes]; ++i) {
-            if ((i & 1023) == 1023 &&
-                std::chrono::duration<double>(std::chrono::steady_clock::now() - began).count() > BB_POLL_SECONDS) {
-                BB_CUDA(cudaStreamSynchronize(side_));
-                PTV3_REQUIRE(host[2 + a_.n_scenes], PTV3_ERR_CUDA,
-                             "ptv3_backbone_fwd: a pooling plan finished without reporting its size");
-            }
-        }
+        BB_STEP(host_wait(flag(made_ - 1) + 2 + a_.n_scenes, side_));
     }
     flying_ = false;
     PTV3_REQUIRE(host[1 + a_.n_scenes] == 0, PTV3_ERR_CUDA, "device status 0x%x (read after a pooling plan; the word is "

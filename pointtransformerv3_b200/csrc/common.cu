@@ -1,6 +1,7 @@
 #include "common.cuh"
 #include <stdarg.h>
 #include <atomic>
+#include <chrono>
 #include "../../include/ptv3_b200.h"
 
 namespace ptv3 {
@@ -42,6 +43,27 @@ int check_launch(const char* what)
 extern "C" const char* ptv3_last_error(void) { return ptv3::g_err; }
 extern "C" int ptv3_version(void) { return 1; }
 extern "C" long long ptv3_launch_count(void) { return ptv3::launches(); }
+namespace ptv3 {
+int host_wait(const int64_t* word, cudaStream_t stream)
+{
+    const volatile int64_t* w = word;
+    if (*w) return PTV3_OK;
+    const auto began = std::chrono::steady_clock::now();
+    for (uint32_t i = 1; !*w; ++i) {
+        if ((i & 4095) == 0 && std::chrono::steady_clock::now() - began > std::chrono::seconds(2)) {
+            if (cudaStreamSynchronize(stream) != cudaSuccess) return check_launch("ptv3_host_wait");
+            PTV3_REQUIRE(*w, PTV3_ERR_CUDA, "the kernels of this call finished without reporting their result");
+        }
+    }
+    return PTV3_OK;
+}
+}  // namespace ptv3
+
+extern "C" int ptv3_host_wait(const int64_t* word, void* stream)
+{
+    PTV3_REQUIRE(word, PTV3_ERR_INVALID_ARGUMENT, "ptv3_host_wait: null pointer");
+    return ptv3::host_wait(word, (cudaStream_t)stream);
+}
 extern "C" int ptv3_status_report(const uint32_t* status, int64_t* host, void* stream)
 {
     PTV3_REQUIRE(status && host, PTV3_ERR_INVALID_ARGUMENT, "ptv3_status_report: null pointer");

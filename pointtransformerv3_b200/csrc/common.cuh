@@ -18,6 +18,8 @@ int check_launch(const char* what);
 // Adds to the process-wide count of kernels this library has launched
 // (read through ptv3_launch_count()).
 void count_launches(int n);
+// polls a word of mapped host memory until a kernel of `stream` has stored it (see ptv3_host_wait)
+int host_wait(const int64_t* word, cudaStream_t stream);
 
 #define PTV3_REQUIRE(cond, code, ...)            \
     do {                                         \

@@ -20,8 +20,8 @@ struct OrderList {
 };
 
 // Hilbert transition tables (see hilbert_lut.cuh), evaluated at compile time
-__device__ const hlut::Table1 g_hilbert_t1 = hlut::make_table1();
-__device__ const hlut::Table2 g_hilbert_t2 = hlut::make_table2();
+__device__ __align__(16) const hlut::Table1 g_hilbert_t1 = hlut::make_table1();
+__device__ __align__(16) const hlut::Table2 g_hilbert_t2 = hlut::make_table2();
 
 // The code is handled as two 24-bit words (levels 8..15 and 0..7) so that all
 // arithmetic is 32-bit.  Hilbert code from the Morton words of the same point,
@@ -65,11 +65,14 @@ __global__ void __launch_bounds__(256) encode_kernel(const int32_t* __restrict__
                                                      int depth, OrderList orders,
                                                      int64_t* __restrict__ codes)
 {
-    __shared__ uint16_t t1[48 * 8];
-    __shared__ uint16_t t2[48 * 64];
+    __shared__ __align__(16) uint16_t t1[48 * 8];
+    __shared__ __align__(16) uint16_t t2[48 * 64];
     __shared__ uint32_t sp[256];   // bit i of a byte -> bit 3 i (as z_order.py:12-50 tabulates)
-    for (int i = threadIdx.x; i < 48 * 8; i += blockDim.x) t1[i] = g_hilbert_t1.v[i];
-    for (int i = threadIdx.x; i < 48 * 64; i += blockDim.x) t2[i] = g_hilbert_t2.v[i];
+    // 16 bytes per load: the tables are most of a small call's time
+    for (int i = threadIdx.x; i < 48 * 8 / 8; i += blockDim.x)
+        reinterpret_cast<uint4*>(t1)[i] = reinterpret_cast<const uint4*>(g_hilbert_t1.v)[i];
+    for (int i = threadIdx.x; i < 48 * 64 / 8; i += blockDim.x)
+        reinterpret_cast<uint4*>(t2)[i] = reinterpret_cast<const uint4*>(g_hilbert_t2.v)[i];
     for (int i = threadIdx.x; i < 256; i += blockDim.x) sp[i] = (uint32_t)spread3((uint32_t)i);
     __syncthreads();
     const uint32_t mask = (1u << depth) - 1u;   // depth <= 16

@@ -256,7 +256,10 @@ __global__ void __launch_bounds__(256) batch_stats_kernel(const int32_t* __restr
     __syncthreads();
     if (!last) return;
     for (int b = threadIdx.x; b < B; b += blockDim.x) out_host[3 + b] = offset[b];
-    if (threadIdx.x < 3) out_host[threadIdx.x] = atomicMax(&scratch[threadIdx.x], INT_MIN);
+    if (threadIdx.x < 4) {      // read, and left as the next call wants to find them
+        const int32_t v = atomicExch(&scratch[threadIdx.x], BS_CLEARED);
+        if (threadIdx.x < 3) out_host[threadIdx.x] = v;
+    }
     __threadfence_system();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -275,8 +278,7 @@ extern "C" int ptv3_batch_stats(const int32_t* grid_coord, int64_t n, const int6
     PTV3_REQUIRE((grid_coord || n == 0) && offset && out_host && scratch, PTV3_ERR_INVALID_ARGUMENT,
                  "ptv3_batch_stats: null pointer");
     cudaStream_t stream = (cudaStream_t)stream_;
-    if (cudaMemsetAsync(scratch, 0x80, 16, stream) != cudaSuccess) return check_launch("ptv3_batch_stats");
-    int64_t blocks = (n + 1023) / 1024;         // four points per thread
+    int64_t blocks = (n + 1023) / 1024;         // four points per thread, at most four blocks per SM
     if (blocks < 1) blocks = 1;
     if (blocks > 148 * 4) blocks = 148 * 4;
     batch_stats_kernel<<<(unsigned)blocks, 256, 0, stream>>>(grid_coord, n, offset, n_scenes, (int32_t*)scratch,

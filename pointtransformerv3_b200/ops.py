@@ -4,7 +4,6 @@ Every wrapper allocates outputs and workspaces with torch, passes raw device
 pointers and the current CUDA stream, and raises on a non-zero status."""
 import ctypes
 import threading
-import time
 
 import torch
 
@@ -121,11 +120,11 @@ def new_status(device):
 def read_status(status):
     """The device status word, once the work queued on the current stream has run: stored in mapped
     host memory by a kernel and polled, which takes a third of the time of a copy and a stream wait."""
-    host = _pinned(2, torch.int64, "status")
-    host[1] = 0
-    _lib.check(_lib.load().ptv3_status_report(_lib.ptr(status), host.data_ptr(), _lib.stream()), "ptv3_status_report")
-    _wait_flag(host)
-    return int(host[0])
+    lib, stream = _lib.load(), _lib.stream()
+    host = _host_words(2, "status", stream)
+    host.words[1] = 0
+    _lib.check(lib.ptv3_status_report(status.data_ptr(), host.address, stream), "ptv3_status_report")
+    return host.wait(lib, stream)[0]
 
 
 def pad_layout(counts, patch):
@@ -291,12 +290,12 @@ def _offsets_to_device(counts, dev):
     """Cumulative counts as a device tensor: summed on the host (the counts are there already) and
     copied from pinned memory in stream order.  The pinned words are reused by the next plan, which
     the host only starts after it has waited for kernels queued behind this copy."""
-    off_host = _pinned(len(counts), torch.int64, "pool_plan.offset")
+    off = _host_words(len(counts), "pool_plan.offset", _lib.stream())
     acc = 0
     for i, c in enumerate(counts):
         acc += int(c)
-        off_host[i] = acc
-    return off_host.to(dev, non_blocking=True)
+        off.words[i] = acc
+    return off.tensor.to(dev, non_blocking=True)
 
 
 def pool_plan(code, order, grid_coord, batch, n_scenes, pooling_depth, row_perm=None, status=None):
@@ -331,17 +330,16 @@ def pool_plan(code, order, grid_coord, batch, n_scenes, pooling_depth, row_perm=
     # the sizes of the coarse level and the status word arrive in mapped host memory, written by
     # the plan's last kernel; the host polls the "done" word behind them (a stream wait through
     # the driver takes several times longer to notice the end of a kernel)
-    meta_host = _pinned(3 + n_scenes, torch.int64, "pool_plan.meta")
-    meta_host[-1] = 0
+    stream = _lib.stream()
+    meta_host = _host_words(3 + n_scenes, "pool_plan.meta", stream)
+    meta_host.words[2 + n_scenes] = 0
     _lib.check(lib.ptv3_pool_plan(_lib.ptr(code), _lib.ptr(order), _lib.ptr(grid_coord), _lib.ptr(batch),
                                   k, n, n_scenes, int(pooling_depth), perm, _lib.ptr(cluster),
                                   _lib.ptr(idx_ptr), _lib.ptr(head), _lib.ptr(pcode), _lib.ptr(porder),
                                   _lib.ptr(pinv), _lib.ptr(pgrid), _lib.ptr(pbatch), _lib.ptr(meta),
-                                  ctypes.c_void_p(meta_host.data_ptr()), _lib.ptr(status), _lib.ptr(ws), nbytes,
-                                  _lib.stream()),
+                                  meta_host.address, _lib.ptr(status), _lib.ptr(ws), nbytes, stream),
                "ptv3_pool_plan")
-    _wait_flag(meta_host)                          # the one wait
-    host = meta_host.tolist()[:-1]
+    host = meta_host.wait(lib, stream)[:-1]                          # the one wait
     if host[-1]:
         raise _lib.Ptv3Error("device status 0x%x (read after ptv3_pool_plan; the word is shared by "
                              "every kernel queued with it)" % host[-1])
@@ -358,52 +356,46 @@ def batch_stats(grid_coord, offset):
     """(largest grid coordinate per axis, offsets) of a batch as Python ints: one kernel that stores
     them in mapped host memory, which the host polls."""
     _lib.require_cuda(grid_coord, offset)
+    lib, stream = _lib.load(), _lib.stream()
     grid_coord = grid_coord.to(torch.int32).contiguous()
     offset = offset.to(torch.int64).contiguous()
     n_scenes = offset.shape[0]
-    host = _pinned(4 + n_scenes, torch.int64, "batch_stats")
-    host[-1] = 0
-    scratch = torch.empty(4, dtype=torch.int32, device=offset.device)
-    _lib.check(_lib.load().ptv3_batch_stats(_lib.ptr(grid_coord), grid_coord.shape[0], _lib.ptr(offset), n_scenes,
-                                            host.data_ptr(), _lib.ptr(scratch), _lib.stream()), "ptv3_batch_stats")
-    _wait_flag(host)
-    got = host.tolist()
+    host = _host_words(4 + n_scenes, "batch_stats", stream, offset.device)
+    host.words[3 + n_scenes] = 0
+    _lib.check(lib.ptv3_batch_stats(grid_coord.data_ptr(), grid_coord.shape[0], offset.data_ptr(), n_scenes,
+                                    host.address, host.scratch.data_ptr(), stream), "ptv3_batch_stats")
+    got = host.wait(lib, stream)
     return got[:3], got[3:-1]
 
 
-POLL_SECONDS = 2.0      # how long a host thread polls a "done" word before it asks the driver
+class _HostWords:
+    """Page-locked int64 words that kernels store results in, the last one meaning "done"; with a few
+    bytes of device scratch (0x80 each) for kernels that count their blocks."""
 
-
-def _wait_flag(buf):
-    """Waits until the last word of the pinned tensor ``buf`` is non-zero (stored by the last
-    kernel of a call).  Falls back to waiting for the stream, so a failed launch cannot hang
-    the host."""
-    flag = buf[-1:]
-    deadline = None
-    while int(flag) == 0:
-        if deadline is None:
-            deadline = time.monotonic() + POLL_SECONDS
-        elif time.monotonic() > deadline:
-            torch.cuda.current_stream().synchronize()
-            if int(flag) == 0:
-                raise _lib.Ptv3Error("the kernels of this call finished without reporting their result")
-            break
-
-
-_PINNED = {}
-
-
-def _pinned(numel, dtype, tag):
-    """A cached pinned host buffer per call site, host thread and CUDA stream (a caller
-    synchronises its stream before reading the buffer, so calls that share all three do
-    not overlap)."""
-    key = (tag, numel, dtype, threading.get_ident(), torch.cuda.current_stream().cuda_stream)
-    buf = _PINNED.get(key)
-    if buf is None:
+    def __init__(self, n, device):
         with torch.inference_mode(False):      # a plain tensor: it is written in and out of inference mode
-            buf = torch.empty(numel, dtype=dtype).pin_memory()
-        _PINNED[key] = buf
-    return buf
+            self.tensor = torch.empty(n, dtype=torch.int64).pin_memory()
+            self.scratch = None if device is None else torch.full((16,), 0x80, dtype=torch.uint8, device=device)
+        self.address = self.tensor.data_ptr()
+        self.words = (ctypes.c_int64 * n).from_address(self.address)
+        self.last = self.address + 8 * (n - 1)
+
+    def wait(self, lib, stream):
+        _lib.check(lib.ptv3_host_wait(self.last, stream), "waiting for a result")
+        return self.words[:]
+
+
+_HOST_WORDS = {}
+
+
+def _host_words(n, tag, stream, device=None):
+    """The words of a call site, host thread and CUDA stream (a caller waits for its result before it
+    comes back here, so calls that share all three do not overlap)."""
+    key = (tag, n, threading.get_ident(), stream, device)
+    host = _HOST_WORDS.get(key)
+    if host is None:
+        host = _HOST_WORDS[key] = _HostWords(n, device)
+    return host
 
 
 REDUCE_IDS = {"max": 0, "min": 1, "sum": 2, "mean": 3}
@@ -747,15 +739,15 @@ def voxelize(coord, feat, offset, grid_size):
     _lib.check(lib.ptv3_status_reset(_lib.ptr(status), _lib.stream()), "ptv3_status_reset")
     nbytes = lib.ptv3_voxelize_workspace_bytes(n)
     ws = _lib.workspace(nbytes, dev)
-    host = _pinned(3, torch.int64, "voxelize")
-    host[-1] = 0
+    stream = _lib.stream()
+    host = _host_words(3, "voxelize", stream)
+    host.words[2] = 0
     with timed("voxelize", 64.0 * n):
         _lib.check(lib.ptv3_voxelize(_lib.ptr(coord), n, float(grid_size), _lib.ptr(offset), n_scenes, _lib.ptr(small),
-                                     _lib.ptr(keep), _lib.ptr(p2v), _lib.ptr(new_offset), host.data_ptr(),
+                                     _lib.ptr(keep), _lib.ptr(p2v), _lib.ptr(new_offset), host.address,
                                      _lib.ptr(small[4:]), _lib.ptr(status), _lib.ptr(ws), nbytes, _lib.stream()),
                    "ptv3_voxelize")
-    _wait_flag(host)
-    m, bits, _ = host.tolist()
+    m, bits, _ = host.wait(lib, stream)
     if bits:
         raise _lib.Ptv3Error("ptv3_voxelize: device status 0x%x" % bits)
     out = dict(keep=keep[:m], point2voxel=p2v, offset=new_offset,
