@@ -325,8 +325,7 @@ int launch_attn_mma(const void* qkv, const int64_t* order, const int64_t* pad, c
     const size_t smem = (size_t)lpad * 68;      // K, V and the row numbers
     // per device and cheap, so it is simply repeated on every call
     auto kern = packed_exp ? attn_mma_d16_kernel<true> : attn_mma_d16_kernel<false>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ATTN_MMA_MAX_SEQLEN * 68) !=
-        cudaSuccess)
+    if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_attention_fwd: shared memory attribute");
     // slice the queries of a sequence over several CTAs when there are few (sequence, head) pairs
     int qsplit = 1;

@@ -542,8 +542,7 @@ int launch_attn_tc05(const void* qkv, const int64_t* order, const int64_t* pad, 
     // second CTA shares the SM (it would wait in tcgen05.alloc).
     const size_t floor_smem = (size_t)(228 * 1024 / 2 + 1024);
     const size_t smem = lay.total + 128 < floor_smem ? floor_smem : (size_t)lay.total + 128;
-    if (cudaFuncSetAttribute(attn_tc05_d16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
+    if (allow_smem(attn_tc05_d16_kernel) != cudaSuccess)
         return check_launch("ptv3_attention_fwd: shared memory attribute");
     // Query tiles of a patch can be sliced over CTAs (each gathers K and V again).  Pick the
     // slicing with the shortest estimated time: waves of 148 CTAs, each taking one gather

@@ -58,20 +58,59 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
-static inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                           cudaStream_t stream, Args... args)
+static inline cudaError_t launch_dependent_cluster(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                                   cudaStream_t stream, dim3 cluster, Args... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster.x;
+    attr[1].val.clusterDim.y = cluster.y;
+    attr[1].val.clusterDim.z = cluster.z;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster.x * cluster.y * cluster.z > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+static inline cudaError_t launch_dependent(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                           cudaStream_t stream, Args... args)
+{
+    return launch_dependent_cluster(kern, grid, block, smem, stream, dim3(1, 1, 1), args...);
+}
+
+// Lets a kernel take all the shared memory of an SM that its static part leaves, asked for once per thread,
+// device and kernel: the driver call costs as much as a third of a launch.  (Always the same value, so that
+// threads do not undo one another's.)
+template <typename K>
+static inline cudaError_t allow_smem(K kern)
+{
+    struct Seen {
+        const void* kern;
+        int device;
+    };
+    static thread_local Seen seen[16] = {};      // kernels of one signature share an instance
+    static thread_local int next = 0;
+    int device = -1;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    for (const Seen& s : seen)
+        if (s.kern == (const void*)kern && s.device == device) return cudaSuccess;
+    cudaFuncAttributes attr;
+    e = cudaFuncGetAttributes(&attr, (const void*)kern);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             227 * 1024 - (int)attr.sharedSizeBytes);
+    if (e == cudaSuccess) {
+        seen[next] = Seen{(const void*)kern, device};
+        next = (next + 1) % 16;
+    }
+    return e;
 }
 #endif
 

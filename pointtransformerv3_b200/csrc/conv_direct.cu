@@ -366,8 +366,7 @@ static int launch_conv_direct_mma(const void* feat, const int32_t* indices, cons
 #define CDM_LAUNCH(NT)                                                                                      \
     do {                                                                                                    \
         auto kern = conv_direct_mma_kernel<NT>;                                                             \
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=           \
-            cudaSuccess)                                                                                    \
+        if (allow_smem(kern) != cudaSuccess)                                                \
             return check_launch("ptv3_subm_conv_direct_fwd: shared memory attribute");                      \
         kern<<<blocks, CD_THREADS, smem, stream>>>(                                                          \
             (const __nv_bfloat16*)feat, indices, (const __nv_bfloat16*)wt, (const __nv_bfloat16*)bias,       \
@@ -405,8 +404,7 @@ static int launch_conv_direct(const void* feat, const int32_t* indices, const vo
 #define CD_LAUNCH(CO)                                                                                    \
     do {                                                                                                 \
         auto kern = conv_direct_kernel<T, CO>;                                                           \
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=        \
-            cudaSuccess)                                                                                 \
+        if (allow_smem(kern) != cudaSuccess)                                                \
             return check_launch("ptv3_subm_conv_direct_fwd: shared memory attribute");                   \
         kern<<<blocks, CD_THREADS, smem, stream>>>((const T*)feat, indices, (const T*)weight,             \
                                                    (const T*)bias, bn_scale, bn_shift, apply_gelu,        \

@@ -274,7 +274,7 @@ static int launch_one(const void* feat, const int32_t* nbr, const void* weight, 
 {
     constexpr size_t smem = conv_mma_smem<CM_TM, CN, KC>();
     auto kern = conv_mma_kernel<CM_TM, CN, KC, WM, WN, false>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_subm_conv_fwd: shared memory attribute");
     const dim3 grid((unsigned)((n + CM_TM - 1) / CM_TM), cout / CN);
     launch_dependent(kern, grid, dim3(WM * WN * 32), smem, stream, (const __nv_bfloat16*)feat, nbr,
@@ -324,7 +324,7 @@ int launch_conv_pairs(const void* feat, const int32_t* pair_in, const int32_t* p
 {
     constexpr size_t smem = conv_mma_smem<128, 128, 64>();
     auto kern = conv_mma_kernel<128, 128, 64, 4, 2, true>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_subm_conv_pairs_fwd: shared memory attribute");
     if (cudaMemsetAsync(acc, 0, (size_t)n * c_out * sizeof(long long), stream) != cudaSuccess)
         return check_launch("ptv3_subm_conv_pairs_fwd: memset");

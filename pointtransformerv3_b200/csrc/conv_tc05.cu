@@ -28,9 +28,16 @@
 // core, 13 % copies and loads), L2 19 %, DRAM 5 %; leaving out the gather copies or the weight
 // loads altogether changes the time by 10 % and 2 %.
 //
+// Few tiles (the coarse levels, small rooms): a cluster of up to eight CTAs shares one tile.  Each takes a
+// contiguous share of the tile's stages; the partial sums meet in shared memory and every CTA adds the
+// peers' parts of its rows, in rank order, through distributed shared memory.  A tile alone walks
+// 27 x c_in / 64 stages one after the other, 49 us at 512 channels on 27 voxels, while most SMs have nothing.
+//
 // Replaces spconv.SubMConv3d.forward at model.py:546-552 for bf16.
 // Useful work: 2 . pairs . C_in . C_out FLOP.  Every mbarrier wait is bounded and reports through
 // the status word.
+#include <atomic>
+
 #include "common.cuh"
 #include "conv_mma.cuh"
 #include "mma_util.cuh"
@@ -56,7 +63,7 @@ struct ConvTcArgs {
     uint32_t* status;
 };
 
-template <int BN, int KC, int STAGES, int NI>
+template <int BN, int KC, int STAGES, int NI, bool SPLIT>
 __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                const ConvTcArgs a)
 {
@@ -79,6 +86,11 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
     // ask for the slot of stage X + NGW only if stage X + NGW - 2 STAGES is known to be consumed,
     // i.e. NGW <= STAGES (the products run in order).
     constexpr int NGW = STAGES < CT_GATHER_WARPS ? STAGES : CT_GATHER_WARPS;
+
+    // partial sums of a split tile, over the ring: rows of BN floats, padded so that 16-byte accesses of
+    // consecutive rows spread over the banks
+    constexpr int PART_PITCH = BN + 4;
+    static_assert(!SPLIT || CT_TM * PART_PITCH * 4 <= STAGES * STAGE_BYTES, "partial sums fit the ring");
 
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -164,7 +176,13 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
     const uint32_t tmem_base = *tmem_slot;
     const int n_act = act[0];
     const int kchunks = a.cin / KC;
-    const int nit = n_act * kchunks;
+    // this CTA's share of the tile's stages (all of them without a cluster)
+    int first = 0, nit = n_act * kchunks;
+    if (SPLIT) {
+        const int total = nit, parts = (int)gridDim.z;
+        first = total * (int)blockIdx.z / parts;
+        nit = total * ((int)blockIdx.z + 1) / parts - first;
+    }
     bool ok = true;
 
     if (warp < CT_GATHER_WARPS) {
@@ -180,8 +198,8 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
                 if (it >= STAGES) ok &= mbar_wait(empty0 + 8 * s, ((it / STAGES) & 1) ^ 1, abort);
             }
             __syncwarp();
-            const int o = act[1 + it / kchunks];
-            const int kc = (it % kchunks) * KC;
+            const int o = act[1 + (first + it) / kchunks];
+            const int kc = ((first + it) % kchunks) * KC;
             const uint32_t sa = sbase + s * STAGE_BYTES;
             const __nv_bfloat16* src0 = a.feat + kc + c * 8;
             const int32_t* nb = nbr_s + o * CT_TM + rr;
@@ -242,6 +260,15 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
 #pragma unroll
                 for (int i = 0; i < 32; ++i) acc[i] = 0;
             }
+            if (SPLIT) {
+                // (the ring is free: every product has completed)
+                float* prow = reinterpret_cast<float*>(smem) + (q * 32 + lane) * PART_PITCH + cb * 32;
+#pragma unroll
+                for (int g = 0; g < 8; ++g)
+                    *reinterpret_cast<uint4*>(prow + g * 4) = make_uint4(acc[g * 4], acc[g * 4 + 1], acc[g * 4 + 2],
+                                                                         acc[g * 4 + 3]);
+                continue;
+            }
             if (v < 0) continue;
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
@@ -278,6 +305,28 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
             else if (nit > 0) mbar_arrive_one(accfull);
         }
     }
+    if (SPLIT) {
+        // this CTA's rows: the peers' partial sums in rank order, bias, bf16
+        cluster_sync();
+        const int parts = (int)gridDim.z, rows = CT_TM / parts, r0 = rows * (int)cluster_rank();
+        for (int e = tid; e < rows * (BN / 4); e += CT_THREADS) {
+            const int r = r0 + e / (BN / 4), c = e % (BN / 4) * 4;
+            const int64_t v = rows_s[r];
+            if (v < 0) continue;
+            const uint32_t at = sbase + (r * PART_PITCH + c) * 4;
+            float4 t = ld_peer_f4(at, 0);
+            for (int z = 1; z < parts; ++z) {
+                const float4 m = ld_peer_f4(at, z);
+                t.x += m.x;
+                t.y += m.y;
+                t.z += m.z;
+                t.w += m.w;
+            }
+            *reinterpret_cast<uint2*>(a.out + v * a.cout + col0 + c) =
+                make_uint2(pack_bf16(t.x + bias_s[c], t.y + bias_s[c + 1]), pack_bf16(t.z + bias_s[c + 2], t.w + bias_s[c + 3]));
+        }
+        cluster_sync();      // a peer's shared memory outlives its readers
+    }
     fence_before_sync();
     __syncthreads();
     if (warp == CT_GATHER_WARPS) {
@@ -294,23 +343,80 @@ bool conv_tc05_supported(int c_in, int c_out, int kernel_volume)
     return c_in % 64 == 0 && c_in <= 4096 && c_out % 64 == 0 && c_out <= 4096;
 }
 
-template <int BN, int KC, int STAGES, int NI>
-static int launch_conv_tc05_as(const void* weight, const ConvTcArgs& a, cudaStream_t stream)
+template <int BN, int KC, int STAGES>
+static constexpr size_t conv_tc05_smem()
+{
+    return (size_t)STAGES * (CT_TM + BN) * KC * 2 + CT_MAX_KVOL * CT_TM * 4 + CT_TM * 8 + 32 * 4 + BN * 4 +
+           8 * (2 * STAGES + 1) + 16 + 1024;
+}
+
+template <int BN, int KC, int STAGES, int NI, bool SPLIT>
+static int launch_conv_tc05_as(const void* weight, const ConvTcArgs& a, cudaStream_t stream, int parts)
 {
     CUtensorMap mw;
     const uint64_t wcols = (uint64_t)a.kvol * a.cin;
     const int rc = make_tensor_map_bf16(&mw, weight, (uint64_t)a.cout, wcols, wcols * 2, BN, KC);
     if (rc) return rc;
-    constexpr size_t smem = (size_t)STAGES * (CT_TM + BN) * KC * 2 + CT_MAX_KVOL * CT_TM * 4 + CT_TM * 8 + 32 * 4 +
-                            BN * 4 + 8 * (2 * STAGES + 1) + 16 + 1024;
-    auto kern = conv_tc05_kernel<BN, KC, STAGES, NI>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    constexpr size_t smem = conv_tc05_smem<BN, KC, STAGES>();
+    auto kern = conv_tc05_kernel<BN, KC, STAGES, NI, SPLIT>;
+    if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_subm_conv_fwd: shared memory attribute");
-    const dim3 grid((unsigned)((a.n + CT_TM - 1) / CT_TM), a.cout / BN);
-    launch_dependent(kern, grid, dim3((CT_GATHER_WARPS + NI) * 32), smem, stream, mw, a);
+    const dim3 grid((unsigned)((a.n + CT_TM - 1) / CT_TM), a.cout / BN, parts);
+    launch_dependent_cluster(kern, grid, dim3((CT_GATHER_WARPS + NI) * 32), smem, stream, dim3(1, 1, parts), mw, a);
     count_launches(1);
     return check_launch("ptv3_subm_conv_fwd");
 }
+
+// CTAs in clusters of `parts` that run at once (the driver's answer: a cluster lives in one GPC)
+template <int BN, int KC, int STAGES, int NI>
+static int conv_tc05_capacity(int parts)
+{
+    static std::atomic<int> known[4];
+    const int slot = parts == 2 ? 1 : parts == 4 ? 2 : 3;
+    int c = known[slot].load(std::memory_order_relaxed);
+    if (c == 0) {
+        auto kern = conv_tc05_kernel<BN, KC, STAGES, NI, true>;
+        if (allow_smem(kern) != cudaSuccess) return 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(148, 1, parts);
+        cfg.blockDim = dim3((CT_GATHER_WARPS + NI) * 32);
+        cfg.dynamicSmemBytes = conv_tc05_smem<BN, KC, STAGES>();
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = parts;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            clusters = 0;
+        }
+        c = clusters > 0 ? clusters * parts : -1;
+        known[slot].store(c, std::memory_order_relaxed);
+    }
+    return c;
+}
+
+struct ConvVariant {
+    int bn, per_sm;
+    double stage_us;
+    int (*plain)(const void*, const ConvTcArgs&, cudaStream_t, int);
+    int (*split)(const void*, const ConvTcArgs&, cudaStream_t, int);
+    int (*capacity)(int);
+};
+constexpr double CT_FIXED_US = 6.5;
+constexpr int CT_VARIANTS = 4;
+static const ConvVariant g_variants[CT_VARIANTS] = {
+    {64, 1, 0.20, launch_conv_tc05_as<64, 64, 8, 2, false>, launch_conv_tc05_as<64, 64, 8, 2, true>,
+     conv_tc05_capacity<64, 64, 8, 2>},
+    // many tiles: two CTAs per SM, so that one tile's prologue and epilogue run beside another's products
+    {64, 2, 0.35, launch_conv_tc05_as<64, 64, 4, 2, false>, nullptr, nullptr},
+    {128, 1, 0.28, launch_conv_tc05_as<128, 64, 6, 2, false>, launch_conv_tc05_as<128, 64, 6, 2, true>,
+     conv_tc05_capacity<128, 64, 6, 2>},
+    {256, 1, 0.44, launch_conv_tc05_as<256, 64, 4, 2, false>, launch_conv_tc05_as<256, 64, 4, 2, true>,
+     conv_tc05_capacity<256, 64, 4, 2>},
+};
 
 int launch_conv_tc05(const void* feat, const int32_t* nbr, const void* weight, const void* bias, void* out,
                      const int64_t* row_order, int64_t n, int c_in, int c_out, int kvol, uint32_t* status,
@@ -327,16 +433,35 @@ int launch_conv_tc05(const void* feat, const int32_t* nbr, const void* weight, c
     a.cout = c_out;
     a.kvol = kvol;
     a.status = status;
-    if (c_in == 32) return launch_conv_tc05_as<32, 32, 6, 2>(weight, a, stream);
-    // 128 output channels per CTA halve the gathers of a tile; 64 when that would leave SMs idle
+    if (c_in == 32) return launch_conv_tc05_as<32, 32, 6, 2, false>(weight, a, stream, 1);
+    // The tile width and the cluster size with the shortest estimated time: waves of CTAs, each taking a
+    // fixed time (prologue, epilogue) and its stages.  Wide tiles gather a row once for more output
+    // channels; clusters fill SMs that a single wave leaves idle.  The constants are measured (us on B200:
+    // 27 voxels x 512 channels in clusters of eight takes 12.2 / 14.6 / 19.9 with 64 / 128 / 256 channels a
+    // tile, 46.3 without a cluster); what they give: 441 x 512 47 -> 19, 1 700 x 256 27 -> 18,
+    // 2 200 x 512 49 -> 39, 12 000 x 256 68 -> 53, 12 000 x 128 31 -> 22.
+    const double stages = (double)kvol * (c_in / 64);
     const int64_t tiles = (n + CT_TM - 1) / CT_TM;
-    // long inputs with wide outputs: 256 output channels per CTA (the gathers of a tile once more halved,
-    // every product twice as wide), four stages of 48 KiB
-    if (c_out % 256 == 0 && tiles * (c_out / 256) >= 148) return launch_conv_tc05_as<256, 64, 4, 2>(weight, a, stream);
-    if (c_out % 128 == 0 && tiles * (c_out / 128) >= 120) return launch_conv_tc05_as<128, 64, 6, 2>(weight, a, stream);
-    // many tiles: two CTAs per SM, so that one tile's prologue and epilogue run beside another's products
-    if (tiles * (c_out / 64) >= 2 * 148) return launch_conv_tc05_as<64, 64, 4, 2>(weight, a, stream);
-    return launch_conv_tc05_as<64, 64, 8, 2>(weight, a, stream);
+    double best = 0;
+    int best_v = -1, best_parts = 1;
+    for (int v = 0; v < CT_VARIANTS; ++v) {
+        const ConvVariant& var = g_variants[v];
+        if (c_out % var.bn) continue;
+        const int64_t ctas = tiles * (c_out / var.bn);
+        for (int parts = 1; parts <= (var.split ? 8 : 1); parts *= 2) {
+            const int64_t room = parts == 1 ? (int64_t)148 * var.per_sm : (int64_t)var.capacity(parts);
+            if (room < parts) continue;
+            if (parts > 1 && (ctas * parts > room || stages < 2 * parts)) continue;       // a cluster only within one wave
+            const double cost = (double)((ctas * parts + room - 1) / room) * (CT_FIXED_US + stages / parts * var.stage_us);
+            if (best_v < 0 || cost < best) {
+                best = cost;
+                best_v = v;
+                best_parts = parts;
+            }
+        }
+    }
+    const ConvVariant& var = g_variants[best_v];
+    return (best_parts > 1 ? var.split : var.plain)(weight, a, stream, best_parts);
 }
 
 }  // namespace ptv3

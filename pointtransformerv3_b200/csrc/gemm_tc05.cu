@@ -284,7 +284,7 @@ static int launch_gemm_mode(const CUtensorMap& mx, const CUtensorMap& mw, const 
                               : (size_t)STAGES * (GM_A_BYTES + b_bytes)) +
                         GM_OUT_TOTAL + BN * 4 + 8 * (2 * STAGES + 5) + 16 + 1024;
     auto kern = gemm_tc05_kernel<BN, STAGES, MODE, WRES>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_gemm_fwd: shared memory attribute");
     a.col_tiles = a.n_out / BN;
     const int64_t tiles = (int64_t)a.row_tiles * a.col_tiles;

@@ -518,8 +518,7 @@ static int launch_linear(const void* x, const void* w, LinearArgs a, int k, cuda
 #define LIN_LAUNCH(KK)                                                                                       \
     do {                                                                                                     \
         auto kern = linear_tc05_kernel<KK>;                                                                  \
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_req) !=        \
-            cudaSuccess)                                                                                     \
+        if (allow_smem(kern) != cudaSuccess)                                                \
             return check_launch("ptv3_linear_fwd: shared memory attribute");                                 \
         launch_dependent(kern, dim3((unsigned)grid), dim3(512), smem_req, stream, mx, mw, mo, a);                \
     } while (0)

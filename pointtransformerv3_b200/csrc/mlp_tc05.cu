@@ -283,7 +283,7 @@ static int launch_mlp(const void* x, const void* w1, const void* b1, const void*
     rc = make_tensor_map_bf16(&mw2, w2, C, Cfg::HD, (uint64_t)Cfg::HD * 2, C, 64);
     if (rc) return rc;
     auto kern = mlp_tc05_kernel<C>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM) != cudaSuccess)
+    if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_mlp_fwd: shared memory attribute");
     const int64_t ntiles = (n + 127) / 128;
     int64_t grid = (ntiles + Cfg::NG - 1) / Cfg::NG;

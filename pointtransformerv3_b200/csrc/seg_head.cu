@@ -94,7 +94,7 @@ static int launch_seg_head(const void* feat, const void* weight, const void* bia
     do {                                                                                                         \
         auto kern = seg_head_kernel<T, KMAX>;                                                                    \
         if (smem > 48 * 1024 &&                                                                                  \
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)   \
+            allow_smem(kern) != cudaSuccess)                                                \
             return check_launch("ptv3_seg_head_fwd: shared memory attribute");                                   \
         kern<<<blocks, SH_THREADS, smem, stream>>>((const T*)feat, (const T*)weight, (const T*)bias, (T*)logits, \
                                                    labels, n, C, K);                                             \

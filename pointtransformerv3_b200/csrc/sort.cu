@@ -426,17 +426,9 @@ extern "C" int ptv3_argsort_inverse(const int64_t* codes, int k, int64_t n, int 
         os_hist_kernel<<<dim3(hb, k), OS_THREADS, (size_t)p.passes * OS_MAX_BINS * sizeof(uint32_t), stream>>>(
             kin, n, sig_bits, p.bits, p.passes, hist);
     }
-    const size_t max_smem = os_pass_smem(OS_MAX_BITS);
-    {
-        auto set = [&](const void* f) {
-            return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
-        };
-        if (set((const void*)os_pass_kernel<true, true>) != cudaSuccess ||
-            set((const void*)os_pass_kernel<true, false>) != cudaSuccess ||
-            set((const void*)os_pass_kernel<false, true>) != cudaSuccess ||
-            set((const void*)os_pass_kernel<false, false>) != cudaSuccess)
-            return check_launch("ptv3_argsort_inverse: shared memory attribute");
-    }
+    if (allow_smem(os_pass_kernel<true, true>) != cudaSuccess || allow_smem(os_pass_kernel<true, false>) != cudaSuccess ||
+        allow_smem(os_pass_kernel<false, true>) != cudaSuccess || allow_smem(os_pass_kernel<false, false>) != cudaSuccess)
+        return check_launch("ptv3_argsort_inverse: shared memory attribute");
     const dim3 grid((unsigned)((size_t)p.ntiles * k));
     const int32_t* vin = nullptr;
     int cur = 0;

@@ -201,6 +201,31 @@ __device__ __forceinline__ void tmem_ld_fence(uint32_t (&r)[32])
                  : "memory");
 }
 
+// ---- clusters -------------------------------------------------------------------
+__device__ __forceinline__ uint32_t cluster_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// all threads of all CTAs of the cluster; shared-memory writes before it are seen by the peers after it
+__device__ __forceinline__ void cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// four floats of a peer's shared memory at this CTA's address `addr`
+__device__ __forceinline__ float4 ld_peer_f4(uint32_t addr, uint32_t rank)
+{
+    uint32_t p;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(p)
+                 : "memory");
+    return v;
+}
+
 __device__ __forceinline__ void named_barrier(int id, int threads)
 {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");

@@ -385,6 +385,25 @@ def test_subm_conv_tcgen05_wide_tiles(voxels, cin, cout):
     assert_close(got, base, atol=1e-2, rtol=1e-2, what="tcgen05 vs mma.sync conv")
 
 
+@pytest.mark.parametrize("n", [1, 127, 129, 900])
+@pytest.mark.parametrize("c", [64, 128, 256, 512])
+def test_subm_conv_tcgen05_clusters(n, c):
+    """Few tiles: a cluster of CTAs shares a tile (up to eight of them), with shares of zero stages,
+    ragged tiles and rows without a neighbour; against the mma.sync path, twice for the same bits."""
+    g = torch.Generator().manual_seed(n + c)
+    cells = torch.randperm(2 * n + 20, generator=g)[:n]
+    ind = torch.stack([torch.zeros_like(cells), cells // 40, cells % 40 // 4, cells % 4], 1).int().cuda()
+    nbr = ops.kmap_build(ind, 3)
+    feat = torch.randn(n, c, generator=g).bfloat16().cuda()
+    w = (torch.randn(c, 3, 3, 3, c, generator=g) / (9 * c) ** 0.5).bfloat16().cuda()
+    b = (torch.randn(c, generator=g) * 0.1).bfloat16().cuda()
+    got = ops.subm_conv(feat, nbr, w, b, algo=3)
+    assert torch.equal(got, ops.subm_conv(feat, nbr, w, b, algo=3))
+    base = ops.subm_conv(feat, nbr, w, b, algo=2)
+    assert_close(got, base, atol=1e-2, rtol=1e-2, what="clusters vs mma.sync conv")
+    assert rel_l2(got, base) < 2e-3
+
+
 @pytest.mark.parametrize("permuted", [False, True])
 @pytest.mark.parametrize("cin,cout,shift", [(32, 32, 0), (64, 64, 0), (128, 128, 1), (256, 256, 2), (512, 512, 3),
                                             (64, 192, 1)])
