@@ -14,6 +14,7 @@
 // their epilogue (linear_tc05.cu) and, up to 64, the fused MLP; wider blocks take the
 // streamed-weight tensor-core kernel (gemm_tc05.cu) and the fused row kernel for the glue.
 #include "common.cuh"
+#include "linear_small.cuh"
 #include "vec.cuh"
 
 namespace ptv3 {
@@ -29,12 +30,23 @@ static bool linear_any_supported(int k, int n_out, bool epilogue)
 static int linear_any(const void* x, const void* w, const void* bias, const void* residual, void* out, int64_t n,
                       int k, int n_out, int gelu, uint32_t* status, void* stream)
 {
+    if (linear_small_wanted(n, k, n_out))
+        return launch_linear_small(x, w, bias, residual, out, n, k, n_out, gelu, status, (cudaStream_t)stream);
     if (ptv3_gemm_supported(k, n_out, PTV3_DTYPE_BF16))
         return ptv3_gemm_fwd(x, w, bias, residual, out, n, k, n_out, gelu, PTV3_DTYPE_BF16, status, stream);
     if (!gelu && !residual && ptv3_linear_supported(k, n_out, 0, PTV3_DTYPE_BF16))
         return ptv3_linear_fwd(x, w, bias, out, n, k, n_out, PTV3_DTYPE_BF16, status, stream);
     set_error("no tensor-core Linear kernel for %d -> %d channels", k, n_out);
     return PTV3_ERR_UNSUPPORTED;
+}
+
+// The two MLP layers in one kernel, where there is one and the input is long enough for it: on short inputs
+// its four groups per CTA leave most SMs idle and two short Linear launches are faster (1 560 x 64: 16 us
+// against 10).
+static bool use_fused_mlp(int64_t n, int channels, int hidden, int dtype)
+{
+    return ptv3_mlp_supported(channels, hidden, dtype) &&
+           !(linear_small_wanted(n, channels, hidden) && linear_small_wanted(n, hidden, channels));
 }
 
 struct BlockBuffers {
@@ -45,7 +57,7 @@ static size_t carve_block(const ptv3_block_args* a, void* base, BlockBuffers* b)
 {
     const size_t row = (size_t)a->channels * 2;
     const size_t n = (size_t)a->n;
-    const bool fused_mlp = ptv3_mlp_supported(a->channels, a->hidden, a->dtype) != 0;
+    const bool fused_mlp = use_fused_mlp(a->n, a->channels, a->hidden, a->dtype);
     Carver c(base);
     BlockBuffers t;
     t.x = c.take<char>(n * row);
@@ -135,7 +147,7 @@ extern "C" int ptv3_block_fwd(const ptv3_block_args* a, void* stream_)
     }
     STEP(ptv3_attention_fwd(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.att, n, a->n_seq, a->max_seqlen, C,
                             a->heads, a->scale, dt, a->attention_algo, a->status, stream_));
-    const bool fused_mlp = ptv3_mlp_supported(C, a->hidden, dt) != 0;
+    const bool fused_mlp = use_fused_mlp(n, C, a->hidden, dt);
     if (tc_lin) {
         STEP(ptv3_linear_ln_fwd(b.att, a->proj_w, a->proj_b, b.f1, nullptr, nullptr, 0.f, b.f2, a->n2_w, a->n2_b,
                                 a->n2_eps, b.a, n, C, dt, a->status, stream_));

@@ -67,7 +67,6 @@ template <int BN, int KC, int STAGES, int NI, bool SPLIT>
 __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                const ConvTcArgs a)
 {
-    pdl_launch_next();
     constexpr int ROWB = KC * 2;                    // bytes per staged row: one swizzle span (128 or 64)
     constexpr int NCH = ROWB / 16;                  // 16-byte chunks per row
     constexpr int A_BYTES = CT_TM * ROWB, B_BYTES = BN * ROWB, STAGE_BYTES = A_BYTES + B_BYTES;
@@ -123,7 +122,11 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
         fence_barrier_init();
         prefetch_tensormap(&map_w);
     }
-    if (warp == CT_GATHER_WARPS) tmem_alloc(smem_u32_generic(tmem_slot), TM_COLS);
+    if (warp == CT_GATHER_WARPS) {
+        tmem_alloc(smem_u32_generic(tmem_slot), TM_COLS);
+        // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
+        pdl_launch_next();
+    }
     // (only the set-up above runs beside the kernel before this one in the stream)
     pdl_wait();
 

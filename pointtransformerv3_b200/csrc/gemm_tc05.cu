@@ -22,6 +22,7 @@
 // the residual sum rounded again).  Every mbarrier wait is bounded and reports through the
 // status word.
 #include "common.cuh"
+#include "linear_small.cuh"
 #include "tc05.cuh"
 #include "vec.cuh"
 #include "mma_util.cuh"
@@ -62,7 +63,6 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tc05_kernel(const __grid_c
                                                                   const __grid_constant__ CUtensorMap map_o,
                                                                   const GemmArgs a)
 {
-    pdl_launch_next();
     constexpr int B_BYTES = BN * GM_BK * 2;
     constexpr int STAGE_BYTES = WRES ? GM_A_BYTES : GM_A_BYTES + B_BYTES;
     constexpr int NBAR = 2 * STAGES + 5;      // full, empty per stage; accumulator full / empty x 2; W
@@ -110,7 +110,11 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tc05_kernel(const __grid_c
         prefetch_tensormap(&map_w);
         prefetch_tensormap(&map_o);
     }
-    if (warp == 1) tmem_alloc(sbase + off_bar + 8 * NBAR, 2 * BN);
+    if (warp == 1) {
+        tmem_alloc(sbase + off_bar + 8 * NBAR, 2 * BN);
+        // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
+        pdl_launch_next();
+    }
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
@@ -345,6 +349,8 @@ extern "C" int ptv3_gemm_fwd(const void* x, const void* weight, const void* bias
     PTV3_REQUIRE(x && weight && out && status, PTV3_ERR_INVALID_ARGUMENT, "ptv3_gemm_fwd: null pointer");
     PTV3_REQUIRE((((uintptr_t)x | (uintptr_t)weight | (uintptr_t)out | (uintptr_t)bias | (uintptr_t)residual) & 15) == 0,
                  PTV3_ERR_INVALID_ARGUMENT, "ptv3_gemm_fwd: tensors must be 16-byte aligned");
+    if (linear_small_wanted(n, k, n_out))
+        return launch_linear_small(x, weight, bias, residual, out, n, k, n_out, gelu, status, (cudaStream_t)stream);
     GemmArgs a{};
     a.bias = (const __nv_bfloat16*)bias;
     a.residual = (const __nv_bfloat16*)residual;

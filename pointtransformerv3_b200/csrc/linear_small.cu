@@ -1,0 +1,410 @@
+// Linear layers on short inputs (the coarse levels, small rooms), tcgen05: one 128 x 64 tile per CTA.
+//
+// On a few hundred rows a layer is bound by the length of its own chain, not by any unit: the persistent
+// kernels (gemm_tc05.cu, linear_tc05.cu) give such a layer a handful of CTAs that walk all of K and then
+// spend most of their time in an epilogue of 128 or 256 columns (27 x 2048 -> 512: 15 us on four CTAs;
+// Linear + two LayerNorms at 128 channels: 13 us; the 64-channel MLP: 16 us).  Here
+//   * tiles are 64 columns wide, eight warps take 32 columns of a row each;
+//   * the weights of the first chunks are on their way before the preceding kernel has finished;
+//   * long K: a cluster of up to eight CTAs takes shares of K; the partial sums meet in distributed
+//     shared memory, every CTA finishing some of the rows (in rank order: the result is the same on
+//     every run);
+//   * Linear + LayerNorm (64 and 128 channels): a CTA, or a cluster of two, holds whole rows; row
+//     statistics are merged from the mean and centred square sum of every 32 columns.
+#include "common.cuh"
+#include "linear_small.cuh"
+#include "tc05.cuh"
+#include "vec.cuh"
+
+namespace ptv3 {
+
+using namespace tc05;
+
+constexpr int LS_BM = 128, LS_BN = 64, LS_BK = 64;
+constexpr int LS_A_BYTES = LS_BM * LS_BK * 2, LS_B_BYTES = LS_BN * LS_BK * 2, LS_STAGE = LS_A_BYTES + LS_B_BYTES;
+constexpr int LS_MAX_STAGES = 8;
+constexpr int LS_EPI_WARPS = 8, LS_THREADS = 64 + 32 * LS_EPI_WARPS;
+constexpr int LS_PITCH = LS_BN + 4;                    // floats of a row of partial sums
+constexpr int LS_PLAIN = 0, LS_GELU = 1, LS_RESIDUAL = 2, LS_LN = 4;
+
+struct LinearSmallArgs {
+    const __nv_bfloat16 *bias, *residual;
+    __nv_bfloat16* out;                                // LN: the sum, or NULL
+    const __nv_bfloat16 *ln1_w, *ln1_b, *ln2_w, *ln2_b;
+    float eps1, eps2;
+    __nv_bfloat16* norm_out;
+    int64_t n;
+    int k, n_out, stages;
+    uint32_t* status;
+};
+
+// bytes of the ring; a split layer's partial sums (128 x 68 floats) lie over it
+__host__ __device__ constexpr int ls_ring_bytes(int stages)
+{
+    return stages * LS_STAGE > LS_BM * LS_PITCH * 4 ? stages * LS_STAGE : (LS_BM * LS_PITCH * 4 + 1023) / 1024 * 1024;
+}
+constexpr int LS_PARAM_BYTES = 5 * LS_BN * 4;          // bias, LN1 and LN2 weights and biases as floats
+constexpr int LS_STAT_BYTES = 2 * 2 * LS_BM * 8;       // (mean, square sum) per LayerNorm, half and row
+static size_t ls_smem(int stages)
+{
+    return ls_ring_bytes(stages) + LS_PARAM_BYTES + LS_STAT_BYTES + 8 * (2 * LS_MAX_STAGES + 1) + 16 + 1024;
+}
+
+// two floats of a peer's shared memory
+__device__ __forceinline__ float2 ld_peer_f2(uint32_t addr, uint32_t rank)
+{
+    uint32_t p;
+    float2 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p) : "r"(addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(p) : "memory");
+    return v;
+}
+
+template <int MODE>
+__device__ __forceinline__ uint4 ls_finish(const float* acc, const float* bias, uint4 res)
+{
+    uint32_t o[4];
+    const uint32_t r[4] = {res.x, res.y, res.z, res.w};
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        // the Linear's own output in bf16, then the activation and the residual
+        uint32_t packed;
+        uint64_t y = round2(pack2(acc[2 * p] + bias[2 * p], acc[2 * p + 1] + bias[2 * p + 1]), packed);
+        if (MODE & LS_GELU) y = gelu_tanh_erf2(y);
+        if (MODE & LS_RESIDUAL) y = add2(y, unpack_bf16x2(r[p]));
+        if (MODE & (LS_GELU | LS_RESIDUAL)) {
+            float lo, hi;
+            unpack2(y, lo, hi);
+            packed = pack_bf16(lo, hi);
+        }
+        o[p] = packed;
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_constant__ CUtensorMap map_x,
+                                                                 const __grid_constant__ CUtensorMap map_w,
+                                                                 const LinearSmallArgs a)
+{
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const uint32_t sbase = smem_u32_generic(smem);
+    const int stages = a.stages;
+    float* params = reinterpret_cast<float*>(smem + ls_ring_bytes(stages));
+    const int off_stat = ls_ring_bytes(stages) + LS_PARAM_BYTES;
+    float2* stat = reinterpret_cast<float2*>(smem + off_stat);
+    const uint32_t full0 = sbase + off_stat + LS_STAT_BYTES, empty0 = full0 + 8 * LS_MAX_STAGES,
+                   accfull = empty0 + 8 * LS_MAX_STAGES;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + off_stat + LS_STAT_BYTES + 8 * (2 * LS_MAX_STAGES + 1));
+    volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int col0 = blockIdx.x * LS_BN, row0 = blockIdx.y * LS_BM;
+    // this CTA's chunks of K
+    const int parts = (MODE & LS_LN) ? 1 : (int)gridDim.z;
+    const int nk = a.k / LS_BK / parts, k0 = nk * (int)blockIdx.z * LS_BK;
+
+    if (tid == 0) {
+        for (int s = 0; s < stages; ++s) {
+            mbar_init(full0 + 8 * s, 1);
+            mbar_init(empty0 + 8 * s, 1);
+        }
+        mbar_init(accfull, 1);
+        *abort = 0;
+        fence_barrier_init();
+        prefetch_tensormap(&map_x);
+        // the weights are not written by the launch before this one: fetched ahead of the wait below
+        for (int kc = 0; kc < nk && kc < stages; ++kc) {
+            mbar_expect_tx(full0 + 8 * kc, LS_STAGE);
+            tma_load_2d(sbase + kc * LS_STAGE + LS_A_BYTES, &map_w, k0 + kc * LS_BK, col0, full0 + 8 * kc);
+        }
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32_generic(tmem_slot), LS_BN);
+        // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
+        pdl_launch_next();
+    }
+    {
+        // parameters of this CTA's columns as floats
+        constexpr int N = (MODE & LS_LN) ? 5 : 1;
+        for (int i = tid; i < N * LS_BN; i += LS_THREADS) {
+            const int j = i / LS_BN;
+            const __nv_bfloat16* p = j == 0 ? a.bias : j == 1 ? a.ln1_w : j == 2 ? a.ln1_b : j == 3 ? a.ln2_w : a.ln2_b;
+            params[i] = p ? __bfloat162float(p[col0 + i % LS_BN]) : 0.f;
+        }
+    }
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+    bool ok = true;
+    pdl_wait();
+
+    // epilogue threads: row r of the tile, 32 of its columns
+    const int q = warp & 3, half = (warp - 2) >> 2, r = q * 32 + lane, c0 = half * 32;
+    const int64_t row = (int64_t)row0 + r;
+    const bool live = warp >= 2 && row < a.n;
+    float v[32];
+    uint4 res[4] = {};
+
+    if (warp == 0) {
+        if (lane == 0)
+            for (int kc = 0; kc < nk; ++kc) {
+                const int s = kc % stages;
+                const uint32_t sa = sbase + s * LS_STAGE;
+                if (kc >= stages) {
+                    ok &= mbar_wait(empty0 + 8 * s, ((kc / stages) & 1) ^ 1, abort);
+                    mbar_expect_tx(full0 + 8 * s, LS_STAGE);
+                    tma_load_2d(sa + LS_A_BYTES, &map_w, k0 + kc * LS_BK, col0, full0 + 8 * s);
+                }
+                tma_load_2d(sa, &map_x, k0 + kc * LS_BK, row0, full0 + 8 * s);
+            }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0) {
+            constexpr uint32_t idesc = umma_idesc_bf16(LS_BM, LS_BN);
+            for (int kc = 0; kc < nk; ++kc) {
+                const int s = kc % stages;
+                ok &= mbar_wait(full0 + 8 * s, (kc / stages) & 1, abort);
+                fence_after_sync();
+                const uint32_t sa = sbase + s * LS_STAGE, sb = sa + LS_A_BYTES;
+#pragma unroll
+                for (int k4 = 0; k4 < LS_BK / 16; ++k4)
+                    umma_bf16(tmem_base, umma_desc_kmajor(sa + k4 * 32, 128), umma_desc_kmajor(sb + k4 * 32, 128), idesc,
+                              kc > 0 || k4 > 0);
+                umma_commit(empty0 + 8 * s);
+            }
+            umma_commit(accfull);
+        }
+        __syncwarp();
+    } else {
+        if ((MODE & (LS_RESIDUAL | LS_LN)) && parts == 1 && live) {
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+                res[g] = *reinterpret_cast<const uint4*>(a.residual + row * a.n_out + col0 + c0 + g * 8);
+        }
+        ok &= mbar_wait(accfull, 0, abort);
+        fence_after_sync();
+        uint32_t acc[32];
+        tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + c0, acc);
+        tmem_ld_wait();
+        tmem_ld_fence(acc);
+#pragma unroll
+        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(acc[i]);
+    }
+
+    if (MODE & LS_LN) {
+        const float inv_c = 1.f / (float)a.n_out;
+        const int ctas = (int)gridDim.x;              // the cluster holds the row
+        // merges the statistics of all 32-column pieces of the row; every piece has the same size
+        auto statistics = [&](int which, float eps, float& mean, float& rstd) {
+            if (warp >= 2) {
+                float s = 0.f, m2 = 0.f;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) s += v[i];
+                s *= 1.f / 32.f;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) m2 = fmaf(v[i] - s, v[i] - s, m2);
+                stat[(which * 2 + half) * LS_BM + r] = make_float2(s, m2);
+            }
+            if (ctas > 1)
+                cluster_sync();
+            else
+                __syncthreads();
+            mean = rstd = 0.f;
+            if (warp >= 2) {
+                float2 p[4];
+#pragma unroll
+                for (int z = 0; z < 4; ++z)
+                    if (z < 2 * ctas)
+                        p[z] = ctas > 1 ? ld_peer_f2(sbase + off_stat + ((which * 2 + (z & 1)) * LS_BM + r) * 8, z >> 1)
+                                        : stat[(which * 2 + z) * LS_BM + r];
+                float m2 = 0.f;
+#pragma unroll
+                for (int z = 0; z < 4; ++z)
+                    if (z < 2 * ctas) mean += p[z].x;
+                mean *= 32.f * inv_c;
+#pragma unroll
+                for (int z = 0; z < 4; ++z)
+                    if (z < 2 * ctas) m2 += fmaf(32.f * (p[z].x - mean), p[z].x - mean, p[z].y);
+                rstd = rsqrtf(m2 * inv_c + eps);
+            }
+        };
+        auto to_bf16 = [](float x) { return __bfloat162float(__float2bfloat16_rn(x)); };
+        if (warp >= 2)
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] = to_bf16(v[i] + params[c0 + i]);
+        float mean, rstd;
+        if (a.ln1_w) {
+            statistics(0, a.eps1, mean, rstd);
+            if (warp >= 2)
+#pragma unroll
+                for (int i = 0; i < 32; ++i)
+                    v[i] = to_bf16(fmaf((v[i] - mean) * rstd, params[LS_BN + c0 + i], params[2 * LS_BN + c0 + i]));
+        }
+        if (warp >= 2) {
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                float f[8];
+                Vec<__nv_bfloat16>::unpack(res[g], f);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) v[g * 8 + i] = to_bf16(f[i] + v[g * 8 + i]);
+                if (live && a.out)
+                    *reinterpret_cast<uint4*>(a.out + row * a.n_out + col0 + c0 + g * 8) =
+                        Vec<__nv_bfloat16>::pack(v + g * 8);
+            }
+        }
+        statistics(1, a.eps2, mean, rstd);
+        // (the wait at the end: a peer's statistics outlive their readers)
+        if (ctas > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        if (live) {
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                float f[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    f[i] = fmaf((v[g * 8 + i] - mean) * rstd, params[3 * LS_BN + c0 + g * 8 + i],
+                                params[4 * LS_BN + c0 + g * 8 + i]);
+                *reinterpret_cast<uint4*>(a.norm_out + row * a.n_out + col0 + c0 + g * 8) =
+                    Vec<__nv_bfloat16>::pack(f);
+            }
+        }
+        __syncwarp();
+        if (ctas > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    } else if (parts == 1) {
+        if (live)
+#pragma unroll
+            for (int g = 0; g < 4; ++g)
+                *reinterpret_cast<uint4*>(a.out + row * a.n_out + col0 + c0 + g * 8) =
+                    ls_finish<MODE>(v + g * 8, params + c0 + g * 8, res[g]);
+    } else {
+        // partial sums over the ring (every product has completed); then this CTA's rows
+        if (warp >= 2) {
+            float* prow = reinterpret_cast<float*>(smem) + r * LS_PITCH + c0;
+#pragma unroll
+            for (int g = 0; g < 8; ++g)
+                *reinterpret_cast<float4*>(prow + g * 4) = make_float4(v[g * 4], v[g * 4 + 1], v[g * 4 + 2], v[g * 4 + 3]);
+        }
+        cluster_sync();
+        const int rows = LS_BM / parts, first = rows * (int)cluster_rank();
+        for (int e = tid; e < rows * (LS_BN / 8); e += LS_THREADS) {
+            const int rr = first + e / (LS_BN / 8), c = e % (LS_BN / 8) * 8;
+            const int64_t orow = (int64_t)row0 + rr;
+            if (orow >= a.n) continue;
+            uint4 r4 = make_uint4(0, 0, 0, 0);
+            if (MODE & LS_RESIDUAL) r4 = *reinterpret_cast<const uint4*>(a.residual + orow * a.n_out + col0 + c);
+            const uint32_t at = sbase + (rr * LS_PITCH + c) * 4;
+            float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            for (int z = 0; z < parts; ++z) {
+                const float4 m = ld_peer_f4(at, z), w = ld_peer_f4(at + 16, z);
+                t[0] += m.x; t[1] += m.y; t[2] += m.z; t[3] += m.w;
+                t[4] += w.x; t[5] += w.y; t[6] += w.z; t[7] += w.w;
+            }
+            *reinterpret_cast<uint4*>(a.out + orow * a.n_out + col0 + c) = ls_finish<MODE>(t, params + c, r4);
+        }
+        cluster_sync();          // a peer's partial sums outlive their readers
+    }
+    fence_before_sync();
+    __syncthreads();
+    if (warp == 1) {
+        fence_after_sync();
+        tmem_dealloc(tmem_base, LS_BN);
+    }
+    if (lane == 0 && (!ok || (tid == 0 && *abort))) atomicOr(a.status, PTV3_STATUS_WAIT_LIMIT);
+}
+
+template <int MODE>
+static int launch_ls(const void* x, const void* w, LinearSmallArgs a, int parts, cudaStream_t stream)
+{
+    const int nk = a.k / LS_BK / parts;
+    a.stages = nk < LS_MAX_STAGES ? nk : LS_MAX_STAGES;
+    CUtensorMap mx, mw;
+    int rc = make_tensor_map_bf16(&mx, x, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.k * 2, LS_BM, LS_BK);
+    if (rc) return rc;
+    rc = make_tensor_map_bf16(&mw, w, (uint64_t)a.n_out, (uint64_t)a.k, (uint64_t)a.k * 2, LS_BN, LS_BK);
+    if (rc) return rc;
+    auto kern = linear_small_kernel<MODE>;
+    if (allow_smem(kern) != cudaSuccess) return check_launch("short Linear: shared memory attribute");
+    const dim3 grid(a.n_out / LS_BN, (unsigned)((a.n + LS_BM - 1) / LS_BM), parts);
+    const dim3 cluster = (MODE & LS_LN) ? dim3(grid.x, 1, 1) : dim3(1, 1, parts);
+    launch_dependent_cluster(kern, grid, dim3(LS_THREADS), ls_smem(a.stages), stream, cluster, mx, mw, a);
+    count_launches(1);
+    return check_launch("short Linear");
+}
+
+// Shares of K: clusters of up to eight CTAs, at least four chunks each.  Below 16 chunks the exchange costs
+// more than it saves (441 x 512 -> 512: 7.1 us in clusters of two, 6.1 with the persistent kernel).
+static int ls_parts(int64_t tiles, int k)
+{
+    const int chunks = k / LS_BK;
+    int parts = 1;
+    if (chunks >= 16)
+        while (parts < 8 && tiles * parts * 2 <= 128 && chunks % (parts * 2) == 0 && chunks / (parts * 2) >= 4) parts *= 2;
+    return parts;
+}
+
+// Where the lines lie (us, this kernel against the persistent ones):
+//   K <= 128: three CTAs share an SM: one wave.  1 560 x 64 -> 192: 3.5 / 6.3, 18 900 x 64 -> 192 (444 tiles):
+//     5.7 / 6.7, 9 400 x 128 -> 384 (444): 6.3 / 7.9; 1 776 tiles lose
+//   K <= 512: 105 x 256 -> 1 024: 4.4 / 5.4, 1 700 x 256 -> 256 (56 tiles): 4.8 / 5.0, -> 768 (168): 5.9 / 5.0
+//   longer K where it can be shared: 27 x 2 048 -> 512: 6.8 / 13.2, 1 000 x 2 048 -> 512 (64): 11.7 / 14.5
+bool linear_small_wanted(int64_t n, int k, int n_out)
+{
+    if (k % LS_BK || k < LS_BK || k > 8192 || n_out % LS_BN) return false;
+    const int64_t tiles = (n + LS_BM - 1) / LS_BM * (n_out / LS_BN);
+    if (k <= 128) return tiles <= 444;
+    if (k < 1024) return tiles <= 74;
+    return ls_parts(tiles, k) > 1;
+}
+
+// One wave of two CTAs per SM: 1 560 x 64: 6.2 / 10.5, 18 900 x 64: 6.7 / 10.8, 40 000 x 64 (313 tiles): 13.9 / 11.3;
+// 405 x 128: 7.9 / 13.0, 18 900 x 128 (296): 11.2 / 13.5.  Wider rows stay with Linear and row kernel: two or three
+// exchanges over four or eight CTAs cost what the second launch does (27 x 512: 11.4 us against 9.0).
+bool linear_ln_small_wanted(int64_t n, int c)
+{
+    return (c == 64 || c == 128) && (n + LS_BM - 1) / LS_BM * (c / LS_BN) <= 296;
+}
+
+int launch_linear_small(const void* x, const void* w, const void* bias, const void* residual, void* out, int64_t n, int k,
+                        int n_out, int gelu, uint32_t* status, cudaStream_t stream)
+{
+    LinearSmallArgs a{};
+    a.bias = (const __nv_bfloat16*)bias;
+    a.residual = (const __nv_bfloat16*)residual;
+    a.out = (__nv_bfloat16*)out;
+    a.n = n;
+    a.k = k;
+    a.n_out = n_out;
+    a.status = status;
+    const int parts = ls_parts((n + LS_BM - 1) / LS_BM * (n_out / LS_BN), k);
+    switch ((gelu ? LS_GELU : 0) | (residual ? LS_RESIDUAL : 0)) {
+    case LS_PLAIN: return launch_ls<LS_PLAIN>(x, w, a, parts, stream);
+    case LS_GELU: return launch_ls<LS_GELU>(x, w, a, parts, stream);
+    case LS_RESIDUAL: return launch_ls<LS_RESIDUAL>(x, w, a, parts, stream);
+    default: return launch_ls<LS_GELU | LS_RESIDUAL>(x, w, a, parts, stream);
+    }
+}
+
+int launch_linear_ln_small(const void* x, const void* w, const void* bias, const void* residual, const void* ln1_w,
+                           const void* ln1_b, float eps1, void* sum_out, const void* ln2_w, const void* ln2_b, float eps2,
+                           void* norm_out, int64_t n, int c, uint32_t* status, cudaStream_t stream)
+{
+    LinearSmallArgs a{};
+    a.bias = (const __nv_bfloat16*)bias;
+    a.residual = (const __nv_bfloat16*)residual;
+    a.out = (__nv_bfloat16*)sum_out;
+    a.ln1_w = (const __nv_bfloat16*)ln1_w;
+    a.ln1_b = (const __nv_bfloat16*)ln1_b;
+    a.ln2_w = (const __nv_bfloat16*)ln2_w;
+    a.ln2_b = (const __nv_bfloat16*)ln2_b;
+    a.eps1 = eps1;
+    a.eps2 = eps2;
+    a.norm_out = (__nv_bfloat16*)norm_out;
+    a.n = n;
+    a.k = a.n_out = c;
+    a.status = status;
+    return launch_ls<LS_LN>(x, w, a, 1, stream);
+}
+
+}  // namespace ptv3

@@ -18,6 +18,7 @@
 // sequence would round to bf16 is rounded at the same place.  Waits are bounded.
 #include "common.cuh"
 #include "mma_util.cuh"
+#include "linear_small.cuh"
 #include "tc05.cuh"
 #include "vec.cuh"
 
@@ -87,7 +88,6 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
                                                              const __grid_constant__ CUtensorMap map_o,
                                                              const LinearArgs a)
 {
-    pdl_launch_next();
     constexpr int SW = K >= 64 ? 128 : 64;       // bytes per shared-memory row (swizzle span)
     constexpr int KB = K >= 64 ? K / 64 : 1;     // 64-wide K blocks
     constexpr int KCOLS = K >= 64 ? 64 : K;      // columns per K block
@@ -128,7 +128,11 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
         g2[i] = a.ln2_w ? __bfloat162float(a.ln2_w[i]) : 1.f;
         b2[i] = a.ln2_b ? __bfloat162float(a.ln2_b[i]) : 0.f;
     }
-    if (warp == 0) tmem_alloc(sbase + off_bar + 136, 512);
+    if (warp == 0) {
+        tmem_alloc(sbase + off_bar + 136, 512);
+        // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
+        pdl_launch_next();
+    }
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
@@ -548,6 +552,8 @@ extern "C" int ptv3_linear_fwd(const void* x, const void* weight, const void* bi
     PTV3_REQUIRE(x && weight && out && status, PTV3_ERR_INVALID_ARGUMENT, "ptv3_linear_fwd: null pointer");
     PTV3_REQUIRE((((uintptr_t)x | (uintptr_t)weight | (uintptr_t)out) & 15) == 0, PTV3_ERR_INVALID_ARGUMENT,
                  "ptv3_linear_fwd: tensors must be 16-byte aligned");
+    if (linear_small_wanted(n, k, n_out))
+        return launch_linear_small(x, weight, bias, nullptr, out, n, k, n_out, 0, status, (cudaStream_t)stream);
     LinearArgs a{};
     a.bias = (const __nv_bfloat16*)bias;
     a.out = (__nv_bfloat16*)out;
@@ -575,6 +581,9 @@ extern "C" int ptv3_linear_ln_fwd(const void* x, const void* weight, const void*
     PTV3_REQUIRE((((uintptr_t)x | (uintptr_t)weight | (uintptr_t)residual | (uintptr_t)norm_out |
                    (uintptr_t)sum_out) & 15) == 0,
                  PTV3_ERR_INVALID_ARGUMENT, "ptv3_linear_ln_fwd: tensors must be 16-byte aligned");
+    if (linear_ln_small_wanted(n, channels))
+        return launch_linear_ln_small(x, weight, bias, residual, ln1_weight, ln1_bias, ln1_eps, sum_out, ln2_weight,
+                                      ln2_bias, ln2_eps, norm_out, n, channels, status, (cudaStream_t)stream);
     LinearArgs a{};
     a.bias = (const __nv_bfloat16*)bias;
     a.residual = (const __nv_bfloat16*)residual;

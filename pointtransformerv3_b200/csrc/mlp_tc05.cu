@@ -61,7 +61,6 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
     const __nv_bfloat16* __restrict__ b2, const __nv_bfloat16* __restrict__ residual,
     __nv_bfloat16* __restrict__ out, int64_t n, uint32_t* __restrict__ status)
 {
-    pdl_launch_next();
     using Cfg = MlpCfg<C>;
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -89,7 +88,11 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
     }
     for (int i = tid; i < Cfg::HD; i += NT) b1s[i] = __bfloat162float(b1[i]);
     for (int i = tid; i < C; i += NT) b2s[i] = __bfloat162float(b2[i]);
-    if (warp == 0) tmem_alloc(sbase + Cfg::OFF_BAR + 8 * Cfg::NBAR, 512);
+    if (warp == 0) {
+        tmem_alloc(sbase + Cfg::OFF_BAR + 8 * Cfg::NBAR, 512);
+        // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
+        pdl_launch_next();
+    }
     fence_before_sync();
     __syncthreads();
     fence_after_sync();

@@ -669,3 +669,51 @@ def test_seg_head_matches_torch(n, C, K, dtype):
     assert torch.equal(labels.cpu()[clear], ref.argmax(1)[clear])
     only_labels = ops.seg_head(feat.cuda(), w.cuda(), b.cuda(), want_logits=False)
     assert only_labels[0] is None and torch.equal(only_labels[1], labels)
+
+
+@pytest.mark.parametrize("n,k,n_out", [(1, 64, 128), (129, 64, 192), (127, 128, 384), (18944, 64, 192), (18945, 64, 192),
+                                       (27, 2048, 512), (130, 1024, 256), (1100, 2048, 512), (300, 256, 1024)])
+@pytest.mark.parametrize("gelu,residual", [(False, False), (True, False), (False, True)])
+def test_short_linear(n, k, n_out, gelu, residual):
+    """Linear layers on short inputs: single chunks, rings, clusters over K, ragged row tiles and both
+    sides of a line of the dispatch, against torch in fp32."""
+    g = torch.Generator().manual_seed(n + k)
+    x, w = torch.randn(n, k, generator=g).bfloat16(), (torch.randn(n_out, k, generator=g) / k ** 0.5).bfloat16()
+    b, r = torch.randn(n_out, generator=g).bfloat16(), torch.randn(n, n_out, generator=g).bfloat16()
+    if n_out % 128:
+        if gelu or residual:
+            pytest.skip("only the plain form takes this width")
+        got = ops.linear(x.cuda(), w.cuda(), b.cuda())
+    else:
+        got = ops.gemm(x.cuda(), w.cuda(), b.cuda(), r.cuda() if residual else None, gelu)
+    ref = torch.nn.functional.linear(x.float(), w.float(), b.float())
+    if gelu:
+        ref = torch.nn.functional.gelu(ref)
+    if residual:
+        ref = ref + r.float()
+    assert_close(got, ref, what="short Linear", **TOL[torch.bfloat16])
+    assert rel_l2(got, ref) < 5e-3
+
+
+@pytest.mark.parametrize("c", [64, 128])
+@pytest.mark.parametrize("n", [1, 128, 1001, 18944, 19000])
+@pytest.mark.parametrize("with_ln1", [False, True])
+def test_short_linear_layernorm(n, c, with_ln1):
+    """Linear + residual + LayerNorms on short inputs (statistics merged over 32-column pieces and
+    clusters of two) and on the other side of the line, against torch in fp32."""
+    g = torch.Generator().manual_seed(n + c)
+    x, r = torch.randn(n, c, generator=g).bfloat16(), torch.randn(n, c, generator=g).bfloat16()
+    w, b = (torch.randn(c, c, generator=g) / c ** 0.5).bfloat16(), torch.randn(c, generator=g).bfloat16()
+    ln1, ln2 = torch.nn.LayerNorm(c), torch.nn.LayerNorm(c)
+    for ln in (ln1, ln2):
+        ln.weight.data = torch.rand(c, generator=g) + 0.5
+        ln.bias.data = torch.randn(c, generator=g) * 0.3
+    ln1, ln2 = ln1.bfloat16(), ln2.bfloat16()
+    s, y = ops.linear_ln(x.cuda(), w.cuda(), b.cuda(), r.cuda(), ln1.cuda() if with_ln1 else None, ln2.cuda())
+    t = torch.nn.functional.linear(x.float(), w.float(), b.float()).bfloat16().float()
+    if with_ln1:
+        t = torch.nn.functional.layer_norm(t, (c,), ln1.weight.float().cpu(), ln1.bias.float().cpu(), ln1.eps)
+    ref = r.float() + t.bfloat16().float()
+    ref_y = torch.nn.functional.layer_norm(ref.bfloat16().float(), (c,), ln2.weight.float().cpu(), ln2.bias.float().cpu(),
+                                           ln2.eps)
+    assert rel_l2(s, ref) < 5e-3 and rel_l2(y, ref_y) < 6e-3
