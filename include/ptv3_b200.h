@@ -474,6 +474,21 @@ typedef struct ptv3_block_args {
 } ptv3_block_args;
 
 int ptv3_block_supported(int channels, int heads, int hidden, int dtype);
+/*
+ * fp32 on the tensor cores: a float is the exact sum of three bf16 values, and a product of floats the sum
+ * of six products of those, accumulated in fp32 (what is left out is below one fp32 rounding).
+ * ptv3_split_f32 writes rows x k floats as rows x 6k bf16, for the features of a product (weight = 0) or its
+ * weights (weight = 1); the two products take both split.  ptv3_block_fwd with PTV3_DTYPE_F32 takes fp32
+ * features, biases and norms and SPLIT conv_weight, cpe_w, qkv_w, proj_w, fc1_w, fc2_w (rows of their inner
+ * dimension: c_in for the convolution), where ptv3_block_f32_supported says so.
+ */
+int ptv3_split_f32(const float* x, int64_t rows, int k, int weight, void* out, void* stream);
+int ptv3_linear_split_fwd(const void* x_split, const void* w_split, const float* bias, const float* residual,
+                          float* out, int64_t n, int k, int n_out, int gelu, uint32_t* status, void* stream);
+int ptv3_subm_conv_split_fwd(const void* feat_split, const int32_t* nbr, const void* w_split, const float* bias,
+                             float* out, const int64_t* row_order, int64_t n, int c_in, int c_out, int kernel_volume,
+                             uint32_t* status, void* stream);
+int ptv3_block_f32_supported(int channels, int heads, int hidden);
 /* reads n, channels, hidden, dtype and pair_in (null or not) of the argument block */
 size_t ptv3_block_workspace_bytes(const ptv3_block_args* args);
 int ptv3_block_fwd(const ptv3_block_args* args, void* stream);
@@ -562,7 +577,7 @@ int ptv3_unpool_stage_fwd(const void* skip_feat, const void* child_feat, const v
                           uint32_t* status, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
- * The whole bf16 backbone in one call (model.py:884-982, PointTransformerV3.forward of a
+ * The whole backbone in one call (model.py:884-982, PointTransformerV3.forward of a
  * segmentation network, inference): serialization, kernel maps, pooling plans, stem, encoder and
  * decoder, queued on two streams from C++.  The kernels are the ones behind the entry points
  * above; what the call saves is host time (a pass over a small room is bounded by it) and the
@@ -592,6 +607,8 @@ typedef struct ptv3_backbone_args {
     /* network */
     int n_enc, n_dec;               /* n_dec == n_enc - 1, decoder stages from coarse to fine */
     const ptv3_stage_args *enc, *dec;
+    int dtype;                      /* features and parameters; fp32: weights split as for ptv3_block_fwd (the
+                                       stem's weight is not), transitions too */
     int stem_c_in, stem_c_out, stem_ksize;
     const void* stem_weight;
     const float *stem_scale, *stem_shift;
@@ -602,7 +619,7 @@ typedef struct ptv3_backbone_args {
     const int64_t* counts;          /* HOST, n_scenes: points of every scene */
     const int* order_ids;           /* HOST, k (as for ptv3_encode, already shuffled) */
     const int* row_perm;            /* HOST, (n_enc - 1) x k or NULL: shuffle of every pooling */
-    const void* feat;               /* n x stem_c_in bf16 */
+    const void* feat;               /* n x stem_c_in */
     const int32_t* grid_coord;      /* n x 3 */
     const int64_t *offset, *batch;  /* n_scenes, n */
     /* outputs of the finest level */

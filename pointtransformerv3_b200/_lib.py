@@ -48,7 +48,7 @@ class BackboneArgs(ctypes.Structure):
     """ptv3_backbone_args of include/ptv3_b200.h (same field order)."""
     _fields_ = (
         [("n_enc", c_int), ("n_dec", c_int), ("enc", ctypes.POINTER(StageArgs)), ("dec", ctypes.POINTER(StageArgs)),
-         ("stem_c_in", c_int), ("stem_c_out", c_int), ("stem_ksize", c_int), ("stem_weight", c_ptr),
+         ("dtype", c_int), ("stem_c_in", c_int), ("stem_c_out", c_int), ("stem_ksize", c_int), ("stem_weight", c_ptr),
          ("stem_scale", c_ptr), ("stem_shift", c_ptr), ("k", c_int), ("n", c_i64), ("n_scenes", c_int),
          ("depth", c_int), ("counts", ctypes.POINTER(c_i64)), ("order_ids", ctypes.POINTER(c_int)),
          ("row_perm", ctypes.POINTER(c_int))]
@@ -123,6 +123,11 @@ SIGNATURES = {
     "ptv3_unpool_stage_fwd": (c_int, [c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_i64, c_i64, c_int, c_int,
                                       c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_int, c_ptr, c_ptr, c_sz, c_ptr]),
     "ptv3_block_supported": (c_int, [c_int, c_int, c_int, c_int]),
+    "ptv3_split_f32": (c_int, [c_ptr, c_i64, c_int, c_int, c_ptr, c_ptr]),
+    "ptv3_linear_split_fwd": (c_int, [c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_i64, c_int, c_int, c_int, c_ptr, c_ptr]),
+    "ptv3_subm_conv_split_fwd": (c_int, [c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_i64, c_int, c_int, c_int, c_ptr,
+                                         c_ptr]),
+    "ptv3_block_f32_supported": (c_int, [c_int, c_int, c_int]),
     "ptv3_block_workspace_bytes": (c_sz, [ctypes.POINTER(BlockArgs)]),
     "ptv3_block_fwd": (c_int, [ctypes.POINTER(BlockArgs), c_ptr]),
     "ptv3_backbone_fwd": (c_int, [ctypes.POINTER(BackboneArgs)]),

@@ -1,6 +1,7 @@
 """One-call form of the backbone's forward (ptv3_backbone_fwd): the argument blocks of a network
 whose modules all have their standard form, kept between passes and rebuilt when a parameter, a
-buffer or a setting changed."""
+buffer or a setting changed.  fp32 networks keep their weights split for the tensor cores there
+(three times their size, see ptv3_split_f32)."""
 import ctypes
 import operator
 import weakref
@@ -33,10 +34,13 @@ def _require(ok):
 
 
 class NativeBackbone:
-    """Argument blocks of ``net`` (bf16).  ``current`` tells whether they still describe it."""
+    """Argument blocks of ``net`` (bf16 or fp32).  ``current`` tells whether they still describe it."""
 
     def __init__(self, net):
         from . import model as M
+        self.dtype = next(net.parameters()).dtype
+        self.f32 = self.dtype == torch.float32
+        _require(self.dtype in (torch.float32, torch.bfloat16))
         self.refs = []           # (owner dict, name): every tensor the blocks point to or were computed from
         self.versions = []       # tensors whose values were read (BatchNorm): recomputed when modified in place
         self.keep = []           # arrays and tensors the blocks point into
@@ -50,6 +54,7 @@ class NativeBackbone:
         _require(type(conv) is spconv.SubMConv3d and conv.uses_direct_path() and conv.bias is None
                  and _eval_bn(bn) and _exact_gelu(act))
         a = self.args = _lib.BackboneArgs()
+        a.dtype = _lib.DTYPE_IDS[self.dtype]
         a.stem_c_in, a.stem_c_out, a.stem_ksize = conv.in_channels, conv.out_channels, conv.kernel_size
         a.stem_weight = self._param(conv, "weight")
         a.stem_scale, a.stem_shift = self._bn(bn)
@@ -67,11 +72,22 @@ class NativeBackbone:
         self.version = [t._version for t in self.versions]
 
     # -- what the blocks are made of
-    def _param(self, module, name, dtype=torch.bfloat16):
+    def _param(self, module, name):
         t = module._parameters[name]
-        _require(t is not None and t.dtype == dtype and t.is_cuda and t.is_contiguous())
+        _require(t is not None and t.dtype == self.dtype and t.is_cuda and t.is_contiguous())
         self.refs.append((module._parameters, name))
         return t.data_ptr()
+
+    def _weight(self, module):
+        """A weight that enters a matrix product: itself, or its split form."""
+        p = self._param(module, "weight")
+        if not self.f32:
+            return p
+        t = module._parameters["weight"]
+        split = ops.split_f32(t, weight=True)
+        self.versions.append(t)
+        self.keep.append(split)
+        return split.data_ptr()
 
     def _bn(self, bn):
         from .model import _bn_eval_affine
@@ -87,8 +103,9 @@ class NativeBackbone:
 
     def _linear(self, lin, supported):
         _require(type(lin) is nn.Linear and lin.bias is not None
-                 and supported(lin.in_features, lin.out_features, torch.bfloat16))
-        return self._param(lin, "weight"), self._param(lin, "bias")
+                 and (lin.in_features % 32 == 0 and lin.out_features % 32 == 0 if self.f32
+                      else supported(lin.in_features, lin.out_features, torch.bfloat16)))
+        return self._weight(lin), self._param(lin, "bias")
 
     def _stages(self, stages, encoder):
         from . import model as M
@@ -120,12 +137,17 @@ class NativeBackbone:
             order_index, patch = (ctypes.c_int * max(1, len(mods)))(), (ctypes.c_int * max(1, len(mods)))()
             for j, m in enumerate(mods):
                 _require(type(m) is M.Block and m._fusable_form() and not m.attn.enable_rpe
-                         and type(m.attn) is M.SerializedAttention and m._native_static_ok(torch.bfloat16)
+                         and type(m.attn) is M.SerializedAttention and m._native_static_ok(self.dtype, f32=self.f32)
                          and m.channels < spconv.PAIR_PATH_MIN_CHANNELS)
-                args = m._native_args(torch.bfloat16, m.attn.qkv.weight.device)
+                args = m._native_args(self.dtype, m.attn.qkv.weight.device)
                 _require(args is not None and args.conv_weight)
                 ctypes.pointer(blocks[j])[0] = args
                 self.refs.extend(m.__dict__["_ptv3_block_args"][0])
+                if self.f32:
+                    b, mlp = blocks[j], m.mlp[0]
+                    for field, owner in (("conv_weight", m.cpe[0]), ("cpe_w", m.cpe[1]), ("qkv_w", m.attn.qkv),
+                                         ("proj_w", m.attn.proj), ("fc1_w", mlp.fc1), ("fc2_w", mlp.fc2)):
+                        setattr(b, field, self._weight(owner))
                 order_index[j] = m.attn.order_index
                 patch[j] = m.attn.patch_size if m.attn.enable_flash else -m.attn.patch_size_max
                 self.blocks.append(m)

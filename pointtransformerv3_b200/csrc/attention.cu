@@ -204,6 +204,10 @@ static int attention_impl(const void* qkv, const int64_t* order, const int64_t* 
     if (mma_ok && algo != 1)
         return launch_attn_mma(qkv, order, pad, unpad, cu_seqlens, out, n_seq, max_seqlen, channels,
                                heads, scale, algo == 3, status, (cudaStream_t)stream);
+    if (dtype == PTV3_DTYPE_F32 && algo == 0 && !rpe.grid_coord && channels / heads == 16 &&
+        (((uintptr_t)qkv | (uintptr_t)out) & 15) == 0)
+        return launch_attn_f32(qkv, order, pad, unpad, cu_seqlens, out, n_seq, max_seqlen, channels, heads, scale, status,
+                               (cudaStream_t)stream);
     if (dtype == PTV3_DTYPE_F32)
         return launch_attn_fma<float>(qkv, order, pad, unpad, cu_seqlens, out, n_seq, max_seqlen,
                                       channels, heads, scale, rpe, status, (cudaStream_t)stream);

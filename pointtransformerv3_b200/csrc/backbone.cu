@@ -1,4 +1,4 @@
-// The whole backbone in one call (model.py:884-982 for segmentation networks, inference, bf16).
+// The whole backbone in one call (model.py:884-982 for segmentation networks, inference).
 //
 // A pass over a small room is bounded by its host: 276 launches queued through a Python-level module
 // tree took 3.9 ms for 1.75 ms of GPU work (6 000 points; 4.7 ms for 3.0 ms at 100 000).  Here the same
@@ -8,7 +8,9 @@
 // for after every block without waiting, so the next plan is launched as soon as the last one is known
 // instead of when its stage comes up.
 #include "common.cuh"
+#include "linear_small.cuh"
 #include "plan.cuh"
+#include "split_f32.cuh"
 #include <string.h>
 
 namespace ptv3 {
@@ -118,6 +120,8 @@ private:
     char* ws_ = nullptr;
     size_t ws_bytes_ = 0;
 
+    const size_t esize_ = a_.dtype == PTV3_DTYPE_F32 ? 4 : 2;
+
     int64_t* flag(int l) const { return a_.meta_host + (int64_t)l * (3 + a_.n_scenes); }
     int out_of_memory() const
     {
@@ -145,6 +149,7 @@ private:
     int launch_plan();
     int take_plan(bool block);
     int block(const ptv3_stage_args& st, int j, BbLevel& l, const void* conv_in, const void* feat, void* out);
+    int project(const void* x, const void* w, const void* bias, int64_t n, int c_in, int c_out, void* split, void* out);
     int encoder(int s);
     int decoder(int d);
 };
@@ -214,10 +219,10 @@ int Pass::finest()
     made_ = 1;
     BB_STEP(launch_plan());
     BB_CUDA(cudaStreamWaitEvent(main_, sorted, 0));
-    void* feat = mem_.take<char>((size_t)a_.n * a_.stem_c_out * 2);
+    void* feat = mem_.take<char>((size_t)a_.n * a_.stem_c_out * esize_);
     if (!feat) return out_of_memory();
     BB_STEP(conv_direct_from_index(vi, a_.feat, a_.indices, a_.stem_weight, a_.stem_scale, a_.stem_shift, feat, a_.order,
-                                   a_.n, a_.stem_c_in, a_.stem_c_out, a_.stem_ksize, a_.status, wt, main_));
+                                   a_.n, a_.stem_c_in, a_.stem_c_out, a_.stem_ksize, a_.dtype, a_.status, wt, main_));
     l.feat = feat;
     return PTV3_OK;
 }
@@ -318,6 +323,14 @@ int Pass::block(const ptv3_stage_args& st, int j, BbLevel& l, const void* conv_i
     return take_plan(false);
 }
 
+// fp32 projection of a stage transition, on split operands
+int Pass::project(const void* x, const void* w, const void* bias, int64_t n, int c_in, int c_out, void* split, void* out)
+{
+    BB_STEP(launch_split_f32((const float*)x, n, c_in, false, split, main_));
+    return launch_linear_split(split, w, (const float*)bias, nullptr, (float*)out, nullptr, n, c_in, c_out, 0, a_.status,
+                               main_);
+}
+
 int Pass::encoder(int s)
 {
     const ptv3_stage_args& st = a_.enc[s];
@@ -327,19 +340,27 @@ int Pass::encoder(int s)
     const void* x = l.feat;
     if (s > 0) {
         BbLevel& p = lv_[s - 1];
-        void* pooled = mem_.take<char>((size_t)l.n * st.c_out * 2);
+        void* pooled = mem_.take<char>((size_t)l.n * st.c_out * esize_);
         if (!pooled) return out_of_memory();
+        if (a_.dtype == PTV3_DTYPE_F32) {
+            const size_t split = align_up((size_t)p.n * st.c_in * 12, 256);
+            BB_STEP(need_ws(split + (size_t)p.n * st.c_out * 4));
+            BB_STEP(project(p.feat, st.w, st.b, p.n, st.c_in, st.c_out, ws_, ws_ + split));
+            BB_STEP(ptv3_pool_fwd(ws_ + split, nullptr, p.order, p.idx_ptr, l.n, st.c_out, st.scale, st.shift, pooled,
+                                  nullptr, st.reduce, a_.dtype, main_));
+        } else {
         const size_t bytes = ptv3_pool_stage_workspace_bytes(p.n, st.c_out);
         BB_STEP(need_ws(bytes));
         BB_STEP(ptv3_pool_stage_fwd(p.feat, st.w, st.b, nullptr, p.order, p.idx_ptr, p.n, l.n, st.c_in, st.c_out,
                                     st.scale, st.shift, pooled, nullptr, st.reduce, PTV3_DTYPE_BF16, a_.status, ws_,
                                     bytes, main_));
+        }
         x = pooled;
     }
     char* buf[2] = {nullptr, nullptr};
     for (int j = 0; j < st.n_blocks; ++j) {
         if (j < 2) {
-            buf[j] = mem_.take<char>((size_t)l.n * st.blocks[j].channels * 2);
+            buf[j] = mem_.take<char>((size_t)l.n * st.blocks[j].channels * esize_);
             if (!buf[j]) return out_of_memory();
         }
         BB_STEP(block(st, j, l, x, x, buf[j & 1]));
@@ -354,17 +375,28 @@ int Pass::decoder(int d)
     const ptv3_stage_args& st = a_.dec[d];
     BbLevel& c = lv_[a_.n_enc - 1 - d];
     BbLevel& l = lv_[a_.n_enc - 2 - d];
-    const size_t row = (size_t)l.n * st.c_out * 2;
+    const size_t row = (size_t)l.n * st.c_out * esize_;
     // out: skip + up-sampled rows; act: the skip branch alone, which the first block's convolution
     // reads (model.py:744-746 adds to `feat` only)
     char* buf[2] = {mem_.take<char>(row), mem_.take<char>(row)};
     char* act = mem_.take<char>(row);
     if (!buf[0] || !buf[1] || !act) return out_of_memory();
-    const size_t bytes = ptv3_unpool_stage_workspace_bytes(l.n, c.n, st.c_out);
-    BB_STEP(need_ws(bytes));
-    BB_STEP(ptv3_unpool_stage_fwd(l.feat, c.feat, st.w_skip, st.b_skip, st.w, st.b, l.cluster, l.n, c.n, st.c_skip, st.c_in,
-                                  st.c_out, st.scale_skip, st.shift_skip, st.scale, st.shift, buf[0], act,
-                                  PTV3_DTYPE_BF16, a_.status, ws_, bytes, main_));
+    if (a_.dtype == PTV3_DTYPE_F32) {
+        const int64_t wide = l.n * st.c_skip > c.n * st.c_in ? l.n * st.c_skip : c.n * st.c_in;
+        const size_t split = align_up((size_t)wide * 12, 256), rows = align_up(row, 256);
+        BB_STEP(need_ws(split + rows + (size_t)c.n * st.c_out * 4));
+        char *skip = ws_ + split, *child = ws_ + split + rows;
+        BB_STEP(project(c.feat, st.w, st.b, c.n, st.c_in, st.c_out, ws_, child));
+        BB_STEP(project(l.feat, st.w_skip, st.b_skip, l.n, st.c_skip, st.c_out, ws_, skip));
+        BB_STEP(ptv3_unpool_fwd(skip, child, l.cluster, l.n, st.c_out, st.scale_skip, st.shift_skip, st.scale, st.shift,
+                                buf[0], act, a_.dtype, main_));
+    } else {
+        const size_t bytes = ptv3_unpool_stage_workspace_bytes(l.n, c.n, st.c_out);
+        BB_STEP(need_ws(bytes));
+        BB_STEP(ptv3_unpool_stage_fwd(l.feat, c.feat, st.w_skip, st.b_skip, st.w, st.b, l.cluster, l.n, c.n, st.c_skip,
+                                      st.c_in, st.c_out, st.scale_skip, st.shift_skip, st.scale, st.shift, buf[0], act,
+                                      PTV3_DTYPE_BF16, a_.status, ws_, bytes, main_));
+    }
     const void *x = buf[0], *conv_in = act;
     for (int j = 0; j < st.n_blocks; ++j) {
         void* out = d == a_.n_dec - 1 && j == st.n_blocks - 1 ? a_.out : buf[(j + 1) & 1];
@@ -391,6 +423,8 @@ extern "C" int ptv3_backbone_fwd(const ptv3_backbone_args* a)
     PTV3_REQUIRE(a != nullptr, PTV3_ERR_INVALID_ARGUMENT, "ptv3_backbone_fwd: null argument block");
     PTV3_REQUIRE(a->n_enc >= 1 && a->n_enc <= BB_MAX_STAGES && a->n_dec == a->n_enc - 1 && a->n_dec >= 1 && a->enc && a->dec,
                  PTV3_ERR_UNSUPPORTED, "ptv3_backbone_fwd: %d encoder and %d decoder stages", a->n_enc, a->n_dec);
+    PTV3_REQUIRE(a->dtype == PTV3_DTYPE_BF16 || (a->dtype == PTV3_DTYPE_F32 && a->n <= 65535ll * 128),
+                 PTV3_ERR_UNSUPPORTED, "ptv3_backbone_fwd: dtype %d, %lld points", a->dtype, (long long)a->n);
     PTV3_REQUIRE(a->dec[a->n_dec - 1].n_blocks >= 1, PTV3_ERR_UNSUPPORTED,
                  "ptv3_backbone_fwd: the last decoder stage has no block");
     PTV3_REQUIRE(a->n >= 1 && a->n < (1ll << 31) && a->n_scenes >= 1 && a->depth >= 1 && a->k >= 1 &&

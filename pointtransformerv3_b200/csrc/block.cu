@@ -14,7 +14,9 @@
 // their epilogue (linear_tc05.cu) and, up to 64, the fused MLP; wider blocks take the
 // streamed-weight tensor-core kernel (gemm_tc05.cu) and the fused row kernel for the glue.
 #include "common.cuh"
+#include "conv_mma.cuh"
 #include "linear_small.cuh"
+#include "split_f32.cuh"
 #include "vec.cuh"
 
 namespace ptv3 {
@@ -72,9 +74,82 @@ static size_t carve_block(const ptv3_block_args* a, void* base, BlockBuffers* b)
     return c.off;
 }
 
+// ---- fp32: the same block with every product on split operands (split_f32.cuh) -----------------------
+// Layers hand their result to the next product as split rows where nothing else reads it (convolution ->
+// Linear, fc1 -> fc2); the others are split by a kernel of their own.
+struct BlockBuffersF32 {
+    float *y, *f1, *a, *qkv, *att, *f2;
+    void *s, *sh;           // split rows: n x 6C, n x 6 hidden
+};
+
+static size_t carve_block_f32(const ptv3_block_args* a, void* base, BlockBuffersF32* b)
+{
+    const size_t row = (size_t)a->n * a->channels * 4;
+    Carver c(base);
+    BlockBuffersF32 t;
+    t.y = (float*)c.take<char>(row);
+    t.f1 = (float*)c.take<char>(row);
+    t.a = (float*)c.take<char>(row);
+    t.qkv = (float*)c.take<char>(3 * row);
+    t.f2 = (float*)c.take<char>(row);
+    t.att = t.y;
+    t.s = c.take<char>(row * 3);
+    t.sh = c.take<char>((size_t)a->n * a->hidden * 12);
+    if (b) *b = t;
+    return c.off;
+}
+
+static int block_f32(const ptv3_block_args* a, cudaStream_t stream)
+{
+    BlockBuffersF32 b;
+    carve_block_f32(a, a->workspace, &b);
+    const int C = a->channels, H = a->hidden;
+    const int64_t n = a->n;
+    int rc;
+#define STEP(call)               \
+    do {                         \
+        rc = (call);             \
+        if (rc != PTV3_OK) return rc; \
+    } while (0)
+    auto f = [](const void* p) { return (const float*)p; };
+    // (the split of the convolution's input lies where the hidden rows come later)
+    STEP(launch_split_f32(f(a->conv_in), n, C, false, b.sh, stream));
+    STEP(launch_conv_split(b.sh, a->nbr, a->conv_weight, f(a->conv_bias), nullptr, b.s, a->row_order, n, C, C, 27, a->status,
+                           stream));
+    STEP(launch_linear_split(b.s, a->cpe_w, f(a->cpe_b), nullptr, b.y, nullptr, n, C, C, 0, a->status, stream));
+    STEP(ptv3_add_layernorm_fwd(b.y, a->feat, a->cpe_ln_w, a->cpe_ln_b, a->cpe_ln_eps, b.f1, a->n1_w, a->n1_b, a->n1_eps, b.a,
+                                n, C, PTV3_DTYPE_F32, stream));
+    STEP(launch_split_f32(b.a, n, C, false, b.s, stream));
+    STEP(launch_linear_split(b.s, a->qkv_w, f(a->qkv_b), nullptr, b.qkv, nullptr, n, C, 3 * C, 0, a->status, stream));
+    STEP(ptv3_attention_fwd(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.att, n, a->n_seq, a->max_seqlen, C, a->heads,
+                            a->scale, PTV3_DTYPE_F32, a->attention_algo, a->status, stream));
+    STEP(launch_split_f32(b.att, n, C, false, b.s, stream));
+    // (b.a is free until the second norm)
+    STEP(launch_linear_split(b.s, a->proj_w, f(a->proj_b), nullptr, b.qkv, nullptr, n, C, C, 0, a->status, stream));
+    STEP(ptv3_add_layernorm_fwd(b.qkv, b.f1, nullptr, nullptr, 0.f, b.f2, a->n2_w, a->n2_b, a->n2_eps, b.a, n, C,
+                                PTV3_DTYPE_F32, stream));
+    STEP(launch_split_f32(b.a, n, C, false, b.s, stream));
+    STEP(launch_linear_split(b.s, a->fc1_w, f(a->fc1_b), nullptr, nullptr, b.sh, n, C, H, 1, a->status, stream));
+    STEP(launch_linear_split(b.sh, a->fc2_w, f(a->fc2_b), b.f2, (float*)a->out, nullptr, n, H, C, 0, a->status, stream));
+#undef STEP
+    return PTV3_OK;
+}
+
+int block_f32_supported(int channels, int heads, int hidden)
+{
+    const int d = heads > 0 && channels % heads == 0 ? channels / heads : 0;
+    return channels >= 32 && channels <= 1024 && (channels & (channels - 1)) == 0 && hidden % 32 == 0 && hidden >= channels &&
+           (d == 8 || d == 16 || d == 32 || d == 64);
+}
+
 }  // namespace ptv3
 
 using namespace ptv3;
+
+extern "C" int ptv3_block_f32_supported(int channels, int heads, int hidden)
+{
+    return block_f32_supported(channels, heads, hidden);
+}
 
 extern "C" int ptv3_block_supported(int channels, int heads, int hidden, int dtype)
 {
@@ -92,14 +167,15 @@ extern "C" int ptv3_block_supported(int channels, int heads, int hidden, int dty
 extern "C" size_t ptv3_block_workspace_bytes(const ptv3_block_args* a)
 {
     if (!a || a->n < 0) return 0;
-    return carve_block(a, nullptr, nullptr);
+    return a->dtype == PTV3_DTYPE_F32 ? carve_block_f32(a, nullptr, nullptr) : carve_block(a, nullptr, nullptr);
 }
 
 extern "C" int ptv3_block_fwd(const ptv3_block_args* a, void* stream_)
 {
     PTV3_REQUIRE(a != nullptr, PTV3_ERR_INVALID_ARGUMENT, "ptv3_block_fwd: null argument block");
-    PTV3_REQUIRE(ptv3_block_supported(a->channels, a->heads, a->hidden, a->dtype), PTV3_ERR_UNSUPPORTED,
-                 "ptv3_block_fwd: bf16 only, channels and hidden multiples of 16 (got %d, %d, dtype %d)",
+    const bool f32 = a->dtype == PTV3_DTYPE_F32 && block_f32_supported(a->channels, a->heads, a->hidden) && a->nbr;
+    PTV3_REQUIRE(f32 || ptv3_block_supported(a->channels, a->heads, a->hidden, a->dtype), PTV3_ERR_UNSUPPORTED,
+                 "ptv3_block_fwd: bf16 (or fp32 with split weights), channels and hidden multiples of 16 (got %d, %d, dtype %d)",
                  a->channels, a->hidden, a->dtype);
     PTV3_REQUIRE(a->n >= 0, PTV3_ERR_INVALID_ARGUMENT, "ptv3_block_fwd: n < 0");
     if (a->n == 0) return PTV3_OK;
@@ -108,10 +184,10 @@ extern "C" int ptv3_block_fwd(const ptv3_block_args* a, void* stream_)
                      a->proj_w && a->proj_b && a->n2_w && a->n2_b && a->fc1_w && a->fc1_b && a->fc2_w &&
                      a->fc2_b && a->order && a->pad && a->unpad && a->cu_seqlens && (a->nbr || a->pair_in),
                  PTV3_ERR_INVALID_ARGUMENT, "ptv3_block_fwd: null pointer");
-    PTV3_REQUIRE(a->workspace_bytes >= carve_block(a, nullptr, nullptr), PTV3_ERR_INVALID_ARGUMENT,
-                 "ptv3_block_fwd: workspace of %zu bytes, %zu needed", a->workspace_bytes,
-                 carve_block(a, nullptr, nullptr));
+    PTV3_REQUIRE(a->workspace_bytes >= ptv3_block_workspace_bytes(a), PTV3_ERR_INVALID_ARGUMENT,
+                 "ptv3_block_fwd: workspace of %zu bytes, %zu needed", a->workspace_bytes, ptv3_block_workspace_bytes(a));
     cudaStream_t stream = (cudaStream_t)stream_;
+    if (f32) return block_f32(a, stream);
     BlockBuffers b;
     carve_block(a, a->workspace, &b);
     const int C = a->channels, dt = a->dtype;
@@ -240,4 +316,33 @@ extern "C" int ptv3_unpool_stage_fwd(const void* skip_feat, const void* child_fe
     if (rc != PTV3_OK) return rc;
     return ptv3_unpool_fwd(skip_lin, child_lin, cluster, n, c_out, skip_scale, skip_shift, child_scale, child_shift,
                            out, skip_act, dtype, stream);
+}
+
+extern "C" int ptv3_linear_split_fwd(const void* x_split, const void* w_split, const float* bias, const float* residual,
+                                     float* out, int64_t n, int k, int n_out, int gelu, uint32_t* status, void* stream)
+{
+    PTV3_REQUIRE(n >= 0 && n <= 65535ll * 128 && k >= 32 && k % 32 == 0 && n_out >= 32 && n_out % 32 == 0 &&
+                     k <= 8192 && n_out <= 8192,
+                 PTV3_ERR_UNSUPPORTED, "ptv3_linear_split_fwd: k and n_out multiples of 32, up to 8 388 480 rows (got %d, %d)", k, n_out);
+    if (n == 0) return PTV3_OK;
+    PTV3_REQUIRE(x_split && w_split && out && status &&
+                     (((uintptr_t)x_split | (uintptr_t)w_split | (uintptr_t)out | (uintptr_t)residual) & 15) == 0,
+                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_linear_split_fwd: null pointer or alignment");
+    return launch_linear_split(x_split, w_split, bias, residual, out, nullptr, n, k, n_out, gelu, status,
+                               (cudaStream_t)stream);
+}
+
+extern "C" int ptv3_subm_conv_split_fwd(const void* feat_split, const int32_t* nbr, const void* w_split, const float* bias,
+                                        float* out, const int64_t* row_order, int64_t n, int c_in, int c_out,
+                                        int kernel_volume, uint32_t* status, void* stream)
+{
+    PTV3_REQUIRE(n >= 0 && n < (1ll << 31) && c_in >= 32 && c_in % 32 == 0 && (c_out == 32 || c_out % 64 == 0) &&
+                     c_in <= 4096 && c_out <= 4096 && c_out >= 32 && kernel_volume >= 1 && kernel_volume <= 27,
+                 PTV3_ERR_UNSUPPORTED, "ptv3_subm_conv_split_fwd: %d -> %d channels, %d offsets", c_in, c_out, kernel_volume);
+    if (n == 0) return PTV3_OK;
+    PTV3_REQUIRE(feat_split && nbr && w_split && out && status &&
+                     (((uintptr_t)feat_split | (uintptr_t)w_split | (uintptr_t)out) & 15) == 0,
+                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_subm_conv_split_fwd: null pointer or alignment");
+    return launch_conv_split(feat_split, nbr, w_split, bias, out, nullptr, row_order, n, c_in, c_out, kernel_volume, status,
+                             (cudaStream_t)stream);
 }

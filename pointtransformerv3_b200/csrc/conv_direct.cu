@@ -435,9 +435,13 @@ static size_t conv_direct_index_bytes(int64_t n) { return voxel_index_bytes(n); 
 
 int conv_direct_from_index(const VoxelIndex& vi, const void* feat, const int32_t* indices, const void* weight,
                            const float* bn_scale, const float* bn_shift, void* out, const int64_t* row_order,
-                           int64_t n, int c_in, int c_out, int ksize, uint32_t* status, void* weight_scratch,
-                           cudaStream_t stream)
+                           int64_t n, int c_in, int c_out, int ksize, int dtype, uint32_t* status,
+                           void* weight_scratch, cudaStream_t stream)
 {
+    if (dtype == PTV3_DTYPE_F32)
+        return launch_conv_direct<float>(feat, indices, weight, nullptr, bn_scale, bn_shift, 1, out, row_order, n, c_in,
+                                         c_out, ksize, vi.keys, vi.vals, vi.cap_mask, vi.cells, status, weight_scratch,
+                                         stream);
     return launch_conv_direct_mma(feat, indices, weight, nullptr, bn_scale, bn_shift, 1, out, row_order, n, c_in, c_out,
                                   ksize, vi.keys, vi.vals, vi.cap_mask, vi.cells, status, weight_scratch, stream);
 }

@@ -41,6 +41,7 @@
 #include "common.cuh"
 #include "conv_mma.cuh"
 #include "mma_util.cuh"
+#include "split_f32.cuh"
 #include "tc05.cuh"
 
 namespace ptv3 {
@@ -55,15 +56,28 @@ constexpr int CT_GATHER_WARPS = 8;
 struct ConvTcArgs {
     const __nv_bfloat16* feat;
     const int32_t* nbr;            // kvol x n, columns in tile order
-    const __nv_bfloat16* bias;     // cout or NULL
-    __nv_bfloat16* out;
+    const void* bias;              // cout or NULL, of the output's type
+    void* out;                     // bf16 or fp32
+    __nv_bfloat16* split_out;      // fp32: the result as split rows (n x 6 cout) instead, or NULL
     const int64_t* row_order;      // voxel of every tile position, or NULL
     int64_t n;
     int cin, cout, kvol;
     uint32_t* status;
 };
 
-template <int BN, int KC, int STAGES, int NI, bool SPLIT>
+// eight finished fp32 columns of a row
+__device__ __forceinline__ void ct_store_f32(const ConvTcArgs& a, int64_t row, int col, const float* y)
+{
+    if (a.split_out) {
+        split_store8(a.split_out + row * 6 * a.cout + col, a.cout, y);
+        return;
+    }
+    float4* o = reinterpret_cast<float4*>((float*)a.out + row * a.cout + col);
+    o[0] = make_float4(y[0], y[1], y[2], y[3]);
+    o[1] = make_float4(y[4], y[5], y[6], y[7]);
+}
+
+template <int BN, int KC, int STAGES, int NI, bool SPLIT, bool F32>
 __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                const ConvTcArgs a)
 {
@@ -75,7 +89,9 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
     // of two for the allocation).  A slot of the ring must always be consumed by the same issuer
     // (STAGES a multiple of NI): an issuer that met a slot whose previous use another, slower issuer had
     // not consumed yet would take the parity of that older phase for its own.
-    constexpr int TM_USED = NI * BN;
+    // fp32: SPLIT_ACCS accumulators each (split_f32.cuh)
+    constexpr int ACCS = F32 ? SPLIT_ACCS : 1;
+    constexpr int TM_USED = NI * ACCS * BN;
     constexpr int TM_COLS = TM_USED <= 32 ? 32 : TM_USED <= 64 ? 64 : TM_USED <= 128 ? 128 : TM_USED <= 256 ? 256 : 512;
     static_assert(TM_USED <= 512 && STAGES % NI == 0, "issuers and accumulators");
     static_assert(STAGE_BYTES % 1024 == 0 && A_BYTES % 1024 == 0, "operand tiles start on a swizzle atom");
@@ -105,6 +121,7 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
     float* bias_s = reinterpret_cast<float*>(smem + OFF_BIAS);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + OFF_BAR + 8 * (2 * STAGES + 1));
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    uint32_t* used_s = tmem_slot + 2;              // fp32: the accumulators an issuer has written
     const uint32_t full0 = sbase + OFF_BAR, empty0 = full0 + 8 * STAGES, accfull = empty0 + 8 * STAGES;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -117,7 +134,7 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
             mbar_init(full0 + 8 * s, 2);        // the gathering warp of the stage + its weight load
             mbar_init(empty0 + 8 * s, 1);
         }
-        mbar_init(accfull, NI);
+        mbar_init(accfull, F32 ? 2 * NI : NI);     // the products of every issuer; fp32: and its word in used_s
         *abort = 0;
         fence_barrier_init();
         prefetch_tensormap(&map_w);
@@ -135,7 +152,7 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
         const int64_t i = row0 + tid;
         rows_s[tid] = i < a.n ? (a.row_order ? a.row_order[i] : i) : -1;
     }
-    for (int c = tid; c < BN; c += CT_THREADS) bias_s[c] = a.bias ? __bfloat162float(a.bias[col0 + c]) : 0.f;
+    for (int c = tid; c < BN; c += CT_THREADS) bias_s[c] = !a.bias ? 0.f : F32 ? ((const float*)a.bias)[col0 + c] : __bfloat162float(((const __nv_bfloat16*)a.bias)[col0 + c]);
     {
         // A warp stages whole offsets (four coalesced rows of 32 entries each), all of its loads issued
         // before the first store, and notes in the same pass whether the tile has the offset at all.
@@ -241,12 +258,29 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
         const int q = warp & 3, half = warp >> 2;      // lane quarter of tensor memory, half of the columns
         const int64_t v = rows_s[q * 32 + lane];
         const uint32_t tm = tmem_base + ((uint32_t)(q * 32) << 16);
-        __nv_bfloat16* orow = a.out + v * a.cout + col0;
+        __nv_bfloat16* orow = (__nv_bfloat16*)a.out + v * a.cout + col0;
         constexpr int NCB = BN / 32;                   // 32-column blocks, split between the two halves
 #pragma unroll 1
         for (int cb = half * ((NCB + 1) / 2); cb < (half == 0 ? (NCB + 1) / 2 : NCB); ++cb) {
             uint32_t acc[32];
-            if (read_acc) {
+            if (F32) {
+                // from the small products to the leading ones, issuer after issuer
+#pragma unroll
+                for (int e = 0; e < 32; ++e) acc[e] = 0;
+#pragma unroll 1
+                for (int z = ACCS - 1; z >= 0; --z)
+#pragma unroll 1
+                    for (int i = 0; i < NI; ++i) {
+                        if (!read_acc || !((*reinterpret_cast<volatile uint32_t*>(used_s + i) >> z) & 1)) continue;
+                        uint32_t more[32];
+                        tmem_ld32(tm + (i * ACCS + z) * BN + cb * 32, more);
+                        tmem_ld_wait();
+                        tmem_ld_fence(more);
+#pragma unroll
+                        for (int e = 0; e < 32; ++e)
+                            acc[e] = __float_as_uint(__uint_as_float(acc[e]) + __uint_as_float(more[e]));
+                    }
+            } else if (read_acc) {
                 tmem_ld32(tm + cb * 32, acc);
                 tmem_ld_wait();
                 // the other issuers' partial sums, added in a fixed order
@@ -273,6 +307,16 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
                 continue;
             }
             if (v < 0) continue;
+            if (F32) {
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    float y[8];
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) y[i] = __uint_as_float(acc[g * 8 + i]) + bias_s[cb * 32 + g * 8 + i];
+                    ct_store_f32(a, v, col0 + cb * 32 + g * 8, y);
+                }
+                continue;
+            }
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
                 uint4 o4;
@@ -292,41 +336,57 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
         if (lane == 0) {
             constexpr uint32_t idesc = umma_idesc_bf16(CT_TM, BN);
             const int me = warp - CT_GATHER_WARPS;
-            const uint32_t tm_acc = tmem_base + me * BN;
+            const uint32_t tm_acc = tmem_base + me * ACCS * BN;
+            uint32_t used = 0;
+            int lead = 0;          // stages of this issuer with leading products
             for (int it = me; it < nit; it += NI) {
                 const int s = it % STAGES;
                 ok &= mbar_wait(full0 + 8 * s, (it / STAGES) & 1, abort);
                 fence_after_sync();
                 const uint32_t sa = sbase + s * STAGE_BYTES, sb = sa + A_BYTES;
 #pragma unroll
-                for (int k4 = 0; k4 < KC / 16; ++k4)
-                    umma_bf16(tm_acc, umma_desc_kmajor(sa + k4 * 32, ROWB), umma_desc_kmajor(sb + k4 * 32, ROWB),
-                              idesc, it >= NI || k4 > 0);
+                for (int k4 = 0; k4 < KC / 16; ++k4) {
+                    uint32_t acc = 0;
+                    if (F32) acc = ((first + it) % kchunks * KC + k4 * 16) * 6 < a.cin ? lead % SPLIT_MAIN : SPLIT_MAIN;
+                    umma_bf16(tm_acc + acc * BN, umma_desc_kmajor(sa + k4 * 32, ROWB), umma_desc_kmajor(sb + k4 * 32, ROWB),
+                              idesc, F32 ? (used >> acc) & 1 : it >= NI || k4 > 0);
+                    used |= 1u << acc;
+                }
+                if (F32) lead += (first + it) % kchunks * KC * 6 < a.cin;
                 umma_commit(empty0 + 8 * s);
             }
             if (nit > me) umma_commit(accfull);
             else if (nit > 0) mbar_arrive_one(accfull);
+            if (F32 && nit > 0) {
+                used_s[me] = used;
+                mbar_arrive_one(accfull);
+            }
         }
     }
     if (SPLIT) {
         // this CTA's rows: the peers' partial sums in rank order, bias, bf16
         cluster_sync();
         const int parts = (int)gridDim.z, rows = CT_TM / parts, r0 = rows * (int)cluster_rank();
-        for (int e = tid; e < rows * (BN / 4); e += CT_THREADS) {
-            const int r = r0 + e / (BN / 4), c = e % (BN / 4) * 4;
+        for (int e = tid; e < rows * (BN / 8); e += CT_THREADS) {
+            const int r = r0 + e / (BN / 8), c = e % (BN / 8) * 8;
             const int64_t v = rows_s[r];
             if (v < 0) continue;
             const uint32_t at = sbase + (r * PART_PITCH + c) * 4;
-            float4 t = ld_peer_f4(at, 0);
-            for (int z = 1; z < parts; ++z) {
-                const float4 m = ld_peer_f4(at, z);
-                t.x += m.x;
-                t.y += m.y;
-                t.z += m.z;
-                t.w += m.w;
+            float y[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i] = 0.f;
+            for (int z = 0; z < parts; ++z) {
+                const float4 m = ld_peer_f4(at, z), w = ld_peer_f4(at + 16, z);
+                y[0] += m.x; y[1] += m.y; y[2] += m.z; y[3] += m.w;
+                y[4] += w.x; y[5] += w.y; y[6] += w.z; y[7] += w.w;
             }
-            *reinterpret_cast<uint2*>(a.out + v * a.cout + col0 + c) =
-                make_uint2(pack_bf16(t.x + bias_s[c], t.y + bias_s[c + 1]), pack_bf16(t.z + bias_s[c + 2], t.w + bias_s[c + 3]));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i] += bias_s[c + i];
+            if (F32)
+                ct_store_f32(a, v, col0 + c, y);
+            else
+                *reinterpret_cast<uint4*>((__nv_bfloat16*)a.out + v * a.cout + col0 + c) =
+                    make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
         }
         cluster_sync();      // a peer's shared memory outlives its readers
     }
@@ -350,10 +410,10 @@ template <int BN, int KC, int STAGES>
 static constexpr size_t conv_tc05_smem()
 {
     return (size_t)STAGES * (CT_TM + BN) * KC * 2 + CT_MAX_KVOL * CT_TM * 4 + CT_TM * 8 + 32 * 4 + BN * 4 +
-           8 * (2 * STAGES + 1) + 16 + 1024;
+           8 * (2 * STAGES + 1) + 32 + 1024;
 }
 
-template <int BN, int KC, int STAGES, int NI, bool SPLIT>
+template <int BN, int KC, int STAGES, int NI, bool SPLIT, bool F32>
 static int launch_conv_tc05_as(const void* weight, const ConvTcArgs& a, cudaStream_t stream, int parts)
 {
     CUtensorMap mw;
@@ -361,7 +421,7 @@ static int launch_conv_tc05_as(const void* weight, const ConvTcArgs& a, cudaStre
     const int rc = make_tensor_map_bf16(&mw, weight, (uint64_t)a.cout, wcols, wcols * 2, BN, KC);
     if (rc) return rc;
     constexpr size_t smem = conv_tc05_smem<BN, KC, STAGES>();
-    auto kern = conv_tc05_kernel<BN, KC, STAGES, NI, SPLIT>;
+    auto kern = conv_tc05_kernel<BN, KC, STAGES, NI, SPLIT, F32>;
     if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_subm_conv_fwd: shared memory attribute");
     const dim3 grid((unsigned)((a.n + CT_TM - 1) / CT_TM), a.cout / BN, parts);
@@ -371,14 +431,14 @@ static int launch_conv_tc05_as(const void* weight, const ConvTcArgs& a, cudaStre
 }
 
 // CTAs in clusters of `parts` that run at once (the driver's answer: a cluster lives in one GPC)
-template <int BN, int KC, int STAGES, int NI>
+template <int BN, int KC, int STAGES, int NI, bool F32>
 static int conv_tc05_capacity(int parts)
 {
     static std::atomic<int> known[4];
     const int slot = parts == 2 ? 1 : parts == 4 ? 2 : 3;
     int c = known[slot].load(std::memory_order_relaxed);
     if (c == 0) {
-        auto kern = conv_tc05_kernel<BN, KC, STAGES, NI, true>;
+        auto kern = conv_tc05_kernel<BN, KC, STAGES, NI, true, F32>;
         if (allow_smem(kern) != cudaSuccess) return 0;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(148, 1, parts);
@@ -409,48 +469,40 @@ struct ConvVariant {
     int (*capacity)(int);
 };
 constexpr double CT_FIXED_US = 6.5;
-constexpr int CT_VARIANTS = 4;
-static const ConvVariant g_variants[CT_VARIANTS] = {
-    {64, 1, 0.20, launch_conv_tc05_as<64, 64, 8, 2, false>, launch_conv_tc05_as<64, 64, 8, 2, true>,
-     conv_tc05_capacity<64, 64, 8, 2>},
-    // many tiles: two CTAs per SM, so that one tile's prologue and epilogue run beside another's products
-    {64, 2, 0.35, launch_conv_tc05_as<64, 64, 4, 2, false>, nullptr, nullptr},
-    {128, 1, 0.28, launch_conv_tc05_as<128, 64, 6, 2, false>, launch_conv_tc05_as<128, 64, 6, 2, true>,
-     conv_tc05_capacity<128, 64, 6, 2>},
-    {256, 1, 0.44, launch_conv_tc05_as<256, 64, 4, 2, false>, launch_conv_tc05_as<256, 64, 4, 2, true>,
-     conv_tc05_capacity<256, 64, 4, 2>},
+constexpr int CT_VARIANTS = 5;
+template <int BN, int STAGES, bool F32>
+static constexpr ConvVariant conv_variant(double stage_us)
+{
+    return {BN, 1, stage_us, launch_conv_tc05_as<BN, 64, STAGES, 2, false, F32>, launch_conv_tc05_as<BN, 64, STAGES, 2, true, F32>,
+            conv_tc05_capacity<BN, 64, STAGES, 2, F32>};
+}
+// [fp32 output][variant].  Second entry: many tiles, two CTAs per SM, so that one tile's prologue and epilogue
+// run beside another's products.  Last: 32 output channels (fp32; bf16 has its own path for them).
+static const ConvVariant g_variants[2][CT_VARIANTS] = {
+    {conv_variant<64, 8, false>(0.20),
+     {64, 2, 0.35, launch_conv_tc05_as<64, 64, 4, 2, false, false>, nullptr, nullptr},
+     conv_variant<128, 6, false>(0.28), conv_variant<256, 4, false>(0.44), {1 << 20, 1, 0, nullptr, nullptr, nullptr}},
+    // (fp32: an issuer's four accumulators of 64 columns fill the tensor memory of an SM)
+    {conv_variant<64, 8, true>(0.20), {1 << 20, 1, 0, nullptr, nullptr, nullptr}, {1 << 20, 1, 0, nullptr, nullptr, nullptr},
+     {1 << 20, 1, 0, nullptr, nullptr, nullptr}, conv_variant<32, 8, true>(0.18)},
 };
 
-int launch_conv_tc05(const void* feat, const int32_t* nbr, const void* weight, const void* bias, void* out,
-                     const int64_t* row_order, int64_t n, int c_in, int c_out, int kvol, uint32_t* status,
-                     cudaStream_t stream)
+// The tile width and the cluster size with the shortest estimated time: waves of CTAs, each taking a
+// fixed time (prologue, epilogue) and its stages.  Wide tiles gather a row once for more output
+// channels; clusters fill SMs that a single wave leaves idle.  The constants are measured (us on B200:
+// 27 voxels x 512 channels in clusters of eight takes 12.2 / 14.6 / 19.9 with 64 / 128 / 256 channels a
+// tile, 46.3 without a cluster); what they give: 441 x 512 47 -> 19, 1 700 x 256 27 -> 18,
+// 2 200 x 512 49 -> 39, 12 000 x 256 68 -> 53, 12 000 x 128 31 -> 22.
+static int launch_conv_tc05_best(const void* weight, const ConvTcArgs& a, bool f32, cudaStream_t stream)
 {
-    ConvTcArgs a{};
-    a.feat = (const __nv_bfloat16*)feat;
-    a.nbr = nbr;
-    a.bias = (const __nv_bfloat16*)bias;
-    a.out = (__nv_bfloat16*)out;
-    a.row_order = row_order;
-    a.n = n;
-    a.cin = c_in;
-    a.cout = c_out;
-    a.kvol = kvol;
-    a.status = status;
-    if (c_in == 32) return launch_conv_tc05_as<32, 32, 6, 2, false>(weight, a, stream, 1);
-    // The tile width and the cluster size with the shortest estimated time: waves of CTAs, each taking a
-    // fixed time (prologue, epilogue) and its stages.  Wide tiles gather a row once for more output
-    // channels; clusters fill SMs that a single wave leaves idle.  The constants are measured (us on B200:
-    // 27 voxels x 512 channels in clusters of eight takes 12.2 / 14.6 / 19.9 with 64 / 128 / 256 channels a
-    // tile, 46.3 without a cluster); what they give: 441 x 512 47 -> 19, 1 700 x 256 27 -> 18,
-    // 2 200 x 512 49 -> 39, 12 000 x 256 68 -> 53, 12 000 x 128 31 -> 22.
-    const double stages = (double)kvol * (c_in / 64);
-    const int64_t tiles = (n + CT_TM - 1) / CT_TM;
+    const double stages = (double)a.kvol * (a.cin / 64);
+    const int64_t tiles = (a.n + CT_TM - 1) / CT_TM;
     double best = 0;
     int best_v = -1, best_parts = 1;
     for (int v = 0; v < CT_VARIANTS; ++v) {
-        const ConvVariant& var = g_variants[v];
-        if (c_out % var.bn) continue;
-        const int64_t ctas = tiles * (c_out / var.bn);
+        const ConvVariant& var = g_variants[f32][v];
+        if (a.cout % var.bn) continue;
+        const int64_t ctas = tiles * (a.cout / var.bn);
         for (int parts = 1; parts <= (var.split ? 8 : 1); parts *= 2) {
             const int64_t room = parts == 1 ? (int64_t)148 * var.per_sm : (int64_t)var.capacity(parts);
             if (room < parts) continue;
@@ -463,8 +515,47 @@ int launch_conv_tc05(const void* feat, const int32_t* nbr, const void* weight, c
             }
         }
     }
-    const ConvVariant& var = g_variants[best_v];
+    const ConvVariant& var = g_variants[f32][best_v];
     return (best_parts > 1 ? var.split : var.plain)(weight, a, stream, best_parts);
+}
+
+int launch_conv_tc05(const void* feat, const int32_t* nbr, const void* weight, const void* bias, void* out,
+                     const int64_t* row_order, int64_t n, int c_in, int c_out, int kvol, uint32_t* status,
+                     cudaStream_t stream)
+{
+    ConvTcArgs a{};
+    a.feat = (const __nv_bfloat16*)feat;
+    a.nbr = nbr;
+    a.bias = bias;
+    a.out = out;
+    a.row_order = row_order;
+    a.n = n;
+    a.cin = c_in;
+    a.cout = c_out;
+    a.kvol = kvol;
+    a.status = status;
+    if (c_in == 32) return launch_conv_tc05_as<32, 32, 6, 2, false, false>(weight, a, stream, 1);
+    return launch_conv_tc05_best(weight, a, false, stream);
+}
+
+// fp32 on split operands (see split_f32.cuh): feat n x 6 c_in, weight c_out x kvol x 6 c_in bf16
+int launch_conv_split(const void* feat, const int32_t* nbr, const void* weight, const float* bias, float* out,
+                      void* split_out, const int64_t* row_order, int64_t n, int c_in, int c_out, int kvol,
+                      uint32_t* status, cudaStream_t stream)
+{
+    ConvTcArgs a{};
+    a.feat = (const __nv_bfloat16*)feat;
+    a.nbr = nbr;
+    a.bias = bias;
+    a.out = out;
+    a.split_out = (__nv_bfloat16*)split_out;
+    a.row_order = row_order;
+    a.n = n;
+    a.cin = 6 * c_in;
+    a.cout = c_out;
+    a.kvol = kvol;
+    a.status = status;
+    return launch_conv_tc05_best(weight, a, true, stream);
 }
 
 }  // namespace ptv3

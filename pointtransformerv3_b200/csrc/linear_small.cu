@@ -13,6 +13,7 @@
 //     statistics are merged from the mean and centred square sum of every 32 columns.
 #include "common.cuh"
 #include "linear_small.cuh"
+#include "split_f32.cuh"
 #include "tc05.cuh"
 #include "vec.cuh"
 
@@ -25,11 +26,12 @@ constexpr int LS_A_BYTES = LS_BM * LS_BK * 2, LS_B_BYTES = LS_BN * LS_BK * 2, LS
 constexpr int LS_MAX_STAGES = 8;
 constexpr int LS_EPI_WARPS = 8, LS_THREADS = 64 + 32 * LS_EPI_WARPS;
 constexpr int LS_PITCH = LS_BN + 4;                    // floats of a row of partial sums
-constexpr int LS_PLAIN = 0, LS_GELU = 1, LS_RESIDUAL = 2, LS_LN = 4;
+constexpr int LS_PLAIN = 0, LS_GELU = 1, LS_RESIDUAL = 2, LS_LN = 4, LS_F32 = 8;
 
 struct LinearSmallArgs {
-    const __nv_bfloat16 *bias, *residual;
-    __nv_bfloat16* out;                                // LN: the sum, or NULL
+    const void *bias, *residual;                       // bf16; fp32 with LS_F32
+    void* out;                                         // LN: the sum, or NULL
+    __nv_bfloat16* split_out;                          // LS_F32: the result as split rows (n x 6 n_out) instead
     const __nv_bfloat16 *ln1_w, *ln1_b, *ln2_w, *ln2_b;
     float eps1, eps2;
     __nv_bfloat16* norm_out;
@@ -58,6 +60,32 @@ __device__ __forceinline__ float2 ld_peer_f2(uint32_t addr, uint32_t rank)
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p) : "r"(addr), "r"(rank));
     asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(p) : "memory");
     return v;
+}
+
+// LS_F32: eight finished columns of a row, as floats or as split bf16 parts (see split_f32.cuh)
+template <int MODE>
+__device__ __forceinline__ void ls_store_f32(const LinearSmallArgs& a, int64_t row, int col, const float* acc,
+                                             const float* bias)
+{
+    float y[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        y[i] = acc[i] + bias[i];
+        if (MODE & LS_GELU) y[i] = 0.5f * y[i] * (1.f + erff(y[i] * 0.70710678118654752f));
+    }
+    if (MODE & LS_RESIDUAL) {
+        const float4* r = reinterpret_cast<const float4*>((const float*)a.residual + row * a.n_out + col);
+        const float4 r0 = r[0], r1 = r[1];
+        y[0] += r0.x; y[1] += r0.y; y[2] += r0.z; y[3] += r0.w;
+        y[4] += r1.x; y[5] += r1.y; y[6] += r1.z; y[7] += r1.w;
+    }
+    if (a.split_out) {
+        split_store8(a.split_out + row * 6 * a.n_out + col, a.n_out, y);
+        return;
+    }
+    float4* o = reinterpret_cast<float4*>((float*)a.out + row * a.n_out + col);
+    o[0] = make_float4(y[0], y[1], y[2], y[3]);
+    o[1] = make_float4(y[4], y[5], y[6], y[7]);
 }
 
 template <int MODE>
@@ -98,6 +126,8 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
                    accfull = empty0 + 8 * LS_MAX_STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + off_stat + LS_STAT_BYTES + 8 * (2 * LS_MAX_STAGES + 1));
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    uint32_t* used_s = tmem_slot + 2;                      // LS_F32: the accumulators in use
+    constexpr int TM_COLS = (MODE & LS_F32) ? SPLIT_ACCS * LS_BN : LS_BN;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int col0 = blockIdx.x * LS_BN, row0 = blockIdx.y * LS_BM;
@@ -110,7 +140,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
             mbar_init(full0 + 8 * s, 1);
             mbar_init(empty0 + 8 * s, 1);
         }
-        mbar_init(accfull, 1);
+        mbar_init(accfull, (MODE & LS_F32) ? 2 : 1);       // the products; LS_F32: and the word below
         *abort = 0;
         fence_barrier_init();
         prefetch_tensormap(&map_x);
@@ -121,7 +151,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
         }
     }
     if (warp == 1) {
-        tmem_alloc(smem_u32_generic(tmem_slot), LS_BN);
+        tmem_alloc(smem_u32_generic(tmem_slot), TM_COLS);
         // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
         pdl_launch_next();
     }
@@ -130,8 +160,17 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
         constexpr int N = (MODE & LS_LN) ? 5 : 1;
         for (int i = tid; i < N * LS_BN; i += LS_THREADS) {
             const int j = i / LS_BN;
-            const __nv_bfloat16* p = j == 0 ? a.bias : j == 1 ? a.ln1_w : j == 2 ? a.ln1_b : j == 3 ? a.ln2_w : a.ln2_b;
-            params[i] = p ? __bfloat162float(p[col0 + i % LS_BN]) : 0.f;
+            const int c = col0 + i % LS_BN;
+            if (MODE & LS_F32) {
+                params[i] = a.bias && c < a.n_out ? ((const float*)a.bias)[c] : 0.f;
+                continue;
+            }
+            const __nv_bfloat16* p = j == 0   ? (const __nv_bfloat16*)a.bias
+                                     : j == 1 ? a.ln1_w
+                                     : j == 2 ? a.ln1_b
+                                     : j == 3 ? a.ln2_w
+                                              : a.ln2_b;
+            params[i] = p ? __bfloat162float(p[c]) : 0.f;
         }
     }
     fence_before_sync();
@@ -164,34 +203,54 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
     } else if (warp == 1) {
         if (lane == 0) {
             constexpr uint32_t idesc = umma_idesc_bf16(LS_BM, LS_BN);
+            uint32_t used = 0;
             for (int kc = 0; kc < nk; ++kc) {
                 const int s = kc % stages;
                 ok &= mbar_wait(full0 + 8 * s, (kc / stages) & 1, abort);
                 fence_after_sync();
                 const uint32_t sa = sbase + s * LS_STAGE, sb = sa + LS_A_BYTES;
 #pragma unroll
-                for (int k4 = 0; k4 < LS_BK / 16; ++k4)
-                    umma_bf16(tmem_base, umma_desc_kmajor(sa + k4 * 32, 128), umma_desc_kmajor(sb + k4 * 32, 128), idesc,
-                              kc > 0 || k4 > 0);
+                for (int k4 = 0; k4 < LS_BK / 16; ++k4) {
+                    uint32_t acc = 0;
+                    if (MODE & LS_F32) {
+                        const int step = (k0 + kc * LS_BK) / 16 + k4;      // of 16 columns; the first sixth is the leading piece
+                        acc = step * 96 < a.k ? step % SPLIT_MAIN : SPLIT_MAIN;
+                    }
+                    umma_bf16(tmem_base + acc * LS_BN, umma_desc_kmajor(sa + k4 * 32, 128),
+                              umma_desc_kmajor(sb + k4 * 32, 128), idesc, (used >> acc) & 1);
+                    used |= 1u << acc;
+                }
                 umma_commit(empty0 + 8 * s);
             }
             umma_commit(accfull);
+            if (MODE & LS_F32) {
+                *used_s = used;
+                mbar_arrive_one(accfull);
+            }
         }
         __syncwarp();
     } else {
-        if ((MODE & (LS_RESIDUAL | LS_LN)) && parts == 1 && live) {
+        if ((MODE & (LS_RESIDUAL | LS_LN)) && !(MODE & LS_F32) && parts == 1 && live) {
 #pragma unroll
             for (int g = 0; g < 4; ++g)
-                res[g] = *reinterpret_cast<const uint4*>(a.residual + row * a.n_out + col0 + c0 + g * 8);
+                res[g] = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)a.residual + row * a.n_out + col0 + c0 + g * 8);
         }
         ok &= mbar_wait(accfull, 0, abort);
         fence_after_sync();
         uint32_t acc[32];
-        tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + c0, acc);
-        tmem_ld_wait();
-        tmem_ld_fence(acc);
+        const uint32_t used = (MODE & LS_F32) ? *reinterpret_cast<volatile uint32_t*>(used_s) : 1u;
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(acc[i]);
+        for (int i = 0; i < 32; ++i) v[i] = 0.f;
+        // (from the small products to the leading ones)
+#pragma unroll 1
+        for (int z = TM_COLS / LS_BN - 1; z >= 0; --z) {
+            if (!((used >> z) & 1)) continue;
+            tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + z * LS_BN + c0, acc);
+            tmem_ld_wait();
+            tmem_ld_fence(acc);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] += __uint_as_float(acc[i]);
+        }
     }
 
     if (MODE & LS_LN) {
@@ -251,7 +310,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
 #pragma unroll
                 for (int i = 0; i < 8; ++i) v[g * 8 + i] = to_bf16(f[i] + v[g * 8 + i]);
                 if (live && a.out)
-                    *reinterpret_cast<uint4*>(a.out + row * a.n_out + col0 + c0 + g * 8) =
+                    *reinterpret_cast<uint4*>((__nv_bfloat16*)a.out + row * a.n_out + col0 + c0 + g * 8) =
                         Vec<__nv_bfloat16>::pack(v + g * 8);
             }
         }
@@ -273,11 +332,16 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
         __syncwarp();
         if (ctas > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     } else if (parts == 1) {
-        if (live)
+        // (LS_F32: the last column tile may be half a tile)
+        if (live && (!(MODE & LS_F32) || col0 + c0 < a.n_out))
 #pragma unroll
-            for (int g = 0; g < 4; ++g)
-                *reinterpret_cast<uint4*>(a.out + row * a.n_out + col0 + c0 + g * 8) =
-                    ls_finish<MODE>(v + g * 8, params + c0 + g * 8, res[g]);
+            for (int g = 0; g < 4; ++g) {
+                if (MODE & LS_F32)
+                    ls_store_f32<MODE>(a, row, col0 + c0 + g * 8, v + g * 8, params + c0 + g * 8);
+                else
+                    *reinterpret_cast<uint4*>((__nv_bfloat16*)a.out + row * a.n_out + col0 + c0 + g * 8) =
+                        ls_finish<MODE>(v + g * 8, params + c0 + g * 8, res[g]);
+            }
     } else {
         // partial sums over the ring (every product has completed); then this CTA's rows
         if (warp >= 2) {
@@ -291,9 +355,10 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
         for (int e = tid; e < rows * (LS_BN / 8); e += LS_THREADS) {
             const int rr = first + e / (LS_BN / 8), c = e % (LS_BN / 8) * 8;
             const int64_t orow = (int64_t)row0 + rr;
-            if (orow >= a.n) continue;
+            if (orow >= a.n || ((MODE & LS_F32) && col0 + c >= a.n_out)) continue;
             uint4 r4 = make_uint4(0, 0, 0, 0);
-            if (MODE & LS_RESIDUAL) r4 = *reinterpret_cast<const uint4*>(a.residual + orow * a.n_out + col0 + c);
+            if ((MODE & LS_RESIDUAL) && !(MODE & LS_F32))
+                r4 = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)a.residual + orow * a.n_out + col0 + c);
             const uint32_t at = sbase + (rr * LS_PITCH + c) * 4;
             float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             for (int z = 0; z < parts; ++z) {
@@ -301,7 +366,11 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
                 t[0] += m.x; t[1] += m.y; t[2] += m.z; t[3] += m.w;
                 t[4] += w.x; t[5] += w.y; t[6] += w.z; t[7] += w.w;
             }
-            *reinterpret_cast<uint4*>(a.out + orow * a.n_out + col0 + c) = ls_finish<MODE>(t, params + c, r4);
+            if (MODE & LS_F32)
+                ls_store_f32<MODE>(a, orow, col0 + c, t, params + c);
+            else
+                *reinterpret_cast<uint4*>((__nv_bfloat16*)a.out + orow * a.n_out + col0 + c) =
+                    ls_finish<MODE>(t, params + c, r4);
         }
         cluster_sync();          // a peer's partial sums outlive their readers
     }
@@ -309,7 +378,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
     __syncthreads();
     if (warp == 1) {
         fence_after_sync();
-        tmem_dealloc(tmem_base, LS_BN);
+        tmem_dealloc(tmem_base, TM_COLS);
     }
     if (lane == 0 && (!ok || (tid == 0 && *abort))) atomicOr(a.status, PTV3_STATUS_WAIT_LIMIT);
 }
@@ -326,7 +395,7 @@ static int launch_ls(const void* x, const void* w, LinearSmallArgs a, int parts,
     if (rc) return rc;
     auto kern = linear_small_kernel<MODE>;
     if (allow_smem(kern) != cudaSuccess) return check_launch("short Linear: shared memory attribute");
-    const dim3 grid(a.n_out / LS_BN, (unsigned)((a.n + LS_BM - 1) / LS_BM), parts);
+    const dim3 grid((a.n_out + LS_BN - 1) / LS_BN, (unsigned)((a.n + LS_BM - 1) / LS_BM), parts);
     const dim3 cluster = (MODE & LS_LN) ? dim3(grid.x, 1, 1) : dim3(1, 1, parts);
     launch_dependent_cluster(kern, grid, dim3(LS_THREADS), ls_smem(a.stages), stream, cluster, mx, mw, a);
     count_launches(1);
@@ -370,9 +439,9 @@ int launch_linear_small(const void* x, const void* w, const void* bias, const vo
                         int n_out, int gelu, uint32_t* status, cudaStream_t stream)
 {
     LinearSmallArgs a{};
-    a.bias = (const __nv_bfloat16*)bias;
-    a.residual = (const __nv_bfloat16*)residual;
-    a.out = (__nv_bfloat16*)out;
+    a.bias = bias;
+    a.residual = residual;
+    a.out = out;
     a.n = n;
     a.k = k;
     a.n_out = n_out;
@@ -391,9 +460,9 @@ int launch_linear_ln_small(const void* x, const void* w, const void* bias, const
                            void* norm_out, int64_t n, int c, uint32_t* status, cudaStream_t stream)
 {
     LinearSmallArgs a{};
-    a.bias = (const __nv_bfloat16*)bias;
-    a.residual = (const __nv_bfloat16*)residual;
-    a.out = (__nv_bfloat16*)sum_out;
+    a.bias = bias;
+    a.residual = residual;
+    a.out = sum_out;
     a.ln1_w = (const __nv_bfloat16*)ln1_w;
     a.ln1_b = (const __nv_bfloat16*)ln1_b;
     a.ln2_w = (const __nv_bfloat16*)ln2_w;
@@ -405,6 +474,27 @@ int launch_linear_ln_small(const void* x, const void* w, const void* bias, const
     a.k = a.n_out = c;
     a.status = status;
     return launch_ls<LS_LN>(x, w, a, 1, stream);
+}
+
+int launch_linear_split(const void* xs, const void* ws, const float* bias, const float* residual, float* out,
+                        void* split_out, int64_t n, int k, int n_out, int gelu, uint32_t* status, cudaStream_t stream)
+{
+    LinearSmallArgs a{};
+    a.bias = bias;
+    a.residual = residual;
+    a.out = out;
+    a.split_out = (__nv_bfloat16*)split_out;
+    a.n = n;
+    a.k = 6 * k;
+    a.n_out = n_out;
+    a.status = status;
+    const int parts = ls_parts((n + LS_BM - 1) / LS_BM * ((n_out + LS_BN - 1) / LS_BN), a.k);
+    switch ((gelu ? LS_GELU : 0) | (residual ? LS_RESIDUAL : 0)) {
+    case LS_PLAIN: return launch_ls<LS_F32>(xs, ws, a, parts, stream);
+    case LS_GELU: return launch_ls<LS_F32 | LS_GELU>(xs, ws, a, parts, stream);
+    case LS_RESIDUAL: return launch_ls<LS_F32 | LS_RESIDUAL>(xs, ws, a, parts, stream);
+    default: return launch_ls<LS_F32 | LS_GELU | LS_RESIDUAL>(xs, ws, a, parts, stream);
+    }
 }
 
 }  // namespace ptv3

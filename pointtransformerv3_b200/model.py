@@ -340,16 +340,18 @@ class Block(PointModule):
         a.attention_algo, a.scale = attn.algo, attn.scale
         return a
 
-    def _native_static_ok(self, dt):
-        """Shape conditions of the single-call path that do not depend on the input."""
-        key = ("_ptv3_native_ok", dt)
+    def _native_static_ok(self, dt, f32=False):
+        """Shape conditions of the single-call path that do not depend on the input (``f32``: of the fp32
+        block on split weights, which only the one-call backbone uses)."""
+        key = ("_ptv3_native_ok", dt, f32)
         ok = self.__dict__.get(key)
         if ok is None:
             attn, mlp, conv = self.attn, self.mlp[0], self.cpe[0]
             ok = (conv.kernel_size == 3 and conv.in_channels == self.channels
                   and conv.out_channels == self.channels and mlp.fc2.out_features == self.channels
                   and mlp.fc1.in_features == self.channels
-                  and ops.block_supported(self.channels, attn.num_heads, mlp.fc1.out_features, dt))
+                  and (ops.block_f32_supported(self.channels, attn.num_heads, mlp.fc1.out_features) if f32 else
+                       ops.block_supported(self.channels, attn.num_heads, mlp.fc1.out_features, dt)))
             self.__dict__[key] = ok
         return ok
 
@@ -750,14 +752,15 @@ class PointTransformerV3(PointModule):
         return _PLAN_STREAMS[key]
 
     def _native(self, point):
-        """The one-call form of this forward, where it covers the network and the input: bf16 on the GPU,
+        """The one-call form of this forward, where it covers the network and the input: bf16 or fp32 on the GPU,
         standard modules, nobody hooked onto a single module, no per-operator timing."""
         feat = point.feat
-        if (feat.dtype != torch.bfloat16 or not feat.is_cuda or feat.dim() != 2 or feat.shape[0] == 0
-                or ops.TIMERS is not None or feat.requires_grad):
+        if (feat.dtype not in (torch.bfloat16, torch.float32) or not feat.is_cuda or feat.dim() != 2
+                or feat.shape[0] == 0 or ops.TIMERS is not None or feat.requires_grad
+                or (feat.dtype == torch.float32 and feat.shape[0] > 65535 * 128)):
             return None
         native = backbone.of(self)
-        if native is None or feat.shape[1] != native.width_in or native.observed():
+        if native is None or feat.dtype != native.dtype or feat.shape[1] != native.width_in or native.observed():
             return None
         return native
 

@@ -633,6 +633,55 @@ def linear_ln(x, weight, bias, residual, ln1, ln2, status=None, want_sum=True):
     return s, y
 
 
+def split_f32(x, weight=False):
+    """(..., k) fp32 -> (..., 6k) bf16: the operand of a product of floats on the bf16 tensor cores
+    (see ptv3_split_f32); ``weight`` for its second operand."""
+    _lib.require_cuda(x)
+    x = x.detach().contiguous()
+    k = x.shape[-1]
+    out = torch.empty(x.shape[:-1] + (6 * k,), dtype=torch.bfloat16, device=x.device)
+    _lib.check(_lib.load().ptv3_split_f32(_lib.ptr(x), x.numel() // k, k, int(weight), _lib.ptr(out), _lib.stream()),
+               "ptv3_split_f32")
+    return out
+
+
+def linear_split(x_split, w_split, bias=None, residual=None, gelu=False, status=None):
+    """fp32 [residual +] act(x W^T + b) from split operands."""
+    _lib.require_cuda(x_split, w_split, bias, residual)
+    n, k6 = x_split.shape
+    out = torch.empty((n, w_split.shape[0]), dtype=torch.float32, device=x_split.device)
+    own = status is None
+    if own:
+        status = new_status(out.device)
+    _lib.check(_lib.load().ptv3_linear_split_fwd(_lib.ptr(x_split), _lib.ptr(w_split), _lib.ptr(bias), _lib.ptr(residual),
+                                                 _lib.ptr(out), n, k6 // 6, out.shape[1], int(bool(gelu)),
+                                                 _lib.ptr(status), _lib.stream()), "ptv3_linear_split_fwd")
+    if own:
+        _lib.raise_on_status(status, "ptv3_linear_split_fwd")
+    return out
+
+
+def subm_conv_split(f_split, nbr, w_split, bias=None, row_order=None, status=None):
+    """fp32 submanifold convolution from split operands (weight (C_out, kvol or k, k, k, 6 C_in))."""
+    _lib.require_cuda(f_split, nbr, w_split, bias)
+    n, c6 = f_split.shape
+    out = torch.empty((n, w_split.shape[0]), dtype=torch.float32, device=f_split.device)
+    own = status is None
+    if own:
+        status = new_status(out.device)
+    _lib.check(_lib.load().ptv3_subm_conv_split_fwd(_lib.ptr(f_split), _lib.ptr(nbr), _lib.ptr(w_split), _lib.ptr(bias),
+                                                    _lib.ptr(out), _lib.ptr(row_order), n, c6 // 6, out.shape[1],
+                                                    nbr.shape[0], _lib.ptr(status), _lib.stream()),
+               "ptv3_subm_conv_split_fwd")
+    if own:
+        _lib.raise_on_status(status, "ptv3_subm_conv_split_fwd")
+    return out
+
+
+def block_f32_supported(channels, heads, hidden):
+    return bool(_lib.load().ptv3_block_f32_supported(int(channels), int(heads), int(hidden)))
+
+
 def block_supported(channels, heads, hidden, dtype):
     return dtype in _lib.DTYPE_IDS and bool(
         _lib.load().ptv3_block_supported(int(channels), int(heads), int(hidden), _lib.DTYPE_IDS[dtype]))

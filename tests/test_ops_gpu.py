@@ -280,6 +280,28 @@ def test_attention_with_and_without_reference_value(n, gain):
     assert rel_l2(b, a) < (5e-3 if gain < 10 else 1e-2)
 
 
+@pytest.mark.parametrize("n", [1, 127, 129, 257, 1500])
+@pytest.mark.parametrize("gain", [0.3, 2.0, 8.0])
+def test_attention_fp32_two_queries_per_thread(n, gain):
+    """The fp32 kernel (algo 0) against the one-query form (algo 1): bounded and unbounded chunks of
+    keys, both in one sequence (the second half has large keys), ragged ends."""
+    C, H, K = 32, 2, 1024
+    g = torch.Generator().manual_seed(n)
+    qkv = torch.randn(n, 3 * C, generator=g)
+    qkv[n // 2:, C:2 * C] *= gain * gain
+    qkv[:, :C] *= gain
+    qkv = qkv.cuda()
+    order = torch.randperm(n, generator=g).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    a = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25, algo=1)
+    b = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25)
+    assert bool(torch.isfinite(b).all()) and rel_l2(b, a) < 1e-5
+    if n <= K:         # one patch: plain attention over all rows, here in float64
+        q, k, v = (t.reshape(n, H, C // H).transpose(0, 1) for t in qkv.double().split(C, dim=1))
+        ref = (torch.softmax(q @ k.transpose(1, 2) * 0.25, 2) @ v).transpose(0, 1).reshape(n, C)
+        assert rel_l2(b.double(), ref) < 1.5 * rel_l2(a.double(), ref) + 1e-7
+
+
 @pytest.mark.parametrize("algo,dtype", [(0, torch.bfloat16), (1, torch.bfloat16), (1, torch.float32),
                                         (4, torch.bfloat16)])
 def test_attention_reports_a_patch_longer_than_max_seqlen(algo, dtype):
@@ -717,3 +739,42 @@ def test_short_linear_layernorm(n, c, with_ln1):
     ref_y = torch.nn.functional.layer_norm(ref.bfloat16().float(), (c,), ln2.weight.float().cpu(), ln2.bias.float().cpu(),
                                            ln2.eps)
     assert rel_l2(s, ref) < 5e-3 and rel_l2(y, ref_y) < 6e-3
+
+
+@pytest.mark.parametrize("n,k,n_out", [(1, 32, 96), (129, 32, 32), (300, 64, 192), (1000, 512, 512), (27, 2048, 512),
+                                       (5000, 128, 384)])
+@pytest.mark.parametrize("gelu,residual", [(False, False), (True, False), (False, True)])
+def test_linear_on_split_floats(n, k, n_out, gelu, residual):
+    """fp32 Linear from bf16 thirds: as close to float64 as torch's own fp32 product, on operands of very
+    different sizes."""
+    g = torch.Generator().manual_seed(n + k)
+    x = torch.randn(n, k, generator=g) * 10.0 ** torch.randint(-3, 3, (n, 1), generator=g)
+    w, b = torch.randn(n_out, k, generator=g) / k ** 0.5, torch.randn(n_out, generator=g)
+    r = torch.randn(n, n_out, generator=g)
+    x, w, b, r = x.cuda(), w.cuda(), b.cuda(), r.cuda()
+    got = ops.linear_split(ops.split_f32(x), ops.split_f32(w, weight=True), b, r if residual else None, gelu)
+
+    def run(*t):
+        y = torch.nn.functional.linear(*t[:3])
+        y = torch.nn.functional.gelu(y) if gelu else y
+        return y + t[3] if residual else y
+    ref, plain = run(x.double(), w.double(), b.double(), r.double()), run(x, w, b, r)
+    assert rel_l2(got.double(), ref) < 1.5 * rel_l2(plain.double(), ref) + 1e-7
+
+
+@pytest.mark.parametrize("n,cin,cout", [(1, 32, 32), (700, 32, 32), (900, 64, 64), (500, 64, 128), (400, 256, 256),
+                                        (60, 512, 512), (40000, 64, 64)])
+def test_subm_conv_on_split_floats(n, cin, cout):
+    """fp32 convolution from bf16 thirds against the CUDA-core kernel and float64."""
+    g = torch.Generator().manual_seed(n + cin)
+    cells = torch.randperm(2 * n + 20, generator=g)[:n]
+    ind = torch.stack([torch.zeros_like(cells), cells // 40, cells % 40 // 4, cells % 4], 1).int().cuda()
+    nbr = ops.kmap_build(ind, 3)
+    feat = torch.randn(n, cin, generator=g).cuda()
+    w = (torch.randn(cout, 3, 3, 3, cin, generator=g) / (9 * cin) ** 0.5).cuda()
+    b = torch.randn(cout, generator=g).cuda()
+    got = ops.subm_conv_split(ops.split_f32(feat), nbr, ops.split_f32(w, weight=True), b)
+    plain = ops.subm_conv(feat, nbr, w, b)
+    rows = torch.cat([feat.double(), feat.new_zeros(1, cin).double()])[nbr.long()]          # -1 -> the zero row
+    ref = torch.einsum("onc,doc->nd", rows, w.double().reshape(cout, 27, cin)) + b.double()
+    assert rel_l2(got.double(), ref) < 1.5 * rel_l2(plain.double(), ref) + 1e-7
