@@ -1,8 +1,9 @@
 """One-call form of the backbone's forward (ptv3_backbone_fwd): the argument blocks of a network
 whose modules all have their standard form, kept between passes and rebuilt when a parameter, a
 buffer or a setting changed.  fp32 networks keep their weights split for the tensor cores there
-(three times their size, see ptv3_split_f32)."""
+(1.5 times their size, see ptv3_split_f32)."""
 import ctypes
+import itertools
 import operator
 import weakref
 
@@ -14,6 +15,7 @@ from . import sparse as spconv
 from .sparse import SparseConvTensor
 
 _GLOBAL_HOOKS = nn.modules.module
+_VERSION = operator.attrgetter("_version")
 
 
 def _exact_gelu(m):
@@ -67,6 +69,7 @@ class NativeBackbone:
         self.width_out = self.blocks[-1].channels
         _require(self.stage_blocks[-1] >= 1)
         self.settings = self._settings()
+        self.owners, self.names = [d for d, _ in self.refs], [k for _, k in self.refs]
         self.tensors = [d[k] for d, k in self.refs]
         self.ptrs = [t.data_ptr() for t in self.tensors]
         self.version = [t._version for t in self.versions]
@@ -169,13 +172,11 @@ class NativeBackbone:
 
     def current(self):
         """Whether every module, parameter, buffer and setting is as it was when the blocks were made."""
-        children = [c for d in self.parents for c in d.values()]
-        if len(children) != len(self.children) or any(map(operator.is_not, children, self.children)):
-            return False
-        now = [d.get(k) for d, k in self.refs]
-        return (not any(map(operator.is_not, now, self.tensors))
-                and [t.data_ptr() for t in now] == self.ptrs
-                and [t._version for t in self.versions] == self.version
+        children = list(itertools.chain.from_iterable(map(dict.values, self.parents)))
+        return (len(children) == len(self.children) and all(map(operator.is_, children, self.children))
+                and all(map(operator.is_, map(dict.get, self.owners, self.names), self.tensors))
+                and list(map(torch.Tensor.data_ptr, self.tensors)) == self.ptrs
+                and list(map(_VERSION, self.versions)) == self.version
                 and self._settings() == self.settings)
 
     def observed(self):

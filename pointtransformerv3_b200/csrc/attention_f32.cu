@@ -6,13 +6,17 @@
 // owns two queries, so a read serves twice the arithmetic, products run on pairs of floats, and the scores
 // are computed once: where |q| max|k| bounds them (AX_BOUND, per chunk of keys and CTA) the exponentials
 // need no reference value; other chunks take the maximum first as before.
+//
+// The four warps of a CTA share its 64 queries and take the keys in turn; their sums meet at the end.
+// With the queries spread over all threads instead, a patch of a coarse level was a serial chain of up to
+// 1 024 keys on a few CTAs (100 us at 700 points x 256 channels as at 40 000 x 64).
 #include "attention_mma.cuh"
 #include "common.cuh"
 #include "mma_util.cuh"
 
 namespace ptv3 {
 
-constexpr int AX_THREADS = 128, AX_Q = 2, AX_QT = AX_THREADS * AX_Q;
+constexpr int AX_THREADS = 128, AX_WARPS = AX_THREADS / 32, AX_Q = 2, AX_QT = 32 * AX_Q;
 constexpr int AX_KC = 128;                   // keys per staged chunk
 constexpr int AX_D = 16, AX_P = AX_D / 2;
 // largest |score| taken without a reference value: the exponent's rounding (16 log2 e 2^-24) stays within
@@ -49,15 +53,17 @@ __device__ __forceinline__ void ax_add(AxRow& r, float p, const ulonglong2* v)
     r.l += p;
 }
 
-__global__ void __launch_bounds__(AX_THREADS) attn_f32_d16_kernel(
+__global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(
     const float* __restrict__ qkv, const int64_t* __restrict__ order, const int64_t* __restrict__ pad,
     const int64_t* __restrict__ unpad, const int32_t* __restrict__ cu_seqlens, float* __restrict__ out, int C,
     float scale, uint32_t* __restrict__ status)
 {
     __shared__ __align__(16) float Ks[AX_KC][AX_D], Vs[AX_KC][AX_D];
-    __shared__ float warp_norm[AX_THREADS / 32];
+    __shared__ float part[AX_WARPS][AX_QT][AX_D + 3];      // sums, l, m; padded against bank conflicts
+    __shared__ float warp_norm[AX_WARPS];
     const int n_heads = C / AX_D;
-    const int seq = blockIdx.y, h = blockIdx.x % n_heads, tile = blockIdx.x / n_heads, tid = threadIdx.x;
+    const int seq = blockIdx.y, h = blockIdx.x % n_heads, tile = blockIdx.x / n_heads, tid = threadIdx.x, warp = tid >> 5,
+              lane = tid & 31;
     const int64_t start = cu_seqlens[seq];
     const int L = (int)(cu_seqlens[seq + 1] - start);
     // a sequence longer than the caller's max_seqlen would leave rows of the output unwritten: reported
@@ -69,7 +75,7 @@ __global__ void __launch_bounds__(AX_THREADS) attn_f32_d16_kernel(
     int64_t dst[AX_Q];
 #pragma unroll
     for (int i = 0; i < AX_Q; ++i) {
-        const int qi = tile * AX_QT + i * AX_THREADS + tid;
+        const int qi = tile * AX_QT + i * 32 + lane;
         AxRow& r = row[i];
         dst[i] = -1;
         r.m = 0.f;
@@ -90,7 +96,7 @@ __global__ void __launch_bounds__(AX_THREADS) attn_f32_d16_kernel(
             }
         }
     }
-    bool first = true;
+    bool first = true;       // no key taken by this warp yet
     for (int c0 = 0; c0 < L; c0 += AX_KC) {
         const int nk = min(AX_KC, L - c0);
         __syncthreads();
@@ -109,28 +115,29 @@ __global__ void __launch_bounds__(AX_THREADS) attn_f32_d16_kernel(
         }
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) kn = max_nan(kn, __shfl_xor_sync(0xffffffffu, kn, d));
-        if ((tid & 31) == 0) warp_norm[tid >> 5] = kn;
+        if (lane == 0) warp_norm[warp] = kn;
         __syncthreads();
 #pragma unroll
-        for (int w = 0; w < AX_THREADS / 32; ++w) kn = max_nan(kn, warp_norm[w]);
+        for (int w = 0; w < AX_WARPS; ++w) kn = max_nan(kn, warp_norm[w]);
         // (a NaN fails the test); a reference value raised by an earlier chunk stays in force
         const bool bounded = row[0].norm * kn <= AX_BOUND * AX_BOUND && row[1].norm * kn <= AX_BOUND * AX_BOUND &&
                              row[0].m == 0.f && row[1].m == 0.f;
         if (__syncthreads_and(bounded)) {
 #pragma unroll 4
-            for (int j = 0; j < nk; ++j) {
+            for (int j = warp; j < nk; j += AX_WARPS) {
                 const ulonglong2* k = reinterpret_cast<const ulonglong2*>(Ks[j]);
                 const ulonglong2* v = reinterpret_cast<const ulonglong2*>(Vs[j]);
                 const float p0 = fast_exp2(ax_dot(row[0].q, k) * AX_LOG2E), p1 = fast_exp2(ax_dot(row[1].q, k) * AX_LOG2E);
                 ax_add(row[0], p0, v);
                 ax_add(row[1], p1, v);
             }
-        } else {
+        } else if (warp < nk) {
 #pragma unroll
             for (int i = 0; i < AX_Q; ++i) {
                 AxRow& r = row[i];
                 float cm = -INFINITY;
-                for (int j = 0; j < nk; ++j) cm = fmaxf(cm, ax_dot(r.q, reinterpret_cast<const ulonglong2*>(Ks[j])));
+                for (int j = warp; j < nk; j += AX_WARPS)
+                    cm = fmaxf(cm, ax_dot(r.q, reinterpret_cast<const ulonglong2*>(Ks[j])));
                 // the first chunk sets the reference; after chunks without one (reference 0) it only rises
                 const float mn = first ? cm : fmaxf(r.m, cm);
                 const float corr = first ? 0.f : __expf(r.m - mn);
@@ -138,26 +145,48 @@ __global__ void __launch_bounds__(AX_THREADS) attn_f32_d16_kernel(
 #pragma unroll
                 for (int d = 0; d < AX_P; ++d) r.acc[d] = mul2(r.acc[d], pack2(corr, corr));
                 r.m = mn;
-                for (int j = 0; j < nk; ++j)
+                for (int j = warp; j < nk; j += AX_WARPS)
                     ax_add(r, __expf(ax_dot(r.q, reinterpret_cast<const ulonglong2*>(Ks[j])) - mn),
                            reinterpret_cast<const ulonglong2*>(Vs[j]));
             }
         }
-        first = false;
+        first = first && warp >= nk;
     }
+    // ---- the warps' sums meet; warps 0 and 1 finish one query of a lane each ----------
 #pragma unroll
     for (int i = 0; i < AX_Q; ++i) {
-        if (dst[i] < 0) continue;
-        const float inv = 1.f / row[i].l;
-        float4* op = reinterpret_cast<float4*>(out + dst[i] * C + h * AX_D);
+        const int qi = i * 32 + lane;
 #pragma unroll
-        for (int d = 0; d < 4; ++d) {
-            float4 v;
-            unpack2(row[i].acc[2 * d], v.x, v.y);
-            unpack2(row[i].acc[2 * d + 1], v.z, v.w);
-            op[d] = make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
+        for (int d = 0; d < AX_P; ++d) {
+            float lo, hi;
+            unpack2(row[i].acc[d], lo, hi);
+            part[warp][qi][2 * d] = lo;
+            part[warp][qi][2 * d + 1] = hi;
         }
+        part[warp][qi][AX_D] = row[i].l;
+        part[warp][qi][AX_D + 1] = row[i].m;
     }
+    __syncthreads();
+    const int64_t mine = warp == 0 ? dst[0] : dst[1];
+    if (warp >= AX_Q || mine < 0) return;
+    const int qi = warp * 32 + lane;
+    float m = -INFINITY;
+    for (int w = 0; w < AX_WARPS; ++w)
+        if (part[w][qi][AX_D] != 0.f) m = fmaxf(m, part[w][qi][AX_D + 1]);      // (a NaN sum stays in)
+    float y[AX_D], l = 0.f;
+#pragma unroll
+    for (int d = 0; d < AX_D; ++d) y[d] = 0.f;
+    for (int w = 0; w < AX_WARPS; ++w) {
+        if (part[w][qi][AX_D] == 0.f) continue;
+        const float c = __expf(part[w][qi][AX_D + 1] - m);
+        l = fmaf(c, part[w][qi][AX_D], l);
+#pragma unroll
+        for (int d = 0; d < AX_D; ++d) y[d] = fmaf(c, part[w][qi][d], y[d]);
+    }
+    const float inv = 1.f / l;
+    float4* op = reinterpret_cast<float4*>(out + mine * C + h * AX_D);
+#pragma unroll
+    for (int d = 0; d < 4; ++d) op[d] = make_float4(y[4 * d] * inv, y[4 * d + 1] * inv, y[4 * d + 2] * inv, y[4 * d + 3] * inv);
 }
 
 int launch_attn_f32(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad, const int32_t* cu,

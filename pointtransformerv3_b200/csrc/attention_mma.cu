@@ -327,12 +327,16 @@ int launch_attn_mma(const void* qkv, const int64_t* order, const int64_t* pad, c
     auto kern = packed_exp ? attn_mma_d16_kernel<true> : attn_mma_d16_kernel<false>;
     if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_attention_fwd: shared memory attribute");
-    // slice the queries of a sequence over several CTAs when there are few (sequence, head) pairs
-    int qsplit = 1;
-    const int pairs = n_seq * H;
+    // Queries of a sequence are sliced over CTAs, each of which gathers K and V again.  A launch wants two
+    // waves of three CTAs per SM, or one that is nearly full: fewer CTAs land unevenly on the SMs (a dependent
+    // launch fills the first ones that the kernel before it leaves), more gather more often.  us in
+    // 1 / 2 / 4 / 8 slices: 400 000 x 64 (1 564 pairs) 449 / 451 / 457 / 507, 105 000 x 64 (412) 133 / 133 / 136 / 144,
+    // 28 000 x 128 (224) 127 / 91 / 83 / 85, 2 200 x 512 (96) 70 / 56 / 42 / 44, 6 000 x 64 (24) 49 / 27 / 24 / 20.
     const int tiles = (max_seqlen + 15) / 16;
-    // three CTAs fit on an SM; aim at several waves so that the last one costs little
-    while (pairs * qsplit < 4 * 3 * 148 && qsplit * 2 * AM_WARPS <= tiles) qsplit *= 2;
+    const int64_t pairs = (int64_t)n_seq * H;
+    int qsplit = 1;
+    while (qsplit < 8 && qsplit * AM_WARPS < tiles && pairs * qsplit < 800 && !(pairs * qsplit >= 370 && pairs * qsplit <= 444))
+        qsplit *= 2;
     const dim3 grid(H * qsplit, n_seq);
     launch_dependent(kern, grid, dim3(AM_THREADS), smem, stream, (const __nv_bfloat16*)qkv, order, pad, unpad, cu,
                      (__nv_bfloat16*)out, C, scale, lpad, status);

@@ -79,7 +79,7 @@ static size_t carve_block(const ptv3_block_args* a, void* base, BlockBuffers* b)
 // Linear, fc1 -> fc2); the others are split by a kernel of their own.
 struct BlockBuffersF32 {
     float *y, *f1, *a, *qkv, *att, *f2;
-    void *s, *sh;           // split rows: n x 6C, n x 6 hidden
+    void *s, *sh;           // split rows of width C (at most 6C bf16) and of the hidden width
 };
 
 static size_t carve_block_f32(const ptv3_block_args* a, void* base, BlockBuffersF32* b)

@@ -30,7 +30,7 @@ int launch_conv_pairs(const void* feat, const int32_t* pair_in, const int32_t* p
                       int c_out, int kernel_volume, cudaStream_t stream);
 
 // fp32 convolution on split operands (split_f32.cuh), c_in a multiple of 32, c_out 32 or a multiple of 64;
-// the result goes to `out`, or as split rows (n x 6 c_out) to `split_out`
+// the result goes to `out`, or as split rows to `split_out`
 int launch_conv_split(const void* feat, const int32_t* nbr, const void* weight, const float* bias, float* out,
                       void* split_out, const int64_t* row_order, int64_t n, int c_in, int c_out, int kvol,
                       uint32_t* status, cudaStream_t stream);

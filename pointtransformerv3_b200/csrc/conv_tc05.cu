@@ -58,7 +58,7 @@ struct ConvTcArgs {
     const int32_t* nbr;            // kvol x n, columns in tile order
     const void* bias;              // cout or NULL, of the output's type
     void* out;                     // bf16 or fp32
-    __nv_bfloat16* split_out;      // fp32: the result as split rows (n x 6 cout) instead, or NULL
+    __nv_bfloat16* split_out;      // fp32: the result as split rows instead, or NULL
     const int64_t* row_order;      // voxel of every tile position, or NULL
     int64_t n;
     int cin, cout, kvol;
@@ -69,7 +69,7 @@ struct ConvTcArgs {
 __device__ __forceinline__ void ct_store_f32(const ConvTcArgs& a, int64_t row, int col, const float* y)
 {
     if (a.split_out) {
-        split_store8(a.split_out + row * 6 * a.cout + col, a.cout, y);
+        split_store8(a.split_out + row * split_stored(a.cout) * a.cout, col, a.cout, y);
         return;
     }
     float4* o = reinterpret_cast<float4*>((float*)a.out + row * a.cout + col);
@@ -196,6 +196,7 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
     const uint32_t tmem_base = *tmem_slot;
     const int n_act = act[0];
     const int kchunks = a.cin / KC;
+    const int stored = F32 ? a.cin / 6 * split_stored(a.cin / 6) : a.cin;      // columns of a feature row
     // this CTA's share of the tile's stages (all of them without a cluster)
     int first = 0, nit = n_act * kchunks;
     if (SPLIT) {
@@ -219,7 +220,9 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
             }
             __syncwarp();
             const int o = act[1 + (first + it) / kchunks];
-            const int kc = ((first + it) % kchunks) * KC;
+            const int chunk = (first + it) % kchunks;
+            const int kc = F32 ? split_column_a(chunk, a.cin / 6) : chunk * KC;
+            const int kw = F32 ? split_column_b(chunk, a.cin / 6) : chunk * KC;
             const uint32_t sa = sbase + s * STAGE_BYTES;
             const __nv_bfloat16* src0 = a.feat + kc + c * 8;
             const int32_t* nb = nbr_s + o * CT_TM + rr;
@@ -232,7 +235,7 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
                 for (int j = 0; j < 8; ++j) {
                     const int r = rr + (j0 + j) * RPP;
                     const int pc = NCH == 8 ? (c ^ (r & 7)) : (c ^ ((r >> 1) & 3));
-                    cp_async16_zfill(sa + r * ROWB + pc * 16, src0 + (int64_t)(src[j] < 0 ? 0 : src[j]) * a.cin,
+                    cp_async16_zfill(sa + r * ROWB + pc * 16, src0 + (int64_t)(src[j] < 0 ? 0 : src[j]) * stored,
                                      src[j] >= 0);
                 }
             }
@@ -241,7 +244,7 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
             // which the rows are already on their way)
             if (lane == 0) {
                 mbar_expect_tx(full0 + 8 * s, B_BYTES);
-                tma_load_2d(sa + A_BYTES, &map_w, o * a.cin + kc, col0, full0 + 8 * s);
+                tma_load_2d(sa + A_BYTES, &map_w, o * stored + kw, col0, full0 + 8 * s);
             }
             cp_async_wait<0>();
             fence_proxy_async();
@@ -417,7 +420,7 @@ template <int BN, int KC, int STAGES, int NI, bool SPLIT, bool F32>
 static int launch_conv_tc05_as(const void* weight, const ConvTcArgs& a, cudaStream_t stream, int parts)
 {
     CUtensorMap mw;
-    const uint64_t wcols = (uint64_t)a.kvol * a.cin;
+    const uint64_t wcols = (uint64_t)a.kvol * (F32 ? a.cin / 6 * split_stored(a.cin / 6) : a.cin);
     const int rc = make_tensor_map_bf16(&mw, weight, (uint64_t)a.cout, wcols, wcols * 2, BN, KC);
     if (rc) return rc;
     constexpr size_t smem = conv_tc05_smem<BN, KC, STAGES>();
@@ -538,7 +541,7 @@ int launch_conv_tc05(const void* feat, const int32_t* nbr, const void* weight, c
     return launch_conv_tc05_best(weight, a, false, stream);
 }
 
-// fp32 on split operands (see split_f32.cuh): feat n x 6 c_in, weight c_out x kvol x 6 c_in bf16
+// fp32 on split operands (see split_f32.cuh)
 int launch_conv_split(const void* feat, const int32_t* nbr, const void* weight, const float* bias, float* out,
                       void* split_out, const int64_t* row_order, int64_t n, int c_in, int c_out, int kvol,
                       uint32_t* status, cudaStream_t stream)

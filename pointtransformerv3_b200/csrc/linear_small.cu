@@ -31,7 +31,7 @@ constexpr int LS_PLAIN = 0, LS_GELU = 1, LS_RESIDUAL = 2, LS_LN = 4, LS_F32 = 8;
 struct LinearSmallArgs {
     const void *bias, *residual;                       // bf16; fp32 with LS_F32
     void* out;                                         // LN: the sum, or NULL
-    __nv_bfloat16* split_out;                          // LS_F32: the result as split rows (n x 6 n_out) instead
+    __nv_bfloat16* split_out;                          // LS_F32: the result as split rows instead
     const __nv_bfloat16 *ln1_w, *ln1_b, *ln2_w, *ln2_b;
     float eps1, eps2;
     __nv_bfloat16* norm_out;
@@ -80,7 +80,7 @@ __device__ __forceinline__ void ls_store_f32(const LinearSmallArgs& a, int64_t r
         y[4] += r1.x; y[5] += r1.y; y[6] += r1.z; y[7] += r1.w;
     }
     if (a.split_out) {
-        split_store8(a.split_out + row * 6 * a.n_out + col, a.n_out, y);
+        split_store8(a.split_out + row * split_stored(a.n_out) * a.n_out, col, a.n_out, y);
         return;
     }
     float4* o = reinterpret_cast<float4*>((float*)a.out + row * a.n_out + col);
@@ -135,6 +135,9 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
     const int parts = (MODE & LS_LN) ? 1 : (int)gridDim.z;
     const int nk = a.k / LS_BK / parts, k0 = nk * (int)blockIdx.z * LS_BK;
 
+    auto column_x = [&](int kc) { return (MODE & LS_F32) ? split_column_a(k0 / LS_BK + kc, a.k / 6) : k0 + kc * LS_BK; };
+    auto column_w = [&](int kc) { return (MODE & LS_F32) ? split_column_b(k0 / LS_BK + kc, a.k / 6) : k0 + kc * LS_BK; };
+
     if (tid == 0) {
         for (int s = 0; s < stages; ++s) {
             mbar_init(full0 + 8 * s, 1);
@@ -147,7 +150,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
         // the weights are not written by the launch before this one: fetched ahead of the wait below
         for (int kc = 0; kc < nk && kc < stages; ++kc) {
             mbar_expect_tx(full0 + 8 * kc, LS_STAGE);
-            tma_load_2d(sbase + kc * LS_STAGE + LS_A_BYTES, &map_w, k0 + kc * LS_BK, col0, full0 + 8 * kc);
+            tma_load_2d(sbase + kc * LS_STAGE + LS_A_BYTES, &map_w, column_w(kc), col0, full0 + 8 * kc);
         }
     }
     if (warp == 1) {
@@ -195,9 +198,9 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
                 if (kc >= stages) {
                     ok &= mbar_wait(empty0 + 8 * s, ((kc / stages) & 1) ^ 1, abort);
                     mbar_expect_tx(full0 + 8 * s, LS_STAGE);
-                    tma_load_2d(sa + LS_A_BYTES, &map_w, k0 + kc * LS_BK, col0, full0 + 8 * s);
+                    tma_load_2d(sa + LS_A_BYTES, &map_w, column_w(kc), col0, full0 + 8 * s);
                 }
-                tma_load_2d(sa, &map_x, k0 + kc * LS_BK, row0, full0 + 8 * s);
+                tma_load_2d(sa, &map_x, column_x(kc), row0, full0 + 8 * s);
             }
         __syncwarp();
     } else if (warp == 1) {
@@ -389,9 +392,10 @@ static int launch_ls(const void* x, const void* w, LinearSmallArgs a, int parts,
     const int nk = a.k / LS_BK / parts;
     a.stages = nk < LS_MAX_STAGES ? nk : LS_MAX_STAGES;
     CUtensorMap mx, mw;
-    int rc = make_tensor_map_bf16(&mx, x, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.k * 2, LS_BM, LS_BK);
+    const uint64_t cols = (MODE & LS_F32) ? (uint64_t)a.k / 6 * split_stored(a.k / 6) : (uint64_t)a.k;      // stored
+    int rc = make_tensor_map_bf16(&mx, x, (uint64_t)a.n, cols, cols * 2, LS_BM, LS_BK);
     if (rc) return rc;
-    rc = make_tensor_map_bf16(&mw, w, (uint64_t)a.n_out, (uint64_t)a.k, (uint64_t)a.k * 2, LS_BN, LS_BK);
+    rc = make_tensor_map_bf16(&mw, w, (uint64_t)a.n_out, cols, cols * 2, LS_BN, LS_BK);
     if (rc) return rc;
     auto kern = linear_small_kernel<MODE>;
     if (allow_smem(kern) != cudaSuccess) return check_launch("short Linear: shared memory attribute");

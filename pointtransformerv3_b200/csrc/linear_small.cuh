@@ -17,8 +17,8 @@ int launch_linear_ln_small(const void* x, const void* w, const void* bias, const
                            const void* ln1_b, float eps1, void* sum_out, const void* ln2_w, const void* ln2_b, float eps2,
                            void* norm_out, int64_t n, int c, uint32_t* status, cudaStream_t stream);
 
-// fp32 Linear on split operands (split_f32.cuh): xs n x 6k, ws n_out x 6k bf16; k and n_out multiples of 32
-// (6k of 64).  The result goes to `out`, or as split rows (n x 6 n_out) to `split_out`.
+// fp32 Linear on split operands (split_f32.cuh); k and n_out multiples of 32.  The result goes to `out`, or as
+// split rows to `split_out`.
 int launch_linear_split(const void* xs, const void* ws, const float* bias, const float* residual, float* out,
                         void* split_out, int64_t n, int k, int n_out, int gelu, uint32_t* status, cudaStream_t stream);
 

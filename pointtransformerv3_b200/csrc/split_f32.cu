@@ -3,7 +3,7 @@
 
 namespace ptv3 {
 
-// a thread splits eight columns; bandwidth bound: 4 bytes in, 12 out
+// a thread splits eight columns; bandwidth bound: 4 bytes in, 6 out
 template <bool WEIGHT>
 __global__ void __launch_bounds__(256) split_f32_kernel(const float* __restrict__ x, int64_t n8, int k,
                                                         __nv_bfloat16* __restrict__ out)
@@ -17,18 +17,7 @@ __global__ void __launch_bounds__(256) split_f32_kernel(const float* __restrict_
     const int c = (int)(e - row * per) * 8;
     const float4 v0 = reinterpret_cast<const float4*>(x)[2 * e], v1 = reinterpret_cast<const float4*>(x)[2 * e + 1];
     const float y[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
-    __nv_bfloat16* at = out + row * 6 * k + c;
-    if (!WEIGHT) {
-        split_store8(at, k, y);
-    } else {
-        uint4 p[3];
-        __nv_bfloat16* q = reinterpret_cast<__nv_bfloat16*>(p);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) split3(y[i], q[i], q[8 + i], q[16 + i]);
-        const int part[6] = {0, 1, 2, 0, 1, 0};
-#pragma unroll
-        for (int i = 0; i < 6; ++i) *reinterpret_cast<uint4*>(at + (int64_t)i * k) = p[part[i]];
-    }
+    split_store8(out + row * split_stored(k) * k, c, k, y, WEIGHT);
 }
 
 int launch_split_f32(const float* x, int64_t rows, int k, bool weight, void* out, cudaStream_t stream)

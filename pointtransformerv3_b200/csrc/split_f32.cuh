@@ -18,6 +18,23 @@
 
 namespace ptv3 {
 
+// Stored are the three parts where a piece is whole 64-column chunks (the products then read a part as
+// often as they need it), all six pieces otherwise.
+__host__ __device__ constexpr int split_stored(int k) { return k % 64 == 0 ? 3 : 6; }
+// column of chunk `c` (64 columns of the six pieces) in a stored row of A or of B
+__host__ __device__ __forceinline__ int split_column_a(int c, int k)
+{
+    if (k % 64) return c * 64;
+    const int piece = c * 64 / k;
+    return (piece < 3 ? 0 : piece < 5 ? 1 : 2) * k + c * 64 % k;
+}
+__host__ __device__ __forceinline__ int split_column_b(int c, int k)
+{
+    if (k % 64) return c * 64;
+    const int piece = c * 64 / k;
+    return (piece < 3 ? piece : piece < 5 ? piece - 3 : 0) * k + c * 64 % k;
+}
+
 constexpr int SPLIT_MAIN = 3, SPLIT_ACCS = SPLIT_MAIN + 1;
 
 __device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16& b, __nv_bfloat16& c)
@@ -28,19 +45,24 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16&
     c = __float2bfloat16_rn(__fsub_rn(r, __bfloat162float(b)));
 }
 
-// eight values of an A row: `at` points at their column of the first piece, `k` is the width of a piece
-__device__ __forceinline__ void split_store8(__nv_bfloat16* at, int k, const float* y)
+// eight values of an A row: `row` is the stored row, `c` their column, `k` the width of a piece
+__device__ __forceinline__ void split_store8(__nv_bfloat16* row, int c, int k, const float* y, bool weight = false)
 {
     uint4 p[3];
     __nv_bfloat16* q = reinterpret_cast<__nv_bfloat16*>(p);
 #pragma unroll
     for (int i = 0; i < 8; ++i) split3(y[i], q[i], q[8 + i], q[16 + i]);
-    const int part[6] = {0, 0, 0, 1, 1, 2};
+    if (k % 64 == 0) {
 #pragma unroll
-    for (int i = 0; i < 6; ++i) *reinterpret_cast<uint4*>(at + (int64_t)i * k) = p[part[i]];
+        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint4*>(row + i * k + c) = p[i];
+    } else {
+        const int pa[6] = {0, 0, 0, 1, 1, 2}, pb[6] = {0, 1, 2, 0, 1, 0};
+#pragma unroll
+        for (int i = 0; i < 6; ++i) *reinterpret_cast<uint4*>(row + i * k + c) = p[weight ? pb[i] : pa[i]];
+    }
 }
 
-// rows x k floats -> rows x 6k bf16; `weight`: in the order of a B row
+// rows x k floats -> rows x split_stored(k) k bf16; `weight`: a B row
 int launch_split_f32(const float* x, int64_t rows, int k, bool weight, void* out, cudaStream_t stream);
 
 }  // namespace ptv3

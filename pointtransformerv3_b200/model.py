@@ -235,7 +235,8 @@ class SerializedAttention(PointModule):
 
     def attend(self, point, feat):
         """qkv projection, patch attention and output projection of ``feat``."""
-        return self.proj_drop(self.proj(self.core(point, self.qkv(feat))))
+        status = point.device_status()
+        return self.proj_drop(_linear_op(self.core(point, _linear_op(feat, self.qkv, status)), self.proj, status))
 
     def forward(self, point):
         point.feat = self.attend(point, point.feat)
@@ -751,7 +752,7 @@ class PointTransformerV3(PointModule):
             _PLAN_STREAMS[key] = torch.cuda.Stream(device=device, priority=-1)
         return _PLAN_STREAMS[key]
 
-    def _native(self, point):
+    def _native(self, point, known_depth):
         """The one-call form of this forward, where it covers the network and the input: bf16 or fp32 on the GPU,
         standard modules, nobody hooked onto a single module, no per-operator timing."""
         feat = point.feat
@@ -759,15 +760,19 @@ class PointTransformerV3(PointModule):
                 or feat.shape[0] == 0 or ops.TIMERS is not None or feat.requires_grad
                 or (feat.dtype == torch.float32 and feat.shape[0] > 65535 * 128)):
             return None
+        # the batch's bounds are on their way while the host looks the network over
+        point._ensure_grid_coord()
+        stats = None
+        if "sparse_shape" not in point.keys() or not known_depth or "_counts" not in point.keys():
+            stats = ops.BatchStats(point.grid_coord, point.offset)
         native = backbone.of(self)
         if native is None or feat.dtype != native.dtype or feat.shape[1] != native.width_in or native.observed():
             return None
-        return native
+        return native, stats
 
-    def _forward_native(self, native, point, depth):
-        point._ensure_grid_coord()
-        if "sparse_shape" not in point.keys() or depth is None or "_counts" not in point.keys():
-            top, ends = ops.batch_stats(point.grid_coord, point.offset)
+    def _forward_native(self, native, stats, point, depth):
+        if stats is not None:
+            top, ends = stats.result()
             if depth is None:
                 depth = max(top).bit_length()
             if "sparse_shape" not in point.keys():
@@ -812,9 +817,9 @@ class PointTransformerV3(PointModule):
         status = point.device_status()
         point["_defer_status"] = True
         feat_dtype = point.feat.dtype
-        native = self._native(point)
+        native = self._native(point, depth is not None)
         if native is not None:
-            return self._forward_native(native, point, depth)
+            return self._forward_native(*native, point, depth)
         # -- Schedule.  Serialization and the pooling plans need only coordinates.  They run on a
         #    second, high-priority stream: a plan has one host read (its size) and a few dozen small
         #    launches, and is made two stages ahead of the features (level 1 while the stem runs,

@@ -353,19 +353,30 @@ def pool_plan(code, order, grid_coord, batch, n_scenes, pooling_depth, row_perm=
 
 
 def batch_stats(grid_coord, offset):
-    """(largest grid coordinate per axis, offsets) of a batch as Python ints: one kernel that stores
-    them in mapped host memory, which the host polls."""
-    _lib.require_cuda(grid_coord, offset)
-    lib, stream = _lib.load(), _lib.stream()
-    grid_coord = grid_coord.to(torch.int32).contiguous()
-    offset = offset.to(torch.int64).contiguous()
-    n_scenes = offset.shape[0]
-    host = _host_words(4 + n_scenes, "batch_stats", stream, offset.device)
-    host.words[3 + n_scenes] = 0
-    _lib.check(lib.ptv3_batch_stats(grid_coord.data_ptr(), grid_coord.shape[0], offset.data_ptr(), n_scenes,
-                                    host.address, host.scratch.data_ptr(), stream), "ptv3_batch_stats")
-    got = host.wait(lib, stream)
-    return got[:3], got[3:-1]
+    """(largest grid coordinate per axis, offsets) of a batch as Python ints."""
+    return BatchStats(grid_coord, offset).result()
+
+
+class BatchStats:
+    """Launches the kernel that stores a batch's bounds in mapped host memory; ``result`` waits for
+    it, so that the host can work in between.  One at a time per host thread and stream."""
+
+    def __init__(self, grid_coord, offset):
+        _lib.require_cuda(grid_coord, offset)
+        self.lib, self.stream = _lib.load(), _lib.stream()
+        grid_coord = grid_coord.to(torch.int32).contiguous()
+        offset = offset.to(torch.int64).contiguous()
+        n_scenes = offset.shape[0]
+        host = self.host = _host_words(4 + n_scenes, "batch_stats", self.stream, offset.device)
+        host.words[3 + n_scenes] = 0
+        _lib.check(self.lib.ptv3_batch_stats(grid_coord.data_ptr(), grid_coord.shape[0], offset.data_ptr(), n_scenes,
+                                             host.address, host.scratch.data_ptr(), self.stream), "ptv3_batch_stats")
+        self.keep = (grid_coord, offset)
+
+    def result(self):
+        """(largest grid coordinate per axis, offsets) as Python ints."""
+        got = self.host.wait(self.lib, self.stream)
+        return got[:3], got[3:-1]
 
 
 class _HostWords:
@@ -634,43 +645,43 @@ def linear_ln(x, weight, bias, residual, ln1, ln2, status=None, want_sum=True):
 
 
 def split_f32(x, weight=False):
-    """(..., k) fp32 -> (..., 6k) bf16: the operand of a product of floats on the bf16 tensor cores
+    """(..., k) fp32 -> (..., 3k) bf16 (6k where k is not a multiple of 64): the operand of a product of floats on the bf16 tensor cores
     (see ptv3_split_f32); ``weight`` for its second operand."""
     _lib.require_cuda(x)
     x = x.detach().contiguous()
     k = x.shape[-1]
-    out = torch.empty(x.shape[:-1] + (6 * k,), dtype=torch.bfloat16, device=x.device)
+    out = torch.empty(x.shape[:-1] + ((3 if k % 64 == 0 else 6) * k,), dtype=torch.bfloat16, device=x.device)
     _lib.check(_lib.load().ptv3_split_f32(_lib.ptr(x), x.numel() // k, k, int(weight), _lib.ptr(out), _lib.stream()),
                "ptv3_split_f32")
     return out
 
 
-def linear_split(x_split, w_split, bias=None, residual=None, gelu=False, status=None):
-    """fp32 [residual +] act(x W^T + b) from split operands."""
+def linear_split(x_split, w_split, k, bias=None, residual=None, gelu=False, status=None):
+    """fp32 [residual +] act(x W^T + b) from split operands of k columns."""
     _lib.require_cuda(x_split, w_split, bias, residual)
-    n, k6 = x_split.shape
+    n = x_split.shape[0]
     out = torch.empty((n, w_split.shape[0]), dtype=torch.float32, device=x_split.device)
     own = status is None
     if own:
         status = new_status(out.device)
     _lib.check(_lib.load().ptv3_linear_split_fwd(_lib.ptr(x_split), _lib.ptr(w_split), _lib.ptr(bias), _lib.ptr(residual),
-                                                 _lib.ptr(out), n, k6 // 6, out.shape[1], int(bool(gelu)),
+                                                 _lib.ptr(out), n, int(k), out.shape[1], int(bool(gelu)),
                                                  _lib.ptr(status), _lib.stream()), "ptv3_linear_split_fwd")
     if own:
         _lib.raise_on_status(status, "ptv3_linear_split_fwd")
     return out
 
 
-def subm_conv_split(f_split, nbr, w_split, bias=None, row_order=None, status=None):
-    """fp32 submanifold convolution from split operands (weight (C_out, kvol or k, k, k, 6 C_in))."""
+def subm_conv_split(f_split, nbr, w_split, c_in, bias=None, row_order=None, status=None):
+    """fp32 submanifold convolution from split operands of c_in columns."""
     _lib.require_cuda(f_split, nbr, w_split, bias)
-    n, c6 = f_split.shape
+    n = f_split.shape[0]
     out = torch.empty((n, w_split.shape[0]), dtype=torch.float32, device=f_split.device)
     own = status is None
     if own:
         status = new_status(out.device)
     _lib.check(_lib.load().ptv3_subm_conv_split_fwd(_lib.ptr(f_split), _lib.ptr(nbr), _lib.ptr(w_split), _lib.ptr(bias),
-                                                    _lib.ptr(out), _lib.ptr(row_order), n, c6 // 6, out.shape[1],
+                                                    _lib.ptr(out), _lib.ptr(row_order), n, int(c_in), out.shape[1],
                                                     nbr.shape[0], _lib.ptr(status), _lib.stream()),
                "ptv3_subm_conv_split_fwd")
     if own:

@@ -120,13 +120,18 @@ class Point(AttrDict):
                 self.coord - self.coord.min(0)[0], self.grid_size, rounding_mode="trunc").int()
 
     def _bounds(self):
-        """Largest grid coordinate per axis as Python ints (the host waits once; the scene sizes come along)."""
+        """A function that returns the largest grid coordinate per axis as Python ints (the host waits there;
+        the scene sizes come along)."""
         if self.grid_coord.is_cuda and "offset" in self.keys() and self.grid_coord.shape[0] > 0:
-            top, ends = ops.batch_stats(self.grid_coord, self.offset)
-            if "_counts" not in self.keys():
-                self["_counts"] = [b - a for a, b in zip([0] + ends, ends)]
-            return top
-        return torch.max(self.grid_coord, dim=0).values.tolist()
+            stats = ops.BatchStats(self.grid_coord, self.offset)
+
+            def wait():
+                top, ends = stats.result()
+                if "_counts" not in self.keys():
+                    self["_counts"] = [b - a for a, b in zip([0] + ends, ends)]
+                return top
+            return wait
+        return torch.max(self.grid_coord, dim=0).values.tolist
 
     def serialization(self, order="z", depth=None, shuffle_orders=False):
         """model.py:81-136: codes of every requested order, their stable argsort
@@ -136,7 +141,7 @@ class Point(AttrDict):
         self._ensure_grid_coord()
         order = [order] if isinstance(order, str) else list(order)
         if depth is None:
-            depth = max(self._bounds()).bit_length()
+            depth = max(self._bounds()()).bit_length()
         depth = max(int(depth), 1)
         self["serialized_depth"] = depth
         n_scene_bits = len(self.offset).bit_length()
@@ -170,16 +175,15 @@ class Point(AttrDict):
         SparseConvTensor for the submanifold convolutions."""
         assert {"feat", "batch"}.issubset(self.keys())
         self._ensure_grid_coord()
-        if "sparse_shape" in self.keys():
-            sparse_shape = self.sparse_shape
-        else:
-            sparse_shape = [v + pad for v in self._bounds()]
+        bounds = None if "sparse_shape" in self.keys() else self._bounds()
+        indices = self._sparse_indices()               # queued while the bounds are on their way
+        if bounds is not None:
+            self["sparse_shape"] = [v + pad for v in bounds()]
             self["_shape_pad"] = pad
-        self["sparse_shape"] = sparse_shape
         self["sparse_conv_feat"] = SparseConvTensor(
             features=self.feat,
-            indices=self._sparse_indices(),
-            spatial_shape=sparse_shape,
+            indices=indices,
+            spatial_shape=self.sparse_shape,
             batch_size=len(self.offset),
             row_order=self.serialized_order[0] if "serialized_order" in self.keys() else None,
             status=self.device_status(),

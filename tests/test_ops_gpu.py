@@ -752,7 +752,7 @@ def test_linear_on_split_floats(n, k, n_out, gelu, residual):
     w, b = torch.randn(n_out, k, generator=g) / k ** 0.5, torch.randn(n_out, generator=g)
     r = torch.randn(n, n_out, generator=g)
     x, w, b, r = x.cuda(), w.cuda(), b.cuda(), r.cuda()
-    got = ops.linear_split(ops.split_f32(x), ops.split_f32(w, weight=True), b, r if residual else None, gelu)
+    got = ops.linear_split(ops.split_f32(x), ops.split_f32(w, weight=True), k, b, r if residual else None, gelu)
 
     def run(*t):
         y = torch.nn.functional.linear(*t[:3])
@@ -773,7 +773,7 @@ def test_subm_conv_on_split_floats(n, cin, cout):
     feat = torch.randn(n, cin, generator=g).cuda()
     w = (torch.randn(cout, 3, 3, 3, cin, generator=g) / (9 * cin) ** 0.5).cuda()
     b = torch.randn(cout, generator=g).cuda()
-    got = ops.subm_conv_split(ops.split_f32(feat), nbr, ops.split_f32(w, weight=True), b)
+    got = ops.subm_conv_split(ops.split_f32(feat), nbr, ops.split_f32(w, weight=True), cin, b)
     plain = ops.subm_conv(feat, nbr, w, b)
     rows = torch.cat([feat.double(), feat.new_zeros(1, cin).double()])[nbr.long()]          # -1 -> the zero row
     ref = torch.einsum("onc,doc->nd", rows, w.double().reshape(cout, 27, cin)) + b.double()
