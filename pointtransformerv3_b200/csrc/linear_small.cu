@@ -390,7 +390,9 @@ template <int MODE>
 static int launch_ls(const void* x, const void* w, LinearSmallArgs a, int parts, cudaStream_t stream)
 {
     const int nk = a.k / LS_BK / parts;
-    a.stages = nk < LS_MAX_STAGES ? nk : LS_MAX_STAGES;
+    // (fp32: two CTAs share an SM, in shared memory as in tensor memory; two rooms of 20 000: 6.79 -> 6.65 ms)
+    const int most = (MODE & LS_F32) ? 4 : LS_MAX_STAGES;
+    a.stages = nk < most ? nk : most;
     CUtensorMap mx, mw;
     const uint64_t cols = (MODE & LS_F32) ? (uint64_t)a.k / 6 * split_stored(a.k / 6) : (uint64_t)a.k;      // stored
     int rc = make_tensor_map_bf16(&mx, x, (uint64_t)a.n, cols, cols * 2, LS_BM, LS_BK);
