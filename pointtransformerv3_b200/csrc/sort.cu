@@ -10,15 +10,19 @@
 // status words of the tiles before it (decoupled look-back), so a pass reads and
 // writes every element exactly once.  Digits are up to 10 bits wide and spread
 // evenly over the significant bits (29 bits -> 3 passes, 49 bits -> 5 passes).
-// The first pass reads the caller's codes and takes an element's value to be its
-// index; the last pass writes order / inverse as int64 and drops the keys.
 //
-// Bytes per element: 8 (histograms) + 8 + 12 (first pass) + 24 per middle pass +
-// 12 + 16 (last pass).  Measured on B200 a pass runs at 50-60 G elements per second
-// (16 M x 4 rows of 49 significant bits: 6.5 ms): a tile's life is a chain of short
-// phases separated by barriers, and the scattered shared-memory accesses of the
-// ranking and the reordering (several bank conflicts per access on random digits)
-// take a third of it, so the kernel sits far below the HBM bound of its 24 bytes.
+// Between passes an element is ONE 64-bit word, its key above its index, where the significant bits
+// and the bits of an index fit (37 + 23 at 8 M points): 8 bytes in and 8 out instead of 12 and 12, one
+// shared-memory access instead of two, and runs of equal digits that fill sectors.  Longer keys travel
+// beside their indices until enough of their digits are done.
+// The first pass reads the caller's codes; the last one writes order / inverse as int64.
+//
+// Bytes per element: 8 (histograms) + 16 per pass + 8 in the last one.  What bounds a pass is shared
+// memory (the counters and masks of the ranking and the reordering are scattered accesses with several bank
+// conflicts each) and a tile's chain of short phases separated by barriers: 33.5 M elements in 280 us against
+// 82 for the bytes (with 12-byte elements, tiles of 4096 and ballots: 470).  The last pass adds 390 us to that
+// for the scattered 8-byte inverses, the rate at which L2 takes single sectors (the same in a kernel of its own).
+// 8.4 M x 4 rows of 37 bits, four passes: 1.65 ms (2.75 before); 100 000 x 4 of 30: 48 us (54).
 //
 // Tiles take their number from a counter when they start, so every tile a tile
 // waits for is already running or finished; all the same every wait is bounded
@@ -30,19 +34,21 @@ namespace ptv3 {
 
 constexpr int OS_THREADS = 512;
 constexpr int OS_WARPS = OS_THREADS / 32;
-constexpr int OS_ITEMS = 8;
-constexpr int OS_TILE = OS_THREADS * OS_ITEMS;   // 4096 keys per tile
 constexpr int OS_MAX_BITS = 10;
 constexpr int OS_MAX_BINS = 1 << OS_MAX_BITS;
 constexpr int OS_DPT = OS_MAX_BINS / OS_THREADS;  // digits a thread looks after
 constexpr int OS_MAX_PASSES = 7;                  // 63 bits / 10 -> 7
 constexpr uint32_t OS_COUNT_MASK = (1u << 28) - 1u;
 constexpr uint32_t OS_SPIN_LIMIT = 1u << 20;
+constexpr int64_t OS_L2_BYTES = (int64_t)96 << 20;   // of the 126 MB, what streams leave to be kept
 constexpr int OS_WINDOW = 8;                     // earlier tiles inspected per round trip
 
 struct SortPlan {
     int passes;
     int bits;      // digit width of every pass but possibly the last
+    int val_bits;  // of an index
+    int wide;      // passes whose elements are held as a key with its index beside it
+    int items;     // per thread of a pass
     int ntiles;
     size_t bytes;
 };
@@ -91,25 +97,35 @@ __device__ __forceinline__ uint64_t os_block_excl_scan(uint64_t v, uint64_t* war
     return base + inc - v;
 }
 
-// lanes of the warp whose digit equals this lane's, among the lanes in `vmask`: one ballot per
-// digit bit, all independent of each other (the match.any instruction takes about a thousand
-// cycles on many distinct values)
-__device__ __forceinline__ uint32_t os_match(uint32_t d, int bits, uint32_t vmask)
+// How elements enter and leave a pass: as the caller's codes, as packed words, as keys with their
+// indices beside them, as the final order
+enum { OS_PACKED = 0, OS_WIDE = 1, OS_FINAL = 2 };
+
+struct OsPass {
+    const uint64_t* in;      // RAW codes, packed words or keys
+    const int32_t* vals_in;  // indices beside wide keys (nullptr: an element's index is its place)
+    uint64_t* out;
+    int32_t* vals_out;
+    int64_t *order, *inverse;
+    const uint32_t* hist;
+    uint32_t *tile_status, *tile_counter, *status;
+    int64_t n;
+    int raw;                 // PACKED: `in` holds codes, the pass packs them
+    int shift, bits;         // of the pass's digit in the key
+    int val_bits;            // of an index inside a packed word
+    int pass, ntiles, rows;
+    int by_row;              // tiles in row-after-row order
+};
+
+// shared memory of a tile's elements (or of the masks that rank them)
+__host__ __device__ constexpr size_t os_element_bytes(int items, int bins, bool wide)
 {
-    uint32_t peers = vmask;
-#pragma unroll
-    for (int b = 0; b < OS_MAX_BITS; ++b) {
-        if (b < bits) {     // uniform over the grid
-            const bool bit = (d >> b) & 1u;
-            const uint32_t bal = __ballot_sync(0xffffffffu, bit);
-            peers &= bit ? bal : ~bal;
-        }
-    }
-    return peers;
+    const size_t elements = (size_t)OS_THREADS * items * (wide ? 12 : 8), masks = (size_t)OS_WARPS * bins * 4;
+    return elements > masks ? elements : masks;
 }
 
-// One pass over one tile.  Element order inside a tile is warp-major: warp w owns
-// [w * 256, (w + 1) * 256), visited 32 consecutive elements at a time, so that
+// One pass over one tile of 512 * ITEMS elements.  Element order inside a tile is warp-major: warp w owns
+// [w * 32 * ITEMS, (w + 1) * 32 * ITEMS), visited 32 consecutive elements at a time, so that
 // (warp, item, lane) order is index order and ranks taken in that order are stable.
 //
 // Order of the steps: counts first (a histogram with shared-memory atomics) and their
@@ -118,62 +134,68 @@ __device__ __forceinline__ uint32_t os_match(uint32_t d, int bits, uint32_t vmas
 // look-back, so the walk finds an inclusive prefix after one or two tiles.  (With the look-back
 // first, a tile meets hundreds of tiles in the "counts only" state; that walk then takes longer
 // than everything else and keeps itself long.)
-template <bool FIRST, bool LAST>
-__global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(
-    const uint64_t* __restrict__ keys_in, const int32_t* __restrict__ vals_in,
-    uint64_t* __restrict__ keys_out, int32_t* __restrict__ vals_out, int64_t* __restrict__ order,
-    int64_t* __restrict__ inverse, const uint32_t* __restrict__ hist, uint32_t* __restrict__ tile_status,
-    uint32_t* __restrict__ tile_counter, uint32_t* __restrict__ status, int64_t n, int shift, int bits,
-    int pass, int ntiles, int k_rows)
+//
+// WIDE: keys of 64 bits with indices beside them; else packed words.  OUT: see above.
+template <int OS_ITEMS, bool WIDE, int OUT>
+__global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(const OsPass a)
 {
     extern __shared__ __align__(16) unsigned char os_raw[];
-    const int bins = 1 << bits;
-    uint64_t* skeys = reinterpret_cast<uint64_t*>(os_raw);                       // [OS_TILE]
-    int32_t* svals = reinterpret_cast<int32_t*>(skeys + OS_TILE);                // [OS_TILE]
-    uint16_t* whist = reinterpret_cast<uint16_t*>(svals + OS_TILE);              // [OS_WARPS][bins]
+    constexpr int OS_TILE = OS_THREADS * OS_ITEMS;
+    const int bins = 1 << a.bits;
+    uint32_t* peer_masks = reinterpret_cast<uint32_t*>(os_raw);                  // [OS_WARPS][bins], until ranked
+    uint64_t* skeys = reinterpret_cast<uint64_t*>(os_raw);                       // [OS_TILE], then
+    int32_t* svals = reinterpret_cast<int32_t*>(skeys + OS_TILE);                // [WIDE ? OS_TILE : 0]
+    uint16_t* whist = reinterpret_cast<uint16_t*>(os_raw + os_element_bytes(OS_ITEMS, bins, WIDE));    // [OS_WARPS][bins]
     uint32_t* local_off = reinterpret_cast<uint32_t*>(whist + OS_WARPS * bins);  // [bins + 1]
-    uint32_t* gprefix = local_off + bins + 1;                                    // [bins]
+    uint32_t* gbase = local_off + bins + 1;                                      // [bins]
     __shared__ uint64_t warp_sums[OS_WARPS];
     __shared__ uint32_t tile_s;
     __shared__ int give_up;
 
-    // rows take turns over the grid, so every row has the same share of the running tiles (a
-    // tile waits only for tiles of its own row)
-    const int row = blockIdx.x % k_rows;
+    const int row = a.by_row ? blockIdx.x / a.ntiles : blockIdx.x % a.rows;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t mask = (uint32_t)bins - 1u;
     if (threadIdx.x == 0) {
-        tile_s = atomicAdd(&tile_counter[pass * k_rows + row], 1u);
+        tile_s = atomicAdd(&a.tile_counter[a.pass * a.rows + row], 1u);
         give_up = 0;
     }
     // (bins >= 2: the 16-bit counters are cleared and counted in pairs)
     for (int i = threadIdx.x; i < OS_WARPS * bins / 2; i += OS_THREADS) reinterpret_cast<uint32_t*>(whist)[i] = 0;
+    for (int i = threadIdx.x; i < OS_WARPS * bins; i += OS_THREADS) peer_masks[i] = 0;
     __syncthreads();
     const int tile = (int)tile_s;
-    if (tile >= ntiles) return;    // cannot happen with a grid of ntiles blocks per row
+    if (tile >= a.ntiles) return;    // cannot happen with a grid of ntiles blocks per row
 
-    const int64_t rbase = (int64_t)row * n;
+    const int64_t rbase = (int64_t)row * a.n;
     const int64_t tbase = (int64_t)tile * OS_TILE;
-    const int64_t wbase = tbase + warp * (32 * OS_ITEMS);
-    const int tile_count = (int)min((int64_t)OS_TILE, n - tbase);
+    const int tile_count = (int)min((int64_t)OS_TILE, a.n - tbase);
+    const int wlo = warp * (32 * OS_ITEMS) + lane;       // this lane's first element inside the tile
+    // place of the pass's digit inside an element as it is held here
+    const int shift = a.shift + (WIDE ? 0 : a.val_bits);
 
     // ---- load; count the digits per warp ------------------------------------------------------
     uint64_t key[OS_ITEMS];
-    int32_t val[OS_ITEMS];
+    int32_t val[WIDE ? OS_ITEMS : 1];
     uint16_t* wh = whist + warp * bins;
-#pragma unroll
-    for (int it = 0; it < OS_ITEMS; ++it) {
-        const int64_t idx = wbase + it * 32 + lane;
-        key[it] = idx < n ? keys_in[rbase + idx] : ~0ull;
-        val[it] = FIRST ? (int32_t)idx : (idx < n ? vals_in[rbase + idx] : 0);
-    }
     {
-        // a warp holds at most 256 elements, so two 16-bit counters share a word without carries
+        const uint64_t* in = a.in + rbase + tbase;
+#pragma unroll
+        for (int it = 0; it < OS_ITEMS; ++it) {
+            const int i = wlo + it * 32;
+            key[it] = i < tile_count ? in[i] : 0ull;
+            if constexpr (WIDE)
+                val[it] = !a.vals_in ? (int32_t)(tbase + i) : i < tile_count ? a.vals_in[rbase + tbase + i] : 0;
+        }
+        if (!WIDE && a.raw) {
+#pragma unroll
+            for (int it = 0; it < OS_ITEMS; ++it)
+                key[it] = (key[it] << a.val_bits) | (uint64_t)(tbase + wlo + it * 32);
+        }
+        // a warp holds 512 elements, so two 16-bit counters share a word without carries
         uint32_t* wh32 = reinterpret_cast<uint32_t*>(wh);
 #pragma unroll
         for (int it = 0; it < OS_ITEMS; ++it) {
-            const int64_t idx = wbase + it * 32 + lane;
-            if (idx < n) {
+            if (wlo + it * 32 < tile_count) {
                 const uint32_t d = (uint32_t)(key[it] >> shift) & mask;
                 atomicAdd(&wh32[d >> 1], (d & 1u) ? 0x10000u : 1u);
             }
@@ -182,47 +204,37 @@ __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(
     __syncthreads();
 
     // ---- per digit: offsets of the warps and of the digit inside the tile -----------------------
-    // For the scans thread t owns the contiguous digits t * dpt .. t * dpt + dpt - 1; for the
-    // status table (below) it owns the interleaved digits t, t + 256, ..., so that a warp's
-    // status reads and writes are contiguous in memory.  The two views meet in shared memory.
-    const int dpt = bins > OS_THREADS ? bins / OS_THREADS : 1;
-    const bool has_digit = threadIdx.x * dpt < bins;
-    uint32_t* st_row = tile_status + ((size_t)row * ntiles) * OS_MAX_BINS;
-    const uint32_t code_agg = (uint32_t)(2 * pass + 1) << 28, code_inc = (uint32_t)(2 * pass + 2) << 28;
+    // For the scans thread t owns the digits 2 t and 2 t + 1, whose counters are one word; for the
+    // status table (below) it owns t and t + 512, so that a warp's status reads and writes are
+    // contiguous in memory.  The two views meet in shared memory.
+    uint32_t* st_row = a.tile_status + ((size_t)row * a.ntiles) * OS_MAX_BINS;
+    const uint32_t code_agg = (uint32_t)(2 * a.pass + 1) << 28, code_inc = (uint32_t)(2 * a.pass + 2) << 28;
     {
-        uint32_t cnt[OS_DPT], gcnt[OS_DPT];
-        uint32_t mine = 0, gmine = 0;
-        const uint32_t* gh = hist + ((size_t)row * OS_MAX_PASSES + pass) * OS_MAX_BINS;
+        const bool mine = threadIdx.x * 2 < bins;
+        uint32_t* column = reinterpret_cast<uint32_t*>(whist) + threadIdx.x;
+        uint32_t total = 0;            // both digits' counts, at most 8192 each
+        uint2 g = make_uint2(0u, 0u);
+        if (mine) {
 #pragma unroll
-        for (int j = 0; j < OS_DPT; ++j) {
-            cnt[j] = gcnt[j] = 0;
-            if (j < dpt && has_digit) {
-                const int d = threadIdx.x * dpt + j;
-                uint32_t run = 0;
-#pragma unroll
-                for (int w = 0; w < OS_WARPS; ++w) {
-                    const uint32_t c = whist[w * bins + d];
-                    whist[w * bins + d] = (uint16_t)run;
-                    run += c;
-                }
-                cnt[j] = run;
-                mine += run;
-                gcnt[j] = gh[d];
-                gmine += gcnt[j];
-            }
+            for (int w = 0; w < OS_WARPS; ++w) total += column[w * (bins >> 1)];
+            g = reinterpret_cast<const uint2*>(a.hist + ((size_t)row * OS_MAX_PASSES + a.pass) * OS_MAX_BINS)[threadIdx.x];
         }
+        const uint32_t lo = total & 0xffffu, hi = total >> 16;
         // exclusive prefixes over the digits: of the tile's counts (low word) and of the global
         // histogram (high word: start of every digit's range in the output)
-        const uint64_t both = os_block_excl_scan(((uint64_t)gmine << 32) | mine, warp_sums);
-        uint32_t excl = (uint32_t)both, gexcl = (uint32_t)(both >> 32);
+        const uint64_t both = os_block_excl_scan(((uint64_t)(g.x + g.y) << 32) | (lo + hi), warp_sums);
+        const uint32_t excl = (uint32_t)both, gexcl = (uint32_t)(both >> 32);
+        if (mine) {
+            local_off[2 * threadIdx.x] = excl;
+            local_off[2 * threadIdx.x + 1] = excl + lo;
+            gbase[2 * threadIdx.x] = gexcl - excl;            // the look-back adds the earlier tiles' counts
+            gbase[2 * threadIdx.x + 1] = gexcl + g.x - (excl + lo);
+            uint32_t run = excl | ((excl + lo) << 16);
 #pragma unroll
-        for (int j = 0; j < OS_DPT; ++j) {
-            if (j < dpt && has_digit) {
-                const int d = threadIdx.x * dpt + j;
-                local_off[d] = excl;
-                gprefix[d] = gexcl;          // the look-back adds the earlier tiles' counts
-                excl += cnt[j];
-                gexcl += gcnt[j];
+            for (int w = 0; w < OS_WARPS; ++w) {
+                const uint32_t c = column[w * (bins >> 1)];
+                column[w * (bins >> 1)] = run;
+                run += c;
             }
         }
         if (threadIdx.x == 0) local_off[bins] = (uint32_t)tile_count;
@@ -242,39 +254,39 @@ __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(
         }
     }
 
-    // ---- rank inside the warp and order the tile by digit in shared memory ------------------------
+    // ---- rank inside the warp, then order the tile by digit in shared memory ------------------------
+    // An element's place is its warp's running offset of the digit plus its rank among the equal digits
+    // of the 32.  The lanes of a digit find each other in a word per digit and warp into which each sets its
+    // bit (a ballot per digit bit, the form before, cost 10 ballots and 140 cycles per 32 elements of a scheduler's
+    // time; match.any about a thousand); the lowest moves the offset on and clears the word.
     {
         const uint32_t lt = (1u << lane) - 1u;
-        // the matches of all items first (independent ballots), then the chain through the
-        // per-warp running offsets
-        uint32_t peers[OS_ITEMS];
+        uint32_t* masks = peer_masks + warp * bins;
+        uint16_t pos[OS_ITEMS];
 #pragma unroll
         for (int it = 0; it < OS_ITEMS; ++it) {
-            const int64_t idx = wbase + it * 32 + lane;
+            const bool valid = wlo + it * 32 < tile_count;
             const uint32_t d = (uint32_t)(key[it] >> shift) & mask;
-            const uint32_t vmask = __ballot_sync(0xffffffffu, idx < n);
-            peers[it] = os_match(d, bits, vmask);
-        }
-#pragma unroll
-        for (int it = 0; it < OS_ITEMS; ++it) {
-            const int64_t idx = wbase + it * 32 + lane;
-            const bool valid = idx < n;
-            const uint32_t d = (uint32_t)(key[it] >> shift) & mask;
-            // every lane takes part in one shuffle with its own source lane (a shuffle per group
-            // of equal digits would run the groups one after the other)
-            const int leader = valid ? __ffs(peers[it]) - 1 : lane;
-            uint32_t base = 0;
-            if (valid && lane == leader) {
-                base = wh[d];
-                wh[d] = (uint16_t)(base + __popc(peers[it]));
-            }
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (valid) {
-                const uint32_t pos = local_off[d] + base + __popc(peers[it] & lt);
-                skeys[pos] = key[it];
-                svals[pos] = val[it];
+            volatile uint32_t* group = masks + d;
+            volatile uint16_t* off = wh + d;
+            if (valid) atomicOr(masks + d, 1u << lane);
+            __syncwarp();
+            const uint32_t peers = *group, before = peers & lt, base = *off;
+            pos[it] = (uint16_t)(base + __popc(before));
+            __syncwarp();
+            if (valid && before == 0) {
+                *group = 0u;
+                *off = (uint16_t)(base + __popc(peers));
             }
             __syncwarp();
+        }
+        __syncthreads();       // the masks make room for the elements
+#pragma unroll
+        for (int it = 0; it < OS_ITEMS; ++it) {
+            if (wlo + it * 32 < tile_count) {
+                skeys[pos[it]] = key[it];
+                if constexpr (WIDE) svals[pos[it]] = val[it];
+            }
         }
     }
     // ---- look back over the earlier tiles: all of this thread's digits at once, and a window of
@@ -337,35 +349,52 @@ __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(
             if (tile > 0)
                 *reinterpret_cast<volatile uint32_t*>(&st_row[(size_t)tile * OS_MAX_BINS + d]) =
                     code_inc | ((look[j] + cnt[j]) & OS_COUNT_MASK);
-            gprefix[d] += look[j];
+            gbase[d] += look[j];
         }
     }
     __syncthreads();
     if (give_up) {
-        if (threadIdx.x == 0 && status) atomicOr(status, PTV3_STATUS_WAIT_LIMIT);
+        if (threadIdx.x == 0 && a.status) atomicOr(a.status, PTV3_STATUS_WAIT_LIMIT);
         return;
     }
 
     // ---- write out: neighbours in shared memory with the same digit are neighbours in global
+#pragma unroll 4
     for (int i = threadIdx.x; i < tile_count; i += OS_THREADS) {
         const uint64_t kx = skeys[i];
-        const uint32_t d = (uint32_t)(kx >> shift) & mask;
-        const int64_t dst = (int64_t)gprefix[d] + (i - (int)local_off[d]);
-        const int32_t v = svals[i];
-        if (LAST) {
-            order[rbase + dst] = v;
-            inverse[rbase + v] = dst;
+        const int64_t dst = rbase + (uint32_t)(gbase[(uint32_t)(kx >> shift) & mask] + (uint32_t)i);
+        if constexpr (OUT == OS_FINAL) {
+            const int64_t v = (int64_t)(kx & ((1ull << a.val_bits) - 1ull));
+            __stcs(&a.order[dst], v);       // (streams past the inverses that L2 collects)
+            a.inverse[rbase + v] = dst - rbase;
+        } else if constexpr (WIDE) {
+            const int32_t v = svals[i];
+            if (OUT == OS_WIDE) {
+                a.out[dst] = kx;
+                a.vals_out[dst] = v;
+            } else {
+                // the digits done make room for the index; the later passes find theirs lower by as much
+                a.out[dst] = ((kx >> (a.shift + a.bits)) << a.val_bits) | (uint64_t)v;
+            }
         } else {
-            keys_out[rbase + dst] = kx;
-            vals_out[rbase + dst] = v;
+            a.out[dst] = kx;
         }
     }
 }
 
-static size_t os_pass_smem(int bits)
+static size_t os_pass_smem(int items, int bits, bool wide)
 {
     const size_t bins = (size_t)1 << bits;
-    return (size_t)OS_TILE * 12 + OS_WARPS * bins * 2 + (2 * bins + 1) * 4;
+    return os_element_bytes(items, (int)bins, wide) + OS_WARPS * bins * 2 + (2 * bins + 1) * 4;
+}
+
+template <int ITEMS, bool WIDE, int OUT>
+static int os_launch(const OsPass& a, cudaStream_t stream)
+{
+    if (allow_smem(os_pass_kernel<ITEMS, WIDE, OUT>) != cudaSuccess)
+        return check_launch("ptv3_argsort_inverse: shared memory attribute");
+    os_pass_kernel<ITEMS, WIDE, OUT><<<a.ntiles * a.rows, OS_THREADS, os_pass_smem(ITEMS, a.bits, WIDE), stream>>>(a);
+    return check_launch("ptv3_argsort_inverse");
 }
 
 static SortPlan sort_plan(int k, int64_t n, int sig_bits)
@@ -373,10 +402,17 @@ static SortPlan sort_plan(int k, int64_t n, int sig_bits)
     SortPlan p;
     p.passes = sig_bits <= 0 ? 1 : (sig_bits + OS_MAX_BITS - 1) / OS_MAX_BITS;
     p.bits = sig_bits <= 0 ? 8 : (sig_bits + p.passes - 1) / p.passes;   // spread evenly
-    p.ntiles = ceil_div(n, OS_TILE);
+    p.val_bits = 1;
+    while (((n - 1) >> p.val_bits) != 0) ++p.val_bits;
+    p.wide = 0;
+    while (sig_bits - p.wide * p.bits + p.val_bits > 64) ++p.wide;
+    // tiles of 8192: half the look-back and status words per element; of 4096, with half the chain from start to
+    // end, while those of all rows run at once (two to an SM)
+    p.items = (int64_t)k * ((n + 8 * OS_THREADS - 1) / (8 * OS_THREADS)) <= 2 * 148 ? 8 : 16;
+    p.ntiles = ceil_div(n, (int64_t)p.items * OS_THREADS);
     size_t b = 0;
-    b += 2 * align_up((size_t)k * n * sizeof(uint64_t), 256);   // key ping-pong
-    b += 2 * align_up((size_t)k * n * sizeof(int32_t), 256);    // value ping-pong
+    b += 2 * align_up((size_t)k * n * sizeof(uint64_t), 256);   // ping-pong of words or keys
+    if (p.wide > 1) b += 2 * align_up((size_t)k * n * sizeof(int32_t), 256);    // and of indices beside keys
     // zeroed region: histograms, tile counters, tile status
     b += align_up((size_t)k * OS_MAX_PASSES * OS_MAX_BINS * sizeof(uint32_t), 256);
     b += align_up((size_t)k * OS_MAX_PASSES * sizeof(uint32_t), 256);
@@ -412,7 +448,9 @@ extern "C" int ptv3_argsort_inverse(const int64_t* codes, int k, int64_t n, int 
     cudaStream_t stream = (cudaStream_t)stream_;
     Carver cv(workspace);
     uint64_t* kbuf[2] = {cv.take<uint64_t>((size_t)k * n), cv.take<uint64_t>((size_t)k * n)};
-    int32_t* vbuf[2] = {cv.take<int32_t>((size_t)k * n), cv.take<int32_t>((size_t)k * n)};
+    int32_t* vbuf[2] = {nullptr, nullptr};
+    if (p.wide > 1)
+        for (int32_t*& v : vbuf) v = cv.take<int32_t>((size_t)k * n);
     char* zero_lo = cv.base + cv.off;
     uint32_t* hist = cv.take<uint32_t>((size_t)k * OS_MAX_PASSES * OS_MAX_BINS);
     uint32_t* counters = cv.take<uint32_t>((size_t)k * OS_MAX_PASSES);
@@ -426,34 +464,45 @@ extern "C" int ptv3_argsort_inverse(const int64_t* codes, int k, int64_t n, int 
         os_hist_kernel<<<dim3(hb, k), OS_THREADS, (size_t)p.passes * OS_MAX_BINS * sizeof(uint32_t), stream>>>(
             kin, n, sig_bits, p.bits, p.passes, hist);
     }
-    if (allow_smem(os_pass_kernel<true, true>) != cudaSuccess || allow_smem(os_pass_kernel<true, false>) != cudaSuccess ||
-        allow_smem(os_pass_kernel<false, true>) != cudaSuccess || allow_smem(os_pass_kernel<false, false>) != cudaSuccess)
-        return check_launch("ptv3_argsort_inverse: shared memory attribute");
-    const dim3 grid((unsigned)((size_t)p.ntiles * k));
-    const int32_t* vin = nullptr;
-    int cur = 0;
-    for (int pass = 0; pass < p.passes; ++pass) {
-        const int shift = pass * p.bits;
-        // the histogram kernel cuts every digit with the full width; the last digit then only
-        // holds the bits that are left, which is the same value (nothing is set above sig_bits)
-        const int bits = p.bits;
-        const size_t smem = os_pass_smem(bits);
-        const bool first = pass == 0, last = pass == p.passes - 1;
-        uint64_t* kout = kbuf[cur];
-        int32_t* vout = vbuf[cur];
-#define OS_LAUNCH(F, L)                                                                              \
-    os_pass_kernel<F, L><<<grid, OS_THREADS, smem, stream>>>(kin, vin, kout, vout, order, inverse, hist, \
-                                                           tile_status, counters, status, n, shift, bits, \
-                                                           pass, p.ntiles, k)
-        if (first && last) OS_LAUNCH(true, true);
-        else if (first) OS_LAUNCH(true, false);
-        else if (last) OS_LAUNCH(false, true);
-        else OS_LAUNCH(false, false);
-#undef OS_LAUNCH
-        kin = kout;
-        vin = vout;
-        cur ^= 1;
+    OsPass a;
+    a.in = kin;
+    a.vals_in = nullptr;
+    a.order = order;
+    a.inverse = inverse;
+    a.hist = hist;
+    a.tile_status = tile_status;
+    a.tile_counter = counters;
+    a.status = status;
+    a.n = n;
+    a.raw = 1;
+    a.val_bits = p.val_bits;
+    a.ntiles = p.ntiles;
+    a.rows = k;
+    // the histogram kernel cuts every digit with the full width; the last digit then only
+    // holds the bits that are left, which is the same value (nothing is set above sig_bits)
+    a.bits = p.bits;
+    a.shift = 0;
+    for (a.pass = 0; a.pass < p.passes; ++a.pass) {
+        const bool wide = a.pass < p.wide, last = a.pass == p.passes - 1;
+        a.out = kbuf[a.pass & 1];
+        a.vals_out = vbuf[a.pass & 1];
+        // rows take turns over the grid, so every row has the same share of the running tiles (a
+        // tile waits only for tiles of its own row); only the last pass goes row after row where the inverses of
+        // all rows together outgrow L2, which holds those of one (its scattered 8-byte writes then meet in L2)
+        a.by_row = last && (int64_t)k * n * 8 > OS_L2_BYTES;
+        const bool small = p.items == 8;
+        int rc;
+        if (wide && a.pass + 1 < p.wide) rc = (small ? os_launch<8, true, OS_WIDE> : os_launch<16, true, OS_WIDE>)(a, stream);
+        else if (wide) rc = (small ? os_launch<8, true, OS_PACKED> : os_launch<16, true, OS_PACKED>)(a, stream);
+        else if (last) rc = (small ? os_launch<8, false, OS_FINAL> : os_launch<16, false, OS_FINAL>)(a, stream);
+        else rc = (small ? os_launch<8, false, OS_PACKED> : os_launch<16, false, OS_PACKED>)(a, stream);
+        if (rc != PTV3_OK) return rc;
+        a.in = a.out;
+        a.vals_in = a.vals_out;
+        // (a wide pass that packs drops the digits that are done)
+        a.shift = wide && a.pass + 1 == p.wide ? 0 : a.shift + a.bits;
+        if (!wide || a.pass + 1 == p.wide) a.raw = 0;
     }
     count_launches(1 + p.passes);
-    return check_launch("ptv3_argsort_inverse");
+    return PTV3_OK;
 }

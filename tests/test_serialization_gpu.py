@@ -71,6 +71,17 @@ def test_argsort_sizes_and_ties(n, bits):
         assert (order[r].cpu().numpy() == np.argsort(codes[r].numpy(), kind="stable")).all()
 
 
+@pytest.mark.parametrize("k,n,bits", [(4, 74 * 4096, 30), (4, 74 * 4096 + 1, 30), (1, 8193, 1), (3, 2049, 62),
+                                      (2, 300001, 62), (1, 1 << 21, 54)])
+def test_argsort_tile_sizes_and_long_keys(k, n, bits):
+    """Both tile sizes, and keys that do not fit into a word with their index (for one pass and for several)."""
+    codes = torch.randint(0, 1 << bits, (k, n), generator=torch.Generator().manual_seed(n)).cuda()
+    codes[:, n // 2:] &= ~0xff                 # ties
+    order, inverse = ops.argsort_inverse(codes, bits)
+    assert torch.equal(order, torch.argsort(codes, dim=1, stable=True))
+    assert torch.equal(inverse.gather(1, order), torch.arange(n, device="cuda").expand(k, n))
+
+
 def test_large_sort_properties():
     """4 M points x 4 orders: sortedness, stability and inverse, checked on device."""
     n = 4_000_000
