@@ -765,12 +765,12 @@ class PointTransformerV3(PointModule):
         stats = None
         if "sparse_shape" not in point.keys() or not known_depth or "_counts" not in point.keys():
             stats = ops.BatchStats(point.grid_coord, point.offset)
-        native = backbone.of(self)
-        if native is None or feat.dtype != native.dtype or feat.shape[1] != native.width_in or native.observed():
+        native, checked = backbone.of(self)
+        if native is None or feat.dtype != native.dtype or feat.shape[1] != native.width_in:
             return None
-        return native, stats
+        return native, checked, stats
 
-    def _forward_native(self, native, stats, point, depth):
+    def _forward_native(self, native, checked, stats, point, depth):
         if stats is not None:
             top, ends = stats.result()
             if depth is None:
@@ -782,7 +782,8 @@ class PointTransformerV3(PointModule):
         depth = max(int(depth), 1)
         assert depth * 3 + len(point["_counts"]).bit_length() <= 63
         assert depth <= 16
-        point = native.run(self, point, depth, self._side_stream(point.feat.device))
+        if native.run(self, point, depth, self._side_stream(point.feat.device), checked) is None:
+            return None
         point["_defer_status"] = False
         if not self.defer_status_check:
             _lib.raise_on_status(point["_status"], "PointTransformerV3.forward")
@@ -818,8 +819,14 @@ class PointTransformerV3(PointModule):
         point["_defer_status"] = True
         feat_dtype = point.feat.dtype
         native = self._native(point, depth is not None)
-        if native is not None:
-            return self._forward_native(*native, point, depth)
+        done = None if native is None else self._forward_native(*native, point, depth)
+        if native is not None and done is None:
+            # the network changed since its last pass: looked over first, and possibly of another form
+            status = point["_status"] = ops.new_status(point.feat.device)
+            native = self._native(point, depth is not None)
+            done = None if native is None else self._forward_native(*native, point, depth)
+        if done is not None:
+            return done
         # -- Schedule.  Serialization and the pooling plans need only coordinates.  They run on a
         #    second, high-priority stream: a plan has one host read (its size) and a few dozen small
         #    launches, and is made two stages ahead of the features (level 1 while the stem runs,

@@ -413,6 +413,49 @@ def test_block_single_call_matches_per_operator_path(channels, heads, n_per_scen
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("change", ["buffer", "parameter", "setting", "hook", "memory"])
+def test_network_changed_between_passes(change):
+    """A pass of a known network is queued before the network is looked over: a change is seen all the same,
+    and the pass that notices it draws the random numbers of one pass."""
+    import copy
+    data = small_batch([900, 500], 7)
+    net = P.PointTransformerV3(in_channels=6, **SMALL_CFG)
+    weights.fill_state_dict(net, prefix="ptv3.")
+    net = net.eval().cuda().bfloat16()
+    fresh, calls = copy.deepcopy(net), []
+
+    def run(n):
+        torch.manual_seed(5)
+        with torch.inference_mode():
+            return n(cuda_data(data, torch.bfloat16)).feat, torch.rand(4)
+
+    def alter(n):
+        block = n.dec.dec0.block0
+        if change == "buffer":
+            n.embedding.stem.norm.running_mean.add_(0.5)
+        elif change == "parameter":
+            block.mlp[0].fc1.weight = torch.nn.Parameter(block.mlp[0].fc1.weight * 2)
+        elif change == "setting":
+            block.attn.scale *= 4
+        elif change == "memory":
+            block.mlp[0].fc1.weight.data = block.mlp[0].fc1.weight.data * 2
+        else:
+            block.register_forward_hook(lambda *a: calls.append(1))
+
+    for _ in range(3):
+        before, _ = run(net)
+    with torch.no_grad():
+        alter(net)
+        alter(fresh)
+    (got, drawn), (ref, ref_drawn) = run(net), run(fresh)
+    assert torch.equal(drawn, ref_drawn)
+    assert torch.equal(got, ref)
+    assert len(calls) == (2 if change == "hook" else 0)
+    assert change == "hook" or not torch.equal(got, before)
+    assert torch.equal(run(net)[0], ref)
+
+
+@pytest.mark.gpu
 def test_forward_with_host_metadata_and_deferred_status():
     """The optional entries that let a caller skip the host waits of a pass (scene sizes,
     code depth and sparse shape known on the host; status word read later) do not change
