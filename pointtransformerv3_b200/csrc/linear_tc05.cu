@@ -10,12 +10,11 @@
 //     and       attn.proj + shortcut + norm2         (model.py:487, 594, 598-600)
 //
 // bf16, input width K in {32, 64, 128}.  A persistent CTA keeps W in shared memory
-// (TMA, once) and runs up to four independent 128-thread groups; a group loads a
+// (TMA, once) and runs independent 128-thread groups; a group loads a
 // 128-row x tile by TMA, issues K/16 tcgen05.mma into its slice of tensor memory and
 // owns one accumulator row per thread, so LayerNorm statistics are thread-local
-// (no shuffles).  The residual sum is parked in tensor memory (tcgen05.st) between the
-// pass that forms it and the pass that normalises it.  Every intermediate the unfused
-// sequence would round to bf16 is rounded at the same place.  Waits are bounded.
+// (no shuffles).  Every intermediate the unfused sequence would round to bf16 is
+// rounded at the same place.  Waits are bounded.
 #include "common.cuh"
 #include "mma_util.cuh"
 #include "linear_small.cuh"
@@ -28,22 +27,13 @@ using namespace tc05;
 
 struct LinearArgs {
     const __nv_bfloat16* bias;       // n_out or NULL
-    __nv_bfloat16* out;              // plain mode: n x n_out
-    const __nv_bfloat16* residual;   // residual mode: n x n_out
-    const __nv_bfloat16* ln1_w;      // optional
-    const __nv_bfloat16* ln1_b;
-    const __nv_bfloat16* ln2_w;      // required in residual mode
-    const __nv_bfloat16* ln2_b;
-    __nv_bfloat16* sum_out;
-    __nv_bfloat16* norm_out;
-    float eps1, eps2;
+    __nv_bfloat16* out;              // n x n_out
     int64_t n;
     int n_out;
     int groups;       // 128-thread groups that work (1..4)
     int nacc;         // accumulators per group in tensor memory (2 where 2 x groups x columns fit in 512)
     int w_box_rows;   // rows per TMA box of W
-    int residual_mode;
-    int out_box;      // plain mode: columns per staging tile and TMA store (64, or 32 when n_out % 64 != 0)
+    int out_box;      // columns per staging tile and TMA store (64, or 32 when n_out % 64 != 0)
     uint32_t* status;
 };
 
@@ -58,30 +48,6 @@ constexpr int LIN_STAGE_BYTES = 128 * LIN_STAGE_ROW;
 
 // A warp copies the 32 rows its own threads filled (t = thread of the group; rows (t / 32) * 32 ...), so
 // that only the warp has to be in step, not the group.
-__device__ __forceinline__ void stage_to_global(const unsigned char* stage, __nv_bfloat16* dst, int64_t row0,
-                                                int64_t n, int pitch, int col0, int t)
-{
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int idx = i * 32 + (t & 31), r = (t & ~31) + (idx >> 3), c = idx & 7;
-        if (row0 + r < n)
-            *reinterpret_cast<uint4*>(dst + (row0 + r) * pitch + col0 + c * 8) =
-                *reinterpret_cast<const uint4*>(stage + r * LIN_STAGE_ROW + c * 16);
-    }
-}
-
-__device__ __forceinline__ void global_to_stage(unsigned char* stage, const __nv_bfloat16* src, int64_t row0,
-                                                int64_t n, int pitch, int col0, int t)
-{
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int idx = i * 32 + (t & 31), r = (t & ~31) + (idx >> 3), c = idx & 7;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (row0 + r < n) v = *reinterpret_cast<const uint4*>(src + (row0 + r) * pitch + col0 + c * 8);
-        *reinterpret_cast<uint4*>(stage + r * LIN_STAGE_ROW + c * 16) = v;
-    }
-}
-
 template <int K>
 __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_constant__ CUtensorMap map_x,
                                                              const __grid_constant__ CUtensorMap map_w,
@@ -100,10 +66,9 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
     const int w_block = n_out * SW;              // one K block of W
     const int off_x = KB * w_block;              // x tiles of the groups
     const int off_stage = off_x + 2 * a.groups * X_BYTES;   // (x tiles are double buffered) one staging tile per group
-    const int off_par = off_stage + a.groups * LIN_STAGE_BYTES;   // bias, ln1 w/b, ln2 w/b as floats (5 x n_out)
-    const int off_bar = off_par + 5 * n_out * 4;
-    float* par = reinterpret_cast<float*>(smem + off_par);
-    float *bias_s = par, *g1 = par + n_out, *b1 = par + 2 * n_out, *g2 = par + 3 * n_out, *b2 = par + 4 * n_out;
+    const int off_par = off_stage + a.groups * LIN_STAGE_BYTES;   // bias as floats
+    const int off_bar = off_par + n_out * 4;
+    float* bias_s = reinterpret_cast<float*>(smem + off_par);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + off_bar);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -121,13 +86,7 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
         prefetch_tensormap(&map_x);
         prefetch_tensormap(&map_w);
     }
-    for (int i = tid; i < n_out; i += 512) {
-        bias_s[i] = a.bias ? __bfloat162float(a.bias[i]) : 0.f;
-        g1[i] = a.ln1_w ? __bfloat162float(a.ln1_w[i]) : 1.f;
-        b1[i] = a.ln1_b ? __bfloat162float(a.ln1_b[i]) : 0.f;
-        g2[i] = a.ln2_w ? __bfloat162float(a.ln2_w[i]) : 1.f;
-        b2[i] = a.ln2_b ? __bfloat162float(a.ln2_b[i]) : 0.f;
-    }
+    for (int i = tid; i < n_out; i += 512) bias_s[i] = a.bias ? __bfloat162float(a.bias[i]) : 0.f;
     if (warp == 0) {
         tmem_alloc(sbase + off_bar + 136, 512);
         // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
@@ -160,34 +119,19 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
     const uint32_t tm_acc_mma0 = tmem_base + g * tm_cols;
     const uint32_t xs0 = sbase + off_x + 2 * g * X_BYTES;   // two x buffers
     unsigned char* stage = smem + off_stage + g * LIN_STAGE_BYTES;
-    unsigned char* my_row = stage + t * LIN_STAGE_ROW;
-    // columns are handled in slabs of 64 (32 when n_out is 32 or 96 leaves a half slab)
-    const int nslabs = (n_out + 63) / 64;
     // one MMA covers at most 256 output columns
     const int n_half = n_out > 256 ? n_out / 2 : n_out;
     const uint32_t idesc = umma_idesc_bf16(128, n_half);
     uint32_t xph[2] = {0, 0};
-    const float inv_c = 1.f / (float)n_out;
-    const int nchunks = n_out / 32;
 
     const int64_t ntiles = (a.n + 127) / 128;
     if (g < a.groups) {
         const int64_t tile_step = (int64_t)gridDim.x * a.groups;
-        const int64_t tile0 = (int64_t)blockIdx.x * a.groups + g;
+        const int64_t tile0 = (int64_t)g * gridDim.x + blockIdx.x;      // (few tiles: one per SM, not four on one)
         auto load_x = [&](int64_t tile, int b) {
             mbar_expect_tx(xbar0 + 8 * b, X_BYTES);
             for (int kb = 0; kb < KB; ++kb)
                 tma_load_2d(xs0 + b * X_BYTES + kb * X_BLOCK, &map_x, kb * KCOLS, (int)(tile * 128), xbar0 + 8 * b);
-        };
-        // The residual rows are read with plain loads in the middle of the epilogue; asking for
-        // them a tile ahead (L2 prefetch, no registers held) takes the DRAM latency out of the
-        // tile's serial chain.
-        auto prefetch_residual = [&](int64_t tile) {
-            const int64_t r = tile * 128 + t;
-            if (a.residual_mode && tile < ntiles && r < a.n) {
-                const char* p = reinterpret_cast<const char*>(a.residual + r * n_out);
-                for (int b = 0; b < n_out * 2; b += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + b));
-            }
         };
         // t == 0 only: the product of the x tile in buffer xb into accumulator acc
         auto issue_mma = [&](int xb, int acc) {
@@ -204,29 +148,6 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
             }
             umma_commit(mbar0 + 8 * acc);
         };
-        // residual slab 0 of a tile into the staging tile, asynchronously (the staging tile is free
-        // from the end of one tile to the residual pass of the next)
-        auto fetch_residual = [&](int64_t row0) {
-            if (!a.residual_mode) return;
-            if (n_out >= 64) {
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int idx = i * 32 + (t & 31), r = (t & ~31) + (idx >> 3), c = idx & 7;
-                    const bool in = row0 + r < a.n;
-                    cp_async16_zfill(smem_u32_generic(stage + r * LIN_STAGE_ROW + c * 16),
-                                     a.residual + (in ? row0 + r : 0) * n_out + c * 8, in);
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int idx = i * 32 + (t & 31), r = (t & ~31) + (idx >> 2), c = idx & 3;
-                    const bool in = row0 + r < a.n;
-                    cp_async16_zfill(smem_u32_generic(stage + r * LIN_STAGE_ROW + c * 16),
-                                     a.residual + (in ? row0 + r : 0) * n_out + c * 8, in);
-                }
-            }
-            cp_async_commit();
-        };
         if (t == 0 && tile0 < ntiles) {
             load_x(tile0, 0);
             if (nacc == 2) {
@@ -240,8 +161,6 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
         for (int64_t tile = tile0; tile < ntiles; tile += tile_step, ++j) {
             const int64_t row0 = tile * 128;
             const int buf = j & 1, cur = nacc == 2 ? buf : 0;
-            fetch_residual(row0);
-            prefetch_residual(tile + tile_step);
             if (nacc == 2) {
                 ok &= mbar_wait(mbar0 + 8 * cur, (j >> 1) & 1, abort);
                 if (t == 0 && tile + tile_step < ntiles) {
@@ -266,208 +185,42 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
             }
             fence_after_sync();
             const uint32_t tm_acc = tm_acc0 + cur * tm_acc_step;
-            if (!a.residual_mode) {
-                // Plain mode: a warp packs `slw` columns of its 32 rows into its own staging tile (rows
-                // slw * 2 bytes wide, swizzled like the tensor map so that the 16-byte stores of a warp
-                // do not collide) and one lane hands the tile to a TMA store, which writes whole lines.
-                const int slw = a.out_box, lane = t & 31;
-                const uint32_t wtile = smem_u32_generic(stage) + (t >> 5) * 4096;
-                const uint32_t my = wtile + lane * (slw * 2), swz = slw == 64 ? (lane & 7) : ((lane >> 1) & 3);
-                for (int sl = 0; sl < n_out / slw; ++sl) {
-                    // the copy of the slab before has finished reading the staging tile
-                    if (lane == 0) bulk_wait_read<0>();
-                    __syncwarp();
-                    for (int c = 0; c < slw / 32; ++c) {
-                        const int ch0 = sl * slw + c * 32;
-                        float4 bb[8];
+            // A warp packs `slw` columns of its 32 rows into its own staging tile (rows
+            // slw * 2 bytes wide, swizzled like the tensor map so that the 16-byte stores of a warp
+            // do not collide) and one lane hands the tile to a TMA store, which writes whole lines.
+            const int slw = a.out_box, lane = t & 31;
+            const uint32_t wtile = smem_u32_generic(stage) + (t >> 5) * 4096;
+            const uint32_t my = wtile + lane * (slw * 2), swz = slw == 64 ? (lane & 7) : ((lane >> 1) & 3);
+            for (int sl = 0; sl < n_out / slw; ++sl) {
+                // the copy of the slab before has finished reading the staging tile
+                if (lane == 0) bulk_wait_read<0>();
+                __syncwarp();
+                for (int c = 0; c < slw / 32; ++c) {
+                    const int ch0 = sl * slw + c * 32;
+                    float4 bb[8];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) bb[i] = *reinterpret_cast<const float4*>(bias_s + ch0 + i * 4);
-                        uint32_t v[32];
-                        tmem_ld32(tm_acc + ch0, v);
-                        tmem_ld_wait();
-                        tmem_ld_fence(v);
+                    for (int i = 0; i < 8; ++i) bb[i] = *reinterpret_cast<const float4*>(bias_s + ch0 + i * 4);
+                    uint32_t v[32];
+                    tmem_ld32(tm_acc + ch0, v);
+                    tmem_ld_wait();
+                    tmem_ld_fence(v);
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const float4 b0 = bb[2 * q], b1 = bb[2 * q + 1];
-                            const uint32_t* vv = v + q * 8;
-                            const uint32_t o0 = pack_bf16(__uint_as_float(vv[0]) + b0.x, __uint_as_float(vv[1]) + b0.y);
-                            const uint32_t o1 = pack_bf16(__uint_as_float(vv[2]) + b0.z, __uint_as_float(vv[3]) + b0.w);
-                            const uint32_t o2 = pack_bf16(__uint_as_float(vv[4]) + b1.x, __uint_as_float(vv[5]) + b1.y);
-                            const uint32_t o3 = pack_bf16(__uint_as_float(vv[6]) + b1.z, __uint_as_float(vv[7]) + b1.w);
-                            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(my + (((c * 4 + q) ^ swz) << 4)),
-                                         "r"(o0), "r"(o1), "r"(o2), "r"(o3));
-                        }
-                    }
-                    fence_proxy_async();
-                    __syncwarp();
-                    if (lane == 0 && row0 + (t & ~31) < a.n) {
-                        tma_store_2d(&map_o, sl * slw, (int)row0 + (t & ~31), wtile);
-                        bulk_commit();
+                    for (int q = 0; q < 4; ++q) {
+                        const float4 b0 = bb[2 * q], b1 = bb[2 * q + 1];
+                        const uint32_t* vv = v + q * 8;
+                        const uint32_t o0 = pack_bf16(__uint_as_float(vv[0]) + b0.x, __uint_as_float(vv[1]) + b0.y);
+                        const uint32_t o1 = pack_bf16(__uint_as_float(vv[2]) + b0.z, __uint_as_float(vv[3]) + b0.w);
+                        const uint32_t o2 = pack_bf16(__uint_as_float(vv[4]) + b1.x, __uint_as_float(vv[5]) + b1.y);
+                        const uint32_t o3 = pack_bf16(__uint_as_float(vv[6]) + b1.z, __uint_as_float(vv[7]) + b1.w);
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(my + (((c * 4 + q) ^ swz) << 4)),
+                                     "r"(o0), "r"(o1), "r"(o2), "r"(o3));
                     }
                 }
-            } else {
-                // The arithmetic below works on pairs of channels (fma.rn.f32x2 / add.rn.f32x2), reads the
-                // per-channel parameters two pairs at a time and converts to bf16 once per rounding
-                // (cvt.rn.bf16x2.f32; the rounded floats are the two halves of that word): the epilogue
-                // is bound by instruction issue, not by memory.
-                // ---- first LayerNorm (optional): statistics of y = round(acc + bias)
-                float mean1 = 0.f, rstd1 = 1.f;
-                if (a.ln1_w) {
-                    // one pass with sums shifted by the row's first value (no cancellation)
-                    float sh = 0.f;
-                    uint64_t nsh2 = 0, s1 = 0, q1 = 0;
-                    for (int c = 0; c < nchunks; ++c) {
-                        uint32_t v[32];
-                        tmem_ld32(tm_acc + c * 32, v);
-                        tmem_ld_wait();
-                        if (c == 0) {
-                            sh = lin_round(__uint_as_float(v[0]) + bias_s[0]);
-                            nsh2 = pack2(-sh, -sh);
-                        }
-#pragma unroll
-                        for (int i = 0; i < 32; i += 4) {
-                            const ulonglong2 bb = *reinterpret_cast<const ulonglong2*>(bias_s + c * 32 + i);
-                            uint32_t pk;
-                            const uint64_t d0 = add2(round2(add2(pack2u(v[i], v[i + 1]), bb.x), pk), nsh2);
-                            const uint64_t d1 = add2(round2(add2(pack2u(v[i + 2], v[i + 3]), bb.y), pk), nsh2);
-                            s1 = add2(s1, add2(d0, d1));
-                            q1 = fma2(d0, d0, q1);
-                            q1 = fma2(d1, d1, q1);
-                        }
-                    }
-                    const float md1 = hsum2(s1) * inv_c;
-                    mean1 = sh + md1;
-                    rstd1 = rsqrtf(fmaxf(hsum2(q1) * inv_c - md1 * md1, 0.f) + a.eps1);
-                }
-                const uint64_t nmean1 = pack2(-mean1, -mean1), rs1 = pack2(rstd1, rstd1);
-                // ---- s = residual + t, stored and parked in tensor memory; shifted sums for LN2
-                float shift = 0.f;
-                uint64_t nshift2 = 0, s2p = 0, q2p = 0;
-                for (int sl = 0; sl < nslabs; ++sl) {
-                    const int cw = min(64, n_out - sl * 64);
-                    // residual slab: coalesced into the staging tile (slab 0 was asked for at the top)
-                    if (sl == 0) {
-                        cp_async_wait<0>();
-                    } else if (cw == 64) {
-                        global_to_stage(stage, a.residual, row0, a.n, n_out, sl * 64, t);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int idx = i * 32 + (t & 31), r = (t & ~31) + (idx >> 2), c = idx & 3;
-                            uint4 v = make_uint4(0, 0, 0, 0);
-                            if (row0 + r < a.n)
-                                v = *reinterpret_cast<const uint4*>(a.residual + (row0 + r) * n_out + sl * 64 + c * 8);
-                            *reinterpret_cast<uint4*>(stage + r * LIN_STAGE_ROW + c * 16) = v;
-                        }
-                    }
-                    __syncwarp();      // the staging rows of a warp are its own
-                    for (int c = 0; c < cw / 32; ++c) {
-                        uint32_t v[32];
-                        tmem_ld32(tm_acc + sl * 64 + c * 32, v);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const uint4 rr = *reinterpret_cast<const uint4*>(my_row + c * 64 + q * 16);
-                            const uint32_t rw[4] = {rr.x, rr.y, rr.z, rr.w};
-                            uint32_t ow[4];
-                            const int ch0 = sl * 64 + c * 32 + q * 8;
-#pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                const ulonglong2 bb = *reinterpret_cast<const ulonglong2*>(bias_s + ch0 + h * 4);
-                                ulonglong2 gg = {0, 0}, hh = {0, 0};
-                                if (a.ln1_w) {
-                                    gg = *reinterpret_cast<const ulonglong2*>(g1 + ch0 + h * 4);
-                                    hh = *reinterpret_cast<const ulonglong2*>(b1 + ch0 + h * 4);
-                                }
-#pragma unroll
-                                for (int e = 0; e < 2; ++e) {
-                                    const int i = q * 8 + h * 4 + e * 2;      // first of the two columns
-                                    uint32_t pk;
-                                    uint64_t y = round2(add2(pack2u(v[i], v[i + 1]), e ? bb.y : bb.x), pk);
-                                    if (a.ln1_w)
-                                        y = round2(fma2(fma2(add2(y, nmean1), rs1, 0ull), e ? gg.y : gg.x,
-                                                        e ? hh.y : hh.x), pk);
-                                    const uint64_t sv = round2(add2(unpack_bf16x2(rw[h * 2 + e]), y), pk);
-                                    ow[h * 2 + e] = pk;
-                                    if (sl == 0 && c == 0 && q == 0 && h == 0 && e == 0) {
-                                        float lo, hi;
-                                        unpack2(sv, lo, hi);
-                                        shift = lo;
-                                        nshift2 = pack2(-lo, -lo);
-                                    }
-                                    const uint64_t d = add2(sv, nshift2);
-                                    s2p = add2(s2p, d);
-                                    q2p = fma2(d, d, q2p);
-                                    v[i] = (uint32_t)sv;
-                                    v[i + 1] = (uint32_t)(sv >> 32);
-                                }
-                            }
-                            *reinterpret_cast<uint4*>(my_row + c * 64 + q * 16) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
-                        }
-                        tmem_st32(tm_acc + sl * 64 + c * 32, v);
-                    }
-                    __syncwarp();      // the staging rows of a warp are its own
-                    if (a.sum_out) {
-                        if (cw == 64) {
-                            stage_to_global(stage, a.sum_out, row0, a.n, n_out, sl * 64, t);
-                        } else {
-#pragma unroll
-                            for (int i = 0; i < 4; ++i) {
-                                const int idx = i * 32 + (t & 31), r = (t & ~31) + (idx >> 2), c = idx & 3;
-                                if (row0 + r < a.n)
-                                    *reinterpret_cast<uint4*>(a.sum_out + (row0 + r) * n_out + sl * 64 + c * 8) =
-                                        *reinterpret_cast<const uint4*>(stage + r * LIN_STAGE_ROW + c * 16);
-                            }
-                        }
-                    }
-                    __syncwarp();      // the staging rows of a warp are its own
-                }
-                const float s2 = hsum2(s2p), q2 = hsum2(q2p);
-                tmem_st_wait();
-                const float md = s2 * inv_c;                      // mean - shift
-                const float var = fmaxf(q2 * inv_c - md * md, 0.f);
-                const float mean2 = shift + md, rstd2 = rsqrtf(var + a.eps2);
-                const uint64_t nmean2 = pack2(-mean2, -mean2), rs2 = pack2(rstd2, rstd2);
-                for (int sl = 0; sl < nslabs; ++sl) {
-                    const int cw = min(64, n_out - sl * 64);
-                    for (int c = 0; c < cw / 32; ++c) {
-                        uint32_t v[32];
-                        tmem_ld32(tm_acc + sl * 64 + c * 32, v);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            uint32_t ow[4];
-                            const int ch0 = sl * 64 + c * 32 + q * 8;
-#pragma unroll
-                            for (int h = 0; h < 2; ++h) {
-                                const ulonglong2 gg = *reinterpret_cast<const ulonglong2*>(g2 + ch0 + h * 4);
-                                const ulonglong2 hh = *reinterpret_cast<const ulonglong2*>(b2 + ch0 + h * 4);
-#pragma unroll
-                                for (int e = 0; e < 2; ++e) {
-                                    const int i = q * 8 + h * 4 + e * 2;
-                                    const uint64_t f = fma2(fma2(add2(pack2u(v[i], v[i + 1]), nmean2), rs2, 0ull),
-                                                            e ? gg.y : gg.x, e ? hh.y : hh.x);
-                                    float lo, hi;
-                                    unpack2(f, lo, hi);
-                                    ow[h * 2 + e] = pack_bf16(lo, hi);
-                                }
-                            }
-                            *reinterpret_cast<uint4*>(my_row + c * 64 + q * 16) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
-                        }
-                    }
-                    __syncwarp();      // the staging rows of a warp are its own
-                    if (cw == 64) {
-                        stage_to_global(stage, a.norm_out, row0, a.n, n_out, sl * 64, t);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const int idx = i * 32 + (t & 31), r = (t & ~31) + (idx >> 2), c = idx & 3;
-                            if (row0 + r < a.n)
-                                *reinterpret_cast<uint4*>(a.norm_out + (row0 + r) * n_out + sl * 64 + c * 8) =
-                                    *reinterpret_cast<const uint4*>(stage + r * LIN_STAGE_ROW + c * 16);
-                        }
-                    }
-                    __syncwarp();      // the staging rows of a warp are its own
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0 && row0 + (t & ~31) < a.n) {
+                    tma_store_2d(&map_o, sl * slw, (int)row0 + (t & ~31), wtile);
+                    bulk_commit();
                 }
             }
             fence_before_sync();
@@ -479,6 +232,299 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
     fence_before_sync();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem_base, 512);
+    if (tid == 0 && (*abort || !ok)) atomicOr(a.status, PTV3_STATUS_WAIT_LIMIT);
+}
+
+template <int VEC, int PITCH>
+__device__ __forceinline__ void stage_to_global(const unsigned char* stage, __nv_bfloat16* dst, int64_t row0,
+                                                int64_t n, int col0, int t)
+{
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int idx = i * 32 + (t & 31), r = (t & ~31) + idx / VEC, c = idx % VEC;
+        if (row0 + r < n)
+            *reinterpret_cast<uint4*>(dst + (row0 + r) * PITCH + col0 + c * 8) =
+                *reinterpret_cast<const uint4*>(stage + r * LIN_STAGE_ROW + c * 16);
+    }
+}
+
+template <int VEC, int PITCH>
+__device__ __forceinline__ void global_to_stage_async(unsigned char* stage, const __nv_bfloat16* src, int64_t row0,
+                                                      int64_t n, int col0, int t)
+{
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int idx = i * 32 + (t & 31), r = (t & ~31) + idx / VEC, c = idx % VEC;
+        const bool in = row0 + r < n;
+        cp_async16_zfill(smem_u32_generic(stage + r * LIN_STAGE_ROW + c * 16),
+                         src + (in ? row0 + r : 0) * PITCH + col0 + c * 8, in);
+    }
+    cp_async_commit();
+}
+
+struct LinearLnArgs {
+    const __nv_bfloat16* bias;       // K or NULL
+    const __nv_bfloat16* residual;   // n x K
+    const __nv_bfloat16 *ln1_w, *ln1_b;   // optional
+    const __nv_bfloat16 *ln2_w, *ln2_b;
+    __nv_bfloat16* sum_out;          // optional
+    __nv_bfloat16* norm_out;
+    float eps1, eps2;
+    int64_t n;
+    uint32_t* status;
+};
+
+__host__ __device__ constexpr int lin_ln_groups(int k) { return k == 128 ? 3 : 4; }
+__host__ __device__ constexpr int lin_ln_xbufs(int k) { return k == 128 ? 1 : 2; }
+constexpr size_t lin_ln_smem(int k)
+{
+    const int sw = k >= 64 ? 128 : 64, kb = k >= 64 ? k / 64 : 1;
+    return (size_t)kb * k * sw + (size_t)lin_ln_groups(k) * (lin_ln_xbufs(k) * kb * 128 * sw + LIN_STAGE_BYTES) + 5 * k * 4 +
+           160 + 1024;
+}
+
+// Linear + residual + LayerNorms (the residual form above).  A thread takes its accumulator row out of tensor
+// memory once, rounded to the bf16 pairs that everything after it works from, so the next tile's product starts
+// before this tile's epilogue, which then runs on registers alone: arithmetic on pairs of channels
+// (fma.rn.f32x2 / add.rn.f32x2), one conversion per rounding, parameters two pairs at a time from shared memory.
+// It is bound by instruction issue and the latency of four warps per scheduler. 
+// 407 678 rows of 64 channels: 60 -> 51 us (49 -> 41 without the first LayerNorm), of 32: 35 -> 26.5, 440 000 of 128:
+// 157 -> 125, against the form that parked the sum in tensor memory between the passes; 105 505 x 64: 20 -> 16.
+// K = 128: three groups with one x buffer each (two groups with two buffers fill shared memory as well).
+template <int K, bool LN1>
+__global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kernel(const __grid_constant__ CUtensorMap map_x,
+                                                                                 const __grid_constant__ CUtensorMap map_w,
+                                                                                 const LinearLnArgs a)
+{
+    constexpr int SW = K >= 64 ? 128 : 64, KB = K >= 64 ? K / 64 : 1, KCOLS = K >= 64 ? 64 : K;
+    constexpr int X_BLOCK = 128 * SW, X_BYTES = KB * X_BLOCK, W_BLOCK = K * SW;
+    constexpr int GROUPS = lin_ln_groups(K), NX = lin_ln_xbufs(K), THREADS = 128 * GROUPS;
+    constexpr int COLS = K < 64 ? K : 64, VEC = COLS / 8;       // a slab of the staging tile
+    constexpr int OFF_X = KB * W_BLOCK, OFF_STAGE = OFF_X + NX * GROUPS * X_BYTES;
+    constexpr int OFF_PAR = OFF_STAGE + GROUPS * LIN_STAGE_BYTES, OFF_BAR = OFF_PAR + 5 * K * 4;
+    constexpr uint32_t TM_COLS = GROUPS * K <= 128 ? 128 : GROUPS * K <= 256 ? 256 : 512;
+    extern __shared__ unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const uint32_t sbase = smem_u32_generic(smem);
+    float* bias_s = reinterpret_cast<float*>(smem + OFF_PAR);
+    float *g1 = bias_s + K, *b1 = bias_s + 2 * K, *g2 = bias_s + 3 * K, *b2 = bias_s + 4 * K;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+    volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, g = tid >> 7, t = tid & 127;
+    const uint32_t wbar = sbase + OFF_BAR;
+    const uint32_t xbar0 = wbar + 8 * (1 + 2 * g), mbar = wbar + 8 * (9 + g);
+
+    if (tid == 0) {
+        for (int i = 0; i < 17; ++i) mbar_init(wbar + 8 * i, 1);
+        *abort = 0;
+        fence_barrier_init();
+        prefetch_tensormap(&map_x);
+        prefetch_tensormap(&map_w);
+    }
+    for (int i = tid; i < K; i += THREADS) {
+        bias_s[i] = a.bias ? __bfloat162float(a.bias[i]) : 0.f;
+        g1[i] = LN1 ? __bfloat162float(a.ln1_w[i]) : 1.f;
+        b1[i] = LN1 ? __bfloat162float(a.ln1_b[i]) : 0.f;
+        g2[i] = __bfloat162float(a.ln2_w[i]);
+        b2[i] = __bfloat162float(a.ln2_b[i]);
+    }
+    if (warp == 0) {
+        tmem_alloc(sbase + OFF_BAR + 136, TM_COLS);
+        // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
+        pdl_launch_next();
+    }
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+    if (tid == 0) {   // weights: once per CTA
+        mbar_expect_tx(wbar, (uint32_t)(KB * W_BLOCK));
+        for (int kb = 0; kb < KB; ++kb) tma_load_2d(sbase + kb * W_BLOCK, &map_w, kb * KCOLS, 0, wbar);
+    }
+    // up to here only weights, biases and LayerNorm parameters were read: everything the kernel before
+    // this one in the stream may have written is touched after this wait
+    pdl_wait();
+    bool ok = mbar_wait(wbar, 0, abort);
+
+    const uint32_t tm_acc = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + g * K;
+    const uint32_t xs0 = sbase + OFF_X + NX * g * X_BYTES;
+    unsigned char* stage = smem + OFF_STAGE + g * LIN_STAGE_BYTES;
+    unsigned char* my_row = stage + t * LIN_STAGE_ROW;
+    constexpr float inv_c = 1.f / (float)K;
+    const int64_t ntiles = (a.n + 127) / 128, tile_step = (int64_t)gridDim.x * GROUPS;
+    const int64_t tile0 = (int64_t)g * gridDim.x + blockIdx.x;      // (few tiles: one per SM, not four on one)
+    uint32_t xph[2] = {0, 0};
+
+    // t == 0 only: an x tile into buffer b; its product
+    auto load_x = [&](int64_t tile, int b) {
+        mbar_expect_tx(xbar0 + 8 * b, X_BYTES);
+        for (int kb = 0; kb < KB; ++kb)
+            tma_load_2d(xs0 + b * X_BYTES + kb * X_BLOCK, &map_x, kb * KCOLS, (int)(tile * 128), xbar0 + 8 * b);
+    };
+    auto multiply = [&](int b) {
+        ok &= mbar_wait(xbar0 + 8 * b, xph[b], abort);
+        xph[b] ^= 1;
+        fence_after_sync();
+#pragma unroll
+        for (int k = 0; k < K / 16; ++k) {
+            const int kb = (k * 16) / KCOLS, kk = (k * 16) % KCOLS;
+            umma_bf16(tmem_base + g * K, umma_desc_kmajor(xs0 + b * X_BYTES + kb * X_BLOCK + kk * 2, SW),
+                      umma_desc_kmajor(sbase + kb * W_BLOCK + kk * 2, SW), umma_idesc_bf16(128, K), k > 0);
+        }
+        umma_commit(mbar);
+    };
+    if (t == 0 && tile0 < ntiles) {
+        load_x(tile0, 0);
+        if (NX == 2 && tile0 + tile_step < ntiles) load_x(tile0 + tile_step, 1);
+        multiply(0);
+    }
+    int j = 0;
+    for (int64_t tile = tile0; tile < ntiles; tile += tile_step, ++j) {
+        const int64_t row0 = tile * 128;
+        const int buf = NX == 2 ? j & 1 : 0;
+        const bool more = tile + tile_step < ntiles;
+        // the residual's first slab into the staging tile; the next tile's rows into L2
+        global_to_stage_async<VEC, K>(stage, a.residual, row0, a.n, 0, t);
+        if (more && row0 + tile_step * 128 + t < a.n) {
+            const char* p = reinterpret_cast<const char*>(a.residual + (row0 + tile_step * 128 + t) * K);
+#pragma unroll
+            for (int b = 0; b < K * 2; b += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(p + b));
+        }
+        ok &= mbar_wait(mbar, j & 1, abort);
+        fence_after_sync();
+        if (t == 0 && tile + NX * tile_step < ntiles) load_x(tile + NX * tile_step, buf);     // (its product is done)
+        // ---- y = round(acc + bias); sums for its LayerNorm, shifted by the row's first value (no cancellation)
+        uint32_t y[K / 2];
+        float shift1 = 0.f;
+        uint64_t nshift = 0, s1 = 0, q1 = 0;
+        // (keeps the compiler from holding raw or unpacked values, twice the registers, across chunks and passes)
+        auto pin = [&](int lo, int hi) {
+#pragma unroll
+            for (int i = 0; i < K / 2; ++i)
+                if (i >= lo && i < hi) asm volatile("" : "+r"(y[i]));
+        };
+#pragma unroll
+        for (int c = 0; c < K; c += 32) {
+            uint32_t v[32];
+            tmem_ld32(tm_acc + c, v);
+            tmem_ld_wait();
+            tmem_ld_fence(v);
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+                const ulonglong2 bb = *reinterpret_cast<const ulonglong2*>(bias_s + c + i);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const uint64_t r = round2(add2(pack2u(v[i + 2 * e], v[i + 2 * e + 1]), e ? bb.y : bb.x),
+                                              y[(c + i) / 2 + e]);
+                    if (LN1) {
+                        if (c == 0 && i == 0 && e == 0) {
+                            float lo, hi;
+                            unpack2(r, lo, hi);
+                            shift1 = lo;
+                            nshift = pack2(-lo, -lo);
+                        }
+                        const uint64_t d = add2(r, nshift);
+                        s1 = add2(s1, d);
+                        q1 = fma2(d, d, q1);
+                    }
+                }
+            }
+            pin(c / 2, c / 2 + 16);
+            if (LN1) asm volatile("" : "+l"(s1), "+l"(q1));
+        }
+        // every thread of the group has its row: the accumulator is free
+        fence_before_sync();
+        named_barrier(1 + g, 128);
+        if (NX == 2 && t == 0 && more) multiply(buf ^ 1);
+        uint64_t nmean1 = 0, rs1 = 0;
+        if (LN1) {
+            const float md = hsum2(s1) * inv_c, mean = shift1 + md;
+            const float rstd = rsqrtf(fmaxf(hsum2(q1) * inv_c - md * md, 0.f) + a.eps1);
+            nmean1 = pack2(-mean, -mean);
+            rs1 = pack2(rstd, rstd);
+        }
+        // ---- s = residual + (LayerNorm of) y, written out; shifted sums for the second LayerNorm
+        float shift2 = 0.f;
+        uint64_t s2 = 0, q2 = 0;
+#pragma unroll
+        for (int sl = 0; sl < K; sl += COLS) {
+            if (sl > 0) global_to_stage_async<VEC, K>(stage, a.residual, row0, a.n, sl, t);
+            cp_async_wait<0>();
+            __syncwarp();      // the staging rows of a warp are its own
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) {
+                const uint4 rr = *reinterpret_cast<const uint4*>(my_row + q * 16);
+                const uint32_t rw[4] = {rr.x, rr.y, rr.z, rr.w};
+                uint32_t* o = y + (sl + q * 8) / 2;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int ch = sl + q * 8 + h * 4;
+                    ulonglong2 gg = {0, 0}, hh = {0, 0};
+                    if (LN1) {
+                        gg = *reinterpret_cast<const ulonglong2*>(g1 + ch);
+                        hh = *reinterpret_cast<const ulonglong2*>(b1 + ch);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int i = h * 2 + e;
+                        uint64_t v = unpack_bf16x2(o[i]);
+                        uint32_t pk;
+                        if (LN1) v = round2(fma2(mul2(add2(v, nmean1), rs1), e ? gg.y : gg.x, e ? hh.y : hh.x), pk);
+                        v = round2(add2(unpack_bf16x2(rw[i]), v), o[i]);
+                        if (sl == 0 && q == 0 && i == 0) {
+                            float lo, hi;
+                            unpack2(v, lo, hi);
+                            shift2 = lo;
+                            nshift = pack2(-lo, -lo);
+                        }
+                        const uint64_t d = add2(v, nshift);
+                        s2 = add2(s2, d);
+                        q2 = fma2(d, d, q2);
+                    }
+                }
+                if (a.sum_out) *reinterpret_cast<uint4*>(my_row + q * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+            __syncwarp();
+            if (a.sum_out) {
+                stage_to_global<VEC, K>(stage, a.sum_out, row0, a.n, sl, t);
+                __syncwarp();
+            }
+        }
+        pin(0, K / 2);
+        const float md = hsum2(s2) * inv_c, mean2 = shift2 + md;
+        const float rstd2 = rsqrtf(fmaxf(hsum2(q2) * inv_c - md * md, 0.f) + a.eps2);
+        const uint64_t nmean2 = pack2(-mean2, -mean2), rs2 = pack2(rstd2, rstd2);
+#pragma unroll
+        for (int sl = 0; sl < K; sl += COLS) {
+#pragma unroll
+            for (int q = 0; q < VEC; ++q) {
+                uint32_t ow[4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int ch = sl + q * 8 + h * 4;
+                    const ulonglong2 gg = *reinterpret_cast<const ulonglong2*>(g2 + ch);
+                    const ulonglong2 hh = *reinterpret_cast<const ulonglong2*>(b2 + ch);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const uint64_t f = fma2(mul2(add2(unpack_bf16x2(y[ch / 2 + e]), nmean2), rs2), e ? gg.y : gg.x,
+                                                e ? hh.y : hh.x);
+                        float lo, hi;
+                        unpack2(f, lo, hi);
+                        ow[h * 2 + e] = pack_bf16(lo, hi);
+                    }
+                }
+                *reinterpret_cast<uint4*>(my_row + q * 16) = make_uint4(ow[0], ow[1], ow[2], ow[3]);
+            }
+            __syncwarp();
+            stage_to_global<VEC, K>(stage, a.norm_out, row0, a.n, sl, t);
+            __syncwarp();
+        }
+        if (NX == 1 && t == 0 && more) multiply(0);      // (at the end, where its x tile has long landed)
+    }
+    fence_before_sync();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem_base, TM_COLS);
     if (tid == 0 && (*abort || !ok)) atomicOr(a.status, PTV3_STATUS_WAIT_LIMIT);
 }
 
@@ -498,27 +544,22 @@ static int launch_linear(const void* x, const void* w, LinearArgs a, int k, cuda
     if (groups > 4) groups = 4;
     // ... and as many as fit in shared memory next to the resident weights
     while (groups > 1 && (size_t)kb * a.n_out * sw + (size_t)groups * (2 * kb * 128 * sw + LIN_STAGE_BYTES) +
-                                 5 * (size_t)a.n_out * 4 + 160 + 1024 > 220 * 1024)
+                                 (size_t)a.n_out * 4 + 160 + 1024 > 220 * 1024)
         --groups;
     a.groups = groups;
     a.nacc = 2 * groups * tm_cols <= 512 ? 2 : 1;
     CUtensorMap mx, mw, mo;
     int rc = make_tensor_map_bf16(&mx, x, (uint64_t)a.n, k, (uint64_t)k * 2, 128, kcols);
     if (rc) return rc;
-    mo = mx;      // residual mode writes its outputs with plain stores
-    if (!a.residual_mode) {
-        a.out_box = a.n_out % 64 == 0 ? 64 : 32;
-        rc = make_tensor_map_bf16(&mo, a.out, (uint64_t)a.n, (uint64_t)a.n_out, (uint64_t)a.n_out * 2, 32, a.out_box);
-        if (rc) return rc;
-    }
+    a.out_box = a.n_out % 64 == 0 ? 64 : 32;
+    rc = make_tensor_map_bf16(&mo, a.out, (uint64_t)a.n, (uint64_t)a.n_out, (uint64_t)a.n_out * 2, 32, a.out_box);
+    if (rc) return rc;
     rc = make_tensor_map_bf16(&mw, w, a.n_out, k, (uint64_t)k * 2, a.w_box_rows, kcols);
     if (rc) return rc;
     const size_t smem = (size_t)kb * a.n_out * sw + (size_t)groups * (2 * kb * 128 * sw + LIN_STAGE_BYTES) +
-                        5 * (size_t)a.n_out * 4 + 160 + 1024;
+                        (size_t)a.n_out * 4 + 160 + 1024;
     const size_t smem_req = smem < 120 * 1024 ? 120 * 1024 : smem;   // one CTA per SM (it takes all of tensor memory)
-    const int64_t ntiles = (a.n + 127) / 128;
-    int64_t grid = (ntiles + groups - 1) / groups;
-    if (grid > 148) grid = 148;
+    const int64_t ntiles = (a.n + 127) / 128, grid = ntiles < 148 ? ntiles : 148;
 #define LIN_LAUNCH(KK)                                                                                       \
     do {                                                                                                     \
         auto kern = linear_tc05_kernel<KK>;                                                                  \
@@ -532,6 +573,23 @@ static int launch_linear(const void* x, const void* w, LinearArgs a, int k, cuda
 #undef LIN_LAUNCH
     count_launches(1);
     return check_launch("ptv3_linear_fwd");
+}
+
+template <int K, bool LN1>
+static int launch_linear_ln(const void* x, const void* w, const LinearLnArgs& a, cudaStream_t stream)
+{
+    constexpr int kcols = K >= 64 ? 64 : K;
+    CUtensorMap mx, mw;
+    int rc = make_tensor_map_bf16(&mx, x, (uint64_t)a.n, K, (uint64_t)K * 2, 128, kcols);
+    if (rc == PTV3_OK) rc = make_tensor_map_bf16(&mw, w, K, K, (uint64_t)K * 2, K, kcols);
+    if (rc != PTV3_OK) return rc;
+    auto kern = linear_ln_tc05_kernel<K, LN1>;
+    if (allow_smem(kern) != cudaSuccess) return check_launch("ptv3_linear_ln_fwd: shared memory attribute");
+    const int64_t ntiles = (a.n + 127) / 128;
+    constexpr size_t smem = lin_ln_smem(K) < 120 * 1024 ? 120 * 1024 : lin_ln_smem(K);      // one CTA per SM
+    launch_dependent(kern, dim3((unsigned)(ntiles < 148 ? ntiles : 148)), dim3(128 * lin_ln_groups(K)), smem, stream, mx, mw, a);
+    count_launches(1);
+    return check_launch("ptv3_linear_ln_fwd");
 }
 
 }  // namespace ptv3
@@ -559,7 +617,6 @@ extern "C" int ptv3_linear_fwd(const void* x, const void* weight, const void* bi
     a.out = (__nv_bfloat16*)out;
     a.n = n;
     a.n_out = n_out;
-    a.residual_mode = 0;
     a.status = status;
     return launch_linear(x, weight, a, k, (cudaStream_t)stream);
 }
@@ -584,20 +641,11 @@ extern "C" int ptv3_linear_ln_fwd(const void* x, const void* weight, const void*
     if (linear_ln_small_wanted(n, channels))
         return launch_linear_ln_small(x, weight, bias, residual, ln1_weight, ln1_bias, ln1_eps, sum_out, ln2_weight,
                                       ln2_bias, ln2_eps, norm_out, n, channels, status, (cudaStream_t)stream);
-    LinearArgs a{};
-    a.bias = (const __nv_bfloat16*)bias;
-    a.residual = (const __nv_bfloat16*)residual;
-    a.ln1_w = (const __nv_bfloat16*)ln1_weight;
-    a.ln1_b = (const __nv_bfloat16*)ln1_bias;
-    a.ln2_w = (const __nv_bfloat16*)ln2_weight;
-    a.ln2_b = (const __nv_bfloat16*)ln2_bias;
-    a.sum_out = (__nv_bfloat16*)sum_out;
-    a.norm_out = (__nv_bfloat16*)norm_out;
-    a.eps1 = ln1_eps;
-    a.eps2 = ln2_eps;
-    a.n = n;
-    a.n_out = channels;
-    a.residual_mode = 1;
-    a.status = status;
-    return launch_linear(x, weight, a, channels, (cudaStream_t)stream);
+    const LinearLnArgs a{(const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)ln1_weight,
+                         (const __nv_bfloat16*)ln1_bias, (const __nv_bfloat16*)ln2_weight, (const __nv_bfloat16*)ln2_bias,
+                         (__nv_bfloat16*)sum_out, (__nv_bfloat16*)norm_out, ln1_eps, ln2_eps, n, status};
+    cudaStream_t st = (cudaStream_t)stream;
+    if (channels == 32) return ln1_weight ? launch_linear_ln<32, true>(x, weight, a, st) : launch_linear_ln<32, false>(x, weight, a, st);
+    if (channels == 64) return ln1_weight ? launch_linear_ln<64, true>(x, weight, a, st) : launch_linear_ln<64, false>(x, weight, a, st);
+    return ln1_weight ? launch_linear_ln<128, true>(x, weight, a, st) : launch_linear_ln<128, false>(x, weight, a, st);
 }

@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
 
     const int64_t ntiles = (n + 127) / 128;
     const int64_t tile_step = (int64_t)gridDim.x * Cfg::NG;
-    const int64_t tile0 = (int64_t)blockIdx.x * Cfg::NG + g;
+    const int64_t tile0 = (int64_t)g * gridDim.x + blockIdx.x;      // (few tiles: one per SM, not four on one)
     if (t == 0 && tile0 < ntiles) {
         mbar_expect_tx(xbar, Cfg::X_BYTES);
         tma_load_2d(xs, &map_x, 0, (int)(tile0 * 128), xbar);
@@ -289,8 +289,7 @@ static int launch_mlp(const void* x, const void* w1, const void* b1, const void*
     if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_mlp_fwd: shared memory attribute");
     const int64_t ntiles = (n + 127) / 128;
-    int64_t grid = (ntiles + Cfg::NG - 1) / Cfg::NG;
-    if (grid > 148) grid = 148;
+    const int64_t grid = ntiles < 148 ? ntiles : 148;
     launch_dependent(kern, dim3((unsigned)grid), dim3(128 * Cfg::NG), Cfg::SMEM, stream, mx, mw1, mw2,
                      (const __nv_bfloat16*)b1, (const __nv_bfloat16*)b2, (const __nv_bfloat16*)residual,
                      (__nv_bfloat16*)out, n, status);

@@ -657,6 +657,22 @@ def test_linear_ln_tcgen05(C, with_ln1):
     assert rel_l2(nrm, n32) <= 1.5 * rel_l2(ref_n, n32) + 1e-3
 
 
+@pytest.mark.parametrize("n,C", [(1, 32), (148 * 128 + 1, 32), (4 * 148 * 128 + 129, 32), (2 * 148 * 128 + 1, 64),
+                                 (9 * 148 * 128 - 5, 64), (148 * 128 + 1, 128), (4 * 148 * 128 + 127, 128)])
+@pytest.mark.parametrize("with_ln1", [True, False])
+def test_linear_ln_long_inputs(n, C, with_ln1):
+    """The persistent kernel from one tile to several per group, against fp32 arithmetic."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rand = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, res, w, b = rand(n, C), rand(n, C), rand(C, C) / C ** 0.5, rand(C)
+    ln1, ln2 = torch.nn.LayerNorm(C, device="cuda").bfloat16(), torch.nn.LayerNorm(C, device="cuda").bfloat16()
+    s, nrm = ops.linear_ln(x, w, b, res, ln1 if with_ln1 else None, ln2)
+    y = F.linear(x.float(), w.float(), b.float()).bfloat16().float()
+    ref_s = (res.float() + (F.layer_norm(y, (C,)).bfloat16().float() if with_ln1 else y)).bfloat16().float()
+    assert_close(s, ref_s, what="sum", **TOL[torch.bfloat16])
+    assert_close(nrm, F.layer_norm(ref_s, (C,)), what="norm", **TOL[torch.bfloat16])
+
+
 @pytest.mark.parametrize("reduce", ["max", "min", "sum", "mean"])
 def test_pool_reduce_modes(reduce):
     """All four reductions of SerializedPooling (model.py:626, 684-686)."""
