@@ -204,7 +204,7 @@ int Pass::finest()
     BB_CUDA(events_.record(side_, &sorted));
     // main stream, beside them: the voxel index that the stem and the 3x3x3 kernel map share
     char* index_ws = mem_.take<char>(voxel_index_bytes(a_.n));
-    char* wt = mem_.take<char>(conv_direct_weight_bytes(a_.stem_ksize));
+    char* wt = mem_.take<char>(conv_direct_scratch_bytes(a_.n, a_.stem_ksize));
     if (!index_ws || !wt) return out_of_memory();
     BB_STEP(ptv3_batch_indices(a_.offset, a_.n_scenes, a_.grid_coord, a_.n, nullptr, a_.indices, main_));
     VoxelIndex vi;

@@ -16,10 +16,12 @@
 // (model.py:848,860 for the stem), rounding, one contiguous store per thread.
 //
 // bf16 features take the tensor-core form of the same kernel (conv_direct_mma_kernel):
-// the staged neighbour rows of 16 offsets are the A operand (128 voxels x K = 16 x 8
+// the staged neighbour rows of a few (dx, dy) rows of offsets are the A operand (128 voxels x K = offsets x 8
 // padded channels, zero rows where a neighbour is absent) of mma.sync against that
 // round's slice of the weights; nothing is skipped because the products are cheap - the
 // CUDA-core form spends most of its instructions unpacking bf16 weights for the FMAs.
+#include <algorithm>
+
 #include "common.cuh"
 #include "convert.cuh"
 #include "kmap.cuh"
@@ -181,54 +183,65 @@ __global__ void __launch_bounds__(CD_THREADS) conv_direct_kernel(
     }
 }
 
-constexpr int CDM_CH = 16;   // kernel offsets per round of the tensor-core form (K = 128)
+constexpr int CDM_ROWS = 2;      // (dx, dy) rows of ksize offsets per round; even, so that K is a multiple of 16
 
-// [cout][kvol][cin] -> [kvol rounded up to CDM_CH][8][cout], zero padded
-__global__ void conv_direct_transpose_pad_kernel(const __nv_bfloat16* __restrict__ w,
-                                                 __nv_bfloat16* __restrict__ wt, int cout, int kvol, int cin,
-                                                 int kvol_pad)
+// What the kernel reads, once per call: the weights [cout][kvol][cin] -> [offset][8][cout], zero padded to whole
+// rounds, and the features with their rows padded to 16 bytes, so that a neighbour is one aligned copy
+__global__ void __launch_bounds__(256) conv_direct_prepare_kernel(const __nv_bfloat16* __restrict__ w,
+                                                                  __nv_bfloat16* __restrict__ wt, int cout, int kvol,
+                                                                  int cin, int kvol_pad,
+                                                                  const __nv_bfloat16* __restrict__ feat,
+                                                                  uint4* __restrict__ rows, int64_t n)
 {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= kvol_pad * 8 * cout) return;
-    const int co = idx % cout, ci = (idx / cout) % 8, o = idx / (8 * cout);
-    wt[idx] = (o < kvol && ci < cin) ? w[((size_t)co * kvol + o) * cin + ci] : __float2bfloat16(0.f);
+    const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t idx = first; idx < (int64_t)kvol_pad * 8 * cout; idx += step) {
+        const int co = (int)idx % cout, ci = ((int)idx / cout) % 8, o = (int)idx / (8 * cout);
+        wt[idx] = (o < kvol && ci < cin) ? w[((size_t)co * kvol + o) * cin + ci] : __float2bfloat16(0.f);
+    }
+    const unsigned short* f = reinterpret_cast<const unsigned short*>(feat);
+    for (int64_t i = first; i < n; i += step) {
+        uint32_t e[8];
+#pragma unroll
+        for (int ci = 0; ci < 8; ++ci) e[ci] = ci < cin ? f[i * cin + ci] : 0u;
+        rows[i] = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
+    }
 }
 
+// Bound by the gathers' passes through L1: a warp's 32 voxels touch 32 cell tables.  The cells of a (dx, dy) row
+// lie in at most two aligned groups of four (z runs fastest in a table), so a thread takes the row's offsets of
+// one voxel with two 16-byte loads where it took five of 4 bytes, and copies each neighbour's padded row
+// straight to shared memory.  Two rows per round and six CTAs per SM: four rows with half the CTAs, or the next
+// round's cells loaded ahead in registers, are slower on long inputs.  408 k voxels of four rooms, 6 channels:
+// 348 -> 249 us; 2.05 M of LiDAR frames, 4 channels: 2.06 -> 1.53 ms; 100 k: 99 -> 59 us.
 // NT: 8-wide output channel tiles (c_out = 8 NT, NT even)
 template <int NT>
-__global__ void __launch_bounds__(CD_THREADS) conv_direct_mma_kernel(
-    const __nv_bfloat16* __restrict__ feat, const int32_t* __restrict__ indices,
+__global__ void __launch_bounds__(CD_THREADS, NT <= 4 ? 6 : 4) conv_direct_mma_kernel(
+    const uint4* __restrict__ feat, const int32_t* __restrict__ indices,
     const __nv_bfloat16* __restrict__ wt, const __nv_bfloat16* __restrict__ bias,
     const float* __restrict__ bn_scale, const float* __restrict__ bn_shift, int apply_gelu,
-    __nv_bfloat16* __restrict__ out, const int64_t* __restrict__ row_order, int64_t n, int cin, int ksize,
+    __nv_bfloat16* __restrict__ out, const int64_t* __restrict__ row_order, int64_t n, int ksize,
     const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ vals, uint64_t cap_mask,
     const uint32_t* __restrict__ cells, uint32_t* __restrict__ status)
 {
     constexpr int COUT = 8 * NT;
     constexpr int WROW = COUT * 2 + 16;   // weight row pitch: 16 bytes of padding keep ldmatrix conflict-free
     extern __shared__ __align__(16) unsigned char smem[];
-    unsigned char* x_s = smem;                                   // [CDM_CH][128] rows of 8 channels (16 B)
-    unsigned char* w_s = smem + CDM_CH * CD_TM * 16;             // [CDM_CH * 8][COUT (+ padding)] of this round
-    __shared__ int4 coord_s[CD_TM];
+    const int per_round = CDM_ROWS * ksize;                      // offsets
+    unsigned char* x_s = smem;                                   // [per_round][128] rows of 8 channels (16 B)
+    unsigned char* w_s = smem + per_round * CD_TM * 16;          // [per_round * 8][COUT (+ padding)] of this round
     __shared__ int row_s[CD_TM];
     __shared__ uint32_t block_s[8][CD_TM];
-    __shared__ char4 delta_s[343];
+    __shared__ char2 delta_s[25];                                // (dx, dy) of a row
 
-    const int kvol = ksize * ksize * ksize;
-    const int kvol_pad = (kvol + CDM_CH - 1) / CDM_CH * CDM_CH;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int v = tid % CD_TM, half = tid / CD_TM;
     const int64_t i = (int64_t)blockIdx.x * CD_TM + v;
     const int64_t row = i < n ? (row_order ? row_order[i] : i) : -1;
     const int r = ksize / 2;
     const int4 c = row >= 0 ? reinterpret_cast<const int4*>(indices)[row] : make_int4(-1, 0, 0, 0);
-    if (half == 0) {
-        coord_s[v] = c;
-        row_s[v] = (int)row;
-    }
-    for (int o = tid; o < kvol; o += CD_THREADS)
-        delta_s[o] = make_char4((char)(o / (ksize * ksize) - r), (char)((o / ksize) % ksize - r),
-                                (char)(o % ksize - r), 0);
+    if (half == 0) row_s[v] = (int)row;
+    const int n_rows = ksize * ksize;
+    if (tid < n_rows) delta_s[tid] = make_char2((char)(tid / ksize - r), (char)(tid % ksize - r));
     bool overflow = false;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -249,59 +262,50 @@ __global__ void __launch_bounds__(CD_THREADS) conv_direct_mma_kernel(
 #pragma unroll
     for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
     const uint32_t xs_base = smem_u32(x_s), ws_base = smem_u32(w_s);
-    const bool words = (cin & 1) == 0;   // rows of an even channel count are 4-byte aligned
 
-    for (int o0 = 0; o0 < kvol_pad; o0 += CDM_CH) {
-        // this round's weights: CDM_CH * 8 rows of COUT
-        for (int idx = tid; idx < CDM_CH * COUT; idx += CD_THREADS)
-            cp_async16(ws_base + (idx / NT) * WROW + (idx % NT) * 16, wt + ((size_t)o0 * 8 * COUT + (size_t)idx * 8));
+    for (int row0 = 0; row0 < n_rows; row0 += CDM_ROWS) {
+        // this round's weights: per_round * 8 rows of COUT
+        for (int idx = tid; idx < per_round * COUT; idx += CD_THREADS)
+            cp_async16(ws_base + (idx / NT) * WROW + (idx % NT) * 16,
+                       wt + ((size_t)row0 * ksize * 8 * COUT + (size_t)idx * 8));
+        // the neighbours of a voxel along one row
+        uint4 cell[CDM_ROWS * CD_TM / CD_THREADS][2];
+#pragma unroll
+        for (int k = 0; k < CDM_ROWS * CD_TM / CD_THREADS; ++k) {
+            const int row = row0 + half + k * (CD_THREADS / CD_TM);
+            cell[k][0] = cell[k][1] = make_uint4(VI_NO_ROW, VI_NO_ROW, VI_NO_ROW, VI_NO_ROW);
+            if (c.x >= 0 && row < n_rows) {
+                const char2 d = delta_s[row];
+                const int x = c.y + d.x, y = c.z + d.y;
+                const int bi = (((x >> 2) - ((c.y - r) >> 2)) << 2) | (((y >> 2) - ((c.z - r) >> 2)) << 1);
+                const size_t at = (size_t)((x & 3) << 4 | (y & 3) << 2);
+                const uint32_t id0 = block_s[bi][v], id1 = block_s[bi | 1][v];
+                if (id0 != VI_NO_ROW) cell[k][0] = *reinterpret_cast<const uint4*>(cells + (size_t)id0 * 64 + at);
+                if (id1 != VI_NO_ROW && ((c.w - r) & 3) + ksize > 4)
+                    cell[k][1] = *reinterpret_cast<const uint4*>(cells + (size_t)id1 * 64 + at);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < CDM_ROWS * CD_TM / CD_THREADS; ++k) {
+            // entry 0 becomes the cell of dz = -r
+            const int s0 = (c.w - r) & 3;
+            uint32_t e[8] = {cell[k][0].x, cell[k][0].y, cell[k][0].z, cell[k][0].w,
+                             cell[k][1].x, cell[k][1].y, cell[k][1].z, cell[k][1].w};
+#pragma unroll
+            for (int q = 0; q < 6; ++q) e[q] = s0 & 2 ? e[q + 2] : e[q];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) e[q] = s0 & 1 ? e[q + 1] : e[q];
+            const uint32_t dst = xs_base + ((half + k * (CD_THREADS / CD_TM)) * ksize * CD_TM + v) * 16;
+#pragma unroll
+            for (int q = 0; q < 5; ++q)
+                if (q < ksize) cp_async16_zfill(dst + q * CD_TM * 16, feat + (e[q] != VI_NO_ROW ? e[q] : 0u), e[q] != VI_NO_ROW);
+        }
         cp_async_commit();
-        // neighbour rows from the cell tables, then their features; all independent
-        uint32_t j[CDM_CH * CD_TM / CD_THREADS];
-#pragma unroll
-        for (int k = 0; k < CDM_CH * CD_TM / CD_THREADS; ++k) {
-            const int idx = tid + k * CD_THREADS;
-            const int ol = idx / CD_TM, vv = idx % CD_TM;
-            const int4 cc = coord_s[vv];
-            j[k] = VI_NO_ROW;
-            if (cc.x >= 0 && o0 + ol < kvol) {
-                const char4 d = delta_s[o0 + ol];
-                const int x = cc.y + d.x, y = cc.z + d.y, z = cc.w + d.z;
-                const int bi = (((x >> 2) - ((cc.y - r) >> 2)) << 2) | (((y >> 2) - ((cc.z - r) >> 2)) << 1) |
-                               ((z >> 2) - ((cc.w - r) >> 2));
-                const uint32_t id = block_s[bi][vv];
-                if (id != VI_NO_ROW) j[k] = cells[(size_t)id * 64 + ((x & 3) << 4 | (y & 3) << 2 | (z & 3))];
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < CDM_CH * CD_TM / CD_THREADS; ++k) {
-            const int idx = tid + k * CD_THREADS;
-            uint4 val = make_uint4(0, 0, 0, 0);
-            if (j[k] != VI_NO_ROW) {
-                const __nv_bfloat16* src = feat + (int64_t)j[k] * cin;
-                if (words) {
-                    const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src);
-                    val.x = s32[0];
-                    if (cin > 2) val.y = s32[1];
-                    if (cin > 4) val.z = s32[2];
-                    if (cin > 6) val.w = s32[3];
-                } else {
-                    unsigned short e[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                    const unsigned short* s16 = reinterpret_cast<const unsigned short*>(src);
-#pragma unroll
-                    for (int ci = 0; ci < 8; ++ci)
-                        if (ci < cin) e[ci] = s16[ci];
-                    val = make_uint4(e[0] | (uint32_t)e[1] << 16, e[2] | (uint32_t)e[3] << 16,
-                                     e[4] | (uint32_t)e[5] << 16, e[6] | (uint32_t)e[7] << 16);
-                }
-            }
-            *reinterpret_cast<uint4*>(x_s + (size_t)idx * 16) = val;
-        }
         cp_async_wait<0>();
         __syncthreads();
-        // out[16 voxels of this warp][COUT] += X[16][128] . W[128][COUT]
-#pragma unroll
-        for (int ks = 0; ks < CDM_CH / 2; ++ks) {
+        // out[16 voxels of this warp][COUT] += X[16][K] . W[K][COUT]
+#pragma unroll 5
+        for (int ks = 0; ks < per_round / 2; ++ks) {
             uint32_t a[4];
             {
                 const int mi = lane >> 3, rr = lane & 7;
@@ -351,6 +355,11 @@ __global__ void __launch_bounds__(CD_THREADS) conv_direct_mma_kernel(
     }
 }
 
+// laid-out weights (whole rounds)
+static size_t conv_direct_weight_bytes(int ksize) { return align_up((size_t)(ksize * ksize + CDM_ROWS) * ksize * 8 * 64 * 4, 256); }
+// ... and the padded features
+size_t conv_direct_scratch_bytes(int64_t n, int ksize) { return conv_direct_weight_bytes(ksize) + align_up((size_t)n * 16, 256); }
+
 static int launch_conv_direct_mma(const void* feat, const int32_t* indices, const void* weight, const void* bias,
                                   const float* bn_scale, const float* bn_shift, int apply_gelu, void* out,
                                   const int64_t* row_order, int64_t n, int cin, int cout, int ksize,
@@ -358,10 +367,13 @@ static int launch_conv_direct_mma(const void* feat, const int32_t* indices, cons
                                   const uint32_t* cells, uint32_t* status, void* wt, cudaStream_t stream)
 {
     const int kvol = ksize * ksize * ksize;
-    const int kvol_pad = (kvol + CDM_CH - 1) / CDM_CH * CDM_CH;
-    conv_direct_transpose_pad_kernel<<<(kvol_pad * 8 * cout + 255) / 256, 256, 0, stream>>>(
-        (const __nv_bfloat16*)weight, (__nv_bfloat16*)wt, cout, kvol, cin, kvol_pad);
-    const size_t smem = (size_t)CDM_CH * CD_TM * 16 + (size_t)CDM_CH * 8 * (cout * 2 + 16);
+    const int rounds = (ksize * ksize + CDM_ROWS - 1) / CDM_ROWS, per_round = CDM_ROWS * ksize;
+    uint4* rows = reinterpret_cast<uint4*>(static_cast<char*>(wt) + conv_direct_weight_bytes(ksize));
+    const int64_t prepare = (std::max<int64_t>(n, rounds * per_round * 8 * cout) + 255) / 256;
+    conv_direct_prepare_kernel<<<(unsigned)std::min<int64_t>(prepare, 148 * 8), 256, 0, stream>>>(
+        (const __nv_bfloat16*)weight, (__nv_bfloat16*)wt, cout, kvol, cin, rounds * per_round, (const __nv_bfloat16*)feat,
+        rows, n);
+    const size_t smem = (size_t)per_round * CD_TM * 16 + (size_t)per_round * 8 * (cout * 2 + 16);
     const unsigned blocks = (unsigned)((n + CD_TM - 1) / CD_TM);
 #define CDM_LAUNCH(NT)                                                                                      \
     do {                                                                                                    \
@@ -369,8 +381,8 @@ static int launch_conv_direct_mma(const void* feat, const int32_t* indices, cons
         if (allow_smem(kern) != cudaSuccess)                                                \
             return check_launch("ptv3_subm_conv_direct_fwd: shared memory attribute");                      \
         kern<<<blocks, CD_THREADS, smem, stream>>>(                                                          \
-            (const __nv_bfloat16*)feat, indices, (const __nv_bfloat16*)wt, (const __nv_bfloat16*)bias,       \
-            bn_scale, bn_shift, apply_gelu, (__nv_bfloat16*)out, row_order, n, cin, ksize, keys, vals,       \
+            rows, indices, (const __nv_bfloat16*)wt, (const __nv_bfloat16*)bias,                             \
+            bn_scale, bn_shift, apply_gelu, (__nv_bfloat16*)out, row_order, n, ksize, keys, vals,            \
             cap_mask, cells, status);                                                                       \
     } while (0)
     switch (cout) {
@@ -429,7 +441,6 @@ static int launch_conv_direct(const void* feat, const int32_t* indices, const vo
     return check_launch("ptv3_subm_conv_direct_fwd");
 }
 
-size_t conv_direct_weight_bytes(int ksize) { return align_up((size_t)ksize * ksize * ksize * 8 * 64 * 4, 256); }
 // hash table of blocks (sized for one block per voxel), block counter, one 64-entry table per block
 static size_t conv_direct_index_bytes(int64_t n) { return voxel_index_bytes(n); }
 
@@ -450,7 +461,7 @@ int conv_direct_from_index(const VoxelIndex& vi, const void* feat, const int32_t
 
 extern "C" size_t ptv3_subm_conv_direct_workspace_bytes(int64_t n, int ksize)
 {
-    return n > 0 ? ptv3::conv_direct_index_bytes(n) + ptv3::conv_direct_weight_bytes(ksize) : 0;
+    return n > 0 ? ptv3::conv_direct_index_bytes(n) + ptv3::conv_direct_scratch_bytes(n, ksize) : 0;
 }
 
 extern "C" int ptv3_subm_conv_direct_fwd(const void* feat, const int32_t* indices, const void* weight,
@@ -474,7 +485,7 @@ extern "C" int ptv3_subm_conv_direct_fwd(const void* feat, const int32_t* indice
                  "ptv3_subm_conv_direct_fwd: null pointer");
     PTV3_REQUIRE(((uintptr_t)indices & 15) == 0, PTV3_ERR_INVALID_ARGUMENT,
                  "ptv3_subm_conv_direct_fwd: indices must be 16-byte aligned");
-    const size_t need = conv_direct_index_bytes(n) + conv_direct_weight_bytes(ksize);
+    const size_t need = conv_direct_index_bytes(n) + conv_direct_scratch_bytes(n, ksize);
     PTV3_REQUIRE(workspace_bytes >= need, PTV3_ERR_WORKSPACE,
                  "ptv3_subm_conv_direct_fwd: workspace %zu < %zu bytes", workspace_bytes, need);
     PTV3_REQUIRE(((size_t)ksize * ksize * ksize * c_in * c_out) % 8 == 0, PTV3_ERR_UNSUPPORTED,

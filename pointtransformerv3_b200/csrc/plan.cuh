@@ -16,9 +16,9 @@ int pool_plan(const int64_t* code, const int64_t* order, const int32_t* grid_coo
 int kmap_from_index(const VoxelIndex& vi, const int32_t* indices, int64_t n, int ksize, const int64_t* row_order,
                     int32_t* nbr, uint32_t* status, cudaStream_t stream);
 
-// stem convolution (+ BatchNorm + GELU) on an existing voxel index; `weight_scratch` holds
-// conv_direct_weight_bytes(ksize) bytes
-size_t conv_direct_weight_bytes(int ksize);
+// stem convolution (+ BatchNorm + GELU) on an existing voxel index; `scratch` holds
+// conv_direct_scratch_bytes(n, ksize) bytes
+size_t conv_direct_scratch_bytes(int64_t n, int ksize);
 int conv_direct_from_index(const VoxelIndex& vi, const void* feat, const int32_t* indices, const void* weight,
                            const float* bn_scale, const float* bn_shift, void* out, const int64_t* row_order,
                            int64_t n, int c_in, int c_out, int ksize, int dtype, uint32_t* status, void* weight_scratch,

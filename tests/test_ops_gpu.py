@@ -516,6 +516,19 @@ def test_subm_conv_direct(cin, cout, k, fuse, dtype):
         assert_close(got, ref, what="direct conv", **TOL[dtype])
 
 
+@pytest.mark.parametrize("cin,cout,k", [(1, 32, 1), (5, 48, 5), (8, 64, 5), (7, 16, 3)])
+def test_subm_conv_direct_rows_of_offsets(cin, cout, k):
+    """Rows of offsets that are not a whole round, odd channel counts, voxels on the border of the grid."""
+    g = torch.Generator().manual_seed(cin)
+    xyz = torch.unique(torch.randint(0, 9, (400, 3), generator=g), dim=0)
+    ind = torch.cat([torch.zeros(len(xyz), 1, dtype=torch.long), xyz], 1).int()
+    feat = torch.randn(len(ind), cin, generator=g).bfloat16()
+    w = (torch.randn(cout, k, k, k, cin, generator=g) / (k ** 3 * cin) ** 0.5).bfloat16()
+    ref = O.subm_conv(feat, O.kernel_map(ind, k), w, None)
+    got = ops.subm_conv_direct(feat.cuda(), ind.cuda(), w.cuda())
+    assert_close(got, ref, what="direct conv", **TOL[torch.bfloat16])
+
+
 @pytest.mark.parametrize("C", [32, 64])
 @pytest.mark.parametrize("n", [128, 1000, 40_000])
 def test_fused_mlp_tcgen05(C, n):
