@@ -41,12 +41,15 @@ __global__ void __launch_bounds__(256) add_ln_kernel(
     const bool active = row < n;
     const float inv_c = 1.f / (float)C;
     float v[E];
+    typename V::Raw res[VPL];
     // channel of element e of this lane: vectors are interleaved over the lanes
     auto ch = [&](int k) { return (k * LANES + lane_in_row) * V::N; };
 #pragma unroll
     for (int k = 0; k < VPL; ++k) {
         if (active) {
             V::unpack(*reinterpret_cast<const typename V::Raw*>(x + row * C + ch(k)), v + k * V::N);
+            // (asked for with x, not after the first LayerNorm's reductions: 164 000 x 256: 91 -> 79 us)
+            if (residual) res[k] = *reinterpret_cast<const typename V::Raw*>(residual + row * C + ch(k));
         } else {
 #pragma unroll
             for (int i = 0; i < V::N; ++i) v[k * V::N + i] = 0.f;
@@ -77,7 +80,7 @@ __global__ void __launch_bounds__(256) add_ln_kernel(
         for (int k = 0; k < VPL; ++k) {
             float r[V::N];
             if (active) {
-                V::unpack(*reinterpret_cast<const typename V::Raw*>(residual + row * C + ch(k)), r);
+                V::unpack(res[k], r);
 #pragma unroll
                 for (int i = 0; i < V::N; ++i) v[k * V::N + i] = V::round(r[i] + v[k * V::N + i]);
             }
