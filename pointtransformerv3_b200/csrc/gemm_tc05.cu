@@ -9,12 +9,12 @@
 // A persistent CTA per SM walks 128-row x BN-column tiles (BN = 256 or 128).  Warp 0 streams
 // 64-wide K chunks of x and W through a ring of stages in shared memory with TMA (128-byte
 // swizzle), warp 1 issues four tcgen05.mma (K = 16 each) per chunk into one of TWO accumulators
-// in tensor memory and releases a stage with tcgen05.commit, warps 2..9 take a finished
-// accumulator (tcgen05.ld, thread = row; two warps per quarter of the tensor-memory lanes, half of
+// in tensor memory and releases a stage with tcgen05.commit, warps 2..9 (2..17 with GELU) take a finished
+// accumulator (tcgen05.ld, thread = row; two or four warps per quarter of the tensor-memory lanes, a share of
 // the tile's columns each), add the bias, apply GELU, add the residual row and write bf16 while
 // the next tile is already being multiplied into the other accumulator.
-// The output leaves through shared memory: each epilogue warp packs 64 columns of its 32 rows
-// into a 4 KiB staging tile (128-byte swizzle, so the 16-byte stores of a warp do not collide)
+// The output leaves through shared memory: each epilogue warp packs 64 (32) columns of its 32 rows
+// into a staging tile (swizzled, so the 16-byte stores of a warp do not collide)
 // and one lane hands the tile to TMA, which writes whole 128-byte lines; a thread that stored
 // its own row directly touched 32 lines per instruction, and that store path, not the tensor
 // pipe or DRAM, set the pace of long inputs (10 000 cycles per 128 x 256 tile).
@@ -34,11 +34,13 @@ using namespace tc05;
 constexpr int GM_BM = 128;
 constexpr int GM_BK = 64;                       // bf16 columns per stage: one 128-byte swizzle span
 constexpr int GM_A_BYTES = GM_BM * GM_BK * 2;   // 16 KiB
-constexpr int GM_EPI_WARPS = 8;                              // two per quarter of the tensor-memory lanes
-constexpr int GM_THREADS = 64 + GM_EPI_WARPS * 32;
-constexpr int GM_OUT_COLS = 64;                              // columns of a staging tile
-constexpr int GM_OUT_BYTES = 32 * GM_OUT_COLS * 2;           // per epilogue warp: 4 KiB
-constexpr int GM_OUT_TOTAL = GM_EPI_WARPS * GM_OUT_BYTES;
+// Epilogue warps, and the columns they take at a time.  Eight (two per quarter of the tensor-memory lanes) with
+// 64 columns, but sixteen with 32 where GELU follows the bias: its arithmetic wants four warps per scheduler
+// (440 000 x 128 -> 512: 136 -> 108 us, 164 000 x 256 -> 1 024: 112 -> 100), while the residual's row-per-thread
+// reads want wide pieces (fc2 of the same rows with sixteen: 110 -> 128, 104 -> 110; without either: equal).
+__host__ __device__ constexpr int gm_epi_warps(int mode) { return mode == 1 ? 16 : 8; }
+__host__ __device__ constexpr int gm_out_cols(int mode) { return mode == 1 ? 32 : 64; }
+constexpr int GM_OUT_TOTAL = 32 * 1024;         // staging tiles of the output, 32 rows per warp
 
 struct GemmArgs {
     const __nv_bfloat16* bias;       // n_out or NULL
@@ -58,11 +60,13 @@ struct GemmArgs {
 // fetches its W chunks again (from L2), which is what paces long inputs once the output path is out
 // of the way: 192 KiB per 128 x 256 tile at K = 256, against 64 KiB of x.
 template <int BN, int STAGES, int MODE, bool WRES>
-__global__ void __launch_bounds__(GM_THREADS, 1) gemm_tc05_kernel(const __grid_constant__ CUtensorMap map_x,
+__global__ void __launch_bounds__(64 + gm_epi_warps(MODE) * 32, 1) gemm_tc05_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                   const __grid_constant__ CUtensorMap map_w,
                                                                   const __grid_constant__ CUtensorMap map_o,
                                                                   const GemmArgs a)
 {
+    constexpr int GM_EPI_WARPS = gm_epi_warps(MODE), GM_OUT_COLS = gm_out_cols(MODE), GM_OUT_BYTES = 32 * GM_OUT_COLS * 2;
+    constexpr int PARTS = GM_EPI_WARPS / 4;               // epilogue warps per quarter of the lanes
     constexpr int B_BYTES = BN * GM_BK * 2;
     constexpr int STAGE_BYTES = WRES ? GM_A_BYTES : GM_A_BYTES + B_BYTES;
     constexpr int NBAR = 2 * STAGES + 5;      // full, empty per stage; accumulator full / empty x 2; W
@@ -179,11 +183,11 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tc05_kernel(const __grid_c
         // ---- epilogue: thread = row of the tile ------------------------------------------------
         const int q = warp & 3;                    // the warp's quarter of the tensor-memory lanes
         const int r = q * 32 + lane;
-        const int half = (warp - 2) >> 2;          // which half of the tile's columns
+        const int part = (warp - 2) >> 2;          // which part of the tile's columns
         const int et = tid - 64;                   // index among the epilogue threads
         const ulonglong2* bias4 = reinterpret_cast<const ulonglong2*>(bias_s);
         const uint32_t so = sbase + off_out + (warp - 2) * GM_OUT_BYTES;
-        const uint32_t my_row = lane * 128, sw = lane & 7;
+        const uint32_t my_row = lane * GM_OUT_COLS * 2, sw = GM_OUT_COLS == 64 ? lane & 7 : (lane >> 1) & 3;
         int row0, col0;
         for (int j = 0; tile_at(j, row0, col0); ++j) {
             const int buf = j & 1;
@@ -199,31 +203,32 @@ __global__ void __launch_bounds__(GM_THREADS, 1) gemm_tc05_kernel(const __grid_c
             fence_after_sync();
             const uint32_t tm = tmem_base + buf * BN + ((uint32_t)(q * 32) << 16);
             const __nv_bfloat16* rrow = (MODE & 2) ? a.residual + row * a.n_out + col0 : nullptr;
-            constexpr int NCH = BN / GM_OUT_COLS / 2;      // 64-column chunks of this warp
-            for (int c = half * NCH; c < (half + 1) * NCH; ++c) {
-                uint32_t v[2][32];
-                tmem_ld32(tm + c * 64, v[0]);
-                tmem_ld32(tm + c * 64 + 32, v[1]);
-                uint4 res4[(MODE & 2) ? 8 : 1] = {};
+            constexpr int NCH = BN / GM_OUT_COLS / PARTS;  // chunks of this warp
+            for (int c = part * NCH; c < (part + 1) * NCH; ++c) {
+                uint32_t v[GM_OUT_COLS / 32][32];
+#pragma unroll
+                for (int h = 0; h < GM_OUT_COLS / 32; ++h) tmem_ld32(tm + c * GM_OUT_COLS + h * 32, v[h]);
+                uint4 res4[(MODE & 2) ? GM_OUT_COLS / 8 : 1] = {};
                 if ((MODE & 2) && live) {
 #pragma unroll
-                    for (int g = 0; g < 8; ++g) res4[g] = *reinterpret_cast<const uint4*>(rrow + c * 64 + g * 8);
+                    for (int g = 0; g < GM_OUT_COLS / 8; ++g)
+                        res4[g] = *reinterpret_cast<const uint4*>(rrow + c * GM_OUT_COLS + g * 8);
                 }
                 // the copy of the chunk before has finished reading the staging tile
                 if (lane == 0) bulk_wait_read<0>();
                 __syncwarp();
                 tmem_ld_wait();
-                tmem_ld_fence(v[0]);
-                tmem_ld_fence(v[1]);
 #pragma unroll
-                for (int g = 0; g < 8; ++g) {
+                for (int h = 0; h < GM_OUT_COLS / 32; ++h) tmem_ld_fence(v[h]);
+#pragma unroll
+                for (int g = 0; g < GM_OUT_COLS / 8; ++g) {
                     const uint32_t* vv = &v[g >> 2][(g & 3) * 8];
                     const uint4 r4 = res4[(MODE & 2) ? g : 0];
                     const uint32_t rw[4] = {r4.x, r4.y, r4.z, r4.w};
                     uint32_t o[4];
 #pragma unroll
                     for (int p2 = 0; p2 < 4; ++p2) {
-                        const ulonglong2 b4 = bias4[c * 16 + g * 2 + (p2 >> 1)];
+                        const ulonglong2 b4 = bias4[c * (GM_OUT_COLS / 4) + g * 2 + (p2 >> 1)];
                         uint64_t y = add2(pack2u(vv[2 * p2], vv[2 * p2 + 1]), (p2 & 1) ? b4.y : b4.x);
                         float lo, hi;
                         unpack2(y, lo, hi);
@@ -294,7 +299,7 @@ static int launch_gemm_mode(const CUtensorMap& mx, const CUtensorMap& mw, const 
     const int64_t tiles = (int64_t)a.row_tiles * a.col_tiles;
     // resident W: the same number of CTAs on every column tile
     const unsigned grid = WRES ? (unsigned)(148 / a.col_tiles * a.col_tiles) : (unsigned)(tiles < 148 ? tiles : 148);
-    launch_dependent(kern, dim3(grid), dim3(GM_THREADS), smem, stream, mx, mw, mo, a);
+    launch_dependent(kern, dim3(grid), dim3(64 + gm_epi_warps(MODE) * 32), smem, stream, mx, mw, mo, a);
     count_launches(1);
     return check_launch("ptv3_gemm_fwd");
 }
@@ -322,7 +327,8 @@ static int launch_gemm(const void* x, const void* w, GemmArgs a, cudaStream_t st
     if (rc) return rc;
     rc = make_tensor_map_bf16(&mw, w, (uint64_t)a.n_out, (uint64_t)a.k, (uint64_t)a.k * 2, bn, GM_BK);
     if (rc) return rc;
-    rc = make_tensor_map_bf16(&mo, a.out, (uint64_t)a.n, (uint64_t)a.n_out, (uint64_t)a.n_out * 2, 32, GM_OUT_COLS);
+    rc = make_tensor_map_bf16(&mo, a.out, (uint64_t)a.n, (uint64_t)a.n_out, (uint64_t)a.n_out * 2, 32,
+                              gm_out_cols((a.gelu ? 1 : 0) | (a.residual ? 2 : 0)));
     if (rc) return rc;
     if (gemm_w_resident(a, bn))
         return bn == 256 ? launch_gemm_as<256, 4, true>(mx, mw, mo, a, stream)
