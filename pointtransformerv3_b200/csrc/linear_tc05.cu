@@ -274,23 +274,24 @@ struct LinearLnArgs {
     uint32_t* status;
 };
 
-__host__ __device__ constexpr int lin_ln_groups(int k) { return k == 128 ? 3 : 4; }
-__host__ __device__ constexpr int lin_ln_xbufs(int k) { return k == 128 ? 1 : 2; }
+__host__ __device__ constexpr int lin_ln_groups(int k) { return k == 128 ? 2 : k == 64 ? 3 : 4; }
 constexpr size_t lin_ln_smem(int k)
 {
     const int sw = k >= 64 ? 128 : 64, kb = k >= 64 ? k / 64 : 1;
-    return (size_t)kb * k * sw + (size_t)lin_ln_groups(k) * (lin_ln_xbufs(k) * kb * 128 * sw + LIN_STAGE_BYTES) + 5 * k * 4 +
+    return (size_t)kb * k * sw + (size_t)lin_ln_groups(k) * (kb * 128 * sw + LIN_STAGE_BYTES) + 5 * k * 4 +
            160 + 1024;
 }
 
 // Linear + residual + LayerNorms (the residual form above).  A thread takes its accumulator row out of tensor
-// memory once, rounded to the bf16 pairs that everything after it works from, so the next tile's product starts
-// before this tile's epilogue, which then runs on registers alone: arithmetic on pairs of channels
+// memory once, rounded to the bf16 pairs that everything after it works from; the epilogue then
+// runs on registers alone: arithmetic on pairs of channels
 // (fma.rn.f32x2 / add.rn.f32x2), one conversion per rounding, parameters two pairs at a time from shared memory.
-// It is bound by instruction issue and the latency of four warps per scheduler. 
-// 407 678 rows of 64 channels: 60 -> 51 us (49 -> 41 without the first LayerNorm), of 32: 35 -> 26.5, 440 000 of 128:
-// 157 -> 125, against the form that parked the sum in tensor memory between the passes; 105 505 x 64: 20 -> 16.
-// K = 128: three groups with one x buffer each (two groups with two buffers fill shared memory as well).
+// It is bound by instruction issue and the latency of few warps per scheduler.  Groups per CTA: as many as leave
+// a thread the registers of its row (two at 128 channels: 112 us for 440 000 rows against 125 with three, whose
+// threads spill; three at 64, four at 32); one x buffer and the next product issued at the end of the epilogue
+// (with two buffers and the product ahead of it the issuing warp waits where the others work: 64 channels
+// 51 -> 48 us, 32: 26.5 -> 25).  Against the form that parked the sum in tensor memory between the passes:
+// 407 678 x 64: 60 -> 48 us (49 -> 38 without the first LayerNorm), x 32: 35 -> 25, 440 000 x 128: 157 -> 112.
 template <int K, bool LN1>
 __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kernel(const __grid_constant__ CUtensorMap map_x,
                                                                                  const __grid_constant__ CUtensorMap map_w,
@@ -298,9 +299,9 @@ __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kern
 {
     constexpr int SW = K >= 64 ? 128 : 64, KB = K >= 64 ? K / 64 : 1, KCOLS = K >= 64 ? 64 : K;
     constexpr int X_BLOCK = 128 * SW, X_BYTES = KB * X_BLOCK, W_BLOCK = K * SW;
-    constexpr int GROUPS = lin_ln_groups(K), NX = lin_ln_xbufs(K), THREADS = 128 * GROUPS;
+    constexpr int GROUPS = lin_ln_groups(K), THREADS = 128 * GROUPS;
     constexpr int COLS = K < 64 ? K : 64, VEC = COLS / 8;       // a slab of the staging tile
-    constexpr int OFF_X = KB * W_BLOCK, OFF_STAGE = OFF_X + NX * GROUPS * X_BYTES;
+    constexpr int OFF_X = KB * W_BLOCK, OFF_STAGE = OFF_X + GROUPS * X_BYTES;
     constexpr int OFF_PAR = OFF_STAGE + GROUPS * LIN_STAGE_BYTES, OFF_BAR = OFF_PAR + 5 * K * 4;
     constexpr uint32_t TM_COLS = GROUPS * K <= 128 ? 128 : GROUPS * K <= 256 ? 256 : 512;
     extern __shared__ unsigned char smem_raw[];
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kern
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const int tid = threadIdx.x, warp = tid >> 5, g = tid >> 7, t = tid & 127;
     const uint32_t wbar = sbase + OFF_BAR;
-    const uint32_t xbar0 = wbar + 8 * (1 + 2 * g), mbar = wbar + 8 * (9 + g);
+    const uint32_t xbar = wbar + 8 * (1 + g), mbar = wbar + 8 * (5 + g);
 
     if (tid == 0) {
         for (int i = 0; i < 17; ++i) mbar_init(wbar + 8 * i, 1);
@@ -348,41 +349,38 @@ __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kern
     bool ok = mbar_wait(wbar, 0, abort);
 
     const uint32_t tm_acc = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + g * K;
-    const uint32_t xs0 = sbase + OFF_X + NX * g * X_BYTES;
+    const uint32_t xs = sbase + OFF_X + g * X_BYTES;
     unsigned char* stage = smem + OFF_STAGE + g * LIN_STAGE_BYTES;
     unsigned char* my_row = stage + t * LIN_STAGE_ROW;
     constexpr float inv_c = 1.f / (float)K;
     const int64_t ntiles = (a.n + 127) / 128, tile_step = (int64_t)gridDim.x * GROUPS;
     const int64_t tile0 = (int64_t)g * gridDim.x + blockIdx.x;      // (few tiles: one per SM, not four on one)
-    uint32_t xph[2] = {0, 0};
+    uint32_t xph = 0;
 
-    // t == 0 only: an x tile into buffer b; its product
-    auto load_x = [&](int64_t tile, int b) {
-        mbar_expect_tx(xbar0 + 8 * b, X_BYTES);
-        for (int kb = 0; kb < KB; ++kb)
-            tma_load_2d(xs0 + b * X_BYTES + kb * X_BLOCK, &map_x, kb * KCOLS, (int)(tile * 128), xbar0 + 8 * b);
+    // t == 0 only: an x tile; its product
+    auto load_x = [&](int64_t tile) {
+        mbar_expect_tx(xbar, X_BYTES);
+        for (int kb = 0; kb < KB; ++kb) tma_load_2d(xs + kb * X_BLOCK, &map_x, kb * KCOLS, (int)(tile * 128), xbar);
     };
-    auto multiply = [&](int b) {
-        ok &= mbar_wait(xbar0 + 8 * b, xph[b], abort);
-        xph[b] ^= 1;
+    auto multiply = [&] {
+        ok &= mbar_wait(xbar, xph, abort);
+        xph ^= 1;
         fence_after_sync();
 #pragma unroll
         for (int k = 0; k < K / 16; ++k) {
             const int kb = (k * 16) / KCOLS, kk = (k * 16) % KCOLS;
-            umma_bf16(tmem_base + g * K, umma_desc_kmajor(xs0 + b * X_BYTES + kb * X_BLOCK + kk * 2, SW),
+            umma_bf16(tmem_base + g * K, umma_desc_kmajor(xs + kb * X_BLOCK + kk * 2, SW),
                       umma_desc_kmajor(sbase + kb * W_BLOCK + kk * 2, SW), umma_idesc_bf16(128, K), k > 0);
         }
         umma_commit(mbar);
     };
     if (t == 0 && tile0 < ntiles) {
-        load_x(tile0, 0);
-        if (NX == 2 && tile0 + tile_step < ntiles) load_x(tile0 + tile_step, 1);
-        multiply(0);
+        load_x(tile0);
+        multiply();
     }
     int j = 0;
     for (int64_t tile = tile0; tile < ntiles; tile += tile_step, ++j) {
         const int64_t row0 = tile * 128;
-        const int buf = NX == 2 ? j & 1 : 0;
         const bool more = tile + tile_step < ntiles;
         // the residual's first slab into the staging tile; the next tile's rows into L2
         global_to_stage_async<VEC, K>(stage, a.residual, row0, a.n, 0, t);
@@ -393,7 +391,7 @@ __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kern
         }
         ok &= mbar_wait(mbar, j & 1, abort);
         fence_after_sync();
-        if (t == 0 && tile + NX * tile_step < ntiles) load_x(tile + NX * tile_step, buf);     // (its product is done)
+        if (t == 0 && more) load_x(tile + tile_step);     // (its product is done)
         // ---- y = round(acc + bias); sums for its LayerNorm, shifted by the row's first value (no cancellation)
         uint32_t y[K / 2];
         float shift1 = 0.f;
@@ -436,7 +434,6 @@ __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kern
         // every thread of the group has its row: the accumulator is free
         fence_before_sync();
         named_barrier(1 + g, 128);
-        if (NX == 2 && t == 0 && more) multiply(buf ^ 1);
         uint64_t nmean1 = 0, rs1 = 0;
         if (LN1) {
             const float md = hsum2(s1) * inv_c, mean = shift1 + md;
@@ -520,7 +517,7 @@ __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kern
             stage_to_global<VEC, K>(stage, a.norm_out, row0, a.n, sl, t);
             __syncwarp();
         }
-        if (NX == 1 && t == 0 && more) multiply(0);      // (at the end, where its x tile has long landed)
+        if (t == 0 && more) multiply();      // (its x tile has long landed)
     }
     fence_before_sync();
     __syncthreads();
