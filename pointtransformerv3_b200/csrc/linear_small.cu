@@ -2,15 +2,14 @@
 //
 // On a few hundred rows a layer is bound by the length of its own chain, not by any unit: the persistent
 // kernels (gemm_tc05.cu, linear_tc05.cu) give such a layer a handful of CTAs that walk all of K and then
-// spend most of their time in an epilogue of 128 or 256 columns (27 x 2048 -> 512: 15 us on four CTAs;
-// Linear + two LayerNorms at 128 channels: 13 us; the 64-channel MLP: 16 us).  Here
+// spend most of their time in an epilogue of 128 or 256 columns (27 x 2048 -> 512: 15 us on four CTAs).  Here
 //   * tiles are 64 columns wide, eight warps take 32 columns of a row each;
 //   * the weights of the first chunks are on their way before the preceding kernel has finished;
 //   * long K: a cluster of up to eight CTAs takes shares of K; the partial sums meet in distributed
 //     shared memory, every CTA finishing some of the rows (in rank order: the result is the same on
-//     every run);
-//   * Linear + LayerNorm (64 and 128 channels): a CTA, or a cluster of two, holds whole rows; row
-//     statistics are merged from the mean and centred square sum of every 32 columns.
+//     every run).
+// (Linear + LayerNorm stays with linear_tc05.cu, whose epilogue holds a row in registers: 1 560 x 64 5.1 us
+// against 6.5 in this form, 6 700 x 128 8.1 against 10.4.)
 #include "common.cuh"
 #include "linear_small.cuh"
 #include "split_f32.cuh"
@@ -26,15 +25,12 @@ constexpr int LS_A_BYTES = LS_BM * LS_BK * 2, LS_B_BYTES = LS_BN * LS_BK * 2, LS
 constexpr int LS_MAX_STAGES = 8;
 constexpr int LS_EPI_WARPS = 8, LS_THREADS = 64 + 32 * LS_EPI_WARPS;
 constexpr int LS_PITCH = LS_BN + 4;                    // floats of a row of partial sums
-constexpr int LS_PLAIN = 0, LS_GELU = 1, LS_RESIDUAL = 2, LS_LN = 4, LS_F32 = 8;
+constexpr int LS_PLAIN = 0, LS_GELU = 1, LS_RESIDUAL = 2, LS_F32 = 8;
 
 struct LinearSmallArgs {
     const void *bias, *residual;                       // bf16; fp32 with LS_F32
-    void* out;                                         // LN: the sum, or NULL
+    void* out;
     __nv_bfloat16* split_out;                          // LS_F32: the result as split rows instead
-    const __nv_bfloat16 *ln1_w, *ln1_b, *ln2_w, *ln2_b;
-    float eps1, eps2;
-    __nv_bfloat16* norm_out;
     int64_t n;
     int k, n_out, stages;
     uint32_t* status;
@@ -45,21 +41,10 @@ __host__ __device__ constexpr int ls_ring_bytes(int stages)
 {
     return stages * LS_STAGE > LS_BM * LS_PITCH * 4 ? stages * LS_STAGE : (LS_BM * LS_PITCH * 4 + 1023) / 1024 * 1024;
 }
-constexpr int LS_PARAM_BYTES = 5 * LS_BN * 4;          // bias, LN1 and LN2 weights and biases as floats
-constexpr int LS_STAT_BYTES = 2 * 2 * LS_BM * 8;       // (mean, square sum) per LayerNorm, half and row
+constexpr int LS_PARAM_BYTES = LS_BN * 4;              // bias as floats
 static size_t ls_smem(int stages)
 {
-    return ls_ring_bytes(stages) + LS_PARAM_BYTES + LS_STAT_BYTES + 8 * (2 * LS_MAX_STAGES + 1) + 16 + 1024;
-}
-
-// two floats of a peer's shared memory
-__device__ __forceinline__ float2 ld_peer_f2(uint32_t addr, uint32_t rank)
-{
-    uint32_t p;
-    float2 v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(p) : "memory");
-    return v;
+    return ls_ring_bytes(stages) + LS_PARAM_BYTES + 8 * (2 * LS_MAX_STAGES + 1) + 16 + 1024;
 }
 
 // LS_F32: eight finished columns of a row, as floats or as split bf16 parts (see split_f32.cuh)
@@ -120,11 +105,10 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
     const uint32_t sbase = smem_u32_generic(smem);
     const int stages = a.stages;
     float* params = reinterpret_cast<float*>(smem + ls_ring_bytes(stages));
-    const int off_stat = ls_ring_bytes(stages) + LS_PARAM_BYTES;
-    float2* stat = reinterpret_cast<float2*>(smem + off_stat);
-    const uint32_t full0 = sbase + off_stat + LS_STAT_BYTES, empty0 = full0 + 8 * LS_MAX_STAGES,
+    const int off_bar = ls_ring_bytes(stages) + LS_PARAM_BYTES;
+    const uint32_t full0 = sbase + off_bar, empty0 = full0 + 8 * LS_MAX_STAGES,
                    accfull = empty0 + 8 * LS_MAX_STAGES;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + off_stat + LS_STAT_BYTES + 8 * (2 * LS_MAX_STAGES + 1));
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + off_bar + 8 * (2 * LS_MAX_STAGES + 1));
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
     uint32_t* used_s = tmem_slot + 2;                      // LS_F32: the accumulators in use
     constexpr int TM_COLS = (MODE & LS_F32) ? SPLIT_ACCS * LS_BN : LS_BN;
@@ -132,7 +116,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int col0 = blockIdx.x * LS_BN, row0 = blockIdx.y * LS_BM;
     // this CTA's chunks of K
-    const int parts = (MODE & LS_LN) ? 1 : (int)gridDim.z;
+    const int parts = (int)gridDim.z;
     const int nk = a.k / LS_BK / parts, k0 = nk * (int)blockIdx.z * LS_BK;
 
     auto column_x = [&](int kc) { return (MODE & LS_F32) ? split_column_a(k0 / LS_BK + kc, a.k / 6) : k0 + kc * LS_BK; };
@@ -158,23 +142,12 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
         // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
         pdl_launch_next();
     }
-    {
-        // parameters of this CTA's columns as floats
-        constexpr int N = (MODE & LS_LN) ? 5 : 1;
-        for (int i = tid; i < N * LS_BN; i += LS_THREADS) {
-            const int j = i / LS_BN;
-            const int c = col0 + i % LS_BN;
-            if (MODE & LS_F32) {
-                params[i] = a.bias && c < a.n_out ? ((const float*)a.bias)[c] : 0.f;
-                continue;
-            }
-            const __nv_bfloat16* p = j == 0   ? (const __nv_bfloat16*)a.bias
-                                     : j == 1 ? a.ln1_w
-                                     : j == 2 ? a.ln1_b
-                                     : j == 3 ? a.ln2_w
-                                              : a.ln2_b;
-            params[i] = p ? __bfloat162float(p[c]) : 0.f;
-        }
+    for (int i = tid; i < LS_BN; i += LS_THREADS) {
+        const int c = col0 + i;
+        if (MODE & LS_F32)
+            params[i] = a.bias && c < a.n_out ? ((const float*)a.bias)[c] : 0.f;
+        else
+            params[i] = a.bias ? __bfloat162float(((const __nv_bfloat16*)a.bias)[c]) : 0.f;
     }
     fence_before_sync();
     __syncthreads();
@@ -233,7 +206,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
         }
         __syncwarp();
     } else {
-        if ((MODE & (LS_RESIDUAL | LS_LN)) && !(MODE & LS_F32) && parts == 1 && live) {
+        if ((MODE & LS_RESIDUAL) && !(MODE & LS_F32) && parts == 1 && live) {
 #pragma unroll
             for (int g = 0; g < 4; ++g)
                 res[g] = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)a.residual + row * a.n_out + col0 + c0 + g * 8);
@@ -256,85 +229,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
         }
     }
 
-    if (MODE & LS_LN) {
-        const float inv_c = 1.f / (float)a.n_out;
-        const int ctas = (int)gridDim.x;              // the cluster holds the row
-        // merges the statistics of all 32-column pieces of the row; every piece has the same size
-        auto statistics = [&](int which, float eps, float& mean, float& rstd) {
-            if (warp >= 2) {
-                float s = 0.f, m2 = 0.f;
-#pragma unroll
-                for (int i = 0; i < 32; ++i) s += v[i];
-                s *= 1.f / 32.f;
-#pragma unroll
-                for (int i = 0; i < 32; ++i) m2 = fmaf(v[i] - s, v[i] - s, m2);
-                stat[(which * 2 + half) * LS_BM + r] = make_float2(s, m2);
-            }
-            if (ctas > 1)
-                cluster_sync();
-            else
-                __syncthreads();
-            mean = rstd = 0.f;
-            if (warp >= 2) {
-                float2 p[4];
-#pragma unroll
-                for (int z = 0; z < 4; ++z)
-                    if (z < 2 * ctas)
-                        p[z] = ctas > 1 ? ld_peer_f2(sbase + off_stat + ((which * 2 + (z & 1)) * LS_BM + r) * 8, z >> 1)
-                                        : stat[(which * 2 + z) * LS_BM + r];
-                float m2 = 0.f;
-#pragma unroll
-                for (int z = 0; z < 4; ++z)
-                    if (z < 2 * ctas) mean += p[z].x;
-                mean *= 32.f * inv_c;
-#pragma unroll
-                for (int z = 0; z < 4; ++z)
-                    if (z < 2 * ctas) m2 += fmaf(32.f * (p[z].x - mean), p[z].x - mean, p[z].y);
-                rstd = rsqrtf(m2 * inv_c + eps);
-            }
-        };
-        auto to_bf16 = [](float x) { return __bfloat162float(__float2bfloat16_rn(x)); };
-        if (warp >= 2)
-#pragma unroll
-            for (int i = 0; i < 32; ++i) v[i] = to_bf16(v[i] + params[c0 + i]);
-        float mean, rstd;
-        if (a.ln1_w) {
-            statistics(0, a.eps1, mean, rstd);
-            if (warp >= 2)
-#pragma unroll
-                for (int i = 0; i < 32; ++i)
-                    v[i] = to_bf16(fmaf((v[i] - mean) * rstd, params[LS_BN + c0 + i], params[2 * LS_BN + c0 + i]));
-        }
-        if (warp >= 2) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                float f[8];
-                Vec<__nv_bfloat16>::unpack(res[g], f);
-#pragma unroll
-                for (int i = 0; i < 8; ++i) v[g * 8 + i] = to_bf16(f[i] + v[g * 8 + i]);
-                if (live && a.out)
-                    *reinterpret_cast<uint4*>((__nv_bfloat16*)a.out + row * a.n_out + col0 + c0 + g * 8) =
-                        Vec<__nv_bfloat16>::pack(v + g * 8);
-            }
-        }
-        statistics(1, a.eps2, mean, rstd);
-        // (the wait at the end: a peer's statistics outlive their readers)
-        if (ctas > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        if (live) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                float f[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-                    f[i] = fmaf((v[g * 8 + i] - mean) * rstd, params[3 * LS_BN + c0 + g * 8 + i],
-                                params[4 * LS_BN + c0 + g * 8 + i]);
-                *reinterpret_cast<uint4*>(a.norm_out + row * a.n_out + col0 + c0 + g * 8) =
-                    Vec<__nv_bfloat16>::pack(f);
-            }
-        }
-        __syncwarp();
-        if (ctas > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    } else if (parts == 1) {
+    if (parts == 1) {
         // (LS_F32: the last column tile may be half a tile)
         if (live && (!(MODE & LS_F32) || col0 + c0 < a.n_out))
 #pragma unroll
@@ -402,7 +297,7 @@ static int launch_ls(const void* x, const void* w, LinearSmallArgs a, int parts,
     auto kern = linear_small_kernel<MODE>;
     if (allow_smem(kern) != cudaSuccess) return check_launch("short Linear: shared memory attribute");
     const dim3 grid((a.n_out + LS_BN - 1) / LS_BN, (unsigned)((a.n + LS_BM - 1) / LS_BM), parts);
-    const dim3 cluster = (MODE & LS_LN) ? dim3(grid.x, 1, 1) : dim3(1, 1, parts);
+    const dim3 cluster(1, 1, parts);
     launch_dependent_cluster(kern, grid, dim3(LS_THREADS), ls_smem(a.stages), stream, cluster, mx, mw, a);
     count_launches(1);
     return check_launch("short Linear");
@@ -433,14 +328,6 @@ bool linear_small_wanted(int64_t n, int k, int n_out)
     return ls_parts(tiles, k) > 1;
 }
 
-// One wave of two CTAs per SM: 1 560 x 64: 6.2 / 10.5, 18 900 x 64: 6.7 / 10.8, 40 000 x 64 (313 tiles): 13.9 / 11.3;
-// 405 x 128: 7.9 / 13.0, 18 900 x 128 (296): 11.2 / 13.5.  Wider rows stay with Linear and row kernel: two or three
-// exchanges over four or eight CTAs cost what the second launch does (27 x 512: 11.4 us against 9.0).
-bool linear_ln_small_wanted(int64_t n, int c)
-{
-    return (c == 64 || c == 128) && (n + LS_BM - 1) / LS_BM * (c / LS_BN) <= 296;
-}
-
 int launch_linear_small(const void* x, const void* w, const void* bias, const void* residual, void* out, int64_t n, int k,
                         int n_out, int gelu, uint32_t* status, cudaStream_t stream)
 {
@@ -459,27 +346,6 @@ int launch_linear_small(const void* x, const void* w, const void* bias, const vo
     case LS_RESIDUAL: return launch_ls<LS_RESIDUAL>(x, w, a, parts, stream);
     default: return launch_ls<LS_GELU | LS_RESIDUAL>(x, w, a, parts, stream);
     }
-}
-
-int launch_linear_ln_small(const void* x, const void* w, const void* bias, const void* residual, const void* ln1_w,
-                           const void* ln1_b, float eps1, void* sum_out, const void* ln2_w, const void* ln2_b, float eps2,
-                           void* norm_out, int64_t n, int c, uint32_t* status, cudaStream_t stream)
-{
-    LinearSmallArgs a{};
-    a.bias = bias;
-    a.residual = residual;
-    a.out = sum_out;
-    a.ln1_w = (const __nv_bfloat16*)ln1_w;
-    a.ln1_b = (const __nv_bfloat16*)ln1_b;
-    a.ln2_w = (const __nv_bfloat16*)ln2_w;
-    a.ln2_b = (const __nv_bfloat16*)ln2_b;
-    a.eps1 = eps1;
-    a.eps2 = eps2;
-    a.norm_out = (__nv_bfloat16*)norm_out;
-    a.n = n;
-    a.k = a.n_out = c;
-    a.status = status;
-    return launch_ls<LS_LN>(x, w, a, 1, stream);
 }
 
 int launch_linear_split(const void* xs, const void* ws, const float* bias, const float* residual, float* out,

@@ -635,9 +635,6 @@ extern "C" int ptv3_linear_ln_fwd(const void* x, const void* weight, const void*
     PTV3_REQUIRE((((uintptr_t)x | (uintptr_t)weight | (uintptr_t)residual | (uintptr_t)norm_out |
                    (uintptr_t)sum_out) & 15) == 0,
                  PTV3_ERR_INVALID_ARGUMENT, "ptv3_linear_ln_fwd: tensors must be 16-byte aligned");
-    if (linear_ln_small_wanted(n, channels))
-        return launch_linear_ln_small(x, weight, bias, residual, ln1_weight, ln1_bias, ln1_eps, sum_out, ln2_weight,
-                                      ln2_bias, ln2_eps, norm_out, n, channels, status, (cudaStream_t)stream);
     const LinearLnArgs a{(const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)ln1_weight,
                          (const __nv_bfloat16*)ln1_bias, (const __nv_bfloat16*)ln2_weight, (const __nv_bfloat16*)ln2_bias,
                          (__nv_bfloat16*)sum_out, (__nv_bfloat16*)norm_out, ln1_eps, ln2_eps, n, status};
