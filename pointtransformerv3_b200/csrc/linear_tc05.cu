@@ -37,8 +37,6 @@ struct LinearArgs {
     uint32_t* status;
 };
 
-__device__ __forceinline__ float lin_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-
 // Staging tile of a group: 128 rows x 64 bf16 columns, rows 144 bytes apart, so that
 // both the row-per-thread accesses of the epilogue and the coalesced copies to and
 // from global memory (consecutive threads on consecutive 16-byte pieces) are free of
