@@ -16,11 +16,11 @@
  *     attention, MLP, pooling) are launched with the programmatic-serialization
  *     attribute: a kernel of this library may be brought up while the kernel
  *     before it in the stream is finishing, and waits (griddepcontrol.wait) before
- *     it reads or writes anything but its weights and parameters.  Stream order is
- *     unchanged for the caller: work queued before or after a call, this
- *     library's or not, sees the same results as with plain launches.  Weights,
- *     biases and normalisation parameters must not be written by the operation
- *     queued directly before a call that reads them
+ *     it reads or writes any tensor.  Stream order is unchanged for the caller: work
+ *     queued before or after a call, this library's or not, sees the same results
+ *     as with plain launches, and the weights of a call may be what the call before
+ *     it computes.  (Inside ptv3_backbone_fwd the Linear kernels fetch weights before
+ *     that wait; they start after everything queued ahead of the pass has finished)
  *
  * "Replaces" lines cite the reference implementation by its path inside the
  * reference project.

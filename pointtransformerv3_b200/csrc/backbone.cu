@@ -8,7 +8,7 @@
 // for after every block without waiting, so the next plan is launched as soon as the last one is known
 // instead of when its stage comes up.
 #include "common.cuh"
-#include "linear_small.cuh"
+#include "linear.cuh"
 #include "plan.cuh"
 #include "split_f32.cuh"
 #include <string.h>
@@ -202,7 +202,8 @@ int Pass::finest()
     BB_STEP(ptv3_argsort_inverse(a_.code, a_.k, a_.n, sig_bits, a_.order, a_.inverse, a_.status, sort_ws, sort_bytes,
                                  side_));
     BB_CUDA(events_.record(side_, &sorted));
-    // main stream, beside them: the voxel index that the stem and the 3x3x3 kernel map share
+    // main stream, beside them: the voxel index that the stem and the 3x3x3 kernel map share.  (Its first
+    // kernel is an ordinary launch: what `settled` stands on, see linear.cuh.)
     char* index_ws = mem_.take<char>(voxel_index_bytes(a_.n));
     char* wt = mem_.take<char>(conv_direct_scratch_bytes(a_.n, a_.stem_ksize));
     if (!index_ws || !wt) return out_of_memory();
@@ -319,7 +320,7 @@ int Pass::block(const ptv3_stage_args& st, int j, BbLevel& l, const void* conv_i
     BB_STEP(need_ws(bytes));
     b.workspace = ws_;
     b.workspace_bytes = bytes;
-    BB_STEP(ptv3_block_fwd(&b, main_));
+    BB_STEP(block_fwd(&b, true, main_));
     return take_plan(false);
 }
 
@@ -327,8 +328,8 @@ int Pass::block(const ptv3_stage_args& st, int j, BbLevel& l, const void* conv_i
 int Pass::project(const void* x, const void* w, const void* bias, int64_t n, int c_in, int c_out, void* split, void* out)
 {
     BB_STEP(launch_split_f32((const float*)x, n, c_in, false, split, main_));
-    return launch_linear_split(split, w, (const float*)bias, nullptr, (float*)out, nullptr, n, c_in, c_out, 0, a_.status,
-                               main_);
+    return launch_linear_split(split, w, (const float*)bias, nullptr, (float*)out, nullptr, n, c_in, c_out, 0, true,
+                               a_.status, main_);
 }
 
 int Pass::encoder(int s)
@@ -349,11 +350,11 @@ int Pass::encoder(int s)
             BB_STEP(ptv3_pool_fwd(ws_ + split, nullptr, p.order, p.idx_ptr, l.n, st.c_out, st.scale, st.shift, pooled,
                                   nullptr, st.reduce, a_.dtype, main_));
         } else {
-        const size_t bytes = ptv3_pool_stage_workspace_bytes(p.n, st.c_out);
-        BB_STEP(need_ws(bytes));
-        BB_STEP(ptv3_pool_stage_fwd(p.feat, st.w, st.b, nullptr, p.order, p.idx_ptr, p.n, l.n, st.c_in, st.c_out,
-                                    st.scale, st.shift, pooled, nullptr, st.reduce, PTV3_DTYPE_BF16, a_.status, ws_,
-                                    bytes, main_));
+            const size_t bytes = ptv3_pool_stage_workspace_bytes(p.n, st.c_out);
+            BB_STEP(need_ws(bytes));
+            BB_STEP(pool_stage_fwd(p.feat, st.w, st.b, nullptr, p.order, p.idx_ptr, p.n, l.n, st.c_in, st.c_out, st.scale,
+                                   st.shift, pooled, nullptr, st.reduce, PTV3_DTYPE_BF16, true, a_.status, ws_, bytes,
+                                   main_));
         }
         x = pooled;
     }
@@ -393,9 +394,9 @@ int Pass::decoder(int d)
     } else {
         const size_t bytes = ptv3_unpool_stage_workspace_bytes(l.n, c.n, st.c_out);
         BB_STEP(need_ws(bytes));
-        BB_STEP(ptv3_unpool_stage_fwd(l.feat, c.feat, st.w_skip, st.b_skip, st.w, st.b, l.cluster, l.n, c.n, st.c_skip,
-                                      st.c_in, st.c_out, st.scale_skip, st.shift_skip, st.scale, st.shift, buf[0], act,
-                                      PTV3_DTYPE_BF16, a_.status, ws_, bytes, main_));
+        BB_STEP(unpool_stage_fwd(l.feat, c.feat, st.w_skip, st.b_skip, st.w, st.b, l.cluster, l.n, c.n, st.c_skip, st.c_in,
+                                 st.c_out, st.scale_skip, st.shift_skip, st.scale, st.shift, buf[0], act, PTV3_DTYPE_BF16,
+                                 true, a_.status, ws_, bytes, main_));
     }
     const void *x = buf[0], *conv_in = act;
     for (int j = 0; j < st.n_blocks; ++j) {

@@ -15,7 +15,7 @@
 // streamed-weight tensor-core kernel (gemm_tc05.cu) and the fused row kernel for the glue.
 #include "common.cuh"
 #include "conv_mma.cuh"
-#include "linear_small.cuh"
+#include "linear.cuh"
 #include "split_f32.cuh"
 #include "vec.cuh"
 
@@ -30,14 +30,14 @@ static bool linear_any_supported(int k, int n_out, bool epilogue)
 }
 
 static int linear_any(const void* x, const void* w, const void* bias, const void* residual, void* out, int64_t n,
-                      int k, int n_out, int gelu, uint32_t* status, void* stream)
+                      int k, int n_out, int gelu, bool settled, uint32_t* status, cudaStream_t stream)
 {
     if (linear_small_wanted(n, k, n_out))
-        return launch_linear_small(x, w, bias, residual, out, n, k, n_out, gelu, status, (cudaStream_t)stream);
+        return launch_linear_small(x, w, bias, residual, out, n, k, n_out, gelu, settled, status, stream);
     if (ptv3_gemm_supported(k, n_out, PTV3_DTYPE_BF16))
-        return ptv3_gemm_fwd(x, w, bias, residual, out, n, k, n_out, gelu, PTV3_DTYPE_BF16, status, stream);
+        return gemm_fwd(x, w, bias, residual, out, n, k, n_out, gelu, PTV3_DTYPE_BF16, settled, status, stream);
     if (!gelu && !residual && ptv3_linear_supported(k, n_out, 0, PTV3_DTYPE_BF16))
-        return ptv3_linear_fwd(x, w, bias, out, n, k, n_out, PTV3_DTYPE_BF16, status, stream);
+        return linear_fwd(x, w, bias, out, n, k, n_out, PTV3_DTYPE_BF16, settled, status, stream);
     set_error("no tensor-core Linear kernel for %d -> %d channels", k, n_out);
     return PTV3_ERR_UNSUPPORTED;
 }
@@ -99,7 +99,7 @@ static size_t carve_block_f32(const ptv3_block_args* a, void* base, BlockBuffers
     return c.off;
 }
 
-static int block_f32(const ptv3_block_args* a, cudaStream_t stream)
+static int block_f32(const ptv3_block_args* a, bool settled, cudaStream_t stream)
 {
     BlockBuffersF32 b;
     carve_block_f32(a, a->workspace, &b);
@@ -116,21 +116,21 @@ static int block_f32(const ptv3_block_args* a, cudaStream_t stream)
     STEP(launch_split_f32(f(a->conv_in), n, C, false, b.sh, stream));
     STEP(launch_conv_split(b.sh, a->nbr, a->conv_weight, f(a->conv_bias), nullptr, b.s, a->row_order, n, C, C, 27, a->status,
                            stream));
-    STEP(launch_linear_split(b.s, a->cpe_w, f(a->cpe_b), nullptr, b.y, nullptr, n, C, C, 0, a->status, stream));
+    STEP(launch_linear_split(b.s, a->cpe_w, f(a->cpe_b), nullptr, b.y, nullptr, n, C, C, 0, settled, a->status, stream));
     STEP(ptv3_add_layernorm_fwd(b.y, a->feat, a->cpe_ln_w, a->cpe_ln_b, a->cpe_ln_eps, b.f1, a->n1_w, a->n1_b, a->n1_eps, b.a,
                                 n, C, PTV3_DTYPE_F32, stream));
     STEP(launch_split_f32(b.a, n, C, false, b.s, stream));
-    STEP(launch_linear_split(b.s, a->qkv_w, f(a->qkv_b), nullptr, b.qkv, nullptr, n, C, 3 * C, 0, a->status, stream));
+    STEP(launch_linear_split(b.s, a->qkv_w, f(a->qkv_b), nullptr, b.qkv, nullptr, n, C, 3 * C, 0, settled, a->status, stream));
     STEP(ptv3_attention_fwd(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.att, n, a->n_seq, a->max_seqlen, C, a->heads,
                             a->scale, PTV3_DTYPE_F32, a->attention_algo, a->status, stream));
     STEP(launch_split_f32(b.att, n, C, false, b.s, stream));
     // (b.a is free until the second norm)
-    STEP(launch_linear_split(b.s, a->proj_w, f(a->proj_b), nullptr, b.qkv, nullptr, n, C, C, 0, a->status, stream));
+    STEP(launch_linear_split(b.s, a->proj_w, f(a->proj_b), nullptr, b.qkv, nullptr, n, C, C, 0, settled, a->status, stream));
     STEP(ptv3_add_layernorm_fwd(b.qkv, b.f1, nullptr, nullptr, 0.f, b.f2, a->n2_w, a->n2_b, a->n2_eps, b.a, n, C,
                                 PTV3_DTYPE_F32, stream));
     STEP(launch_split_f32(b.a, n, C, false, b.s, stream));
-    STEP(launch_linear_split(b.s, a->fc1_w, f(a->fc1_b), nullptr, nullptr, b.sh, n, C, H, 1, a->status, stream));
-    STEP(launch_linear_split(b.sh, a->fc2_w, f(a->fc2_b), b.f2, (float*)a->out, nullptr, n, H, C, 0, a->status, stream));
+    STEP(launch_linear_split(b.s, a->fc1_w, f(a->fc1_b), nullptr, nullptr, b.sh, n, C, H, 1, settled, a->status, stream));
+    STEP(launch_linear_split(b.sh, a->fc2_w, f(a->fc2_b), b.f2, (float*)a->out, nullptr, n, H, C, 0, settled, a->status, stream));
 #undef STEP
     return PTV3_OK;
 }
@@ -140,6 +140,129 @@ int block_f32_supported(int channels, int heads, int hidden)
     const int d = heads > 0 && channels % heads == 0 ? channels / heads : 0;
     return channels >= 32 && channels <= 1024 && (channels & (channels - 1)) == 0 && hidden % 32 == 0 && hidden >= channels &&
            (d == 8 || d == 16 || d == 32 || d == 64);
+}
+
+int block_fwd(const ptv3_block_args* a, bool settled, cudaStream_t stream)
+{
+    PTV3_REQUIRE(a != nullptr, PTV3_ERR_INVALID_ARGUMENT, "ptv3_block_fwd: null argument block");
+    const bool f32 = a->dtype == PTV3_DTYPE_F32 && block_f32_supported(a->channels, a->heads, a->hidden) && a->nbr;
+    PTV3_REQUIRE(f32 || ptv3_block_supported(a->channels, a->heads, a->hidden, a->dtype), PTV3_ERR_UNSUPPORTED,
+                 "ptv3_block_fwd: bf16 (or fp32 with split weights), channels and hidden multiples of 16 (got %d, %d, dtype %d)",
+                 a->channels, a->hidden, a->dtype);
+    PTV3_REQUIRE(a->n >= 0, PTV3_ERR_INVALID_ARGUMENT, "ptv3_block_fwd: n < 0");
+    if (a->n == 0) return PTV3_OK;
+    PTV3_REQUIRE(a->conv_in && a->feat && a->out && a->status && a->workspace && a->conv_weight && a->cpe_w &&
+                     a->cpe_b && a->cpe_ln_w && a->cpe_ln_b && a->n1_w && a->n1_b && a->qkv_w && a->qkv_b &&
+                     a->proj_w && a->proj_b && a->n2_w && a->n2_b && a->fc1_w && a->fc1_b && a->fc2_w &&
+                     a->fc2_b && a->order && a->pad && a->unpad && a->cu_seqlens && (a->nbr || a->pair_in),
+                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_block_fwd: null pointer");
+    PTV3_REQUIRE(a->workspace_bytes >= ptv3_block_workspace_bytes(a), PTV3_ERR_INVALID_ARGUMENT,
+                 "ptv3_block_fwd: workspace of %zu bytes, %zu needed", a->workspace_bytes, ptv3_block_workspace_bytes(a));
+    if (f32) return block_f32(a, settled, stream);
+    BlockBuffers b;
+    carve_block(a, a->workspace, &b);
+    const int C = a->channels, dt = a->dtype;
+    const int64_t n = a->n;
+    int rc;
+#define STEP(call)               \
+    do {                         \
+        rc = (call);             \
+        if (rc != PTV3_OK) return rc; \
+    } while (0)
+
+    // xCPE convolution
+    if (a->pair_in)
+        STEP(ptv3_subm_conv_pairs_fwd(a->conv_in, a->pair_in, a->pair_out, a->off_start, a->tile_start,
+                                      a->conv_weight, a->conv_bias, b.x, b.acc32, (size_t)n * C * 8, n, C, C, 27,
+                                      dt, stream));
+    else
+        STEP(ptv3_subm_conv_fwd(a->conv_in, a->nbr, a->conv_weight, a->conv_bias, b.x, a->row_order, n, C, C, 27,
+                                dt, 0, a->status, stream));
+
+    const bool tc_lin = ptv3_linear_supported(C, C, 1, dt) && ptv3_linear_supported(C, 3 * C, 0, dt);
+    if (tc_lin) {
+        STEP(linear_ln_fwd(b.x, a->cpe_w, a->cpe_b, a->feat, a->cpe_ln_w, a->cpe_ln_b, a->cpe_ln_eps, b.f1, a->n1_w,
+                           a->n1_b, a->n1_eps, b.a, n, C, dt, settled, a->status, stream));
+        STEP(linear_fwd(b.a, a->qkv_w, a->qkv_b, b.qkv, n, C, 3 * C, dt, settled, a->status, stream));
+    } else {
+        // streamed-weight Linear, then f1 = feat + LN_cpe(.), a = LN_1(f1) in the fused row kernel
+        // (the qkv buffer is free here and serves as the Linear's output)
+        STEP(linear_any(b.x, a->cpe_w, a->cpe_b, nullptr, b.qkv, n, C, C, 0, settled, a->status, stream));
+        STEP(ptv3_add_layernorm_fwd(b.qkv, a->feat, a->cpe_ln_w, a->cpe_ln_b, a->cpe_ln_eps, b.f1, a->n1_w, a->n1_b,
+                                    a->n1_eps, b.a, n, C, dt, stream));
+        STEP(linear_any(b.a, a->qkv_w, a->qkv_b, nullptr, b.qkv, n, C, 3 * C, 0, settled, a->status, stream));
+    }
+    STEP(ptv3_attention_fwd(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.att, n, a->n_seq, a->max_seqlen, C,
+                            a->heads, a->scale, dt, a->attention_algo, a->status, stream));
+    const bool fused_mlp = use_fused_mlp(n, C, a->hidden, dt);
+    if (tc_lin) {
+        STEP(linear_ln_fwd(b.att, a->proj_w, a->proj_b, b.f1, nullptr, nullptr, 0.f, b.f2, a->n2_w, a->n2_b, a->n2_eps,
+                           b.a, n, C, dt, settled, a->status, stream));
+    } else {
+        STEP(linear_any(b.att, a->proj_w, a->proj_b, nullptr, b.qkv, n, C, C, 0, settled, a->status, stream));
+        STEP(ptv3_add_layernorm_fwd(b.qkv, b.f1, nullptr, nullptr, 0.f, b.f2, a->n2_w, a->n2_b, a->n2_eps, b.a, n, C,
+                                    dt, stream));
+    }
+    if (fused_mlp) {
+        STEP(mlp_fwd(b.a, a->fc1_w, a->fc1_b, a->fc2_w, a->fc2_b, b.f2, a->out, n, C, a->hidden, dt, settled, a->status,
+                     stream));
+    } else {
+        // hidden = GELU(fc1(b)), out = f2 + fc2(hidden): bias, activation and residual in the epilogues
+        STEP(linear_any(b.a, a->fc1_w, a->fc1_b, nullptr, b.hidden, n, C, a->hidden, 1, settled, a->status, stream));
+        STEP(linear_any(b.hidden, a->fc2_w, a->fc2_b, b.f2, a->out, n, a->hidden, C, 0, settled, a->status, stream));
+    }
+#undef STEP
+    return PTV3_OK;
+}
+
+int pool_stage_fwd(const void* x, const void* weight, const void* bias, const float* coord, const int64_t* indices,
+                   const int64_t* idx_ptr, int64_t n, int64_t m, int c_in, int c_out, const float* bn_scale,
+                   const float* bn_shift, void* out, float* coord_out, int reduce, int dtype, bool settled,
+                   uint32_t* status, void* workspace, size_t workspace_bytes, cudaStream_t stream)
+{
+    PTV3_REQUIRE(ptv3_pool_stage_supported(c_in, c_out, dtype), PTV3_ERR_UNSUPPORTED,
+                 "ptv3_pool_stage_fwd: bf16 only, and a projection %d -> %d that one of the tensor-core Linear "
+                 "kernels takes", c_in, c_out);
+    PTV3_REQUIRE(n >= 0 && m >= 0, PTV3_ERR_INVALID_ARGUMENT, "ptv3_pool_stage_fwd: bad sizes");
+    if (n == 0 || m == 0) return PTV3_OK;
+    PTV3_REQUIRE(x && weight && bias && indices && idx_ptr && out && workspace && status,
+                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_pool_stage_fwd: null pointer");
+    PTV3_REQUIRE(workspace_bytes >= ptv3_pool_stage_workspace_bytes(n, c_out), PTV3_ERR_WORKSPACE,
+                 "ptv3_pool_stage_fwd: workspace too small");
+    Carver cv(workspace);
+    char* proj = cv.take<char>((size_t)n * c_out * 2);
+    int rc = linear_any(x, weight, bias, nullptr, proj, n, c_in, c_out, 0, settled, status, stream);
+    if (rc != PTV3_OK) return rc;
+    return ptv3_pool_fwd(proj, coord, indices, idx_ptr, m, c_out, bn_scale, bn_shift, out, coord_out, reduce, dtype,
+                         stream);
+}
+
+int unpool_stage_fwd(const void* skip_feat, const void* child_feat, const void* w_skip, const void* b_skip,
+                     const void* w_child, const void* b_child, const int64_t* cluster, int64_t n, int64_t m, int c_skip,
+                     int c_child, int c_out, const float* skip_scale, const float* skip_shift, const float* child_scale,
+                     const float* child_shift, void* out, void* skip_act, int dtype, bool settled, uint32_t* status,
+                     void* workspace, size_t workspace_bytes, cudaStream_t stream)
+{
+    PTV3_REQUIRE(ptv3_pool_stage_supported(c_skip, c_out, dtype) && ptv3_pool_stage_supported(c_child, c_out, dtype),
+                 PTV3_ERR_UNSUPPORTED,
+                 "ptv3_unpool_stage_fwd: bf16 only, and projections %d -> %d, %d -> %d that the tensor-core Linear "
+                 "kernels take", c_skip, c_out, c_child, c_out);
+    PTV3_REQUIRE(n >= 0 && m >= 0, PTV3_ERR_INVALID_ARGUMENT, "ptv3_unpool_stage_fwd: bad sizes");
+    if (n == 0) return PTV3_OK;
+    PTV3_REQUIRE(m > 0 && skip_feat && child_feat && w_skip && b_skip && w_child && b_child && cluster && out &&
+                     workspace && status,
+                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_unpool_stage_fwd: null pointer or empty coarse level");
+    PTV3_REQUIRE(workspace_bytes >= ptv3_unpool_stage_workspace_bytes(n, m, c_out), PTV3_ERR_WORKSPACE,
+                 "ptv3_unpool_stage_fwd: workspace too small");
+    Carver cv(workspace);
+    char* skip_lin = cv.take<char>((size_t)n * c_out * 2);
+    char* child_lin = cv.take<char>((size_t)m * c_out * 2);
+    int rc = linear_any(child_feat, w_child, b_child, nullptr, child_lin, m, c_child, c_out, 0, settled, status, stream);
+    if (rc != PTV3_OK) return rc;
+    rc = linear_any(skip_feat, w_skip, b_skip, nullptr, skip_lin, n, c_skip, c_out, 0, settled, status, stream);
+    if (rc != PTV3_OK) return rc;
+    return ptv3_unpool_fwd(skip_lin, child_lin, cluster, n, c_out, skip_scale, skip_shift, child_scale, child_shift,
+                           out, skip_act, dtype, stream);
 }
 
 }  // namespace ptv3
@@ -170,78 +293,9 @@ extern "C" size_t ptv3_block_workspace_bytes(const ptv3_block_args* a)
     return a->dtype == PTV3_DTYPE_F32 ? carve_block_f32(a, nullptr, nullptr) : carve_block(a, nullptr, nullptr);
 }
 
-extern "C" int ptv3_block_fwd(const ptv3_block_args* a, void* stream_)
+extern "C" int ptv3_block_fwd(const ptv3_block_args* a, void* stream)
 {
-    PTV3_REQUIRE(a != nullptr, PTV3_ERR_INVALID_ARGUMENT, "ptv3_block_fwd: null argument block");
-    const bool f32 = a->dtype == PTV3_DTYPE_F32 && block_f32_supported(a->channels, a->heads, a->hidden) && a->nbr;
-    PTV3_REQUIRE(f32 || ptv3_block_supported(a->channels, a->heads, a->hidden, a->dtype), PTV3_ERR_UNSUPPORTED,
-                 "ptv3_block_fwd: bf16 (or fp32 with split weights), channels and hidden multiples of 16 (got %d, %d, dtype %d)",
-                 a->channels, a->hidden, a->dtype);
-    PTV3_REQUIRE(a->n >= 0, PTV3_ERR_INVALID_ARGUMENT, "ptv3_block_fwd: n < 0");
-    if (a->n == 0) return PTV3_OK;
-    PTV3_REQUIRE(a->conv_in && a->feat && a->out && a->status && a->workspace && a->conv_weight && a->cpe_w &&
-                     a->cpe_b && a->cpe_ln_w && a->cpe_ln_b && a->n1_w && a->n1_b && a->qkv_w && a->qkv_b &&
-                     a->proj_w && a->proj_b && a->n2_w && a->n2_b && a->fc1_w && a->fc1_b && a->fc2_w &&
-                     a->fc2_b && a->order && a->pad && a->unpad && a->cu_seqlens && (a->nbr || a->pair_in),
-                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_block_fwd: null pointer");
-    PTV3_REQUIRE(a->workspace_bytes >= ptv3_block_workspace_bytes(a), PTV3_ERR_INVALID_ARGUMENT,
-                 "ptv3_block_fwd: workspace of %zu bytes, %zu needed", a->workspace_bytes, ptv3_block_workspace_bytes(a));
-    cudaStream_t stream = (cudaStream_t)stream_;
-    if (f32) return block_f32(a, stream);
-    BlockBuffers b;
-    carve_block(a, a->workspace, &b);
-    const int C = a->channels, dt = a->dtype;
-    const int64_t n = a->n;
-    int rc;
-#define STEP(call)               \
-    do {                         \
-        rc = (call);             \
-        if (rc != PTV3_OK) return rc; \
-    } while (0)
-
-    // xCPE convolution
-    if (a->pair_in)
-        STEP(ptv3_subm_conv_pairs_fwd(a->conv_in, a->pair_in, a->pair_out, a->off_start, a->tile_start,
-                                      a->conv_weight, a->conv_bias, b.x, b.acc32, (size_t)n * C * 8, n, C, C, 27,
-                                      dt, stream_));
-    else
-        STEP(ptv3_subm_conv_fwd(a->conv_in, a->nbr, a->conv_weight, a->conv_bias, b.x, a->row_order, n, C, C, 27,
-                                dt, 0, a->status, stream_));
-
-    const bool tc_lin = ptv3_linear_supported(C, C, 1, dt) && ptv3_linear_supported(C, 3 * C, 0, dt);
-    if (tc_lin) {
-        STEP(ptv3_linear_ln_fwd(b.x, a->cpe_w, a->cpe_b, a->feat, a->cpe_ln_w, a->cpe_ln_b, a->cpe_ln_eps, b.f1,
-                                a->n1_w, a->n1_b, a->n1_eps, b.a, n, C, dt, a->status, stream_));
-        STEP(ptv3_linear_fwd(b.a, a->qkv_w, a->qkv_b, b.qkv, n, C, 3 * C, dt, a->status, stream_));
-    } else {
-        // streamed-weight Linear, then f1 = feat + LN_cpe(.), a = LN_1(f1) in the fused row kernel
-        // (the qkv buffer is free here and serves as the Linear's output)
-        STEP(linear_any(b.x, a->cpe_w, a->cpe_b, nullptr, b.qkv, n, C, C, 0, a->status, stream_));
-        STEP(ptv3_add_layernorm_fwd(b.qkv, a->feat, a->cpe_ln_w, a->cpe_ln_b, a->cpe_ln_eps, b.f1, a->n1_w, a->n1_b,
-                                    a->n1_eps, b.a, n, C, dt, stream_));
-        STEP(linear_any(b.a, a->qkv_w, a->qkv_b, nullptr, b.qkv, n, C, 3 * C, 0, a->status, stream_));
-    }
-    STEP(ptv3_attention_fwd(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.att, n, a->n_seq, a->max_seqlen, C,
-                            a->heads, a->scale, dt, a->attention_algo, a->status, stream_));
-    const bool fused_mlp = use_fused_mlp(n, C, a->hidden, dt);
-    if (tc_lin) {
-        STEP(ptv3_linear_ln_fwd(b.att, a->proj_w, a->proj_b, b.f1, nullptr, nullptr, 0.f, b.f2, a->n2_w, a->n2_b,
-                                a->n2_eps, b.a, n, C, dt, a->status, stream_));
-    } else {
-        STEP(linear_any(b.att, a->proj_w, a->proj_b, nullptr, b.qkv, n, C, C, 0, a->status, stream_));
-        STEP(ptv3_add_layernorm_fwd(b.qkv, b.f1, nullptr, nullptr, 0.f, b.f2, a->n2_w, a->n2_b, a->n2_eps, b.a, n, C,
-                                    dt, stream_));
-    }
-    if (fused_mlp) {
-        STEP(ptv3_mlp_fwd(b.a, a->fc1_w, a->fc1_b, a->fc2_w, a->fc2_b, b.f2, a->out, n, C, a->hidden, dt, a->status,
-                          stream_));
-    } else {
-        // hidden = GELU(fc1(b)), out = f2 + fc2(hidden): bias, activation and residual in the epilogues
-        STEP(linear_any(b.a, a->fc1_w, a->fc1_b, nullptr, b.hidden, n, C, a->hidden, 1, a->status, stream_));
-        STEP(linear_any(b.hidden, a->fc2_w, a->fc2_b, b.f2, a->out, n, a->hidden, C, 0, a->status, stream_));
-    }
-#undef STEP
-    return PTV3_OK;
+    return block_fwd(a, false, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -265,21 +319,8 @@ extern "C" int ptv3_pool_stage_fwd(const void* x, const void* weight, const void
                                    float* coord_out, int reduce, int dtype, uint32_t* status, void* workspace,
                                    size_t workspace_bytes, void* stream)
 {
-    PTV3_REQUIRE(ptv3_pool_stage_supported(c_in, c_out, dtype), PTV3_ERR_UNSUPPORTED,
-                 "ptv3_pool_stage_fwd: bf16 only, and a projection %d -> %d that one of the tensor-core Linear "
-                 "kernels takes", c_in, c_out);
-    PTV3_REQUIRE(n >= 0 && m >= 0, PTV3_ERR_INVALID_ARGUMENT, "ptv3_pool_stage_fwd: bad sizes");
-    if (n == 0 || m == 0) return PTV3_OK;
-    PTV3_REQUIRE(x && weight && bias && indices && idx_ptr && out && workspace && status,
-                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_pool_stage_fwd: null pointer");
-    PTV3_REQUIRE(workspace_bytes >= ptv3_pool_stage_workspace_bytes(n, c_out), PTV3_ERR_WORKSPACE,
-                 "ptv3_pool_stage_fwd: workspace too small");
-    Carver cv(workspace);
-    char* proj = cv.take<char>((size_t)n * c_out * 2);
-    int rc = linear_any(x, weight, bias, nullptr, proj, n, c_in, c_out, 0, status, stream);
-    if (rc != PTV3_OK) return rc;
-    return ptv3_pool_fwd(proj, coord, indices, idx_ptr, m, c_out, bn_scale, bn_shift, out, coord_out, reduce, dtype,
-                         stream);
+    return pool_stage_fwd(x, weight, bias, coord, indices, idx_ptr, n, m, c_in, c_out, bn_scale, bn_shift, out, coord_out,
+                          reduce, dtype, false, status, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 extern "C" size_t ptv3_unpool_stage_workspace_bytes(int64_t n, int64_t m, int c_out)
@@ -296,26 +337,9 @@ extern "C" int ptv3_unpool_stage_fwd(const void* skip_feat, const void* child_fe
                                      void* skip_act, int dtype, uint32_t* status, void* workspace,
                                      size_t workspace_bytes, void* stream)
 {
-    PTV3_REQUIRE(ptv3_pool_stage_supported(c_skip, c_out, dtype) && ptv3_pool_stage_supported(c_child, c_out, dtype),
-                 PTV3_ERR_UNSUPPORTED,
-                 "ptv3_unpool_stage_fwd: bf16 only, and projections %d -> %d, %d -> %d that the tensor-core Linear "
-                 "kernels take", c_skip, c_out, c_child, c_out);
-    PTV3_REQUIRE(n >= 0 && m >= 0, PTV3_ERR_INVALID_ARGUMENT, "ptv3_unpool_stage_fwd: bad sizes");
-    if (n == 0) return PTV3_OK;
-    PTV3_REQUIRE(m > 0 && skip_feat && child_feat && w_skip && b_skip && w_child && b_child && cluster && out &&
-                     workspace && status,
-                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_unpool_stage_fwd: null pointer or empty coarse level");
-    PTV3_REQUIRE(workspace_bytes >= ptv3_unpool_stage_workspace_bytes(n, m, c_out), PTV3_ERR_WORKSPACE,
-                 "ptv3_unpool_stage_fwd: workspace too small");
-    Carver cv(workspace);
-    char* skip_lin = cv.take<char>((size_t)n * c_out * 2);
-    char* child_lin = cv.take<char>((size_t)m * c_out * 2);
-    int rc = linear_any(child_feat, w_child, b_child, nullptr, child_lin, m, c_child, c_out, 0, status, stream);
-    if (rc != PTV3_OK) return rc;
-    rc = linear_any(skip_feat, w_skip, b_skip, nullptr, skip_lin, n, c_skip, c_out, 0, status, stream);
-    if (rc != PTV3_OK) return rc;
-    return ptv3_unpool_fwd(skip_lin, child_lin, cluster, n, c_out, skip_scale, skip_shift, child_scale, child_shift,
-                           out, skip_act, dtype, stream);
+    return unpool_stage_fwd(skip_feat, child_feat, w_skip, b_skip, w_child, b_child, cluster, n, m, c_skip, c_child, c_out,
+                            skip_scale, skip_shift, child_scale, child_shift, out, skip_act, dtype, false, status,
+                            workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 extern "C" int ptv3_linear_split_fwd(const void* x_split, const void* w_split, const float* bias, const float* residual,
@@ -328,7 +352,7 @@ extern "C" int ptv3_linear_split_fwd(const void* x_split, const void* w_split, c
     PTV3_REQUIRE(x_split && w_split && out && status &&
                      (((uintptr_t)x_split | (uintptr_t)w_split | (uintptr_t)out | (uintptr_t)residual) & 15) == 0,
                  PTV3_ERR_INVALID_ARGUMENT, "ptv3_linear_split_fwd: null pointer or alignment");
-    return launch_linear_split(x_split, w_split, bias, residual, out, nullptr, n, k, n_out, gelu, status,
+    return launch_linear_split(x_split, w_split, bias, residual, out, nullptr, n, k, n_out, gelu, false, status,
                                (cudaStream_t)stream);
 }
 

@@ -22,7 +22,7 @@
 // the residual sum rounded again).  Every mbarrier wait is bounded and reports through the
 // status word.
 #include "common.cuh"
-#include "linear_small.cuh"
+#include "linear.cuh"
 #include "tc05.cuh"
 #include "vec.cuh"
 #include "mma_util.cuh"
@@ -50,6 +50,7 @@ struct GemmArgs {
     int k, n_out;
     int gelu;
     int row_tiles, col_tiles;
+    bool settled;                    // see linear.cuh
     uint32_t* status;
 };
 
@@ -124,8 +125,9 @@ __global__ void __launch_bounds__(64 + gm_epi_warps(MODE) * 32, 1) gemm_tc05_ker
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     bool ok = true;
+    if (WRES && !a.settled) pdl_wait();
     if (WRES && tid == 0) {
-        // the weights are not written by the launch before this one: fetched ahead of the wait below
+        // the weights are settled: fetched ahead of the wait below
         int row0, col0;
         tile_at(0, row0, col0);
         mbar_expect_tx(wbar, (uint32_t)w_bytes);
@@ -337,6 +339,31 @@ static int launch_gemm(const void* x, const void* w, GemmArgs a, cudaStream_t st
     return launch_gemm_as<128, 6, false>(mx, mw, mo, a, stream);
 }
 
+int gemm_fwd(const void* x, const void* weight, const void* bias, const void* residual, void* out, int64_t n, int k,
+             int n_out, int gelu, int dtype, bool settled, uint32_t* status, cudaStream_t stream)
+{
+    PTV3_REQUIRE(n >= 0 && n < (1ll << 31), PTV3_ERR_INVALID_ARGUMENT, "ptv3_gemm_fwd: bad n");
+    PTV3_REQUIRE(ptv3_gemm_supported(k, n_out, dtype), PTV3_ERR_UNSUPPORTED,
+                 "ptv3_gemm_fwd: supported: bf16, k a multiple of 64, n_out a multiple of 128 (got %d, %d)", k, n_out);
+    if (n == 0) return PTV3_OK;
+    PTV3_REQUIRE(x && weight && out && status, PTV3_ERR_INVALID_ARGUMENT, "ptv3_gemm_fwd: null pointer");
+    PTV3_REQUIRE((((uintptr_t)x | (uintptr_t)weight | (uintptr_t)out | (uintptr_t)bias | (uintptr_t)residual) & 15) == 0,
+                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_gemm_fwd: tensors must be 16-byte aligned");
+    if (linear_small_wanted(n, k, n_out))
+        return launch_linear_small(x, weight, bias, residual, out, n, k, n_out, gelu, settled, status, stream);
+    GemmArgs a{};
+    a.bias = (const __nv_bfloat16*)bias;
+    a.residual = (const __nv_bfloat16*)residual;
+    a.out = (__nv_bfloat16*)out;
+    a.n = n;
+    a.k = k;
+    a.n_out = n_out;
+    a.gelu = gelu ? 1 : 0;
+    a.settled = settled;
+    a.status = status;
+    return launch_gemm(x, weight, a, stream);
+}
+
 }  // namespace ptv3
 
 extern "C" int ptv3_gemm_supported(int k, int n_out, int dtype)
@@ -347,24 +374,5 @@ extern "C" int ptv3_gemm_supported(int k, int n_out, int dtype)
 extern "C" int ptv3_gemm_fwd(const void* x, const void* weight, const void* bias, const void* residual, void* out,
                              int64_t n, int k, int n_out, int gelu, int dtype, uint32_t* status, void* stream)
 {
-    using namespace ptv3;
-    PTV3_REQUIRE(n >= 0 && n < (1ll << 31), PTV3_ERR_INVALID_ARGUMENT, "ptv3_gemm_fwd: bad n");
-    PTV3_REQUIRE(ptv3_gemm_supported(k, n_out, dtype), PTV3_ERR_UNSUPPORTED,
-                 "ptv3_gemm_fwd: supported: bf16, k a multiple of 64, n_out a multiple of 128 (got %d, %d)", k, n_out);
-    if (n == 0) return PTV3_OK;
-    PTV3_REQUIRE(x && weight && out && status, PTV3_ERR_INVALID_ARGUMENT, "ptv3_gemm_fwd: null pointer");
-    PTV3_REQUIRE((((uintptr_t)x | (uintptr_t)weight | (uintptr_t)out | (uintptr_t)bias | (uintptr_t)residual) & 15) == 0,
-                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_gemm_fwd: tensors must be 16-byte aligned");
-    if (linear_small_wanted(n, k, n_out))
-        return launch_linear_small(x, weight, bias, residual, out, n, k, n_out, gelu, status, (cudaStream_t)stream);
-    GemmArgs a{};
-    a.bias = (const __nv_bfloat16*)bias;
-    a.residual = (const __nv_bfloat16*)residual;
-    a.out = (__nv_bfloat16*)out;
-    a.n = n;
-    a.k = k;
-    a.n_out = n_out;
-    a.gelu = gelu ? 1 : 0;
-    a.status = status;
-    return launch_gemm(x, weight, a, (cudaStream_t)stream);
+    return ptv3::gemm_fwd(x, weight, bias, residual, out, n, k, n_out, gelu, dtype, false, status, (cudaStream_t)stream);
 }

@@ -1,0 +1,53 @@
+// Linear layers as the one-call block and backbone queue them (linear_small.cu, linear_tc05.cu, gemm_tc05.cu,
+// mlp_tc05.cu, block.cu): the entry points of the same names, with what the caller knows of the weights.
+//
+// `settled`: nothing in flight on the stream writes weights, biases or norm parameters.  The kernels then fetch
+// them before they wait for the launch ahead of them.  That holds inside ptv3_backbone_fwd, whose first kernel on
+// the stream is an ordinary launch: it starts when everything before it has finished, and every later kernel
+// starts after it.  An entry point of its own cannot know: its weights may be what the call before it
+// computes, and a distance of several launches does not help, because launches in between let theirs start early too.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "../../include/ptv3_b200.h"
+
+namespace ptv3 {
+
+// Whether the short form (linear_small.cu) is the faster one for n rows; bf16, 16-byte aligned rows
+bool linear_small_wanted(int64_t n, int k, int n_out);
+
+// out = [residual +] act(x W^T + b) by the short form
+int launch_linear_small(const void* x, const void* w, const void* bias, const void* residual, void* out, int64_t n, int k,
+                        int n_out, int gelu, bool settled, uint32_t* status, cudaStream_t stream);
+
+// fp32 Linear on split operands (split_f32.cuh); k and n_out multiples of 32.  The result goes to `out`, or as
+// split rows to `split_out`.
+int launch_linear_split(const void* xs, const void* ws, const float* bias, const float* residual, float* out,
+                        void* split_out, int64_t n, int k, int n_out, int gelu, bool settled, uint32_t* status,
+                        cudaStream_t stream);
+
+int linear_fwd(const void* x, const void* weight, const void* bias, void* out, int64_t n, int k, int n_out, int dtype,
+               bool settled, uint32_t* status, cudaStream_t stream);
+int linear_ln_fwd(const void* x, const void* weight, const void* bias, const void* residual, const void* ln1_weight,
+                  const void* ln1_bias, float ln1_eps, void* sum_out, const void* ln2_weight, const void* ln2_bias,
+                  float ln2_eps, void* norm_out, int64_t n, int channels, int dtype, bool settled, uint32_t* status,
+                  cudaStream_t stream);
+int gemm_fwd(const void* x, const void* weight, const void* bias, const void* residual, void* out, int64_t n, int k,
+             int n_out, int gelu, int dtype, bool settled, uint32_t* status, cudaStream_t stream);
+int mlp_fwd(const void* x, const void* fc1_weight, const void* fc1_bias, const void* fc2_weight, const void* fc2_bias,
+            const void* residual, void* out, int64_t n, int channels, int hidden, int dtype, bool settled,
+            uint32_t* status, cudaStream_t stream);
+
+int block_fwd(const ptv3_block_args* a, bool settled, cudaStream_t stream);
+int pool_stage_fwd(const void* x, const void* weight, const void* bias, const float* coord, const int64_t* indices,
+                   const int64_t* idx_ptr, int64_t n, int64_t m, int c_in, int c_out, const float* bn_scale,
+                   const float* bn_shift, void* out, float* coord_out, int reduce, int dtype, bool settled,
+                   uint32_t* status, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+int unpool_stage_fwd(const void* skip_feat, const void* child_feat, const void* w_skip, const void* b_skip,
+                     const void* w_child, const void* b_child, const int64_t* cluster, int64_t n, int64_t m, int c_skip,
+                     int c_child, int c_out, const float* skip_scale, const float* skip_shift, const float* child_scale,
+                     const float* child_shift, void* out, void* skip_act, int dtype, bool settled, uint32_t* status,
+                     void* workspace, size_t workspace_bytes, cudaStream_t stream);
+
+}  // namespace ptv3

@@ -4,14 +4,15 @@
 // kernels (gemm_tc05.cu, linear_tc05.cu) give such a layer a handful of CTAs that walk all of K and then
 // spend most of their time in an epilogue of 128 or 256 columns (27 x 2048 -> 512: 15 us on four CTAs).  Here
 //   * tiles are 64 columns wide, eight warps take 32 columns of a row each;
-//   * the weights of the first chunks are on their way before the preceding kernel has finished;
+//   * the weights of the first chunks are on their way before the preceding kernel has finished (where the
+//     caller vouches for them, see linear.cuh);
 //   * long K: a cluster of up to eight CTAs takes shares of K; the partial sums meet in distributed
 //     shared memory, every CTA finishing some of the rows (in rank order: the result is the same on
 //     every run).
 // (Linear + LayerNorm stays with linear_tc05.cu, whose epilogue holds a row in registers: 1 560 x 64 5.1 us
 // against 6.5 in this form, 6 700 x 128 8.1 against 10.4.)
 #include "common.cuh"
-#include "linear_small.cuh"
+#include "linear.cuh"
 #include "split_f32.cuh"
 #include "tc05.cuh"
 #include "vec.cuh"
@@ -33,6 +34,7 @@ struct LinearSmallArgs {
     __nv_bfloat16* split_out;                          // LS_F32: the result as split rows instead
     int64_t n;
     int k, n_out, stages;
+    bool settled;                                      // see linear.cuh
     uint32_t* status;
 };
 
@@ -122,6 +124,13 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
     auto column_x = [&](int kc) { return (MODE & LS_F32) ? split_column_a(k0 / LS_BK + kc, a.k / 6) : k0 + kc * LS_BK; };
     auto column_w = [&](int kc) { return (MODE & LS_F32) ? split_column_b(k0 / LS_BK + kc, a.k / 6) : k0 + kc * LS_BK; };
 
+    // those of the first chunks: settled ones are fetched ahead of the wait below
+    auto weights = [&] {
+        for (int kc = 0; kc < nk && kc < stages; ++kc) {
+            mbar_expect_tx(full0 + 8 * kc, LS_STAGE);
+            tma_load_2d(sbase + kc * LS_STAGE + LS_A_BYTES, &map_w, column_w(kc), col0, full0 + 8 * kc);
+        }
+    };
     if (tid == 0) {
         for (int s = 0; s < stages; ++s) {
             mbar_init(full0 + 8 * s, 1);
@@ -131,16 +140,16 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
         *abort = 0;
         fence_barrier_init();
         prefetch_tensormap(&map_x);
-        // the weights are not written by the launch before this one: fetched ahead of the wait below
-        for (int kc = 0; kc < nk && kc < stages; ++kc) {
-            mbar_expect_tx(full0 + 8 * kc, LS_STAGE);
-            tma_load_2d(sbase + kc * LS_STAGE + LS_A_BYTES, &map_w, column_w(kc), col0, full0 + 8 * kc);
-        }
+        if (a.settled) weights();
     }
     if (warp == 1) {
         tmem_alloc(smem_u32_generic(tmem_slot), TM_COLS);
         // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
         pdl_launch_next();
+    }
+    if (!a.settled) {
+        pdl_wait();
+        if (tid == 0) weights();
     }
     for (int i = tid; i < LS_BN; i += LS_THREADS) {
         const int c = col0 + i;
@@ -329,7 +338,7 @@ bool linear_small_wanted(int64_t n, int k, int n_out)
 }
 
 int launch_linear_small(const void* x, const void* w, const void* bias, const void* residual, void* out, int64_t n, int k,
-                        int n_out, int gelu, uint32_t* status, cudaStream_t stream)
+                        int n_out, int gelu, bool settled, uint32_t* status, cudaStream_t stream)
 {
     LinearSmallArgs a{};
     a.bias = bias;
@@ -338,6 +347,7 @@ int launch_linear_small(const void* x, const void* w, const void* bias, const vo
     a.n = n;
     a.k = k;
     a.n_out = n_out;
+    a.settled = settled;
     a.status = status;
     const int parts = ls_parts((n + LS_BM - 1) / LS_BM * (n_out / LS_BN), k);
     switch ((gelu ? LS_GELU : 0) | (residual ? LS_RESIDUAL : 0)) {
@@ -349,7 +359,8 @@ int launch_linear_small(const void* x, const void* w, const void* bias, const vo
 }
 
 int launch_linear_split(const void* xs, const void* ws, const float* bias, const float* residual, float* out,
-                        void* split_out, int64_t n, int k, int n_out, int gelu, uint32_t* status, cudaStream_t stream)
+                        void* split_out, int64_t n, int k, int n_out, int gelu, bool settled, uint32_t* status,
+                        cudaStream_t stream)
 {
     LinearSmallArgs a{};
     a.bias = bias;
@@ -359,6 +370,7 @@ int launch_linear_split(const void* xs, const void* ws, const float* bias, const
     a.n = n;
     a.k = 6 * k;
     a.n_out = n_out;
+    a.settled = settled;
     a.status = status;
     const int parts = ls_parts((n + LS_BM - 1) / LS_BM * ((n_out + LS_BN - 1) / LS_BN), a.k);
     switch ((gelu ? LS_GELU : 0) | (residual ? LS_RESIDUAL : 0)) {

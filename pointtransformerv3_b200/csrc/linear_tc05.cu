@@ -17,7 +17,7 @@
 // rounded at the same place.  Waits are bounded.
 #include "common.cuh"
 #include "mma_util.cuh"
-#include "linear_small.cuh"
+#include "linear.cuh"
 #include "tc05.cuh"
 #include "vec.cuh"
 
@@ -34,6 +34,7 @@ struct LinearArgs {
     int nacc;         // accumulators per group in tensor memory (2 where 2 x groups x columns fit in 512)
     int w_box_rows;   // rows per TMA box of W
     int out_box;      // columns per staging tile and TMA store (64, or 32 when n_out % 64 != 0)
+    bool settled;     // see linear.cuh
     uint32_t* status;
 };
 
@@ -84,11 +85,18 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
         prefetch_tensormap(&map_x);
         prefetch_tensormap(&map_w);
     }
-    for (int i = tid; i < n_out; i += 512) bias_s[i] = a.bias ? __bfloat162float(a.bias[i]) : 0.f;
+    auto parameters = [&] {
+        for (int i = tid; i < n_out; i += 512) bias_s[i] = a.bias ? __bfloat162float(a.bias[i]) : 0.f;
+    };
+    if (a.settled) parameters();
     if (warp == 0) {
         tmem_alloc(sbase + off_bar + 136, 512);
         // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
         pdl_launch_next();
+    }
+    if (!a.settled) {
+        pdl_wait();
+        parameters();
     }
     fence_before_sync();
     __syncthreads();
@@ -101,7 +109,7 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
             for (int r = 0; r < n_out; r += a.w_box_rows)
                 tma_load_2d(sbase + kb * w_block + r * SW, &map_w, kb * KCOLS, r, wbar);
     }
-    // up to here only weights, biases and LayerNorm parameters were read: everything the kernel before
+    // up to here only settled weights, biases and LayerNorm parameters were read: everything the kernel before
     // this one in the stream may have written is touched after this wait
     pdl_wait();
     bool ok = mbar_wait(wbar, 0, abort);
@@ -269,6 +277,7 @@ struct LinearLnArgs {
     __nv_bfloat16* norm_out;
     float eps1, eps2;
     int64_t n;
+    bool settled;                    // see linear.cuh
     uint32_t* status;
 };
 
@@ -321,17 +330,24 @@ __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kern
         prefetch_tensormap(&map_x);
         prefetch_tensormap(&map_w);
     }
-    for (int i = tid; i < K; i += THREADS) {
-        bias_s[i] = a.bias ? __bfloat162float(a.bias[i]) : 0.f;
-        g1[i] = LN1 ? __bfloat162float(a.ln1_w[i]) : 1.f;
-        b1[i] = LN1 ? __bfloat162float(a.ln1_b[i]) : 0.f;
-        g2[i] = __bfloat162float(a.ln2_w[i]);
-        b2[i] = __bfloat162float(a.ln2_b[i]);
-    }
+    auto parameters = [&] {
+        for (int i = tid; i < K; i += THREADS) {
+            bias_s[i] = a.bias ? __bfloat162float(a.bias[i]) : 0.f;
+            g1[i] = LN1 ? __bfloat162float(a.ln1_w[i]) : 1.f;
+            b1[i] = LN1 ? __bfloat162float(a.ln1_b[i]) : 0.f;
+            g2[i] = __bfloat162float(a.ln2_w[i]);
+            b2[i] = __bfloat162float(a.ln2_b[i]);
+        }
+    };
+    if (a.settled) parameters();
     if (warp == 0) {
         tmem_alloc(sbase + OFF_BAR + 136, TM_COLS);
         // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
         pdl_launch_next();
+    }
+    if (!a.settled) {
+        pdl_wait();
+        parameters();
     }
     fence_before_sync();
     __syncthreads();
@@ -341,7 +357,7 @@ __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kern
         mbar_expect_tx(wbar, (uint32_t)(KB * W_BLOCK));
         for (int kb = 0; kb < KB; ++kb) tma_load_2d(sbase + kb * W_BLOCK, &map_w, kb * KCOLS, 0, wbar);
     }
-    // up to here only weights, biases and LayerNorm parameters were read: everything the kernel before
+    // up to here only settled weights, biases and LayerNorm parameters were read: everything the kernel before
     // this one in the stream may have written is touched after this wait
     pdl_wait();
     bool ok = mbar_wait(wbar, 0, abort);
@@ -587,17 +603,9 @@ static int launch_linear_ln(const void* x, const void* w, const LinearLnArgs& a,
     return check_launch("ptv3_linear_ln_fwd");
 }
 
-}  // namespace ptv3
-
-extern "C" int ptv3_linear_supported(int k, int n_out, int residual_mode, int dtype)
+int linear_fwd(const void* x, const void* weight, const void* bias, void* out, int64_t n, int k, int n_out, int dtype,
+               bool settled, uint32_t* status, cudaStream_t stream)
 {
-    return dtype == PTV3_DTYPE_BF16 && ptv3::linear_shape_ok(k, n_out, residual_mode != 0);
-}
-
-extern "C" int ptv3_linear_fwd(const void* x, const void* weight, const void* bias, void* out, int64_t n, int k,
-                               int n_out, int dtype, uint32_t* status, void* stream)
-{
-    using namespace ptv3;
     PTV3_REQUIRE(n >= 0 && n < (1ll << 31), PTV3_ERR_INVALID_ARGUMENT, "ptv3_linear_fwd: bad n");
     PTV3_REQUIRE(ptv3_linear_supported(k, n_out, 0, dtype), PTV3_ERR_UNSUPPORTED,
                  "ptv3_linear_fwd: supported: bf16, k in {32, 64, 128}, n_out a multiple of 32 up to 384");
@@ -606,22 +614,22 @@ extern "C" int ptv3_linear_fwd(const void* x, const void* weight, const void* bi
     PTV3_REQUIRE((((uintptr_t)x | (uintptr_t)weight | (uintptr_t)out) & 15) == 0, PTV3_ERR_INVALID_ARGUMENT,
                  "ptv3_linear_fwd: tensors must be 16-byte aligned");
     if (linear_small_wanted(n, k, n_out))
-        return launch_linear_small(x, weight, bias, nullptr, out, n, k, n_out, 0, status, (cudaStream_t)stream);
+        return launch_linear_small(x, weight, bias, nullptr, out, n, k, n_out, 0, settled, status, stream);
     LinearArgs a{};
     a.bias = (const __nv_bfloat16*)bias;
     a.out = (__nv_bfloat16*)out;
     a.n = n;
     a.n_out = n_out;
+    a.settled = settled;
     a.status = status;
-    return launch_linear(x, weight, a, k, (cudaStream_t)stream);
+    return launch_linear(x, weight, a, k, stream);
 }
 
-extern "C" int ptv3_linear_ln_fwd(const void* x, const void* weight, const void* bias, const void* residual,
-                                  const void* ln1_weight, const void* ln1_bias, float ln1_eps, void* sum_out,
-                                  const void* ln2_weight, const void* ln2_bias, float ln2_eps, void* norm_out,
-                                  int64_t n, int channels, int dtype, uint32_t* status, void* stream)
+int linear_ln_fwd(const void* x, const void* weight, const void* bias, const void* residual, const void* ln1_weight,
+                  const void* ln1_bias, float ln1_eps, void* sum_out, const void* ln2_weight, const void* ln2_bias,
+                  float ln2_eps, void* norm_out, int64_t n, int channels, int dtype, bool settled, uint32_t* status,
+                  cudaStream_t stream)
 {
-    using namespace ptv3;
     PTV3_REQUIRE(n >= 0 && n < (1ll << 31), PTV3_ERR_INVALID_ARGUMENT, "ptv3_linear_ln_fwd: bad n");
     PTV3_REQUIRE(ptv3_linear_supported(channels, channels, 1, dtype), PTV3_ERR_UNSUPPORTED,
                  "ptv3_linear_ln_fwd: supported: bf16, channels in {32, 64, 128}");
@@ -635,9 +643,30 @@ extern "C" int ptv3_linear_ln_fwd(const void* x, const void* weight, const void*
                  PTV3_ERR_INVALID_ARGUMENT, "ptv3_linear_ln_fwd: tensors must be 16-byte aligned");
     const LinearLnArgs a{(const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)ln1_weight,
                          (const __nv_bfloat16*)ln1_bias, (const __nv_bfloat16*)ln2_weight, (const __nv_bfloat16*)ln2_bias,
-                         (__nv_bfloat16*)sum_out, (__nv_bfloat16*)norm_out, ln1_eps, ln2_eps, n, status};
-    cudaStream_t st = (cudaStream_t)stream;
-    if (channels == 32) return ln1_weight ? launch_linear_ln<32, true>(x, weight, a, st) : launch_linear_ln<32, false>(x, weight, a, st);
-    if (channels == 64) return ln1_weight ? launch_linear_ln<64, true>(x, weight, a, st) : launch_linear_ln<64, false>(x, weight, a, st);
-    return ln1_weight ? launch_linear_ln<128, true>(x, weight, a, st) : launch_linear_ln<128, false>(x, weight, a, st);
+                         (__nv_bfloat16*)sum_out, (__nv_bfloat16*)norm_out, ln1_eps, ln2_eps, n, settled, status};
+    if (channels == 32) return ln1_weight ? launch_linear_ln<32, true>(x, weight, a, stream) : launch_linear_ln<32, false>(x, weight, a, stream);
+    if (channels == 64) return ln1_weight ? launch_linear_ln<64, true>(x, weight, a, stream) : launch_linear_ln<64, false>(x, weight, a, stream);
+    return ln1_weight ? launch_linear_ln<128, true>(x, weight, a, stream) : launch_linear_ln<128, false>(x, weight, a, stream);
+}
+
+}  // namespace ptv3
+
+extern "C" int ptv3_linear_supported(int k, int n_out, int residual_mode, int dtype)
+{
+    return dtype == PTV3_DTYPE_BF16 && ptv3::linear_shape_ok(k, n_out, residual_mode != 0);
+}
+
+extern "C" int ptv3_linear_fwd(const void* x, const void* weight, const void* bias, void* out, int64_t n, int k,
+                               int n_out, int dtype, uint32_t* status, void* stream)
+{
+    return ptv3::linear_fwd(x, weight, bias, out, n, k, n_out, dtype, false, status, (cudaStream_t)stream);
+}
+
+extern "C" int ptv3_linear_ln_fwd(const void* x, const void* weight, const void* bias, const void* residual,
+                                  const void* ln1_weight, const void* ln1_bias, float ln1_eps, void* sum_out,
+                                  const void* ln2_weight, const void* ln2_bias, float ln2_eps, void* norm_out,
+                                  int64_t n, int channels, int dtype, uint32_t* status, void* stream)
+{
+    return ptv3::linear_ln_fwd(x, weight, bias, residual, ln1_weight, ln1_bias, ln1_eps, sum_out, ln2_weight, ln2_bias,
+                               ln2_eps, norm_out, n, channels, dtype, false, status, (cudaStream_t)stream);
 }

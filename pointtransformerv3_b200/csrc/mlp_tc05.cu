@@ -17,6 +17,7 @@
 // Completion is tracked with mbarriers (TMA transaction bytes, tcgen05.commit);
 // every wait is bounded and reports through the status word instead of hanging.
 #include "common.cuh"
+#include "linear.cuh"
 #include "tc05.cuh"
 #include "vec.cuh"
 
@@ -59,7 +60,7 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
     const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w1,
     const __grid_constant__ CUtensorMap map_w2, const __nv_bfloat16* __restrict__ b1,
     const __nv_bfloat16* __restrict__ b2, const __nv_bfloat16* __restrict__ residual,
-    __nv_bfloat16* __restrict__ out, int64_t n, uint32_t* __restrict__ status)
+    __nv_bfloat16* __restrict__ out, int64_t n, bool settled, uint32_t* __restrict__ status)
 {
     using Cfg = MlpCfg<C>;
     extern __shared__ unsigned char smem_raw[];
@@ -86,12 +87,19 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
         prefetch_tensormap(&map_w1);
         prefetch_tensormap(&map_w2);
     }
-    for (int i = tid; i < Cfg::HD; i += NT) b1s[i] = __bfloat162float(b1[i]);
-    for (int i = tid; i < C; i += NT) b2s[i] = __bfloat162float(b2[i]);
+    auto parameters = [&] {
+        for (int i = tid; i < Cfg::HD; i += NT) b1s[i] = __bfloat162float(b1[i]);
+        for (int i = tid; i < C; i += NT) b2s[i] = __bfloat162float(b2[i]);
+    };
+    if (settled) parameters();
     if (warp == 0) {
         tmem_alloc(sbase + Cfg::OFF_BAR + 8 * Cfg::NBAR, 512);
         // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
         pdl_launch_next();
+    }
+    if (!settled) {
+        pdl_wait();
+        parameters();
     }
     fence_before_sync();
     __syncthreads();
@@ -106,7 +114,7 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
         for (int kb = 0; kb < Cfg::HD / 64; ++kb)
             tma_load_2d(sbase + Cfg::OFF_W2 + kb * Cfg::W2_BLOCK, &map_w2, kb * 64, 0, wbar);
     }
-    // up to here only weights and biases were read: everything the kernel before this one in the
+    // up to here only settled weights and biases were read: everything the kernel before this one in the
     // stream may have written is touched after this wait
     pdl_wait();
     bool ok = mbar_wait(wbar, 0, abort);
@@ -275,7 +283,7 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
 
 template <int C>
 static int launch_mlp(const void* x, const void* w1, const void* b1, const void* w2, const void* b2,
-                      const void* residual, void* out, int64_t n, uint32_t* status, cudaStream_t stream)
+                      const void* residual, void* out, int64_t n, bool settled, uint32_t* status, cudaStream_t stream)
 {
     using Cfg = MlpCfg<C>;
     CUtensorMap mx, mw1, mw2;
@@ -292,9 +300,29 @@ static int launch_mlp(const void* x, const void* w1, const void* b1, const void*
     const int64_t grid = ntiles < 148 ? ntiles : 148;
     launch_dependent(kern, dim3((unsigned)grid), dim3(128 * Cfg::NG), Cfg::SMEM, stream, mx, mw1, mw2,
                      (const __nv_bfloat16*)b1, (const __nv_bfloat16*)b2, (const __nv_bfloat16*)residual,
-                     (__nv_bfloat16*)out, n, status);
+                     (__nv_bfloat16*)out, n, settled, status);
     count_launches(1);
     return check_launch("ptv3_mlp_fwd");
+}
+
+int mlp_fwd(const void* x, const void* fc1_weight, const void* fc1_bias, const void* fc2_weight, const void* fc2_bias,
+            const void* residual, void* out, int64_t n, int channels, int hidden, int dtype, bool settled,
+            uint32_t* status, cudaStream_t stream)
+{
+    PTV3_REQUIRE(n >= 0 && n < (1ll << 31), PTV3_ERR_INVALID_ARGUMENT, "ptv3_mlp_fwd: bad n");
+    PTV3_REQUIRE(ptv3_mlp_supported(channels, hidden, dtype), PTV3_ERR_UNSUPPORTED,
+                 "ptv3_mlp_fwd: supported: bf16, channels 32 or 64, hidden = 4 x channels");
+    if (n == 0) return PTV3_OK;
+    PTV3_REQUIRE(x && fc1_weight && fc1_bias && fc2_weight && fc2_bias && residual && out && status,
+                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_mlp_fwd: null pointer");
+    PTV3_REQUIRE((((uintptr_t)x | (uintptr_t)fc1_weight | (uintptr_t)fc2_weight | (uintptr_t)residual |
+                   (uintptr_t)out) & 15) == 0,
+                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_mlp_fwd: tensors must be 16-byte aligned");
+    if (channels == 32)
+        return launch_mlp<32>(x, fc1_weight, fc1_bias, fc2_weight, fc2_bias, residual, out, n, settled, status,
+                              stream);
+    return launch_mlp<64>(x, fc1_weight, fc1_bias, fc2_weight, fc2_bias, residual, out, n, settled, status,
+                          stream);
 }
 
 }  // namespace ptv3
@@ -308,19 +336,6 @@ extern "C" int ptv3_mlp_fwd(const void* x, const void* fc1_weight, const void* f
                             const void* fc2_weight, const void* fc2_bias, const void* residual, void* out,
                             int64_t n, int channels, int hidden, int dtype, uint32_t* status, void* stream)
 {
-    using namespace ptv3;
-    PTV3_REQUIRE(n >= 0 && n < (1ll << 31), PTV3_ERR_INVALID_ARGUMENT, "ptv3_mlp_fwd: bad n");
-    PTV3_REQUIRE(ptv3_mlp_supported(channels, hidden, dtype), PTV3_ERR_UNSUPPORTED,
-                 "ptv3_mlp_fwd: supported: bf16, channels 32 or 64, hidden = 4 x channels");
-    if (n == 0) return PTV3_OK;
-    PTV3_REQUIRE(x && fc1_weight && fc1_bias && fc2_weight && fc2_bias && residual && out && status,
-                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_mlp_fwd: null pointer");
-    PTV3_REQUIRE((((uintptr_t)x | (uintptr_t)fc1_weight | (uintptr_t)fc2_weight | (uintptr_t)residual |
-                   (uintptr_t)out) & 15) == 0,
-                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_mlp_fwd: tensors must be 16-byte aligned");
-    if (channels == 32)
-        return launch_mlp<32>(x, fc1_weight, fc1_bias, fc2_weight, fc2_bias, residual, out, n, status,
-                              (cudaStream_t)stream);
-    return launch_mlp<64>(x, fc1_weight, fc1_bias, fc2_weight, fc2_bias, residual, out, n, status,
-                          (cudaStream_t)stream);
+    return ptv3::mlp_fwd(x, fc1_weight, fc1_bias, fc2_weight, fc2_bias, residual, out, n, channels, hidden, dtype, false,
+                         status, (cudaStream_t)stream);
 }

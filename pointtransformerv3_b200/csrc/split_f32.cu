@@ -8,7 +8,8 @@ template <bool WEIGHT>
 __global__ void __launch_bounds__(256) split_f32_kernel(const float* __restrict__ x, int64_t n8, int k,
                                                         __nv_bfloat16* __restrict__ out)
 {
-    pdl_launch_next();
+    // (the product behind the weight form fetches weights before it waits for anything)
+    if (!WEIGHT) pdl_launch_next();
     pdl_wait();
     const int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (e >= n8) return;

@@ -807,3 +807,56 @@ def test_subm_conv_on_split_floats(n, cin, cout):
     rows = torch.cat([feat.double(), feat.new_zeros(1, cin).double()])[nbr.long()]          # -1 -> the zero row
     ref = torch.einsum("onc,doc->nd", rows, w.double().reshape(cout, 27, cin)) + b.double()
     assert rel_l2(got.double(), ref) < 1.5 * rel_l2(plain.double(), ref) + 1e-7
+
+
+@pytest.mark.parametrize("op", ["linear_short", "linear", "gemm_short", "gemm_streamed", "gemm_resident", "linear_ln",
+                                "mlp", "linear_split", "block"])
+def test_weights_computed_by_the_call_before(op):
+    """Weights that the call queued directly before computes, or one a few calls before: kernels are brought up
+    while those run, and must not have fetched what lay there.  One status word, so that nothing else is queued
+    in between.  (Products with the identity copy bf16 rows exactly.)"""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    rand = lambda *shape: torch.randn(*shape, generator=g, device="cuda").bfloat16()
+    n, k, n_out = {"linear_short": (300, 64, 192), "linear": (70_000, 64, 192), "gemm_short": (300, 128, 256),
+                   "gemm_streamed": (20_000, 512, 512), "gemm_resident": (60_000, 256, 256), "linear_ln": (5000, 64, 64),
+                   "mlp": (5000, 64, 64), "linear_split": (600, 128, 128), "block": (700, 64, 64)}[op]
+    status = ops.new_status("cuda")
+    x, r = rand(n, k), rand(n, n_out)
+    eye, eye4, zero = torch.eye(k, device="cuda").bfloat16(), torch.eye(4 * k, device="cuda").bfloat16(), rand(4 * k) * 0
+    ln = torch.nn.LayerNorm(k).cuda().bfloat16()
+    copy = lambda w: (ops.gemm if w.shape[1] % 128 == 0 else ops.linear)(
+        w, eye if w.shape[1] == k else eye4, zero[:w.shape[1]], status=status)
+
+    def use(ws):
+        with torch.inference_mode():
+            if op == "linear_ln":
+                return ops.linear_ln(x, ws[0], ws[1].view(-1)[:k], r, ln, ln, status)[1]
+            if op == "mlp":
+                return ops.mlp(x, ws[0], zero, ws[1], zero[:k], r, status)
+            if op == "linear_split":
+                return ops.linear_split(xs, ops.split_f32(ws[0], weight=True), k, status=status)
+            if op.startswith("gemm"):
+                return ops.gemm(x, ws[0], ws[1].view(-1)[:n_out], r, status=status)
+            if op == "block":
+                for t in ws:                                  # three kernels between the weights and their use
+                    y = ops.linear(x, ws[-1], zero[:k], status)
+                return ops.linear_ln(y, ws[0], zero[:k], r, ln, ln, status)[1]
+            return ops.linear(x, ws[0], ws[1].view(-1)[:n_out], status)
+
+    shapes = [(4 * k, k), (k, 4 * k)] if op == "mlp" else [(n_out, k)] * 3
+    scale = 1.0 / k ** 0.5
+    if op == "linear_split":
+        xs = ops.split_f32(x.float())
+    for i in range(12):
+        want_w = [rand(*s) * scale for s in shapes]
+        if op == "linear_split":
+            want_w = [w.float() for w in want_w]
+        torch.cuda.synchronize()
+        ref = use(want_w)
+        torch.cuda.synchronize()
+        ws = want_w if op == "linear_split" else [copy(w) for w in want_w]
+        got = use(ws)
+        assert all(torch.equal(a, b) for a, b in zip(ws, want_w))
+        assert torch.equal(got, ref)
+        del ws                                                # the next weights find these in their memory
+    assert int(status.item()) == 0
