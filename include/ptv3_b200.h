@@ -608,7 +608,7 @@ typedef struct ptv3_backbone_args {
     int n_enc, n_dec;               /* n_dec == n_enc - 1, decoder stages from coarse to fine */
     const ptv3_stage_args *enc, *dec;
     int dtype;                      /* features and parameters; fp32: weights split as for ptv3_block_fwd (the
-                                       stem's weight is not), transitions too */
+                                       stem's weight is not), transitions too, unless plain_weights is set */
     int stem_c_in, stem_c_out, stem_ksize;
     const void* stem_weight;
     const float *stem_scale, *stem_shift;
@@ -635,6 +635,7 @@ typedef struct ptv3_backbone_args {
     ptv3_alloc_fn alloc;
     void* alloc_ctx;
     void *main_stream, *plan_stream;
+    int plain_weights;              /* fp32: not zero if weights are plain fp32; the call then splits them for itself */
 } ptv3_backbone_args;
 
 int ptv3_backbone_fwd(const ptv3_backbone_args* args);

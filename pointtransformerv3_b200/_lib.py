@@ -55,7 +55,8 @@ class BackboneArgs(ctypes.Structure):
         + [(name, c_ptr) for name in ("feat", "grid_coord", "offset", "batch", "code", "order", "inverse", "indices",
                                       "nbr", "pad", "unpad", "cu_seqlens", "out")]
         + [("level_counts", ctypes.POINTER(c_i64)), ("meta_host", c_ptr), ("status", c_ptr), ("alloc", ALLOC_FN),
-           ("alloc_ctx", c_ptr), ("main_stream", c_ptr), ("plan_stream", c_ptr)])
+           ("alloc_ctx", c_ptr), ("main_stream", c_ptr), ("plan_stream", c_ptr),
+           ("plain_weights", c_int)])
 
 
 # name -> (restype, argtypes); must list every symbol of include/ptv3_b200.h

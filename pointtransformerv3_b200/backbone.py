@@ -1,7 +1,7 @@
 """One-call form of the backbone's forward (ptv3_backbone_fwd): the argument blocks of a network
 whose modules all have their standard form, kept between passes and rebuilt when a parameter, a
-buffer or a setting changed.  fp32 networks keep their weights split for the tensor cores there
-(1.5 times their size, see ptv3_split_f32)."""
+buffer or a setting changed.  Weights are read where the parameters are, on every pass (fp32 networks have
+them split for the tensor cores by the call)."""
 import ctypes
 import itertools
 import operator
@@ -62,7 +62,7 @@ class NativeBackbone:
         _require(type(conv) is spconv.SubMConv3d and conv.uses_direct_path() and conv.bias is None
                  and _eval_bn(bn) and _exact_gelu(act))
         a = self.args = _lib.BackboneArgs()
-        a.dtype = _lib.DTYPE_IDS[self.dtype]
+        a.dtype, a.plain_weights = _lib.DTYPE_IDS[self.dtype], 1
         a.stem_c_in, a.stem_c_out, a.stem_ksize = conv.in_channels, conv.out_channels, conv.kernel_size
         a.stem_weight = self._param(conv, "weight")
         a.stem_scale, a.stem_shift = self._bn(bn)
@@ -87,17 +87,6 @@ class NativeBackbone:
         self.refs.append((module._parameters, name))
         return t.data_ptr()
 
-    def _weight(self, module):
-        """A weight that enters a matrix product: itself, or its split form."""
-        p = self._param(module, "weight")
-        if not self.f32:
-            return p
-        t = module._parameters["weight"]
-        split = ops.split_f32(t, weight=True)
-        self.versions.append(t)
-        self.keep.append(split)
-        return split.data_ptr()
-
     def _bn(self, bn):
         from .model import _bn_eval_affine
         _require(_eval_bn(bn))
@@ -114,7 +103,7 @@ class NativeBackbone:
         _require(type(lin) is nn.Linear and lin.bias is not None
                  and (lin.in_features % 32 == 0 and lin.out_features % 32 == 0 if self.f32
                       else supported(lin.in_features, lin.out_features, torch.bfloat16)))
-        return self._weight(lin), self._param(lin, "bias")
+        return self._param(lin, "weight"), self._param(lin, "bias")
 
     def _stages(self, stages, encoder):
         from . import model as M
@@ -152,11 +141,6 @@ class NativeBackbone:
                 _require(args is not None and args.conv_weight)
                 ctypes.pointer(blocks[j])[0] = args
                 self.refs.extend(m.__dict__["_ptv3_block_args"][0])
-                if self.f32:
-                    b, mlp = blocks[j], m.mlp[0]
-                    for field, owner in (("conv_weight", m.cpe[0]), ("cpe_w", m.cpe[1]), ("qkv_w", m.attn.qkv),
-                                         ("proj_w", m.attn.proj), ("fc1_w", mlp.fc1), ("fc2_w", mlp.fc2)):
-                        setattr(b, field, self._weight(owner))
                 order_index[j] = m.attn.order_index
                 patch[j] = m.attn.patch_size if m.attn.enable_flash else -m.attn.patch_size_max
                 self.blocks.append(m)

@@ -12,6 +12,8 @@
 #include "plan.cuh"
 #include "split_f32.cuh"
 #include <string.h>
+#include <memory>
+#include <new>
 
 namespace ptv3 {
 
@@ -102,6 +104,8 @@ public:
         : a_(*a), main_((cudaStream_t)a->main_stream), side_((cudaStream_t)a->plan_stream), mem_(a->alloc, a->alloc_ctx, 0),
           plan_mem_(a->alloc, a->alloc_ctx, 1)
     {
+        memcpy(enc_, a->enc, a->n_enc * sizeof(ptv3_stage_args));
+        memcpy(dec_, a->dec, a->n_dec * sizeof(ptv3_stage_args));
     }
     int run();
 
@@ -110,6 +114,8 @@ private:
     cudaStream_t main_, side_;
     Arena mem_, plan_mem_;
     Events events_;
+    ptv3_stage_args enc_[BB_MAX_STAGES], dec_[BB_MAX_STAGES];       // as given, with this pass's split weights
+    std::unique_ptr<ptv3_block_args[]> blocks_;                     // ... and the blocks they point to
     BbLevel lv_[BB_MAX_STAGES];
     int made_ = 0;                  // levels whose geometry is queued
     // the plan in flight (pooling of level made_ - 1): packed outputs whose row stride is not known yet
@@ -145,6 +151,9 @@ private:
         return (int)least;
     }
     int pad_level(BbLevel& l, int patch, Arena& mem, cudaStream_t stream, int64_t* pad, int64_t* unpad, int32_t* cu);
+    template <typename F>
+    int each_weight(F&& f);
+    int split_weights();
     int finest();
     int launch_plan();
     int take_plan(bool block);
@@ -172,6 +181,67 @@ int Pass::pad_level(BbLevel& l, int patch, Arena& mem, cudaStream_t stream, int6
     l.patch = patch;
     l.n_seq = (int)n_seq;
     return ptv3_pad_plan(l.offset, a_.n_scenes, patch, l.n, n_pad, (int)n_seq, l.pad, l.unpad, l.cu, a_.status, stream);
+}
+
+// f(pointer, rows, inner dimension) of every weight that enters a matrix product; `blocks_` holds the blocks
+template <typename F>
+int Pass::each_weight(F&& f)
+{
+    for (int s = 0; s < a_.n_enc + a_.n_dec; ++s) {
+        const bool encoder = s < a_.n_enc;
+        ptv3_stage_args& st = encoder ? enc_[s] : dec_[s - a_.n_enc];
+        if (s > 0) BB_STEP(f(st.w, st.c_out, st.c_in));
+        if (!encoder) BB_STEP(f(st.w_skip, st.c_out, st.c_skip));
+        ptv3_block_args* b = const_cast<ptv3_block_args*>(st.blocks);
+        for (int j = 0; j < st.n_blocks; ++j, ++b) {
+            const int C = b->channels, H = b->hidden;
+            BB_STEP(f(b->conv_weight, (int64_t)27 * C, C));
+            BB_STEP(f(b->cpe_w, C, C));
+            BB_STEP(f(b->qkv_w, (int64_t)3 * C, C));
+            BB_STEP(f(b->proj_w, C, C));
+            BB_STEP(f(b->fc1_w, H, C));
+            BB_STEP(f(b->fc2_w, C, H));
+        }
+    }
+    return PTV3_OK;
+}
+
+// fp32 weights, split for this pass: what the caller writes to them is seen by the next pass, whichever way it
+// is written and on whatever stream.  The default network's 183 MB become 275, one launch that runs on the main
+// stream while that waits for the sort (two rooms of 20 000 points: 6.39 ms a pass, 6.36 with splits that were kept).
+int Pass::split_weights()
+{
+    if (a_.dtype != PTV3_DTYPE_F32 || !a_.plain_weights) return PTV3_OK;
+    int n_blocks = 0, count = 0;
+    for (int s = 0; s < a_.n_enc; ++s) n_blocks += enc_[s].n_blocks;
+    for (int d = 0; d < a_.n_dec; ++d) n_blocks += dec_[d].n_blocks;
+    blocks_.reset(new (std::nothrow) ptv3_block_args[n_blocks]);
+    std::unique_ptr<SplitWeight[]> jobs(new (std::nothrow) SplitWeight[6 * n_blocks + a_.n_enc + 2 * a_.n_dec]);
+    PTV3_REQUIRE(blocks_ && jobs, PTV3_ERR_WORKSPACE, "ptv3_backbone_fwd: out of host memory");
+    ptv3_block_args* at = blocks_.get();
+    for (int s = 0; s < a_.n_enc + a_.n_dec; ++s) {
+        ptv3_stage_args& st = s < a_.n_enc ? enc_[s] : dec_[s - a_.n_enc];
+        memcpy(at, st.blocks, st.n_blocks * sizeof(ptv3_block_args));
+        st.blocks = at;
+        at += st.n_blocks;
+    }
+    size_t bytes = 0;
+    BB_STEP(each_weight([&](const void*& w, int64_t rows, int k) {
+        PTV3_REQUIRE(w && ((uintptr_t)w & 15) == 0 && rows > 0 && k >= 32 && k % 32 == 0, PTV3_ERR_INVALID_ARGUMENT,
+                     "ptv3_backbone_fwd: a weight of %lld x %d: null, alignment or width", (long long)rows, k);
+        jobs[count++] = SplitWeight{(const float*)w, rows, k, nullptr};
+        bytes += align_up((size_t)rows * split_stored(k) * k * 2, 256);
+        return PTV3_OK;
+    }));
+    char* out = mem_.take<char>(bytes);
+    if (!out) return out_of_memory();
+    int j = 0;
+    BB_STEP(each_weight([&](const void*& w, int64_t rows, int k) {
+        w = jobs[j++].out = out;
+        out += align_up((size_t)rows * split_stored(k) * k * 2, 256);
+        return PTV3_OK;
+    }));
+    return launch_split_weights(jobs.get(), count, main_);
 }
 
 // serialization, voxel index, kernel map and stem of the finest level
@@ -211,10 +281,11 @@ int Pass::finest()
     VoxelIndex vi;
     BB_STEP(build_voxel_index(a_.indices, a_.n, index_ws, a_.status, main_, &vi));
     BB_CUDA(events_.record(main_, &indexed));
+    BB_STEP(split_weights());
     BB_CUDA(cudaStreamWaitEvent(side_, indexed, 0));
     BB_STEP(kmap_from_index(vi, a_.indices, a_.n, 3, a_.order, a_.nbr, a_.status, side_));
-    if (a_.enc[0].n_blocks > 0)
-        BB_STEP(pad_level(l, patch_of(a_.enc[0].patch[0], l, a_.n_scenes), plan_mem_, side_, a_.pad, a_.unpad,
+    if (enc_[0].n_blocks > 0)
+        BB_STEP(pad_level(l, patch_of(enc_[0].patch[0], l, a_.n_scenes), plan_mem_, side_, a_.pad, a_.unpad,
                           a_.cu_seqlens));
     BB_CUDA(events_.record(side_, &l.ready));
     made_ = 1;
@@ -233,7 +304,7 @@ int Pass::launch_plan()
 {
     if (made_ >= a_.n_enc) return PTV3_OK;
     BbLevel& p = lv_[made_ - 1];
-    const int depth = a_.enc[made_].pooling_depth <= p.depth ? a_.enc[made_].pooling_depth : 0;
+    const int depth = enc_[made_].pooling_depth <= p.depth ? enc_[made_].pooling_depth : 0;
     const size_t bytes = ptv3_pool_plan_workspace_bytes(a_.k, p.n, a_.n_scenes);
     p.cluster = plan_mem_.take<int64_t>(p.n);
     p.idx_ptr = plan_mem_.take<int64_t>(p.n + 1);
@@ -290,7 +361,7 @@ int Pass::take_plan(bool block)
     BB_STEP(ptv3_batch_indices(l.offset, a_.n_scenes, l.grid, l.n, nullptr, indices, side_));
     BB_STEP(ptv3_kmap_build_ordered(indices, l.n, 3, l.order, nbr, a_.status, ws, bytes, side_));
     l.nbr = nbr;
-    const ptv3_stage_args& st = a_.enc[made_];
+    const ptv3_stage_args& st = enc_[made_];
     if (st.n_blocks > 0)
         BB_STEP(pad_level(l, patch_of(st.patch[0], l, a_.n_scenes), plan_mem_, side_, nullptr, nullptr, nullptr));
     BB_CUDA(events_.record(side_, &l.ready));
@@ -327,14 +398,14 @@ int Pass::block(const ptv3_stage_args& st, int j, BbLevel& l, const void* conv_i
 // fp32 projection of a stage transition, on split operands
 int Pass::project(const void* x, const void* w, const void* bias, int64_t n, int c_in, int c_out, void* split, void* out)
 {
-    BB_STEP(launch_split_f32((const float*)x, n, c_in, false, split, main_));
+    BB_STEP(launch_split_f32((const float*)x, n, c_in, split, main_));
     return launch_linear_split(split, w, (const float*)bias, nullptr, (float*)out, nullptr, n, c_in, c_out, 0, true,
                                a_.status, main_);
 }
 
 int Pass::encoder(int s)
 {
-    const ptv3_stage_args& st = a_.enc[s];
+    const ptv3_stage_args& st = enc_[s];
     while (made_ <= s) BB_STEP(take_plan(true));
     BbLevel& l = lv_[s];
     BB_CUDA(cudaStreamWaitEvent(main_, l.ready, 0));
@@ -373,7 +444,7 @@ int Pass::encoder(int s)
 
 int Pass::decoder(int d)
 {
-    const ptv3_stage_args& st = a_.dec[d];
+    const ptv3_stage_args& st = dec_[d];
     BbLevel& c = lv_[a_.n_enc - 1 - d];
     BbLevel& l = lv_[a_.n_enc - 2 - d];
     const size_t row = (size_t)l.n * st.c_out * esize_;

@@ -113,22 +113,22 @@ static int block_f32(const ptv3_block_args* a, bool settled, cudaStream_t stream
     } while (0)
     auto f = [](const void* p) { return (const float*)p; };
     // (the split of the convolution's input lies where the hidden rows come later)
-    STEP(launch_split_f32(f(a->conv_in), n, C, false, b.sh, stream));
+    STEP(launch_split_f32(f(a->conv_in), n, C, b.sh, stream));
     STEP(launch_conv_split(b.sh, a->nbr, a->conv_weight, f(a->conv_bias), nullptr, b.s, a->row_order, n, C, C, 27, a->status,
                            stream));
     STEP(launch_linear_split(b.s, a->cpe_w, f(a->cpe_b), nullptr, b.y, nullptr, n, C, C, 0, settled, a->status, stream));
     STEP(ptv3_add_layernorm_fwd(b.y, a->feat, a->cpe_ln_w, a->cpe_ln_b, a->cpe_ln_eps, b.f1, a->n1_w, a->n1_b, a->n1_eps, b.a,
                                 n, C, PTV3_DTYPE_F32, stream));
-    STEP(launch_split_f32(b.a, n, C, false, b.s, stream));
+    STEP(launch_split_f32(b.a, n, C, b.s, stream));
     STEP(launch_linear_split(b.s, a->qkv_w, f(a->qkv_b), nullptr, b.qkv, nullptr, n, C, 3 * C, 0, settled, a->status, stream));
     STEP(ptv3_attention_fwd(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.att, n, a->n_seq, a->max_seqlen, C, a->heads,
                             a->scale, PTV3_DTYPE_F32, a->attention_algo, a->status, stream));
-    STEP(launch_split_f32(b.att, n, C, false, b.s, stream));
+    STEP(launch_split_f32(b.att, n, C, b.s, stream));
     // (b.a is free until the second norm)
     STEP(launch_linear_split(b.s, a->proj_w, f(a->proj_b), nullptr, b.qkv, nullptr, n, C, C, 0, settled, a->status, stream));
     STEP(ptv3_add_layernorm_fwd(b.qkv, b.f1, nullptr, nullptr, 0.f, b.f2, a->n2_w, a->n2_b, a->n2_eps, b.a, n, C,
                                 PTV3_DTYPE_F32, stream));
-    STEP(launch_split_f32(b.a, n, C, false, b.s, stream));
+    STEP(launch_split_f32(b.a, n, C, b.s, stream));
     STEP(launch_linear_split(b.s, a->fc1_w, f(a->fc1_b), nullptr, nullptr, b.sh, n, C, H, 1, settled, a->status, stream));
     STEP(launch_linear_split(b.sh, a->fc2_w, f(a->fc2_b), b.f2, (float*)a->out, nullptr, n, H, C, 0, settled, a->status, stream));
 #undef STEP

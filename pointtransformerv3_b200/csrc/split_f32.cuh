@@ -62,7 +62,15 @@ __device__ __forceinline__ void split_store8(__nv_bfloat16* row, int c, int k, c
     }
 }
 
-// rows x k floats -> rows x split_stored(k) k bf16; `weight`: a B row
-int launch_split_f32(const float* x, int64_t rows, int k, bool weight, void* out, cudaStream_t stream);
+// rows x k floats -> rows x split_stored(k) k bf16, as A rows
+int launch_split_f32(const float* x, int64_t rows, int k, void* out, cudaStream_t stream);
+// ... as B rows, any number of weights
+struct SplitWeight {
+    const float* x;
+    int64_t rows;
+    int k;
+    void* out;
+};
+int launch_split_weights(const SplitWeight* w, int count, cudaStream_t stream);
 
 }  // namespace ptv3

@@ -456,6 +456,43 @@ def test_network_changed_between_passes(change):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("name", ["embedding.stem.conv.weight", "enc.enc0.block0.cpe.0.weight", "enc.enc1.down.proj.weight",
+                                  "dec.dec0.up.proj_skip.0.weight", "dec.dec0.block0.mlp.0.fc1.weight"])
+def test_values_written_through_data_between_passes(name, dtype):
+    """A write through ``.data`` (weight averaging, a broadcast) moves neither a tensor's identity nor its address
+    nor its version counter: the next pass sees the new values all the same, on another stream too."""
+    import copy
+    from pointtransformerv3_b200 import backbone
+    data = small_batch([900, 500], 7)
+    net = P.PointTransformerV3(in_channels=6, **SMALL_CFG)
+    weights.fill_state_dict(net, prefix="ptv3.")
+    net = net.eval().cuda().to(dtype)
+    fresh = copy.deepcopy(net)
+
+    def run(n):
+        torch.manual_seed(5)
+        with torch.inference_mode():
+            return n(cuda_data(data, dtype)).feat
+
+    for _ in range(3):
+        before = run(net)
+    assert backbone.of(net)[0] is not None
+    for n in (net, fresh):
+        tensor = n.get_parameter(name)
+        version = tensor._version
+        tensor.data.mul_(2)
+        assert tensor._version == version
+    got, ref = run(net), run(fresh)
+    assert torch.equal(got, ref) and not torch.equal(got, before)
+    side = torch.cuda.Stream()
+    net.get_parameter(name).data.mul_(0.5)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        assert torch.equal(run(net), before)
+
+
+@pytest.mark.gpu
 def test_forward_with_host_metadata_and_deferred_status():
     """The optional entries that let a caller skip the host waits of a pass (scene sizes,
     code depth and sparse shape known on the host; status word read later) do not change
