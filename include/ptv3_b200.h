@@ -377,6 +377,20 @@ int ptv3_add_layernorm_fwd(const void* x, const void* residual, const void* ln1_
                            int dtype, void* stream);
 
 /*
+ * BatchNorm in eval mode (model.py:830) as fp32 scale and shift per channel for the kernels that apply it:
+ * scale = weight / sqrt(var + eps), shift = bias - mean scale; `count` layers in one launch.  Parameters and
+ * buffers are fp32 or bf16, each with its own type; weight / bias may be NULL (1 / 0).
+ *   layers  HOST array       out  per layer its `channels` scales, then its shifts
+ */
+typedef struct ptv3_bn_args {
+    const void *weight, *bias, *mean, *var;
+    int weight_dtype, bias_dtype, mean_dtype, var_dtype;
+    int channels;
+    float eps;
+} ptv3_bn_args;
+int ptv3_bn_affine(const ptv3_bn_args* layers, int count, float* out, void* stream);
+
+/*
  * Fused MLP of a block: out = residual + fc2(GELU(fc1(x) + b1)) + b2, the hidden
  * activation kept on chip (tcgen05 tensor cores, TMEM accumulators, TMA loads).
  * Replaces MLP.forward and the residual addition, model.py:510-516, 601-602.
@@ -600,7 +614,8 @@ typedef struct ptv3_stage_args {
     int c_in, c_skip, c_out;
     int pooling_depth, reduce;
     const void *w, *b, *w_skip, *b_skip;
-    const float *scale, *shift, *scale_skip, *shift_skip;   /* BatchNorm(eval) as fp32 scale and shift */
+    const float *scale, *shift, *scale_skip, *shift_skip;   /* BatchNorm(eval) as fp32 scale and shift, */
+    const ptv3_bn_args *bn, *bn_skip;   /* HOST; or, where not NULL, the layers themselves: the call computes both */
 } ptv3_stage_args;
 
 typedef struct ptv3_backbone_args {
@@ -635,6 +650,7 @@ typedef struct ptv3_backbone_args {
     ptv3_alloc_fn alloc;
     void* alloc_ctx;
     void *main_stream, *plan_stream;
+    const ptv3_bn_args* stem_bn;    /* HOST, or NULL: instead of stem_scale / stem_shift, as in ptv3_stage_args */
     int plain_weights;              /* fp32: not zero if weights are plain fp32; the call then splits them for itself */
 } ptv3_backbone_args;
 

@@ -35,13 +35,20 @@ class BlockArgs(ctypes.Structure):
 ALLOC_FN = ctypes.CFUNCTYPE(c_ptr, c_ptr, c_sz, c_int)
 
 
+class BnArgs(ctypes.Structure):
+    """ptv3_bn_args of include/ptv3_b200.h (same field order)."""
+    _fields_ = ([(name, c_ptr) for name in ("weight", "bias", "mean", "var")]
+                + [(name, c_int) for name in ("weight_dtype", "bias_dtype", "mean_dtype", "var_dtype", "channels")]
+                + [("eps", c_f32)])
+
+
 class StageArgs(ctypes.Structure):
     """ptv3_stage_args of include/ptv3_b200.h (same field order)."""
     _fields_ = ([("n_blocks", c_int), ("blocks", ctypes.POINTER(BlockArgs)), ("order_index", ctypes.POINTER(c_int)),
                  ("patch", ctypes.POINTER(c_int)), ("c_in", c_int), ("c_skip", c_int), ("c_out", c_int),
                  ("pooling_depth", c_int), ("reduce", c_int)]
                 + [(name, c_ptr) for name in ("w", "b", "w_skip", "b_skip", "scale", "shift", "scale_skip",
-                                              "shift_skip")])
+                                              "shift_skip", "bn", "bn_skip")])
 
 
 class BackboneArgs(ctypes.Structure):
@@ -56,7 +63,7 @@ class BackboneArgs(ctypes.Structure):
                                       "nbr", "pad", "unpad", "cu_seqlens", "out")]
         + [("level_counts", ctypes.POINTER(c_i64)), ("meta_host", c_ptr), ("status", c_ptr), ("alloc", ALLOC_FN),
            ("alloc_ctx", c_ptr), ("main_stream", c_ptr), ("plan_stream", c_ptr),
-           ("plain_weights", c_int)])
+           ("stem_bn", c_ptr), ("plain_weights", c_int)])
 
 
 # name -> (restype, argtypes); must list every symbol of include/ptv3_b200.h
@@ -99,6 +106,7 @@ SIGNATURES = {
                               c_ptr]),
     "ptv3_add_layernorm_fwd": (c_int, [c_ptr, c_ptr, c_ptr, c_ptr, c_f32, c_ptr, c_ptr, c_ptr, c_f32, c_ptr,
                                        c_i64, c_int, c_int, c_ptr]),
+    "ptv3_bn_affine": (c_int, [ctypes.POINTER(BnArgs), c_int, c_ptr, c_ptr]),
     "ptv3_linear_supported": (c_int, [c_int, c_int, c_int, c_int]),
     "ptv3_gemm_supported": (c_int, [c_int, c_int, c_int]),
     "ptv3_gemm_fwd": (c_int, [c_ptr, c_ptr, c_ptr, c_ptr, c_ptr, c_i64, c_int, c_int, c_int, c_int, c_ptr, c_ptr]),

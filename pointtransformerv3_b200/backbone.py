@@ -15,7 +15,6 @@ from . import sparse as spconv
 from .sparse import SparseConvTensor
 
 _GLOBAL_HOOKS = nn.modules.module
-_VERSION = operator.attrgetter("_version")
 
 
 def _exact_gelu(m):
@@ -49,9 +48,9 @@ class NativeBackbone:
         self.dtype = next(net.parameters()).dtype
         self.f32 = self.dtype == torch.float32
         _require(self.dtype in (torch.float32, torch.bfloat16))
-        self.refs = []           # (owner dict, name): every tensor the blocks point to or were computed from
-        self.versions = []       # tensors whose values were read (BatchNorm): recomputed when modified in place
-        self.keep = []           # arrays and tensors the blocks point into
+        self.refs = []           # (owner dict, name): every tensor the blocks point to
+        self.norms = []          # BatchNorm layers
+        self.keep = []           # arrays the blocks point into
         self.modules = [m.__dict__ for m in net.modules()]
         self.parents = [d["_modules"] for d in self.modules if d["_modules"]]
         self.children = [c for d in self.parents for c in d.values()]
@@ -65,7 +64,7 @@ class NativeBackbone:
         a.dtype, a.plain_weights = _lib.DTYPE_IDS[self.dtype], 1
         a.stem_c_in, a.stem_c_out, a.stem_ksize = conv.in_channels, conv.out_channels, conv.kernel_size
         a.stem_weight = self._param(conv, "weight")
-        a.stem_scale, a.stem_shift = self._bn(bn)
+        a.stem_bn = self._bn(bn)
         self.width_in = conv.in_channels
         enc, dec = list(net.enc._modules.values()), list(net.dec._modules.values())
         _require(len(enc) == net.num_stages and len(dec) == net.num_stages - 1 and len(enc) >= 2)
@@ -78,7 +77,6 @@ class NativeBackbone:
         self.owners, self.names = [d for d, _ in self.refs], [k for _, k in self.refs]
         self.tensors = [d[k] for d, k in self.refs]
         self.ptrs = [t.data_ptr() for t in self.tensors]
-        self.version = [t._version for t in self.versions]
 
     # -- what the blocks are made of
     def _param(self, module, name):
@@ -88,16 +86,13 @@ class NativeBackbone:
         return t.data_ptr()
 
     def _bn(self, bn):
-        from .model import _bn_eval_affine
-        _require(_eval_bn(bn))
-        for d, names in ((bn._parameters, ("weight", "bias")), (bn._buffers, ("running_mean", "running_var"))):
-            for name in names:
-                if d[name] is not None:
-                    self.refs.append((d, name))
-                    self.versions.append(d[name])
-        scale, shift = _bn_eval_affine(bn)
-        self.keep.append((scale, shift))
-        return scale.data_ptr(), shift.data_ptr()
+        got = ops.bn_args(bn) if _eval_bn(bn) else None
+        _require(got is not None)
+        args, refs = got
+        self.refs.extend(refs)
+        self.norms.append(bn)
+        self.keep.append(args)
+        return ctypes.addressof(args)
 
     def _linear(self, lin, supported):
         _require(type(lin) is nn.Linear and lin.bias is not None
@@ -119,8 +114,8 @@ class NativeBackbone:
                 _require(up.proj_skip[0].out_features == st.c_out)
                 st.w, st.b = self._linear(up.proj[0], ops.pool_stage_supported)
                 st.w_skip, st.b_skip = self._linear(up.proj_skip[0], ops.pool_stage_supported)
-                st.scale, st.shift = self._bn(up.proj[1])
-                st.scale_skip, st.shift_skip = self._bn(up.proj_skip[1])
+                st.bn = self._bn(up.proj[1])
+                st.bn_skip = self._bn(up.proj_skip[1])
             elif s > 0:
                 _require(mods and type(mods[0]) is M.SerializedPooling)
                 down = mods.pop(0)
@@ -128,7 +123,7 @@ class NativeBackbone:
                          and _exact_gelu(down.act[0]))
                 st.c_in, st.c_out = down.proj.in_features, down.proj.out_features
                 st.w, st.b = self._linear(down.proj, ops.pool_stage_supported)
-                st.scale, st.shift = self._bn(down.norm[0])
+                st.bn = self._bn(down.norm[0])
                 st.pooling_depth, st.reduce = down.pooling_depth(), ops.REDUCE_IDS[down.reduce]
                 self.pools.append(down)
             blocks = (_lib.BlockArgs * max(1, len(mods)))()
@@ -158,6 +153,7 @@ class NativeBackbone:
                         t.patch_size if t.enable_flash else t.patch_size_max))
         for p in self.pools:
             got.append((p.stride, p.reduce))
+        got.extend([bn.eps for bn in self.norms])
         return got
 
     def current(self):
@@ -166,7 +162,6 @@ class NativeBackbone:
         return (len(children) == len(self.children) and all(map(operator.is_, children, self.children))
                 and all(map(operator.is_, map(dict.get, self.owners, self.names), self.tensors))
                 and list(map(torch.Tensor.data_ptr, self.tensors)) == self.ptrs
-                and list(map(_VERSION, self.versions)) == self.version
                 and self._settings() == self.settings)
 
     def observed(self):

@@ -151,6 +151,8 @@ private:
         return (int)least;
     }
     int pad_level(BbLevel& l, int patch, Arena& mem, cudaStream_t stream, int64_t* pad, int64_t* unpad, int32_t* cu);
+    const float *stem_scale_ = a_.stem_scale, *stem_shift_ = a_.stem_shift;
+    int norms(BnJobs* jobs);
     template <typename F>
     int each_weight(F&& f);
     int split_weights();
@@ -181,6 +183,41 @@ int Pass::pad_level(BbLevel& l, int patch, Arena& mem, cudaStream_t stream, int6
     l.patch = patch;
     l.n_seq = (int)n_seq;
     return ptv3_pad_plan(l.offset, a_.n_scenes, patch, l.n, n_pad, (int)n_seq, l.pad, l.unpad, l.cu, a_.status, stream);
+}
+
+// BatchNorm layers as scale and shift, computed for this pass (as the weights below): where they will lie
+int Pass::norms(BnJobs* jobs)
+{
+    constexpr int MOST = 1 + 3 * BB_MAX_STAGES;
+    static_assert(MOST <= BN_JOBS, "one launch holds them");
+    ptv3_bn_args layers[MOST];
+    const float** slots[MOST][2];
+    int count = 0;
+    size_t floats = 0;
+    auto add = [&](const ptv3_bn_args* bn, int channels, const float*& scale, const float*& shift) {
+        if (!bn) return PTV3_OK;
+        PTV3_REQUIRE(bn->channels == channels, PTV3_ERR_INVALID_ARGUMENT,
+                     "ptv3_backbone_fwd: BatchNorm over %d channels where %d go in", bn->channels, channels);
+        slots[count][0] = &scale;
+        slots[count][1] = &shift;
+        layers[count++] = *bn;
+        floats += 2 * (size_t)channels;
+        return PTV3_OK;
+    };
+    BB_STEP(add(a_.stem_bn, a_.stem_c_out, stem_scale_, stem_shift_));
+    for (int s = 1; s < a_.n_enc; ++s) BB_STEP(add(enc_[s].bn, enc_[s].c_out, enc_[s].scale, enc_[s].shift));
+    for (int d = 0; d < a_.n_dec; ++d) {
+        BB_STEP(add(dec_[d].bn, dec_[d].c_out, dec_[d].scale, dec_[d].shift));
+        BB_STEP(add(dec_[d].bn_skip, dec_[d].c_out, dec_[d].scale_skip, dec_[d].shift_skip));
+    }
+    float* out = count ? mem_.take<float>(floats) : nullptr;
+    if (count && !out) return out_of_memory();
+    BB_STEP(bn_jobs(layers, count, out, jobs));
+    for (int i = 0; i < count; ++i) {
+        *slots[i][0] = jobs->out[i];
+        *slots[i][1] = jobs->out[i] + layers[i].channels;
+    }
+    return PTV3_OK;
 }
 
 // f(pointer, rows, inner dimension) of every weight that enters a matrix product; `blocks_` holds the blocks
@@ -277,7 +314,9 @@ int Pass::finest()
     char* index_ws = mem_.take<char>(voxel_index_bytes(a_.n));
     char* wt = mem_.take<char>(conv_direct_scratch_bytes(a_.n, a_.stem_ksize));
     if (!index_ws || !wt) return out_of_memory();
-    BB_STEP(ptv3_batch_indices(a_.offset, a_.n_scenes, a_.grid_coord, a_.n, nullptr, a_.indices, main_));
+    BnJobs bn;
+    BB_STEP(norms(&bn));
+    BB_STEP(batch_indices_and_norms(a_.offset, a_.n_scenes, a_.grid_coord, a_.n, a_.indices, bn, main_));
     VoxelIndex vi;
     BB_STEP(build_voxel_index(a_.indices, a_.n, index_ws, a_.status, main_, &vi));
     BB_CUDA(events_.record(main_, &indexed));
@@ -293,7 +332,7 @@ int Pass::finest()
     BB_CUDA(cudaStreamWaitEvent(main_, sorted, 0));
     void* feat = mem_.take<char>((size_t)a_.n * a_.stem_c_out * esize_);
     if (!feat) return out_of_memory();
-    BB_STEP(conv_direct_from_index(vi, a_.feat, a_.indices, a_.stem_weight, a_.stem_scale, a_.stem_shift, feat, a_.order,
+    BB_STEP(conv_direct_from_index(vi, a_.feat, a_.indices, a_.stem_weight, stem_scale_, stem_shift_, feat, a_.order,
                                    a_.n, a_.stem_c_in, a_.stem_c_out, a_.stem_ksize, a_.dtype, a_.status, wt, main_));
     l.feat = feat;
     return PTV3_OK;

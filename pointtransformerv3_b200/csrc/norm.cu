@@ -11,6 +11,7 @@
 // intermediate that the unfused sequence would write is rounded to the element
 // type exactly where that sequence rounds it.  HBM-bound: each tensor is read
 // or written once, with 16-byte accesses; a row is owned by 4..32 lanes.
+#include "bn.cuh"
 #include "common.cuh"
 #include "vec.cuh"
 #include "../../include/ptv3_b200.h"
@@ -144,6 +145,24 @@ static int dispatch_add_ln(const void* x, const void* residual, const void* g1, 
     return check_launch("ptv3_add_layernorm_fwd");
 }
 
+__global__ void __launch_bounds__(128) bn_affine_kernel(const __grid_constant__ BnJobs jobs) { bn_layer(jobs, blockIdx.x); }
+
+int bn_jobs(const ptv3_bn_args* layers, int count, float* out, BnJobs* jobs)
+{
+    auto known = [](int dtype) { return dtype == PTV3_DTYPE_F32 || dtype == PTV3_DTYPE_BF16; };
+    jobs->count = count < BN_JOBS ? count : BN_JOBS;
+    for (int i = 0; i < jobs->count; ++i) {
+        const ptv3_bn_args& l = layers[i];
+        PTV3_REQUIRE(l.channels >= 1 && l.mean && l.var && known(l.mean_dtype) && known(l.var_dtype) &&
+                         (!l.weight || known(l.weight_dtype)) && (!l.bias || known(l.bias_dtype)),
+                     PTV3_ERR_INVALID_ARGUMENT, "BatchNorm of %d channels: pointers or types", l.channels);
+        jobs->layer[i] = l;
+        jobs->out[i] = out;
+        out += 2 * (size_t)l.channels;
+    }
+    return PTV3_OK;
+}
+
 }  // namespace ptv3
 
 extern "C" int ptv3_add_layernorm_fwd(const void* x, const void* residual, const void* ln1_weight,
@@ -172,4 +191,24 @@ extern "C" int ptv3_add_layernorm_fwd(const void* x, const void* residual, const
                                       ln2_bias, ln2_eps, norm_out, n, channels, (cudaStream_t)stream);
     return dispatch_add_ln<__nv_bfloat16>(x, residual, ln1_weight, ln1_bias, ln1_eps, sum_out, ln2_weight,
                                           ln2_bias, ln2_eps, norm_out, n, channels, (cudaStream_t)stream);
+}
+
+extern "C" int ptv3_bn_affine(const ptv3_bn_args* layers, int count, float* out, void* stream)
+{
+    using namespace ptv3;
+    PTV3_REQUIRE(count >= 0 && (count == 0 || (layers && out)), PTV3_ERR_INVALID_ARGUMENT,
+                 "ptv3_bn_affine: null pointer or bad count");
+    while (count > 0) {
+        BnJobs jobs;
+        int rc = bn_jobs(layers, count, out, &jobs);
+        if (rc != PTV3_OK) return rc;
+        bn_affine_kernel<<<jobs.count, 128, 0, (cudaStream_t)stream>>>(jobs);
+        count_launches(1);
+        rc = check_launch("ptv3_bn_affine");
+        if (rc != PTV3_OK) return rc;
+        out = jobs.out[jobs.count - 1] + 2 * (size_t)layers[jobs.count - 1].channels;
+        layers += jobs.count;
+        count -= jobs.count;
+    }
+    return PTV3_OK;
 }

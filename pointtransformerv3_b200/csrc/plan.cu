@@ -210,15 +210,28 @@ static PoolWs pool_ws(int k, int64_t n, int B)
 // batch index of every point from the scene offsets, and the (batch, x, y, z) rows
 // of the sparse tensor (model.py:35-40 and :150-152)
 // ----------------------------------------------------------------------------
+// NORMS: the last blocks turn a BatchNorm layer each into scale and shift, which costs a pass no launch of its own
+struct NoNorms {};
+__device__ __forceinline__ int norm_blocks(const NoNorms&) { return 0; }
+__device__ __forceinline__ int norm_blocks(const BnJobs& norms) { return norms.count; }
+__device__ __forceinline__ void norm_block(const NoNorms&, int) {}
+__device__ __forceinline__ void norm_block(const BnJobs& norms, int i) { bn_layer(norms, i); }
+
+template <typename Norms>
 __global__ void __launch_bounds__(256) batch_indices_kernel(const int64_t* __restrict__ offset, int B,
                                                             const int32_t* __restrict__ grid_coord, int64_t n,
-                                                            int64_t* __restrict__ batch,
-                                                            int32_t* __restrict__ indices)
+                                                            int64_t* __restrict__ batch, int32_t* __restrict__ indices,
+                                                            const __grid_constant__ Norms norms)
 {
     extern __shared__ int64_t sm[];      // B scene ends
+    const int blocks = (int)gridDim.x - norm_blocks(norms);
+    if ((int)blockIdx.x >= blocks) {
+        norm_block(norms, (int)blockIdx.x - blocks);
+        return;
+    }
     for (int s = threadIdx.x; s < B; s += blockDim.x) sm[s] = offset[s];
     __syncthreads();
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const int64_t stride = (int64_t)blocks * blockDim.x;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += stride) {
         int lo = 0, hi = B - 1;          // first scene whose end lies beyond i (the last one at worst)
         while (lo < hi) {
@@ -268,6 +281,32 @@ __global__ void __launch_bounds__(256) batch_stats_kernel(const int32_t* __restr
     }
 }
 
+static int check_batch_indices(const int64_t* offset, int n_scenes, const int32_t* grid_coord, int64_t n,
+                               const int32_t* indices)
+{
+    PTV3_REQUIRE(n_scenes >= 1 && n_scenes <= PAD_MAX_SCENES, PTV3_ERR_UNSUPPORTED,
+                 "ptv3_batch_indices: %d scenes outside [1, %d]", n_scenes, PAD_MAX_SCENES);
+    PTV3_REQUIRE(n >= 0, PTV3_ERR_INVALID_ARGUMENT, "ptv3_batch_indices: n < 0");
+    PTV3_REQUIRE(n == 0 || (offset && (!indices || grid_coord)), PTV3_ERR_INVALID_ARGUMENT,
+                 "ptv3_batch_indices: null pointer");
+    PTV3_REQUIRE(((uintptr_t)indices & 15) == 0, PTV3_ERR_INVALID_ARGUMENT,
+                 "ptv3_batch_indices: indices must be 16-byte aligned");
+    return PTV3_OK;
+}
+
+static unsigned batch_indices_blocks(int64_t n) { return (unsigned)((n + 255) / 256 > 148 * 8 ? 148 * 8 : (n + 255) / 256); }
+
+int batch_indices_and_norms(const int64_t* offset, int n_scenes, const int32_t* grid_coord, int64_t n, int32_t* indices,
+                            const BnJobs& norms, cudaStream_t stream)
+{
+    const int rc = check_batch_indices(offset, n_scenes, grid_coord, n, indices);
+    if (rc != PTV3_OK) return rc;
+    batch_indices_kernel<<<batch_indices_blocks(n) + norms.count, 256, (size_t)n_scenes * sizeof(int64_t), stream>>>(
+        offset, n_scenes, grid_coord, n, nullptr, indices, norms);
+    count_launches(1);
+    return check_launch("ptv3_batch_indices");
+}
+
 }  // namespace ptv3
 
 extern "C" int ptv3_batch_stats(const int32_t* grid_coord, int64_t n, const int64_t* offset, int n_scenes,
@@ -291,18 +330,11 @@ extern "C" int ptv3_batch_indices(const int64_t* offset, int n_scenes, const int
                                   int64_t* batch, int32_t* indices, void* stream)
 {
     using namespace ptv3;
-    PTV3_REQUIRE(n_scenes >= 1 && n_scenes <= PAD_MAX_SCENES, PTV3_ERR_UNSUPPORTED,
-                 "ptv3_batch_indices: %d scenes outside [1, %d]", n_scenes, PAD_MAX_SCENES);
-    PTV3_REQUIRE(n >= 0, PTV3_ERR_INVALID_ARGUMENT, "ptv3_batch_indices: n < 0");
-    if (n == 0 || (!batch && !indices)) return PTV3_OK;
-    PTV3_REQUIRE(offset && (!indices || grid_coord), PTV3_ERR_INVALID_ARGUMENT,
-                 "ptv3_batch_indices: null pointer");
-    PTV3_REQUIRE(((uintptr_t)indices & 15) == 0, PTV3_ERR_INVALID_ARGUMENT,
-                 "ptv3_batch_indices: indices must be 16-byte aligned");
-    int64_t blocks = (n + 255) / 256;
-    if (blocks > 148 * 8) blocks = 148 * 8;
-    batch_indices_kernel<<<(unsigned)blocks, 256, (size_t)n_scenes * sizeof(int64_t), (cudaStream_t)stream>>>(
-        offset, n_scenes, grid_coord, n, batch, indices);
+    if (n == 0 || (n > 0 && !batch && !indices)) return check_batch_indices(offset, n_scenes, grid_coord, 0, nullptr);
+    const int rc = check_batch_indices(offset, n_scenes, grid_coord, n, indices);
+    if (rc != PTV3_OK) return rc;
+    batch_indices_kernel<<<batch_indices_blocks(n), 256, (size_t)n_scenes * sizeof(int64_t), (cudaStream_t)stream>>>(
+        offset, n_scenes, grid_coord, n, batch, indices, NoNorms());
     count_launches(1);
     return check_launch("ptv3_batch_indices");
 }

@@ -1,5 +1,6 @@
 // Index-side launches that the one-call backbone queues itself.
 #pragma once
+#include "bn.cuh"
 #include "common.cuh"
 #include "voxel_index.cuh"
 
@@ -11,6 +12,10 @@ int pool_plan(const int64_t* code, const int64_t* order, const int32_t* grid_coo
               int64_t* head, int64_t* pooled_code, int64_t* pooled_order, int64_t* pooled_inverse,
               int32_t* pooled_grid_coord, int64_t* pooled_batch, int64_t* meta, int64_t* meta_host,
               int64_t* pooled_offset, uint32_t* status, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+
+// ptv3_batch_indices (indices only) with the network's BatchNorm layers done beside it
+int batch_indices_and_norms(const int64_t* offset, int n_scenes, const int32_t* grid_coord, int64_t n, int32_t* indices,
+                            const BnJobs& norms, cudaStream_t stream);
 
 // kernel map of a voxel set whose index exists already
 int kmap_from_index(const VoxelIndex& vi, const int32_t* indices, int64_t n, int ksize, const int64_t* row_order,

@@ -118,22 +118,6 @@ class PDNorm(PointModule):
         return point
 
 
-def _bn_eval_affine(bn):
-    """Per-channel (scale, shift) of a BatchNorm1d in eval mode, fp32.  Cached on
-    the module and recomputed when a parameter or buffer was modified or moved."""
-    tensors = (bn.weight, bn.bias, bn.running_mean, bn.running_var)
-    key = tuple((t._version, t.data_ptr(), t.dtype) if t is not None else None for t in tensors)
-    cached = bn.__dict__.get("_ptv3_affine")
-    if cached is not None and cached[0] == key:
-        return cached[1], cached[2]
-    w = bn.weight.float() if bn.weight is not None else torch.ones_like(bn.running_var)
-    b = bn.bias.float() if bn.bias is not None else torch.zeros_like(bn.running_var)
-    scale = (w * torch.rsqrt(bn.running_var.float() + bn.eps)).contiguous()
-    shift = (b - bn.running_mean.float() * scale).contiguous()
-    bn.__dict__["_ptv3_affine"] = (key, scale, shift)
-    return scale, shift
-
-
 def _is_bn_gelu(norm, act):
     """True when (norm, act) is the BatchNorm1d(eval) + exact GELU pair the fused
     pooling kernels implement."""
@@ -520,7 +504,7 @@ class SerializedPooling(PointModule):
         fused = _is_bn_gelu(self.norm, self.act)
         scale = shift = None
         if fused:
-            scale, shift = _bn_eval_affine(self.norm[0])
+            scale, shift = ops.bn_affine(self.norm[0])
         src_coord = point.coord if "coord" in point.keys() else None
         if _single_call_ok(point.feat, self.proj):
             # projection and reduction queued by one C call
@@ -585,8 +569,8 @@ class SerializedUnpooling(PointModule):
         parent = point.pop("pooling_parent")
         inverse = point.pop("pooling_inverse")
         if self._fusable():
-            cs, cb = _bn_eval_affine(self.proj[1])
-            ss, sb = _bn_eval_affine(self.proj_skip[1])
+            cs, cb = ops.bn_affine(self.proj[1])
+            ss, sb = ops.bn_affine(self.proj_skip[1])
             child_lin = None
             if (not self.traceable and _single_call_ok(point.feat, self.proj[0])
                     and _single_call_ok(parent.feat, self.proj_skip[0])):
@@ -641,7 +625,7 @@ class Embedding(PointModule):
                 and type(mods[1]) is nn.BatchNorm1d and not mods[1].training and mods[1].track_running_stats
                 and type(mods[2]) is nn.GELU and getattr(mods[2], "approximate", "none") == "none"
                 and "sparse_conv_feat" in point.keys()):
-            scale, shift = _bn_eval_affine(mods[1])
+            scale, shift = ops.bn_affine(mods[1])
             point.sparse_conv_feat = conv(point.sparse_conv_feat, scale, shift, True)
             point.feat = point.sparse_conv_feat.features
             return point

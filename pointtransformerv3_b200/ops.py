@@ -477,6 +477,41 @@ def add_layernorm(x, residual=None, ln1=None, ln2=None, want_sum=True):
     return s, y
 
 
+def bn_args(bn):
+    """(the ptv3_bn_args of a BatchNorm1d with running statistics, (owner dict, name) of each of its tensors), or
+    None where a tensor has another form than the kernel reads."""
+    args, refs = _lib.BnArgs(), []
+    for field, owner, name in (("weight", bn._parameters, "weight"), ("bias", bn._parameters, "bias"),
+                               ("mean", bn._buffers, "running_mean"), ("var", bn._buffers, "running_var")):
+        t = owner[name]
+        if t is None:
+            if field in ("mean", "var"):
+                return None
+            continue
+        if not t.is_cuda or t.dtype not in _lib.DTYPE_IDS or not t.is_contiguous() or t.numel() != bn.num_features:
+            return None
+        setattr(args, field, t.data_ptr())
+        setattr(args, field + "_dtype", _lib.DTYPE_IDS[t.dtype])
+        refs.append((owner, name))
+    args.channels, args.eps = bn.num_features, bn.eps
+    return args, refs
+
+
+def bn_affine(bn):
+    """Per-channel (scale, shift) of a BatchNorm1d in eval mode, fp32, from the values that its parameters and
+    buffers have now."""
+    got = bn_args(bn)
+    if got is None:                      # other types or layouts
+        w = bn.weight.float() if bn.weight is not None else torch.ones_like(bn.running_var, dtype=torch.float32)
+        b = bn.bias.float() if bn.bias is not None else torch.zeros_like(bn.running_var, dtype=torch.float32)
+        scale = (w * torch.rsqrt(bn.running_var.float() + bn.eps)).contiguous()
+        return scale, (b - bn.running_mean.float() * scale).contiguous()
+    c = bn.num_features
+    out = torch.empty(2 * c, dtype=torch.float32, device=bn.running_var.device)
+    _lib.check(_lib.load().ptv3_bn_affine(ctypes.byref(got[0]), 1, out.data_ptr(), _lib.stream()), "ptv3_bn_affine")
+    return out[:c], out[c:]
+
+
 def subm_conv_direct(feat, indices, weight, bias=None, bn_scale=None, bn_shift=None, gelu=False,
                      row_order=None, status=None):
     """Submanifold convolution for few input channels / large kernels that probes

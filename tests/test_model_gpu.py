@@ -458,7 +458,9 @@ def test_network_changed_between_passes(change):
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("name", ["embedding.stem.conv.weight", "enc.enc0.block0.cpe.0.weight", "enc.enc1.down.proj.weight",
-                                  "dec.dec0.up.proj_skip.0.weight", "dec.dec0.block0.mlp.0.fc1.weight"])
+                                  "dec.dec0.up.proj_skip.0.weight", "dec.dec0.block0.mlp.0.fc1.weight",
+                                  "embedding.stem.norm.running_mean", "enc.enc2.down.norm.0.weight",
+                                  "dec.dec1.up.proj.1.running_var", "dec.dec0.up.proj_skip.1.bias"])
 def test_values_written_through_data_between_passes(name, dtype):
     """A write through ``.data`` (weight averaging, a broadcast) moves neither a tensor's identity nor its address
     nor its version counter: the next pass sees the new values all the same, on another stream too."""
@@ -479,14 +481,14 @@ def test_values_written_through_data_between_passes(name, dtype):
         before = run(net)
     assert backbone.of(net)[0] is not None
     for n in (net, fresh):
-        tensor = n.get_parameter(name)
+        tensor = n.state_dict()[name]
         version = tensor._version
         tensor.data.mul_(2)
         assert tensor._version == version
     got, ref = run(net), run(fresh)
     assert torch.equal(got, ref) and not torch.equal(got, before)
     side = torch.cuda.Stream()
-    net.get_parameter(name).data.mul_(0.5)
+    net.state_dict()[name].data.mul_(0.5)
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
         assert torch.equal(run(net), before)

@@ -6,7 +6,7 @@ import torch.nn.functional as F
 
 from helpers import TOL, assert_close, rel_l2, small_batch
 from oracle import ptv3_oracle as O
-from pointtransformerv3_b200 import ops
+from pointtransformerv3_b200 import _lib, ops
 
 pytestmark = pytest.mark.gpu
 ORDERS = ["z", "z-trans", "hilbert", "hilbert-trans"]
@@ -807,6 +807,38 @@ def test_subm_conv_on_split_floats(n, cin, cout):
     rows = torch.cat([feat.double(), feat.new_zeros(1, cin).double()])[nbr.long()]          # -1 -> the zero row
     ref = torch.einsum("onc,doc->nd", rows, w.double().reshape(cout, 27, cin)) + b.double()
     assert rel_l2(got.double(), ref) < 1.5 * rel_l2(plain.double(), ref) + 1e-7
+
+
+@pytest.mark.parametrize("count", [1, 48, 49, 100])
+@pytest.mark.parametrize("param,buffer,affine", [(torch.float32, torch.float32, True), (torch.bfloat16, torch.bfloat16, True),
+                                                 (torch.bfloat16, torch.float32, True), (None, torch.float32, False)])
+def test_batchnorm_as_scale_and_shift(count, param, buffer, affine):
+    """One launch for several layers of different widths, mixed types, and both sides of what a launch holds:
+    against float64 (two roundings of the scale, two of the shift)."""
+    g = torch.Generator().manual_seed(count)
+    layers = []
+    for i in range(count):
+        bn = torch.nn.BatchNorm1d((1, 32, 200)[i % 3], eps=1e-3, affine=affine)
+        bn.running_mean = torch.randn(bn.num_features, generator=g).to(buffer)
+        bn.running_var = (torch.rand(bn.num_features, generator=g) * 3).to(buffer)
+        if affine:
+            bn.weight.data = torch.randn(bn.num_features, generator=g).to(param)
+            bn.bias.data = torch.randn(bn.num_features, generator=g).to(param)
+        layers.append(bn.cuda().eval())
+    args = (_lib.BnArgs * count)(*[ops.bn_args(bn)[0] for bn in layers])
+    out = torch.empty(2 * sum(bn.num_features for bn in layers), device="cuda")
+    _lib.check(_lib.load().ptv3_bn_affine(args, count, out.data_ptr(), _lib.stream()), "ptv3_bn_affine")
+    at = 0
+    for bn in layers:
+        c = bn.num_features
+        scale = (bn.running_var.double() + bn.eps).rsqrt() * (bn.weight.double() if affine else 1.0)
+        shift = (bn.bias.double() if affine else 0.0) - bn.running_mean.double() * scale
+        assert ((out[at:at + c] - scale).abs() <= 2 ** -22 * scale.abs()).all()
+        bound = 2 ** -22 * ((bn.running_mean.double() * scale).abs() + shift.abs())
+        assert ((out[at + c:at + 2 * c] - shift).abs() <= bound).all()
+        one = ops.bn_affine(bn)
+        assert torch.equal(one[0], out[at:at + c]) and torch.equal(one[1], out[at + c:at + 2 * c])
+        at += 2 * c
 
 
 @pytest.mark.parametrize("op", ["linear_short", "linear", "gemm_short", "gemm_streamed", "gemm_resident", "linear_ln",
