@@ -67,7 +67,9 @@ long long ptv3_launch_count(void);
 /* clears a device status word in stream order (a memset, not a kernel) */
 int ptv3_status_reset(uint32_t* status, void* stream);
 /* stores the status word, then 1, in page-locked HOST memory the device can address (2 int64) once the
-   work queued before it has run; the caller zeroes the second word and polls it */
+   work queued before it has run; the caller zeroes the second word and polls it.  (Here and below: the words
+   belong to the kernel from its launch until its "done" word has been seen; none of them may be written or
+   given to another call before that) */
 int ptv3_status_report(const uint32_t* status, int64_t* host, void* stream);
 /* polls a word of such memory until it is not zero; after two seconds it waits for the stream instead, and
    fails if the word is still zero then */

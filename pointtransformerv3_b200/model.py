@@ -737,31 +737,38 @@ class PointTransformerV3(PointModule):
         return _PLAN_STREAMS[key]
 
     def _native(self, point, known_depth):
-        """The one-call form of this forward, where it covers the network and the input: bf16 or fp32 on the GPU,
-        standard modules, nobody hooked onto a single module, no per-operator timing."""
+        """(native, checked, stats): the one-call form of this forward, where it covers the network and the input
+        (bf16 or fp32 on the GPU, standard modules, nobody hooked onto a single module, no per-operator timing), else
+        None; and the bounds of the batch where they are not known and on their way."""
         feat = point.feat
         if (feat.dtype not in (torch.bfloat16, torch.float32) or not feat.is_cuda or feat.dim() != 2
                 or feat.shape[0] == 0 or ops.TIMERS is not None or feat.requires_grad
                 or (feat.dtype == torch.float32 and feat.shape[0] > 65535 * 128)):
-            return None
+            return None, False, None
         # the batch's bounds are on their way while the host looks the network over
         point._ensure_grid_coord()
         stats = None
         if "sparse_shape" not in point.keys() or not known_depth or "_counts" not in point.keys():
             stats = ops.BatchStats(point.grid_coord, point.offset)
         native, checked = backbone.of(self)
-        if native is None or feat.dtype != native.dtype or feat.shape[1] != native.width_in:
-            return None
+        if native is not None and (feat.dtype != native.dtype or feat.shape[1] != native.width_in):
+            native = None
         return native, checked, stats
+
+    @staticmethod
+    def _take_bounds(point, depth, top, ends):
+        """Puts the largest coordinates and the offsets of a batch where the point lacks them; the code depth."""
+        if depth is None:
+            depth = max(top).bit_length()
+        if "sparse_shape" not in point.keys():
+            point["sparse_shape"] = [v + 96 for v in top]
+            point["_shape_pad"] = 96
+        point["_counts"] = [b - a for a, b in zip([0] + ends, ends)]
+        return depth
 
     def _forward_native(self, native, checked, stats, point, depth):
         if stats is not None:
-            top, ends = stats.result()
-            if depth is None:
-                depth = max(top).bit_length()
-            if "sparse_shape" not in point.keys():
-                point["sparse_shape"] = [v + 96 for v in top]
-            point["_counts"] = [b - a for a, b in zip([0] + ends, ends)]
+            depth = self._take_bounds(point, depth, *stats.result())
         point["_shape_pad"] = point.get("_shape_pad", 96)
         depth = max(int(depth), 1)
         assert depth * 3 + len(point["_counts"]).bit_length() <= 63
@@ -802,13 +809,13 @@ class PointTransformerV3(PointModule):
         status = point.device_status()
         point["_defer_status"] = True
         feat_dtype = point.feat.dtype
-        native = self._native(point, depth is not None)
-        done = None if native is None else self._forward_native(*native, point, depth)
+        native, checked, stats = self._native(point, depth is not None)
+        done = None if native is None else self._forward_native(native, checked, stats, point, depth)
         if native is not None and done is None:
             # the network changed since its last pass: looked over first, and possibly of another form
             status = point["_status"] = ops.new_status(point.feat.device)
-            native = self._native(point, depth is not None)
-            done = None if native is None else self._forward_native(*native, point, depth)
+            native, checked, stats = self._native(point, depth is not None)
+            done = None if native is None else self._forward_native(native, checked, stats, point, depth)
         if done is not None:
             return done
         # -- Schedule.  Serialization and the pooling plans need only coordinates.  They run on a
@@ -832,15 +839,13 @@ class PointTransformerV3(PointModule):
                 # model.py:162-164); the shapes of the coarse levels then follow without reading the device
                 point["_shape_pad"] = 96
             if "sparse_shape" not in point.keys() or depth is None or "_counts" not in point.keys():
-                stats = torch.cat([point.grid_coord.max(0).values.to(torch.int64), point.offset.to(torch.int64)])
-                stats = stats.tolist()                                     # one host read
-                if depth is None:
-                    depth = max(stats[:3]).bit_length()
-                if "sparse_shape" not in point.keys():
-                    point["sparse_shape"] = [v + 96 for v in stats[:3]]
-                    point["_shape_pad"] = 96
-                off = [0] + stats[3:]
-                point["_counts"] = [off[i + 1] - off[i] for i in range(len(off) - 1)]
+                if stats is not None:
+                    top, ends = stats.result()
+                else:
+                    read = torch.cat([point.grid_coord.max(0).values.to(torch.int64), point.offset.to(torch.int64)])
+                    read = read.tolist()                                   # one host read
+                    top, ends = read[:3], read[3:]
+                depth = self._take_bounds(point, depth, top, ends)
             point.serialization(order=self.order, depth=depth, shuffle_orders=self.shuffle_orders)
             point["_sparse_indices"] = point._sparse_indices()
         # what was made there is consumed (and later dropped) by work queued on the main stream

@@ -121,9 +121,9 @@ def read_status(status):
     """The device status word, once the work queued on the current stream has run: stored in mapped
     host memory by a kernel and polled, which takes a third of the time of a copy and a stream wait."""
     lib, stream = _lib.load(), _lib.stream()
-    host = _host_words(2, "status", stream)
-    host.words[1] = 0
+    host = _host_words(2, "status", stream).begin(lib, stream)
     _lib.check(lib.ptv3_status_report(status.data_ptr(), host.address, stream), "ptv3_status_report")
+    host.pending = True
     return host.wait(lib, stream)[0]
 
 
@@ -331,14 +331,14 @@ def pool_plan(code, order, grid_coord, batch, n_scenes, pooling_depth, row_perm=
     # the plan's last kernel; the host polls the "done" word behind them (a stream wait through
     # the driver takes several times longer to notice the end of a kernel)
     stream = _lib.stream()
-    meta_host = _host_words(3 + n_scenes, "pool_plan.meta", stream)
-    meta_host.words[2 + n_scenes] = 0
+    meta_host = _host_words(3 + n_scenes, "pool_plan.meta", stream).begin(lib, stream)
     _lib.check(lib.ptv3_pool_plan(_lib.ptr(code), _lib.ptr(order), _lib.ptr(grid_coord), _lib.ptr(batch),
                                   k, n, n_scenes, int(pooling_depth), perm, _lib.ptr(cluster),
                                   _lib.ptr(idx_ptr), _lib.ptr(head), _lib.ptr(pcode), _lib.ptr(porder),
                                   _lib.ptr(pinv), _lib.ptr(pgrid), _lib.ptr(pbatch), _lib.ptr(meta),
                                   meta_host.address, _lib.ptr(status), _lib.ptr(ws), nbytes, stream),
                "ptv3_pool_plan")
+    meta_host.pending = True
     host = meta_host.wait(lib, stream)[:-1]                          # the one wait
     if host[-1]:
         raise _lib.Ptv3Error("device status 0x%x (read after ptv3_pool_plan; the word is shared by "
@@ -367,10 +367,10 @@ class BatchStats:
         grid_coord = grid_coord.to(torch.int32).contiguous()
         offset = offset.to(torch.int64).contiguous()
         n_scenes = offset.shape[0]
-        host = self.host = _host_words(4 + n_scenes, "batch_stats", self.stream, offset.device)
-        host.words[3 + n_scenes] = 0
+        host = self.host = _host_words(4 + n_scenes, "batch_stats", self.stream, offset.device).begin(self.lib, self.stream)
         _lib.check(self.lib.ptv3_batch_stats(grid_coord.data_ptr(), grid_coord.shape[0], offset.data_ptr(), n_scenes,
                                              host.address, host.scratch.data_ptr(), self.stream), "ptv3_batch_stats")
+        host.pending = True
         self.keep = (grid_coord, offset)
 
     def result(self):
@@ -381,7 +381,11 @@ class BatchStats:
 
 class _HostWords:
     """Page-locked int64 words that kernels store results in, the last one meaning "done"; with a few
-    bytes of device scratch (0x80 each) for kernels that count their blocks."""
+    bytes of device scratch (0x80 each) for kernels that count their blocks.  From its launch until ``wait`` has
+    seen it a kernel owns them (``pending``): a result that its caller gave up is waited for by the next one,
+    who would otherwise take that kernel's "done" for its own."""
+
+    pending = False
 
     def __init__(self, n, device):
         with torch.inference_mode(False):      # a plain tensor: it is written in and out of inference mode
@@ -391,8 +395,15 @@ class _HostWords:
         self.words = (ctypes.c_int64 * n).from_address(self.address)
         self.last = self.address + 8 * (n - 1)
 
+    def begin(self, lib, stream):
+        if self.pending:
+            self.wait(lib, stream)
+        self.words[len(self.words) - 1] = 0
+        return self
+
     def wait(self, lib, stream):
         _lib.check(lib.ptv3_host_wait(self.last, stream), "waiting for a result")
+        self.pending = False
         return self.words[:]
 
 
@@ -400,8 +411,7 @@ _HOST_WORDS = {}
 
 
 def _host_words(n, tag, stream, device=None):
-    """The words of a call site, host thread and CUDA stream (a caller waits for its result before it
-    comes back here, so calls that share all three do not overlap)."""
+    """The words of a call site, host thread and CUDA stream."""
     key = (tag, n, threading.get_ident(), stream, device)
     host = _HOST_WORDS.get(key)
     if host is None:
@@ -835,13 +845,13 @@ def voxelize(coord, feat, offset, grid_size):
     nbytes = lib.ptv3_voxelize_workspace_bytes(n)
     ws = _lib.workspace(nbytes, dev)
     stream = _lib.stream()
-    host = _host_words(3, "voxelize", stream)
-    host.words[2] = 0
+    host = _host_words(3, "voxelize", stream).begin(lib, stream)
     with timed("voxelize", 64.0 * n):
         _lib.check(lib.ptv3_voxelize(_lib.ptr(coord), n, float(grid_size), _lib.ptr(offset), n_scenes, _lib.ptr(small),
                                      _lib.ptr(keep), _lib.ptr(p2v), _lib.ptr(new_offset), host.address,
                                      _lib.ptr(small[4:]), _lib.ptr(status), _lib.ptr(ws), nbytes, _lib.stream()),
                    "ptv3_voxelize")
+    host.pending = True
     m, bits, _ = host.wait(lib, stream)
     if bits:
         raise _lib.Ptv3Error("ptv3_voxelize: device status 0x%x" % bits)

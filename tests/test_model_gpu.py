@@ -495,6 +495,37 @@ def test_values_written_through_data_between_passes(name, dtype):
 
 
 @pytest.mark.gpu
+def test_bounds_of_a_batch_are_read_once_in_either_form():
+    """A hooked network runs as a module tree: the bounds that were asked for before that was known serve it, and
+    no report is left that nobody waited for."""
+    from pointtransformerv3_b200 import ops
+    data = small_batch([900, 500], 9)
+    net = P.PointTransformerV3(in_channels=6, **SMALL_CFG)
+    weights.fill_state_dict(net, prefix="ptv3.")
+    net = net.eval().cuda().bfloat16()
+
+    def run():
+        torch.manual_seed(5)
+        with torch.inference_mode():
+            return net(cuda_data(data, torch.bfloat16))
+    ref, made = run(), []
+    handle = net.dec.dec0.block0.register_forward_hook(lambda *a: None)
+    run()                                # (finds the hook: a pass given up, then the module tree)
+    real = ops.BatchStats.result
+    ops.BatchStats.result = lambda self: made.append(self) or real(self)
+    try:
+        out = run()
+    finally:
+        ops.BatchStats.result = real
+        handle.remove()
+    assert len(made) == 1
+    assert not any(h.pending for h in ops._HOST_WORDS.values())
+    assert out.serialized_depth == ref.serialized_depth and out.sparse_shape == ref.sparse_shape
+    assert out["_counts"] == ref["_counts"] and torch.equal(out.serialized_order, ref.serialized_order)
+    assert rel_l2(out.feat, ref.feat) < 1e-2
+
+
+@pytest.mark.gpu
 def test_forward_with_host_metadata_and_deferred_status():
     """The optional entries that let a caller skip the host waits of a pass (scene sizes,
     code depth and sparse shape known on the host; status word read later) do not change
