@@ -364,6 +364,8 @@ class BatchStats:
     def __init__(self, grid_coord, offset):
         _lib.require_cuda(grid_coord, offset)
         self.lib, self.stream = _lib.load(), _lib.stream()
+        if grid_coord.dtype == torch.int64:        # beyond 32 bits: the bounds still say that it is too much
+            grid_coord = grid_coord.clamp(-2 ** 31, 2 ** 31 - 1)
         grid_coord = grid_coord.to(torch.int32).contiguous()
         offset = offset.to(torch.int64).contiguous()
         n_scenes = offset.shape[0]

@@ -186,3 +186,17 @@ def test_voxelize_in_one_call(sizes, width, dtype):
     assert torch.equal(data["row"], want["keep"])
     for key, full in (("coord", coord), ("grid_coord", grid), ("feat", feat)):
         assert torch.equal(data[key], full[want["keep"]]), key
+
+
+@pytest.mark.parametrize("far", [1 << 16, 1 << 31, 1 << 33, (1 << 40) + 5])
+def test_coordinates_beyond_the_code_are_refused(far):
+    """64-bit grid coordinates whose low 32 bits look harmless: the depth is taken from their real size."""
+    from pointtransformerv3_b200 import Point, PointTransformerV3
+    grid = torch.randint(0, 50, (64, 3)).cuda()
+    grid[7, 1] = far
+    offset = torch.tensor([64]).cuda()
+    with pytest.raises(AssertionError):
+        Point(grid_coord=grid, offset=offset).serialization(order=["z"])
+    net = PointTransformerV3(in_channels=6).eval().cuda().bfloat16()
+    with torch.inference_mode(), pytest.raises(AssertionError):
+        net(dict(feat=torch.zeros(64, 6).cuda().bfloat16(), grid_coord=grid, offset=offset))
