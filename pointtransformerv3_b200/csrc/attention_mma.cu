@@ -311,6 +311,9 @@ __global__ void __launch_bounds__(AM_THREADS, 3) attn_mma_d16_kernel(
     }
 }
 
+constexpr int AM_WAVE = 3 * SMS;                    // CTAs that run at once
+constexpr int AM_ENOUGH = AM_WAVE * 9 / 5;          // nearly two waves
+
 bool attn_mma_supported(int channels, int heads, int max_seqlen)
 {
     return channels % heads == 0 && channels / heads == AM_D && channels % 8 == 0 &&
@@ -327,15 +330,22 @@ int launch_attn_mma(const void* qkv, const int64_t* order, const int64_t* pad, c
     auto kern = packed_exp ? attn_mma_d16_kernel<true> : attn_mma_d16_kernel<false>;
     if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_attention_fwd: shared memory attribute");
-    // Queries of a sequence are sliced over CTAs, each of which gathers K and V again.  A launch wants two
+    // Queries of a sequence are sliced over CTAs, each of which gathers K and V again.  A launch wants nearly two
     // waves of three CTAs per SM, or one that is nearly full: fewer CTAs land unevenly on the SMs (a dependent
-    // launch fills the first ones that the kernel before it leaves), more gather more often.  us in
-    // 1 / 2 / 4 / 8 slices: 400 000 x 64 (1 564 pairs) 449 / 451 / 457 / 507, 105 000 x 64 (412) 133 / 133 / 136 / 144,
-    // 28 000 x 128 (224) 127 / 91 / 83 / 85, 2 200 x 512 (96) 70 / 56 / 42 / 44, 6 000 x 64 (24) 49 / 27 / 24 / 20.
+    // launch fills the first ones that the kernel before it leaves), more gather more often.  us in 1 / 2 / 4 / 8
+    // slices by (sequence, head) pairs, sequences of 1 024:
+    //      16   49 /  27 /  16 /  14        96   88 /  55 /  40 /  42       200   90 /  71 /  71 /  72
+    //      48   49 /  49 /  32 /  25       108   98 /  49 /  40 /  42       224  128 /  89 /  81 /  83
+    //      80   75 /  66 /  40 /  37       128  109 /  69 /  50 /  49       320  131 / 110 / 103 / 112
+    //     436  131 / 131 / 135 / 148       640  210 / 192 / 198 / 215     1 564  449 / 451 / 456 / 507
+    // The wave that is nearly full decides at 93 to 111 pairs (5 %) and costs nothing at 186 to 222 and above 412.
+    // The rule is behind the best of the four at 144 and 176 pairs (54 and 66 us, 50 and 61 in four slices), at
+    // 370 to 400 (131, 124 in four) and at 1 200 (368, 351 in two); elsewhere within 3 %.
     const int tiles = (max_seqlen + 15) / 16;
     const int64_t pairs = (int64_t)n_seq * H;
     int qsplit = 1;
-    while (qsplit < 8 && qsplit * AM_WARPS < tiles && pairs * qsplit < 800 && !(pairs * qsplit >= 370 && pairs * qsplit <= 444))
+    while (qsplit < 8 && qsplit * AM_WARPS < tiles && pairs * qsplit < AM_ENOUGH &&
+           !(pairs * qsplit >= AM_WAVE * 5 / 6 && pairs * qsplit <= AM_WAVE))
         qsplit *= 2;
     const dim3 grid(H * qsplit, n_seq);
     launch_dependent(kern, grid, dim3(AM_THREADS), smem, stream, (const __nv_bfloat16*)qkv, order, pad, unpad, cu,

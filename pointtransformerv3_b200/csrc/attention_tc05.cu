@@ -545,14 +545,14 @@ int launch_attn_tc05(const void* qkv, const int64_t* order, const int64_t* pad, 
     if (allow_smem(attn_tc05_d16_kernel) != cudaSuccess)
         return check_launch("ptv3_attention_fwd: shared memory attribute");
     // Query tiles of a patch can be sliced over CTAs (each gathers K and V again).  Pick the
-    // slicing with the shortest estimated time: waves of 148 CTAs, each taking one gather
+    // slicing with the shortest estimated time: waves of a CTA per SM, each taking one gather
     // (about 0.2 of a tile round) plus its rounds of up to four tiles.
     const int tiles = lpad / AT_BM;
     const long pairs = (long)n_seq * H;
     int qsplit = 1;
     double best = 0;
     for (int q = 1; q <= tiles; q *= 2) {
-        const long waves = (pairs * q + 147) / 148;
+        const long waves = (pairs * q + SMS - 1) / SMS;
         const int rounds = ((tiles + q - 1) / q + AT_WG - 1) / AT_WG;
         const double cost = (double)waves * (rounds + 0.2);
         if (q == 1 || cost < best) {

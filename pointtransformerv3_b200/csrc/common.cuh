@@ -44,6 +44,9 @@ struct Carver {
     }
 };
 
+// streaming multiprocessors of a B200: grids and the lines of dispatch rules are stated in them
+constexpr int SMS = 148;
+
 static inline int ceil_div(int64_t a, int64_t b) { return static_cast<int>((a + b - 1) / b); }
 
 // ---- programmatic dependent launch -------------------------------------------------------------

@@ -370,7 +370,7 @@ static int launch_conv_direct_mma(const void* feat, const int32_t* indices, cons
     const int rounds = (ksize * ksize + CDM_ROWS - 1) / CDM_ROWS, per_round = CDM_ROWS * ksize;
     uint4* rows = reinterpret_cast<uint4*>(static_cast<char*>(wt) + conv_direct_weight_bytes(ksize));
     const int64_t prepare = (std::max<int64_t>(n, rounds * per_round * 8 * cout) + 255) / 256;
-    conv_direct_prepare_kernel<<<(unsigned)std::min<int64_t>(prepare, 148 * 8), 256, 0, stream>>>(
+    conv_direct_prepare_kernel<<<(unsigned)std::min<int64_t>(prepare, SMS * 8), 256, 0, stream>>>(
         (const __nv_bfloat16*)weight, (__nv_bfloat16*)wt, cout, kvol, cin, rounds * per_round, (const __nv_bfloat16*)feat,
         rows, n);
     const size_t smem = (size_t)per_round * CD_TM * 16 + (size_t)per_round * 8 * (cout * 2 + 16);

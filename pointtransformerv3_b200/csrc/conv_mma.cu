@@ -348,10 +348,10 @@ int launch_conv_mma(const void* feat, const int32_t* nbr, const void* weight, co
     // few voxels: 64 x 64 tiles on 4 warps so that enough CTAs exist to fill the GPU
     const int64_t big_ctas = ((n + 127) / 128) * ((c_out + 127) / 128);
     if (c_out == 64) {
-        if (big_ctas * 2 < 2 * 148) return launch_one<64, 64, 64, 2, 2>(CM_ARGS);
+        if (big_ctas * 2 < 2 * SMS) return launch_one<64, 64, 64, 2, 2>(CM_ARGS);
         return launch_one<128, 64, 64, 4, 2>(CM_ARGS);
     }
-    if (big_ctas < 2 * 148) return launch_one<64, 64, 64, 2, 2>(CM_ARGS);
+    if (big_ctas < 2 * SMS) return launch_one<64, 64, 64, 2, 2>(CM_ARGS);
     return launch_one<128, 128, 64, 4, 2>(CM_ARGS);
 #undef CM_ARGS
 }

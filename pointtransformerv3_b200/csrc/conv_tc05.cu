@@ -152,7 +152,12 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
         const int64_t i = row0 + tid;
         rows_s[tid] = i < a.n ? (a.row_order ? a.row_order[i] : i) : -1;
     }
-    for (int c = tid; c < BN; c += CT_THREADS) bias_s[c] = !a.bias ? 0.f : F32 ? ((const float*)a.bias)[col0 + c] : __bfloat162float(((const __nv_bfloat16*)a.bias)[col0 + c]);
+    for (int c = tid; c < BN; c += CT_THREADS) {
+        if (F32)
+            bias_s[c] = a.bias ? ((const float*)a.bias)[col0 + c] : 0.f;
+        else
+            bias_s[c] = a.bias ? __bfloat162float(((const __nv_bfloat16*)a.bias)[col0 + c]) : 0.f;
+    }
     {
         // A warp stages whole offsets (four coalesced rows of 32 entries each), all of its loads issued
         // before the first store, and notes in the same pass whether the tile has the offset at all.
@@ -444,7 +449,7 @@ static int conv_tc05_capacity(int parts)
         auto kern = conv_tc05_kernel<BN, KC, STAGES, NI, true, F32>;
         if (allow_smem(kern) != cudaSuccess) return 0;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(148, 1, parts);
+        cfg.gridDim = dim3(SMS, 1, parts);
         cfg.blockDim = dim3((CT_GATHER_WARPS + NI) * 32);
         cfg.dynamicSmemBytes = conv_tc05_smem<BN, KC, STAGES>();
         cudaLaunchAttribute attr[1];
@@ -507,7 +512,7 @@ static int launch_conv_tc05_best(const void* weight, const ConvTcArgs& a, bool f
         if (a.cout % var.bn) continue;
         const int64_t ctas = tiles * (a.cout / var.bn);
         for (int parts = 1; parts <= (var.split ? 8 : 1); parts *= 2) {
-            const int64_t room = parts == 1 ? (int64_t)148 * var.per_sm : (int64_t)var.capacity(parts);
+            const int64_t room = parts == 1 ? (int64_t)SMS * var.per_sm : (int64_t)var.capacity(parts);
             if (room < parts) continue;
             if (parts > 1 && (ctas * parts > room || stages < 2 * parts)) continue;       // a cluster only within one wave
             const double cost = (double)((ctas * parts + room - 1) / room) * (CT_FIXED_US + stages / parts * var.stage_us);

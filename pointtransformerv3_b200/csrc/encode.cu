@@ -146,7 +146,7 @@ extern "C" int ptv3_decode(const int64_t* codes, int64_t n, int depth, int order
     if (n == 0) return PTV3_OK;
     PTV3_REQUIRE(codes && grid_coord, PTV3_ERR_INVALID_ARGUMENT, "ptv3_decode: null pointer");
     int64_t blocks = (n + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
+    if (blocks > SMS * 16) blocks = SMS * 16;
     decode_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(codes, n, depth, order == PTV3_ORDER_HILBERT,
                                                                       grid_coord, batch);
     count_launches(1);
@@ -175,7 +175,7 @@ extern "C" int ptv3_encode(const int32_t* grid_coord, const int64_t* batch, int6
     PTV3_REQUIRE(grid_coord && codes, PTV3_ERR_INVALID_ARGUMENT, "ptv3_encode: null pointer");
     const int threads = 256;
     int64_t blocks = (n + threads - 1) / threads;
-    if (blocks > 148 * 16) blocks = 148 * 16;
+    if (blocks > SMS * 16) blocks = SMS * 16;
     encode_kernel<<<(unsigned)blocks, threads, 0, (cudaStream_t)stream>>>(grid_coord, batch, n, depth,
                                                                            ol, codes);
     count_launches(1);

@@ -283,7 +283,7 @@ static bool gemm_shape_ok(int k, int n_out)
 // enough tiles to repay loading it
 static bool gemm_w_resident(const GemmArgs& a, int bn)
 {
-    return a.k <= 256 && (size_t)a.k * bn * 2 <= 131072 && (int64_t)a.row_tiles * (a.n_out / bn) >= 3 * 148;
+    return a.k <= 256 && (size_t)a.k * bn * 2 <= 131072 && (int64_t)a.row_tiles * (a.n_out / bn) >= 3 * SMS;
 }
 
 template <int BN, int STAGES, int MODE, bool WRES>
@@ -300,7 +300,7 @@ static int launch_gemm_mode(const CUtensorMap& mx, const CUtensorMap& mw, const 
     a.col_tiles = a.n_out / BN;
     const int64_t tiles = (int64_t)a.row_tiles * a.col_tiles;
     // resident W: the same number of CTAs on every column tile
-    const unsigned grid = WRES ? (unsigned)(148 / a.col_tiles * a.col_tiles) : (unsigned)(tiles < 148 ? tiles : 148);
+    const unsigned grid = WRES ? (unsigned)(SMS / a.col_tiles * a.col_tiles) : (unsigned)(tiles < SMS ? tiles : SMS);
     launch_dependent(kern, dim3(grid), dim3(64 + gm_epi_warps(MODE) * 32), smem, stream, mx, mw, mo, a);
     count_launches(1);
     return check_launch("ptv3_gemm_fwd");
@@ -323,7 +323,7 @@ static int launch_gemm(const void* x, const void* w, GemmArgs a, cudaStream_t st
     a.row_tiles = (int)((a.n + GM_BM - 1) / GM_BM);
     // 256-column tiles halve the traffic of x; 128-column tiles when those would leave SMs idle
     int bn = a.n_out % 256 == 0 ? 256 : 128;
-    if (bn == 256 && (int64_t)a.row_tiles * (a.n_out / 256) < 148) bn = 128;
+    if (bn == 256 && (int64_t)a.row_tiles * (a.n_out / 256) < SMS) bn = 128;
     CUtensorMap mx, mw, mo;
     int rc = make_tensor_map_bf16(&mx, x, (uint64_t)a.n, (uint64_t)a.k, (uint64_t)a.k * 2, GM_BM, GM_BK);
     if (rc) return rc;

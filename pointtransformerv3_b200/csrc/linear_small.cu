@@ -314,17 +314,18 @@ static int launch_ls(const void* x, const void* w, LinearSmallArgs a, int parts,
 
 // Shares of K: clusters of up to eight CTAs, at least four chunks each.  Below 16 chunks the exchange costs
 // more than it saves (441 x 512 -> 512: 7.1 us in clusters of two, 6.1 with the persistent kernel).
+constexpr int LS_CLUSTER_CTAS = 128;                   // one wave: sixteen clusters of eight (a cluster lives in one GPC)
 static int ls_parts(int64_t tiles, int k)
 {
     const int chunks = k / LS_BK;
     int parts = 1;
     if (chunks >= 16)
-        while (parts < 8 && tiles * parts * 2 <= 128 && chunks % (parts * 2) == 0 && chunks / (parts * 2) >= 4) parts *= 2;
+        while (parts < 8 && tiles * parts * 2 <= LS_CLUSTER_CTAS && chunks % (parts * 2) == 0 && chunks / (parts * 2) >= 4) parts *= 2;
     return parts;
 }
 
 // Where the lines lie (us, this kernel against the persistent ones):
-//   K <= 128: three CTAs share an SM: one wave.  1 560 x 64 -> 192: 3.5 / 6.3, 18 900 x 64 -> 192 (444 tiles):
+//   K <= 128: three CTAs share an SM: one wave.  1 560 x 64 -> 192: 3.5 / 6.3, 18 900 x 64 -> 192 (3 x 148 tiles):
 //     5.7 / 6.7, 9 400 x 128 -> 384 (444): 6.3 / 7.9; 1 776 tiles lose
 //   K <= 512: 105 x 256 -> 1 024: 4.4 / 5.4, 1 700 x 256 -> 256 (56 tiles): 4.8 / 5.0, -> 768 (168): 5.9 / 5.0
 //   longer K where it can be shared: 27 x 2 048 -> 512: 6.8 / 13.2, 1 000 x 2 048 -> 512 (64): 11.7 / 14.5
@@ -332,8 +333,8 @@ bool linear_small_wanted(int64_t n, int k, int n_out)
 {
     if (k % LS_BK || k < LS_BK || k > 8192 || n_out % LS_BN) return false;
     const int64_t tiles = (n + LS_BM - 1) / LS_BM * (n_out / LS_BN);
-    if (k <= 128) return tiles <= 444;
-    if (k < 1024) return tiles <= 74;
+    if (k <= 128) return tiles <= 3 * SMS;
+    if (k < 1024) return tiles <= SMS / 2;
     return ls_parts(tiles, k) > 1;
 }
 

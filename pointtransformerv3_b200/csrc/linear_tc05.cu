@@ -570,7 +570,7 @@ static int launch_linear(const void* x, const void* w, LinearArgs a, int k, cuda
     const size_t smem = (size_t)kb * a.n_out * sw + (size_t)groups * (2 * kb * 128 * sw + LIN_STAGE_BYTES) +
                         (size_t)a.n_out * 4 + 160 + 1024;
     const size_t smem_req = smem < 120 * 1024 ? 120 * 1024 : smem;   // one CTA per SM (it takes all of tensor memory)
-    const int64_t ntiles = (a.n + 127) / 128, grid = ntiles < 148 ? ntiles : 148;
+    const int64_t ntiles = (a.n + 127) / 128, grid = ntiles < SMS ? ntiles : SMS;
 #define LIN_LAUNCH(KK)                                                                                       \
     do {                                                                                                     \
         auto kern = linear_tc05_kernel<KK>;                                                                  \
@@ -598,7 +598,8 @@ static int launch_linear_ln(const void* x, const void* w, const LinearLnArgs& a,
     if (allow_smem(kern) != cudaSuccess) return check_launch("ptv3_linear_ln_fwd: shared memory attribute");
     const int64_t ntiles = (a.n + 127) / 128;
     constexpr size_t smem = lin_ln_smem(K) < 120 * 1024 ? 120 * 1024 : lin_ln_smem(K);      // one CTA per SM
-    launch_dependent(kern, dim3((unsigned)(ntiles < 148 ? ntiles : 148)), dim3(128 * lin_ln_groups(K)), smem, stream, mx, mw, a);
+    launch_dependent(kern, dim3((unsigned)(ntiles < SMS ? ntiles : SMS)), dim3(128 * lin_ln_groups(K)), smem, stream, mx,
+                     mw, a);
     count_launches(1);
     return check_launch("ptv3_linear_ln_fwd");
 }

@@ -297,7 +297,7 @@ static int launch_mlp(const void* x, const void* w1, const void* b1, const void*
     if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_mlp_fwd: shared memory attribute");
     const int64_t ntiles = (n + 127) / 128;
-    const int64_t grid = ntiles < 148 ? ntiles : 148;
+    const int64_t grid = ntiles < SMS ? ntiles : SMS;
     launch_dependent(kern, dim3((unsigned)grid), dim3(128 * Cfg::NG), Cfg::SMEM, stream, mx, mw1, mw2,
                      (const __nv_bfloat16*)b1, (const __nv_bfloat16*)b2, (const __nv_bfloat16*)residual,
                      (__nv_bfloat16*)out, n, settled, status);

@@ -294,7 +294,7 @@ static int check_batch_indices(const int64_t* offset, int n_scenes, const int32_
     return PTV3_OK;
 }
 
-static unsigned batch_indices_blocks(int64_t n) { return (unsigned)((n + 255) / 256 > 148 * 8 ? 148 * 8 : (n + 255) / 256); }
+static unsigned batch_indices_blocks(int64_t n) { return (unsigned)((n + 255) / 256 > SMS * 8 ? SMS * 8 : (n + 255) / 256); }
 
 int batch_indices_and_norms(const int64_t* offset, int n_scenes, const int32_t* grid_coord, int64_t n, int32_t* indices,
                             const BnJobs& norms, cudaStream_t stream)
@@ -319,7 +319,7 @@ extern "C" int ptv3_batch_stats(const int32_t* grid_coord, int64_t n, const int6
     cudaStream_t stream = (cudaStream_t)stream_;
     int64_t blocks = (n + 1023) / 1024;         // four points per thread, at most four blocks per SM
     if (blocks < 1) blocks = 1;
-    if (blocks > 148 * 4) blocks = 148 * 4;
+    if (blocks > SMS * 4) blocks = SMS * 4;
     batch_stats_kernel<<<(unsigned)blocks, 256, 0, stream>>>(grid_coord, n, offset, n_scenes, (int32_t*)scratch,
                                                              out_host);
     count_launches(1);
@@ -352,7 +352,7 @@ extern "C" int ptv3_pad_plan(const int64_t* offset, int n_scenes, int patch, int
                  PTV3_ERR_INVALID_ARGUMENT, "ptv3_pad_plan: null pointer");
     int64_t blocks = (n_pad + 255) / 256;
     if (blocks < 1) blocks = 1;
-    if (blocks > 148 * 8) blocks = 148 * 8;
+    if (blocks > SMS * 8) blocks = SMS * 8;
     const size_t smem = 3 * (size_t)(n_scenes + 1) * sizeof(int64_t);
     pad_plan_kernel<<<(unsigned)blocks, 256, smem, (cudaStream_t)stream>>>(
         offset, n_scenes, patch, n, n_pad, n_seq, pad, unpad, cu_seqlens, status);

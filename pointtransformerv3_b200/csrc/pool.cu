@@ -224,7 +224,7 @@ extern "C" int ptv3_unpool_fwd(const void* skip, const void* child, const int64_
                  PTV3_ERR_INVALID_ARGUMENT, "ptv3_unpool_fwd: null pointer");
     cudaStream_t stream = (cudaStream_t)stream_;
     int64_t blocks = (n * (channels / vn) + 255) / 256;
-    if (blocks > 148 * 16) blocks = 148 * 16;
+    if (blocks > SMS * 16) blocks = SMS * 16;
     if (dtype == PTV3_DTYPE_F32)
         launch_dependent(unpool_kernel<float>, dim3((unsigned)blocks), dim3(256), 0, stream, (const float*)skip,
                          (const float*)child, cluster, n, channels, skip_scale, skip_shift, child_scale,

@@ -408,7 +408,7 @@ static SortPlan sort_plan(int k, int64_t n, int sig_bits)
     while (sig_bits - p.wide * p.bits + p.val_bits > 64) ++p.wide;
     // tiles of 8192: half the look-back and status words per element; of 4096, with half the chain from start to
     // end, while those of all rows run at once (two to an SM)
-    p.items = (int64_t)k * ((n + 8 * OS_THREADS - 1) / (8 * OS_THREADS)) <= 2 * 148 ? 8 : 16;
+    p.items = (int64_t)k * ((n + 8 * OS_THREADS - 1) / (8 * OS_THREADS)) <= 2 * SMS ? 8 : 16;
     p.ntiles = ceil_div(n, (int64_t)p.items * OS_THREADS);
     size_t b = 0;
     b += 2 * align_up((size_t)k * n * sizeof(uint64_t), 256);   // ping-pong of words or keys
@@ -460,7 +460,7 @@ extern "C" int ptv3_argsort_inverse(const int64_t* codes, int k, int64_t n, int 
 
     const uint64_t* kin = reinterpret_cast<const uint64_t*>(codes);
     {
-        const int hb = (int)std::min<int64_t>(ceil_div(n, OS_THREADS * 8), 4 * 148);
+        const int hb = (int)std::min<int64_t>(ceil_div(n, OS_THREADS * 8), 4 * SMS);
         os_hist_kernel<<<dim3(hb, k), OS_THREADS, (size_t)p.passes * OS_MAX_BINS * sizeof(uint32_t), stream>>>(
             kin, n, sig_bits, p.bits, p.passes, hist);
     }

@@ -344,7 +344,7 @@ extern "C" int ptv3_grid_coord(const float* coord, int64_t n, float grid_size, f
     PTV3_REQUIRE(coord && origin && grid_coord, PTV3_ERR_INVALID_ARGUMENT, "ptv3_grid_coord: null pointer");
     cudaStream_t stream = (cudaStream_t)stream_;
     vox_origin_init_kernel<<<1, 32, 0, stream>>>(origin);
-    const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, 148 * 8);
+    const unsigned blocks = (unsigned)std::min<int64_t>((n + 255) / 256, SMS * 8);
     vox_min_kernel<<<blocks, 256, 0, stream>>>(coord, n, origin);
     vox_grid_kernel<<<(unsigned)((3 * n + 255) / 256), 256, 0, stream>>>(coord, 3 * n, grid_size, origin, grid_coord);
     count_launches(3);
@@ -434,7 +434,7 @@ extern "C" int ptv3_voxelize(const float* coord, int64_t n, float grid_size, con
     if (cudaMemsetAsync(keys, 0xff, clear, stream) != cudaSuccess) return check_launch("ptv3_voxelize: table reset");
     vox_origin_init_kernel<<<1, 32, 0, stream>>>(origin);
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    vz_min_kernel<<<(unsigned)std::min<int64_t>((n + 1023) / 1024, 148 * 8), 256, 0, stream>>>(
+    vz_min_kernel<<<(unsigned)std::min<int64_t>((n + 1023) / 1024, SMS * 8), 256, 0, stream>>>(
         coord, n, ((uintptr_t)coord & 15) == 0, origin);
     vz_insert_kernel<<<blocks, 256, (size_t)n_scenes * sizeof(int64_t), stream>>>(
         coord, n, grid_size, origin, offset, n_scenes, keys, vals, cap, first, status);
