@@ -494,9 +494,10 @@ int ptv3_block_supported(int channels, int heads, int hidden, int dtype);
  * fp32 on the tensor cores: a float is the exact sum of three bf16 values, and a product of floats the sum
  * of six products of those, accumulated in fp32 (what is left out is below one fp32 rounding).
  * ptv3_split_f32 writes rows x k floats as rows x 3k bf16 (6k where k is not a multiple of 64), for the
- * features of a product (weight = 0) or its weights (weight = 1); the two products take both split.  ptv3_block_fwd with PTV3_DTYPE_F32 takes fp32
- * features, biases and norms and SPLIT conv_weight, cpe_w, qkv_w, proj_w, fc1_w, fc2_w (rows of their inner
- * dimension: c_in for the convolution), where ptv3_block_f32_supported says so.
+ * features of a product (weight = 0) or its weights (weight = 1); the two products take both split.
+ * ptv3_block_fwd with PTV3_DTYPE_F32 takes fp32 features, biases and norms and SPLIT conv_weight, cpe_w, qkv_w,
+ * proj_w, fc1_w, fc2_w (rows of their inner dimension: c_in for the convolution), where
+ * ptv3_block_f32_supported says so.
  */
 int ptv3_split_f32(const float* x, int64_t rows, int k, int weight, void* out, void* stream);
 int ptv3_linear_split_fwd(const void* x_split, const void* w_split, const float* bias, const float* residual,

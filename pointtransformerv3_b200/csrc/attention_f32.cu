@@ -186,7 +186,8 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(
     const float inv = 1.f / l;
     float4* op = reinterpret_cast<float4*>(out + mine * C + h * AX_D);
 #pragma unroll
-    for (int d = 0; d < 4; ++d) op[d] = make_float4(y[4 * d] * inv, y[4 * d + 1] * inv, y[4 * d + 2] * inv, y[4 * d + 3] * inv);
+    for (int d = 0; d < 4; ++d)
+        op[d] = make_float4(y[4 * d] * inv, y[4 * d + 1] * inv, y[4 * d + 2] * inv, y[4 * d + 3] * inv);
 }
 
 int launch_attn_f32(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad, const int32_t* cu,

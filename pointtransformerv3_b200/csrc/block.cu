@@ -32,6 +32,7 @@ static bool linear_any_supported(int k, int n_out, bool epilogue)
 static int linear_any(const void* x, const void* w, const void* bias, const void* residual, void* out, int64_t n,
                       int k, int n_out, int gelu, bool settled, uint32_t* status, cudaStream_t stream)
 {
+    // (also the only one to take 64 output columns with GELU or a residual: see use_fused_mlp)
     if (linear_small_wanted(n, k, n_out))
         return launch_linear_small(x, w, bias, residual, out, n, k, n_out, gelu, settled, status, stream);
     if (ptv3_gemm_supported(k, n_out, PTV3_DTYPE_BF16))
@@ -114,13 +115,14 @@ static int block_f32(const ptv3_block_args* a, bool settled, cudaStream_t stream
     auto f = [](const void* p) { return (const float*)p; };
     // (the split of the convolution's input lies where the hidden rows come later)
     STEP(launch_split_f32(f(a->conv_in), n, C, b.sh, stream));
-    STEP(launch_conv_split(b.sh, a->nbr, a->conv_weight, f(a->conv_bias), nullptr, b.s, a->row_order, n, C, C, 27, a->status,
-                           stream));
+    STEP(launch_conv_split(b.sh, a->nbr, a->conv_weight, f(a->conv_bias), nullptr, b.s, a->row_order, n, C, C, 27,
+                           a->status, stream));
     STEP(launch_linear_split(b.s, a->cpe_w, f(a->cpe_b), nullptr, b.y, nullptr, n, C, C, 0, settled, a->status, stream));
-    STEP(ptv3_add_layernorm_fwd(b.y, a->feat, a->cpe_ln_w, a->cpe_ln_b, a->cpe_ln_eps, b.f1, a->n1_w, a->n1_b, a->n1_eps, b.a,
-                                n, C, PTV3_DTYPE_F32, stream));
+    STEP(ptv3_add_layernorm_fwd(b.y, a->feat, a->cpe_ln_w, a->cpe_ln_b, a->cpe_ln_eps, b.f1, a->n1_w, a->n1_b, a->n1_eps,
+                                b.a, n, C, PTV3_DTYPE_F32, stream));
     STEP(launch_split_f32(b.a, n, C, b.s, stream));
-    STEP(launch_linear_split(b.s, a->qkv_w, f(a->qkv_b), nullptr, b.qkv, nullptr, n, C, 3 * C, 0, settled, a->status, stream));
+    STEP(launch_linear_split(b.s, a->qkv_w, f(a->qkv_b), nullptr, b.qkv, nullptr, n, C, 3 * C, 0, settled, a->status,
+                             stream));
     STEP(ptv3_attention_fwd(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.att, n, a->n_seq, a->max_seqlen, C, a->heads,
                             a->scale, PTV3_DTYPE_F32, a->attention_algo, a->status, stream));
     STEP(launch_split_f32(b.att, n, C, b.s, stream));
@@ -130,7 +132,8 @@ static int block_f32(const ptv3_block_args* a, bool settled, cudaStream_t stream
                                 PTV3_DTYPE_F32, stream));
     STEP(launch_split_f32(b.a, n, C, b.s, stream));
     STEP(launch_linear_split(b.s, a->fc1_w, f(a->fc1_b), nullptr, nullptr, b.sh, n, C, H, 1, settled, a->status, stream));
-    STEP(launch_linear_split(b.sh, a->fc2_w, f(a->fc2_b), b.f2, (float*)a->out, nullptr, n, H, C, 0, settled, a->status, stream));
+    STEP(launch_linear_split(b.sh, a->fc2_w, f(a->fc2_b), b.f2, (float*)a->out, nullptr, n, H, C, 0, settled, a->status,
+                             stream));
 #undef STEP
     return PTV3_OK;
 }
@@ -138,8 +141,8 @@ static int block_f32(const ptv3_block_args* a, bool settled, cudaStream_t stream
 int block_f32_supported(int channels, int heads, int hidden)
 {
     const int d = heads > 0 && channels % heads == 0 ? channels / heads : 0;
-    return channels >= 32 && channels <= 1024 && (channels & (channels - 1)) == 0 && hidden % 32 == 0 && hidden >= channels &&
-           (d == 8 || d == 16 || d == 32 || d == 64);
+    return channels >= 32 && channels <= 1024 && (channels & (channels - 1)) == 0 && hidden % 32 == 0 &&
+           hidden >= channels && (d == 8 || d == 16 || d == 32 || d == 64);
 }
 
 int block_fwd(const ptv3_block_args* a, bool settled, cudaStream_t stream)
@@ -147,7 +150,8 @@ int block_fwd(const ptv3_block_args* a, bool settled, cudaStream_t stream)
     PTV3_REQUIRE(a != nullptr, PTV3_ERR_INVALID_ARGUMENT, "ptv3_block_fwd: null argument block");
     const bool f32 = a->dtype == PTV3_DTYPE_F32 && block_f32_supported(a->channels, a->heads, a->hidden) && a->nbr;
     PTV3_REQUIRE(f32 || ptv3_block_supported(a->channels, a->heads, a->hidden, a->dtype), PTV3_ERR_UNSUPPORTED,
-                 "ptv3_block_fwd: bf16 (or fp32 with split weights), channels and hidden multiples of 16 (got %d, %d, dtype %d)",
+                 "ptv3_block_fwd: bf16 (or fp32 with split weights), channels and hidden multiples of 16 (got %d, %d, "
+                 "dtype %d)",
                  a->channels, a->hidden, a->dtype);
     PTV3_REQUIRE(a->n >= 0, PTV3_ERR_INVALID_ARGUMENT, "ptv3_block_fwd: n < 0");
     if (a->n == 0) return PTV3_OK;
@@ -347,7 +351,8 @@ extern "C" int ptv3_linear_split_fwd(const void* x_split, const void* w_split, c
 {
     PTV3_REQUIRE(n >= 0 && n <= 65535ll * 128 && k >= 32 && k % 32 == 0 && n_out >= 32 && n_out % 32 == 0 &&
                      k <= 8192 && n_out <= 8192,
-                 PTV3_ERR_UNSUPPORTED, "ptv3_linear_split_fwd: k and n_out multiples of 32, up to 8 388 480 rows (got %d, %d)", k, n_out);
+                 PTV3_ERR_UNSUPPORTED,
+                 "ptv3_linear_split_fwd: k and n_out multiples of 32, up to 8 388 480 rows (got %d, %d)", k, n_out);
     if (n == 0) return PTV3_OK;
     PTV3_REQUIRE(x_split && w_split && out && status &&
                      (((uintptr_t)x_split | (uintptr_t)w_split | (uintptr_t)out | (uintptr_t)residual) & 15) == 0,
@@ -362,7 +367,8 @@ extern "C" int ptv3_subm_conv_split_fwd(const void* feat_split, const int32_t* n
 {
     PTV3_REQUIRE(n >= 0 && n < (1ll << 31) && c_in >= 32 && c_in % 32 == 0 && (c_out == 32 || c_out % 64 == 0) &&
                      c_in <= 4096 && c_out <= 4096 && c_out >= 32 && kernel_volume >= 1 && kernel_volume <= 27,
-                 PTV3_ERR_UNSUPPORTED, "ptv3_subm_conv_split_fwd: %d -> %d channels, %d offsets", c_in, c_out, kernel_volume);
+                 PTV3_ERR_UNSUPPORTED, "ptv3_subm_conv_split_fwd: %d -> %d channels, %d offsets", c_in, c_out,
+                 kernel_volume);
     if (n == 0) return PTV3_OK;
     PTV3_REQUIRE(feat_split && nbr && w_split && out && status &&
                      (((uintptr_t)feat_split | (uintptr_t)w_split | (uintptr_t)out) & 15) == 0,

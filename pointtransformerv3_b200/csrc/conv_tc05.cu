@@ -481,8 +481,8 @@ constexpr int CT_VARIANTS = 5;
 template <int BN, int STAGES, bool F32>
 static constexpr ConvVariant conv_variant(double stage_us)
 {
-    return {BN, 1, stage_us, launch_conv_tc05_as<BN, 64, STAGES, 2, false, F32>, launch_conv_tc05_as<BN, 64, STAGES, 2, true, F32>,
-            conv_tc05_capacity<BN, 64, STAGES, 2, F32>};
+    return {BN, 1, stage_us, launch_conv_tc05_as<BN, 64, STAGES, 2, false, F32>,
+            launch_conv_tc05_as<BN, 64, STAGES, 2, true, F32>, conv_tc05_capacity<BN, 64, STAGES, 2, F32>};
 }
 // [fp32 output][variant].  Second entry: many tiles, two CTAs per SM, so that one tile's prologue and epilogue
 // run beside another's products.  Last: 32 output channels (fp32; bf16 has its own path for them).

@@ -320,7 +320,8 @@ static int ls_parts(int64_t tiles, int k)
     const int chunks = k / LS_BK;
     int parts = 1;
     if (chunks >= 16)
-        while (parts < 8 && tiles * parts * 2 <= LS_CLUSTER_CTAS && chunks % (parts * 2) == 0 && chunks / (parts * 2) >= 4) parts *= 2;
+        while (parts < 8 && tiles * parts * 2 <= LS_CLUSTER_CTAS && chunks % (parts * 2) == 0 && chunks / (parts * 2) >= 4)
+            parts *= 2;
     return parts;
 }
 

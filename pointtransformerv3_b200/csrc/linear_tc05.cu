@@ -645,9 +645,10 @@ int linear_ln_fwd(const void* x, const void* weight, const void* bias, const voi
     const LinearLnArgs a{(const __nv_bfloat16*)bias, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)ln1_weight,
                          (const __nv_bfloat16*)ln1_bias, (const __nv_bfloat16*)ln2_weight, (const __nv_bfloat16*)ln2_bias,
                          (__nv_bfloat16*)sum_out, (__nv_bfloat16*)norm_out, ln1_eps, ln2_eps, n, settled, status};
-    if (channels == 32) return ln1_weight ? launch_linear_ln<32, true>(x, weight, a, stream) : launch_linear_ln<32, false>(x, weight, a, stream);
-    if (channels == 64) return ln1_weight ? launch_linear_ln<64, true>(x, weight, a, stream) : launch_linear_ln<64, false>(x, weight, a, stream);
-    return ln1_weight ? launch_linear_ln<128, true>(x, weight, a, stream) : launch_linear_ln<128, false>(x, weight, a, stream);
+    auto launch = channels == 32   ? (ln1_weight ? launch_linear_ln<32, true> : launch_linear_ln<32, false>)
+                  : channels == 64 ? (ln1_weight ? launch_linear_ln<64, true> : launch_linear_ln<64, false>)
+                                   : (ln1_weight ? launch_linear_ln<128, true> : launch_linear_ln<128, false>);
+    return launch(x, weight, a, stream);
 }
 
 }  // namespace ptv3

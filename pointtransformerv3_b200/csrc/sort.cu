@@ -3,7 +3,8 @@
 // pass.  Replaces torch.argsort + scatter_ at model.py:118-126 and :667-674
 // (ties are resolved by original index, the canonical order).
 //
-// One-sweep form: one kernel reads every key once and builds the digit
+// One-sweep form (Adinets and Merrill, "Onesweep: A Faster Least Significant Digit Radix Sort for GPUs",
+// 2022; the look-back is Merrill and Garland's, 2016): one kernel reads every key once and builds the digit
 // histograms of ALL passes; after that every pass is a single kernel.  A tile of
 // a pass ranks its keys by digit in shared memory, publishes its per-digit counts
 // in a status table and obtains its global offsets by looking back over the

@@ -9,6 +9,9 @@
 // accumulator would lose more than a chain of FMAs: the leading piece goes to SPLIT_MAIN accumulators in turn,
 // the five small ones to one of their own (their truncation is 2^-8 of the leading one's), and the epilogue
 // adds them in fp32.  Against float64 the products come out as close as CUDA-core fp32.
+// (The split and its six products: Henry, Tang and Heinecke, "Leveraging the bfloat16 Artificial Intelligence
+// Datatype for Higher-Precision Computations", 2019; small products in accumulators of their own, because of the
+// truncation: Ootomo and Yokota, "Recovering Single Precision Accuracy from Tensor Cores", 2022.)
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -352,11 +352,6 @@ def pool_plan(code, order, grid_coord, batch, n_scenes, pooling_depth, row_perm=
                 batch=pbatch[:m], counts=host[1:], m=m, offset=_offsets_to_device(host[1:], dev))
 
 
-def batch_stats(grid_coord, offset):
-    """(largest grid coordinate per axis, offsets) of a batch as Python ints."""
-    return BatchStats(grid_coord, offset).result()
-
-
 class BatchStats:
     """Launches the kernel that stores a batch's bounds in mapped host memory; ``result`` waits for
     it, so that the host can work in between.  One at a time per host thread and stream."""
@@ -692,8 +687,8 @@ def linear_ln(x, weight, bias, residual, ln1, ln2, status=None, want_sum=True):
 
 
 def split_f32(x, weight=False):
-    """(..., k) fp32 -> (..., 3k) bf16 (6k where k is not a multiple of 64): the operand of a product of floats on the bf16 tensor cores
-    (see ptv3_split_f32); ``weight`` for its second operand."""
+    """(..., k) fp32 -> (..., 3k) bf16 (6k where k is not a multiple of 64): the operand of a product of
+    floats on the bf16 tensor cores (see ptv3_split_f32); ``weight`` for its second operand."""
     _lib.require_cuda(x)
     x = x.detach().contiguous()
     k = x.shape[-1]

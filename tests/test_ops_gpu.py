@@ -750,8 +750,8 @@ def test_short_linear(n, k, n_out, gelu, residual):
 @pytest.mark.parametrize("n", [1, 128, 1001, 18944, 19000])
 @pytest.mark.parametrize("with_ln1", [False, True])
 def test_short_linear_layernorm(n, c, with_ln1):
-    """Linear + residual + LayerNorms on short inputs (statistics merged over 32-column pieces and
-    clusters of two) and on the other side of the line, against torch in fp32."""
+    """Linear + residual + LayerNorms on short inputs: fewer rows than a tile, whole tiles, a ragged last tile,
+    one tile per SM (18 944 rows) and a few more, against torch in fp32."""
     g = torch.Generator().manual_seed(n + c)
     x, r = torch.randn(n, c, generator=g).bfloat16(), torch.randn(n, c, generator=g).bfloat16()
     w, b = (torch.randn(c, c, generator=g) / c ** 0.5).bfloat16(), torch.randn(c, generator=g).bfloat16()
