@@ -10,6 +10,7 @@ struct BnJobs {
     float* out[BN_JOBS];
     int count;
 };
+static_assert(sizeof(BnJobs) <= 3584, "kernel parameters, with those of batch_indices_kernel");
 
 // the first of `count` layers (at most BN_JOBS), checked; each has its scales and shifts behind one another in `out`
 int bn_jobs(const ptv3_bn_args* layers, int count, float* out, BnJobs* jobs);

@@ -21,7 +21,7 @@ __global__ void __launch_bounds__(256) split_f32_kernel(const float* __restrict_
 
 // Weights, many to a launch: a block takes 256 x 8 values of one of them.  Neither launched ahead of the work
 // before it nor letting the kernel behind it start early: the Linear kernels fetch weights before they wait.
-constexpr int SPLIT_JOBS = 128;          // 3.6 KB of the 4 KB of kernel parameters
+constexpr int SPLIT_JOBS = 144;          // those of the default network; 4 036 of the 4 096 bytes of kernel parameters
 struct SplitJobs {
     const float* x[SPLIT_JOBS];
     __nv_bfloat16* out[SPLIT_JOBS];
@@ -29,6 +29,7 @@ struct SplitJobs {
     int k[SPLIT_JOBS];
     int count;
 };
+static_assert(sizeof(SplitJobs) <= 4096, "kernel parameters");
 
 __global__ void __launch_bounds__(256) split_weights_kernel(const __grid_constant__ SplitJobs jobs)
 {
