@@ -45,8 +45,8 @@ CPU_SAMPLE_VOXELS = 100_000
 LIDAR_SCENES = 16
 LIDAR_GRID = 0.05
 # DRAM read + write bytes per row and channel of one attention launch (ncu, dram__bytes_read.sum +
-# dram__bytes_write.sum of a single launch on 407 552 padded rows x 64 channels: 166.2 + 34.5 MB)
-ATTENTION_DRAM_BYTES_PER_ROW_CHANNEL = 7.70
+# dram__bytes_write.sum of a single launch on 407 000 rows x 64 channels: 166.1 + 31.9 MB)
+ATTENTION_DRAM_BYTES_PER_ROW_CHANNEL = 7.60
 
 
 def workload_config(n_gpus, gather=False):

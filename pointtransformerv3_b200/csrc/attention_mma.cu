@@ -19,9 +19,10 @@
 // Softmax needs no reference value where no score can leave the range of exp2: |q . k| <= |q| max|k|, so a
 // tile whose rows pass that test (AM_BOUND) runs without maxima, votes and rescaling, and its 16-key
 // groups do not depend on one another; the other tiles, and the ragged end of a sequence, run the
-// online form.  400 000 points x 64 channels: 0.502 -> 0.455 ms, exp unit 71 -> 81 % busy.  What is left:
-// 20 mma.sync of 8 cycles per 16 x 64 scores share register ports with the FMA pipe, so exponentials
-// moved there (a quartic on 2 to 8 of 16 pairs) gain nothing: 0.446 to 0.498 ms.
+// online form.  400 000 points x 64 channels: 0.502 -> 0.455 ms, 70 -> 77 % of the exp unit's rate over
+// the launch (83 % of it while warps are active, at 120 000 points).  What is left: the gather before a CTA's
+// first product, the last wave, and 20 mma.sync of 8 cycles per 16 x 64 scores, which share register ports with
+// the FMA pipe, so that exponentials moved there (a quartic on 2 to 8 of 16 pairs) gain nothing: 0.446 to 0.498 ms.
 #include "common.cuh"
 #include "attention_mma.cuh"
 #include "mma_util.cuh"

@@ -245,7 +245,7 @@ int Pass::each_weight(F&& f)
 
 // fp32 weights, split for this pass: what the caller writes to them is seen by the next pass, whichever way it
 // is written and on whatever stream.  The default network's 183 MB become 275, one launch that runs on the main
-// stream while that waits for the sort (two rooms of 20 000 points: 6.39 ms a pass, 6.36 with splits that were kept).
+// stream while that waits for the sort (two rooms of 20 000 points: 6.58 ms a pass, 6.50 with splits that were kept).
 int Pass::split_weights()
 {
     if (a_.dtype != PTV3_DTYPE_F32 || !a_.plain_weights) return PTV3_OK;

@@ -18,9 +18,9 @@
 // beside their indices until enough of their digits are done.
 // The first pass reads the caller's codes; the last one writes order / inverse as int64.
 //
-// Bytes per element: 8 (histograms) + 16 per pass + 8 in the last one.  What bounds a pass is shared
-// memory (the counters and masks of the ranking and the reordering are scattered accesses with several bank
-// conflicts each) and a tile's chain of short phases separated by barriers: 33.5 M elements in 280 us against
+// Bytes per element: 8 (histograms) + 16 per pass + 8 in the last one.  What bounds a pass is a
+// tile's chain of short phases separated by barriers, two tiles per SM, most of each phase scattered accesses to
+// shared memory (its wavefronts 51 % of peak, issue 50 %: neither is full): 33.5 M elements in 280 us against
 // 82 for the bytes (with 12-byte elements, tiles of 4096 and ballots: 470).  The last pass adds 390 us to that
 // for the scattered 8-byte inverses, the rate at which L2 takes single sectors (the same in a kernel of its own).
 // 8.4 M x 4 rows of 37 bits, four passes: 1.65 ms (2.75 before); 100 000 x 4 of 30: 48 us (54).
