@@ -122,8 +122,7 @@ def read_status(status):
     host memory by a kernel and polled, which takes a third of the time of a copy and a stream wait."""
     lib, stream = _lib.load(), _lib.stream()
     host = _host_words(2, "status", stream).begin(lib, stream)
-    _lib.check(lib.ptv3_status_report(status.data_ptr(), host.address, stream), "ptv3_status_report")
-    host.pending = True
+    host.launched(lib.ptv3_status_report(status.data_ptr(), host.address, stream), "ptv3_status_report")
     return host.wait(lib, stream)[0]
 
 
@@ -332,13 +331,12 @@ def pool_plan(code, order, grid_coord, batch, n_scenes, pooling_depth, row_perm=
     # the driver takes several times longer to notice the end of a kernel)
     stream = _lib.stream()
     meta_host = _host_words(3 + n_scenes, "pool_plan.meta", stream).begin(lib, stream)
-    _lib.check(lib.ptv3_pool_plan(_lib.ptr(code), _lib.ptr(order), _lib.ptr(grid_coord), _lib.ptr(batch),
-                                  k, n, n_scenes, int(pooling_depth), perm, _lib.ptr(cluster),
-                                  _lib.ptr(idx_ptr), _lib.ptr(head), _lib.ptr(pcode), _lib.ptr(porder),
-                                  _lib.ptr(pinv), _lib.ptr(pgrid), _lib.ptr(pbatch), _lib.ptr(meta),
-                                  meta_host.address, _lib.ptr(status), _lib.ptr(ws), nbytes, stream),
-               "ptv3_pool_plan")
-    meta_host.pending = True
+    meta_host.launched(lib.ptv3_pool_plan(_lib.ptr(code), _lib.ptr(order), _lib.ptr(grid_coord), _lib.ptr(batch),
+                                         k, n, n_scenes, int(pooling_depth), perm, _lib.ptr(cluster),
+                                         _lib.ptr(idx_ptr), _lib.ptr(head), _lib.ptr(pcode), _lib.ptr(porder),
+                                         _lib.ptr(pinv), _lib.ptr(pgrid), _lib.ptr(pbatch), _lib.ptr(meta),
+                                         meta_host.address, _lib.ptr(status), _lib.ptr(ws), nbytes, stream),
+                      "ptv3_pool_plan")
     host = meta_host.wait(lib, stream)[:-1]                          # the one wait
     if host[-1]:
         raise _lib.Ptv3Error("device status 0x%x (read after ptv3_pool_plan; the word is shared by "
@@ -365,9 +363,8 @@ class BatchStats:
         offset = offset.to(torch.int64).contiguous()
         n_scenes = offset.shape[0]
         host = self.host = _host_words(4 + n_scenes, "batch_stats", self.stream, offset.device).begin(self.lib, self.stream)
-        _lib.check(self.lib.ptv3_batch_stats(grid_coord.data_ptr(), grid_coord.shape[0], offset.data_ptr(), n_scenes,
-                                             host.address, host.scratch.data_ptr(), self.stream), "ptv3_batch_stats")
-        host.pending = True
+        host.launched(self.lib.ptv3_batch_stats(grid_coord.data_ptr(), grid_coord.shape[0], offset.data_ptr(), n_scenes,
+                                                host.address, host.scratch.data_ptr(), self.stream), "ptv3_batch_stats")
         self.keep = (grid_coord, offset)
 
     def result(self):
@@ -397,6 +394,12 @@ class _HostWords:
             self.wait(lib, stream)
         self.words[len(self.words) - 1] = 0
         return self
+
+    def launched(self, rc, what):
+        if rc != 0:
+            torch.cuda.synchronize()       # some of the call may be queued and write here yet
+        _lib.check(rc, what)
+        self.pending = True
 
     def wait(self, lib, stream):
         _lib.check(lib.ptv3_host_wait(self.last, stream), "waiting for a result")
@@ -844,11 +847,10 @@ def voxelize(coord, feat, offset, grid_size):
     stream = _lib.stream()
     host = _host_words(3, "voxelize", stream).begin(lib, stream)
     with timed("voxelize", 64.0 * n):
-        _lib.check(lib.ptv3_voxelize(_lib.ptr(coord), n, float(grid_size), _lib.ptr(offset), n_scenes, _lib.ptr(small),
-                                     _lib.ptr(keep), _lib.ptr(p2v), _lib.ptr(new_offset), host.address,
-                                     _lib.ptr(small[4:]), _lib.ptr(status), _lib.ptr(ws), nbytes, _lib.stream()),
-                   "ptv3_voxelize")
-    host.pending = True
+        host.launched(lib.ptv3_voxelize(_lib.ptr(coord), n, float(grid_size), _lib.ptr(offset), n_scenes, _lib.ptr(small),
+                                        _lib.ptr(keep), _lib.ptr(p2v), _lib.ptr(new_offset), host.address,
+                                        _lib.ptr(small[4:]), _lib.ptr(status), _lib.ptr(ws), nbytes, _lib.stream()),
+                      "ptv3_voxelize")
     m, bits, _ = host.wait(lib, stream)
     if bits:
         raise _lib.Ptv3Error("ptv3_voxelize: device status 0x%x" % bits)

@@ -35,7 +35,7 @@ def test_result_given_up_is_not_taken_for_the_next_one():
         host.begin(lib, 0)
         assert not any(v in (6, 7) for v in lib.queued), "a kernel that nobody waited for still owns the words"
         lib.launch(value)
-        host.pending = True
+        host.launched(0, "kernel")
         if not given_up:
             assert host.wait(lib, 0)[0] == value and not host.pending
     assert not lib.queued
@@ -46,5 +46,5 @@ def test_launch_that_failed_is_not_waited_for():
     host.begin(lib, 0)                   # the launch raises: no kernel will ever store anything
     host.begin(lib, 0)
     lib.launch(3)
-    host.pending = True
+    host.launched(0, "kernel")
     assert host.wait(lib, 0)[0] == 3
