@@ -49,7 +49,7 @@ class NativeBackbone:
         self.f32 = self.dtype == torch.float32
         _require(self.dtype in (torch.float32, torch.bfloat16))
         self.refs = []           # (owner dict, name): every tensor the blocks point to
-        self.norms = []          # BatchNorm layers
+        self.norms = []          # BatchNorm and LayerNorm layers
         self.keep = []           # arrays the blocks point into
         self.modules = [m.__dict__ for m in net.modules()]
         self.parents = [d["_modules"] for d in self.modules if d["_modules"]]
@@ -139,6 +139,7 @@ class NativeBackbone:
                 order_index[j] = m.attn.order_index
                 patch[j] = m.attn.patch_size if m.attn.enable_flash else -m.attn.patch_size_max
                 self.blocks.append(m)
+                self.norms.extend(m.__dict__["_ptv3_block_args"][4])
             st.n_blocks, st.blocks, st.order_index, st.patch = len(mods), blocks, order_index, patch
             self.stage_blocks.append(len(mods))
             self.keep.append((blocks, order_index, patch))
@@ -153,7 +154,7 @@ class NativeBackbone:
                         t.patch_size if t.enable_flash else t.patch_size_max))
         for p in self.pools:
             got.append((p.stride, p.reduce))
-        got.extend([bn.eps for bn in self.norms])
+        got.extend([norm.eps for norm in self.norms])
         return got
 
     def current(self):

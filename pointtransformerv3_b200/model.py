@@ -296,13 +296,14 @@ class Block(PointModule):
         microseconds instead of the attribute lookups of a rebuild."""
         cached = self.__dict__.get("_ptv3_block_args")
         if cached is not None:
-            holders, params, ptrs, a = cached
+            holders, params, ptrs, a, norms = cached
             for (owner, name), p, ptr in zip(holders, params, ptrs):
                 if owner[name] is not p or p.data_ptr() != ptr:
                     break
             else:
                 if params[0].dtype == dt and params[0].device == device:
                     a.attention_algo, a.scale = self.attn.algo, self.attn.scale
+                    a.cpe_ln_eps, a.n1_eps, a.n2_eps = (n.eps for n in norms)
                     return a
         conv, lin, attn, mlp = self.cpe[0], self.cpe[1], self.attn, self.mlp[0]
         names = ("conv_weight", "conv_bias", "cpe_w", "cpe_b", "cpe_ln_w", "cpe_ln_b", "n1_w", "n1_b", "qkv_w",
@@ -318,10 +319,11 @@ class Block(PointModule):
         a = _lib.BlockArgs()
         a.channels, a.heads, a.hidden = self.channels, attn.num_heads, mlp.fc1.out_features
         a.dtype = _lib.DTYPE_IDS[dt]
-        a.cpe_ln_eps, a.n1_eps, a.n2_eps = self.cpe[2].eps, self.norm1[0].eps, self.norm2[0].eps
+        norms = (self.cpe[2], self.norm1[0], self.norm2[0])
+        a.cpe_ln_eps, a.n1_eps, a.n2_eps = (n.eps for n in norms)
         for name, ptr in zip(names, ptrs):
             setattr(a, name, ptr)
-        self.__dict__["_ptv3_block_args"] = (holders, params, ptrs, a)
+        self.__dict__["_ptv3_block_args"] = (holders, params, ptrs, a, norms)
         a.attention_algo, a.scale = attn.algo, attn.scale
         return a
 

@@ -495,6 +495,33 @@ def test_values_written_through_data_between_passes(name, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("name", ["embedding.stem.norm", "enc.enc1.down.norm.0", "enc.enc0.block0.cpe.2",
+                                  "dec.dec0.block0.norm1.0", "dec.dec0.block0.norm2.0"])
+@pytest.mark.parametrize("hooked", [False, True])
+def test_norm_eps_changed_between_passes(name, hooked):
+    """A norm's eps is a setting like an attention's scale: in the one-call form and in the module tree (block by block)."""
+    import copy
+    data = small_batch([900, 500], 7)
+    net = P.PointTransformerV3(in_channels=6, **SMALL_CFG)
+    weights.fill_state_dict(net, prefix="ptv3.")
+    net = net.eval().cuda().bfloat16()
+    if hooked:
+        net.enc.enc2.block0.register_forward_hook(lambda *a: None)
+    fresh = copy.deepcopy(net)
+
+    def run(n):
+        torch.manual_seed(5)
+        with torch.inference_mode():
+            return n(cuda_data(data, torch.bfloat16)).feat
+    for _ in range(2):
+        before = run(net)
+    for n in (net, fresh):
+        n.get_submodule(name).eps = 0.5
+    got, ref = run(net), run(fresh)
+    assert torch.equal(got, ref) and not torch.equal(got, before)
+
+
+@pytest.mark.gpu
 def test_bounds_of_a_batch_are_read_once_in_either_form():
     """A hooked network runs as a module tree: the bounds that were asked for before that was known serve it, and
     no report is left that nobody waited for."""
