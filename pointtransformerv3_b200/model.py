@@ -289,6 +289,19 @@ class Block(PointModule):
         return (self._fusable_form() and point.feat.dtype in (torch.float32, torch.bfloat16)
                 and "sparse_conv_feat" in point.keys())
 
+    def _same_modules(self):
+        """Whether the block is still made of the modules that it was made of when this was last asked."""
+        chain = self.__dict__.get("_ptv3_modules")
+        if chain is not None:
+            for owner, name, child in chain:
+                if owner.get(name) is not child:
+                    break
+            else:
+                return True
+        self.__dict__["_ptv3_modules"] = [(m._modules, name, child) for m in self.modules()
+                                          for name, child in m._modules.items()]
+        return False
+
     def _native_args(self, dt, device):
         """The argument block of ptv3_block_fwd with this block's parameters filled
         in.  It is rebuilt whenever a parameter object or its storage changed; the
@@ -330,6 +343,9 @@ class Block(PointModule):
     def _native_static_ok(self, dt, f32=False):
         """Shape conditions of the single-call path that do not depend on the input (``f32``: of the fp32
         block on split weights, which only the one-call backbone uses)."""
+        if not self._same_modules():
+            for k in [k for k in self.__dict__ if k == "_ptv3_block_args" or k[0] == "_ptv3_native_ok"]:
+                del self.__dict__[k]
         key = ("_ptv3_native_ok", dt, f32)
         ok = self.__dict__.get(key)
         if ok is None:

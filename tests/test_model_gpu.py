@@ -495,6 +495,39 @@ def test_values_written_through_data_between_passes(name, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("name", ["enc.enc0.block0.cpe.0", "enc.enc1.block0.norm1.0", "enc.enc1.down.proj",
+                                  "dec.dec0.block0.attn.qkv", "dec.dec0.block0.mlp.0.fc1", "dec.dec0.block0.mlp.0"])
+@pytest.mark.parametrize("hooked", [False, True])
+def test_module_replaced_between_passes(name, hooked):
+    """A layer exchanged for another one of its kind, in the one-call form and in the module tree: its weights count,
+    not those of the layer that was there."""
+    import copy
+    data = small_batch([900, 500], 7)
+    net = P.PointTransformerV3(in_channels=6, **SMALL_CFG)
+    weights.fill_state_dict(net, prefix="ptv3.")
+    net = net.eval().cuda().bfloat16()
+    if hooked:
+        net.enc.enc2.block0.register_forward_hook(lambda *a: None)
+    fresh = copy.deepcopy(net)
+
+    def run(n):
+        torch.manual_seed(5)
+        with torch.inference_mode():
+            return n(cuda_data(data, torch.bfloat16)).feat
+    for _ in range(2):
+        before = run(net)
+    other = copy.deepcopy(net.get_submodule(name))
+    with torch.no_grad():
+        for p in other.parameters():
+            p.mul_(2)
+    for n in (net, fresh):
+        owner, _, key = name.rpartition(".")
+        n.get_submodule(owner)._modules[key] = copy.deepcopy(other)
+    got, ref = run(net), run(fresh)
+    assert torch.equal(got, ref) and not torch.equal(got, before)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("name", ["embedding.stem.norm", "enc.enc1.down.norm.0", "enc.enc0.block0.cpe.2",
                                   "dec.dec0.block0.norm1.0", "dec.dec0.block0.norm2.0"])
 @pytest.mark.parametrize("hooked", [False, True])
