@@ -289,10 +289,18 @@ class Block(PointModule):
         return (self._fusable_form() and point.feat.dtype in (torch.float32, torch.bfloat16)
                 and "sparse_conv_feat" in point.keys())
 
+    def _kept(self, *names):
+        return [k for k in self.__dict__ if (k[0] if type(k) is tuple else k) in names]
+
+    def __getstate__(self):
+        """Copies and pickles go without what was made for this block alone (addresses of its parameters)."""
+        kept = self._kept("_ptv3_block_args", "_ptv3_native_ok", "_ptv3_modules")
+        return {k: v for k, v in self.__dict__.items() if k not in kept}
+
     def _same_modules(self):
         """Whether the block is still made of the modules that it was made of when this was last asked."""
         chain = self.__dict__.get("_ptv3_modules")
-        if chain is not None:
+        if chain is not None and chain[0][0] is self._modules:
             for owner, name, child in chain:
                 if owner.get(name) is not child:
                     break
@@ -344,7 +352,7 @@ class Block(PointModule):
         """Shape conditions of the single-call path that do not depend on the input (``f32``: of the fp32
         block on split weights, which only the one-call backbone uses)."""
         if not self._same_modules():
-            for k in [k for k in self.__dict__ if k == "_ptv3_block_args" or k[0] == "_ptv3_native_ok"]:
+            for k in self._kept("_ptv3_block_args", "_ptv3_native_ok"):
                 del self.__dict__[k]
         key = ("_ptv3_native_ok", dt, f32)
         ok = self.__dict__.get(key)

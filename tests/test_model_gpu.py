@@ -495,6 +495,38 @@ def test_values_written_through_data_between_passes(name, dtype):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("hooked", [False, True])
+def test_network_copied_after_a_pass(hooked):
+    """A network that has run can be copied and pickled, and the copies run on their own parameters."""
+    import copy
+    import io
+    data = small_batch([900, 500], 7)
+    net = P.PointTransformerV3(in_channels=6, **SMALL_CFG)
+    weights.fill_state_dict(net, prefix="ptv3.")
+    net = net.eval().cuda().bfloat16()
+    if hooked:
+        net.enc.enc2.block0.register_forward_pre_hook(_look)
+
+    def run(n):
+        torch.manual_seed(5)
+        with torch.inference_mode():
+            return n(cuda_data(data, torch.bfloat16)).feat
+    ref = run(net)
+    buf = io.BytesIO()
+    torch.save(net, buf)
+    buf.seek(0)
+    for other in (copy.deepcopy(net), torch.load(buf, weights_only=False)):
+        assert torch.equal(run(other), ref)
+        with torch.no_grad():
+            other.dec.dec0.block0.mlp[0].fc1.weight.mul_(2)
+        assert not torch.equal(run(other), ref) and torch.equal(run(net), ref)
+
+
+def _look(*args):
+    return None
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("name", ["enc.enc0.block0.cpe.0", "enc.enc1.block0.norm1.0", "enc.enc1.down.proj",
                                   "dec.dec0.block0.attn.qkv", "dec.dec0.block0.mlp.0.fc1", "dec.dec0.block0.mlp.0"])
 @pytest.mark.parametrize("hooked", [False, True])
