@@ -33,6 +33,8 @@ constexpr int AM_THREADS = 256;
 constexpr int AM_WARPS = AM_THREADS / 32;
 constexpr int AM_KC = 64;           // keys per online-softmax step
 constexpr int AM_D = 16;
+constexpr int AM_MAX_SLICES = 16;
+constexpr size_t AM_SM_SMEM = 228 * 1024;    // shared memory of an SM, of which a CTA takes 1 KiB more than it asks for
 constexpr float AM_LOG2E = 1.4426950408889634f;
 constexpr float AM_LAZY = 8.f;       // slack of the running maximum, in powers of two
 constexpr float AM_BOUND = 80.f;     // largest |score| (exp2 domain) taken without a reference value
@@ -312,8 +314,49 @@ __global__ void __launch_bounds__(AM_THREADS, 3) attn_mma_d16_kernel(
     }
 }
 
-constexpr int AM_WAVE = 3 * SMS;                    // CTAs that run at once
-constexpr int AM_ENOUGH = AM_WAVE * 9 / 5;          // nearly two waves
+// How a launch is cut: slices of the queries of a (sequence, head) pair, each a CTA that gathers K and V again, and
+// CTAs per SM.
+struct AmCut {
+    int slices, per_sm;
+};
+
+// The cut with the shortest estimated time.  Up to three CTAs share an SM (four schedulers, two warps of a CTA on
+// each); a launch that gives no SM more than one or two is held to that number, because CTAs otherwise
+// pile up on the SMs that are free first (2 sequences of 1 024 x 16 heads in eight slices: 23.9 us, 17.3 with two per SM).
+// The estimate, in cycles (measured on sequences of 27 to 1 024; within 5 % from 32 pairs of 1 024 up):
+//   * a CTA starts with a gather, 4 800 and 3 800 more per 1 024 rows and CTA of the SM, one after another;
+//   * a scheduler takes 78 per tile and 16 keys, but one of its two warps in a CTA at least 172, the chain through
+//     the units (a warp alone 136);
+//   * where an SM has more CTAs than run at once they follow one another, at 1 500 more each (a gather, where
+//     there is room for one).
+// us with the cut before (a power of two of slices up to nearly two waves of three per SM) and now, 1 024 points a
+// sequence: 12 pairs 17.1 / 10.6, 32 pairs 23.9 / 16.3, 56 pairs 29.3 / 25.7, 196 pairs 69.5 / 65.1, 392 pairs
+// 130 / 121, 784 pairs 231 / 231; 32 pairs of 457 points 10.0 / 7.1, 128 pairs of 560 25.3 / 20.7.
+static AmCut am_cut(int64_t pairs, int max_seqlen, size_t smem)
+{
+    const int tiles = (max_seqlen + 15) / 16;
+    int fit = (int)(AM_SM_SMEM / (smem + 1024));
+    fit = fit < 1 ? 1 : fit > 3 ? 3 : fit;
+    const double rows = max_seqlen / 1024.0, steps = (max_seqlen + 15) / 16;
+    AmCut best{1, fit};
+    double least = 0;
+    for (int q = 1; q <= AM_MAX_SLICES && (q - 1) * 4 < tiles; ++q) {
+        const int per = (tiles + q - 1) / q, slices = (tiles + per - 1) / per;
+        if (slices < q) continue;
+        const int64_t on_sm = (pairs * slices + SMS - 1) / SMS;
+        const int c = on_sm < fit ? (int)on_sm : fit;
+        const double busy = 78. * on_sm * (on_sm > c && per >= 8 ? per / 4. : (per + 3) / 4);
+        const double chain = (double)((on_sm + c - 1) / c) * (per / 8 * 172 + (per % 8 > 4 ? 172 : per % 8 ? 136 : 0));
+        const double start = 4800 + 3800 * rows * c;
+        const double t = start + steps * (busy > chain ? busy : chain) +
+                         (on_sm - c) * (fit == 1 ? start : 700 + 800 * rows);
+        if (q == 1 || t < least) {
+            least = t;
+            best = AmCut{slices, c};
+        }
+    }
+    return best;
+}
 
 bool attn_mma_supported(int channels, int heads, int max_seqlen)
 {
@@ -327,30 +370,15 @@ int launch_attn_mma(const void* qkv, const int64_t* order, const int64_t* pad, c
 {
     const int lpad = (max_seqlen + AM_KC - 1) / AM_KC * AM_KC;
     const size_t smem = (size_t)lpad * 68;      // K, V and the row numbers
-    // per device and cheap, so it is simply repeated on every call
     auto kern = packed_exp ? attn_mma_d16_kernel<true> : attn_mma_d16_kernel<false>;
     if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_attention_fwd: shared memory attribute");
-    // Queries of a sequence are sliced over CTAs, each of which gathers K and V again.  A launch wants nearly two
-    // waves of three CTAs per SM, or one that is nearly full: fewer CTAs land unevenly on the SMs (a dependent
-    // launch fills the first ones that the kernel before it leaves), more gather more often.  us in 1 / 2 / 4 / 8
-    // slices by (sequence, head) pairs, sequences of 1 024:
-    //      16   49 /  27 /  16 /  14        96   88 /  55 /  40 /  42       200   90 /  71 /  71 /  72
-    //      48   49 /  49 /  32 /  25       108   98 /  49 /  40 /  42       224  128 /  89 /  81 /  83
-    //      80   75 /  66 /  40 /  37       128  109 /  69 /  50 /  49       320  131 / 110 / 103 / 112
-    //     436  131 / 131 / 135 / 148       640  210 / 192 / 198 / 215     1 564  449 / 451 / 456 / 507
-    // The wave that is nearly full decides at 93 to 111 pairs (5 %) and costs nothing at 186 to 222 and above 412.
-    // The rule is behind the best of the four at 144 and 176 pairs (54 and 66 us, 50 and 61 in four slices), at
-    // 370 to 400 (131, 124 in four) and at 1 200 (368, 351 in two); elsewhere within 3 %.
-    const int tiles = (max_seqlen + 15) / 16;
-    const int64_t pairs = (int64_t)n_seq * H;
-    int qsplit = 1;
-    while (qsplit < 8 && qsplit * AM_WARPS < tiles && pairs * qsplit < AM_ENOUGH &&
-           !(pairs * qsplit >= AM_WAVE * 5 / 6 && pairs * qsplit <= AM_WAVE))
-        qsplit *= 2;
-    const dim3 grid(H * qsplit, n_seq);
-    launch_dependent(kern, grid, dim3(AM_THREADS), smem, stream, (const __nv_bfloat16*)qkv, order, pad, unpad, cu,
-                     (__nv_bfloat16*)out, C, scale, lpad, status);
+    const AmCut cut = am_cut((int64_t)n_seq * H, max_seqlen, smem);
+    // (shared memory that only so many CTAs find room for)
+    const size_t least = cut.per_sm < 3 ? AM_SM_SMEM / (cut.per_sm + 1) : 0;
+    const dim3 grid(H * cut.slices, n_seq);
+    launch_dependent(kern, grid, dim3(AM_THREADS), smem > least ? smem : least, stream, (const __nv_bfloat16*)qkv,
+                     order, pad, unpad, cu, (__nv_bfloat16*)out, C, scale, lpad, status);
     count_launches(1);
     return check_launch("ptv3_attention_fwd");
 }

@@ -91,7 +91,7 @@ struct BbLevel {
     const int32_t *grid = nullptr, *nbr = nullptr;
     int64_t *cluster = nullptr, *idx_ptr = nullptr;         // pooling of this level into the next
     // patch layout, made for patch size `patch`
-    int patch = 0, n_seq = 0;
+    int patch = 0, n_seq = 0, longest = 0;                  // (longest: no sequence has more rows)
     int64_t *pad = nullptr, *unpad = nullptr;
     int32_t* cu = nullptr;
     const void* feat = nullptr;                             // encoder output (skip connection)
@@ -170,12 +170,14 @@ int Pass::pad_level(BbLevel& l, int patch, Arena& mem, cudaStream_t stream, int6
 {
     if (l.patch == patch) return PTV3_OK;
     PTV3_REQUIRE(patch >= 1, PTV3_ERR_INVALID_ARGUMENT, "ptv3_backbone_fwd: patch size %d", patch);
-    int64_t n_pad = 0, n_seq = 0;
+    int64_t n_pad = 0, n_seq = 0, longest = 1;
     for (int b = 0; b < a_.n_scenes; ++b) {
         const int64_t c = l.counts[b], cp = c > patch ? (c + patch - 1) / patch * patch : c;
         n_pad += cp;
         n_seq += (cp + patch - 1) / patch;
+        longest = c > longest ? c : longest;
     }
+    l.longest = longest < patch ? (int)longest : patch;
     l.pad = pad ? pad : mem.take<int64_t>(n_pad);
     l.unpad = unpad ? unpad : mem.take<int64_t>(l.n);
     l.cu = cu ? cu : mem.take<int32_t>(n_seq + 1);
@@ -414,7 +416,7 @@ int Pass::block(const ptv3_stage_args& st, int j, BbLevel& l, const void* conv_i
     BB_STEP(pad_level(l, patch_of(st.patch[j], l, a_.n_scenes), mem_, main_, nullptr, nullptr, nullptr));
     b.n = l.n;
     b.n_seq = l.n_seq;
-    b.max_seqlen = l.patch;
+    b.max_seqlen = l.longest;
     b.conv_in = conv_in;
     b.feat = feat;
     b.out = out;

@@ -243,6 +243,24 @@ def test_attention_tcgen05_path_matches_cuda_core_path(sizes, C, H, K):
         assert rel_l2(b, a) < 5e-3
 
 
+@pytest.mark.parametrize("n,H,K", [(16, 1, 16), (17, 32, 1024), (105, 16, 1024), (457, 32, 1024), (1757, 16, 1024),
+                                   (3001, 2, 256), (6760, 8, 1024), (26000, 4, 1024), (2049, 2, 2048)])
+def test_attention_cuts_cover_every_row_once(n, H, K):
+    """Launches from one slice per (sequence, head) pair to sixteen, held to one, two or three CTAs per SM: every
+    row of the mma.sync kernel (algo 2) as the CUDA-core kernel has it, whether the stated longest sequence is the real one
+    or longer."""
+    C = 16 * H
+    g = torch.Generator().manual_seed(n)
+    qkv = (torch.randn(n, 3 * C, generator=g) * 1.5).bfloat16().cuda()
+    order = torch.randperm(n, generator=g).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    a = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25, algo=1)
+    for stated in (K, min(n, K)):
+        b = ops.attention(qkv, order, pad, unpad, cu, H, stated, 0.25, algo=2)
+        assert_close(b, a, atol=1e-2, rtol=1e-2, what="slices of attention")
+        assert rel_l2(b, a) < 5e-3
+
+
 def test_attention_tcgen05_large_scores():
     """Scores far from zero (|s| up to a few hundred): the running maximum and the
     rescaling of the output across key blocks must hold."""
