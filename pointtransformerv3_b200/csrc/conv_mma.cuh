@@ -20,6 +20,12 @@ int launch_conv_tc05(const void* feat, const int32_t* nbr, const void* weight, c
                      const int64_t* row_order, int64_t n, int c_in, int c_out, int kernel_volume,
                      uint32_t* status, cudaStream_t stream);
 
+// The same as a persistent kernel (conv_stream.cu), tiles of `bn` output channels: 32 (32 -> 32 channels only), 64, 128
+// or 256
+int launch_conv_stream(const void* feat, const int32_t* nbr, const void* weight, const void* bias, void* out,
+                       const int64_t* row_order, int64_t n, int c_in, int c_out, int kernel_volume, int bn,
+                       uint32_t* status, cudaStream_t stream);
+
 // Pair-list form (coarse levels): pairs sorted by kernel offset, 128-pair tiles,
 // atomic fixed-point accumulation into acc (n x c_out 64-bit integers of workspace), then
 // bias + rounding into out.

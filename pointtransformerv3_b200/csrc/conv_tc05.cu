@@ -1,39 +1,32 @@
-// Submanifold convolution (3x3x3) for bf16 features on the 5th-generation tensor cores:
-// an implicit GEMM, output-stationary over tiles of 128 voxels, accumulated in tensor memory.
+// Submanifold convolution (3x3x3) on the 5th-generation tensor cores where tiles are few (the coarse levels, small
+// rooms), and for fp32 features: an implicit GEMM, output-stationary over tiles of 128 voxels, accumulated in tensor
+// memory.  bf16 inputs of many tiles take the persistent kernel in conv_stream.cu.
 //
 // A CTA owns 128 voxels (consecutive in the tile order, which follows a space-filling curve) and
 // BN output channels.  It stages the 27 x 128 neighbour rows of its tile in shared memory and
 // drops the offsets for which no voxel of the tile has a neighbour.  Then, for each remaining
 // offset o and each KC-wide slice of the input channels,
-//   warps 0..3  each fill every fourth stage: the 128 neighbour rows (zero rows where there is none)
-//               gathered with cp.async into the 128-byte (64-byte for KC = 32) swizzled K-major
-//               operand layout, and the matching BN x KC slice of W[:, o, :] fetched with TMA into
-//               the same layout,
-//   warp 4      issues KC / 16 tcgen05.mma (M = 128, N = BN, K = 16) that add A_o W_o^T to the
-//               accumulator in tensor memory, and releases the stage with tcgen05.commit,
-// through a ring of stages guarded by mbarriers.  When the last product has completed, warps 0..3
+//   gather warps  each fill every NGW-th stage: the 128 neighbour rows (zero rows where there is none)
+//                 gathered with cp.async into the 128-byte swizzled K-major operand layout, and the
+//                 matching BN x KC slice of W[:, o, :] fetched with TMA into the same layout,
+//   issuers       issue KC / 16 tcgen05.mma (M = 128, N = BN, K = 16) that add A_o W_o^T to the
+//                 accumulator in tensor memory, and release the stage with tcgen05.commit,
+// through a ring of stages guarded by mbarriers.  When the last product has completed, the gather warps
 // read the accumulator (thread = voxel), add the bias, round to bf16 and store their rows.
 //
-// Two threads issue the products, taking the stages in turn, each into its own accumulator (one
-// thread can start a stage only every ~450 cycles: looking at a stage's barrier costs it as much as
-// issuing the stage's four products); the epilogue adds the two partial sums.  Every sum is taken
-// in one fixed order, so the result is the same bit for bit on every run, on every level: no
-// atomics, no pair lists, no second pass.  Products with zero rows are not skipped (on coarse
-// levels about two thirds of the rows of an active offset are empty): the tensor pipe has time to
-// spare.  What bounds the kernel is the length of a slot's cycle, not a throughput: once a slot is
-// free its warp issues the weight load and 32 copies per lane (~1100 cycles), the rows land (~1200),
-// the warp fences and arrives, an issuer notices, issues, the products complete and the commit
-// frees the slot (~1500 more): ~4000 cycles for six slots, one stage per ~700 cycles.  Counters of
-// one launch: tensor pipe 22 % active, shared-memory pipe 29 % (16 % operand reads of the tensor
-// core, 13 % copies and loads), L2 19 %, DRAM 5 %; leaving out the gather copies or the weight
-// loads altogether changes the time by 10 % and 2 %.
+// Two threads issue the products, taking the stages in turn, each into its own accumulator; the epilogue adds
+// the two partial sums.  Every sum is taken in one fixed order, so the result is the same bit for bit on every run, on
+// every level: no atomics, no pair lists, no second pass.  Products with zero rows are not skipped.
+// What bounds it on few tiles: ~7 us before the first and after the last product, and ~370 cycles per stage of 64
+// channels, 500 of 128, 700 of 256 (see conv_stream.cu for what a stage is made of).
 //
-// Few tiles (the coarse levels, small rooms): a cluster of up to eight CTAs shares one tile.  Each takes a
+// A cluster of up to eight CTAs shares one tile.  Each takes a
 // contiguous share of the tile's stages; the partial sums meet in shared memory and every CTA adds the
 // peers' parts of its rows, in rank order, through distributed shared memory.  A tile alone walks
-// 27 x c_in / 64 stages one after the other, 49 us at 512 channels on 27 voxels, while most SMs have nothing.
+// 27 x c_in / 64 stages one after the other, 49 us at 512 channels on 27 voxels, while most SMs have nothing; in
+// clusters of eight that is 10 us.
 //
-// Replaces spconv.SubMConv3d.forward at model.py:546-552 for bf16.
+// Replaces spconv.SubMConv3d.forward at model.py:546-552.
 // Useful work: 2 . pairs . C_in . C_out FLOP.  Every mbarrier wait is bounded and reports through
 // the status word.
 #include <atomic>
@@ -470,61 +463,79 @@ static int conv_tc05_capacity(int parts)
 }
 
 struct ConvVariant {
-    int bn, per_sm;
-    double stage_us;
+    int bn;
+    double fixed_us, load_us, stage_us;      // load_us: more for a CTA on every SM
     int (*plain)(const void*, const ConvTcArgs&, cudaStream_t, int);
     int (*split)(const void*, const ConvTcArgs&, cudaStream_t, int);
     int (*capacity)(int);
 };
-constexpr double CT_FIXED_US = 6.5;
-constexpr int CT_VARIANTS = 5;
-template <int BN, int STAGES, bool F32>
-static constexpr ConvVariant conv_variant(double stage_us)
-{
-    return {BN, 1, stage_us, launch_conv_tc05_as<BN, 64, STAGES, 2, false, F32>,
-            launch_conv_tc05_as<BN, 64, STAGES, 2, true, F32>, conv_tc05_capacity<BN, 64, STAGES, 2, F32>};
-}
-// [fp32 output][variant].  Second entry: many tiles, two CTAs per SM, so that one tile's prologue and epilogue
-// run beside another's products.  Last: 32 output channels (fp32; bf16 has its own path for them).
-static const ConvVariant g_variants[2][CT_VARIANTS] = {
-    {conv_variant<64, 8, false>(0.20),
-     {64, 2, 0.35, launch_conv_tc05_as<64, 64, 4, 2, false, false>, nullptr, nullptr},
-     conv_variant<128, 6, false>(0.28), conv_variant<256, 4, false>(0.44), {1 << 20, 1, 0, nullptr, nullptr, nullptr}},
-    // (fp32: an issuer's four accumulators of 64 columns fill the tensor memory of an SM)
-    {conv_variant<64, 8, true>(0.20), {1 << 20, 1, 0, nullptr, nullptr, nullptr}, {1 << 20, 1, 0, nullptr, nullptr, nullptr},
-     {1 << 20, 1, 0, nullptr, nullptr, nullptr}, conv_variant<32, 8, true>(0.18)},
-};
+constexpr int CT_VARIANTS = 3;
+// fp32 output (an issuer's four accumulators of 64 columns fill the tensor memory of an SM).  Last: 32 channels.
+static const ConvVariant g_variants_f32[CT_VARIANTS] = {
+    {64, 6.5, 0, 0.20, launch_conv_tc05_as<64, 64, 8, 2, false, true>, launch_conv_tc05_as<64, 64, 8, 2, true, true>,
+     conv_tc05_capacity<64, 64, 8, 2, true>},
+    {32, 6.5, 0, 0.18, launch_conv_tc05_as<32, 64, 8, 2, false, true>, launch_conv_tc05_as<32, 64, 8, 2, true, true>,
+     conv_tc05_capacity<32, 64, 8, 2, true>},
+    {1 << 20, 0, 0, 0, nullptr, nullptr, nullptr}};
+// bf16: clusters here, whole tiles in conv_stream.cu
+static const ConvVariant g_variants[CT_VARIANTS] = {
+    {64, 6.9, 1.6, 0.19, nullptr, launch_conv_tc05_as<64, 64, 8, 2, true, false>, conv_tc05_capacity<64, 64, 8, 2, false>},
+    {128, 8.7, 1.6, 0.26, nullptr, launch_conv_tc05_as<128, 64, 6, 2, true, false>, conv_tc05_capacity<128, 64, 6, 2, false>},
+    {256, 12., 1.6, 0.37, nullptr, launch_conv_tc05_as<256, 64, 4, 2, true, false>, conv_tc05_capacity<256, 64, 4, 2, false>}};
 
-// The tile width and the cluster size with the shortest estimated time: waves of CTAs, each taking a
+// The cluster size and tile width with the shortest estimated time: waves of CTAs, each taking a
 // fixed time (prologue, epilogue) and its stages.  Wide tiles gather a row once for more output
-// channels; clusters fill SMs that a single wave leaves idle.  The constants are measured (us on B200:
-// 27 voxels x 512 channels in clusters of eight takes 12.2 / 14.6 / 19.9 with 64 / 128 / 256 channels a
-// tile, 46.3 without a cluster); what they give: 441 x 512 47 -> 19, 1 700 x 256 27 -> 18,
-// 2 200 x 512 49 -> 39, 12 000 x 256 68 -> 53, 12 000 x 128 31 -> 22.
-static int launch_conv_tc05_best(const void* weight, const ConvTcArgs& a, bool f32, cudaStream_t stream)
+// channels; clusters fill SMs that a single wave leaves idle.  `stages`: of a tile.  The constants are measured.
+static double conv_cluster_cost(const ConvVariant* variants, const ConvTcArgs& a, double stages, int* best_v, int* best_parts)
 {
-    const double stages = (double)a.kvol * (a.cin / 64);
     const int64_t tiles = (a.n + CT_TM - 1) / CT_TM;
     double best = 0;
-    int best_v = -1, best_parts = 1;
+    *best_v = -1;
     for (int v = 0; v < CT_VARIANTS; ++v) {
-        const ConvVariant& var = g_variants[f32][v];
+        const ConvVariant& var = variants[v];
         if (a.cout % var.bn) continue;
         const int64_t ctas = tiles * (a.cout / var.bn);
-        for (int parts = 1; parts <= (var.split ? 8 : 1); parts *= 2) {
-            const int64_t room = parts == 1 ? (int64_t)SMS * var.per_sm : (int64_t)var.capacity(parts);
+        for (int parts = var.plain ? 1 : 2; parts <= 8; parts *= 2) {
+            const int64_t room = parts == 1 ? (int64_t)SMS : (int64_t)var.capacity(parts);
             if (room < parts) continue;
             if (parts > 1 && (ctas * parts > room || stages < 2 * parts)) continue;       // a cluster only within one wave
-            const double cost = (double)((ctas * parts + room - 1) / room) * (CT_FIXED_US + stages / parts * var.stage_us);
-            if (best_v < 0 || cost < best) {
+            const double cost = (double)((ctas * parts + room - 1) / room) *
+                                (var.fixed_us + var.load_us * (double)(ctas * parts) / SMS + stages / parts * var.stage_us);
+            if (*best_v < 0 || cost < best) {
                 best = cost;
-                best_v = v;
-                best_parts = parts;
+                *best_v = v;
+                *best_parts = parts;
             }
         }
     }
-    const ConvVariant& var = g_variants[f32][best_v];
-    return (best_parts > 1 ? var.split : var.plain)(weight, a, stream, best_parts);
+    return best;
+}
+
+// bf16: persistent CTAs on whole tiles (conv_stream.cu) or clusters that share them, whichever should be faster.  About
+// half of the offsets of a tile are in use (9 to 19 of 27 on rooms from fine to coarse levels).  A persistent CTA
+// takes a fixed time and its stages, at the pace of its own chain or, with all SMs at work, of what they share.
+// us, estimated best of the clusters against the persistent kernel, measured: 1 757 x 256 13.4 / 18.3 (it was 19.9 in
+// clusters of eight with 256-wide tiles, when all offsets were counted), 457 x 512 15.5 / 32, 2 240 x 512 25.3 / 30,
+// 6 760 x 128 11.9 / 11.7, 7 700 x 256 23.0 / 22.8, 5 200 x 512 56.7 / 44.8, 26 000 x 64 12.3 / 10.8.
+static int conv_stream_width(const ConvTcArgs& a, double stages, double* cost)
+{
+    static const struct {
+        int bn;
+        double fixed_us, chain_us, shared_us;
+    } widths[3] = {{64, 6.3, 0.19, 0.31}, {128, 9.5, 0.21, 0.36}, {256, 12., 0.53, 0.57}};
+    const int64_t tiles = (a.n + CT_TM - 1) / CT_TM;
+    int best = 0;
+    for (const auto& w : widths) {
+        if (a.cout % w.bn) continue;
+        const int64_t ctas = tiles * (a.cout / w.bn);
+        const double chain = (double)((ctas + SMS - 1) / SMS) * w.chain_us, shared = (double)ctas / SMS * w.shared_us;
+        const double t = w.fixed_us + stages * (chain > shared ? chain : shared);
+        if (!best || t < *cost) {
+            best = w.bn;
+            *cost = t;
+        }
+    }
+    return best;
 }
 
 int launch_conv_tc05(const void* feat, const int32_t* nbr, const void* weight, const void* bias, void* out,
@@ -542,8 +553,17 @@ int launch_conv_tc05(const void* feat, const int32_t* nbr, const void* weight, c
     a.cout = c_out;
     a.kvol = kvol;
     a.status = status;
-    if (c_in == 32) return launch_conv_tc05_as<32, 32, 6, 2, false, false>(weight, a, stream, 1);
-    return launch_conv_tc05_best(weight, a, false, stream);
+    auto stream_form = [&](int bn) {
+        return launch_conv_stream(feat, nbr, weight, bias, out, row_order, n, c_in, c_out, kvol, bn, status, stream);
+    };
+    if (c_in == 32) return stream_form(32);
+    const double stages = 0.5 * kvol * (c_in / 64);
+    double whole = 0;
+    int v, parts = 1;
+    const int bn = conv_stream_width(a, stages, &whole);
+    const double shared = conv_cluster_cost(g_variants, a, stages, &v, &parts);
+    if (v < 0 || whole <= shared) return stream_form(bn);
+    return g_variants[v].split(weight, a, stream, parts);
 }
 
 // fp32 on split operands (see split_f32.cuh)
@@ -563,7 +583,9 @@ int launch_conv_split(const void* feat, const int32_t* nbr, const void* weight, 
     a.cout = c_out;
     a.kvol = kvol;
     a.status = status;
-    return launch_conv_tc05_best(weight, a, true, stream);
+    int v, parts = 1;
+    conv_cluster_cost(g_variants_f32, a, (double)a.kvol * (a.cin / 64), &v, &parts);
+    return (parts > 1 ? g_variants_f32[v].split : g_variants_f32[v].plain)(weight, a, stream, parts);
 }
 
 }  // namespace ptv3

@@ -444,6 +444,33 @@ def test_subm_conv_tcgen05_clusters(n, c):
     assert rel_l2(got, base) < 2e-3
 
 
+@pytest.mark.parametrize("n,cin,cout", [(1, 32, 32), (127, 64, 64), (129, 64, 192), (19100, 32, 32), (19100, 64, 64),
+                                        (19100, 64, 128), (40000, 128, 128), (19500, 256, 256), (10100, 128, 512)])
+def test_subm_conv_tcgen05_many_tiles(n, cin, cout):
+    """More tiles than SMs, so that a persistent CTA goes on to a second and third tile: ring, index buffers and
+    accumulators wrap round.  A tile without any neighbour, one with a single offset in use, a ragged last tile, rows in
+    another order; against the CUDA-core kernel, and the same bits twice."""
+    g = torch.Generator().manual_seed(n + cin)
+    nbr = torch.randint(0, n, (27, n), generator=g, dtype=torch.int32)
+    nbr[torch.rand(27, n, generator=g) > 0.3] = -1
+    nbr[torch.randperm(27, generator=g)[:12]] = -1
+    nbr[:, 128:256] = -1
+    nbr[:, 256:384] = -1
+    nbr[4, 300:384] = torch.randint(0, n, (84,), generator=g, dtype=torch.int32)[:nbr[4, 300:384].numel()]
+    nbr = nbr.cuda()
+    feat = torch.randn(n, cin, generator=g).bfloat16().cuda()
+    w = (torch.randn(cout, 3, 3, 3, cin, generator=g) / (8 * cin) ** 0.5).bfloat16().cuda()
+    b = torch.randn(cout, generator=g).bfloat16().cuda()
+    row_order = torch.randperm(n, generator=g).cuda()
+    got = ops.subm_conv(feat, nbr, w, b, algo=3, row_order=row_order)
+    assert torch.equal(got, ops.subm_conv(feat, nbr, w, b, algo=3, row_order=row_order))
+    base = ops.subm_conv(feat, nbr, w, b, algo=1, row_order=row_order)
+    assert_close(got, base, atol=1e-2, rtol=1e-2, what="persistent convolution vs CUDA-core kernel")
+    assert rel_l2(got, base) < 5e-3
+    assert_close(ops.subm_conv(feat, nbr, w, None, algo=3, row_order=row_order),
+                 ops.subm_conv(feat, nbr, w, None, algo=1, row_order=row_order), atol=1e-2, rtol=1e-2, what="no bias")
+
+
 @pytest.mark.parametrize("permuted", [False, True])
 @pytest.mark.parametrize("cin,cout,shift", [(32, 32, 0), (64, 64, 0), (128, 128, 1), (256, 256, 2), (512, 512, 3),
                                             (64, 192, 1)])
