@@ -11,7 +11,7 @@
 //                   (zero rows where there is none) into the 128-byte (64 for 32 channels) swizzled K-major layout
 //                   and asks TMA for the slice of W,
 //   issuers         take the stages in turn, each into its own accumulator: tcgen05.mma (M = 128, N = BN, K = 16) into
-//                   one of two sets of accumulators in tensor memory,
+//                   one of two sets of accumulators in tensor memory (256 columns: the only set),
 //   epilogue warps  add the issuers' partial sums and the bias and store the rows, while the next tile is multiplied.
 // The stages of a tile go round the issuers and every sum is taken in one fixed order, so the result is the same bit
 // for bit on every run.
@@ -69,14 +69,14 @@ struct ConvIndex {
     unsigned mask[4];
 };
 
-template <int BN, int KC, int STAGES, int NI, int GW>
-__global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + 4) * 32, 1) conv_stream_kernel(
+template <int BN, int KC, int STAGES, int NI, int GW, int SETS, int EW>
+__global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + EW) * 32, 1) conv_stream_kernel(
     const __grid_constant__ CUtensorMap map_w, const ConvStreamArgs a)
 {
     constexpr int ROWB = KC * 2, NCH = ROWB / 16;
     constexpr int A_BYTES = CS_TM * ROWB, B_BYTES = BN * ROWB, STAGE_BYTES = A_BYTES + B_BYTES;
     constexpr int EPI = cs_epi_warp<GW, NI>();
-    constexpr int TM_COLS = 2 * NI * BN;
+    constexpr int TM_COLS = SETS * NI * BN;
     static_assert(TM_COLS >= 32 && TM_COLS <= 512 && (TM_COLS & (TM_COLS - 1)) == 0, "tensor memory");
     static_assert(STAGE_BYTES % 1024 == 0 && A_BYTES % 1024 == 0, "operand tiles start on a swizzle atom");
     // a parity wait can only tell a phase from the one before it: see conv_tc05.cu
@@ -101,9 +101,9 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + 4) * 32, 1) conv_stre
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(accfull0 + 8 * b, NI);
-            mbar_init(accempty0 + 8 * b, 4);
+            mbar_init(accempty0 + 8 * b, EW);
             mbar_init(idxfull0 + 8 * b, 2);
-            mbar_init(idxempty0 + 8 * b, GW + NI + 4);
+            mbar_init(idxempty0 + 8 * b, GW + NI + EW);
         }
         *abort = 0;
         fence_barrier_init();
@@ -190,10 +190,10 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + 4) * 32, 1) conv_stre
             __syncwarp();
             if (lane == 0) mbar_arrive_one(idxempty0 + 8 * b);
             // the epilogue has read this set of accumulators (first use: free)
-            ok &= mbar_wait(accempty0 + 8 * b, ((i >> 1) & 1) ^ 1, abort);
+            ok &= mbar_wait(accempty0 + 8 * (i % SETS), ((i / SETS) & 1) ^ 1, abort);
             if (!__all_sync(0xffffffffu, ok)) break;
             fence_after_sync();
-            const uint32_t acc = tmem_base + (b * NI + me) * BN;
+            const uint32_t acc = tmem_base + (i % SETS * NI + me) * BN;
             bool more = false;
             for (; g < end; g += NI) {
                 const uint64_t da = da0 + s * (STAGE_BYTES >> 4), db = db0 + s * (STAGE_BYTES >> 4);
@@ -213,8 +213,8 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + 4) * 32, 1) conv_stre
                 }
             }
             if (lane == 0) {
-                if (more) umma_commit(accfull0 + 8 * b);
-                else mbar_arrive_one(accfull0 + 8 * b);
+                if (more) umma_commit(accfull0 + 8 * (i % SETS));
+                else mbar_arrive_one(accfull0 + 8 * (i % SETS));
             }
             __syncwarp();
             seen = end;
@@ -272,18 +272,21 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + 4) * 32, 1) conv_stre
         }
     } else if (warp >= EPI) {
         // ---- epilogue ------------------------------------------------------------------------------
-        const int q = warp & 3;
+        // A warp takes its share of the columns out of tensor memory, rounded, before it stores any: where there is
+        // one set of accumulators the next tile waits for no more than that.
+        constexpr int BLOCKS = BN / 32 / (EW / 4);        // of 32 columns
+        const int q = warp & 3, cb0 = (warp - EPI) / 4 * BLOCKS;
         for (int i = 0, t = first; t < a.tiles; ++i, t += step) {
-            const int b = i & 1, col0 = t % col_tiles * BN;
-            ok = mbar_wait(idxfull0 + 8 * b, (i >> 1) & 1, abort) && mbar_wait(accfull0 + 8 * b, (i >> 1) & 1, abort);
+            const int b = i & 1, set = i % SETS, col0 = t % col_tiles * BN;
+            ok = mbar_wait(idxfull0 + 8 * b, (i >> 1) & 1, abort) && mbar_wait(accfull0 + 8 * set, (i / SETS) & 1, abort);
             if (!__all_sync(0xffffffffu, ok)) break;
             fence_after_sync();
             const ConvIndex<BN>& x = index[b];
             const int stages = x.act[0] * kchunks;
             // (the issuers' sums are added from that of the tile's first stage on, whoever had it)
-            const uint32_t tm = tmem_base + b * NI * BN + ((uint32_t)(q * 32) << 16);
-#pragma unroll 1
-            for (int cb = 0; cb < BN / 32; ++cb) {
+            const uint32_t tm = tmem_base + set * NI * BN + ((uint32_t)(q * 32) << 16);
+            uint32_t o[SETS == 1 ? BLOCKS : 1][4][4];
+            auto take = [&](int cb, uint32_t (&y)[4][4]) {
                 uint32_t acc[32];
                 if (stages > 0) {
                     tmem_ld32(tm + seen % NI * BN + cb * 32, acc);
@@ -303,45 +306,61 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + 4) * 32, 1) conv_stre
                     for (int e = 0; e < 32; ++e)
                         acc[e] = __float_as_uint(__uint_as_float(acc[e]) + __uint_as_float(more[e]));
                 }
-                uint32_t o[4][4];
 #pragma unroll
                 for (int c = 0; c < 4; ++c)
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         const float2 bias = *reinterpret_cast<const float2*>(&x.bias[cb * 32 + c * 8 + 2 * e]);
-                        o[c][e] = pack_bf16(__uint_as_float(acc[c * 8 + 2 * e]) + bias.x,
+                        y[c][e] = pack_bf16(__uint_as_float(acc[c * 8 + 2 * e]) + bias.x,
                                             __uint_as_float(acc[c * 8 + 2 * e + 1]) + bias.y);
                     }
-                // Four lanes exchange their rows' 16-byte chunks, so that a store writes 64 bytes of eight rows and not
-                // 16 of 32 (with row-per-thread stores 101 us at 407 000 x 64, 88 so, 85 without any).  Afterwards
-                // o[k] is chunk `m` of the row of the k-th of the four.
+            };
+            // Four lanes exchange their rows' 16-byte chunks, so that a store writes 64 bytes of eight rows and not
+            // 16 of 32 (with row-per-thread stores 101 us at 407 000 x 64, 88 so, 85 without any).  Afterwards
+            // y[k] is chunk `m` of the row of the k-th of the four.
+            auto store = [&](int cb, uint32_t (&y)[4][4]) {
                 const int m = lane & 3;
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
-                    uint32_t p0 = __shfl_xor_sync(0xffffffffu, m & 1 ? o[0][e] : o[1][e], 1);
-                    uint32_t p1 = __shfl_xor_sync(0xffffffffu, m & 1 ? o[2][e] : o[3][e], 1);
-                    if (m & 1) o[0][e] = p0, o[2][e] = p1;
-                    else o[1][e] = p0, o[3][e] = p1;
-                    p0 = __shfl_xor_sync(0xffffffffu, m & 2 ? o[0][e] : o[2][e], 2);
-                    p1 = __shfl_xor_sync(0xffffffffu, m & 2 ? o[1][e] : o[3][e], 2);
-                    if (m & 2) o[0][e] = p0, o[1][e] = p1;
-                    else o[2][e] = p0, o[3][e] = p1;
+                    uint32_t p0 = __shfl_xor_sync(0xffffffffu, m & 1 ? y[0][e] : y[1][e], 1);
+                    uint32_t p1 = __shfl_xor_sync(0xffffffffu, m & 1 ? y[2][e] : y[3][e], 1);
+                    if (m & 1) y[0][e] = p0, y[2][e] = p1;
+                    else y[1][e] = p0, y[3][e] = p1;
+                    p0 = __shfl_xor_sync(0xffffffffu, m & 2 ? y[0][e] : y[2][e], 2);
+                    p1 = __shfl_xor_sync(0xffffffffu, m & 2 ? y[1][e] : y[3][e], 2);
+                    if (m & 2) y[0][e] = p0, y[1][e] = p1;
+                    else y[2][e] = p0, y[3][e] = p1;
                 }
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     const int row = x.row[q * 32 + (lane & ~3) + k];
                     if (row >= 0)
                         *reinterpret_cast<uint4*>(a.out + (int64_t)row * a.cout + col0 + cb * 32 + m * 8) =
-                            make_uint4(o[k][0], o[k][1], o[k][2], o[k][3]);
+                            make_uint4(y[k][0], y[k][1], y[k][2], y[k][3]);
                 }
+            };
+            auto release = [&] {
+                fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_one(accempty0 + 8 * set);
+            };
+            if (SETS == 1) {
+#pragma unroll
+                for (int j = 0; j < BLOCKS; ++j) take(cb0 + j, o[SETS == 1 ? j : 0]);
+                release();
+#pragma unroll
+                for (int j = 0; j < BLOCKS; ++j) store(cb0 + j, o[SETS == 1 ? j : 0]);
+            } else {
+#pragma unroll 1
+                for (int j = 0; j < BLOCKS; ++j) {
+                    take(cb0 + j, o[0]);
+                    store(cb0 + j, o[0]);
+                }
+                release();
             }
             seen += stages;
-            fence_before_sync();
             __syncwarp();
-            if (lane == 0) {
-                mbar_arrive_one(accempty0 + 8 * b);
-                mbar_arrive_one(idxempty0 + 8 * b);
-            }
+            if (lane == 0) mbar_arrive_one(idxempty0 + 8 * b);
         }
     }
     __syncwarp();
@@ -354,7 +373,7 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + 4) * 32, 1) conv_stre
     if (lane == 0 && (!ok || (tid == 0 && *abort))) atomicOr(a.status, PTV3_STATUS_WAIT_LIMIT);
 }
 
-template <int BN, int KC, int STAGES, int NI, int GW>
+template <int BN, int KC, int STAGES, int NI, int GW, int SETS, int EW>
 static int launch_as(const void* weight, ConvStreamArgs a, cudaStream_t stream)
 {
     CUtensorMap mw;
@@ -363,11 +382,11 @@ static int launch_as(const void* weight, ConvStreamArgs a, cudaStream_t stream)
     if (rc) return rc;
     constexpr size_t smem = (size_t)STAGES * (CS_TM + BN) * KC * 2 + 2 * sizeof(ConvIndex<BN>) + 8 * (2 * STAGES + 8) + 16 + 1024;
     static_assert(smem <= 227 * 1024, "shared memory of a CTA");
-    auto kern = conv_stream_kernel<BN, KC, STAGES, NI, GW>;
+    auto kern = conv_stream_kernel<BN, KC, STAGES, NI, GW, SETS, EW>;
     if (allow_smem(kern) != cudaSuccess) return check_launch("ptv3_subm_conv_fwd: shared memory attribute");
     a.tiles = (int)((a.n + CS_TM - 1) / CS_TM) * (a.cout / BN);
     // one CTA per SM (it may take all of tensor memory)
-    launch_dependent(kern, dim3(a.tiles < SMS ? a.tiles : SMS), dim3((cs_epi_warp<GW, NI>() + 4) * 32),
+    launch_dependent(kern, dim3(a.tiles < SMS ? a.tiles : SMS), dim3((cs_epi_warp<GW, NI>() + EW) * 32),
                      smem < 120 * 1024 ? (size_t)120 * 1024 : smem, stream, mw, a);
     count_launches(1);
     return check_launch("ptv3_subm_conv_fwd");
@@ -380,10 +399,10 @@ int launch_conv_stream(const void* feat, const int32_t* nbr, const void* weight,
     const ConvStreamArgs a{(const __nv_bfloat16*)feat, nbr, (const __nv_bfloat16*)bias, (__nv_bfloat16*)out, row_order, n,
                            c_in, c_out, kvol, 0, status};
     switch (bn) {
-    case 32: return launch_as<32, 32, 16, 4, 8>(weight, a, stream);
-    case 64: return launch_as<64, 64, 8, 2, 8>(weight, a, stream);
-    case 128: return launch_as<128, 64, 6, 2, 6>(weight, a, stream);
-    default: return launch_as<256, 64, 4, 1, 4>(weight, a, stream);
+    case 32: return launch_as<32, 32, 16, 4, 8, 2, 4>(weight, a, stream);
+    case 64: return launch_as<64, 64, 8, 2, 8, 2, 4>(weight, a, stream);
+    case 128: return launch_as<128, 64, 6, 2, 6, 2, 4>(weight, a, stream);
+    default: return launch_as<256, 64, 4, 2, 4, 1, 8>(weight, a, stream);
     }
 }
 
