@@ -13,6 +13,7 @@
 // one thread per query row, keys/values staged through shared memory in chunks
 // with a per-chunk running-max rescale, so any sequence length works.
 #include "common.cuh"
+#include "linear.cuh"
 #include "convert.cuh"
 #include "attention_mma.cuh"
 #include "../../include/ptv3_b200.h"
@@ -173,7 +174,7 @@ static int launch_attn_fma(const void* qkv, const int64_t* order, const int64_t*
 static int attention_impl(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad,
                           const int32_t* cu_seqlens, void* out, int64_t n, int n_seq, int max_seqlen,
                           int channels, int heads, float scale, int dtype, int algo, ptv3::RpeArgs rpe,
-                          uint32_t* status, void* stream)
+                          bool planned, uint32_t* status, void* stream)
 {
     using namespace ptv3;
     PTV3_REQUIRE(n >= 0 && n_seq >= 0 && max_seqlen >= 1 && channels >= 1 && heads >= 1 &&
@@ -203,7 +204,7 @@ static int attention_impl(const void* qkv, const int64_t* order, const int64_t* 
                  "16-byte aligned qkv", ATTN_MMA_MAX_SEQLEN);
     if (mma_ok && algo != 1)
         return launch_attn_mma(qkv, order, pad, unpad, cu_seqlens, out, n_seq, max_seqlen, channels,
-                               heads, scale, algo == 3, status, (cudaStream_t)stream);
+                               heads, scale, algo == 3, planned, status, (cudaStream_t)stream);
     if (dtype == PTV3_DTYPE_F32 && algo == 0 && !rpe.grid_coord && channels / heads == 16 &&
         (((uintptr_t)qkv | (uintptr_t)out) & 15) == 0)
         return launch_attn_f32(qkv, order, pad, unpad, cu_seqlens, out, n_seq, max_seqlen, channels, heads, scale, status,
@@ -215,13 +216,21 @@ static int attention_impl(const void* qkv, const int64_t* order, const int64_t* 
                                           channels, heads, scale, rpe, status, (cudaStream_t)stream);
 }
 
+int ptv3::attention_fwd(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad,
+                        const int32_t* cu_seqlens, void* out, int64_t n, int n_seq, int max_seqlen, int channels, int heads,
+                        float scale, int dtype, int algo, bool planned, uint32_t* status, cudaStream_t stream)
+{
+    return attention_impl(qkv, order, pad, unpad, cu_seqlens, out, n, n_seq, max_seqlen, channels, heads, scale, dtype, algo,
+                          RpeArgs{nullptr, nullptr, 0, 0, 0}, planned, status, stream);
+}
+
 extern "C" int ptv3_attention_fwd(const void* qkv, const int64_t* order, const int64_t* pad,
                                   const int64_t* unpad, const int32_t* cu_seqlens, void* out,
                                   int64_t n, int n_seq, int max_seqlen, int channels, int heads,
                                   float scale, int dtype, int algo, uint32_t* status, void* stream)
 {
-    return attention_impl(qkv, order, pad, unpad, cu_seqlens, out, n, n_seq, max_seqlen, channels, heads,
-                          scale, dtype, algo, ptv3::RpeArgs{nullptr, nullptr, 0, 0, 0}, status, stream);
+    return ptv3::attention_fwd(qkv, order, pad, unpad, cu_seqlens, out, n, n_seq, max_seqlen, channels, heads, scale, dtype,
+                               algo, false, status, (cudaStream_t)stream);
 }
 
 extern "C" int ptv3_attention_rpe_fwd(const void* qkv, const int64_t* order, const int64_t* pad,
@@ -236,5 +245,5 @@ extern "C" int ptv3_attention_rpe_fwd(const void* qkv, const int64_t* order, con
                  "ptv3_attention_rpe_fwd: pos_bnd %d outside [0, 64]", pos_bnd);
     return attention_impl(qkv, order, pad, unpad, cu_seqlens, out, n, n_seq, max_seqlen, channels, heads,
                           scale, dtype, 1, RpeArgs{grid_coord, rpe_table, pos_bnd, 2 * pos_bnd + 1, heads},
-                          nullptr, stream);
+                          false, nullptr, stream);
 }

@@ -53,7 +53,8 @@ __device__ __forceinline__ uint32_t scale_bf16x2(uint32_t v, float s)
     return pack_bf16(f.x * s, f.y * s);
 }
 
-template <bool PACKED>
+// PLANNED: the geometry may be read before the wait for the kernel ahead (see linear.cuh)
+template <bool PACKED, bool PLANNED>
 __global__ void __launch_bounds__(AM_THREADS, 3) attn_mma_d16_kernel(
     const __nv_bfloat16* __restrict__ qkv, const int64_t* __restrict__ order,
     const int64_t* __restrict__ pad, const int64_t* __restrict__ unpad,
@@ -61,7 +62,7 @@ __global__ void __launch_bounds__(AM_THREADS, 3) attn_mma_d16_kernel(
     int lpad_max, uint32_t* __restrict__ status)
 {
     pdl_launch_next();
-    pdl_wait();
+    if (!PLANNED) pdl_wait();
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char* Ks = smem;
     unsigned char* Vs = smem + (size_t)lpad_max * 32;
@@ -79,10 +80,14 @@ __global__ void __launch_bounds__(AM_THREADS, 3) attn_mma_d16_kernel(
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t start = cu_seqlens[seq];
     const int L = (int)(cu_seqlens[seq + 1] - start);
-    if (L <= 0) return;
+    if (L <= 0) {
+        pdl_wait();          // (no CTA ends before the kernel ahead has: the one behind relies on it)
+        return;
+    }
     // shared memory was sized from the caller's max_seqlen: a longer sequence (a plan made
     // for a larger patch) is reported and skipped, uniformly over the CTA, before any write
     if (L > lpad_max) {
+        pdl_wait();
         if (tid == 0 && status) atomicOr(status, PTV3_STATUS_BAD_INDEX);
         return;
     }
@@ -91,27 +96,37 @@ __global__ void __launch_bounds__(AM_THREADS, 3) attn_mma_d16_kernel(
     const int tiles_per_slice = (ntiles + n_slices - 1) / n_slices;
     const int tile_lo = slice * tiles_per_slice;
     const int tile_hi = min(ntiles, tile_lo + tiles_per_slice);
-    if (tile_lo >= tile_hi) return;
+    if (tile_lo >= tile_hi) {
+        pdl_wait();
+        return;
+    }
     const int64_t row_stride = 3 * (int64_t)C;
 
-    // ---- gather K and V of the whole sequence ------------------------------
-    // four rows per thread at a time: the chain pad -> order -> row is three dependent loads long
-    for (int rb = tid; rb < Lp; rb += 4 * AM_THREADS) {
-        int64_t pd[4], src[4], own[4];
+    if (PLANNED) {
+        // ---- rows of the sequence: four per thread at a time, a chain of two dependent loads ------------------
+        for (int rb = tid; rb < L; rb += 4 * AM_THREADS) {
+            int64_t pd[4], src[4], own[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) pd[i] = rb + i * AM_THREADS < L ? pad[start + rb + i * AM_THREADS] : -1;
+            for (int i = 0; i < 4; ++i) pd[i] = rb + i * AM_THREADS < L ? pad[start + rb + i * AM_THREADS] : -1;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            src[i] = pd[i] >= 0 ? order[pd[i]] : 0;
-            own[i] = pd[i] >= 0 ? unpad[pd[i]] : 0;
+            for (int i = 0; i < 4; ++i) {
+                src[i] = pd[i] >= 0 ? order[pd[i]] : 0;
+                own[i] = pd[i] >= 0 ? unpad[pd[i]] : 0;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = rb + i * AM_THREADS;
+                if (r < L) src_s[r] = own[i] == start + r ? (int32_t)src[i] : -(int32_t)src[i] - 1;
+            }
         }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int r = rb + i * AM_THREADS;
-            if (r >= Lp) break;
-            if (pd[i] >= 0) {
-                src_s[r] = own[i] == start + r ? (int32_t)src[i] : -(int32_t)src[i] - 1;
-                const __nv_bfloat16* kp = qkv + src[i] * row_stride + C + h * AM_D;
+        // (so far only the geometry was read: planned, that happens beside the kernel before this one in the stream)
+        pdl_wait();
+        // ---- gather K and V of the whole sequence ------------------------------
+#pragma unroll 4
+        for (int r = tid; r < Lp; r += AM_THREADS) {
+            if (r < L) {
+                const int32_t e = src_s[r];          // (this thread's own)
+                const __nv_bfloat16* kp = qkv + (int64_t)(e >= 0 ? e : -(e + 1)) * row_stride + C + h * AM_D;
                 cp_async16(smem_u32(Ks) + kv_offset(r, 0), kp);
                 cp_async16(smem_u32(Ks) + kv_offset(r, 1), kp + 8);
                 cp_async16(smem_u32(Vs) + kv_offset(r, 0), kp + C);
@@ -122,6 +137,38 @@ __global__ void __launch_bounds__(AM_THREADS, 3) attn_mma_d16_kernel(
                 *reinterpret_cast<uint4*>(Ks + kv_offset(r, 1)) = z;
                 *reinterpret_cast<uint4*>(Vs + kv_offset(r, 0)) = z;
                 *reinterpret_cast<uint4*>(Vs + kv_offset(r, 1)) = z;
+            }
+        }
+    } else {
+        // ---- gather K and V of the whole sequence ------------------------------
+        // four rows per thread at a time: the chain pad -> order -> row is three dependent loads long
+        for (int rb = tid; rb < Lp; rb += 4 * AM_THREADS) {
+            int64_t pd[4], src[4], own[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) pd[i] = rb + i * AM_THREADS < L ? pad[start + rb + i * AM_THREADS] : -1;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                src[i] = pd[i] >= 0 ? order[pd[i]] : 0;
+                own[i] = pd[i] >= 0 ? unpad[pd[i]] : 0;
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = rb + i * AM_THREADS;
+                if (r >= Lp) break;
+                if (pd[i] >= 0) {
+                    src_s[r] = own[i] == start + r ? (int32_t)src[i] : -(int32_t)src[i] - 1;
+                    const __nv_bfloat16* kp = qkv + src[i] * row_stride + C + h * AM_D;
+                    cp_async16(smem_u32(Ks) + kv_offset(r, 0), kp);
+                    cp_async16(smem_u32(Ks) + kv_offset(r, 1), kp + 8);
+                    cp_async16(smem_u32(Vs) + kv_offset(r, 0), kp + C);
+                    cp_async16(smem_u32(Vs) + kv_offset(r, 1), kp + C + 8);
+                } else {
+                    const uint4 z = make_uint4(0, 0, 0, 0);
+                    *reinterpret_cast<uint4*>(Ks + kv_offset(r, 0)) = z;
+                    *reinterpret_cast<uint4*>(Ks + kv_offset(r, 1)) = z;
+                    *reinterpret_cast<uint4*>(Vs + kv_offset(r, 0)) = z;
+                    *reinterpret_cast<uint4*>(Vs + kv_offset(r, 1)) = z;
+                }
             }
         }
     }
@@ -366,14 +413,19 @@ bool attn_mma_supported(int channels, int heads, int max_seqlen)
 
 int launch_attn_mma(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad,
                     const int32_t* cu, void* out, int n_seq, int max_seqlen, int C, int H, float scale,
-                    bool packed_exp, uint32_t* status, cudaStream_t stream)
+                    bool packed_exp, bool planned, uint32_t* status, cudaStream_t stream)
 {
     const int lpad = (max_seqlen + AM_KC - 1) / AM_KC * AM_KC;
     const size_t smem = (size_t)lpad * 68;      // K, V and the row numbers
-    auto kern = packed_exp ? attn_mma_d16_kernel<true> : attn_mma_d16_kernel<false>;
+    const AmCut cut = am_cut((int64_t)n_seq * H, max_seqlen, smem);
+    // The look-up ahead of the wait pays where a launch has at most one CTA per SM, all of them at their beginning when the
+    // kernel ahead ends (a pass over 6 000 points 1 550 -> 1 498 us); the two-step gather costs 2 to 3 % of a long one
+    // (400 000 x 64 447 -> 461).
+    const bool ahead = planned && !packed_exp && (int64_t)n_seq * H * cut.slices <= SMS;
+    auto kern = packed_exp ? attn_mma_d16_kernel<true, false> : ahead ? attn_mma_d16_kernel<false, true>
+                                                                       : attn_mma_d16_kernel<false, false>;
     if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_attention_fwd: shared memory attribute");
-    const AmCut cut = am_cut((int64_t)n_seq * H, max_seqlen, smem);
     // (shared memory that only so many CTAs find room for)
     const size_t least = cut.per_sm < 3 ? AM_SM_SMEM / (cut.per_sm + 1) : 0;
     const dim3 grid(H * cut.slices, n_seq);

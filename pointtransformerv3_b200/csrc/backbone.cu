@@ -96,6 +96,7 @@ struct BbLevel {
     int32_t* cu = nullptr;
     const void* feat = nullptr;                             // encoder output (skip connection)
     cudaEvent_t ready = nullptr;                            // kernel map and patch layout are queued
+    bool begun = false;                                     // a kernel of the level is queued behind that event
 };
 
 class Pass {
@@ -432,7 +433,9 @@ int Pass::block(const ptv3_stage_args& st, int j, BbLevel& l, const void* conv_i
     BB_STEP(need_ws(bytes));
     b.workspace = ws_;
     b.workspace_bytes = bytes;
-    BB_STEP(block_fwd(&b, true, main_));
+    // (the first block of the finest level comes straight behind the event of its geometry)
+    BB_STEP(block_fwd(&b, true, l.begun, main_));
+    l.begun = true;
     return take_plan(false);
 }
 
@@ -469,6 +472,7 @@ int Pass::encoder(int s)
                                    main_));
         }
         x = pooled;
+        l.begun = true;
     }
     char* buf[2] = {nullptr, nullptr};
     for (int j = 0; j < st.n_blocks; ++j) {

@@ -145,7 +145,8 @@ int block_f32_supported(int channels, int heads, int hidden)
            hidden >= channels && (d == 8 || d == 16 || d == 32 || d == 64);
 }
 
-int block_fwd(const ptv3_block_args* a, bool settled, cudaStream_t stream)
+// (`planned`: for the convolution; attention is never the first kernel of a level, so `settled` covers its geometry)
+int block_fwd(const ptv3_block_args* a, bool settled, bool planned, cudaStream_t stream)
 {
     PTV3_REQUIRE(a != nullptr, PTV3_ERR_INVALID_ARGUMENT, "ptv3_block_fwd: null argument block");
     const bool f32 = a->dtype == PTV3_DTYPE_F32 && block_f32_supported(a->channels, a->heads, a->hidden) && a->nbr;
@@ -180,8 +181,8 @@ int block_fwd(const ptv3_block_args* a, bool settled, cudaStream_t stream)
                                       a->conv_weight, a->conv_bias, b.x, b.acc32, (size_t)n * C * 8, n, C, C, 27,
                                       dt, stream));
     else
-        STEP(ptv3_subm_conv_fwd(a->conv_in, a->nbr, a->conv_weight, a->conv_bias, b.x, a->row_order, n, C, C, 27,
-                                dt, 0, a->status, stream));
+        STEP(subm_conv_fwd(a->conv_in, a->nbr, a->conv_weight, a->conv_bias, b.x, a->row_order, n, C, C, 27, dt, 0, planned,
+                           a->status, stream));
 
     const bool tc_lin = ptv3_linear_supported(C, C, 1, dt) && ptv3_linear_supported(C, 3 * C, 0, dt);
     if (tc_lin) {
@@ -196,8 +197,8 @@ int block_fwd(const ptv3_block_args* a, bool settled, cudaStream_t stream)
                                     a->n1_eps, b.a, n, C, dt, stream));
         STEP(linear_any(b.a, a->qkv_w, a->qkv_b, nullptr, b.qkv, n, C, 3 * C, 0, settled, a->status, stream));
     }
-    STEP(ptv3_attention_fwd(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.att, n, a->n_seq, a->max_seqlen, C,
-                            a->heads, a->scale, dt, a->attention_algo, a->status, stream));
+    STEP(attention_fwd(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.att, n, a->n_seq, a->max_seqlen, C, a->heads,
+                       a->scale, dt, a->attention_algo, settled, a->status, stream));
     const bool fused_mlp = use_fused_mlp(n, C, a->hidden, dt);
     if (tc_lin) {
         STEP(linear_ln_fwd(b.att, a->proj_w, a->proj_b, b.f1, nullptr, nullptr, 0.f, b.f2, a->n2_w, a->n2_b, a->n2_eps,
@@ -299,7 +300,7 @@ extern "C" size_t ptv3_block_workspace_bytes(const ptv3_block_args* a)
 
 extern "C" int ptv3_block_fwd(const ptv3_block_args* a, void* stream)
 {
-    return block_fwd(a, false, (cudaStream_t)stream);
+    return block_fwd(a, false, false, (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------

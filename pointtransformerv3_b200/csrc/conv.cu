@@ -10,6 +10,7 @@
 #include "common.cuh"
 #include "convert.cuh"
 #include "conv_mma.cuh"
+#include "linear.cuh"
 #include "../../include/ptv3_b200.h"
 
 namespace ptv3 {
@@ -118,12 +119,10 @@ static int launch_conv_fma(const void* feat, const int32_t* nbr, const void* wei
 
 }  // namespace ptv3
 
-extern "C" int ptv3_subm_conv_fwd(const void* feat, const int32_t* nbr, const void* weight,
-                                  const void* bias, void* out, const int64_t* row_order, int64_t n,
-                                  int c_in, int c_out, int kernel_volume, int dtype, int algo,
-                                  uint32_t* status, void* stream)
+int ptv3::subm_conv_fwd(const void* feat, const int32_t* nbr, const void* weight, const void* bias, void* out,
+                        const int64_t* row_order, int64_t n, int c_in, int c_out, int kernel_volume, int dtype, int algo,
+                        bool planned, uint32_t* status, cudaStream_t stream)
 {
-    using namespace ptv3;
     PTV3_REQUIRE(n >= 0 && c_in >= 1 && c_out >= 1 && kernel_volume >= 1, PTV3_ERR_INVALID_ARGUMENT,
                  "ptv3_subm_conv_fwd: bad sizes");
     PTV3_REQUIRE(dtype == PTV3_DTYPE_F32 || dtype == PTV3_DTYPE_BF16, PTV3_ERR_UNSUPPORTED,
@@ -146,14 +145,23 @@ extern "C" int ptv3_subm_conv_fwd(const void* feat, const int32_t* nbr, const vo
                  "64, a status word and 16-byte aligned tensors");
     // automatic choice: tensor memory wherever it can be used (mma.sync with 32 channels: 83 us at 407 000 voxels, 62)
     if (tc_ok && (algo == 3 || algo == 0))
-        return launch_conv_tc05(feat, nbr, weight, bias, out, row_order, n, c_in, c_out, kernel_volume, status,
-                                (cudaStream_t)stream);
+        return launch_conv_tc05(feat, nbr, weight, bias, out, row_order, n, c_in, c_out, kernel_volume, planned, status,
+                                stream);
     if (mma_ok && algo != 1)
         return launch_conv_mma(feat, nbr, weight, bias, out, row_order, n, c_in, c_out, kernel_volume,
-                               (cudaStream_t)stream);
+                               stream);
     if (dtype == PTV3_DTYPE_F32)
         return launch_conv_fma<float>(feat, nbr, weight, bias, out, row_order, n, c_in, c_out,
-                                      kernel_volume, (cudaStream_t)stream);
+                                      kernel_volume, stream);
     return launch_conv_fma<__nv_bfloat16>(feat, nbr, weight, bias, out, row_order, n, c_in, c_out,
-                                          kernel_volume, (cudaStream_t)stream);
+                                          kernel_volume, stream);
+}
+
+extern "C" int ptv3_subm_conv_fwd(const void* feat, const int32_t* nbr, const void* weight,
+                                  const void* bias, void* out, const int64_t* row_order, int64_t n,
+                                  int c_in, int c_out, int kernel_volume, int dtype, int algo,
+                                  uint32_t* status, void* stream)
+{
+    return ptv3::subm_conv_fwd(feat, nbr, weight, bias, out, row_order, n, c_in, c_out, kernel_volume, dtype, algo, false,
+                               status, (cudaStream_t)stream);
 }

@@ -13,18 +13,18 @@ int launch_conv_mma(const void* feat, const int32_t* nbr, const void* weight, co
                     void* out, const int64_t* row_order, int64_t n, int c_in, int c_out,
                     int kernel_volume, cudaStream_t stream);
 
-// tcgen05 form (conv_tc05.cu): same operands, accumulator in tensor memory; `status` receives
+// tcgen05 form (conv_tc05.cu; `planned`: see linear.cuh): same operands, accumulator in tensor memory; `status` receives
 // PTV3_STATUS_WAIT_LIMIT if a device wait runs out.
 bool conv_tc05_supported(int c_in, int c_out, int kernel_volume);
 int launch_conv_tc05(const void* feat, const int32_t* nbr, const void* weight, const void* bias, void* out,
-                     const int64_t* row_order, int64_t n, int c_in, int c_out, int kernel_volume,
+                     const int64_t* row_order, int64_t n, int c_in, int c_out, int kernel_volume, bool planned,
                      uint32_t* status, cudaStream_t stream);
 
 // The same as a persistent kernel (conv_stream.cu), tiles of `bn` output channels: 32 (32 -> 32 channels only), 64, 128
 // or 256
 int launch_conv_stream(const void* feat, const int32_t* nbr, const void* weight, const void* bias, void* out,
                        const int64_t* row_order, int64_t n, int c_in, int c_out, int kernel_volume, int bn,
-                       uint32_t* status, cudaStream_t stream);
+                       bool planned, uint32_t* status, cudaStream_t stream);
 
 // Pair-list form (coarse levels): pairs sorted by kernel offset, 128-pair tiles,
 // atomic fixed-point accumulation into acc (n x c_out 64-bit integers of workspace), then

@@ -51,6 +51,7 @@ struct ConvStreamArgs {
     int64_t n;
     int cin, cout, kvol;
     int tiles;                         // row tiles x column tiles
+    bool planned;                      // see linear.cuh
     uint32_t* status;
 };
 
@@ -118,8 +119,9 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + EW) * 32, 1) conv_str
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    // (only the set-up above runs beside the kernel before this one in the stream)
-    pdl_wait();
+    // the kernel before this one in the stream may still run: the set-up above and, planned, the index warps (which read
+    // nothing but the geometry and the bias) go on beside it
+    if (!a.planned || warp < GW + NI || warp >= GW + NI + 2) pdl_wait();
     bool ok = true;
     int seen = 0;              // stages of the tiles before this one
     const int first = (int)blockIdx.x, step = (int)gridDim.x;
@@ -393,11 +395,11 @@ static int launch_as(const void* weight, ConvStreamArgs a, cudaStream_t stream)
 }
 
 int launch_conv_stream(const void* feat, const int32_t* nbr, const void* weight, const void* bias, void* out,
-                       const int64_t* row_order, int64_t n, int c_in, int c_out, int kvol, int bn, uint32_t* status,
-                       cudaStream_t stream)
+                       const int64_t* row_order, int64_t n, int c_in, int c_out, int kvol, int bn, bool planned,
+                       uint32_t* status, cudaStream_t stream)
 {
     const ConvStreamArgs a{(const __nv_bfloat16*)feat, nbr, (const __nv_bfloat16*)bias, (__nv_bfloat16*)out, row_order, n,
-                           c_in, c_out, kvol, 0, status};
+                           c_in, c_out, kvol, 0, planned, status};
     switch (bn) {
     case 32: return launch_as<32, 32, 16, 4, 8, 2, 4>(weight, a, stream);
     case 64: return launch_as<64, 64, 8, 2, 8, 2, 4>(weight, a, stream);

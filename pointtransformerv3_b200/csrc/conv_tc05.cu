@@ -55,6 +55,7 @@ struct ConvTcArgs {
     const int64_t* row_order;      // voxel of every tile position, or NULL
     int64_t n;
     int cin, cout, kvol;
+    bool planned;                  // see linear.cuh
     uint32_t* status;
 };
 
@@ -137,8 +138,8 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
         // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
         pdl_launch_next();
     }
-    // (only the set-up above runs beside the kernel before this one in the stream)
-    pdl_wait();
+    // (only the set-up above, and planned the look-up below, runs beside the kernel before this one in the stream)
+    if (!a.planned) pdl_wait();
 
     // ---- voxels of this tile, their neighbour rows, the offsets in use -------------------------
     if (tid < CT_TM) {
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
+    if (a.planned) pdl_wait();
     const uint32_t tmem_base = *tmem_slot;
     const int n_act = act[0];
     const int kchunks = a.cin / KC;
@@ -539,8 +541,8 @@ static int conv_stream_width(const ConvTcArgs& a, double stages, double* cost)
 }
 
 int launch_conv_tc05(const void* feat, const int32_t* nbr, const void* weight, const void* bias, void* out,
-                     const int64_t* row_order, int64_t n, int c_in, int c_out, int kvol, uint32_t* status,
-                     cudaStream_t stream)
+                     const int64_t* row_order, int64_t n, int c_in, int c_out, int kvol, bool planned,
+                     uint32_t* status, cudaStream_t stream)
 {
     ConvTcArgs a{};
     a.feat = (const __nv_bfloat16*)feat;
@@ -552,9 +554,11 @@ int launch_conv_tc05(const void* feat, const int32_t* nbr, const void* weight, c
     a.cin = c_in;
     a.cout = c_out;
     a.kvol = kvol;
+    a.planned = planned;
     a.status = status;
     auto stream_form = [&](int bn) {
-        return launch_conv_stream(feat, nbr, weight, bias, out, row_order, n, c_in, c_out, kvol, bn, status, stream);
+        return launch_conv_stream(feat, nbr, weight, bias, out, row_order, n, c_in, c_out, kvol, bn, planned, status,
+                                  stream);
     };
     if (c_in == 32) return stream_form(32);
     const double stages = 0.5 * kvol * (c_in / 64);

@@ -6,6 +6,11 @@
 // the stream is an ordinary launch: it starts when everything before it has finished, and every later kernel
 // starts after it.  An entry point of its own cannot know: its weights may be what the call before it
 // computes, and a distance of several launches does not help, because launches in between let theirs start early too.
+//
+// `planned`: nothing in flight writes the geometry that a convolution or attention reads (neighbours, orders, patch
+// layout).  The kernels then look it up before that wait.  Inside ptv3_backbone_fwd it is made on the planning stream,
+// for whose event the main stream waits before the first kernel of a level; only that kernel, the first one
+// behind the event, must not count on it.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -39,7 +44,14 @@ int mlp_fwd(const void* x, const void* fc1_weight, const void* fc1_bias, const v
             const void* residual, void* out, int64_t n, int channels, int hidden, int dtype, bool settled,
             uint32_t* status, cudaStream_t stream);
 
-int block_fwd(const ptv3_block_args* a, bool settled, cudaStream_t stream);
+int attention_fwd(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad, const int32_t* cu_seqlens,
+                  void* out, int64_t n, int n_seq, int max_seqlen, int channels, int heads, float scale, int dtype,
+                  int algo, bool planned, uint32_t* status, cudaStream_t stream);
+int subm_conv_fwd(const void* feat, const int32_t* nbr, const void* weight, const void* bias, void* out,
+                  const int64_t* row_order, int64_t n, int c_in, int c_out, int kernel_volume, int dtype, int algo,
+                  bool planned, uint32_t* status, cudaStream_t stream);
+
+int block_fwd(const ptv3_block_args* a, bool settled, bool planned, cudaStream_t stream);
 int pool_stage_fwd(const void* x, const void* weight, const void* bias, const float* coord, const int64_t* indices,
                    const int64_t* idx_ptr, int64_t n, int64_t m, int c_in, int c_out, const float* bn_scale,
                    const float* bn_shift, void* out, float* coord_out, int reduce, int dtype, bool settled,
