@@ -303,7 +303,7 @@ int Pass::finest()
     BB_CUDA(cudaStreamWaitEvent(side_, inputs, 0));
     // planning stream: codes, orders, inverses
     int scene_bits = 0;
-    while ((a_.n_scenes >> scene_bits) != 0) ++scene_bits;
+    while (((a_.n_scenes - 1) >> scene_bits) != 0) ++scene_bits;
     const int sig_bits = 3 * a_.depth + scene_bits;
     const size_t sort_bytes = ptv3_argsort_workspace_bytes(a_.k, a_.n, sig_bits);
     char* sort_ws = plan_mem_.take<char>(sort_bytes);

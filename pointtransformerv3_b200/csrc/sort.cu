@@ -20,10 +20,13 @@
 //
 // Bytes per element: 8 (histograms) + 16 per pass + 8 in the last one.  What bounds a pass is a
 // tile's chain of short phases separated by barriers, two tiles per SM, most of each phase scattered accesses to
-// shared memory (its wavefronts 51 % of peak, issue 50 %: neither is full): 33.5 M elements in 280 us against
-// 82 for the bytes (with 12-byte elements, tiles of 4096 and ballots: 470).  The last pass adds 390 us to that
-// for the scattered 8-byte inverses, the rate at which L2 takes single sectors (the same in a kernel of its own).
-// 8.4 M x 4 rows of 37 bits, four passes: 1.65 ms (2.75 before); 100 000 x 4 of 30: 48 us (54).
+// shared memory.  Of the 26 000 cycles of a tile of 8 192 with 512 bins: 1 700 until it has its number, 4 200 its loads,
+// 4 400 counting, 3 500 the scan over warps and digits, 3 900 putting its elements in order, 2 800 the look-back, 4 300
+// writing.  32 M elements take ~185 us a pass against 79 for the bytes (270 with ranks from masks, see below).
+// The last pass adds ~350 us to that for the scattered 8-byte inverses, the rate at which L2 takes single sectors (the
+// same in a kernel of its own; 25 us more without the hint that keeps them there).
+// 8 M x 4 rows: 37 bits 1 548 -> 1 384 us, 36 bits (a single scene has no scene number) 1 383 -> 1 215; 1 M x 4 of 34
+// bits 214 -> 166; 100 000 x 4 of 27 bits 46.  Measured and dropped: CTAs of 256 threads, four to an SM (1 367).
 //
 // Tiles take their number from a counter when they start, so every tile a tile
 // waits for is already running or finished; all the same every wait is bounded
@@ -98,6 +101,14 @@ __device__ __forceinline__ uint64_t os_block_excl_scan(uint64_t v, uint64_t* war
     return base + inc - v;
 }
 
+// a store that L2 keeps rather than what streams past it
+__device__ __forceinline__ void store_kept(int64_t* p, int64_t v)
+{
+    uint64_t policy;
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(policy));
+    asm volatile("st.global.L2::cache_hint.b64 [%0], %1, %2;" ::"l"(p), "l"(v), "l"(policy) : "memory");
+}
+
 // How elements enter and leave a pass: as the caller's codes, as packed words, as keys with their
 // indices beside them, as the final order
 enum { OS_PACKED = 0, OS_WIDE = 1, OS_FINAL = 2 };
@@ -119,10 +130,10 @@ struct OsPass {
 };
 
 // shared memory of a tile's elements (or of the masks that rank them)
-__host__ __device__ constexpr size_t os_element_bytes(int items, int bins, bool wide)
+__host__ __device__ constexpr size_t os_element_bytes(int items, int bins, bool wide, bool masks)
 {
-    const size_t elements = (size_t)OS_THREADS * items * (wide ? 12 : 8), masks = (size_t)OS_WARPS * bins * 4;
-    return elements > masks ? elements : masks;
+    const size_t elements = (size_t)OS_THREADS * items * (wide ? 12 : 8), words = masks ? (size_t)OS_WARPS * bins * 4 : 0;
+    return elements > words ? elements : words;
 }
 
 // One pass over one tile of 512 * ITEMS elements.  Element order inside a tile is warp-major: warp w owns
@@ -136,17 +147,27 @@ __host__ __device__ constexpr size_t os_element_bytes(int items, int bins, bool 
 // first, a tile meets hundreds of tiles in the "counts only" state; that walk then takes longer
 // than everything else and keeps itself long.)
 //
+// Ranks among the equal digits of a warp: the counters that the histogram adds to hand them out (atomicAdd
+// returns the count so far).  That is the order of the elements except among lanes of one instruction with the same digit,
+// whose order of service nobody promises.  But a packed word holds, below the digit, everything that the order among equal
+// digits goes by (the digits done and the index), so the ordered tile is checked against its words and neighbours out
+// of order are exchanged until none is left (32 lanes at most; on this hardware none has been seen).
+// MASKS: sorts that dropped digits on the way (see `wide`) cannot tell; their ranks come from masks of the lanes with
+// the same digit, one shared-memory word per warp and digit, which cost five accesses per element: of the 33 000 cycles
+// of a tile of 8 192 that form spent 11 700 there (8 M x 4 rows of 36 bits: 1 383 us, 1 296 with ranks from the counters).
+//
 // WIDE: keys of 64 bits with indices beside them; else packed words.  OUT: see above.
-template <int OS_ITEMS, bool WIDE, int OUT>
+template <int OS_ITEMS, bool WIDE, int OUT, bool MASKS>
 __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(const OsPass a)
 {
+    static_assert(MASKS || !WIDE, "the check reads packed words");
     extern __shared__ __align__(16) unsigned char os_raw[];
     constexpr int OS_TILE = OS_THREADS * OS_ITEMS;
     const int bins = 1 << a.bits;
     uint32_t* peer_masks = reinterpret_cast<uint32_t*>(os_raw);                  // [OS_WARPS][bins], until ranked
     uint64_t* skeys = reinterpret_cast<uint64_t*>(os_raw);                       // [OS_TILE], then
     int32_t* svals = reinterpret_cast<int32_t*>(skeys + OS_TILE);                // [WIDE ? OS_TILE : 0]
-    uint16_t* whist = reinterpret_cast<uint16_t*>(os_raw + os_element_bytes(OS_ITEMS, bins, WIDE));    // [OS_WARPS][bins]
+    uint16_t* whist = reinterpret_cast<uint16_t*>(os_raw + os_element_bytes(OS_ITEMS, bins, WIDE, MASKS));    // [OS_WARPS][bins]
     uint32_t* local_off = reinterpret_cast<uint32_t*>(whist + OS_WARPS * bins);  // [bins + 1]
     uint32_t* gbase = local_off + bins + 1;                                      // [bins]
     __shared__ uint64_t warp_sums[OS_WARPS];
@@ -162,11 +183,16 @@ __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(const OsPass a)
     }
     // (bins >= 2: the 16-bit counters are cleared and counted in pairs)
     for (int i = threadIdx.x; i < OS_WARPS * bins / 2; i += OS_THREADS) reinterpret_cast<uint32_t*>(whist)[i] = 0;
-    for (int i = threadIdx.x; i < OS_WARPS * bins; i += OS_THREADS) peer_masks[i] = 0;
+    if (MASKS)
+        for (int i = threadIdx.x; i < OS_WARPS * bins; i += OS_THREADS) peer_masks[i] = 0;
     __syncthreads();
     const int tile = (int)tile_s;
     if (tile >= a.ntiles) return;    // cannot happen with a grid of ntiles blocks per row
 
+    // (asked for now, wanted for the scan)
+    uint2 ghist = make_uint2(0u, 0u);
+    if (threadIdx.x * 2 < bins)
+        ghist = reinterpret_cast<const uint2*>(a.hist + ((size_t)row * OS_MAX_PASSES + a.pass) * OS_MAX_BINS)[threadIdx.x];
     const int64_t rbase = (int64_t)row * a.n;
     const int64_t tbase = (int64_t)tile * OS_TILE;
     const int tile_count = (int)min((int64_t)OS_TILE, a.n - tbase);
@@ -177,6 +203,7 @@ __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(const OsPass a)
     // ---- load; count the digits per warp ------------------------------------------------------
     uint64_t key[OS_ITEMS];
     int32_t val[WIDE ? OS_ITEMS : 1];
+    uint16_t pos[OS_ITEMS];              // place in the ordered tile; first the rank inside the warp
     uint16_t* wh = whist + warp * bins;
     {
         const uint64_t* in = a.in + rbase + tbase;
@@ -198,7 +225,8 @@ __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(const OsPass a)
         for (int it = 0; it < OS_ITEMS; ++it) {
             if (wlo + it * 32 < tile_count) {
                 const uint32_t d = (uint32_t)(key[it] >> shift) & mask;
-                atomicAdd(&wh32[d >> 1], (d & 1u) ? 0x10000u : 1u);
+                const uint32_t old = atomicAdd(&wh32[d >> 1], (d & 1u) ? 0x10000u : 1u);
+                pos[it] = (uint16_t)((d & 1u) ? old >> 16 : old);
             }
         }
     }
@@ -214,11 +242,10 @@ __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(const OsPass a)
         const bool mine = threadIdx.x * 2 < bins;
         uint32_t* column = reinterpret_cast<uint32_t*>(whist) + threadIdx.x;
         uint32_t total = 0;            // both digits' counts, at most 8192 each
-        uint2 g = make_uint2(0u, 0u);
+        const uint2 g = ghist;
         if (mine) {
 #pragma unroll
             for (int w = 0; w < OS_WARPS; ++w) total += column[w * (bins >> 1)];
-            g = reinterpret_cast<const uint2*>(a.hist + ((size_t)row * OS_MAX_PASSES + a.pass) * OS_MAX_BINS)[threadIdx.x];
         }
         const uint32_t lo = total & 0xffffu, hi = total >> 16;
         // exclusive prefixes over the digits: of the tile's counts (low word) and of the global
@@ -260,10 +287,9 @@ __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(const OsPass a)
     // of the 32.  The lanes of a digit find each other in a word per digit and warp into which each sets its
     // bit (a ballot per digit bit, the form before, cost 10 ballots and 140 cycles per 32 elements of a scheduler's
     // time; match.any about a thousand); the lowest moves the offset on and clears the word.
-    {
+    if constexpr (MASKS) {
         const uint32_t lt = (1u << lane) - 1u;
         uint32_t* masks = peer_masks + warp * bins;
-        uint16_t pos[OS_ITEMS];
 #pragma unroll
         for (int it = 0; it < OS_ITEMS; ++it) {
             const bool valid = wlo + it * 32 < tile_count;
@@ -282,12 +308,16 @@ __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(const OsPass a)
             __syncwarp();
         }
         __syncthreads();       // the masks make room for the elements
+    } else {
 #pragma unroll
-        for (int it = 0; it < OS_ITEMS; ++it) {
-            if (wlo + it * 32 < tile_count) {
-                skeys[pos[it]] = key[it];
-                if constexpr (WIDE) svals[pos[it]] = val[it];
-            }
+        for (int it = 0; it < OS_ITEMS; ++it)
+            if (wlo + it * 32 < tile_count) pos[it] += wh[(uint32_t)(key[it] >> shift) & mask];
+    }
+#pragma unroll
+    for (int it = 0; it < OS_ITEMS; ++it) {
+        if (wlo + it * 32 < tile_count) {
+            skeys[pos[it]] = key[it];
+            if constexpr (WIDE) svals[pos[it]] = val[it];
         }
     }
     // ---- look back over the earlier tiles: all of this thread's digits at once, and a window of
@@ -358,43 +388,72 @@ __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(const OsPass a)
         if (threadIdx.x == 0 && a.status) atomicOr(a.status, PTV3_STATUS_WAIT_LIMIT);
         return;
     }
-
     // ---- write out: neighbours in shared memory with the same digit are neighbours in global
+    const uint64_t below = (1ull << shift) - 1ull;
+    // whether two neighbours of one digit are out of the order of what lies below it
+    auto wrong = [&](uint64_t x, uint64_t y) { return (((x ^ y) >> shift) & mask) == 0 && (x & below) > (y & below); };
+    auto write = [&] {
+        bool bad = false;
 #pragma unroll 4
-    for (int i = threadIdx.x; i < tile_count; i += OS_THREADS) {
-        const uint64_t kx = skeys[i];
-        const int64_t dst = rbase + (uint32_t)(gbase[(uint32_t)(kx >> shift) & mask] + (uint32_t)i);
-        if constexpr (OUT == OS_FINAL) {
-            const int64_t v = (int64_t)(kx & ((1ull << a.val_bits) - 1ull));
-            __stcs(&a.order[dst], v);       // (streams past the inverses that L2 collects)
-            a.inverse[rbase + v] = dst - rbase;
-        } else if constexpr (WIDE) {
-            const int32_t v = svals[i];
-            if (OUT == OS_WIDE) {
-                a.out[dst] = kx;
-                a.vals_out[dst] = v;
+        for (int i = threadIdx.x; i < tile_count; i += OS_THREADS) {
+            const uint64_t kx = skeys[i];
+            if (!MASKS && i > 0) bad |= wrong(skeys[i - 1], kx);
+            const int64_t dst = rbase + (uint32_t)(gbase[(uint32_t)(kx >> shift) & mask] + (uint32_t)i);
+            if constexpr (OUT == OS_FINAL) {
+                const int64_t v = (int64_t)(kx & ((1ull << a.val_bits) - 1ull));
+                __stcs(&a.order[dst], v);       // (streams past the inverses that L2 collects)
+                store_kept(&a.inverse[rbase + v], dst - rbase);
+            } else if constexpr (WIDE) {
+                const int32_t v = svals[i];
+                if (OUT == OS_WIDE) {
+                    a.out[dst] = kx;
+                    a.vals_out[dst] = v;
+                } else {
+                    // the digits done make room for the index; the later passes find theirs lower by as much
+                    a.out[dst] = ((kx >> (a.shift + a.bits)) << a.val_bits) | (uint64_t)v;
+                }
             } else {
-                // the digits done make room for the index; the later passes find theirs lower by as much
-                a.out[dst] = ((kx >> (a.shift + a.bits)) << a.val_bits) | (uint64_t)v;
+                a.out[dst] = kx;
             }
-        } else {
-            a.out[dst] = kx;
+        }
+        return bad;
+    };
+    bool bad = write();
+    if constexpr (!MASKS) {
+        if (__syncthreads_or(bad)) {            // (nobody reads the output before this kernel has ended)
+            for (int round = 0; round < 64; ++round) {
+                bad = false;
+                for (int odd = 0; odd < 2; ++odd) {
+                    for (int i = 2 * threadIdx.x + 1 + odd; i < tile_count; i += 2 * OS_THREADS) {
+                        const uint64_t x = skeys[i - 1], y = skeys[i];
+                        if (wrong(x, y)) {
+                            skeys[i - 1] = y;
+                            skeys[i] = x;
+                            bad = true;
+                        }
+                    }
+                    __syncthreads();
+                }
+                if (!__syncthreads_or(bad)) break;
+            }
+            write();
         }
     }
 }
 
-static size_t os_pass_smem(int items, int bits, bool wide)
+static size_t os_pass_smem(int items, int bits, bool wide, bool masks)
 {
     const size_t bins = (size_t)1 << bits;
-    return os_element_bytes(items, (int)bins, wide) + OS_WARPS * bins * 2 + (2 * bins + 1) * 4;
+    return os_element_bytes(items, (int)bins, wide, masks) + OS_WARPS * bins * 2 + (2 * bins + 1) * 4;
 }
 
-template <int ITEMS, bool WIDE, int OUT>
+template <int ITEMS, bool WIDE, int OUT, bool MASKS>
 static int os_launch(const OsPass& a, cudaStream_t stream)
 {
-    if (allow_smem(os_pass_kernel<ITEMS, WIDE, OUT>) != cudaSuccess)
+    if (allow_smem(os_pass_kernel<ITEMS, WIDE, OUT, MASKS>) != cudaSuccess)
         return check_launch("ptv3_argsort_inverse: shared memory attribute");
-    os_pass_kernel<ITEMS, WIDE, OUT><<<a.ntiles * a.rows, OS_THREADS, os_pass_smem(ITEMS, a.bits, WIDE), stream>>>(a);
+    os_pass_kernel<ITEMS, WIDE, OUT, MASKS><<<a.ntiles * a.rows, OS_THREADS, os_pass_smem(ITEMS, a.bits, WIDE, MASKS),
+                                              stream>>>(a);
     return check_launch("ptv3_argsort_inverse");
 }
 
@@ -493,10 +552,12 @@ extern "C" int ptv3_argsort_inverse(const int64_t* codes, int k, int64_t n, int 
         a.by_row = last && (int64_t)k * n * 8 > OS_L2_BYTES;
         const bool small = p.items == 8;
         int rc;
-        if (wide && a.pass + 1 < p.wide) rc = (small ? os_launch<8, true, OS_WIDE> : os_launch<16, true, OS_WIDE>)(a, stream);
-        else if (wide) rc = (small ? os_launch<8, true, OS_PACKED> : os_launch<16, true, OS_PACKED>)(a, stream);
-        else if (last) rc = (small ? os_launch<8, false, OS_FINAL> : os_launch<16, false, OS_FINAL>)(a, stream);
-        else rc = (small ? os_launch<8, false, OS_PACKED> : os_launch<16, false, OS_PACKED>)(a, stream);
+        if (wide && a.pass + 1 < p.wide) rc = (small ? os_launch<8, true, OS_WIDE, true> : os_launch<16, true, OS_WIDE, true>)(a, stream);
+        else if (wide) rc = (small ? os_launch<8, true, OS_PACKED, true> : os_launch<16, true, OS_PACKED, true>)(a, stream);
+        else if (p.wide > 0 && last) rc = (small ? os_launch<8, false, OS_FINAL, true> : os_launch<16, false, OS_FINAL, true>)(a, stream);
+        else if (p.wide > 0) rc = (small ? os_launch<8, false, OS_PACKED, true> : os_launch<16, false, OS_PACKED, true>)(a, stream);
+        else if (last) rc = (small ? os_launch<8, false, OS_FINAL, false> : os_launch<16, false, OS_FINAL, false>)(a, stream);
+        else rc = (small ? os_launch<8, false, OS_PACKED, false> : os_launch<16, false, OS_PACKED, false>)(a, stream);
         if (rc != PTV3_OK) return rc;
         a.in = a.out;
         a.vals_in = a.vals_out;

@@ -144,8 +144,8 @@ class Point(AttrDict):
             depth = max(self._bounds()()).bit_length()
         depth = max(int(depth), 1)
         self["serialized_depth"] = depth
-        n_scene_bits = len(self.offset).bit_length()
-        assert depth * 3 + n_scene_bits <= 63
+        assert depth * 3 + len(self.offset).bit_length() <= 63
+        n_scene_bits = (len(self.offset) - 1).bit_length()       # of the largest scene number
         assert depth <= 16
         if shuffle_orders:
             # the reference shuffles the finished rows (model.py:128-132); the rows are independent of

@@ -71,6 +71,25 @@ def test_argsort_sizes_and_ties(n, bits):
         assert (order[r].cpu().numpy() == np.argsort(codes[r].numpy(), kind="stable")).all()
 
 
+@pytest.mark.parametrize("n", [1, 31, 33, 4095, 8193, 20000, 700000])
+@pytest.mark.parametrize("kind", ["one", "two", "runs", "alternating", "random"])
+def test_argsort_equal_digits_in_a_warp(n, kind):
+    """Ranks from the histogram's counters: lanes of one instruction with the same digit in every pass, in some, in
+    none; tiles of both sizes, ragged ends; sorts of one, two and three passes and one whose passes drop digits."""
+    g = torch.Generator().manual_seed(n)
+    i = torch.arange(n)
+    for bits in (1, 9, 20, 30, 52):
+        top = 1 << bits
+        codes = {"one": torch.full((n,), top - 1), "two": torch.where(torch.rand(n, generator=g) < 0.5, 0, top - 1),
+                 "runs": (n - 1 - i) // 7 % top, "alternating": torch.where(i % 2 == 0, top - 1, i % top),
+                 "random": torch.randint(0, top, (n,), generator=g)}[kind].repeat(2, 1)
+        codes[1] = codes[1].flip(0)
+        order, inverse = ops.argsort_inverse(codes.cuda(), bits)
+        ref = torch.sort(codes, dim=1, stable=True).indices
+        assert torch.equal(order.cpu(), ref)
+        assert torch.equal(inverse.cpu().gather(1, ref), i.expand(2, n))
+
+
 @pytest.mark.parametrize("k,n,bits", [(4, 74 * 4096, 30), (4, 74 * 4096 + 1, 30), (1, 8193, 1), (3, 2049, 62),
                                       (2, 300001, 62), (1, 1 << 21, 54)])
 def test_argsort_tile_sizes_and_long_keys(k, n, bits):
