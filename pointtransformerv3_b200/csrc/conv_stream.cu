@@ -146,9 +146,11 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + EW) * 32, 1) conv_str
             if (!__all_sync(0xffffffffu, ok)) break;
             const ConvIndex<BN>& x = index[b];
             const int end = seen + x.act[0] * kchunks, col0 = t % col_tiles * BN;
+            // offset (by its place in the list) and chunk of stage g: counted, not divided, from stage to stage
+            int at = (g - seen) / kchunks, chunk = (g - seen) - at * kchunks;
             for (; g < end; g += GW) {
-                const int o = x.act[1 + (g - seen) / kchunks];
-                const char* src0 = reinterpret_cast<const char*>(a.feat) + (g - seen) % kchunks * ROWB + c * 16;
+                const int o = x.act[1 + at];
+                const char* src0 = reinterpret_cast<const char*>(a.feat) + chunk * ROWB + c * 16;
                 const int32_t* nb = x.nbr + o * CS_TM + rg * 4;
                 const uint32_t sa = sbase + s * STAGE_BYTES;
                 ok &= mbar_wait(empty0 + 8 * s, phase, abort);
@@ -161,14 +163,19 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + EW) * 32, 1) conv_str
                         cp_async16_zfill(sa + j0 * ROWB + dst[j], src0 + (uint64_t)(uint32_t)max(src[j], 0) * pitch, src[j] >= 0);
                 }
                 cp_async_commit();
-                if (lane == 0) {
+                if (elect_one()) {
                     mbar_expect_tx(full0 + 8 * s, B_BYTES);
-                    tma_load_2d(sa + A_BYTES, &map_w, o * a.cin + (g - seen) % kchunks * KC, col0, full0 + 8 * s);
+                    tma_load_2d(sa + A_BYTES, &map_w, o * a.cin + chunk * KC, col0, full0 + 8 * s);
                 }
                 cp_async_wait<0>();
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_one(full0 + 8 * s);
+                chunk += GW;
+                while (chunk >= kchunks) {
+                    chunk -= kchunks;
+                    ++at;
+                }
                 s += GW;
                 if (s >= STAGES) {
                     s -= STAGES;
@@ -201,7 +208,7 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + EW) * 32, 1) conv_str
                 const uint64_t da = da0 + s * (STAGE_BYTES >> 4), db = db0 + s * (STAGE_BYTES >> 4);
                 ok &= mbar_wait(full0 + 8 * s, phase, abort);
                 fence_after_sync();
-                if (lane == 0) {
+                if (elect_one()) {
 #pragma unroll
                     for (int k4 = 0; k4 < KC / 16; ++k4) umma_bf16(acc, da + 2 * k4, db + 2 * k4, idesc, more || k4 > 0);
                     umma_commit(empty0 + 8 * s);
@@ -214,7 +221,7 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + EW) * 32, 1) conv_str
                     phase ^= 1;
                 }
             }
-            if (lane == 0) {
+            if (elect_one()) {
                 if (more) umma_commit(accfull0 + 8 * (i % SETS));
                 else mbar_arrive_one(accfull0 + 8 * (i % SETS));
             }

@@ -211,38 +211,38 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
         // act[it / kchunks], channels of chunk it % kchunks, and (lane 0) the matching slice of W.
         // The warps run independent pipelines, so the fixed cost of a stage (barrier waits, the TMA
         // issue, the proxy fence) and the latency of its copies overlap with the other warps' stages.
-        constexpr int RPP = 32 / NCH;                     // rows per pass of the warp
-        const int c = lane % NCH, rr = lane / NCH;        // this lane's chunk and first row
+        // A lane copies one 16-byte chunk of a row; the lanes of a row take four rows, the next ones the four
+        // after them, so that the numbers of four rows are one load.
+        constexpr int GROUPS = 32 / NCH;                  // rows per instruction
+        const int c = lane % NCH, rg = lane / NCH;
+        uint32_t dst[4];                                  // within a stage's rows, of the four rows
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int r = rg * 4 + j;
+            dst[j] = (uint32_t)(r * ROWB + ((NCH == 8 ? c ^ (r & 7) : c ^ ((r >> 1) & 3)) << 4));
+        }
+        const uint32_t pitch = (uint32_t)stored * 2;
+        // offset (by its place in the list) and chunk of the stage: counted, not divided, from stage to stage
+        int at = (first + warp) / kchunks, chunk = (first + warp) - at * kchunks, s = warp % STAGES, phase = 1;
         for (int it = warp < NGW ? warp : nit; it < nit; it += NGW) {
-            const int s = it % STAGES;
-            if (lane == 0) {
-                if (it >= STAGES) ok &= mbar_wait(empty0 + 8 * s, ((it / STAGES) & 1) ^ 1, abort);
-            }
-            __syncwarp();
-            const int o = act[1 + (first + it) / kchunks];
-            const int chunk = (first + it) % kchunks;
+            const int o = act[1 + at];
             const int kc = F32 ? split_column_a(chunk, a.cin / 6) : chunk * KC;
             const int kw = F32 ? split_column_b(chunk, a.cin / 6) : chunk * KC;
             const uint32_t sa = sbase + s * STAGE_BYTES;
-            const __nv_bfloat16* src0 = a.feat + kc + c * 8;
-            const int32_t* nb = nbr_s + o * CT_TM + rr;
+            const char* src0 = reinterpret_cast<const char*>(a.feat + kc) + c * 16;
+            const int32_t* nb = nbr_s + o * CT_TM + rg * 4;
+            ok &= mbar_wait(empty0 + 8 * s, phase, abort);
 #pragma unroll
-            for (int j0 = 0; j0 < CT_TM / RPP; j0 += 8) {
-                int32_t src[8];
+            for (int j0 = 0; j0 < CT_TM; j0 += GROUPS * 4) {
+                const int4 n4 = *reinterpret_cast<const int4*>(nb + j0);
+                const int src[4] = {n4.x, n4.y, n4.z, n4.w};
 #pragma unroll
-                for (int j = 0; j < 8; ++j) src[j] = nb[(j0 + j) * RPP];
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int r = rr + (j0 + j) * RPP;
-                    const int pc = NCH == 8 ? (c ^ (r & 7)) : (c ^ ((r >> 1) & 3));
-                    cp_async16_zfill(sa + r * ROWB + pc * 16, src0 + (int64_t)(src[j] < 0 ? 0 : src[j]) * stored,
-                                     src[j] >= 0);
-                }
+                for (int j = 0; j < 4; ++j)
+                    cp_async16_zfill(sa + j0 * ROWB + dst[j], src0 + (uint64_t)(uint32_t)max(src[j], 0) * pitch, src[j] >= 0);
             }
             cp_async_commit();
-            // (the weight load is issued after the copies: its issue costs lane 0 ~350 cycles, during
-            // which the rows are already on their way)
-            if (lane == 0) {
+            // (the weight load is issued after the copies, which are already on their way then)
+            if (elect_one()) {
                 mbar_expect_tx(full0 + 8 * s, B_BYTES);
                 tma_load_2d(sa + A_BYTES, &map_w, o * stored + kw, col0, full0 + 8 * s);
             }
@@ -250,6 +250,16 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) mbar_arrive_one(full0 + 8 * s);
+            chunk += NGW;
+            while (chunk >= kchunks) {
+                chunk -= kchunks;
+                ++at;
+            }
+            s += NGW;
+            if (s >= STAGES) {
+                s -= STAGES;
+                phase ^= 1;
+            }
         }
 
         // ---- epilogue: thread = voxel ----------------------------------------------------------
@@ -336,32 +346,55 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
         // its own accumulator.  One thread can start a stage's products only every ~450 cycles (a look
         // at the stage's barrier costs it as much as the four products), which is what bounded the
         // kernel with a single issuer; the partial sums are added in the epilogue.
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(CT_TM, BN);
-            const int me = warp - CT_GATHER_WARPS;
-            const uint32_t tm_acc = tmem_base + me * ACCS * BN;
-            uint32_t used = 0;
-            int lead = 0;          // stages of this issuer with leading products
-            for (int it = me; it < nit; it += NI) {
-                const int s = it % STAGES;
-                ok &= mbar_wait(full0 + 8 * s, (it / STAGES) & 1, abort);
-                fence_after_sync();
-                const uint32_t sa = sbase + s * STAGE_BYTES, sb = sa + A_BYTES;
+        constexpr uint32_t idesc = umma_idesc_bf16(CT_TM, BN);
+        const int me = warp - CT_GATHER_WARPS;
+        const uint32_t tm_acc = tmem_base + me * ACCS * BN;
+        const uint64_t da0 = umma_desc_kmajor(sbase, ROWB), db0 = umma_desc_kmajor(sbase + A_BYTES, ROWB);
+        uint32_t used = 0;
+        int lead = 0;          // stages of this issuer with leading products
+        int s = me, phase = 0, chunk = F32 ? (first + me) % kchunks : 0;
+        for (int it = me; it < nit; it += NI) {
+            ok &= mbar_wait(full0 + 8 * s, phase, abort);
+            fence_after_sync();
+            const uint64_t da = da0 + s * (STAGE_BYTES >> 4), db = db0 + s * (STAGE_BYTES >> 4);
+            // accumulator of a product: the leading ones go round the first three (split_f32.cuh)
+            auto target = [&](int k4) { return F32 ? ((chunk * KC + k4 * 16) * 6 < a.cin ? lead % SPLIT_MAIN : SPLIT_MAIN) : 0; };
+            if (elect_one()) {
+                uint32_t seen = used;
 #pragma unroll
                 for (int k4 = 0; k4 < KC / 16; ++k4) {
-                    uint32_t acc = 0;
-                    if (F32) acc = ((first + it) % kchunks * KC + k4 * 16) * 6 < a.cin ? lead % SPLIT_MAIN : SPLIT_MAIN;
-                    umma_bf16(tm_acc + acc * BN, umma_desc_kmajor(sa + k4 * 32, ROWB), umma_desc_kmajor(sb + k4 * 32, ROWB),
-                              idesc, F32 ? (used >> acc) & 1 : it >= NI || k4 > 0);
-                    used |= 1u << acc;
+                    const uint32_t acc = target(k4);
+                    umma_bf16(tm_acc + acc * BN, da + 2 * k4, db + 2 * k4, idesc, F32 ? (seen >> acc) & 1 : it >= NI || k4 > 0);
+                    seen |= 1u << acc;
                 }
-                if (F32) lead += (first + it) % kchunks * KC * 6 < a.cin;
                 umma_commit(empty0 + 8 * s);
+                if (it + NI >= nit) {
+                    umma_commit(accfull);
+                    if (F32) {
+                        used_s[me] = seen;
+                        mbar_arrive_one(accfull);
+                    }
+                }
             }
-            if (nit > me) umma_commit(accfull);
-            else if (nit > 0) mbar_arrive_one(accfull);
-            if (F32 && nit > 0) {
-                used_s[me] = used;
+            __syncwarp();
+            if (F32) {
+#pragma unroll
+                for (int k4 = 0; k4 < KC / 16; ++k4) used |= 1u << target(k4);
+                lead += chunk * KC * 6 < a.cin;
+                chunk += NI;
+                while (chunk >= kchunks) chunk -= kchunks;
+            }
+            s += NI;
+            if (s >= STAGES) {
+                s -= STAGES;
+                phase ^= 1;
+            }
+        }
+        // an issuer without a stage
+        if (nit > 0 && nit <= me && lane == 0) {
+            mbar_arrive_one(accfull);
+            if (F32) {
+                used_s[me] = 0;
                 mbar_arrive_one(accfull);
             }
         }

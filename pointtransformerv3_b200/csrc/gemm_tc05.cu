@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(64 + gm_epi_warps(MODE) * 32, 1) gemm_tc05_ker
     const uint32_t tmem_base = *tmem_slot;
     bool ok = true;
     if (WRES && !a.settled) pdl_wait();
-    if (WRES && tid == 0) {
+    if (WRES && warp == 0 && elect_one()) {
         // the weights are settled: fetched ahead of the wait below
         int row0, col0;
         tile_at(0, row0, col0);
@@ -139,46 +139,52 @@ __global__ void __launch_bounds__(64 + gm_epi_warps(MODE) * 32, 1) gemm_tc05_ker
 
     if (warp == 0) {
         // ---- producer: K chunks of the x tile and of the W tile, tile after tile -----------------
-        if (lane == 0) {
-            int it = 0, row0, col0;
-            for (int i = 0; tile_at(i, row0, col0); ++i) {
-                for (int kc = 0; kc < nk; ++kc, ++it) {
-                    const int s = it % STAGES;
-                    // a stage is free once the products that read it have completed (the first pass
-                    // over the ring finds every stage free: waiting for the phase before the first)
-                    ok &= mbar_wait(empty0 + 8 * s, ((it / STAGES) & 1) ^ 1, abort);
-                    const uint32_t sa = ring + s * STAGE_BYTES;
+        int s = 0, phase = 1, row0, col0;
+        for (int i = 0; tile_at(i, row0, col0); ++i) {
+            for (int kc = 0; kc < nk; ++kc) {
+                // a stage is free once the products that read it have completed (the first pass
+                // over the ring finds every stage free: waiting for the phase before the first)
+                ok &= mbar_wait(empty0 + 8 * s, phase, abort);
+                const uint32_t sa = ring + s * STAGE_BYTES;
+                if (elect_one()) {
                     mbar_expect_tx(full0 + 8 * s, STAGE_BYTES);
                     tma_load_2d(sa, &map_x, kc * GM_BK, row0, full0 + 8 * s);
                     if (!WRES) tma_load_2d(sa + GM_A_BYTES, &map_w, kc * GM_BK, col0, full0 + 8 * s);
+                }
+                __syncwarp();
+                if (++s == STAGES) {
+                    s = 0;
+                    phase ^= 1;
                 }
             }
         }
     } else if (warp == 1) {
         // ---- issuer -----------------------------------------------------------------------------
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(GM_BM, BN);
-            int it = 0, row0, col0;
-            if (WRES) ok &= mbar_wait(wbar, 0, abort);
-            for (int j = 0; tile_at(j, row0, col0); ++j) {
-                const int buf = j & 1;
-                // the epilogue has read the accumulator's previous tile (first use: free)
-                ok &= mbar_wait(accempty0 + 8 * buf, ((j >> 1) & 1) ^ 1, abort);
+        constexpr uint32_t idesc = umma_idesc_bf16(GM_BM, BN);
+        const uint64_t da0 = umma_desc_kmajor(ring, 128), db0 = umma_desc_kmajor(WRES ? sbase : ring + GM_A_BYTES, 128);
+        int s = 0, phase = 0, row0, col0;
+        if (WRES) ok &= mbar_wait(wbar, 0, abort);
+        for (int j = 0; tile_at(j, row0, col0); ++j) {
+            const int buf = j & 1;
+            // the epilogue has read the accumulator's previous tile (first use: free)
+            ok &= mbar_wait(accempty0 + 8 * buf, ((j >> 1) & 1) ^ 1, abort);
+            fence_after_sync();
+            for (int kc = 0; kc < nk; ++kc) {
+                ok &= mbar_wait(full0 + 8 * s, phase, abort);
                 fence_after_sync();
-                for (int kc = 0; kc < nk; ++kc, ++it) {
-                    const int s = it % STAGES;
-                    ok &= mbar_wait(full0 + 8 * s, (it / STAGES) & 1, abort);
-                    fence_after_sync();
-                    const uint32_t sa = ring + s * STAGE_BYTES, sb = WRES ? sbase + kc * B_BYTES : sa + GM_A_BYTES;
+                const uint64_t da = da0 + s * (STAGE_BYTES >> 4), db = db0 + (WRES ? kc * (B_BYTES >> 4) : s * (STAGE_BYTES >> 4));
+                if (elect_one()) {
 #pragma unroll
-                    for (int k4 = 0; k4 < GM_BK / 16; ++k4) {
-                        const uint64_t da = umma_desc_kmajor(sa + k4 * 32, 128);
-                        const uint64_t db = umma_desc_kmajor(sb + k4 * 32, 128);
-                        umma_bf16(tmem_base + buf * BN, da, db, idesc, kc > 0 || k4 > 0);
-                    }
-                    umma_commit(empty0 + 8 * s);       // the stage may be refilled when these have run
+                    for (int k4 = 0; k4 < GM_BK / 16; ++k4)
+                        umma_bf16(tmem_base + buf * BN, da + 2 * k4, db + 2 * k4, idesc, kc > 0 || k4 > 0);
+                    umma_commit(empty0 + 8 * s);                              // the stage may be refilled when these have run
+                    if (kc == nk - 1) umma_commit(accfull0 + 8 * buf);        // the accumulator is complete
                 }
-                umma_commit(accfull0 + 8 * buf);       // the accumulator is complete
+                __syncwarp();
+                if (++s == STAGES) {
+                    s = 0;
+                    phase ^= 1;
+                }
             }
         }
     } else {
@@ -251,7 +257,7 @@ __global__ void __launch_bounds__(64 + gm_epi_warps(MODE) * 32, 1) gemm_tc05_ker
                 }
                 fence_proxy_async();
                 __syncwarp();
-                if (lane == 0 && row0 + q * 32 < a.n) {
+                if (row0 + q * 32 < a.n && lane == 0) {
                     tma_store_2d(&map_o, col0 + c * GM_OUT_COLS, row0 + q * 32, so);
                     bulk_commit();
                 }

@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
             tma_load_2d(sbase + kc * LS_STAGE + LS_A_BYTES, &map_w, column_w(kc), col0, full0 + 8 * kc);
         }
     };
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
         for (int s = 0; s < stages; ++s) {
             mbar_init(full0 + 8 * s, 1);
             mbar_init(empty0 + 8 * s, 1);
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
     }
     if (!a.settled) {
         pdl_wait();
-        if (tid == 0) weights();
+        if (warp == 0 && elect_one()) weights();
     }
     for (int i = tid; i < LS_BN; i += LS_THREADS) {
         const int c = col0 + i;
@@ -173,27 +173,35 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
     uint4 res[4] = {};
 
     if (warp == 0) {
-        if (lane == 0)
-            for (int kc = 0; kc < nk; ++kc) {
-                const int s = kc % stages;
-                const uint32_t sa = sbase + s * LS_STAGE;
+        // (slots and phases are counted, not divided: a division by `stages` takes longer than the rest of a turn)
+        int s = 0, phase = 1;
+        for (int kc = 0; kc < nk; ++kc) {
+            const uint32_t sa = sbase + s * LS_STAGE;
+            if (kc >= stages) ok &= mbar_wait(empty0 + 8 * s, phase, abort);
+            if (elect_one()) {
                 if (kc >= stages) {
-                    ok &= mbar_wait(empty0 + 8 * s, ((kc / stages) & 1) ^ 1, abort);
                     mbar_expect_tx(full0 + 8 * s, LS_STAGE);
                     tma_load_2d(sa + LS_A_BYTES, &map_w, column_w(kc), col0, full0 + 8 * s);
                 }
                 tma_load_2d(sa, &map_x, column_x(kc), row0, full0 + 8 * s);
             }
-        __syncwarp();
+            __syncwarp();
+            if (++s == stages) {
+                s = 0;
+                phase ^= 1;
+            }
+        }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc_bf16(LS_BM, LS_BN);
-            uint32_t used = 0;
-            for (int kc = 0; kc < nk; ++kc) {
-                const int s = kc % stages;
-                ok &= mbar_wait(full0 + 8 * s, (kc / stages) & 1, abort);
-                fence_after_sync();
-                const uint32_t sa = sbase + s * LS_STAGE, sb = sa + LS_A_BYTES;
+        constexpr uint32_t idesc = umma_idesc_bf16(LS_BM, LS_BN);
+        const uint64_t da0 = umma_desc_kmajor(sbase, 128), db0 = umma_desc_kmajor(sbase + LS_A_BYTES, 128);
+        uint32_t used = 0;
+        int s = 0, phase = 0;
+        for (int kc = 0; kc < nk; ++kc) {
+            ok &= mbar_wait(full0 + 8 * s, phase, abort);
+            fence_after_sync();
+            const uint64_t da = da0 + s * (LS_STAGE >> 4), db = db0 + s * (LS_STAGE >> 4);
+            if (elect_one()) {
+                uint32_t seen = used;
 #pragma unroll
                 for (int k4 = 0; k4 < LS_BK / 16; ++k4) {
                     uint32_t acc = 0;
@@ -201,19 +209,34 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
                         const int step = (k0 + kc * LS_BK) / 16 + k4;      // of 16 columns; the first sixth is the leading piece
                         acc = step * 96 < a.k ? step % SPLIT_MAIN : SPLIT_MAIN;
                     }
-                    umma_bf16(tmem_base + acc * LS_BN, umma_desc_kmajor(sa + k4 * 32, 128),
-                              umma_desc_kmajor(sb + k4 * 32, 128), idesc, (used >> acc) & 1);
-                    used |= 1u << acc;
+                    umma_bf16(tmem_base + acc * LS_BN, da + 2 * k4, db + 2 * k4, idesc, (seen >> acc) & 1);
+                    seen |= 1u << acc;
                 }
-                umma_commit(empty0 + 8 * s);
+                if (kc + stages < nk) umma_commit(empty0 + 8 * s);
+                if (kc == nk - 1) {
+                    umma_commit(accfull);
+                    if (MODE & LS_F32) {
+                        *used_s = seen;
+                        mbar_arrive_one(accfull);
+                    }
+                }
             }
-            umma_commit(accfull);
+            __syncwarp();
+            // (what the elected lane has seen, for every lane)
             if (MODE & LS_F32) {
-                *used_s = used;
-                mbar_arrive_one(accfull);
+#pragma unroll
+                for (int k4 = 0; k4 < LS_BK / 16; ++k4) {
+                    const int step = (k0 + kc * LS_BK) / 16 + k4;
+                    used |= 1u << (step * 96 < a.k ? step % SPLIT_MAIN : SPLIT_MAIN);
+                }
+            } else {
+                used = 1;
+            }
+            if (++s == stages) {
+                s = 0;
+                phase ^= 1;
             }
         }
-        __syncwarp();
     } else {
         if ((MODE & LS_RESIDUAL) && !(MODE & LS_F32) && parts == 1 && live) {
 #pragma unroll

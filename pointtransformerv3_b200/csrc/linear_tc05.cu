@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (tid == 0) {   // weights: once per CTA
+    if (warp == 0 && elect_one()) {   // weights: once per CTA
         mbar_expect_tx(wbar, (uint32_t)(KB * w_block));
         for (int kb = 0; kb < KB; ++kb)
             for (int r = 0; r < n_out; r += a.w_box_rows)
@@ -134,27 +134,34 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
     if (g < a.groups) {
         const int64_t tile_step = (int64_t)gridDim.x * a.groups;
         const int64_t tile0 = (int64_t)g * gridDim.x + blockIdx.x;      // (few tiles: one per SM, not four on one)
+        // both by the group's first warp, one lane of it issuing
+        const bool first_warp = (t >> 5) == 0;
         auto load_x = [&](int64_t tile, int b) {
-            mbar_expect_tx(xbar0 + 8 * b, X_BYTES);
-            for (int kb = 0; kb < KB; ++kb)
-                tma_load_2d(xs0 + b * X_BYTES + kb * X_BLOCK, &map_x, kb * KCOLS, (int)(tile * 128), xbar0 + 8 * b);
-        };
-        // t == 0 only: the product of the x tile in buffer xb into accumulator acc
-        auto issue_mma = [&](int xb, int acc) {
-            const uint32_t xs = xs0 + xb * X_BYTES;
-            fence_after_sync();
-            for (int h = 0; h < n_out; h += n_half) {
-#pragma unroll
-                for (int k = 0; k < K / 16; ++k) {
-                    const int kb = (k * 16) / KCOLS, kk = (k * 16) % KCOLS;
-                    const uint64_t da = umma_desc_kmajor(xs + kb * X_BLOCK + kk * 2, SW);
-                    const uint64_t db = umma_desc_kmajor(sbase + kb * w_block + h * SW + kk * 2, SW);
-                    umma_bf16(tm_acc_mma0 + acc * tm_acc_step + h, da, db, idesc, k > 0);
-                }
+            if (elect_one()) {
+                mbar_expect_tx(xbar0 + 8 * b, X_BYTES);
+                for (int kb = 0; kb < KB; ++kb)
+                    tma_load_2d(xs0 + b * X_BYTES + kb * X_BLOCK, &map_x, kb * KCOLS, (int)(tile * 128), xbar0 + 8 * b);
             }
-            umma_commit(mbar0 + 8 * acc);
+            __syncwarp();
         };
-        if (t == 0 && tile0 < ntiles) {
+        // the product of the x tile in buffer xb into accumulator acc
+        const uint64_t dx0 = umma_desc_kmajor(xs0, SW), dw0 = umma_desc_kmajor(sbase, SW);
+        auto issue_mma = [&](int xb, int acc) {
+            fence_after_sync();
+            if (elect_one()) {
+                for (int h = 0; h < n_out; h += n_half) {
+#pragma unroll
+                    for (int k = 0; k < K / 16; ++k) {
+                        const int kb = (k * 16) / KCOLS, kk = (k * 16) % KCOLS;
+                        umma_bf16(tm_acc_mma0 + acc * tm_acc_step + h, dx0 + ((xb * X_BYTES + kb * X_BLOCK + kk * 2) >> 4),
+                                  dw0 + ((kb * w_block + h * SW + kk * 2) >> 4), idesc, k > 0);
+                    }
+                }
+                umma_commit(mbar0 + 8 * acc);
+            }
+            __syncwarp();
+        };
+        if (first_warp && tile0 < ntiles) {
             load_x(tile0, 0);
             if (nacc == 2) {
                 ok &= mbar_wait(xbar0, xph[0], abort);
@@ -169,7 +176,7 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
             const int buf = j & 1, cur = nacc == 2 ? buf : 0;
             if (nacc == 2) {
                 ok &= mbar_wait(mbar0 + 8 * cur, (j >> 1) & 1, abort);
-                if (t == 0 && tile + tile_step < ntiles) {
+                if (first_warp && tile + tile_step < ntiles) {
                     // the next tile's product into the other accumulator (its epilogue ended with
                     // the barrier that closed the previous tile), then the x tile after that into
                     // the buffer this tile's product has finished with
@@ -181,7 +188,7 @@ __global__ void __launch_bounds__(512, 1) linear_tc05_kernel(const __grid_consta
             } else {
                 ok &= mbar_wait(xbar0 + 8 * buf, xph[buf], abort);
                 xph[buf] ^= 1;
-                if (t == 0) {
+                if (first_warp) {
                     // the other buffer was consumed by the previous tile's MMAs, which have completed:
                     // fetch the next tile into it while this tile is multiplied and written out
                     if (tile + tile_step < ntiles) load_x(tile + tile_step, buf ^ 1);
@@ -353,7 +360,7 @@ __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kern
     __syncthreads();
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    if (tid == 0) {   // weights: once per CTA
+    if (warp == 0 && elect_one()) {   // weights: once per CTA
         mbar_expect_tx(wbar, (uint32_t)(KB * W_BLOCK));
         for (int kb = 0; kb < KB; ++kb) tma_load_2d(sbase + kb * W_BLOCK, &map_w, kb * KCOLS, 0, wbar);
     }
@@ -371,24 +378,32 @@ __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kern
     const int64_t tile0 = (int64_t)g * gridDim.x + blockIdx.x;      // (few tiles: one per SM, not four on one)
     uint32_t xph = 0;
 
-    // t == 0 only: an x tile; its product
+    // by the group's first warp, one lane of it issuing: an x tile; its product
+    const bool first_warp = (t >> 5) == 0;
     auto load_x = [&](int64_t tile) {
-        mbar_expect_tx(xbar, X_BYTES);
-        for (int kb = 0; kb < KB; ++kb) tma_load_2d(xs + kb * X_BLOCK, &map_x, kb * KCOLS, (int)(tile * 128), xbar);
+        if (elect_one()) {
+            mbar_expect_tx(xbar, X_BYTES);
+            for (int kb = 0; kb < KB; ++kb) tma_load_2d(xs + kb * X_BLOCK, &map_x, kb * KCOLS, (int)(tile * 128), xbar);
+        }
+        __syncwarp();
     };
     auto multiply = [&] {
         ok &= mbar_wait(xbar, xph, abort);
         xph ^= 1;
         fence_after_sync();
+        if (elect_one()) {
+            const uint64_t dx = umma_desc_kmajor(xs, SW), dw = umma_desc_kmajor(sbase, SW);
 #pragma unroll
-        for (int k = 0; k < K / 16; ++k) {
-            const int kb = (k * 16) / KCOLS, kk = (k * 16) % KCOLS;
-            umma_bf16(tmem_base + g * K, umma_desc_kmajor(xs + kb * X_BLOCK + kk * 2, SW),
-                      umma_desc_kmajor(sbase + kb * W_BLOCK + kk * 2, SW), umma_idesc_bf16(128, K), k > 0);
+            for (int k = 0; k < K / 16; ++k) {
+                const int kb = (k * 16) / KCOLS, kk = (k * 16) % KCOLS;
+                umma_bf16(tmem_base + g * K, dx + ((kb * X_BLOCK + kk * 2) >> 4), dw + ((kb * W_BLOCK + kk * 2) >> 4),
+                          umma_idesc_bf16(128, K), k > 0);
+            }
+            umma_commit(mbar);
         }
-        umma_commit(mbar);
+        __syncwarp();
     };
-    if (t == 0 && tile0 < ntiles) {
+    if (first_warp && tile0 < ntiles) {
         load_x(tile0);
         multiply();
     }
@@ -405,7 +420,7 @@ __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kern
         }
         ok &= mbar_wait(mbar, j & 1, abort);
         fence_after_sync();
-        if (t == 0 && more) load_x(tile + tile_step);     // (its product is done)
+        if (first_warp && more) load_x(tile + tile_step);     // (its product is done)
         // ---- y = round(acc + bias); sums for its LayerNorm, shifted by the row's first value (no cancellation)
         uint32_t y[K / 2];
         float shift1 = 0.f;
@@ -531,7 +546,7 @@ __global__ void __launch_bounds__(128 * lin_ln_groups(K), 1) linear_ln_tc05_kern
             stage_to_global<VEC, K>(stage, a.norm_out, row0, a.n, sl, t);
             __syncwarp();
         }
-        if (t == 0 && more) multiply();      // (its x tile has long landed)
+        if (first_warp && more) multiply();      // (its x tile has long landed)
     }
     fence_before_sync();
     __syncthreads();

@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
     fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (tid == 0) {   // weights: once per CTA
+    if (warp == 0 && elect_one()) {   // weights: once per CTA
         mbar_expect_tx(wbar, Cfg::W1_BYTES + Cfg::W2_BYTES);
         constexpr int W1_ROWS_PER_BOX = Cfg::HD > 256 ? 256 : Cfg::HD;
         for (int r = 0; r < Cfg::HD; r += W1_ROWS_PER_BOX)
@@ -131,31 +131,29 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
     constexpr uint32_t IDESC2 = umma_idesc_bf16(128, C);
     uint32_t xph = 0, m1ph = 0, m2ph = 0;
 
+    // (by one lane of the group's first warp)
+    const uint64_t dx = umma_desc_kmajor(xs, Cfg::SWX), dw1 = umma_desc_kmajor(sbase + Cfg::OFF_W1, Cfg::SWX);
+    const uint64_t dh = umma_desc_kmajor(hs, 128), dw2 = umma_desc_kmajor(sbase + Cfg::OFF_W2, 128);
     auto issue_gemm1 = [&](int ch) {
 #pragma unroll
-        for (int k = 0; k < C / 16; ++k) {
-            const uint64_t da = umma_desc_kmajor(xs + k * 32, Cfg::SWX);
-            const uint64_t db = umma_desc_kmajor(sbase + Cfg::OFF_W1 + ch * Cfg::HC * Cfg::SWX + k * 32, Cfg::SWX);
-            umma_bf16(tm_d1_mma, da, db, IDESC1, k > 0);
-        }
+        for (int k = 0; k < C / 16; ++k)
+            umma_bf16(tm_d1_mma, dx + 2 * k, dw1 + ch * (Cfg::HC * Cfg::SWX >> 4) + 2 * k, IDESC1, k > 0);
     };
     auto issue_gemm2 = [&](int ch) {
 #pragma unroll
-        for (int kb = 0; kb < Cfg::HC / 64; ++kb) {
+        for (int kb = 0; kb < Cfg::HC / 64; ++kb)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint64_t da = umma_desc_kmajor(hs + kb * Cfg::H_BLOCK + k * 32, 128);
-                const uint64_t db = umma_desc_kmajor(
-                    sbase + Cfg::OFF_W2 + (ch * (Cfg::HC / 64) + kb) * Cfg::W2_BLOCK + k * 32, 128);
-                umma_bf16(tm_d2_mma, da, db, IDESC2, !(ch == 0 && kb == 0 && k == 0));
-            }
-        }
+            for (int k = 0; k < 4; ++k)
+                umma_bf16(tm_d2_mma, dh + kb * (Cfg::H_BLOCK >> 4) + 2 * k,
+                          dw2 + (ch * (Cfg::HC / 64) + kb) * (Cfg::W2_BLOCK >> 4) + 2 * k, IDESC2,
+                          !(ch == 0 && kb == 0 && k == 0));
     };
 
     const int64_t ntiles = (n + 127) / 128;
     const int64_t tile_step = (int64_t)gridDim.x * Cfg::NG;
     const int64_t tile0 = (int64_t)g * gridDim.x + blockIdx.x;      // (few tiles: one per SM, not four on one)
-    if (t == 0 && tile0 < ntiles) {
+    const bool first_warp = (t >> 5) == 0;
+    if (first_warp && tile0 < ntiles && elect_one()) {
         mbar_expect_tx(xbar, Cfg::X_BYTES);
         tma_load_2d(xs, &map_x, 0, (int)(tile0 * 128), xbar);
     }
@@ -163,10 +161,13 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
         const int64_t row0 = tile * 128;
         ok &= mbar_wait(xbar, xph, abort);
         xph ^= 1;
-        if (t == 0) {
+        if (first_warp) {
             fence_after_sync();
-            issue_gemm1(0);
-            umma_commit(m1bar);
+            if (elect_one()) {
+                issue_gemm1(0);
+                umma_commit(m1bar);
+            }
+            __syncwarp();
         }
 #pragma unroll 1
         for (int ch = 0; ch < Cfg::NCH; ++ch) {
@@ -175,9 +176,12 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
             fence_after_sync();
             // the x tile has been consumed once the last first-GEMM is done: fetch the next one
             // while this tile's activation, second GEMM and output are still in progress
-            if (t == 0 && ch == Cfg::NCH - 1 && tile + tile_step < ntiles) {
-                mbar_expect_tx(xbar, Cfg::X_BYTES);
-                tma_load_2d(xs, &map_x, 0, (int)((tile + tile_step) * 128), xbar);
+            if (first_warp && ch == Cfg::NCH - 1 && tile + tile_step < ntiles) {
+                if (elect_one()) {
+                    mbar_expect_tx(xbar, Cfg::X_BYTES);
+                    tma_load_2d(xs, &map_x, 0, (int)((tile + tile_step) * 128), xbar);
+                }
+                __syncwarp();
             }
             // D1 -> + b1 -> GELU -> bf16 -> activation tile (K-major, 128-byte swizzle)
 #pragma unroll 1
@@ -211,15 +215,18 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
             fence_proxy_async();
             fence_before_sync();
             named_barrier(1 + g, 128);
-            if (t == 0) {
+            if (first_warp) {
                 fence_after_sync();
-                issue_gemm2(ch);
-                if (ch + 1 < Cfg::NCH) {
-                    issue_gemm1(ch + 1);
-                    umma_commit(m1bar);
-                } else {
-                    umma_commit(m2bar);
+                if (elect_one()) {
+                    issue_gemm2(ch);
+                    if (ch + 1 < Cfg::NCH) {
+                        issue_gemm1(ch + 1);
+                        umma_commit(m1bar);
+                    } else {
+                        umma_commit(m2bar);
+                    }
                 }
+                __syncwarp();
             }
         }
         ok &= mbar_wait(m2bar, m2ph, abort);
