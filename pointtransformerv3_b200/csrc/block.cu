@@ -33,7 +33,7 @@ static int linear_any(const void* x, const void* w, const void* bias, const void
                       int k, int n_out, int gelu, bool settled, uint32_t* status, cudaStream_t stream)
 {
     // (also the only one to take 64 output columns with GELU or a residual: see use_fused_mlp)
-    if (linear_small_wanted(n, k, n_out))
+    if (linear_small_wanted(n, k, n_out, gelu || residual))
         return launch_linear_small(x, w, bias, residual, out, n, k, n_out, gelu, settled, status, stream);
     if (ptv3_gemm_supported(k, n_out, PTV3_DTYPE_BF16))
         return gemm_fwd(x, w, bias, residual, out, n, k, n_out, gelu, PTV3_DTYPE_BF16, settled, status, stream);
@@ -49,7 +49,7 @@ static int linear_any(const void* x, const void* w, const void* bias, const void
 static bool use_fused_mlp(int64_t n, int channels, int hidden, int dtype)
 {
     return ptv3_mlp_supported(channels, hidden, dtype) &&
-           !(linear_small_wanted(n, channels, hidden) && linear_small_wanted(n, hidden, channels));
+           !(linear_small_wanted(n, channels, hidden, true) && linear_small_wanted(n, hidden, channels, true));
 }
 
 struct BlockBuffers {

@@ -355,7 +355,7 @@ int gemm_fwd(const void* x, const void* weight, const void* bias, const void* re
     PTV3_REQUIRE(x && weight && out && status, PTV3_ERR_INVALID_ARGUMENT, "ptv3_gemm_fwd: null pointer");
     PTV3_REQUIRE((((uintptr_t)x | (uintptr_t)weight | (uintptr_t)out | (uintptr_t)bias | (uintptr_t)residual) & 15) == 0,
                  PTV3_ERR_INVALID_ARGUMENT, "ptv3_gemm_fwd: tensors must be 16-byte aligned");
-    if (linear_small_wanted(n, k, n_out))
+    if (linear_small_wanted(n, k, n_out, gelu || residual))
         return launch_linear_small(x, weight, bias, residual, out, n, k, n_out, gelu, settled, status, stream);
     GemmArgs a{};
     a.bias = (const __nv_bfloat16*)bias;

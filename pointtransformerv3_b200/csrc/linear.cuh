@@ -19,8 +19,9 @@
 
 namespace ptv3 {
 
-// Whether the short form (linear_small.cu) is the faster one for n rows; bf16, 16-byte aligned rows
-bool linear_small_wanted(int64_t n, int k, int n_out);
+// Whether the short form (linear_small.cu) is the faster one for n rows, with GELU or a residual (`epilogue`) or
+// without; bf16, 16-byte aligned rows
+bool linear_small_wanted(int64_t n, int k, int n_out, bool epilogue);
 
 // out = [residual +] act(x W^T + b) by the short form
 int launch_linear_small(const void* x, const void* w, const void* bias, const void* residual, void* out, int64_t n, int k,

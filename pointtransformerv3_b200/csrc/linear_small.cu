@@ -349,17 +349,20 @@ static int ls_parts(int64_t tiles, int k)
 }
 
 // Where the lines lie (us, this kernel against the persistent ones):
-//   K <= 128: three CTAs share an SM: one wave.  1 560 x 64 -> 192: 3.5 / 6.3, 18 900 x 64 -> 192 (3 x 148 tiles):
-//     5.7 / 6.7, 9 400 x 128 -> 384 (444): 6.3 / 7.9; 1 776 tiles lose
-//   K <= 512: 105 x 256 -> 1 024: 4.4 / 5.4, 1 700 x 256 -> 256 (56 tiles): 4.8 / 5.0, -> 768 (168): 5.9 / 5.0
-//   longer K where it can be shared: 27 x 2 048 -> 512: 6.8 / 13.2, 1 000 x 2 048 -> 512 (64): 11.7 / 14.5
-bool linear_small_wanted(int64_t n, int k, int n_out)
+//   K <= 128: three CTAs share an SM: one wave.  1 560 x 64 -> 192: 3.5 / 5.0, 6 760 x 128 -> 512 with GELU (424 tiles)
+//     5.5 / 5.8; 1 776 tiles lose
+//   longer K with GELU or a residual: one wave of one CTA per SM.  105 x 256 -> 1 024: 3.9 / 4.3, 457 x 512 -> 2 048
+//     (128 tiles) 5.3 / 5.7, 6 760 x 512 -> 128 (106) 5.2 / 6.8, 4 000 x 1 024 -> 256 (128) 7.3 / 8.9, 2 200 x 2 048 -> 512
+//     (144) 11.3 / 13.2, 11 400 x 1 024 -> 256 (360) 21.0 / 13.6; shared over K: 27 x 2 048 -> 512 5.6 / 11.0
+//   without: half a wave from K = 512 (800 x 512 -> 512, 56 tiles: 5.0 / 5.1, 457 x 512 -> 1 536, 96: 5.3 / 5.1), a
+//     handful of tiles below (105 x 256 -> 256, 4 tiles: 3.6 / 3.7, -> 768, 12: 3.9 / 3.8, 1 757 x 256 -> 256, 56: 4.4 / 4.0)
+bool linear_small_wanted(int64_t n, int k, int n_out, bool epilogue)
 {
     if (k % LS_BK || k < LS_BK || k > 8192 || n_out % LS_BN) return false;
     const int64_t tiles = (n + LS_BM - 1) / LS_BM * (n_out / LS_BN);
     if (k <= 128) return tiles <= 3 * SMS;
-    if (k < 1024) return tiles <= SMS / 2;
-    return ls_parts(tiles, k) > 1;
+    if (epilogue || k >= 1024) return tiles <= SMS;
+    return tiles <= (k < 512 ? 8 : SMS / 2);
 }
 
 int launch_linear_small(const void* x, const void* w, const void* bias, const void* residual, void* out, int64_t n, int k,

@@ -629,7 +629,7 @@ int linear_fwd(const void* x, const void* weight, const void* bias, void* out, i
     PTV3_REQUIRE(x && weight && out && status, PTV3_ERR_INVALID_ARGUMENT, "ptv3_linear_fwd: null pointer");
     PTV3_REQUIRE((((uintptr_t)x | (uintptr_t)weight | (uintptr_t)out) & 15) == 0, PTV3_ERR_INVALID_ARGUMENT,
                  "ptv3_linear_fwd: tensors must be 16-byte aligned");
-    if (linear_small_wanted(n, k, n_out))
+    if (linear_small_wanted(n, k, n_out, false))
         return launch_linear_small(x, weight, bias, nullptr, out, n, k, n_out, 0, settled, status, stream);
     LinearArgs a{};
     a.bias = (const __nv_bfloat16*)bias;
