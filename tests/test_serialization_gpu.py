@@ -207,6 +207,38 @@ def test_voxelize_in_one_call(sizes, width, dtype):
         assert torch.equal(data[key], full[want["keep"]]), key
 
 
+@pytest.mark.parametrize("sizes", [[2048 * 33 + 1], [2048 * 32, 2048 * 65 - 1, 7], [1] * 4096])
+@pytest.mark.parametrize("kind", ["one voxel", "own voxels", "some"])
+def test_voxelize_in_one_call_many_tiles(sizes, kind):
+    """Look-backs over more than one window of tiles; a table as full as it gets, and every point in one slot;
+    coordinates that are not 16-byte aligned; feature rows wider than a block's share."""
+    import pointtransformerv3_b200 as P
+    from pointtransformerv3_b200 import ops
+    n = sum(sizes)
+    g = torch.Generator().manual_seed(n)
+    row = torch.randperm(n, generator=g)
+    if kind == "one voxel":
+        coord = torch.rand(n, 3, generator=g) * 0.9 + torch.tensor([-7.0, 3.0, 0.0])
+        coord[0] = torch.tensor([-7.0, 3.0, 0.0])
+    else:
+        coord = torch.stack([row % 61, row // 61 % 67, row // (61 * 67)], 1).float() + 0.25
+        if kind == "some":
+            coord = (coord / 3).floor() + torch.rand(n, 3, generator=g) * 0.5
+    coord = torch.cat([torch.zeros(1), coord.flatten()]).cuda()[1:].view(n, 3)
+    assert coord.data_ptr() % 16 != 0 and coord.is_contiguous()
+    feat = torch.randint(0, 255, (n, 1200 if n < 5000 else 5), generator=g).to(torch.uint8).cuda()
+    offset = torch.tensor(sizes).cumsum(0).cuda()
+    data, p2v = P.voxelize(coord, feat, offset, 1.0)
+    grid, _ = ops.grid_coord(coord, 1.0)
+    indices = torch.cat([P.offset2batch(offset, n).unsqueeze(-1).int(), grid], 1).contiguous()
+    want = ops.voxel_dedup(indices, offset)
+    if kind != "some":
+        assert want["m"] == (n if kind == "own voxels" else len(sizes))
+    assert torch.equal(p2v, want["point2voxel"]) and torch.equal(data["offset"], want["offset"])
+    for key, full in (("coord", coord), ("grid_coord", grid), ("feat", feat)):
+        assert torch.equal(data[key], full[want["keep"]]), key
+
+
 @pytest.mark.parametrize("far", [1 << 16, 1 << 31, 1 << 33, (1 << 40) + 5])
 def test_coordinates_beyond_the_code_are_refused(far):
     """64-bit grid coordinates whose low 32 bits look harmless: the depth is taken from their real size."""
