@@ -16,16 +16,17 @@
 // The stages of a tile go round the issuers and every sum is taken in one fixed order, so the result is the same bit
 // for bit on every run.
 //
-// What bounds it (407 000 x 64, 88 us; cycle stamps): the products.  A stage takes 550 to 700 cycles, of which the
-// copies alone would need 250; without any copy it still takes 510.  An instruction of 128 x 64 x 16 or 128 x 128 x 16
-// occupies the tensor pipe for ~125 cycles (its accumulation waits for the one before), 128 x 256 x 16 ~220, and an
-// issuer spends ~1 100 cycles on a stage of four: 370 in a wait that is over already, because the shared-memory pipe is
-// busy with copies, 370 on the instructions, 270 around them.  Measured and dropped: neighbour rows by TMA gather
+// What bounds it (cycle stamps, shared-memory bytes): the shared memory of an SM.  A stage is written once and read
+// once by its products: 48 KB at 64 channels, 64 KB at 128, 96 KB at 256, of which 128 bytes pass in a cycle, so 384
+// of the ~495 cycles that a stage takes, 512 of 544 and 768 of 754.  Products issued by an elected lane of a converged
+// warp take their share of issue out of that (with `lane == 0` in a diverged one an issuer needed 1 100 cycles per stage
+// of four, which was the limit).  Not tried: pairs of CTAs that share the slice of W (cta_group::2), which would move 17,
+// 25 and 33 % fewer bytes.  Measured and dropped: neighbour rows by TMA gather
 // (~11 cycles a row, twice the time), one warp for all weight loads (65 -> 77 us at 32 channels), waits by one
 // elected lane (101 -> 162 us), with a time hint or as a spin (163 to 199), a look at the next stage ahead of the
 // products (equal), copies through L1 (2 to 7 % slower).
-// us here and as one CTA per tile (conv_tc05.cu, 32 channels: conv_mma.cu): 407 000 x 32 62 / 83, x 64 88 / 114,
-// 2 000 000 x 32 332 / 528, x 64 491 / 653, 440 000 x 128 204 / 290, 172 000 x 256 203 / 231, 70 000 x 512 300 / 313.
+// us here and as one CTA per tile (conv_tc05.cu, 32 channels: conv_mma.cu): 407 000 x 32 64 / 83, x 64 88 / 114,
+// 2 000 000 x 32 343 / 528, x 64 492 / 653, 440 000 x 128 198 / 290, 172 000 x 256 195 / 231, 70 000 x 512 288 / 313.
 //
 // Replaces spconv.SubMConv3d.forward at model.py:546-552 for bf16.  Every wait is bounded and reports through the
 // status word.

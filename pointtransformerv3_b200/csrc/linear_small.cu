@@ -2,7 +2,7 @@
 //
 // On a few hundred rows a layer is bound by the length of its own chain, not by any unit: the persistent
 // kernels (gemm_tc05.cu, linear_tc05.cu) give such a layer a handful of CTAs that walk all of K and then
-// spend most of their time in an epilogue of 128 or 256 columns (27 x 2048 -> 512: 15 us on four CTAs).  Here
+// spend most of their time in an epilogue of 128 or 256 columns (27 x 2048 -> 512: 11 us on four CTAs).  Here
 //   * tiles are 64 columns wide, eight warps take 32 columns of a row each;
 //   * the weights of the first chunks are on their way before the preceding kernel has finished (where the
 //     caller vouches for them, see linear.cuh);
