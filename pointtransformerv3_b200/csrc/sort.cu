@@ -25,8 +25,8 @@
 // writing.  32 M elements take ~185 us a pass against 79 for the bytes (270 with ranks from masks, see below).
 // The last pass adds ~350 us to that for the scattered 8-byte inverses, the rate at which L2 takes single sectors (the
 // same in a kernel of its own; 25 us more without the hint that keeps them there).
-// 8 M x 4 rows: 37 bits 1 548 -> 1 384 us, 36 bits (a single scene has no scene number) 1 383 -> 1 215; 1 M x 4 of 34
-// bits 214 -> 166; 100 000 x 4 of 27 bits 46.  Measured and dropped: CTAs of 256 threads, four to an SM (1 367).
+// 8 M x 4 rows: 37 bits 1 548 -> 1 362 us, 36 bits (a single scene has no scene number) 1 383 -> 1 195; 1 M x 4 of 34
+// bits 214 -> 164; 100 000 x 4 of 27 bits 47.  Measured and dropped: CTAs of 256 threads, four to an SM (1 367).
 //
 // Tiles take their number from a counter when they start, so every tile a tile
 // waits for is already running or finished; all the same every wait is bounded
@@ -58,6 +58,9 @@ struct SortPlan {
 };
 
 // Digit histograms of every pass in one read of the keys: hist[row][pass][digit].
+// Four keys of a thread are under way at once: one at a time, a block waited for memory between its shared-memory
+// atomics (8 M x 4 rows, 36 bits: 1 220 -> 1 195 us for the sort; eight keys, or a quarter of the blocks: the same).
+constexpr int OS_HIST_KEYS = 4;
 __global__ void __launch_bounds__(OS_THREADS) os_hist_kernel(const uint64_t* __restrict__ keys, int64_t n,
                                                             int sig_bits, int bits, int passes,
                                                             uint32_t* __restrict__ hist)
@@ -68,11 +71,17 @@ __global__ void __launch_bounds__(OS_THREADS) os_hist_kernel(const uint64_t* __r
     __syncthreads();
     const uint64_t* k = keys + (int64_t)row * n;
     const uint32_t mask = (1u << bits) - 1u;
-    for (int64_t idx = (int64_t)blockIdx.x * OS_THREADS + threadIdx.x; idx < n;
-         idx += (int64_t)gridDim.x * OS_THREADS) {
-        const uint64_t key = k[idx];
-        for (int p = 0; p < passes; ++p)
-            atomicAdd(&os_smem[p * OS_MAX_BINS + ((uint32_t)(key >> (p * bits)) & mask)], 1u);
+    const int64_t stride = (int64_t)gridDim.x * OS_THREADS;
+    for (int64_t idx = (int64_t)blockIdx.x * OS_THREADS + threadIdx.x; idx < n; idx += OS_HIST_KEYS * stride) {
+        uint64_t key[OS_HIST_KEYS];
+#pragma unroll
+        for (int q = 0; q < OS_HIST_KEYS; ++q) key[q] = idx + q * stride < n ? k[idx + q * stride] : 0;
+#pragma unroll
+        for (int q = 0; q < OS_HIST_KEYS; ++q) {
+            if (idx + q * stride >= n) break;
+            for (int p = 0; p < passes; ++p)
+                atomicAdd(&os_smem[p * OS_MAX_BINS + ((uint32_t)(key[q] >> (p * bits)) & mask)], 1u);
+        }
     }
     __syncthreads();
     uint32_t* out = hist + (size_t)row * OS_MAX_PASSES * OS_MAX_BINS;
