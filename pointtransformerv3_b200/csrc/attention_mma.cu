@@ -56,10 +56,8 @@ __device__ __forceinline__ uint32_t scale_bf16x2(uint32_t v, float s)
 // PLANNED: the geometry may be read before the wait for the kernel ahead (see linear.cuh)
 template <bool PACKED, bool PLANNED>
 __global__ void __launch_bounds__(AM_THREADS, 3) attn_mma_d16_kernel(
-    const __nv_bfloat16* __restrict__ qkv, const int64_t* __restrict__ order,
-    const int64_t* __restrict__ pad, const int64_t* __restrict__ unpad,
-    const int32_t* __restrict__ cu_seqlens, __nv_bfloat16* __restrict__ out, int C, float scale,
-    int lpad_max, uint32_t* __restrict__ status)
+    const __nv_bfloat16* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad, const int32_t* cu_seqlens,
+    __nv_bfloat16* out, int C, float scale, int lpad_max, uint32_t* status)
 {
     pdl_launch_next();
     if (!PLANNED) pdl_wait();

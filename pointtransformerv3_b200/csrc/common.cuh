@@ -56,6 +56,12 @@ static inline int ceil_div(int64_t a, int64_t b) { return static_cast<int>((a + 
 // such kernels here call it first thing), and pdl_launch_next() tells the scheduler that the
 // kernel after it may be brought up.  The launch latency and the start-up of a kernel then overlap
 // the tail of its predecessor.
+//
+// Such a kernel takes plain pointers: the memory clobber of the wait holds back loads through those.  A load through
+// const __restrict__ or by __ldg says that nobody writes there while the kernel runs; it may be moved ahead of the
+// wait, and takes the path that is not kept coherent with the kernel ahead.  (Voxelisation read slots before they were
+// written that way, an illegal address.)  What the compiler then no longer moves by itself stands early in the source:
+// the MLP's residual rows, for one (400 000 x 64: 74 us; 91 where they were asked for as they were stored).
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -54,10 +54,8 @@ struct PairList {
 
 template <int CM_TM, int CN, int KC, int WM, int WN, bool PAIRS>
 __global__ void __launch_bounds__(WM * WN * 32) conv_mma_kernel(
-    const __nv_bfloat16* __restrict__ feat, const int32_t* __restrict__ nbr,
-    const __nv_bfloat16* __restrict__ weight, const __nv_bfloat16* __restrict__ bias,
-    __nv_bfloat16* __restrict__ out, const int64_t* __restrict__ row_order, int64_t n, int cin,
-    int cout, int kvol, PairList pl)
+    const __nv_bfloat16* feat, const int32_t* nbr, const __nv_bfloat16* weight, const __nv_bfloat16* bias,
+    __nv_bfloat16* out, const int64_t* row_order, int64_t n, int cin, int cout, int kvol, PairList pl)
 {
     pdl_launch_next();
     pdl_wait();
@@ -117,7 +115,7 @@ __global__ void __launch_bounds__(WM * WN * 32) conv_mma_kernel(
 #pragma unroll
                 for (int i = 0; i < RPL; ++i) {
                     const int r = lane + 32 * i;
-                    v[j][i] = (o < kvol && row0 + r < n) ? __ldg(nbr + (int64_t)o * n + row0 + r) : -1;
+                    v[j][i] = (o < kvol && row0 + r < n) ? nbr[(int64_t)o * n + row0 + r] : -1;
                 }
             }
 #pragma unroll

@@ -244,7 +244,7 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + EW) * 32, 1) conv_str
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const int64_t r = row0 + lane + 32 * e;
-                    v[j][e] = o < a.kvol && r < a.n ? __ldg(a.nbr + (int64_t)o * a.n + r) : -1;
+                    v[j][e] = o < a.kvol && r < a.n ? a.nbr[(int64_t)o * a.n + r] : -1;
                 }
             }
             int32_t row[2];

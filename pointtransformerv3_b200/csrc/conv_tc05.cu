@@ -163,7 +163,7 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int r = lane + 32 * i;
-                v[j][i] = (o < kvol && row0 + r < a.n) ? __ldg(a.nbr + (int64_t)o * a.n + row0 + r) : -1;
+                v[j][i] = (o < kvol && row0 + r < a.n) ? a.nbr[(int64_t)o * a.n + row0 + r] : -1;
             }
         }
 #pragma unroll

@@ -58,9 +58,8 @@ __device__ __forceinline__ float bf16_round(float v) { return __bfloat162float(_
 template <int C>
 __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
     const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w1,
-    const __grid_constant__ CUtensorMap map_w2, const __nv_bfloat16* __restrict__ b1,
-    const __nv_bfloat16* __restrict__ b2, const __nv_bfloat16* __restrict__ residual,
-    __nv_bfloat16* __restrict__ out, int64_t n, bool settled, uint32_t* __restrict__ status)
+    const __grid_constant__ CUtensorMap map_w2, const __nv_bfloat16* b1, const __nv_bfloat16* b2,
+    const __nv_bfloat16* residual, __nv_bfloat16* out, int64_t n, bool settled, uint32_t* status)
 {
     using Cfg = MlpCfg<C>;
     extern __shared__ unsigned char smem_raw[];
@@ -229,19 +228,25 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
                 __syncwarp();
             }
         }
+        // the residual rows are asked for while the second GEMM runs, all at once
+        constexpr int PIECES = C / 8;   // 16-byte pieces per row
+        uint4 res[PIECES];
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) {
+            const int idx = i * 128 + t, r = idx / PIECES, c = idx % PIECES;
+            res[i] = make_uint4(0, 0, 0, 0);
+            if (row0 + r < n) res[i] = *reinterpret_cast<const uint4*>(residual + (row0 + r) * C + c * 8);
+        }
         ok &= mbar_wait(m2bar, m2ph, abort);
         m2ph ^= 1;
         fence_after_sync();
         // D2 -> + b2 -> + residual -> out.  The activation tile is free now and serves as a
         // staging tile (same 128-byte-pitch swizzle): the residual comes in and the result goes
         // out with coalesced 16-byte pieces, the row-per-thread arithmetic runs on shared memory.
-        constexpr int PIECES = C / 8;   // 16-byte pieces per row
 #pragma unroll
         for (int i = 0; i < PIECES; ++i) {
             const int idx = i * 128 + t, r = idx / PIECES, c = idx % PIECES;
-            uint4 v = make_uint4(0, 0, 0, 0);
-            if (row0 + r < n) v = *reinterpret_cast<const uint4*>(residual + (row0 + r) * C + c * 8);
-            *reinterpret_cast<uint4*>(hs_ptr + r * 128 + ((c ^ (r & 7)) << 4)) = v;
+            *reinterpret_cast<uint4*>(hs_ptr + r * 128 + ((c ^ (r & 7)) << 4)) = res[i];
         }
         named_barrier(1 + g, 128);
 #pragma unroll 1
@@ -275,9 +280,12 @@ __global__ void __launch_bounds__(128 * MlpCfg<C>::NG, 1) mlp_tc05_kernel(
 #pragma unroll
         for (int i = 0; i < PIECES; ++i) {
             const int idx = i * 128 + t, r = idx / PIECES, c = idx % PIECES;
-            if (row0 + r < n)
-                *reinterpret_cast<uint4*>(out + (row0 + r) * C + c * 8) =
-                    *reinterpret_cast<const uint4*>(hs_ptr + r * 128 + ((c ^ (r & 7)) << 4));
+            res[i] = *reinterpret_cast<const uint4*>(hs_ptr + r * 128 + ((c ^ (r & 7)) << 4));
+        }
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) {
+            const int idx = i * 128 + t, r = idx / PIECES, c = idx % PIECES;
+            if (row0 + r < n) *reinterpret_cast<uint4*>(out + (row0 + r) * C + c * 8) = res[i];
         }
         fence_before_sync();
         named_barrier(1 + g, 128);

@@ -29,9 +29,8 @@ __device__ __forceinline__ float group_sum(float v)
 // LANES lanes own a row; each lane holds VPL vectors (VPL * Vec<T>::N channels)
 template <typename T, int LANES, int VPL>
 __global__ void __launch_bounds__(256) add_ln_kernel(
-    const T* __restrict__ x, const T* __restrict__ residual, const T* __restrict__ g1,
-    const T* __restrict__ b1, float eps1, T* __restrict__ sum_out, const T* __restrict__ g2,
-    const T* __restrict__ b2, float eps2, T* __restrict__ norm_out, int64_t n, int C)
+    const T* x, const T* residual, const T* g1, const T* b1, float eps1, T* sum_out, const T* g2, const T* b2,
+    float eps2, T* norm_out, int64_t n, int C)
 {
     pdl_launch_next();
     pdl_wait();

@@ -32,12 +32,9 @@ __device__ __forceinline__ float gelu_for(float x)
 // lanes of a group also average the coordinates.  C must be a multiple of Vec<T>::N.
 // REDUCE: 0 max, 1 min, 2 sum, 3 mean (torch_scatter.segment_csr's reduce argument)
 template <typename T, int LANES, int REDUCE>
-__global__ void __launch_bounds__(256, 4) pool_max_kernel(const T* __restrict__ x, const float* __restrict__ coord,
-                                                       const int64_t* __restrict__ indices,
-                                                       const int64_t* __restrict__ idx_ptr, int64_t m, int C,
-                                                       const float* __restrict__ scale,
-                                                       const float* __restrict__ shift, T* __restrict__ out,
-                                                       float* __restrict__ coord_out)
+__global__ void __launch_bounds__(256, 4) pool_max_kernel(const T* x, const float* coord, const int64_t* indices,
+                                                       const int64_t* idx_ptr, int64_t m, int C, const float* scale,
+                                                       const float* shift, T* out, float* coord_out)
 {
     pdl_launch_next();
     pdl_wait();
@@ -96,14 +93,9 @@ __global__ void __launch_bounds__(256, 4) pool_max_kernel(const T* __restrict__ 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) unpool_kernel(const T* __restrict__ skip,
-                                                     const T* __restrict__ child,
-                                                     const int64_t* __restrict__ cluster, int64_t n,
-                                                     int C, const float* __restrict__ s_scale,
-                                                     const float* __restrict__ s_shift,
-                                                     const float* __restrict__ c_scale,
-                                                     const float* __restrict__ c_shift,
-                                                     T* __restrict__ out, T* __restrict__ skip_act)
+__global__ void __launch_bounds__(256) unpool_kernel(const T* skip, const T* child, const int64_t* cluster,
+                                                     int64_t n, int C, const float* s_scale, const float* s_shift,
+                                                     const float* c_scale, const float* c_shift, T* out, T* skip_act)
 {
     pdl_launch_next();
     pdl_wait();

@@ -4,8 +4,7 @@
 namespace ptv3 {
 
 // rows of features: a thread splits eight columns; bandwidth bound: 4 bytes in, 6 out
-__global__ void __launch_bounds__(256) split_f32_kernel(const float* __restrict__ x, int64_t n8, int k,
-                                                        __nv_bfloat16* __restrict__ out)
+__global__ void __launch_bounds__(256) split_f32_kernel(const float* x, int64_t n8, int k, __nv_bfloat16* out)
 {
     pdl_launch_next();
     pdl_wait();

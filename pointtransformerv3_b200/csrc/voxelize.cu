@@ -156,8 +156,7 @@ constexpr int VZ_TILE_ITEMS = 16, VZ_TILE = 256 * VZ_TILE_ITEMS;     // points o
 constexpr int VZ_WORDS = VZ_TILE / 32, VZ_GROUP = 256;
 constexpr int VZ_COUNTERS = 64;                                      // of claimed slots, a sector each
 
-// Loads of what an earlier kernel of the chain makes.  They have to stay behind pdl_wait(): one through a
-// const __restrict__ pointer may be moved ahead of it, since nothing in this kernel writes there.
+// Loads of what an earlier kernel of the chain makes: in their place behind pdl_wait() (see common.cuh).
 __device__ __forceinline__ uint32_t vz_made(const uint32_t* p)
 {
     uint32_t v;
@@ -186,9 +185,8 @@ __global__ void vz_origin_init_kernel(float* origin)
 // Clears the table and the tile words (`clear` 16-byte pieces) and takes the minimum over the points, four
 // points (three 16-byte loads) per step, one atomic per block and axis.  One kernel: the stores go to L2
 // while the coordinates come from memory (2.4 M points: one launch of 14 us, apart 11 and 8 us and a gap).
-__global__ void __launch_bounds__(256) vz_prepare_kernel(const float* __restrict__ coord, int64_t n, bool vec,
-                                                         float* __restrict__ origin, uint4* __restrict__ table,
-                                                         int64_t clear)
+__global__ void __launch_bounds__(256) vz_prepare_kernel(const float* coord, int64_t n, bool vec, float* origin,
+                                                         uint4* table, int64_t clear)
 {
     pdl_launch_next();
     const float inf = __int_as_float(0x7f800000);
@@ -247,8 +245,8 @@ __device__ __forceinline__ void vz_look(const VoxelSlot* pair, unsigned long lon
 // slot counts as one): the number of voxels is known when this kernel ends.
 // One point per thread: with two or four the looks of more points pass before their voxels' first claims (38,
 // 42 and 49 us at 2.4 M points).
-__global__ void __launch_bounds__(256) vz_insert_kernel(const float* __restrict__ coord, int64_t n, float grid_size,
-                                                        const float* origin, const int64_t* __restrict__ offset,
+__global__ void __launch_bounds__(256) vz_insert_kernel(const float* coord, int64_t n, float grid_size,
+                                                        const float* origin, const int64_t* offset,
                                                         int B, VoxelSlot* table, uint32_t pairs,
                                                         uint32_t* slot_of, uint32_t* claimed, uint32_t* status)
 {
@@ -424,8 +422,8 @@ __global__ void __launch_bounds__(256) vz_number_kernel(const uint32_t* slot_of,
 
 // every point's voxel number from its slot, and the scenes' ends among the kept points
 __global__ void __launch_bounds__(256) vz_inverse_kernel(const uint32_t* slot_of, int64_t n, const VoxelSlot* table,
-                                                         uint32_t slots, const int64_t* __restrict__ offset,
-                                                         int n_scenes, const int64_t* count, int64_t* point2voxel,
+                                                         uint32_t slots, const int64_t* offset, int n_scenes,
+                                                         const int64_t* count, int64_t* point2voxel,
                                                          int64_t* new_offset)
 {
     pdl_launch_next();
@@ -458,11 +456,10 @@ __global__ void __launch_bounds__(256) vz_inverse_kernel(const uint32_t* slot_of
 // feature bytes: 21 us with one piece per thread, a 64-bit division and a load of its source row each).
 constexpr int VZ_ROWS = 128, VZ_PIECES = 1024;
 template <typename W>
-__global__ void __launch_bounds__(256) vz_gather_kernel(const int64_t* keep, int64_t m, const float* __restrict__ coord,
-                                                        const float* origin, float grid_size,
-                                                        const W* __restrict__ feat, uint32_t words, int block_rows,
-                                                        float* __restrict__ out_coord, int32_t* __restrict__ out_grid,
-                                                        W* __restrict__ out_feat)
+__global__ void __launch_bounds__(256) vz_gather_kernel(const int64_t* keep, int64_t m, const float* coord,
+                                                        const float* origin, float grid_size, const W* feat,
+                                                        uint32_t words, int block_rows, float* out_coord,
+                                                        int32_t* out_grid, W* out_feat)
 {
     __shared__ int64_t source[VZ_ROWS];
     pdl_launch_next();
