@@ -321,6 +321,8 @@ int ptv3_subm_conv_direct_fwd(const void* feat, const int32_t* indices, const vo
  *               are written packed, k x m with row stride m, at the start of
  *               their k x n buffers, so that a view of the first k * m
  *               elements is the contiguous result
+ *   batch       n int64 below n_scenes; a cluster with another number is counted for no
+ *               scene and sets PTV3_STATUS_BAD_INDEX
  *   meta        1 + n_scenes int64: m, then the number of clusters per scene
  *   meta_host   NULL, or 3 + n_scenes int64 of page-locked HOST memory that the
  *               device can address (cudaHostAlloc / a pinned torch tensor): the last

@@ -102,6 +102,8 @@ struct ClusterSink {
     int64_t* pbatch;        // cap
     const uint32_t* total;  // number of clusters (written by the scan of the tile sums)
     unsigned long long* scene_count;  // B
+    int B;
+    uint32_t* status;
     __device__ void operator()(int, int64_t j, uint32_t pos, bool f) const
     {
         const int64_t p = order0[j];
@@ -120,8 +122,12 @@ struct ClusterSink {
             // one atomic per scene and warp instead of one per cluster: the lanes that reached
             // this point with the same scene elect a leader (clusters of a warp mostly share it)
             const unsigned peers = __match_any_sync(__activemask(), (unsigned long long)b);
-            if ((int)(threadIdx.x & 31) == __ffs(peers) - 1)
-                atomicAdd(&scene_count[b], (unsigned long long)__popc(peers));
+            if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) {
+                if ((unsigned long long)b < (unsigned long long)B)
+                    atomicAdd(&scene_count[b], (unsigned long long)__popc(peers));
+                else       // a number that the offsets know nothing of: it has no counter
+                    atomicOr(status, PTV3_STATUS_BAD_INDEX);
+            }
         }
     }
 };
@@ -401,7 +407,7 @@ int ptv3::pool_plan(const int64_t* code, const int64_t* order, const int32_t* gr
     // clusters along row 0 of the caller's (already shuffled) rows
     ClusterFlag cf{code, order, shift};
     ClusterSink cs{code, order, grid_coord, batch, n, k, shift, pooling_depth, perm, cluster, idx_ptr,
-                   head, pooled_code, pooled_grid_coord, pooled_batch, totals, scene_count};
+                   head, pooled_code, pooled_grid_coord, pooled_batch, totals, scene_count, n_scenes, status};
     scan_tile_sums_kernel<<<dim3(w.ntiles, 1), SC_THREADS, 0, stream>>>(cf, n, w.ntiles, tile_sums);
     scan_sums_kernel<<<1, SC_THREADS, 0, stream>>>(tile_sums, w.ntiles, totals);
     scan_apply_kernel<<<dim3(w.ntiles, 1), SC_THREADS, 0, stream>>>(cf, cs, n, w.ntiles, tile_sums);

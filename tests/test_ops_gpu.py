@@ -169,6 +169,17 @@ def test_pool_plan_matches_oracle(sizes, perm):
         code, order, depth, grid, b = ref["code"], ref["order"], ref["depth"], rg, rb
 
 
+@pytest.mark.parametrize("number", [2, 33, 1 << 40, -1])
+def test_pool_plan_reports_a_scene_number_without_a_scene(number):
+    """Clusters are counted per scene: a number outside the scenes has no counter and is reported."""
+    data = small_batch([700, 300], 3)
+    batch = O.offset_to_batch(data["offset"])
+    code, order, _, _ = O.serialization(data["grid_coord"], batch, ORDERS)
+    wrong = torch.where(batch == 1, number, batch)
+    with pytest.raises(_lib.Ptv3Error, match="status 0x1"):
+        ops.pool_plan(code.cuda(), order.cuda(), data["grid_coord"].cuda(), wrong.cuda(), 2, 1)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_pool_and_unpool_features(dtype):
     data = small_batch([4000, 1000], 4)
