@@ -670,6 +670,14 @@ int ptv3_backbone_fwd(const ptv3_backbone_args* args);
 int ptv3_batch_stats(const int32_t* grid_coord, int64_t n, const int64_t* offset, int n_scenes,
                      int64_t* out_host, void* scratch, void* stream);
 
+/*
+ * The same with the largest scene number of `batch` (n int64; as 32 bits, larger ones are INT32_MAX), which says
+ * how many bits its codes have: out_host = {max x, max y, max z, max batch, offset[0 .. n_scenes), 1}; scratch: 20
+ * bytes.
+ */
+int ptv3_scene_stats(const int32_t* grid_coord, const int64_t* batch, int64_t n, const int64_t* offset, int n_scenes,
+                     int64_t* out_host, void* scratch, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -141,6 +141,7 @@ SIGNATURES = {
     "ptv3_block_fwd": (c_int, [ctypes.POINTER(BlockArgs), c_ptr]),
     "ptv3_backbone_fwd": (c_int, [ctypes.POINTER(BackboneArgs)]),
     "ptv3_batch_stats": (c_int, [c_ptr, c_i64, c_ptr, c_int, c_ptr, c_ptr, c_ptr]),
+    "ptv3_scene_stats": (c_int, [c_ptr, c_ptr, c_i64, c_ptr, c_int, c_ptr, c_ptr, c_ptr]),
     "ptv3_unpool_fwd": (c_int, [c_ptr, c_ptr, c_ptr, c_i64, c_int, c_ptr, c_ptr, c_ptr, c_ptr, c_ptr,
                                 c_ptr, c_int, c_ptr]),
 }

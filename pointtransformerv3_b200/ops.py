@@ -352,24 +352,36 @@ def pool_plan(code, order, grid_coord, batch, n_scenes, pooling_depth, row_perm=
 
 class BatchStats:
     """Launches the kernel that stores a batch's bounds in mapped host memory; ``result`` waits for
-    it, so that the host can work in between.  One at a time per host thread and stream."""
+    it, so that the host can work in between.  With ``batch`` its largest scene number is among them.  One at a time
+    per host thread and stream."""
 
-    def __init__(self, grid_coord, offset):
-        _lib.require_cuda(grid_coord, offset)
+    def __init__(self, grid_coord, offset, batch=None):
+        _lib.require_cuda(grid_coord, offset, batch)
         self.lib, self.stream = _lib.load(), _lib.stream()
         if grid_coord.dtype == torch.int64:        # beyond 32 bits: the bounds still say that it is too much
             grid_coord = grid_coord.clamp(-2 ** 31, 2 ** 31 - 1)
         grid_coord = grid_coord.to(torch.int32).contiguous()
         offset = offset.to(torch.int64).contiguous()
-        n_scenes = offset.shape[0]
-        host = self.host = _host_words(4 + n_scenes, "batch_stats", self.stream, offset.device).begin(self.lib, self.stream)
-        host.launched(self.lib.ptv3_batch_stats(grid_coord.data_ptr(), grid_coord.shape[0], offset.data_ptr(), n_scenes,
-                                                host.address, host.scratch.data_ptr(), self.stream), "ptv3_batch_stats")
-        self.keep = (grid_coord, offset)
+        n, n_scenes = grid_coord.shape[0], offset.shape[0]
+        self.numbered = batch is not None
+        if self.numbered:
+            batch = batch.to(torch.int64).contiguous()
+            if batch.shape != (n,):
+                raise ValueError("batch must be (N,)")
+        host = self.host = _host_words(4 + self.numbered + n_scenes, "batch_stats", self.stream, offset.device)
+        host.begin(self.lib, self.stream)
+        bounds = (n, offset.data_ptr(), n_scenes, host.address, host.scratch.data_ptr(), self.stream)
+        if self.numbered:
+            host.launched(self.lib.ptv3_scene_stats(grid_coord.data_ptr(), batch.data_ptr(), *bounds), "ptv3_scene_stats")
+        else:
+            host.launched(self.lib.ptv3_batch_stats(grid_coord.data_ptr(), *bounds), "ptv3_batch_stats")
+        self.keep = (grid_coord, offset, batch)
 
     def result(self):
-        """(largest grid coordinate per axis, offsets) as Python ints."""
+        """(largest grid coordinate per axis, offsets) as Python ints; ``top_scene``: the largest scene number."""
         got = self.host.wait(self.lib, self.stream)
+        if self.numbered:
+            self.top_scene = got.pop(3)
         return got[:3], got[3:-1]
 
 
@@ -384,7 +396,7 @@ class _HostWords:
     def __init__(self, n, device):
         with torch.inference_mode(False):      # a plain tensor: it is written in and out of inference mode
             self.tensor = torch.empty(n, dtype=torch.int64).pin_memory()
-            self.scratch = None if device is None else torch.full((16,), 0x80, dtype=torch.uint8, device=device)
+            self.scratch = None if device is None else torch.full((32,), 0x80, dtype=torch.uint8, device=device)
         self.address = self.tensor.data_ptr()
         self.words = (ctypes.c_int64 * n).from_address(self.address)
         self.last = self.address + 8 * (n - 1)

@@ -119,19 +119,20 @@ class Point(AttrDict):
             self["grid_coord"] = torch.div(
                 self.coord - self.coord.min(0)[0], self.grid_size, rounding_mode="trunc").int()
 
-    def _bounds(self):
-        """A function that returns the largest grid coordinate per axis as Python ints (the host waits there;
-        the scene sizes come along)."""
+    def _bounds(self, numbered=False):
+        """A function that returns the largest grid coordinate per axis as Python ints, with ``numbered`` the largest
+        number in ``batch`` behind them (the host waits there; the scene sizes come along)."""
         if self.grid_coord.is_cuda and "offset" in self.keys() and self.grid_coord.shape[0] > 0:
-            stats = ops.BatchStats(self.grid_coord, self.offset)
+            stats = ops.BatchStats(self.grid_coord, self.offset, self.batch if numbered else None)
 
             def wait():
                 top, ends = stats.result()
                 if "_counts" not in self.keys():
                     self["_counts"] = [b - a for a, b in zip([0] + ends, ends)]
-                return top
+                return top + [stats.top_scene] if numbered else top
             return wait
-        return torch.max(self.grid_coord, dim=0).values.tolist
+        top = torch.max(self.grid_coord, dim=0).values
+        return (lambda: top.tolist() + [int(self.batch.max())]) if numbered else top.tolist
 
     def serialization(self, order="z", depth=None, shuffle_orders=False):
         """model.py:81-136: codes of every requested order, their stable argsort
@@ -140,12 +141,18 @@ class Point(AttrDict):
         assert "batch" in self.keys()
         self._ensure_grid_coord()
         order = [order] if isinstance(order, str) else list(order)
+        # Bits of the scene numbers that are sorted by.  ``batch`` may be the caller's own and follow other numbers
+        # than the offsets do: its largest one is read with the bounds; where nothing is read, one bit more than the
+        # offsets' numbers need.
+        n_scene_bits = len(self.offset).bit_length()
         if depth is None:
-            depth = max(self._bounds()()).bit_length()
+            *top, scene = self._bounds(numbered=True)()
+            depth = max(top).bit_length()
+            n_scene_bits = max(scene, 0).bit_length()
         depth = max(int(depth), 1)
         self["serialized_depth"] = depth
         assert depth * 3 + len(self.offset).bit_length() <= 63
-        n_scene_bits = (len(self.offset) - 1).bit_length()       # of the largest scene number
+        n_scene_bits = min(n_scene_bits, 63 - depth * 3)
         assert depth <= 16
         if shuffle_orders:
             # the reference shuffles the finished rows (model.py:128-132); the rows are independent of

@@ -101,6 +101,43 @@ def test_argsort_tile_sizes_and_long_keys(k, n, bits):
     assert torch.equal(inverse.gather(1, order), torch.arange(n, device="cuda").expand(k, n))
 
 
+@pytest.mark.parametrize("numbers,depth,given", [((0, 2), 13, False), ((0, 2), 13, True), ((1, 3), 13, True),
+                                                 ((0, 4), 13, False), ((5, 1), 9, False), ((0, 1000), 16, False),
+                                                 ((0, 1), 13, False), ((1, 0), 13, True)])
+def test_scene_numbers_that_do_not_follow_the_offsets(numbers, depth, given):
+    """``batch`` may be the caller's own, next to ``offset``: the codes are sorted by all bits of its numbers, those
+    that the number of scenes does not need included (depth 13 and two scenes: four digits of ten bits and none over)."""
+    from pointtransformerv3_b200 import Point
+    g = torch.Generator().manual_seed(depth)
+    grid = torch.randint(0, 1 << depth, (3000, 3), generator=g, dtype=torch.int32)
+    grid[0] = (1 << depth) - 1
+    batch = torch.tensor(numbers).repeat_interleave(1500)
+    point = Point(grid_coord=grid.cuda(), batch=batch.cuda(), offset=torch.tensor([1500, 3000]).cuda())
+    point.serialization(order=ORDERS, depth=depth if given else None)
+    assert point.serialized_depth == depth
+    for r, o in enumerate(ORDERS):
+        ref = cenc.encode(grid.numpy(), batch.numpy(), depth, o)
+        assert (point.serialized_code[r].cpu().numpy() == ref).all(), o
+        assert (point.serialized_order[r].cpu().numpy() == cenc.argsort_stable(ref)).all(), o
+
+
+@pytest.mark.parametrize("n", [1, 255, 1024, 1025, 700_001])
+def test_batch_stats_hold_the_largest_of_everything(n):
+    """Largest coordinate per axis, and largest scene number as 32 bits, wherever the largest point lies; in turn, since
+    both leave the same scratch words behind for the next call."""
+    g = torch.Generator().manual_seed(n)
+    grid = torch.randint(-70000, 0, (n, 3), generator=g, dtype=torch.int32)
+    batch = torch.randint(-5, 7, (n,), generator=g)
+    offset = torch.tensor([n // 2, n], device="cuda")
+    for where, number in ((0, 9), (n - 1, 1 << 40), (n // 3, 123)):
+        grid[where] = torch.tensor([5, 60000 + where, 1])
+        batch[where] = number
+        for b in (batch.cuda(), None):
+            stats = ops.BatchStats(grid.cuda(), offset, b)
+            assert stats.result() == (grid.amax(0).tolist(), [n // 2, n])
+            assert b is None or stats.top_scene == min(int(batch.max()), 2 ** 31 - 1)
+
+
 def test_large_sort_properties():
     """4 M points x 4 orders: sortedness, stability and inverse, checked on device."""
     n = 4_000_000
