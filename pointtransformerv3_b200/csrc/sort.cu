@@ -32,6 +32,7 @@
 // waits for is already running or finished; all the same every wait is bounded
 // and a wait that runs out sets PTV3_STATUS_WAIT_LIMIT.
 #include "common.cuh"
+#include "sort_order.cuh"
 #include "../../include/ptv3_b200.h"
 
 namespace ptv3 {
@@ -158,9 +159,9 @@ __host__ __device__ constexpr size_t os_element_bytes(int items, int bins, bool 
 //
 // Ranks among the equal digits of a warp: the counters that the histogram adds to hand them out (atomicAdd
 // returns the count so far).  That is the order of the elements except among lanes of one instruction with the same digit,
-// whose order of service nobody promises.  But a packed word holds, below the digit, everything that the order among equal
-// digits goes by (the digits done and the index), so the ordered tile is checked against its words and neighbours out
-// of order are exchanged until none is left (32 lanes at most; on this hardware none has been seen).
+// whose order of service nobody promises.  But a packed word holds everything that the order among equal
+// digits goes by, so neighbours in the ordered tile are compared as they are written, and exchanged until none is out
+// of order (sort_order.cuh; on this hardware none has been seen, so the tests run it on the host).
 // MASKS: sorts that dropped digits on the way (see `wide`) cannot tell; their ranks come from masks of the lanes with
 // the same digit, one shared-memory word per warp and digit, which cost five accesses per element: of the 33 000 cycles
 // of a tile of 8 192 that form spent 11 700 there (8 M x 4 rows of 36 bits: 1 383 us, 1 296 with ranks from the counters).
@@ -398,15 +399,13 @@ __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(const OsPass a)
         return;
     }
     // ---- write out: neighbours in shared memory with the same digit are neighbours in global
-    const uint64_t below = (1ull << shift) - 1ull;
-    // whether two neighbours of one digit are out of the order of what lies below it
-    auto wrong = [&](uint64_t x, uint64_t y) { return (((x ^ y) >> shift) & mask) == 0 && (x & below) > (y & below); };
+    const OsOrder in_digit{shift, mask};
     auto write = [&] {
         bool bad = false;
 #pragma unroll 4
         for (int i = threadIdx.x; i < tile_count; i += OS_THREADS) {
             const uint64_t kx = skeys[i];
-            if (!MASKS && i > 0) bad |= wrong(skeys[i - 1], kx);
+            if (!MASKS && i > 0) bad |= os_wrong(in_digit, skeys[i - 1], kx);
             const int64_t dst = rbase + (uint32_t)(gbase[(uint32_t)(kx >> shift) & mask] + (uint32_t)i);
             if constexpr (OUT == OS_FINAL) {
                 const int64_t v = (int64_t)(kx & ((1ull << a.val_bits) - 1ull));
@@ -430,17 +429,10 @@ __global__ void __launch_bounds__(OS_THREADS, 2) os_pass_kernel(const OsPass a)
     bool bad = write();
     if constexpr (!MASKS) {
         if (__syncthreads_or(bad)) {            // (nobody reads the output before this kernel has ended)
-            for (int round = 0; round < 64; ++round) {
+            for (int round = 0; round < os_rounds(tile_count); ++round) {
                 bad = false;
                 for (int odd = 0; odd < 2; ++odd) {
-                    for (int i = 2 * threadIdx.x + 1 + odd; i < tile_count; i += 2 * OS_THREADS) {
-                        const uint64_t x = skeys[i - 1], y = skeys[i];
-                        if (wrong(x, y)) {
-                            skeys[i - 1] = y;
-                            skeys[i] = x;
-                            bad = true;
-                        }
-                    }
+                    bad |= os_exchange(in_digit, skeys, tile_count, odd, threadIdx.x, OS_THREADS);
                     __syncthreads();
                 }
                 if (!__syncthreads_or(bad)) break;
