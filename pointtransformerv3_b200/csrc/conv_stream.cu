@@ -31,6 +31,7 @@
 // Replaces spconv.SubMConv3d.forward at model.py:546-552 for bf16.  Every wait is bounded and reports through the
 // status word.
 #include "common.cuh"
+#include "conv_gather.cuh"
 #include "conv_mma.cuh"
 #include "mma_util.cuh"
 #include "tc05.cuh"
@@ -39,7 +40,7 @@ namespace ptv3 {
 
 using namespace tc05;
 
-constexpr int CS_TM = 128;             // voxels per tile
+constexpr int CS_TM = CG_ROWS;         // voxels per tile
 constexpr int CS_KVOL = 27;            // offsets, at most
 constexpr int CS_SPLIT_O = 14;         // those of the first index warp
 
@@ -75,7 +76,7 @@ template <int BN, int KC, int STAGES, int NI, int GW, int SETS, int EW>
 __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + EW) * 32, 1) conv_stream_kernel(
     const __grid_constant__ CUtensorMap map_w, const ConvStreamArgs a)
 {
-    constexpr int ROWB = KC * 2, NCH = ROWB / 16;
+    constexpr int ROWB = KC * 2;
     constexpr int A_BYTES = CS_TM * ROWB, B_BYTES = BN * ROWB, STAGE_BYTES = A_BYTES + B_BYTES;
     constexpr int EPI = cs_epi_warp<GW, NI>();
     constexpr int TM_COLS = SETS * NI * BN;
@@ -129,59 +130,25 @@ __global__ void __launch_bounds__((cs_epi_warp<GW, NI>() + EW) * 32, 1) conv_str
 
     if (warp < GW) {
         // ---- gather: stages warp, warp + GW, ... of the CTA's sequence ---------------------------
-        // A lane copies one 16-byte chunk of a row; the lanes of a row take four rows, the next ones the four
-        // after them, so that the numbers of four rows are one load.
-        constexpr int GROUPS = 32 / NCH;                  // rows per instruction
-        const int c = lane % NCH, rg = lane / NCH;
-        uint32_t dst[4];                                  // within a stage's rows, of the four rows
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int r = rg * 4 + j;
-            dst[j] = (uint32_t)(r * ROWB + ((NCH == 8 ? c ^ (r & 7) : c ^ ((r >> 1) & 3)) << 4));
-        }
+        const RowGather<KC> gather(lane);
         const uint32_t pitch = (uint32_t)a.cin * 2;
-        int g = warp, s = warp, phase = 1;                // (GW <= STAGES)
+        int g = warp;
+        StageCursor cur{0, 0, warp, 1};                   // (GW <= STAGES)
         for (int i = 0, t = first; t < a.tiles; ++i, t += step) {
             const int b = i & 1;
             ok &= mbar_wait(idxfull0 + 8 * b, (i >> 1) & 1, abort);
             if (!__all_sync(0xffffffffu, ok)) break;
             const ConvIndex<BN>& x = index[b];
             const int end = seen + x.act[0] * kchunks, col0 = t % col_tiles * BN;
-            // offset (by its place in the list) and chunk of stage g: counted, not divided, from stage to stage
-            int at = (g - seen) / kchunks, chunk = (g - seen) - at * kchunks;
+            cur.at = (g - seen) / kchunks;
+            cur.chunk = (g - seen) - cur.at * kchunks;
             for (; g < end; g += GW) {
-                const int o = x.act[1 + at];
-                const char* src0 = reinterpret_cast<const char*>(a.feat) + chunk * ROWB + c * 16;
-                const int32_t* nb = x.nbr + o * CS_TM + rg * 4;
-                const uint32_t sa = sbase + s * STAGE_BYTES;
-                ok &= mbar_wait(empty0 + 8 * s, phase, abort);
-#pragma unroll
-                for (int j0 = 0; j0 < CS_TM; j0 += GROUPS * 4) {
-                    const int4 n4 = *reinterpret_cast<const int4*>(nb + j0);
-                    const int src[4] = {n4.x, n4.y, n4.z, n4.w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        cp_async16_zfill(sa + j0 * ROWB + dst[j], src0 + (uint64_t)(uint32_t)max(src[j], 0) * pitch, src[j] >= 0);
-                }
-                cp_async_commit();
-                if (elect_one()) {
-                    mbar_expect_tx(full0 + 8 * s, B_BYTES);
-                    tma_load_2d(sa + A_BYTES, &map_w, o * a.cin + chunk * KC, col0, full0 + 8 * s);
-                }
-                cp_async_wait<0>();
-                fence_proxy_async();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_one(full0 + 8 * s);
-                chunk += GW;
-                while (chunk >= kchunks) {
-                    chunk -= kchunks;
-                    ++at;
-                }
-                s += GW;
-                if (s >= STAGES) {
-                    s -= STAGES;
-                    phase ^= 1;
-                }
+                const int o = x.act[1 + cur.at], chunk = cur.chunk;
+                ok &= mbar_wait(empty0 + 8 * cur.slot, cur.phase, abort);
+                fill_stage<KC, B_BYTES>(gather, sbase + cur.slot * STAGE_BYTES, x.nbr + o * CS_TM,
+                                        reinterpret_cast<const char*>(a.feat) + chunk * ROWB, pitch, &map_w,
+                                        o * a.cin + chunk * KC, col0, full0 + 8 * cur.slot, lane);
+                cur.step<GW, STAGES>(kchunks);
             }
             seen = end;
             __syncwarp();

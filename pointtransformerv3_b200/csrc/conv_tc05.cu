@@ -32,6 +32,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "conv_gather.cuh"
 #include "conv_mma.cuh"
 #include "mma_util.cuh"
 #include "split_f32.cuh"
@@ -41,10 +42,10 @@ namespace ptv3 {
 
 using namespace tc05;
 
-constexpr int CT_TM = 128;         // voxels per tile
+constexpr int CT_TM = CG_ROWS;     // voxels per tile
+constexpr int CT_KC = 64;          // channels per stage
 constexpr int CT_MAX_KVOL = 27;
 constexpr int CT_GATHER_WARPS = 8;
-
 
 struct ConvTcArgs {
     const __nv_bfloat16* feat;
@@ -71,23 +72,22 @@ __device__ __forceinline__ void ct_store_f32(const ConvTcArgs& a, int64_t row, i
     o[1] = make_float4(y[4], y[5], y[6], y[7]);
 }
 
-template <int BN, int KC, int STAGES, int NI, bool SPLIT, bool F32>
+template <int BN, int STAGES, int NI, bool SPLIT, bool F32>
 __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                const ConvTcArgs a)
 {
-    constexpr int ROWB = KC * 2;                    // bytes per staged row: one swizzle span (128 or 64)
-    constexpr int NCH = ROWB / 16;                  // 16-byte chunks per row
+    static_assert(SPLIT || F32, "whole bf16 tiles: conv_stream.cu");
+    constexpr int KC = CT_KC, ROWB = KC * 2;        // bytes per staged row: one swizzle span
     constexpr int A_BYTES = CT_TM * ROWB, B_BYTES = BN * ROWB, STAGE_BYTES = A_BYTES + B_BYTES;
     constexpr int CT_THREADS = (CT_GATHER_WARPS + NI) * 32;
-    // NI issuing threads, each with its own accumulator in tensor memory (columns rounded up to a power
-    // of two for the allocation).  A slot of the ring must always be consumed by the same issuer
-    // (STAGES a multiple of NI): an issuer that met a slot whose previous use another, slower issuer had
-    // not consumed yet would take the parity of that older phase for its own.
+    // NI issuing warps, each with its own accumulator in tensor memory.  A slot of the ring must always be
+    // consumed by the same issuer (STAGES a multiple of NI): an issuer that met a slot whose previous use
+    // another, slower issuer had not consumed yet would take the parity of that older phase for its own.
     // fp32: SPLIT_ACCS accumulators each (split_f32.cuh)
     constexpr int ACCS = F32 ? SPLIT_ACCS : 1;
-    constexpr int TM_USED = NI * ACCS * BN;
-    constexpr int TM_COLS = TM_USED <= 32 ? 32 : TM_USED <= 64 ? 64 : TM_USED <= 128 ? 128 : TM_USED <= 256 ? 256 : 512;
-    static_assert(TM_USED <= 512 && STAGES % NI == 0, "issuers and accumulators");
+    constexpr int TM_COLS = NI * ACCS * BN;
+    static_assert(TM_COLS >= 32 && TM_COLS <= 512 && (TM_COLS & (TM_COLS - 1)) == 0, "tensor memory");
+    static_assert(STAGES % NI == 0, "issuers and accumulators");
     static_assert(STAGE_BYTES % 1024 == 0 && A_BYTES % 1024 == 0, "operand tiles start on a swizzle atom");
     // Warps that gather: at most one per stage of the ring.  A parity wait on an mbarrier can only tell
     // the current phase from the one before it, so a warp must never be two uses ahead of a slot: its
@@ -211,55 +211,18 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
         // act[it / kchunks], channels of chunk it % kchunks, and (lane 0) the matching slice of W.
         // The warps run independent pipelines, so the fixed cost of a stage (barrier waits, the TMA
         // issue, the proxy fence) and the latency of its copies overlap with the other warps' stages.
-        // A lane copies one 16-byte chunk of a row; the lanes of a row take four rows, the next ones the four
-        // after them, so that the numbers of four rows are one load.
-        constexpr int GROUPS = 32 / NCH;                  // rows per instruction
-        const int c = lane % NCH, rg = lane / NCH;
-        uint32_t dst[4];                                  // within a stage's rows, of the four rows
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int r = rg * 4 + j;
-            dst[j] = (uint32_t)(r * ROWB + ((NCH == 8 ? c ^ (r & 7) : c ^ ((r >> 1) & 3)) << 4));
-        }
+        const RowGather<KC> gather(lane);
         const uint32_t pitch = (uint32_t)stored * 2;
-        // offset (by its place in the list) and chunk of the stage: counted, not divided, from stage to stage
-        int at = (first + warp) / kchunks, chunk = (first + warp) - at * kchunks, s = warp % STAGES, phase = 1;
+        StageCursor cur{(first + warp) / kchunks, (first + warp) % kchunks, warp % STAGES, 1};
         for (int it = warp < NGW ? warp : nit; it < nit; it += NGW) {
-            const int o = act[1 + at];
-            const int kc = F32 ? split_column_a(chunk, a.cin / 6) : chunk * KC;
-            const int kw = F32 ? split_column_b(chunk, a.cin / 6) : chunk * KC;
-            const uint32_t sa = sbase + s * STAGE_BYTES;
-            const char* src0 = reinterpret_cast<const char*>(a.feat + kc) + c * 16;
-            const int32_t* nb = nbr_s + o * CT_TM + rg * 4;
-            ok &= mbar_wait(empty0 + 8 * s, phase, abort);
-#pragma unroll
-            for (int j0 = 0; j0 < CT_TM; j0 += GROUPS * 4) {
-                const int4 n4 = *reinterpret_cast<const int4*>(nb + j0);
-                const int src[4] = {n4.x, n4.y, n4.z, n4.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-                    cp_async16_zfill(sa + j0 * ROWB + dst[j], src0 + (uint64_t)(uint32_t)max(src[j], 0) * pitch, src[j] >= 0);
-            }
-            cp_async_commit();
-            // (the weight load is issued after the copies, which are already on their way then)
-            if (elect_one()) {
-                mbar_expect_tx(full0 + 8 * s, B_BYTES);
-                tma_load_2d(sa + A_BYTES, &map_w, o * stored + kw, col0, full0 + 8 * s);
-            }
-            cp_async_wait<0>();
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_one(full0 + 8 * s);
-            chunk += NGW;
-            while (chunk >= kchunks) {
-                chunk -= kchunks;
-                ++at;
-            }
-            s += NGW;
-            if (s >= STAGES) {
-                s -= STAGES;
-                phase ^= 1;
-            }
+            const int o = act[1 + cur.at];
+            const int kc = F32 ? split_column_a(cur.chunk, a.cin / 6) : cur.chunk * KC;
+            const int kw = F32 ? split_column_b(cur.chunk, a.cin / 6) : cur.chunk * KC;
+            ok &= mbar_wait(empty0 + 8 * cur.slot, cur.phase, abort);
+            fill_stage<KC, B_BYTES>(gather, sbase + cur.slot * STAGE_BYTES, nbr_s + o * CT_TM,
+                                    reinterpret_cast<const char*>(a.feat + kc), pitch, &map_w, o * stored + kw, col0,
+                                    full0 + 8 * cur.slot, lane);
+            cur.step<NGW, STAGES>(kchunks);
         }
 
         // ---- epilogue: thread = voxel ----------------------------------------------------------
@@ -271,7 +234,6 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
         const int q = warp & 3, half = warp >> 2;      // lane quarter of tensor memory, half of the columns
         const int64_t v = rows_s[q * 32 + lane];
         const uint32_t tm = tmem_base + ((uint32_t)(q * 32) << 16);
-        __nv_bfloat16* orow = (__nv_bfloat16*)a.out + v * a.cout + col0;
         constexpr int NCB = BN / 32;                   // 32-column blocks, split between the two halves
 #pragma unroll 1
         for (int cb = half * ((NCB + 1) / 2); cb < (half == 0 ? (NCB + 1) / 2 : NCB); ++cb) {
@@ -320,25 +282,12 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
                 continue;
             }
             if (v < 0) continue;
-            if (F32) {
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    float y[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) y[i] = __uint_as_float(acc[g * 8 + i]) + bias_s[cb * 32 + g * 8 + i];
-                    ct_store_f32(a, v, col0 + cb * 32 + g * 8, y);
-                }
-                continue;
-            }
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
-                uint4 o4;
-                uint32_t* o = reinterpret_cast<uint32_t*>(&o4);
+                float y[8];
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    o[i] = pack_bf16(__uint_as_float(acc[g * 8 + 2 * i]) + bias_s[cb * 32 + g * 8 + 2 * i],
-                                     __uint_as_float(acc[g * 8 + 2 * i + 1]) + bias_s[cb * 32 + g * 8 + 2 * i + 1]);
-                *reinterpret_cast<uint4*>(orow + cb * 32 + g * 8) = o4;
+                for (int i = 0; i < 8; ++i) y[i] = __uint_as_float(acc[g * 8 + i]) + bias_s[cb * 32 + g * 8 + i];
+                ct_store_f32(a, v, col0 + cb * 32 + g * 8, y);
             }
         }
     } else {
@@ -442,22 +391,22 @@ bool conv_tc05_supported(int c_in, int c_out, int kernel_volume)
     return c_in % 64 == 0 && c_in <= 4096 && c_out % 64 == 0 && c_out <= 4096;
 }
 
-template <int BN, int KC, int STAGES>
+template <int BN, int STAGES>
 static constexpr size_t conv_tc05_smem()
 {
-    return (size_t)STAGES * (CT_TM + BN) * KC * 2 + CT_MAX_KVOL * CT_TM * 4 + CT_TM * 8 + 32 * 4 + BN * 4 +
+    return (size_t)STAGES * (CT_TM + BN) * CT_KC * 2 + CT_MAX_KVOL * CT_TM * 4 + CT_TM * 8 + 32 * 4 + BN * 4 +
            8 * (2 * STAGES + 1) + 32 + 1024;
 }
 
-template <int BN, int KC, int STAGES, int NI, bool SPLIT, bool F32>
+template <int BN, int STAGES, int NI, bool SPLIT, bool F32>
 static int launch_conv_tc05_as(const void* weight, const ConvTcArgs& a, cudaStream_t stream, int parts)
 {
     CUtensorMap mw;
     const uint64_t wcols = (uint64_t)a.kvol * (F32 ? a.cin / 6 * split_stored(a.cin / 6) : a.cin);
-    const int rc = make_tensor_map_bf16(&mw, weight, (uint64_t)a.cout, wcols, wcols * 2, BN, KC);
+    const int rc = make_tensor_map_bf16(&mw, weight, (uint64_t)a.cout, wcols, wcols * 2, BN, CT_KC);
     if (rc) return rc;
-    constexpr size_t smem = conv_tc05_smem<BN, KC, STAGES>();
-    auto kern = conv_tc05_kernel<BN, KC, STAGES, NI, SPLIT, F32>;
+    constexpr size_t smem = conv_tc05_smem<BN, STAGES>();
+    auto kern = conv_tc05_kernel<BN, STAGES, NI, SPLIT, F32>;
     if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_subm_conv_fwd: shared memory attribute");
     const dim3 grid((unsigned)((a.n + CT_TM - 1) / CT_TM), a.cout / BN, parts);
@@ -467,19 +416,19 @@ static int launch_conv_tc05_as(const void* weight, const ConvTcArgs& a, cudaStre
 }
 
 // CTAs in clusters of `parts` that run at once (the driver's answer: a cluster lives in one GPC)
-template <int BN, int KC, int STAGES, int NI, bool F32>
+template <int BN, int STAGES, int NI, bool F32>
 static int conv_tc05_capacity(int parts)
 {
     static std::atomic<int> known[4];
     const int slot = parts == 2 ? 1 : parts == 4 ? 2 : 3;
     int c = known[slot].load(std::memory_order_relaxed);
     if (c == 0) {
-        auto kern = conv_tc05_kernel<BN, KC, STAGES, NI, true, F32>;
+        auto kern = conv_tc05_kernel<BN, STAGES, NI, true, F32>;
         if (allow_smem(kern) != cudaSuccess) return 0;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(SMS, 1, parts);
         cfg.blockDim = dim3((CT_GATHER_WARPS + NI) * 32);
-        cfg.dynamicSmemBytes = conv_tc05_smem<BN, KC, STAGES>();
+        cfg.dynamicSmemBytes = conv_tc05_smem<BN, STAGES>();
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = attr[0].val.clusterDim.y = 1;
@@ -507,16 +456,16 @@ struct ConvVariant {
 constexpr int CT_VARIANTS = 3;
 // fp32 output (an issuer's four accumulators of 64 columns fill the tensor memory of an SM).  Last: 32 channels.
 static const ConvVariant g_variants_f32[CT_VARIANTS] = {
-    {64, 6.5, 0, 0.20, launch_conv_tc05_as<64, 64, 8, 2, false, true>, launch_conv_tc05_as<64, 64, 8, 2, true, true>,
-     conv_tc05_capacity<64, 64, 8, 2, true>},
-    {32, 6.5, 0, 0.18, launch_conv_tc05_as<32, 64, 8, 2, false, true>, launch_conv_tc05_as<32, 64, 8, 2, true, true>,
-     conv_tc05_capacity<32, 64, 8, 2, true>},
+    {64, 6.5, 0, 0.20, launch_conv_tc05_as<64, 8, 2, false, true>, launch_conv_tc05_as<64, 8, 2, true, true>,
+     conv_tc05_capacity<64, 8, 2, true>},
+    {32, 6.5, 0, 0.18, launch_conv_tc05_as<32, 8, 2, false, true>, launch_conv_tc05_as<32, 8, 2, true, true>,
+     conv_tc05_capacity<32, 8, 2, true>},
     {1 << 20, 0, 0, 0, nullptr, nullptr, nullptr}};
 // bf16: clusters here, whole tiles in conv_stream.cu
 static const ConvVariant g_variants[CT_VARIANTS] = {
-    {64, 6.9, 1.6, 0.19, nullptr, launch_conv_tc05_as<64, 64, 8, 2, true, false>, conv_tc05_capacity<64, 64, 8, 2, false>},
-    {128, 8.7, 1.6, 0.26, nullptr, launch_conv_tc05_as<128, 64, 6, 2, true, false>, conv_tc05_capacity<128, 64, 6, 2, false>},
-    {256, 12., 1.6, 0.37, nullptr, launch_conv_tc05_as<256, 64, 4, 2, true, false>, conv_tc05_capacity<256, 64, 4, 2, false>}};
+    {64, 6.9, 1.6, 0.19, nullptr, launch_conv_tc05_as<64, 8, 2, true, false>, conv_tc05_capacity<64, 8, 2, false>},
+    {128, 8.7, 1.6, 0.26, nullptr, launch_conv_tc05_as<128, 6, 2, true, false>, conv_tc05_capacity<128, 6, 2, false>},
+    {256, 12., 1.6, 0.37, nullptr, launch_conv_tc05_as<256, 4, 2, true, false>, conv_tc05_capacity<256, 4, 2, false>}};
 
 // The cluster size and tile width with the shortest estimated time: waves of CTAs, each taking a
 // fixed time (prologue, epilogue) and its stages.  Wide tiles gather a row once for more output
