@@ -660,11 +660,12 @@ def run_operator_case(args):
         out.update(config={"workload": "SubMConv3d 3x3x3, C=%d, bf16, one indoor scene" % c, "voxels": n,
                            "pairs": pairs, "algo": args.algo},
                    metric="conv_voxels_per_sec", unit="voxels/s", value=n / (t * 1e-3), ms=t, kmap_ms=t_map,
-                   roofline={"kernel": "conv_mma_kernel" if args.algo == 2 else "conv_tc05_kernel",
+                   roofline={"kernel": "conv_mma_kernel" if args.algo == 2 else
+                             "conv_stream_kernel (few tiles: conv_tc05_kernel)",
                              "bound": "tensor", "achieved": flops / t / 1e9,
                              "peak": tf, "unit": "TFLOP/s (useful FLOPs: 2 x pairs x C^2)",
                              "frac": flops / t / 1e9 / tf, "traffic": None},
-                   roofline_kmap={"kernel": "km_insert + km_probe", "bound": "hbm",
+                   roofline_kmap={"kernel": "vi_block_insert + vi_cell_fill + km_block_probe", "bound": "hbm",
                                   "achieved": 124.0 * n / t_map / 1e6, "peak": hbm, "unit": "GB/s",
                                   "frac": 124.0 * n / t_map / 1e6 / hbm, "traffic": None})
     elif args.case == "stem":

@@ -40,23 +40,18 @@
 // columns of its S; O|l in 96..127).
 // Every mbarrier wait is bounded; a wait that runs out sets PTV3_STATUS_WAIT_LIMIT.
 //
-// Measured on B200 (240 000 points, C = 64, 4 heads): 0.41 ms against 0.31 ms of the mma.sync
-// kernel (attention_mma.cu), which therefore stays the automatic choice.  Cycle stamps of one
-// group against its issuer show what bounds this kernel: a key block takes a group ~2400
-// cycles whatever the softmax does (all exponentials on the exponential unit, three of eight
-// on the FMA pipe, or none at all), and the next S is seen one block period after the product
-// that makes it was issued.  The period is the asynchronous tensor path working through the
-// 16 products of a round of the four groups (3 x P V' + 1 x Q K^T each): at head dimension 16
-// every product is tiny (128 x 32 x 16 or 128 x 48 x 16), K is 16 per instruction by the
-// instruction set, so a (patch, head) pair needs ~690 of them at ~150 cycles each, whatever
-// their size.  The arithmetic is not what takes the time: the profiler shows the tensor pipe
-// 12 % active, the exponential unit 41 % and instruction issue 65 %; the time goes to the
-// latency of each product through that path (issue, operand fetch from shared and tensor
-// memory, commit), which at this size is not hidden by the next product.  The mma.sync kernel
-// pays for its products with issue slots of the CUDA cores instead, which it has.
+// Measured on B200 (C = 64, 4 heads; us here and by the mma.sync kernel, attention_mma.cu, which therefore
+// stays the automatic choice): 120 000 points 213 / 147, 240 000 399 / 273, 407 000 628 / 449.  Cycle stamps of one
+// group against its issuer: a key block takes a group ~2400 cycles whatever the softmax does (all exponentials
+// on the exponential unit, three of eight on the FMA pipe, or none at all), and the next S is seen one block
+// period after the product that makes it was issued.  No single unit is what that time goes to: the
+// profiler shows the tensor pipe 12 % active, the exponential unit 41 % and instruction issue 65 %.  Nor is it the
+// issue of the products: here a lane of a diverged warp issues them, ~150 cycles each (see elect_one in tc05.cuh), and
+// with an elected lane of a converged one the three sizes take 207, 389 and 610 us, 3 % less (219, 399 and 628 with all
+// exponentials on their unit).  What is left is the chain of a block (S out of tensor memory, exponentials, P back,
+// P V', the next S) with four groups in flight; which part of it could be shorter is not known.
 // Earlier forms of this kernel (scores read back every block with the output in registers;
-// two passes with the exact maximum first; one score buffer) all ran at 0.42-0.49 ms for
-// the same reason.
+// two passes with the exact maximum first; one score buffer) all ran at 0.42-0.49 ms at 240 000 points.
 #include "common.cuh"
 #include "attention_mma.cuh"
 #include "mma_util.cuh"

@@ -291,10 +291,10 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
             }
         }
     } else {
-        // ---- issuers: thread i takes stages i, i + NI, ... in order and accumulates them in
-        // its own accumulator.  One thread can start a stage's products only every ~450 cycles (a look
-        // at the stage's barrier costs it as much as the four products), which is what bounded the
-        // kernel with a single issuer; the partial sums are added in the epilogue.
+        // ---- issuers: warp i takes stages i, i + NI, ... in order and accumulates them in
+        // its own accumulator; the partial sums are added in the epilogue.  (Two, because a lane of a diverged warp
+        // took ~150 cycles to issue a product, which held a single issuer up; an elected lane takes ~30.  The second
+        // accumulator stays for the sums: the tensor core truncates as it adds, see conv_cluster_cost.)
         constexpr uint32_t idesc = umma_idesc_bf16(CT_TM, BN);
         const int me = warp - CT_GATHER_WARPS;
         const uint32_t tm_acc = tmem_base + me * ACCS * BN;
@@ -470,6 +470,13 @@ static const ConvVariant g_variants[CT_VARIANTS] = {
 // The cluster size and tile width with the shortest estimated time: waves of CTAs, each taking a
 // fixed time (prologue, epilogue) and its stages.  Wide tiles gather a row once for more output
 // channels; clusters fill SMs that a single wave leaves idle.  `stages`: of a tile.  The constants are measured.
+//
+// The choice also sets how many partial sums a tile has, issuers x CTAs of its cluster, and the tensor core truncates where
+// an fp32 addition rounds.  Share of the results (bf16) that are not the rounded 64-bit sum, with the lines as they are and
+// with twice to four times the sums (clusters of up to eight wherever they fit a wave): 3 900 x 64 0.007 / 0.005 %,
+// 9 000 x 64 0.013 / 0.008, 5 000 x 128 0.032 / 0.017, 1 200 x 256 0.035 / 0.011, 2 500 x 256 0.067 / 0.021, 2 400 x 512
+// 0.133 / 0.072; the persistent kernel's two sums 9 000 x 512 0.147.  The error against 64 bits is that of the rounding to
+// bf16 in all of them (0.00165 of the norm, the same to six digits).
 static double conv_cluster_cost(const ConvVariant* variants, const ConvTcArgs& a, double stages, int* best_v, int* best_parts)
 {
     const int64_t tiles = (a.n + CT_TM - 1) / CT_TM;
