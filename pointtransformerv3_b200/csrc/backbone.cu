@@ -302,10 +302,9 @@ int Pass::finest()
     BB_CUDA(events_.record(main_, &inputs));
     BB_CUDA(cudaStreamWaitEvent(side_, inputs, 0));
     // planning stream: codes, orders, inverses
-    // (bits of the largest scene number; the pooling plans report one that has no scene, and without any a number is
-    // free to be larger)
+    // (bits of the largest scene number: a larger one in `batch` is reported by the first pooling plan)
     int scene_bits = 0;
-    while (((a_.n_scenes - (a_.n_enc > 1 ? 1 : 0)) >> scene_bits) != 0) ++scene_bits;
+    while (((a_.n_scenes - 1) >> scene_bits) != 0) ++scene_bits;
     const int sig_bits = 3 * a_.depth + scene_bits;
     const size_t sort_bytes = ptv3_argsort_workspace_bytes(a_.k, a_.n, sig_bits);
     char* sort_ws = plan_mem_.take<char>(sort_bytes);
