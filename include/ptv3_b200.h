@@ -156,14 +156,14 @@ int ptv3_pad_plan(const int64_t* offset, int n_scenes, int patch, int64_t n, int
  *   max_seqlen  longest patch (rows); head_dim = channels / heads in {8,16,32,64}
  *   dtype       PTV3_DTYPE_*; algo 0 = automatic, 1 = CUDA-core path,
  *               2 = mma.sync tensor-core path (bf16, head_dim 16, max_seqlen
- *               <= 2048; what "automatic" takes when it applies), 3 = the same
- *               with the exponent arguments rounded to bf16 and two exps per
- *               instruction (measured no faster on B200: the exp unit's rate
- *               per element is the same; kept for comparison), 4 = tcgen05 /
- *               tensor-memory path (bf16, head_dim 16, max_seqlen <= 1024,
- *               needs `status`; measured 40 % slower than 2 on B200: at head
- *               dimension 16 the tensor pipe is bound by the number of tiny
- *               products, not by their arithmetic)
+ *               <= 2048), 3 = the same with the exponent arguments rounded
+ *               to bf16 and two exps per instruction (measured no faster on
+ *               B200: the exp unit's rate per element is the same; kept for
+ *               comparison), 4 = tcgen05 / tensor-memory path (bf16,
+ *               head_dim 16, max_seqlen <= 1024, out 16-byte aligned, needs
+ *               `status`).  "Automatic" takes 4 where it is the faster one
+ *               (long patches, from about 33 blocks of 128 x 128 scores per
+ *               SM), else 2, else 1
  *   status      one uint32 or NULL.  Every path ORs PTV3_STATUS_BAD_INDEX into it
  *               when cu_seqlens holds a patch longer than max_seqlen (that patch is
  *               skipped, its output rows stay unwritten; with NULL it is skipped

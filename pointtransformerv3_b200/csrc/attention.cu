@@ -191,14 +191,14 @@ static int attention_impl(const void* qkv, const int64_t* order, const int64_t* 
     const bool mma_ok = rpe.grid_coord == nullptr && dtype == PTV3_DTYPE_BF16 &&
                         attn_mma_supported(channels, heads, max_seqlen) &&
                         n <= 2147483647ll && ((uintptr_t)qkv & 15) == 0 && ((uintptr_t)out & 3) == 0;
-    const bool tc05_ok = mma_ok && status != nullptr && attn_tc05_supported(channels, heads, max_seqlen) &&
+    const bool tc05_ok = mma_ok && status != nullptr && attn_tc05_supported(n_seq, channels, heads, max_seqlen) &&
                          ((uintptr_t)out & 15) == 0;
     PTV3_REQUIRE(algo != 4 || tc05_ok, PTV3_ERR_UNSUPPORTED,
                  "ptv3_attention_fwd: the tcgen05 path needs bf16, head dim 16, max_seqlen <= %d, 16-byte "
                  "aligned qkv and out, and a status word", ATTN_TC05_MAX_SEQLEN);
-    if (algo == 4)
+    if (algo == 4 || (algo == 0 && tc05_ok && attn_tc05_wanted(n, n_seq, heads, max_seqlen)))
         return launch_attn_tc05(qkv, order, pad, unpad, cu_seqlens, out, n_seq, max_seqlen, channels,
-                                heads, scale, status, (cudaStream_t)stream);
+                                heads, scale, planned, status, (cudaStream_t)stream);
     PTV3_REQUIRE(algo < 2 || mma_ok, PTV3_ERR_UNSUPPORTED,
                  "ptv3_attention_fwd: the tensor-core path needs bf16, head dim 16, max_seqlen <= %d and "
                  "16-byte aligned qkv", ATTN_MMA_MAX_SEQLEN);

@@ -1,57 +1,41 @@
-// Patch attention core on the 5th-generation tensor cores (tcgen05 + tensor memory)
-// for bf16 features, head dimension 16 and patches of up to 1024 rows: the shape
-// of every stage of the default backbone (model.py:452-484).
+// Patch attention core on the 5th-generation tensor cores (tcgen05 + tensor memory) for bf16 features, head
+// dimension 16 and patches of up to 1024 rows (model.py:452-484; see attention.cu for the contract).
 //
-// At head dimension 16 a score costs 64 tensor FLOPs and one exponential, so the
-// exponential unit bounds the kernel, not the tensor pipe.  With tcgen05 the two
-// matrix products cost the CUDA cores nothing (one thread issues one instruction
-// per block instead of an ldmatrix + mma.sync stream in every warp), and a thread
-// owns a whole score row (tensor-memory lane = query row), so row maxima need no
-// shuffles.  What is left per score on the CUDA cores is half a max, half a packed
-// multiply-add, the exponential and half a conversion.
+// At head dimension 16 a score costs 64 tensor FLOPs and one exponential.  tcgen05 takes both products off the CUDA
+// cores, whose issue slots are then free to evaluate a share of the exponentials on the FMA pipe beside the
+// exponential unit (AT_POLY of 16).
 //
-// One CTA owns one (patch, head) pair (optionally a slice of its query tiles).
-//   gather   K and V of the whole patch, through order[pad[.]], with cp.async into
-//            the no-swizzle UMMA operand layout: planes [d chunk][key] of 16-byte
-//            chunks, which is K-major for K (B of Q K^T) and MN-major for V (B of P V).
-//            V carries a third plane holding a column of ones, so that P V' also
-//            yields the row sums of the rounded probabilities.  The gather is issued
-//            by the four issuing warps in blocks of 128 keys, each with its own
-//            mbarrier, so the first products start when the first block has landed.
-//   four softmax groups of 128 threads, each walking 128-query tiles on its own, and
-//   one issuing warp per group; they talk through mbarriers only.  Per 48-key block:
-//     issuer   S[128 x 48] = Q K_j^T into one of two score buffers (one tcgen05.mma, K = 16),
-//              always one block ahead of the group
-//     softmax  tcgen05.ld S -> registers, block maximum, P = exp2(S - m) rounded to bf16
-//              and written over the first half of that S (tcgen05.st), arrive "P ready"
-//     issuer   O|l [128 x 32] += P V'_j  (A from tensor memory, accumulating over all key
-//              blocks), then S_j+2 into the buffer P_j occupied
-//   and at the end of a tile the group reads O|l once, divides and writes its rows.
-//   With two score buffers the next S is ready when a group has finished a block, so the
-//   groups never wait in step and the exponential unit always has a group to serve.
-//   The output stays in tensor memory for the whole tile.  The reference value m of the
-//   exponentials is raised lazily (only when a score exceeds it by 2^8); in that rare case
-//   the group waits for the product before it and rescales O|l in place.
-//   A share of the exponentials (AT_POLY of every 8 pairs) is evaluated on the FMA pipe
-//   (range reduction + cubic), the rest on the exponential unit: with the products off
-//   the CUDA cores there are issue slots to spare, and the exponential unit is the
-//   bottleneck otherwise.
-// Tensor memory: 128 columns per group (S_0 in 0..47, S_1 in 48..95, each P over the first 24
-// columns of its S; O|l in 96..127).
+// One persistent CTA per SM owns a contiguous range of query tiles (128 rows of a (patch, head) pair).
+//   three softmax groups of 128 threads (thread = query row = tensor-memory lane); group g takes tiles g, g + 3, ...
+//   one issuing warp per group; per block of 128 keys S[128 x 128] = Q K^T, and O|l[128 x 32] += P V' (A from tensor
+//     memory) once the group has written P over the first half of S, with the next S right behind it
+//   four loading warps: K and V of a pair through order[pad[.]] into one of two slots, Q tiles into two slots per
+//     group, both ahead of their use.
+// All of them talk through mbarriers only.  V' has a column of ones beside V, so that P V' also yields the row sums of
+// the rounded probabilities.  Keys behind a patch's end have zero K, V and ones: their probabilities (1) add nothing.
+//
+// Softmax needs no reference value where no score can leave the range of exp2: |q . k| <= |q| max|k| (AT_BOUND, checked by
+// the loading warps).  A tile with a row that fails the test takes its scores twice, first for the row maxima.
+//
+// Tensor memory per group: S (128 columns, P over the first 64) | O|l (32) = 160 columns.
 // Every mbarrier wait is bounded; a wait that runs out sets PTV3_STATUS_WAIT_LIMIT.
 //
-// Measured on B200 (C = 64, 4 heads; us here and by the mma.sync kernel, attention_mma.cu, which therefore
-// stays the automatic choice): 120 000 points 213 / 147, 240 000 399 / 273, 407 000 628 / 449.  Cycle stamps of one
-// group against its issuer: a key block takes a group ~2400 cycles whatever the softmax does (all exponentials
-// on the exponential unit, three of eight on the FMA pipe, or none at all), and the next S is seen one block
-// period after the product that makes it was issued.  No single unit is what that time goes to: the
-// profiler shows the tensor pipe 12 % active, the exponential unit 41 % and instruction issue 65 %.  Nor is it the
-// issue of the products: here a lane of a diverged warp issues them, ~150 cycles each (see elect_one in tc05.cuh), and
-// with an elected lane of a converged one the three sizes take 207, 389 and 610 us, 3 % less (219, 399 and 628 with all
-// exponentials on their unit).  What is left is the chain of a block (S out of tensor memory, exponentials, P back,
-// P V', the next S) with four groups in flight; which part of it could be shorter is not known.
-// Earlier forms of this kernel (scores read back every block with the output in registers;
-// two passes with the exact maximum first; one score buffer) all ran at 0.42-0.49 ms at 240 000 points.
+// Measured (C = 64, 4 heads, patches of 1 024; us here and by the mma.sync kernel, attention_mma.cu): 100 000 points
+// 100 / 121, 400 000 352 / 447, 912 000 785 / 991, 98 to 103 % of the exponential unit's rate at 1 965 MHz.  128 x 128 scores
+// take an SM 975 cycles (mma.sync 1 250): the exponential unit needs 640 of them for its ten of sixteen; a loop of the
+// same reads, arithmetic and stores without any hand-over runs at 784.  What is left is a block's way through the roles
+// (softmax -> issuing warp -> product -> softmax, ~900 cycles), which the two other groups cover only in part.
+//   * Blocks of 128 keys and one buffer, not 64 and two (505 us where this takes 406, 444 patches of 4 heads): a
+//     hand-over costs ~170 cycles in the issuing warp's wait and ~160 in issuing, whatever the block's size, and
+//     an issuing warp that keeps three groups waiting bounded the earlier forms of this kernel, not the products
+//     (16 cycles each for P V', 64 for S).
+//   * 16 columns per read of tensor memory, two reads in flight: 32 columns take registers that spill (437 us for 406).
+//   * Two groups with larger blocks (511) or four with blocks of 96 keys (418) are slower; so is handing a block over
+//     in halves (408 to 420), probabilities in registers with P V on mma.sync (583), and a patch's rows looked up
+//     ahead by the loading warps (their instructions count: 100 000 points 105 us).
+//   * AT_POLY 4, 5, 6, 7, 8: 430, 414, 406, 406, 418 us; 0 (all on the exponential unit): 510.
+//   * 80 registers a thread, so that kernels of the planning stream fit beside a CTA: 377 us for 361 at 400 000
+//     points, and no pass gained (16 LiDAR frames 42.0 ms, with 96 registers 41.3).
 #include "common.cuh"
 #include "attention_mma.cuh"
 #include "mma_util.cuh"
@@ -61,46 +45,47 @@ namespace ptv3 {
 
 using namespace tc05;
 
-constexpr int AT_WG = 4;                    // softmax groups of 128 threads
-constexpr int AT_SOFTMAX_THREADS = 128 * AT_WG;
-constexpr int AT_THREADS = AT_SOFTMAX_THREADS + 32 * AT_WG;   // + one issuing warp per group
-constexpr int AT_BM = 128;                  // query rows per tile
-constexpr int AT_BK = 48;                   // keys per block (two score buffers of 48 columns)
-constexpr int AT_POLY = 3;                  // of every 8 pairs of exponentials, this many on the FMA pipe
-constexpr float AT_LAZY = 8.f;              // slack of the reference value, in powers of two
+constexpr int AT_GROUPS = 3;
+constexpr int AT_LOAD_WARP = AT_GROUPS;           // first loading warp, behind the issuing ones; the others come last
+constexpr int AT_SOFT_WARP = 4;                   // first softmax warp (a multiple of 4: a quarter of the lanes each)
+constexpr int AT_REST_WARP = AT_SOFT_WARP + 4 * AT_GROUPS;
+constexpr int AT_THREADS = 32 * (AT_REST_WARP + 3);
+static_assert(AT_LOAD_WARP + 1 == AT_SOFT_WARP, "roles of the warps");
+constexpr int AT_BM = 128;                        // query rows of a tile
+constexpr int AT_BK = 128;                        // keys of a block
 constexpr int AT_D = 16;
-constexpr int AT_KV_BLOCK = 128;            // keys per gather block (one mbarrier each)
-constexpr int AT_KV_BLOCKS = ATTN_TC05_MAX_SEQLEN / AT_KV_BLOCK;
+constexpr int AT_MAX_TILES = ATTN_TC05_MAX_SEQLEN / AT_BM;
+constexpr int AT_POLY = 6;                        // of 16 pairs of exponentials, this many on the FMA pipe
 constexpr float AT_LOG2E = 1.4426950408889634f;
-constexpr int AT_Q_BYTES = 128 * AT_D * 2;
-// tensor-memory columns of a group: two score buffers (P re-uses the first half of its S), O|l
-constexpr int AT_TM_S = 0, AT_TM_O = 2 * AT_BK, AT_TMEM_GROUP = 128;
-static_assert(AT_TM_O + 32 <= AT_TMEM_GROUP, "two score buffers and the output fit a group's columns");
-constexpr int AT_PAD_ROWS = AT_BK;          // zero rows behind the last 128-row block (key blocks of 48)
-constexpr int AT_TMEM_COLS = AT_TMEM_GROUP * AT_WG;
-static_assert(AT_TMEM_COLS == 512, "the CTA takes the whole tensor memory of its SM");
-// mbarriers of a group
-constexpr int AT_BAR_Q = 0, AT_BAR_S = 1 /* two */, AT_BAR_P = 3, AT_BAR_PV = 4, AT_BARS_PER_WG = 5;
-constexpr int AT_NBAR = AT_BARS_PER_WG * AT_WG + AT_KV_BLOCKS;
+constexpr float AT_BOUND = 80.f;                  // largest |score| (exp2 domain) taken without a reference value
+constexpr int AT_Q_BYTES = AT_BM * AT_D * 2;
+constexpr int AT_TM_GROUP = AT_BK + 32, AT_TM_O = AT_BK;
+static_assert(AT_TM_GROUP * AT_GROUPS <= 512, "tensor memory");
 
-// shared-memory map for a patch padded to lpad keys
+// mbarriers of a group, and of the CTA behind those of the groups
+constexpr int AT_B_QFULL = 0, AT_B_QFREE = 2, AT_B_S = 4, AT_B_P = 5, AT_B_O = 6, AT_B_DONE = 7, AT_B_GROUP = 8;
+constexpr int AT_B_V = AT_B_GROUP * AT_GROUPS, AT_B_KVFREE = AT_B_V + 2, AT_NBAR = AT_B_V + 4;
+
+// shared-memory map for patches padded to lpad (a multiple of 128) keys
 struct AtLayout {
-    int off_k, off_v, off_q, off_bar, total;
+    int plane, slot, off_q, off_src, off_qrow, off_flag, off_kn, off_bar, total;
     __host__ __device__ explicit AtLayout(int lpad)
     {
-        const int rows = lpad + AT_PAD_ROWS;
-        off_k = 0;                      // 2 planes of 16-byte chunks
-        off_v = off_k + rows * 32;      // 4 planes: V d 0-7, V d 8-15, the ones column, zeros
-        off_q = off_v + rows * 64;
-        off_bar = off_q + AT_WG * AT_Q_BYTES;
+        plane = lpad * 16;                          // a 16-byte chunk of every key
+        slot = 5 * plane;                           // V d 0-7, V d 8-15, ones, K d 0-7, K d 8-15
+        off_q = 2 * slot;
+        off_src = off_q + AT_GROUPS * 2 * AT_Q_BYTES;
+        off_qrow = off_src + lpad * 4;
+        off_flag = off_qrow + AT_GROUPS * 2 * AT_BM * 4;
+        off_kn = off_flag + AT_GROUPS * 2 * 16;
+        off_bar = off_kn + 2 * 16;
         total = off_bar + 8 * AT_NBAR + 16;
     }
 };
 
-// Descriptor of a no-swizzle operand: `lbo` / `sbo` are the leading / stride byte
-// offsets of the canonical layouts (K-major: lbo between the two 8-element halves of
-// K = 16, sbo between 8-row groups; MN-major: lbo between 8-deep K groups, sbo
-// between 8-element chunks along M/N).
+// Descriptor of a no-swizzle operand: `lbo` / `sbo` are the leading / stride byte offsets of the canonical layouts
+// (K-major: lbo between the two 8-element halves of K = 16, sbo between 8-row groups; MN-major: lbo between 8-deep K
+// groups, sbo between 8-element chunks along M/N).
 __device__ __forceinline__ uint64_t umma_desc_plain(uint32_t smem_addr, uint32_t lbo, uint32_t sbo)
 {
     uint64_t d = 0;
@@ -121,10 +106,6 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
         ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"((uint32_t)accumulate)
         : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint32_t bar)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
 
 __device__ __forceinline__ uint32_t at_scale_bf16x2(uint32_t v, float s)
 {
@@ -132,435 +113,569 @@ __device__ __forceinline__ uint32_t at_scale_bf16x2(uint32_t v, float s)
     return pack_bf16(f.x * s, f.y * s);
 }
 
-__device__ __forceinline__ float max3(float a, float b, float c) { return fmaxf(fmaxf(a, b), c); }
-
-// waits until this thread's cp.async groups, except the newest `pending`, have landed
-__device__ __forceinline__ void cp_async_wait_pending(int pending)
+// exp2(s log2e) of a pair on the FMA pipe, |s log2e| <= AT_BOUND: n = round(s log2e) by adding 1.5 * 2^23, 2^r on
+// [-0.5, 0.5] by the degree-4 polynomial of least relative error (2.7e-6 with its coefficients in fp32), n added to
+// the exponent field.
+struct AtPoly {
+    uint64_t log2e, magic, neg_one, c4, c3, c2, c1, c0;
+    __device__ __forceinline__ AtPoly()
+    {
+        log2e = pack2(AT_LOG2E, AT_LOG2E);
+        magic = pack2(12582912.f, 12582912.f);
+        neg_one = pack2(-1.f, -1.f);
+        c4 = pack2(0.009570102207362652f, 0.009570102207362652f);
+        c3 = pack2(0.05591785907745361f, 0.05591785907745361f);
+        c2 = pack2(0.240247443318367f, 0.240247443318367f);
+        c1 = pack2(0.6931217908859253f, 0.6931217908859253f);
+        c0 = pack2(0.9999992847442627f, 0.9999992847442627f);
+    }
+};
+__device__ __forceinline__ uint32_t at_exp2_poly(uint64_t s2, const AtPoly& k)
 {
-    switch (pending) {
-        case 0: cp_async_wait<0>(); break;
-        case 1: cp_async_wait<1>(); break;
-        case 2: cp_async_wait<2>(); break;
-        case 3: cp_async_wait<3>(); break;
-        case 4: cp_async_wait<4>(); break;
-        case 5: cp_async_wait<5>(); break;
-        case 6: cp_async_wait<6>(); break;
-        default: cp_async_wait<7>(); break;
+    const uint64_t t2 = fma2(s2, k.log2e, k.magic);
+    const uint64_t r2 = fma2(s2, k.log2e, fma2(t2, k.neg_one, k.magic));
+    uint64_t p2 = fma2(r2, k.c4, k.c3);
+    p2 = fma2(p2, r2, k.c2);
+    p2 = fma2(p2, r2, k.c1);
+    p2 = fma2(p2, r2, k.c0);
+    float px, py, tx, ty;
+    unpack2(p2, px, py);
+    unpack2(t2, tx, ty);
+    px = __int_as_float(__float_as_int(px) + (__float_as_int(tx) << 23));
+    py = __int_as_float(__float_as_int(py) + (__float_as_int(ty) << 23));
+    return pack_bf16(px, py);
+}
+
+// 16 scores of a row -> 8 packed probabilities; CH: number of the chunk in its block
+template <int CH>
+__device__ __forceinline__ void at_probabilities(const uint32_t (&s)[16], uint32_t (&pk)[8], const AtPoly& k)
+{
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint64_t s2 = pack2u(s[2 * i], s[2 * i + 1]);
+        if (((8 * (CH & 1) + i) * AT_POLY) % 16 < AT_POLY) {          // AT_POLY of 16, spread evenly
+            pk[i] = at_exp2_poly(s2, k);
+        } else {
+            float x, y;
+            unpack2(mul2(s2, k.log2e), x, y);
+            pk[i] = pack_bf16(fast_exp2(x), fast_exp2(y));
+        }
+    }
+}
+__device__ __forceinline__ void tmem_ld16_fence(uint32_t (&r)[16])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
+                 :
+                 : "memory");
+}
+// chunk CH of a block of NCH: x holds it (in flight), y takes the next one
+template <int CH, int NCH>
+__device__ __forceinline__ void at_chunks(uint32_t (&x)[16], uint32_t (&y)[16], uint32_t tm_s, const AtPoly& k)
+{
+    uint32_t pk[8];
+    tmem_ld16_fence(x);
+    if (CH + 1 < NCH) tmem_ld16(tm_s + 16 * (CH + 1), y);
+    at_probabilities<CH>(x, pk, k);
+    tmem_st8(tm_s + 8 * CH, pk);
+    if constexpr (CH + 1 < NCH) at_chunks<CH + 1, NCH>(y, x, tm_s, k);
+}
+// the same with a reference value (mb = -m log2e) and `valid` real keys
+__device__ __forceinline__ void at_probabilities_ref(const uint32_t (&s)[16], uint32_t (&pk)[8], float mb, int valid)
+{
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float x = fast_exp2(fmaf(__uint_as_float(s[2 * i]), AT_LOG2E, mb));
+        const float y = fast_exp2(fmaf(__uint_as_float(s[2 * i + 1]), AT_LOG2E, mb));
+        pk[i] = pack_bf16(2 * i < valid ? x : 0.f, 2 * i + 1 < valid ? y : 0.f);
     }
 }
 
-__global__ void __launch_bounds__(AT_THREADS, 1) attn_tc05_d16_kernel(
-    const __nv_bfloat16* __restrict__ qkv, const int64_t* __restrict__ order,
-    const int64_t* __restrict__ pad, const int64_t* __restrict__ unpad,
-    const int32_t* __restrict__ cu_seqlens, __nv_bfloat16* __restrict__ out, int C, float scale,
-    int lpad_max, uint32_t* __restrict__ status)
+struct AtArgs {
+    const __nv_bfloat16* qkv;
+    const int64_t *order, *pad, *unpad;
+    const int32_t* cu;
+    __nv_bfloat16* out;
+    int n_seq, heads, tiles, lpad;
+    float scale;
+    bool planned;                 // the geometry may be read before the wait for the kernel ahead (see linear.cuh)
+    uint32_t* status;
+};
+
+// The CTA's tiles, pair after pair.  Every role walks them by itself, in the same order.
+struct AtWalk {
+    const AtArgs* a;
+    int w0, w1, pair, last, seq, head, start, L, lo, hi, counted, before;
+    __device__ __forceinline__ explicit AtWalk(const AtArgs& args) : a(&args)
+    {
+        const int64_t total = (int64_t)a->n_seq * a->heads * a->tiles;
+        w0 = (int)(total * blockIdx.x / gridDim.x);
+        w1 = (int)(total * (blockIdx.x + 1) / gridDim.x);
+        pair = w0 / a->tiles - 1;
+        last = w1 > w0 ? (w1 - 1) / a->tiles : pair;
+        counted = -1;
+        before = lo = hi = 0;
+    }
+    // next pair with tiles of this CTA: `counted` is its number, `before` the tiles of those ahead of it
+    __device__ __forceinline__ bool next(bool report = false)
+    {
+        before += hi - lo;
+        lo = hi = 0;
+        while (++pair <= last) {
+            seq = pair / a->heads;
+            head = pair - seq * a->heads;
+            start = __shfl_sync(0xffffffffu, a->cu[seq], 0);
+            L = __shfl_sync(0xffffffffu, a->cu[seq + 1], 0) - start;
+            // a patch that the caller's max_seqlen does not cover is reported and skipped
+            if (L > a->lpad) {
+                if (report) atomicOr(a->status, PTV3_STATUS_BAD_INDEX);
+                continue;
+            }
+            lo = max(w0 - pair * a->tiles, 0);
+            hi = min(w1 - pair * a->tiles, L <= 0 ? 0 : (L + AT_BM - 1) / AT_BM);
+            if (hi > lo) {
+                ++counted;
+                return true;
+            }
+            lo = hi = 0;
+        }
+        return false;
+    }
+    // first tile of the pair that is group g's (tile number `before + i - lo` goes to group number % 3)
+    __device__ __forceinline__ int first(int g) const
+    {
+        return lo + (g + AT_GROUPS - before % AT_GROUPS) % AT_GROUPS;
+    }
+    __device__ __forceinline__ int blocks() const { return (L + AT_BK - 1) / AT_BK; }
+    // 16-key steps of the last block
+    __device__ __forceinline__ int tail() const { return ((L - 1) % AT_BK + 16) / 16; }
+};
+
+__global__ void __launch_bounds__(AT_THREADS, 1) attn_tc05_d16_kernel(const AtArgs a)
 {
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 127) & ~(uintptr_t)127);
-    const AtLayout lay(lpad_max);
+    const AtLayout lay(a.lpad);
     const uint32_t sbase = smem_u32_generic(smem);
-
-    // heads and query slices vary fastest over the grid (blockIdx.x = slice * heads + head): the
-    // CTAs of one patch run together, so the rows they all gather from (a row holds every head's
-    // q, k and v side by side) are fetched from DRAM once
-    const int n_heads = C / 16;
-    const int seq = blockIdx.y, h = blockIdx.x % n_heads;
-    const int slice = blockIdx.x / n_heads, n_slices = gridDim.x / n_heads;
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int start = cu_seqlens[seq];
-    const int L = cu_seqlens[seq + 1] - start;
-    // uniform over the CTA, and before anything is allocated
-    if (L <= 0) return;
-    if (L > lpad_max) {   // the caller's max_seqlen does not cover this patch
-        if (tid == 0) atomicOr(status, PTV3_STATUS_BAD_INDEX);
-        return;
-    }
-    const int ntiles = (L + AT_BM - 1) / AT_BM;      // query tiles
-    const int nkv = ntiles;                          // gather blocks (128 keys, zero padded)
-    const int nb = (L + AT_BK - 1) / AT_BK;          // key blocks of pass 2
-    const int Lp = ntiles * AT_BM;                   // rows covered by the gather blocks
-    const int Lk = max(Lp, nb * AT_BK);              // rows of the zero-padded K / V planes
-    const int tiles_per_slice = (ntiles + n_slices - 1) / n_slices;
-    const int tile_lo = slice * tiles_per_slice;
-    const int tile_hi = min(ntiles, tile_lo + tiles_per_slice);
-    if (tile_lo >= tile_hi) return;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int C = a.heads * AT_D;
     const int64_t row_stride = 3 * (int64_t)C;
 
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + lay.off_bar);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + AT_NBAR);
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const uint32_t bar0 = sbase + lay.off_bar;
-    const uint32_t kvbar0 = bar0 + 8 * AT_BARS_PER_WG * AT_WG;
+    const uint32_t vbar = bar0 + 8 * AT_B_V, kvfree = bar0 + 8 * AT_B_KVFREE;
+    int32_t* qrow = reinterpret_cast<int32_t*>(smem + lay.off_qrow);      // [group][slot][128]
+    uint32_t* qflag = reinterpret_cast<uint32_t*>(smem + lay.off_flag);   // [group][slot][4]
+    float* kn_s = reinterpret_cast<float*>(smem + lay.off_kn);            // [slot][4]
 
     if (tid == 0) {
-        for (int g = 0; g < AT_WG; ++g) {
-            const uint32_t b = bar0 + 8 * AT_BARS_PER_WG * g;
-            mbar_init(b + 8 * AT_BAR_Q, 4);      // one arrival per warp of the group
-            mbar_init(b + 8 * AT_BAR_S, 1);
-            mbar_init(b + 8 * (AT_BAR_S + 1), 1);
-            mbar_init(b + 8 * AT_BAR_PV, 1);
-            mbar_init(b + 8 * AT_BAR_P, 4);
+        for (int g = 0; g < AT_GROUPS; ++g) {
+            const uint32_t b = bar0 + 8 * AT_B_GROUP * g;
+            for (int s = 0; s < 2; ++s) {
+                mbar_init(b + 8 * (AT_B_QFULL + s), 4);       // a loading warp each
+                mbar_init(b + 8 * (AT_B_QFREE + s), 4);       // a softmax warp each
+            }
+            mbar_init(b + 8 * AT_B_S, 1);
+            mbar_init(b + 8 * AT_B_P, 4);
+            mbar_init(b + 8 * AT_B_O, 1);
+            mbar_init(b + 8 * AT_B_DONE, 1);
         }
-        for (int b = 0; b < AT_KV_BLOCKS; ++b) mbar_init(kvbar0 + 8 * b, 32 * AT_WG);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(vbar + 8 * s, 4);
+            mbar_init(kvfree + 8 * s, 4 * AT_GROUPS);
+        }
         *abort = 0;
         fence_barrier_init();
     }
-    if (warp == 0) tmem_alloc(sbase + lay.off_bar + 8 * AT_NBAR, AT_TMEM_COLS);
+    if (warp == AT_LOAD_WARP) {
+        tmem_alloc(sbase + lay.off_bar + 8 * AT_NBAR, 512);
+        // only now: the kernel brought up behind this one may take tensor memory and then wait for this one
+        pdl_launch_next();
+    }
+    if (!a.planned) pdl_wait();
     fence_before_sync();
     __syncthreads();
     fence_after_sync();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
 
-    const uint32_t ks = sbase + lay.off_k, vs = sbase + lay.off_v;
-    const uint32_t plane = (uint32_t)Lk * 16;
-    const bool issuer = tid >= AT_SOFTMAX_THREADS;
-    const int wg = issuer ? warp - AT_SOFTMAX_THREADS / 32 : tid >> 7;
-    const int t = tid & 127;
-
-    const uint32_t wbar = bar0 + 8 * AT_BARS_PER_WG * wg;
-    const uint32_t qbar = wbar + 8 * AT_BAR_Q, sbar = wbar + 8 * AT_BAR_S, pbar = wbar + 8 * AT_BAR_P,
-                   pvbar = wbar + 8 * AT_BAR_PV;
-    const uint32_t tm_group = tmem_base + wg * AT_TMEM_GROUP;
-
-    // The issuing warps (one whole warpgroup) need few registers; they hand theirs to the
-    // softmax warpgroups.  The kernel starts with 96 registers per thread (640 threads); the
-    // increase must fit in what the decrease releases, or it would wait for ever:
-    // 128 x (96 - 64) = 4096 >= 512 x (104 - 96) = 4096.
-    static_assert(AT_THREADS == 640, "the setmaxnreg budget below assumes 640 threads at 96 registers");
-    static_assert(AT_WG == 4, "the issuing warps must form one warpgroup for setmaxnreg");
-    if (issuer) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
-        // ---- gather: the 128 issuer threads own one key row of every 128-key block -----------
-        const int a = tid - AT_SOFTMAX_THREADS;     // 0..127
-        {
-            int src[AT_KV_BLOCKS];
+    if (warp == AT_LOAD_WARP || warp >= AT_REST_WARP) {
+        // ---- loading warps: thread t owns rows t, t + 128, ... of every pair ------------------------------------
+        const int lw = warp == AT_LOAD_WARP ? 0 : warp - AT_REST_WARP + 1, t = 32 * lw + lane;
+        int32_t* src_s = reinterpret_cast<int32_t*>(smem + lay.off_src);
+        int ones0 = -1, ones1 = -1;          // rows of the slots' planes of ones
+        int seq = -1;
+        bool waited = false;
+        AtWalk w(a);
+        while (w.next(t == 0)) {
+            const int slot = w.counted & 1, L = w.L, Lk = (L + 15) / 16 * 16;
+            if (w.seq != seq) {
+                // point row of every padded row, negated - 1 where the padded row does not own its point
+                // (borrowed rows); read back by this thread alone
+                seq = w.seq;
+                for (int r = t; r < L; r += 4 * AT_BM) {
+                    int64_t pd[4], src[4], own[4];
 #pragma unroll
-            for (int b = 0; b < AT_KV_BLOCKS; ++b) {
-                const int r = b * AT_KV_BLOCK + a;
-                src[b] = (b < nkv && r < L) ? (int)pad[start + r] : -1;
-            }
+                    for (int i = 0; i < 4; ++i) pd[i] = r + i * AT_BM < L ? a.pad[w.start + r + i * AT_BM] : -1;
 #pragma unroll
-            for (int b = 0; b < AT_KV_BLOCKS; ++b)
-                if (src[b] >= 0) src[b] = (int)order[src[b]];
-#pragma unroll
-            for (int b = 0; b < AT_KV_BLOCKS; ++b) {
-                if (b < nkv) {
-                    const int r = b * AT_KV_BLOCK + a;
-                    // V is extended by a column of ones (and seven of zeros, then a plane of zeros):
-                    // the product P V' also yields the row sums of the rounded probabilities
-                    *reinterpret_cast<uint4*>(smem + lay.off_v + 2 * plane + r * 16) = make_uint4(0x3f80u, 0, 0, 0);
-                    *reinterpret_cast<uint4*>(smem + lay.off_v + 3 * plane + r * 16) = make_uint4(0, 0, 0, 0);
-                    if (src[b] >= 0) {
-                        const __nv_bfloat16* kp = qkv + (int64_t)src[b] * row_stride + C + h * AT_D;
-                        cp_async16(ks + r * 16, kp);
-                        cp_async16(ks + plane + r * 16, kp + 8);
-                        cp_async16(vs + r * 16, kp + C);
-                        cp_async16(vs + plane + r * 16, kp + C + 8);
-                    } else {
-                        const uint4 z = make_uint4(0, 0, 0, 0);
-                        *reinterpret_cast<uint4*>(smem + lay.off_k + r * 16) = z;
-                        *reinterpret_cast<uint4*>(smem + lay.off_k + plane + r * 16) = z;
-                        *reinterpret_cast<uint4*>(smem + lay.off_v + r * 16) = z;
-                        *reinterpret_cast<uint4*>(smem + lay.off_v + plane + r * 16) = z;
+                    for (int i = 0; i < 4; ++i) {
+                        src[i] = pd[i] >= 0 ? a.order[pd[i]] : 0;
+                        own[i] = pd[i] >= 0 ? a.unpad[pd[i]] : 0;
                     }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (pd[i] >= 0)
+                            src_s[r + i * AT_BM] = own[i] == w.start + r + i * AT_BM ? (int32_t)src[i] : -(int32_t)src[i] - 1;
                 }
-                cp_async_commit();      // one group per block, empty ones included
             }
-            // key blocks are 48 rows: the last one may reach behind the last gather block
-            if (Lp + a < Lk) {
-                const int r = Lp + a;
-                const uint4 z = make_uint4(0, 0, 0, 0);
+            // (planned: so far only the geometry was read)
+            if (!waited) pdl_wait();
+            waited = true;
+            if (w.counted >= 2) mbar_wait(kvfree + 8 * slot, ((w.counted >> 1) - 1) & 1, abort);
+
+            unsigned char* vs = smem + slot * lay.slot;
+            unsigned char* ks = vs + 3 * lay.plane;
+            const uint32_t vs_a = sbase + slot * lay.slot, ks_a = vs_a + 3 * lay.plane;
+            auto row_of = [&](int r) {
+                const int32_t e = src_s[r];
+                return (int64_t)(e >= 0 ? e : -(e + 1)) * row_stride + w.head * AT_D;
+            };
+            const uint4 zero = make_uint4(0, 0, 0, 0);
 #pragma unroll
-                for (int pl = 0; pl < 2; ++pl) *reinterpret_cast<uint4*>(smem + lay.off_k + pl * plane + r * 16) = z;
-#pragma unroll
-                for (int pl = 0; pl < 4; ++pl) *reinterpret_cast<uint4*>(smem + lay.off_v + pl * plane + r * 16) = z;
+            for (int i = 0; i < AT_MAX_TILES; ++i) {
+                const int r = i * AT_BM + t;
+                if (i * AT_BM >= Lk) break;
+                if (r < L) {
+                    const __nv_bfloat16* kp = a.qkv + row_of(r) + C;
+                    cp_async16(ks_a + r * 16, kp);
+                    cp_async16(ks_a + lay.plane + r * 16, kp + 8);
+                } else if (r < Lk) {
+                    *reinterpret_cast<uint4*>(ks + r * 16) = zero;
+                    *reinterpret_cast<uint4*>(ks + lay.plane + r * 16) = zero;
+                }
             }
-        }
-        // ---- one warp per group: waits for the group's mbarriers, lane 0 issues ----------
-        const bool lead = (tid & 31) == 0;
-        constexpr uint32_t IDESC_S = umma_idesc_bf16(128, AT_BK);
-        constexpr uint32_t IDESC_R = umma_idesc_bf16(128, 32) | (1u << 16);   // B is MN-major
-        // S = Q K_j^T: A = Q planes [d half][row], B = K planes [d half][key]
-        const uint64_t desc_q = umma_desc_plain(sbase + lay.off_q + wg * AT_Q_BYTES, AT_BM * 16, 128);
-        const uint64_t desc_k = umma_desc_plain(ks, plane, 128);
-        // O|l += P V': A = P (tensor memory), B = V' planes [d chunk][key]
-        const uint64_t desc_v = umma_desc_plain(vs, 128, plane);
-        uint32_t qph = 0, pph = 0;
-        int landed = 0;      // gather blocks handed over so far
-        // this thread's copies of the gather blocks up to the one holding key row `row` have
-        // landed: tell the tensor-core proxy and the other issuing warps, then wait for theirs
-        auto land_upto = [&](int row) {
-            const int need = min(row / AT_KV_BLOCK, nkv - 1);
-            while (landed <= need) {
-                cp_async_wait_pending(AT_KV_BLOCKS - 1 - landed);
+            cp_async_commit();
+            // query row of the pair's first tile
+            uint4 q0 = zero, q1 = zero;
+            auto fetch_q = [&](int tile) {
+                const int r = tile * AT_BM + t;
+                q0 = q1 = zero;
+                if (tile < w.hi && r < L) {
+                    const uint4* qp = reinterpret_cast<const uint4*>(a.qkv + row_of(r));
+                    q0 = qp[0];
+                    q1 = qp[1];
+                }
+            };
+            fetch_q(w.lo);
+#pragma unroll
+            for (int i = 0; i < AT_MAX_TILES; ++i) {
+                const int r = i * AT_BM + t;
+                if (i * AT_BM >= Lk) break;
+                if (r < L) {
+                    const __nv_bfloat16* vp = a.qkv + row_of(r) + 2 * C;
+                    cp_async16(vs_a + r * 16, vp);
+                    cp_async16(vs_a + lay.plane + r * 16, vp + 8);
+                } else if (r < Lk) {
+                    *reinterpret_cast<uint4*>(vs + r * 16) = zero;
+                    *reinterpret_cast<uint4*>(vs + lay.plane + r * 16) = zero;
+                }
+            }
+            cp_async_commit();
+            if ((slot ? ones1 : ones0) != L) {
+                (slot ? ones1 : ones0) = L;
+                for (int r = t; r < Lk; r += AT_BM)
+                    *reinterpret_cast<uint4*>(vs + 2 * lay.plane + r * 16) = make_uint4(r < L ? 0x3f80u : 0u, 0, 0, 0);
+            }
+            // largest squared norm of a key (every thread reads back the rows it copied itself)
+            cp_async_wait<1>();
+            float kn = 0.f;
+            for (int r = t; r < L; r += AT_BM)
+                kn = max_nan(kn, sq_norm16(*reinterpret_cast<const uint4*>(ks + r * 16),
+                                           *reinterpret_cast<const uint4*>(ks + lay.plane + r * 16)));
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) kn = max_nan(kn, __shfl_xor_sync(0xffffffffu, kn, d));
+            if (lane == 0) kn_s[slot * 4 + lw] = kn;
+            named_barrier(1, 128);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) kn = max_nan(kn, kn_s[slot * 4 + i]);
+
+            const float lim = (AT_BOUND / AT_LOG2E) * (AT_BOUND / AT_LOG2E);
+            for (int tile = w.lo; tile < w.hi; ++tile) {
+                const int number = w.before + tile - w.lo, g = number % AT_GROUPS, k = number / AT_GROUPS, qs = k & 1;
+                const uint32_t gbar = bar0 + 8 * AT_B_GROUP * g;
+                if (k >= 2) mbar_wait(gbar + 8 * (AT_B_QFREE + qs), ((k >> 1) - 1) & 1, abort);
+                uint4 s0, s1;
+                s0.x = at_scale_bf16x2(q0.x, a.scale); s0.y = at_scale_bf16x2(q0.y, a.scale);
+                s0.z = at_scale_bf16x2(q0.z, a.scale); s0.w = at_scale_bf16x2(q0.w, a.scale);
+                s1.x = at_scale_bf16x2(q1.x, a.scale); s1.y = at_scale_bf16x2(q1.y, a.scale);
+                s1.z = at_scale_bf16x2(q1.z, a.scale); s1.w = at_scale_bf16x2(q1.w, a.scale);
+                unsigned char* qp = smem + lay.off_q + (g * 2 + qs) * AT_Q_BYTES;
+                *reinterpret_cast<uint4*>(qp + t * 16) = s0;
+                *reinterpret_cast<uint4*>(qp + AT_Q_BYTES / 2 + t * 16) = s1;
+                const int r = tile * AT_BM + t;
+                qrow[(g * 2 + qs) * AT_BM + t] = r < L ? src_s[r] : -1;
+                // (a NaN fails the test)
+                const bool bounded = sq_norm16(s0, s1) * kn <= lim;
+                const uint32_t flag = __all_sync(0xffffffffu, bounded) ? 0u : 1u;
+                if (lane == 0) qflag[(g * 2 + qs) * 4 + lw] = flag;
+                fetch_q(tile + 1);
+                // (this and, with a pair's first tile, K: in every warp ahead of V, and V ahead of the next pair's K)
                 fence_proxy_async();
-                mbar_arrive(kvbar0 + 8 * landed);
-                mbar_wait(kvbar0 + 8 * landed, 0, abort);
-                ++landed;
-            }
-        };
-        auto issue_s = [&](int jj) {      // S_jj = Q K_jj^T into buffer jj & 1
-            // a descriptor's low word holds the address / 16: blocks are AT_BK chunks apart
-            umma_bf16(tm_group + AT_TM_S + (jj & 1) * AT_BK, desc_q, desc_k + (uint64_t)(jj * AT_BK), IDESC_S, false);
-            umma_commit(sbar + 8 * (jj & 1));
-        };
-        for (int tile = tile_lo + wg; tile < tile_hi; tile += AT_WG) {
-            mbar_wait(qbar, qph, abort);
-            qph ^= 1;
-            land_upto(min(2, nb) * AT_BK - 1);
-            if (lead) {
-                fence_after_sync();
-                issue_s(0);
-                if (nb > 1) issue_s(1);
-            }
-            __syncwarp();
-            for (int j = 0; j < nb; ++j) {
-                mbar_wait(pbar, pph, abort);    // P_j is in tensor memory (over the first half of S_j)
-                pph ^= 1;
-                if (j + 2 < nb) land_upto((j + 3) * AT_BK - 1);
-                if (lead) {
-                    fence_after_sync();
-                    const uint64_t dv = desc_v + (uint64_t)(j * AT_BK);
-                    const uint32_t tm_p = tm_group + AT_TM_S + (j & 1) * AT_BK;
-#pragma unroll
-                    for (int i = 0; i < AT_BK / 16; ++i)
-                        umma_bf16_ts(tm_group + AT_TM_O, tm_p + 8 * i, dv + 16 * i, IDESC_R, j > 0 || i > 0);
-                    umma_commit(pvbar);
-                    // the next product into this buffer runs after the ones above, which read it
-                    if (j + 2 < nb) issue_s(j + 2);
-                }
                 __syncwarp();
+                if (lane == 0) mbar_arrive_one(gbar + 8 * (AT_B_QFULL + qs));
+                if (tile == w.lo) {
+                    cp_async_wait<0>();
+                    fence_proxy_async();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_one(vbar + 8 * slot);
+                }
             }
         }
-        const bool kv_landed = landed >= nkv;
-        if (!kv_landed) {
-            // a warp whose group has no tile in this CTA (or a patch shorter than its planes): its
-            // share of the gather still has to be handed over, the other issuing warps wait for it
-            for (int jb = landed; jb < nkv; ++jb) {
-                cp_async_wait_pending(AT_KV_BLOCKS - 1 - jb);
-                fence_proxy_async();
-                mbar_arrive(kvbar0 + 8 * jb);
-            }
-        }
+        if (!waited) pdl_wait();          // (no CTA ends before the kernel ahead has: the one behind relies on it)
         cp_async_wait<0>();
-    } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
-        // ---- softmax groups: thread t owns query row t of the tile ---------------------
-        unsigned char* qs_ptr = smem + lay.off_q + wg * AT_Q_BYTES;
-        const uint32_t tm_lane = (uint32_t)((warp & 3) * 32) << 16;
-        const uint32_t tm_s0 = tm_group + tm_lane + AT_TM_S, tm_o = tm_group + tm_lane + AT_TM_O;
-        uint32_t sph0 = 0, sph1 = 0, pvph = 0;
-        const Exp2Const kexp;
-
-        // pad -> order -> q row of this thread's row in the group's NEXT tile is walked one level
-        // per key block while the current tile is computed
-        int pd = 0, src = 0, pd_next = 0, src_next = 0;
-        {
-            const int r = (tile_lo + wg) * AT_BM + t;
-            if (tile_lo + wg < tile_hi && r < L) {
-                pd = (int)pad[start + r];
-                src = (int)order[pd];
+    } else if (warp < AT_GROUPS) {
+        // ---- issuing warp of group g ------------------------------------------------------------------------------
+        const int g = warp;
+        const uint32_t gbar = bar0 + 8 * AT_B_GROUP * g;
+        const uint32_t tm = tmem_base + g * AT_TM_GROUP;
+        constexpr uint32_t IDESC_S = umma_idesc_bf16(AT_BM, AT_BK);
+        constexpr uint32_t IDESC_O = umma_idesc_bf16(AT_BM, 32) | (1u << 16);   // B is MN-major
+        // A = Q planes [d half][row], B = K planes [d half][key]
+        const uint64_t desc_q = umma_desc_plain(sbase + lay.off_q + g * 2 * AT_Q_BYTES, AT_Q_BYTES / 2, 128);
+        const uint64_t desc_k = umma_desc_plain(sbase + 3 * lay.plane, lay.plane, 128);
+        // B = planes [d chunk][key]: V, V, ones, and K's first (columns that nobody reads)
+        const uint64_t desc_v = umma_desc_plain(sbase, 128, lay.plane);
+        uint32_t pphase = 0;
+        int k = 0;                    // tiles so far
+        AtWalk w(a);
+        while (w.next()) {
+            const int nb = w.blocks(), tail = w.tail();
+            const uint32_t vparity = (w.counted >> 1) & 1, vb = vbar + 8 * (w.counted & 1);
+            const uint64_t slot = w.counted & 1 ? lay.slot >> 4 : 0;
+            for (int tile = w.first(g); tile < w.hi; tile += AT_GROUPS, ++k) {
+                mbar_wait(gbar + 8 * (AT_B_QFULL + (k & 1)), (k >> 1) & 1, abort);      // and K of the pair
+                const uint4 f = *reinterpret_cast<const uint4*>(qflag + (g * 2 + (k & 1)) * 4);
+                const uint64_t dq = desc_q + (k & 1) * (AT_Q_BYTES >> 4);
+                const uint64_t dk = desc_k + slot;
+                uint64_t dv = desc_v + slot;
+                // P V' of a full block, or of the tile's last one
+                auto issue_pv = [&](bool first, int steps) {
+                    if (steps == AT_BK / 16) {
+#pragma unroll
+                        for (int i = 0; i < AT_BK / 16; ++i)
+                            umma_bf16_ts(tm + AT_TM_O, tm + 8 * i, dv + 16 * i, IDESC_O, !first || i > 0);
+                    } else {
+                        for (int i = 0; i < steps; ++i)
+                            umma_bf16_ts(tm + AT_TM_O, tm + 8 * i, dv + 16 * i, IDESC_O, !first || i > 0);
+                    }
+                };
+                auto issue_s = [&](int j) {
+                    const uint32_t idesc = j + 1 < nb ? IDESC_S : umma_idesc_bf16(AT_BM, 16 * tail);
+                    umma_bf16(tm, dq, dk + (uint64_t)(j * AT_BK), idesc, false);
+                    umma_commit(gbar + 8 * AT_B_S);
+                };
+                auto wait_p = [&]() {
+                    mbar_wait(gbar + 8 * AT_B_P, pphase, abort);
+                    pphase ^= 1;
+                    __syncwarp();
+                };
+                __syncwarp();
+                if ((f.x | f.y | f.z | f.w) != 0)           // the scores once for their maxima
+                    for (int j = 0; j < nb; ++j) {
+                        if (elect_one()) {
+                            fence_after_sync();
+                            issue_s(j);
+                        }
+                        wait_p();
+                    }
+                if (elect_one()) {
+                    fence_after_sync();
+                    issue_s(0);
+                }
+                __syncwarp();
+                // (the pair before in this slot is complete: its V was there before this tile's Q)
+                mbar_wait(vb, vparity, abort);
+                for (int j = 0; j + 1 < nb; ++j) {
+                    wait_p();
+                    if (elect_one()) {
+                        fence_after_sync();
+                        issue_pv(j == 0, AT_BK / 16);
+                        issue_s(j + 1);
+                    }
+                    __syncwarp();
+                    dv += AT_BK;
+                }
+                wait_p();
+                if (elect_one()) {
+                    fence_after_sync();
+                    issue_pv(nb == 1, tail);
+                    umma_commit(gbar + 8 * AT_B_O);
+                }
+                __syncwarp();
             }
         }
-        for (int tile = tile_lo + wg; tile < tile_hi; tile += AT_WG) {
-            const int r = tile * AT_BM + t;
-            const bool ok = r < L;
-            if (tile != tile_lo + wg) {
-                pd = pd_next;
-                src = src_next;
-            }
-            uint4 q0 = make_uint4(0, 0, 0, 0), q1 = q0;
-            if (ok) {
-                const uint4* qp = reinterpret_cast<const uint4*>(qkv + (int64_t)src * row_stride + h * AT_D);
-                q0 = qp[0];
-                q1 = qp[1];
-                q0.x = at_scale_bf16x2(q0.x, scale); q0.y = at_scale_bf16x2(q0.y, scale);
-                q0.z = at_scale_bf16x2(q0.z, scale); q0.w = at_scale_bf16x2(q0.w, scale);
-                q1.x = at_scale_bf16x2(q1.x, scale); q1.y = at_scale_bf16x2(q1.y, scale);
-                q1.z = at_scale_bf16x2(q1.z, scale); q1.w = at_scale_bf16x2(q1.w, scale);
-            }
-            // used at the end of the tile only
-            const bool own = ok && unpad[pd] == start + r;
-            const int rn = r + AT_WG * AT_BM;
-            const bool okn = tile + AT_WG < tile_hi && rn < L;
-            if (okn) pd_next = (int)pad[start + rn];
-            // every product that read the previous tile's Q has completed (its O was awaited)
-            *reinterpret_cast<uint4*>(qs_ptr + t * 16) = q0;
-            *reinterpret_cast<uint4*>(qs_ptr + 2048 + t * 16) = q1;
-            fence_proxy_async();
-            // one arrival per warp: 128 arrivals on one mbarrier are 128 updates of one shared-memory
-            // word, one after the other
-            __syncwarp();
-            if ((tid & 31) == 0) mbar_arrive(qbar);
-
-            float m = -INFINITY;     // reference value of the exponentials (raw score units)
-            float mb = 0.f;          // -m * log2(e)
-            for (int j = 0; j < nb; ++j) {
-                const int buf = j & 1;
-                const uint32_t tm_s = tm_s0 + buf * AT_BK;
-                if (buf) {
-                    mbar_wait(sbar + 8, sph1, abort);
-                    sph1 ^= 1;
-                } else {
-                    mbar_wait(sbar, sph0, abort);
-                    sph0 ^= 1;
-                }
-                fence_after_sync();
-                float v[AT_BK];
-                {
-                    uint32_t* u = reinterpret_cast<uint32_t*>(v);
-#pragma unroll
-                    for (int c = 0; c < AT_BK / 16; ++c) tmem_ld16(tm_s + 16 * c, u + 16 * c);
-                    tmem_ld_wait();
-                }
-                const int valid = L - j * AT_BK;
-                if (valid < AT_BK) {
-#pragma unroll
-                    for (int i = 0; i < AT_BK; ++i)
-                        if (i >= valid) v[i] = -INFINITY;
-                }
-                float mx0 = v[0], mx1 = v[1], mx2 = v[2], mx3 = v[3];
-#pragma unroll
-                for (int i = 4; i < AT_BK; i += 8) {
-                    mx0 = max3(mx0, v[i], v[i + 1]);
-                    mx1 = max3(mx1, v[i + 2], v[i + 3]);
-                    if (i + 4 < AT_BK) {
-                        mx2 = max3(mx2, v[i + 4], v[i + 5]);
-                        mx3 = max3(mx3, v[i + 6], v[i + 7]);
-                    }
-                }
-                // every block holds at least one real key, so the block maximum is finite
-                const float bm = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
-                const bool raise = (bm - m) * AT_LOG2E > AT_LAZY;     // always on the first block
-                // tensor-memory loads and stores are warp-wide: the rare rescaling is taken by the
-                // whole warp, with factor 1 for the rows that keep their reference value
-                bool pv_awaited = j == 0;
-                if (__any_sync(0xffffffffu, raise)) {
-                    const float mn = raise ? bm : m;
-                    if (j > 0) {
-                        // the product P_j-1 V' may still be running
-                        mbar_wait(pvbar, pvph, abort);
-                        pvph ^= 1;
-                        pv_awaited = true;
-                        fence_after_sync();
-                        const float alpha = raise ? fast_exp2((m - mn) * AT_LOG2E) : 1.f;
-                        uint32_t rr[32];
-                        tmem_ld32(tm_o, rr);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i <= AT_D; ++i) rr[i] = __float_as_uint(__uint_as_float(rr[i]) * alpha);
-                        tmem_st32(tm_o, rr);
-                    }
-                    m = mn;
-                    mb = -m * AT_LOG2E;
-                }
-                uint32_t pk[AT_BK / 2];
-                const uint64_t mb2 = pack2(mb, mb);
-#pragma unroll
-                for (int i = 0; i < AT_BK / 2; ++i) {
-                    const uint64_t x2 = fma2(pack2(v[2 * i], v[2 * i + 1]), kexp.log2e, mb2);
-                    if ((i & 7) < AT_POLY) {
-                        pk[i] = exp2_poly2_bf16(x2, kexp);
-                    } else {
-                        float x, y;
-                        unpack2(x2, x, y);
-                        pk[i] = pack_bf16(fast_exp2(x), fast_exp2(y));
-                    }
-                }
-                // every block consumes one completion of the "P V done" barrier (of the block before
-                // it), here in the common case, where that product has long finished
-                if (!pv_awaited) {
-                    mbar_wait(pvbar, pvph, abort);
-                    pvph ^= 1;
-                }
-                // P over the first half of S_j (all of S_j is in registers)
-#pragma unroll
-                for (int c = 0; c < AT_BK / 16; ++c) tmem_st8(tm_s + 8 * c, pk + 8 * c);
-                tmem_st_wait();
-                fence_before_sync();
-                __syncwarp();
-                if ((tid & 31) == 0) mbar_arrive(pbar);
-                // walk the next tile's pad -> order -> row chain one level per key block
-                if (j == 0 && okn) src_next = (int)order[pd_next];
-                if (j == 1 && okn)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(qkv + (int64_t)src_next * row_stride + h * AT_D));
-            }
-            mbar_wait(pvbar, pvph, abort);      // the last product of the tile
-            pvph ^= 1;
+        // nothing of this warp's is in flight when the CTA ends, whatever happened
+        if (elect_one()) umma_commit(gbar + 8 * AT_B_DONE);
+        __syncwarp();
+        int give_up = 0;
+        mbar_wait(gbar + 8 * AT_B_DONE, 0, &give_up);
+    } else {
+        // ---- softmax: thread t owns query row t of its group's tiles -----------------------------------------------
+        const int g = warp / 4 - 1, t = tid & 127;
+        const uint32_t gbar = bar0 + 8 * AT_B_GROUP * g;
+        const uint32_t tm = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + g * AT_TM_GROUP;
+        const AtPoly poly;
+        uint32_t sphase = 0;
+        int k = 0;               // tiles so far
+        auto wait_s = [&]() {
+            mbar_wait(gbar + 8 * AT_B_S, sphase, abort);
+            sphase ^= 1;
             fence_after_sync();
-            {
-                uint32_t rr[32];
-                tmem_ld32(tm_o, rr);
-                tmem_ld_wait();
-                // the next tile's first product overwrites these columns; it is issued only after
-                // this thread's arrival on the Q barrier, which comes after this load
-                fence_before_sync();
-                if (own) {
-                    const float inv = 1.f / __uint_as_float(rr[16]);
-                    uint4 w0, w1;
-#define AT_O(i) (__uint_as_float(rr[i]) * inv)
-                    w0.x = pack_bf16(AT_O(0), AT_O(1));   w0.y = pack_bf16(AT_O(2), AT_O(3));
-                    w0.z = pack_bf16(AT_O(4), AT_O(5));   w0.w = pack_bf16(AT_O(6), AT_O(7));
-                    w1.x = pack_bf16(AT_O(8), AT_O(9));   w1.y = pack_bf16(AT_O(10), AT_O(11));
-                    w1.z = pack_bf16(AT_O(12), AT_O(13)); w1.w = pack_bf16(AT_O(14), AT_O(15));
-#undef AT_O
-                    uint4* op = reinterpret_cast<uint4*>(out + (int64_t)src * C + h * AT_D);
-                    op[0] = w0;
-                    op[1] = w1;
+        };
+        auto hand_over = [&]() {  // this warp's P (or its reads of S) are done
+            fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_one(gbar + 8 * AT_B_P);
+        };
+        AtWalk w(a);
+        while (w.next()) {
+            const int nb = w.blocks(), tail = w.tail(), L = w.L;
+            for (int tile = w.first(g); tile < w.hi; tile += AT_GROUPS, ++k) {
+                const int qs = k & 1;
+                uint32_t x[16], y[16];
+                wait_s();
+                // (the issuing warp has waited for the Q tile that S was made from)
+                const int32_t e = qrow[(g * 2 + qs) * AT_BM + t];
+                const uint4 f = *reinterpret_cast<const uint4*>(qflag + (g * 2 + qs) * 4);
+                if ((f.x | f.y | f.z | f.w) == 0) {
+                    for (int j = 0; j < nb; ++j) {
+                        if (j) wait_s();
+                        if (j + 1 < nb || tail == AT_BK / 16) {
+                            tmem_ld16(tm, x);
+                            at_chunks<0, AT_BK / 16>(x, y, tm, poly);
+                        } else {
+                            for (int i = 0; i < tail; ++i) {
+                                uint32_t pk[8];
+                                tmem_ld16(tm + 16 * i, x);
+                                tmem_ld16_fence(x);
+                                at_probabilities<0>(x, pk, poly);
+                                tmem_st8(tm + 8 * i, pk);
+                            }
+                        }
+                        tmem_st_wait();
+                        hand_over();
+                    }
+                } else {
+                    float m = -INFINITY;
+                    for (int j = 0; j < nb; ++j) {
+                        if (j) wait_s();
+                        const int steps = j + 1 < nb ? AT_BK / 16 : tail;
+                        for (int i = 0; i < steps; ++i) {
+                            tmem_ld16(tm + 16 * i, x);
+                            tmem_ld16_fence(x);
+                            const int valid = L - j * AT_BK - 16 * i;
+#pragma unroll
+                            for (int c = 0; c < 16; ++c)
+                                if (c < valid) m = fmaxf(m, __uint_as_float(x[c]));
+                        }
+                        hand_over();
+                    }
+                    const float mb = -m * AT_LOG2E;
+                    for (int j = 0; j < nb; ++j) {
+                        wait_s();
+                        const int steps = j + 1 < nb ? AT_BK / 16 : tail;
+                        for (int i = 0; i < steps; ++i) {
+                            uint32_t pk[8];
+                            tmem_ld16(tm + 16 * i, x);
+                            tmem_ld16_fence(x);
+                            at_probabilities_ref(x, pk, mb, L - j * AT_BK - 16 * i);
+                            tmem_st8(tm + 8 * i, pk);
+                        }
+                        tmem_st_wait();
+                        hand_over();
+                    }
+                }
+                mbar_wait(gbar + 8 * AT_B_O, k & 1, abort);
+                fence_after_sync();
+                // (the next tile's first P V overwrites these columns: issued behind this warp's next hand-over)
+                tmem_ld16(tm + AT_TM_O, x);
+                tmem_ld16(tm + AT_TM_O + 16, y);
+                tmem_ld16_fence(x);
+                tmem_ld16_fence(y);
+                __syncwarp();
+                if (lane == 0) mbar_arrive_one(gbar + 8 * (AT_B_QFREE + qs));
+                if (e >= 0) {
+                    const float inv = 1.f / __uint_as_float(y[0]);
+                    uint4 o[2];
+                    uint32_t* ow = reinterpret_cast<uint32_t*>(o);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        ow[i] = pack_bf16(__uint_as_float(x[2 * i]) * inv, __uint_as_float(x[2 * i + 1]) * inv);
+                    uint4* op = reinterpret_cast<uint4*>(a.out + (int64_t)e * C + w.head * AT_D);
+                    op[0] = o[0];
+                    op[1] = o[1];
                 }
             }
+            // this warp's products with K and V of the pair are complete (and a group without a tile in it waits, or it
+            // would count twice for the pair before in this slot)
+            mbar_wait(vbar + 8 * (w.counted & 1), (w.counted >> 1) & 1, abort);
+            __syncwarp();
+            if (lane == 0) mbar_arrive_one(kvfree + 8 * (w.counted & 1));
         }
     }
 
     fence_before_sync();
     __syncthreads();
-    if (tid == 0 && *abort) atomicOr(status, PTV3_STATUS_WAIT_LIMIT);
-    if (warp == 0) {
+    if (tid == 0 && *abort) atomicOr(a.status, PTV3_STATUS_WAIT_LIMIT);
+    if (warp == AT_LOAD_WARP) {
         fence_after_sync();
-        tmem_dealloc(tmem_base, AT_TMEM_COLS);
+        tmem_dealloc(tmem_base, 512);
     }
 }
 
-bool attn_tc05_supported(int channels, int heads, int max_seqlen)
+bool attn_tc05_supported(int n_seq, int channels, int heads, int max_seqlen)
 {
-    return channels % heads == 0 && channels / heads == AT_D && channels % 16 == 0 &&
-           max_seqlen <= ATTN_TC05_MAX_SEQLEN;
+    return channels % heads == 0 && channels / heads == AT_D && max_seqlen <= ATTN_TC05_MAX_SEQLEN &&
+           (int64_t)n_seq * heads * AT_MAX_TILES < (1ll << 31);
+}
+
+// Whether this kernel is faster than the mma.sync one (attention_mma.cu) on n points in n_seq patches.  Three things speak
+// against it: few blocks (a CTA starts with ~7 us of gather, and a group alone on an SM takes 1 800 cycles a block, three
+// together 975 each), short patches (a pair's gather takes the loading warps ~5 us) and rows of a tile that
+// the patch does not have.  us here and there, H heads of 16, blocks of 128 x 128 scores per SM:
+//   patches of 1 024: 8 192 points H 8 (28 blocks) 28.9 / 27.6, 12 288 H 8 (42) 34.7 / 37.9, 100 000 H 4 (169) 102 / 121,
+//     400 000 H 4 (676) 361 / 448;  of 800: 3 200 H 32 (38) 33.9 / 39.0;  of 640: 2 560 H 32 (22) 22.4 / 22.7
+//   of 512: 20 000 H 8 (35) 28.7 / 33.7;  of 384: 30 000 H 8 (38) 34.7 / 35.6, 200 000 H 4 (127) 91.6 / 99.5
+//   of 320: 200 000 H 4 (106) 103 / 88;  of 256: 400 000 H 4 (169) 168 / 146
+bool attn_tc05_wanted(int64_t n, int n_seq, int heads, int max_seqlen)
+{
+    const int64_t mean = (n + n_seq - 1) / n_seq;      // (a caller may state a longer patch than there is)
+    const int64_t len = mean < max_seqlen ? mean : max_seqlen;
+    const int64_t tiles = (len + AT_BM - 1) / AT_BM, steps = (len + 15) / 16;
+    if (len < 384 || (len < 640 && tiles * AT_BM * steps * 16 * 10 > len * len * 11)) return false;
+    return (int64_t)n_seq * heads * tiles * steps >= 33 * SMS * (AT_BK / 16);
 }
 
 int launch_attn_tc05(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad,
                      const int32_t* cu, void* out, int n_seq, int max_seqlen, int C, int H, float scale,
-                     uint32_t* status, cudaStream_t stream)
+                     bool planned, uint32_t* status, cudaStream_t stream)
 {
-    const int lpad = (max_seqlen + AT_BM - 1) / AT_BM * AT_BM;
-    const AtLayout lay(lpad);
+    AtArgs a{(const __nv_bfloat16*)qkv, order, pad, unpad, cu, (__nv_bfloat16*)out, n_seq, H,
+             (max_seqlen + AT_BM - 1) / AT_BM, (max_seqlen + AT_BM - 1) / AT_BM * AT_BM, scale, planned, status};
+    const AtLayout lay(a.lpad);
     // A CTA takes the whole tensor memory of its SM: ask for enough shared memory that no
     // second CTA shares the SM (it would wait in tcgen05.alloc).
     const size_t floor_smem = (size_t)(228 * 1024 / 2 + 1024);
     const size_t smem = lay.total + 128 < floor_smem ? floor_smem : (size_t)lay.total + 128;
     if (allow_smem(attn_tc05_d16_kernel) != cudaSuccess)
         return check_launch("ptv3_attention_fwd: shared memory attribute");
-    // Query tiles of a patch can be sliced over CTAs (each gathers K and V again).  Pick the
-    // slicing with the shortest estimated time: waves of a CTA per SM, each taking one gather
-    // (about 0.2 of a tile round) plus its rounds of up to four tiles.
-    const int tiles = lpad / AT_BM;
-    const long pairs = (long)n_seq * H;
-    int qsplit = 1;
-    double best = 0;
-    for (int q = 1; q <= tiles; q *= 2) {
-        const long waves = (pairs * q + SMS - 1) / SMS;
-        const int rounds = ((tiles + q - 1) / q + AT_WG - 1) / AT_WG;
-        const double cost = (double)waves * (rounds + 0.2);
-        if (q == 1 || cost < best) {
-            best = cost;
-            qsplit = q;
-        }
-    }
-    const dim3 grid(H * qsplit, n_seq);
-    attn_tc05_d16_kernel<<<grid, AT_THREADS, smem, stream>>>(
-        (const __nv_bfloat16*)qkv, order, pad, unpad, cu, (__nv_bfloat16*)out, C, scale, lpad, status);
+    const int64_t total = (int64_t)n_seq * H * a.tiles;
+    const dim3 grid((unsigned)(total < SMS ? total : SMS));
+    launch_dependent(attn_tc05_d16_kernel, grid, dim3(AT_THREADS), smem, stream, a);
     count_launches(1);
     return check_launch("ptv3_attention_fwd");
 }
 
 }  // namespace ptv3
-

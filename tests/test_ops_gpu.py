@@ -254,6 +254,60 @@ def test_attention_tcgen05_path_matches_cuda_core_path(sizes, C, H, K):
         assert rel_l2(b, a) < 5e-3
 
 
+# (more than one pair per CTA from 149 tiles on; patches of up to 128 rows leave groups without a tile in most pairs; ends
+# of a tile, of a block and of a 16-key step)
+@pytest.mark.parametrize("n,H,K", [(1, 1, 1024), (16, 2, 16), (17, 1, 1024), (128, 2, 1024), (129, 2, 1024), (384, 4, 384),
+                                   (1024, 32, 1024), (5000, 8, 40), (40000, 8, 128), (20000, 8, 200), (9000, 16, 385),
+                                   (30000, 4, 1000), (50000, 4, 1024)])
+@pytest.mark.parametrize("gain", [1.0, 12.0])
+def test_attention_tcgen05_tiles_pairs_and_reference_values(n, H, K, gain):
+    """The tcgen05 kernel (algo 4) against the CUDA-core kernel (algo 1): tiles that take their exponentials without a
+    reference value, with one, and (large queries in one half of the points, gain 12) both kinds side by side."""
+    C = 16 * H
+    g = torch.Generator().manual_seed(n)
+    qkv = torch.randn(n, 3 * C, generator=g)
+    qkv[: n // 2, :C] *= gain
+    qkv = qkv.bfloat16().cuda()
+    order = torch.arange(n).cuda() if gain > 1 else torch.randperm(n, generator=g).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    a = ops.attention(qkv, order, pad, unpad, cu, H, min(n, K), 0.25, algo=1)
+    b = ops.attention(qkv, order, pad, unpad, cu, H, min(n, K), 0.25, algo=4)
+    assert_close(b, a, atol=1e-2, rtol=1e-2, what="tcgen05 attention")
+    assert rel_l2(b, a) < 5e-3
+
+
+def test_attention_tcgen05_keeps_nan_and_infinity_in_their_patch():
+    """A NaN key reaches every row of its patch and head, an infinite query its own row, as in the mma.sync kernel, and
+    nothing else."""
+    n, H, K = 4096, 2, 512
+    g = torch.Generator().manual_seed(0)
+    qkv = torch.randn(n, 96, generator=g).bfloat16()
+    qkv[700, 32:48] = float("nan")                 # key of head 0
+    qkv[2000, 16:32] = float("inf")                # query of head 1
+    qkv, order = qkv.cuda(), torch.arange(n).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    a, b = (ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25, algo=i).float() for i in (2, 4))
+    assert torch.equal(torch.isnan(a), torch.isnan(b))
+    assert bool(torch.isnan(b[512:1024, :16]).all()) and bool(torch.isnan(b[2000, 16:]).all())
+    assert int(torch.isnan(b).sum()) == 512 * 16 + 16
+    assert_close(torch.nan_to_num(b), torch.nan_to_num(a), atol=1e-2, rtol=1e-2, what="rows beside a NaN")
+
+
+@pytest.mark.parametrize("n,H,K,algo", [(9000, 8, 1024, 2), (20480, 4, 1024, 4), (60000, 4, 512, 4), (60000, 4, 320, 2),
+                                        (200000, 4, 256, 2)])
+def test_attention_automatic_choice(n, H, K, algo):
+    """Both sides of the lines between the mma.sync and the tcgen05 kernel: the automatic choice gives the bits of the
+    one that it stands for."""
+    g = torch.Generator().manual_seed(n)
+    qkv = torch.randn(n, 48 * H, generator=g).bfloat16().cuda()
+    order = torch.randperm(n, generator=g).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    got = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25)
+    assert torch.equal(got, ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25, algo=algo))
+    other = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25, algo=6 - algo)
+    assert not torch.equal(got, other)
+
+
 @pytest.mark.parametrize("n,H,K", [(16, 1, 16), (17, 32, 1024), (105, 16, 1024), (457, 32, 1024), (1757, 16, 1024),
                                    (3001, 2, 256), (6760, 8, 1024), (26000, 4, 1024), (2049, 2, 2048)])
 def test_attention_cuts_cover_every_row_once(n, H, K):
