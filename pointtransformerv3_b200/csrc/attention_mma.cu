@@ -53,14 +53,25 @@ __device__ __forceinline__ uint32_t scale_bf16x2(uint32_t v, float s)
     return pack_bf16(f.x * s, f.y * s);
 }
 
-// PLANNED: the geometry may be read before the wait for the kernel ahead (see linear.cuh)
-template <bool PACKED, bool PLANNED>
+// How K and V come to shared memory.  A copy instruction costs a cycle per line it touches, so two lanes that take the
+// halves of one row cost half of one lane per row with a half at a time.  That shortens the start of launches of a few
+// waves, where CTAs gather at the same time (us: 405 points of 8 heads 5.5 -> 5.1, 1 560 of 4 9.1 -> 8.0, 6 000 of 2
+// 10.7 -> 9.8, 1 757 of 16 16.3 -> 15.7, 4 x 560 of 32 20.8 -> 19.8, 632 CTAs of 256 points 19.7 -> 19.0); in long ones a CTA's
+// gather is hidden by the two beside it, and the loop behind it gets worse registers (6 252 CTAs of 256 points 146.5 ->
+// 148.1, 60 000 points of 2 048 174.7 -> 183).
+enum AmGather {
+    AM_LONG,          // a row per lane
+    AM_SHORT,         // half a row per lane
+    AM_PLANNED        // the same, and the geometry may be read before the wait for the kernel ahead (see linear.cuh)
+};
+
+template <bool PACKED, AmGather GATHER>
 __global__ void __launch_bounds__(AM_THREADS, 3) attn_mma_d16_kernel(
     const __nv_bfloat16* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad, const int32_t* cu_seqlens,
     __nv_bfloat16* out, int C, float scale, int lpad_max, uint32_t* status)
 {
     pdl_launch_next();
-    if (!PLANNED) pdl_wait();
+    if (GATHER != AM_PLANNED) pdl_wait();
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char* Ks = smem;
     unsigned char* Vs = smem + (size_t)lpad_max * 32;
@@ -100,42 +111,51 @@ __global__ void __launch_bounds__(AM_THREADS, 3) attn_mma_d16_kernel(
     }
     const int64_t row_stride = 3 * (int64_t)C;
 
-    if (PLANNED) {
-        // ---- rows of the sequence: four per thread at a time, a chain of two dependent loads ------------------
-        for (int rb = tid; rb < L; rb += 4 * AM_THREADS) {
-            int64_t pd[4], src[4], own[4];
+    if (GATHER != AM_LONG) {
+        // ---- K and V of the whole sequence: two lanes a row, a 16-byte half each ------------------------------
+        const int half = lane & 1;
+        auto gather32 = [&](int base, int32_t e) {      // rows base .. base + 31, of which this lane knows one
 #pragma unroll
-            for (int i = 0; i < 4; ++i) pd[i] = rb + i * AM_THREADS < L ? pad[start + rb + i * AM_THREADS] : -1;
+            for (int k = 0; k < 2; ++k) {
+                const int r = base + 16 * k + (lane >> 1);
+                const int32_t er = __shfl_sync(0xffffffffu, e, 16 * k + (lane >> 1));
+                if (r < L) {
+                    const __nv_bfloat16* kp = qkv + C + h * AM_D + (int64_t)(er >= 0 ? er : -(er + 1)) * row_stride + 8 * half;
+                    cp_async16(smem_u32(Ks) + kv_offset(r, half), kp);
+                    cp_async16(smem_u32(Vs) + kv_offset(r, half), kp + C);
+                } else if (r < Lp) {
+                    const uint4 z = make_uint4(0, 0, 0, 0);
+                    *reinterpret_cast<uint4*>(Ks + kv_offset(r, half)) = z;
+                    *reinterpret_cast<uint4*>(Vs + kv_offset(r, half)) = z;
+                }
+            }
+        };
+        // rows of the sequence, four rounds at a time: a chain of two dependent loads (points and padded rows are numbered
+        // in 32 bits, as the caller's n and cu_seqlens are)
+        for (int base = 32 * warp; base < Lp; base += 4 * AM_THREADS) {
+            const int rb = base + lane;
+            int32_t pd[4], src[4], own[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) pd[i] = rb + i * AM_THREADS < L ? (int32_t)pad[start + rb + i * AM_THREADS] : -1;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                src[i] = pd[i] >= 0 ? order[pd[i]] : 0;
-                own[i] = pd[i] >= 0 ? unpad[pd[i]] : 0;
+                src[i] = pd[i] >= 0 ? (int32_t)order[pd[i]] : 0;
+                own[i] = pd[i] >= 0 ? (int32_t)unpad[pd[i]] : 0;
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (GATHER == AM_SHORT && base + i * AM_THREADS < Lp) gather32(base + i * AM_THREADS, src[i]);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int r = rb + i * AM_THREADS;
-                if (r < L) src_s[r] = own[i] == start + r ? (int32_t)src[i] : -(int32_t)src[i] - 1;
+                if (r < L) src_s[r] = own[i] == (int32_t)start + r ? src[i] : -src[i] - 1;
             }
         }
-        // (so far only the geometry was read: planned, that happens beside the kernel before this one in the stream)
-        pdl_wait();
-        // ---- gather K and V of the whole sequence ------------------------------
-#pragma unroll 4
-        for (int r = tid; r < Lp; r += AM_THREADS) {
-            if (r < L) {
-                const int32_t e = src_s[r];          // (this thread's own)
-                const __nv_bfloat16* kp = qkv + (int64_t)(e >= 0 ? e : -(e + 1)) * row_stride + C + h * AM_D;
-                cp_async16(smem_u32(Ks) + kv_offset(r, 0), kp);
-                cp_async16(smem_u32(Ks) + kv_offset(r, 1), kp + 8);
-                cp_async16(smem_u32(Vs) + kv_offset(r, 0), kp + C);
-                cp_async16(smem_u32(Vs) + kv_offset(r, 1), kp + C + 8);
-            } else {
-                const uint4 z = make_uint4(0, 0, 0, 0);
-                *reinterpret_cast<uint4*>(Ks + kv_offset(r, 0)) = z;
-                *reinterpret_cast<uint4*>(Ks + kv_offset(r, 1)) = z;
-                *reinterpret_cast<uint4*>(Vs + kv_offset(r, 0)) = z;
-                *reinterpret_cast<uint4*>(Vs + kv_offset(r, 1)) = z;
-            }
+        if (GATHER == AM_PLANNED) {
+            // (so far only the geometry was read: planned, that happens beside the kernel before this one in the stream)
+            pdl_wait();
+            for (int base = 32 * warp; base < Lp; base += AM_THREADS)
+                gather32(base, base + lane < L ? src_s[base + lane] : 0);          // (this lane's own)
         }
     } else {
         // ---- gather K and V of the whole sequence ------------------------------
@@ -173,11 +193,21 @@ __global__ void __launch_bounds__(AM_THREADS, 3) attn_mma_d16_kernel(
     __shared__ float knorm_s[AM_WARPS];
     cp_async_commit();
     cp_async_wait<0>();
-    // largest squared norm of a key (every thread reads back the rows it copied itself)
+    // largest squared norm of a key (every thread reads back what it copied itself)
     float knorm = 0.f;
-    for (int r = tid; r < L; r += AM_THREADS)
-        knorm = max_nan(knorm, sq_norm16(*reinterpret_cast<const uint4*>(Ks + kv_offset(r, 0)),
-                                         *reinterpret_cast<const uint4*>(Ks + kv_offset(r, 1))));
+    if (GATHER != AM_LONG) {
+        for (int base = 32 * warp; base < Lp; base += AM_THREADS)
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                float n = sq_norm8(*reinterpret_cast<const uint4*>(Ks + kv_offset(base + 16 * k + (lane >> 1), lane & 1)));
+                n += __shfl_xor_sync(0xffffffffu, n, 1);
+                knorm = max_nan(knorm, n);
+            }
+    } else {
+        for (int r = tid; r < L; r += AM_THREADS)
+            knorm = max_nan(knorm, sq_norm16(*reinterpret_cast<const uint4*>(Ks + kv_offset(r, 0)),
+                                             *reinterpret_cast<const uint4*>(Ks + kv_offset(r, 1))));
+    }
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) knorm = max_nan(knorm, __shfl_xor_sync(0xffffffffu, knorm, d));
     if (lane == 0) knorm_s[warp] = knorm;
@@ -417,11 +447,13 @@ int launch_attn_mma(const void* qkv, const int64_t* order, const int64_t* pad, c
     const size_t smem = (size_t)lpad * 68;      // K, V and the row numbers
     const AmCut cut = am_cut((int64_t)n_seq * H, max_seqlen, smem);
     // The look-up ahead of the wait pays where a launch has at most one CTA per SM, all of them at their beginning when the
-    // kernel ahead ends (a pass over 6 000 points 1 550 -> 1 498 us); the two-step gather costs 2 to 3 % of a long one
-    // (400 000 x 64 447 -> 461).
-    const bool ahead = planned && !packed_exp && (int64_t)n_seq * H * cut.slices <= SMS;
-    auto kern = packed_exp ? attn_mma_d16_kernel<true, false> : ahead ? attn_mma_d16_kernel<false, true>
-                                                                       : attn_mma_d16_kernel<false, false>;
+    // kernel ahead ends (a pass over 6 000 points 1 550 -> 1 498 us).
+    const int64_t ctas = (int64_t)n_seq * H * cut.slices;
+    // (patches of more than 1 024 rows: one CTA per SM, which takes too long for its start to count)
+    auto kern = packed_exp                                  ? attn_mma_d16_kernel<true, AM_LONG>
+                : planned && ctas <= SMS                   ? attn_mma_d16_kernel<false, AM_PLANNED>
+                : ctas <= 8 * SMS && max_seqlen <= 1024 ? attn_mma_d16_kernel<false, AM_SHORT>
+                                                            : attn_mma_d16_kernel<false, AM_LONG>;
     if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_attention_fwd: shared memory attribute");
     // (shared memory that only so many CTAs find room for)

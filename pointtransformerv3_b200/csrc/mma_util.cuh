@@ -169,12 +169,13 @@ __device__ __forceinline__ float sq_norm_bf16x2(uint32_t v, float acc)
     const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v));
     return fmaf(f.x, f.x, fmaf(f.y, f.y, acc));
 }
-// squared norm of 16 bf16 values
-__device__ __forceinline__ float sq_norm16(const uint4& a, const uint4& b)
+// squared norm of 8 bf16 values
+__device__ __forceinline__ float sq_norm8(const uint4& a, float acc = 0.f)
 {
-    float v = sq_norm_bf16x2(a.x, sq_norm_bf16x2(a.y, sq_norm_bf16x2(a.z, sq_norm_bf16x2(a.w, 0.f))));
-    return sq_norm_bf16x2(b.x, sq_norm_bf16x2(b.y, sq_norm_bf16x2(b.z, sq_norm_bf16x2(b.w, v))));
+    return sq_norm_bf16x2(a.x, sq_norm_bf16x2(a.y, sq_norm_bf16x2(a.z, sq_norm_bf16x2(a.w, acc))));
 }
+// and of 16
+__device__ __forceinline__ float sq_norm16(const uint4& a, const uint4& b) { return sq_norm8(b, sq_norm8(a)); }
 // maximum that keeps a NaN
 __device__ __forceinline__ float max_nan(float a, float b)
 {
