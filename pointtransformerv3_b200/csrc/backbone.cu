@@ -122,7 +122,7 @@ private:
     // the plan in flight (pooling of level made_ - 1): packed outputs whose row stride is not known yet
     bool flying_ = false;
     int64_t *pcode_ = nullptr, *porder_ = nullptr, *pbatch_ = nullptr, *poffset_ = nullptr;
-    int32_t* pgrid_ = nullptr;
+    int32_t *pgrid_ = nullptr, *pindices_ = nullptr;
     // scratch of the main stream, reused in stream order
     char* ws_ = nullptr;
     size_t ws_bytes_ = 0;
@@ -151,7 +151,8 @@ private:
         for (int b = 0; b < n_scenes; ++b) least = l.counts[b] < least ? l.counts[b] : least;
         return (int)least;
     }
-    int pad_level(BbLevel& l, int patch, Arena& mem, cudaStream_t stream, int64_t* pad, int64_t* unpad, int32_t* cu);
+    int pad_level(BbLevel& l, int patch, Arena& mem, cudaStream_t stream, int64_t* pad, int64_t* unpad, int32_t* cu,
+                  const VoxelClear& index);
     const float *stem_scale_ = a_.stem_scale, *stem_shift_ = a_.stem_shift;
     int norms(BnJobs* jobs);
     template <typename F>
@@ -166,8 +167,9 @@ private:
     int decoder(int d);
 };
 
-// patch layout of a level (model.py:382-438); pad / unpad / cu may be given
-int Pass::pad_level(BbLevel& l, int patch, Arena& mem, cudaStream_t stream, int64_t* pad, int64_t* unpad, int32_t* cu)
+// patch layout of a level (model.py:382-438); pad / unpad / cu may be given; a layout that is made clears `index` too
+int Pass::pad_level(BbLevel& l, int patch, Arena& mem, cudaStream_t stream, int64_t* pad, int64_t* unpad, int32_t* cu,
+                    const VoxelClear& index)
 {
     if (l.patch == patch) return PTV3_OK;
     PTV3_REQUIRE(patch >= 1, PTV3_ERR_INVALID_ARGUMENT, "ptv3_backbone_fwd: patch size %d", patch);
@@ -185,7 +187,7 @@ int Pass::pad_level(BbLevel& l, int patch, Arena& mem, cudaStream_t stream, int6
     if (!l.pad || !l.unpad || !l.cu) return out_of_memory();
     l.patch = patch;
     l.n_seq = (int)n_seq;
-    return ptv3_pad_plan(l.offset, a_.n_scenes, patch, l.n, n_pad, (int)n_seq, l.pad, l.unpad, l.cu, a_.status, stream);
+    return pad_plan(l.offset, a_.n_scenes, patch, l.n, n_pad, (int)n_seq, l.pad, l.unpad, l.cu, a_.status, index, stream);
 }
 
 // BatchNorm layers as scale and shift, computed for this pass (as the weights below): where they will lie
@@ -320,16 +322,17 @@ int Pass::finest()
     if (!index_ws || !wt) return out_of_memory();
     BnJobs bn;
     BB_STEP(norms(&bn));
-    BB_STEP(batch_indices_and_norms(a_.offset, a_.n_scenes, a_.grid_coord, a_.n, a_.indices, bn, main_));
     VoxelIndex vi;
-    BB_STEP(build_voxel_index(a_.indices, a_.n, index_ws, a_.status, main_, &vi));
+    const VoxelClear empty = place_voxel_index(a_.n, index_ws, &vi);
+    BB_STEP(batch_indices_and_norms(a_.offset, a_.n_scenes, a_.grid_coord, a_.n, a_.indices, empty, bn, main_));
+    BB_STEP(fill_voxel_index(vi, empty, a_.indices, a_.n, a_.status, main_));
     BB_CUDA(events_.record(main_, &indexed));
     BB_STEP(split_weights());
     BB_CUDA(cudaStreamWaitEvent(side_, indexed, 0));
     BB_STEP(kmap_from_index(vi, a_.indices, a_.n, 3, a_.order, a_.nbr, a_.status, side_));
     if (enc_[0].n_blocks > 0)
         BB_STEP(pad_level(l, patch_of(enc_[0].patch[0], l, a_.n_scenes), plan_mem_, side_, a_.pad, a_.unpad,
-                          a_.cu_seqlens));
+                          a_.cu_seqlens, VoxelClear{}));
     BB_CUDA(events_.record(side_, &l.ready));
     made_ = 1;
     BB_STEP(launch_plan());
@@ -358,16 +361,17 @@ int Pass::launch_plan()
     pgrid_ = plan_mem_.take<int32_t>((size_t)3 * p.n);
     pbatch_ = plan_mem_.take<int64_t>(p.n);
     poffset_ = plan_mem_.take<int64_t>(a_.n_scenes);
+    pindices_ = plan_mem_.take<int32_t>((size_t)4 * p.n);
     int64_t* meta = plan_mem_.take<int64_t>(1 + a_.n_scenes);
     char* ws = plan_mem_.take<char>(bytes);
     if (!p.cluster || !p.idx_ptr || !head || !pcode_ || !porder_ || !pinverse || !pgrid_ || !pbatch_ || !poffset_ ||
-        !meta || !ws)
+        !pindices_ || !meta || !ws)
         return out_of_memory();
     int64_t* host = flag(made_ - 1);
     reinterpret_cast<volatile int64_t*>(host)[2 + a_.n_scenes] = 0;
     BB_STEP(pool_plan(p.code, p.order, p.grid, p.batch, a_.k, p.n, a_.n_scenes, depth,
                       a_.row_perm ? a_.row_perm + (size_t)(made_ - 1) * a_.k : nullptr, p.cluster, p.idx_ptr, head, pcode_,
-                      porder_, pinverse, pgrid_, pbatch_, meta, host, poffset_, a_.status, ws, bytes, side_));
+                      porder_, pinverse, pgrid_, pbatch_, meta, host, poffset_, pindices_, a_.status, ws, bytes, side_));
     lv_[made_].depth = p.depth - depth;
     flying_ = true;
     return PTV3_OK;
@@ -396,17 +400,20 @@ int Pass::take_plan(bool block)
     l.grid = pgrid_;
     l.batch = pbatch_;
     l.offset = poffset_;
-    const size_t bytes = ptv3_kmap_workspace_bytes(l.n);
-    int32_t* indices = plan_mem_.take<int32_t>((size_t)4 * l.n);
     int32_t* nbr = plan_mem_.take<int32_t>((size_t)27 * l.n);
-    char* ws = plan_mem_.take<char>(bytes);
-    if (!indices || !nbr || !ws) return out_of_memory();
-    BB_STEP(ptv3_batch_indices(l.offset, a_.n_scenes, l.grid, l.n, nullptr, indices, side_));
-    BB_STEP(ptv3_kmap_build_ordered(indices, l.n, 3, l.order, nbr, a_.status, ws, bytes, side_));
-    l.nbr = nbr;
+    char* ws = plan_mem_.take<char>(voxel_index_bytes(l.n));
+    if (!nbr || !ws) return out_of_memory();
+    VoxelIndex vi;
     const ptv3_stage_args& st = enc_[made_];
-    if (st.n_blocks > 0)
-        BB_STEP(pad_level(l, patch_of(st.patch[0], l, a_.n_scenes), plan_mem_, side_, nullptr, nullptr, nullptr));
+    if (st.n_blocks > 0) {
+        const VoxelClear empty = place_voxel_index(l.n, ws, &vi);
+        BB_STEP(pad_level(l, patch_of(st.patch[0], l, a_.n_scenes), plan_mem_, side_, nullptr, nullptr, nullptr, empty));
+        BB_STEP(fill_voxel_index(vi, empty, pindices_, l.n, a_.status, side_));
+    } else {
+        BB_STEP(build_voxel_index(pindices_, l.n, ws, a_.status, side_, &vi));
+    }
+    BB_STEP(kmap_from_index(vi, pindices_, l.n, 3, l.order, nbr, a_.status, side_));
+    l.nbr = nbr;
     BB_CUDA(events_.record(side_, &l.ready));
     ++made_;
     return launch_plan();
@@ -415,7 +422,8 @@ int Pass::take_plan(bool block)
 int Pass::block(const ptv3_stage_args& st, int j, BbLevel& l, const void* conv_in, const void* feat, void* out)
 {
     ptv3_block_args b = st.blocks[j];
-    BB_STEP(pad_level(l, patch_of(st.patch[j], l, a_.n_scenes), mem_, main_, nullptr, nullptr, nullptr));
+    BB_STEP(pad_level(l, patch_of(st.patch[j], l, a_.n_scenes), mem_, main_, nullptr, nullptr, nullptr,
+                      VoxelClear{}));
     b.n = l.n;
     b.n_seq = l.n_seq;
     b.max_seqlen = l.longest;

@@ -83,43 +83,60 @@ __global__ void __launch_bounds__(256) km_probe_kernel(const int32_t* __restrict
     nbr[(int64_t)o * n + i] = found;
 }
 
-// Neighbour table from the two-level voxel index: one thread per voxel looks up the 8 blocks
+// Neighbour table from the two-level voxel index: one thread per voxel looks up the (up to 8) blocks
 // its neighbourhood touches, then every offset is one cell-table load (kernel sizes up to 5).
-__global__ void __launch_bounds__(256) km_block_probe_kernel(const int32_t* __restrict__ indices, int64_t n,
-                                                             int ksize, VoxelIndex vi,
-                                                             int32_t* __restrict__ nbr,
-                                                             const int64_t* __restrict__ row_order,
-                                                             uint32_t* __restrict__ status)
+// A thread's time is its chain of dependent loads, so those of a step go out together: the first slots of all
+// blocks, their table numbers, the cells of one dx.  (One block and one cell after another, the stores between them:
+// 6 000 voxels 9.7 us for 5.9, 85 000 10.7 for 7.8, the five levels of 2 M LiDAR points 455 for 315.)
+template <int KSIZE>
+__global__ void __launch_bounds__(256) km_block_probe_kernel(const int32_t* indices, int64_t n, VoxelIndex vi, int32_t* nbr,
+                                                             const int64_t* row_order, uint32_t* status)
 {
-    __shared__ uint32_t block_s[8][256];
+    __shared__ uint32_t block_s[8][256];       // a thread's own column each
+    pdl_launch_next();
+    pdl_wait();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const int r = ksize / 2;
+    constexpr int R = KSIZE / 2;
     // column i of the table describes voxel row_order[i] (voxel i without an order)
     const int4 c = reinterpret_cast<const int4*>(indices)[row_order ? row_order[i] : i];
+    const int bx0 = (c.y - R) >> 2, by0 = (c.z - R) >> 2, bz0 = (c.w - R) >> 2;
+    const bool more_x = ((c.y + R) >> 2) != bx0, more_y = ((c.z + R) >> 2) != by0, more_z = ((c.w + R) >> 2) != bz0;
+    uint64_t key[8];
+    unsigned long long first[8];
+    bool wanted[8];
+#pragma unroll
+    for (int bi = 0; bi < 8; ++bi) {
+        wanted[bi] = vi_block_key(c.x, bx0 + ((bi >> 2) & 1), by0 + ((bi >> 1) & 1), bz0 + (bi & 1), key[bi]) &&
+                     (!(bi & 4) || more_x) && (!(bi & 2) || more_y) && (!(bi & 1) || more_z);
+        first[bi] = wanted[bi] ? vi.keys[km_mix(key[bi]) & vi.cap_mask] : KM_EMPTY;
+    }
+    uint32_t id[8];
+#pragma unroll
+    for (int bi = 0; bi < 8; ++bi)
+        id[bi] = wanted[bi] && first[bi] == key[bi] ? vi.vals[km_mix(key[bi]) & vi.cap_mask] : VI_NO_ROW;
     bool overflow = false;
 #pragma unroll
     for (int bi = 0; bi < 8; ++bi) {
-        uint64_t key;
-        uint32_t id = VI_NO_ROW;
-        if (vi_block_key(c.x, ((c.y - r) >> 2) + ((bi >> 2) & 1), ((c.z - r) >> 2) + ((bi >> 1) & 1),
-                         ((c.w - r) >> 2) + (bi & 1), key))
-            id = vi_block_lookup(vi.keys, vi.vals, vi.cap_mask, key, &overflow);
-        block_s[bi][threadIdx.x] = id;
+        if (wanted[bi] && first[bi] != key[bi] && first[bi] != KM_EMPTY)
+            id[bi] = vi_block_lookup(vi.keys, vi.vals, vi.cap_mask, key[bi], &overflow);
+        block_s[bi][threadIdx.x] = id[bi];
     }
     if (overflow) atomicOr(status, PTV3_STATUS_PROBE_LIMIT);
-    const int bx0 = (c.y - r) >> 2, by0 = (c.z - r) >> 2, bz0 = (c.w - r) >> 2;
-    int o = 0;
-    for (int dx = -r; dx <= r; ++dx)
-        for (int dy = -r; dy <= r; ++dy)
-            for (int dz = -r; dz <= r; ++dz, ++o) {
-                const int x = c.y + dx, y = c.z + dy, z = c.w + dz;
-                const int bi = (((x >> 2) - bx0) << 2) | (((y >> 2) - by0) << 1) | ((z >> 2) - bz0);
-                const uint32_t id = block_s[bi][threadIdx.x];
-                uint32_t j = VI_NO_ROW;
-                if (id != VI_NO_ROW) j = vi.cells[(size_t)id * 64 + vi_cell(x, y, z)];
-                nbr[(int64_t)o * n + i] = (int32_t)j;   // VI_NO_ROW is -1 as an int32
-            }
+#pragma unroll 1
+    for (int dx = -R; dx <= R; ++dx) {
+        uint32_t found[KSIZE * KSIZE];
+#pragma unroll
+        for (int q = 0; q < KSIZE * KSIZE; ++q) {
+            const int x = c.y + dx, y = c.z + q / KSIZE - R, z = c.w + q % KSIZE - R;
+            const int bi = (((x >> 2) - bx0) << 2) | (((y >> 2) - by0) << 1) | ((z >> 2) - bz0);
+            const uint32_t table = block_s[bi][threadIdx.x];
+            found[q] = table != VI_NO_ROW ? vi.cells[(size_t)table * 64 + vi_cell(x, y, z)] : VI_NO_ROW;
+        }
+        int32_t* out = nbr + (int64_t)((dx + R) * KSIZE * KSIZE) * n + i;
+#pragma unroll
+        for (int q = 0; q < KSIZE * KSIZE; ++q) out[(int64_t)q * n] = (int32_t)found[q];   // VI_NO_ROW is -1 as an int32
+    }
 }
 
 uint64_t km_capacity(int64_t n)
@@ -157,8 +174,9 @@ int km_build_table(const int32_t* indices, int64_t n, void* workspace, uint32_t*
 int kmap_from_index(const VoxelIndex& vi, const int32_t* indices, int64_t n, int ksize, const int64_t* row_order,
                     int32_t* nbr, uint32_t* status, cudaStream_t stream)
 {
-    km_block_probe_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(indices, n, ksize, vi, nbr, row_order,
-                                                                           status);
+    const dim3 blocks((unsigned)((n + 255) / 256)), threads(256);
+    const auto kernel = ksize == 1 ? km_block_probe_kernel<1> : ksize == 3 ? km_block_probe_kernel<3> : km_block_probe_kernel<5>;
+    launch_dependent(kernel, blocks, threads, 0, stream, indices, n, vi, nbr, row_order, status);
     count_launches(1);
     return check_launch("ptv3_kmap_build");
 }

@@ -3,13 +3,13 @@
 namespace ptv3 {
 
 // every voxel claims its block: the first claimant takes the next table and clears it
-__global__ void __launch_bounds__(256) vi_block_insert_kernel(const int32_t* __restrict__ indices, int64_t n,
-                                                              unsigned long long* __restrict__ keys,
-                                                              uint32_t* __restrict__ vals, uint64_t cap_mask,
-                                                              uint32_t* __restrict__ counter,
-                                                              uint32_t* __restrict__ cells,
-                                                              uint32_t* __restrict__ status)
+__global__ void __launch_bounds__(256) vi_block_insert_kernel(const int32_t* indices, int64_t n,
+                                                              unsigned long long* keys, uint32_t* vals,
+                                                              uint64_t cap_mask, uint32_t* counter, uint32_t* cells,
+                                                              uint32_t* status)
 {
+    pdl_launch_next();
+    pdl_wait();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int4 v = reinterpret_cast<const int4*>(indices)[i];
@@ -39,12 +39,12 @@ __global__ void __launch_bounds__(256) vi_block_insert_kernel(const int32_t* __r
 
 // second pass (all tables exist now): every voxel writes its row into its cell;
 // duplicates resolve to the lowest row
-__global__ void __launch_bounds__(256) vi_cell_fill_kernel(const int32_t* __restrict__ indices, int64_t n,
-                                                           const unsigned long long* __restrict__ keys,
-                                                           const uint32_t* __restrict__ vals, uint64_t cap_mask,
-                                                           uint32_t* __restrict__ cells,
-                                                           uint32_t* __restrict__ status)
+__global__ void __launch_bounds__(256) vi_cell_fill_kernel(const int32_t* indices, int64_t n,
+                                                           const unsigned long long* keys, const uint32_t* vals,
+                                                           uint64_t cap_mask, uint32_t* cells, uint32_t* status)
 {
+    pdl_launch_next();
+    pdl_wait();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int4 v = reinterpret_cast<const int4*>(indices)[i];
@@ -65,8 +65,7 @@ __global__ void __launch_bounds__(256) vi_cell_fill_kernel(const int32_t* __rest
 // hash table of blocks (sized for one block per voxel), block counter, one 64-entry table per voxel at most
 size_t voxel_index_bytes(int64_t n) { return km_table_bytes(n) + 256 + align_up((size_t)n * 256, 256); }
 
-int build_voxel_index(const int32_t* indices, int64_t n, void* workspace, uint32_t* status, cudaStream_t stream,
-                      VoxelIndex* out)
+VoxelClear place_voxel_index(int64_t n, void* workspace, VoxelIndex* out)
 {
     const uint64_t cap = km_capacity(n);
     Carver cv(workspace);
@@ -74,17 +73,38 @@ int build_voxel_index(const int32_t* indices, int64_t n, void* workspace, uint32
     uint32_t* vals = cv.take<uint32_t>(cap);
     uint32_t* counter = cv.take<uint32_t>(64);
     uint32_t* cells = cv.take<uint32_t>((size_t)n * 64);
-    cudaMemsetAsync(keys, 0xff, cap * sizeof(uint64_t), stream);
-    cudaMemsetAsync(counter, 0, sizeof(uint32_t), stream);
-    const unsigned vb = (unsigned)((n + 255) / 256);
-    vi_block_insert_kernel<<<vb, 256, 0, stream>>>(indices, n, keys, vals, cap - 1, counter, cells, status);
-    vi_cell_fill_kernel<<<vb, 256, 0, stream>>>(indices, n, keys, vals, cap - 1, cells, status);
+    *out = VoxelIndex{keys, vals, cap - 1, cells};
+    return VoxelClear{reinterpret_cast<ulonglong2*>(keys), (int64_t)(cap / 2), counter};
+}
+
+int fill_voxel_index(const VoxelIndex& vi, const VoxelClear& cleared, const int32_t* indices, int64_t n, uint32_t* status,
+                     cudaStream_t stream)
+{
+    const dim3 blocks((unsigned)((n + 255) / 256)), threads(256);
+    uint32_t *vals = const_cast<uint32_t*>(vi.vals), *cells = const_cast<uint32_t*>(vi.cells);
+    launch_dependent(vi_block_insert_kernel, blocks, threads, 0, stream, indices, n,
+                     reinterpret_cast<unsigned long long*>(cleared.keys), vals, vi.cap_mask, cleared.counter, cells,
+                     status);
+    launch_dependent(vi_cell_fill_kernel, blocks, threads, 0, stream, indices, n, vi.keys, vi.vals, vi.cap_mask, cells,
+                     status);
     count_launches(2);
-    out->keys = keys;
-    out->vals = vals;
-    out->cap_mask = cap - 1;
-    out->cells = cells;
     return check_launch("voxel index");
+}
+
+__global__ void __launch_bounds__(256) vi_clear_kernel(const VoxelClear job)
+{
+    pdl_launch_next();
+    pdl_wait();
+    job.clear();
+}
+
+int build_voxel_index(const int32_t* indices, int64_t n, void* workspace, uint32_t* status, cudaStream_t stream,
+                      VoxelIndex* out)
+{
+    const VoxelClear job = place_voxel_index(n, workspace, out);
+    launch_dependent(vi_clear_kernel, dim3(voxel_clear_blocks(job)), dim3(256), 0, stream, job);
+    count_launches(1);
+    return fill_voxel_index(*out, job, indices, n, status, stream);
 }
 
 }  // namespace ptv3

@@ -169,6 +169,62 @@ def test_pool_plan_matches_oracle(sizes, perm):
         code, order, depth, grid, b = ref["code"], ref["order"], ref["depth"], rg, rb
 
 
+@pytest.mark.parametrize("n,k,scenes,depth", [
+    (1, 1, 1, 1), (31, 4, 1, 1), (32, 2, 3, 1), (33, 5, 1, 2), (255, 4, 2, 1), (256, 8, 40, 1), (257, 4, 33, 0),
+    (70000, 4, 3, 1), (1 << 17, 2, 2, 1), ((1 << 17) + 1, 4, 70, 1), (300001, 8, 5, 2),
+    (4096 * 1024, 1, 2, 1), (4096 * 1024 + 1, 2, 3, 1)])
+def test_pool_plan_at_the_edges_of_its_tiles(n, k, scenes, depth):
+    """Tiles of 256 and of 1024 points, rows beyond one group of four, more scenes than lanes, counts that a kernel of
+    its own scans: whole numbers, equal to torch's.  Orders are sorts of shuffled cells, so that the plan sees rows of
+    points in no order of their own."""
+    g = torch.Generator().manual_seed(n + k)
+    side = max(2, int(round((n / scenes) ** (1 / 3) * 1.3)))
+    batch = torch.randint(0, scenes, (n,), generator=g).sort().values.cuda()
+    grid = torch.randint(0, side, (n, 3), generator=g, dtype=torch.int32).cuda()
+    # every row numbers the parent cells of a scene in its own way and the children within them alike
+    bits = 24
+    parent = grid.long() >> depth
+    child = grid.long() & ((1 << depth) - 1)
+    low = (child[:, 0] << (2 * depth)) | (child[:, 1] << depth) | child[:, 2]
+    wide = 1 << (bits // 3)
+    code = []
+    for r in range(k):
+        p = parent[:, torch.tensor([[0, 1, 2], [2, 1, 0], [1, 0, 2]][r % 3])]
+        cell = p[:, 0] * wide * wide + p[:, 1] * wide + p[:, 2]
+        cell = cell if r < 3 else (cell * (2 * r + 1)) % (1 << bits)      # odd factor: a permutation of the cells
+        code.append(((batch << bits) + cell << (3 * depth)) | low)
+    code = torch.stack(code)
+    order = code.argsort(dim=1, stable=True)
+    perm = list(range(1, k)) + [0]
+    got = ops.pool_plan(code, order, grid, batch, scenes, depth, perm)
+    cells, cluster, count = torch.unique(code[0] >> (3 * depth), return_inverse=True, return_counts=True)
+    m = cells.shape[0]
+    assert got["m"] == m and torch.equal(got["cluster"], cluster)
+    ptr = torch.cat([count.new_zeros(1), count.cumsum(0)])
+    assert torch.equal(got["idx_ptr"], ptr)
+    head = order[0][ptr[:-1]]
+    assert torch.equal(got["head"], head)
+    assert torch.equal(got["batch"], batch[head]) and torch.equal(got["grid_coord"], grid[head] >> depth)
+    assert got["counts"] == torch.bincount(batch[head], minlength=scenes).tolist()
+    assert got["offset"].tolist() == torch.tensor(got["counts"]).cumsum(0).tolist()
+    want = code[torch.tensor(perm).cuda()][:, head] >> (3 * depth)
+    assert torch.equal(got["code"], want)
+    worder = want.argsort(dim=1)
+    assert torch.equal(got["order"], worder)
+    assert torch.equal(got["inverse"], worder.argsort(dim=1))
+
+
+def test_pool_plan_reports_rows_that_do_not_belong_together():
+    """Codes of one row cut clusters of another in two: as many runs must start in every row."""
+    data = small_batch([3000], 3)
+    batch = O.offset_to_batch(data["offset"])
+    code, order, _, _ = O.serialization(data["grid_coord"], batch, ORDERS)
+    code = code.clone()
+    code[2, :] = torch.arange(code.shape[1]) << 3
+    with pytest.raises(_lib.Ptv3Error, match="status 0x1"):
+        ops.pool_plan(code.cuda(), order.cuda(), data["grid_coord"].cuda(), batch.cuda(), 1, 1)
+
+
 @pytest.mark.parametrize("number", [2, 33, 1 << 40, -1])
 def test_pool_plan_reports_a_scene_number_without_a_scene(number):
     """Clusters are counted per scene: a number outside the scenes has no counter and is reported."""
