@@ -3,11 +3,11 @@
 // The first form of this path (attention.cu, which keeps the other head dimensions, the position bias and
 // the bf16 cross-check) gave a thread one query: every key cost eight 16-byte shared-memory reads for 32
 // multiply-adds, and the scores were computed twice (maximum first, probabilities second).  Here a thread
-// owns two queries, so a read serves twice the arithmetic, products run on pairs of floats, and the scores
+// owns two or four queries, so a read serves as much more arithmetic, products run on pairs of floats, and the scores
 // are computed once: where |q| max|k| bounds them (AX_BOUND, per chunk of keys and CTA) the exponentials
 // need no reference value; other chunks take the maximum first as before.
 //
-// The four warps of a CTA share its 64 queries and take the keys in turn; their sums meet at the end.
+// The four warps of a CTA share its 64 or 128 queries and take the keys in turn; their sums meet at the end.
 // With the queries spread over all threads instead, a patch of a coarse level was a serial chain of up to
 // 1 024 keys on a few CTAs (100 us at 700 points x 256 channels as at 40 000 x 64).
 #include "attention_mma.cuh"
@@ -16,7 +16,7 @@
 
 namespace ptv3 {
 
-constexpr int AX_THREADS = 128, AX_WARPS = AX_THREADS / 32, AX_Q = 2, AX_QT = 32 * AX_Q;
+constexpr int AX_THREADS = 128, AX_WARPS = AX_THREADS / 32;
 constexpr int AX_KC = 128;                   // keys per staged chunk
 constexpr int AX_D = 16, AX_P = AX_D / 2;
 // largest |score| taken without a reference value: the exponent's rounding (16 log2 e 2^-24) stays within
@@ -53,13 +53,23 @@ __device__ __forceinline__ void ax_add(AxRow& r, float p, const ulonglong2* v)
     r.l += p;
 }
 
-__global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(
+// AX_Q queries per thread (2 or 4): AX_QT of a CTA
+template <int AX_Q>
+__global__ void __launch_bounds__(AX_THREADS, AX_Q == 2 ? 4 : 3) attn_f32_d16_kernel(
     const float* __restrict__ qkv, const int64_t* __restrict__ order, const int64_t* __restrict__ pad,
     const int64_t* __restrict__ unpad, const int32_t* __restrict__ cu_seqlens, float* __restrict__ out, int C,
     float scale, uint32_t* __restrict__ status)
 {
-    __shared__ __align__(16) float Ks[AX_KC][AX_D], Vs[AX_KC][AX_D];
-    __shared__ float part[AX_WARPS][AX_QT][AX_D + 3];      // sums, l, m; padded against bank conflicts
+    constexpr int AX_QT = 32 * AX_Q;
+    // keys and values of a chunk; in the end, in their place, the warps' sums
+    struct Chunk {
+        float k[AX_KC][AX_D], v[AX_KC][AX_D];
+    };
+    typedef float Sums[AX_WARPS][AX_QT][AX_D + 3];         // sums, l, m; padded against bank conflicts
+    __shared__ __align__(16) unsigned char shared[sizeof(Chunk) > sizeof(Sums) ? sizeof(Chunk) : sizeof(Sums)];
+    float(&Ks)[AX_KC][AX_D] = reinterpret_cast<Chunk*>(shared)->k;
+    float(&Vs)[AX_KC][AX_D] = reinterpret_cast<Chunk*>(shared)->v;
+    Sums& part = *reinterpret_cast<Sums*>(shared);
     __shared__ float warp_norm[AX_WARPS];
     const int n_heads = C / AX_D;
     const int seq = blockIdx.y, h = blockIdx.x % n_heads, tile = blockIdx.x / n_heads, tid = threadIdx.x, warp = tid >> 5,
@@ -72,20 +82,16 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(
     const int64_t stride = 3 * (int64_t)C;
 
     AxRow row[AX_Q];
-    int64_t dst[AX_Q];
 #pragma unroll
     for (int i = 0; i < AX_Q; ++i) {
         const int qi = tile * AX_QT + i * 32 + lane;
         AxRow& r = row[i];
-        dst[i] = -1;
         r.m = 0.f;
         r.l = r.norm = 0.f;
 #pragma unroll
         for (int d = 0; d < AX_P; ++d) r.q[d] = r.acc[d] = 0ull;
         if (qi < L) {
-            const int64_t pd = pad[start + qi], src = order[pd];
-            if (unpad[pd] == start + qi) dst[i] = src;
-            const float4* qp = reinterpret_cast<const float4*>(qkv + src * stride + h * AX_D);
+            const float4* qp = reinterpret_cast<const float4*>(qkv + order[pad[start + qi]] * stride + h * AX_D);
 #pragma unroll
             for (int d = 0; d < 4; ++d) {
                 float4 v = qp[d];
@@ -120,16 +126,19 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(
 #pragma unroll
         for (int w = 0; w < AX_WARPS; ++w) kn = max_nan(kn, warp_norm[w]);
         // (a NaN fails the test); a reference value raised by an earlier chunk stays in force
-        const bool bounded = row[0].norm * kn <= AX_BOUND * AX_BOUND && row[1].norm * kn <= AX_BOUND * AX_BOUND &&
-                             row[0].m == 0.f && row[1].m == 0.f;
+        bool bounded = true;
+#pragma unroll
+        for (int i = 0; i < AX_Q; ++i) bounded = bounded && row[i].norm * kn <= AX_BOUND * AX_BOUND && row[i].m == 0.f;
         if (__syncthreads_and(bounded)) {
-#pragma unroll 4
+#pragma unroll(AX_Q == 2 ? 4 : 2)
             for (int j = warp; j < nk; j += AX_WARPS) {
                 const ulonglong2* k = reinterpret_cast<const ulonglong2*>(Ks[j]);
                 const ulonglong2* v = reinterpret_cast<const ulonglong2*>(Vs[j]);
-                const float p0 = fast_exp2(ax_dot(row[0].q, k) * AX_LOG2E), p1 = fast_exp2(ax_dot(row[1].q, k) * AX_LOG2E);
-                ax_add(row[0], p0, v);
-                ax_add(row[1], p1, v);
+                float p[AX_Q];
+#pragma unroll
+                for (int i = 0; i < AX_Q; ++i) p[i] = fast_exp2(ax_dot(row[i].q, k) * AX_LOG2E);
+#pragma unroll
+                for (int i = 0; i < AX_Q; ++i) ax_add(row[i], p[i], v);
             }
         } else if (warp < nk) {
 #pragma unroll
@@ -152,7 +161,8 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(
         }
         first = first && warp >= nk;
     }
-    // ---- the warps' sums meet; warps 0 and 1 finish one query of a lane each ----------
+    // ---- the warps' sums meet; the first warps finish one query of a lane each ----------
+    __syncthreads();
 #pragma unroll
     for (int i = 0; i < AX_Q; ++i) {
         const int qi = i * 32 + lane;
@@ -167,9 +177,11 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(
         part[warp][qi][AX_D + 1] = row[i].m;
     }
     __syncthreads();
-    const int64_t mine = warp == 0 ? dst[0] : dst[1];
-    if (warp >= AX_Q || mine < 0) return;
-    const int qi = warp * 32 + lane;
+    const int qi = warp * 32 + lane, at = tile * AX_QT + qi;
+    if (warp >= AX_Q || at >= L) return;
+    const int64_t pd = pad[start + at];
+    if (unpad[pd] != start + at) return;       // a row that fills the last patch: its owner is elsewhere
+    const int64_t mine = order[pd];
     float m = -INFINITY;
     for (int w = 0; w < AX_WARPS; ++w)
         if (part[w][qi][AX_D] != 0.f) m = fmaxf(m, part[w][qi][AX_D + 1]);      // (a NaN sum stays in)
@@ -190,15 +202,29 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(
         op[d] = make_float4(y[4 * d] * inv, y[4 * d + 1] * inv, y[4 * d + 2] * inv, y[4 * d + 3] * inv);
 }
 
+template <int Q>
+static int launch_attn_f32_as(const float* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad,
+                              const int32_t* cu, float* out, int n_seq, int tiles, int C, int H, float scale,
+                              uint32_t* status, cudaStream_t stream)
+{
+    attn_f32_d16_kernel<Q><<<dim3(H * tiles, n_seq), AX_THREADS, 0, stream>>>(qkv, order, pad, unpad, cu, out, C, scale,
+                                                                            status);
+    count_launches(1);
+    return check_launch("ptv3_attention_fwd");
+}
+
 int launch_attn_f32(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad, const int32_t* cu,
                     void* out, int n_seq, int max_seqlen, int C, int H, float scale, uint32_t* status,
                     cudaStream_t stream)
 {
-    const int tiles = (max_seqlen + AX_QT - 1) / AX_QT;
-    attn_f32_d16_kernel<<<dim3(H * tiles, n_seq), AX_THREADS, 0, stream>>>((const float*)qkv, order, pad, unpad, cu,
-                                                                        (float*)out, C, scale, status);
-    count_launches(1);
-    return check_launch("ptv3_attention_fwd");
+    // Four queries per thread read shared memory half as often and keep the FMA pipe busier, in half as many CTAs: from
+    // two of them to an SM.  us, two / four: 90 000 x 64 791 / 672, 40 000 x 64 374 / 315, 20 000 x 64 (640 CTAs of four) 196 / 183,
+    // 10 500 x 64 (352) 114.6 / 111.9, 5 000 x 64 (160) 72.1 / 82.5, 820 x 256 24.8 / 28.9; patches of 1 024.
+    const int64_t ctas = (int64_t)H * n_seq * ((max_seqlen + 127) / 128);
+    const bool four = ctas > SMS * 2;
+    return (four ? launch_attn_f32_as<4> : launch_attn_f32_as<2>)((const float*)qkv, order, pad, unpad, cu, (float*)out, n_seq,
+                                                                  (max_seqlen + (four ? 127 : 63)) / (four ? 128 : 64), C, H,
+                                                                  scale, status, stream);
 }
 
 }  // namespace ptv3

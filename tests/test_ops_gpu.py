@@ -419,6 +419,24 @@ def test_attention_with_and_without_reference_value(n, gain):
     assert rel_l2(b, a) < (5e-3 if gain < 10 else 1e-2)
 
 
+@pytest.mark.parametrize("n,K", [(1281, 128), (1290, 129), (700, 65), (1500, 1024), (330, 31)])
+@pytest.mark.parametrize("gain", [0.3, 8.0])
+def test_attention_fp32_four_queries_per_thread(n, K, gain):
+    """Launches of more than two CTAs to an SM: ragged tiles, patches and chunks of keys, bounded and not, against the
+    one-query form (the order of 32-bit sums: a few 2^-24 per term, as in the test below)."""
+    C, H = 512, 32
+    g = torch.Generator().manual_seed(n)
+    qkv = torch.randn(n, 3 * C, generator=g)
+    qkv[n // 2:, C:2 * C] *= gain * gain
+    qkv[:, :C] *= gain
+    qkv = qkv.cuda()
+    order = torch.randperm(n, generator=g).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    a = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25, algo=1)
+    b = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25)
+    assert bool(torch.isfinite(b).all()) and rel_l2(b, a) < 1e-5
+
+
 @pytest.mark.parametrize("n", [1, 127, 129, 257, 1500])
 @pytest.mark.parametrize("gain", [0.3, 2.0, 8.0])
 def test_attention_fp32_two_queries_per_thread(n, gain):
