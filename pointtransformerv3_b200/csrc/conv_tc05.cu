@@ -72,11 +72,23 @@ __device__ __forceinline__ void ct_store_f32(const ConvTcArgs& a, int64_t row, i
     o[1] = make_float4(y[4], y[5], y[6], y[7]);
 }
 
-template <int BN, int STAGES, int NI, bool SPLIT, bool F32>
+// Operands: bf16; fp32 as the six pieces of split_f32.cuh, a stage for each (32 channels); fp32 as three parts, a stage
+// for each, from which the six products are taken.  A stage for every product, the form before for all widths, moves
+// each part twice in the mean.  us, before / now (L2 flushed, ~5 us of it the timing): 1 830 x 256 73.7 / 48.1, 822 x 256
+// 41.0 / 33.8, 261 x 512 88 / 59.5, 2 855 x 128 36.9 / 29.6, 10 542 x 64 35.8 / 33.8, 100 000 x 64 122.8 / 119.8.  What is left is
+// shared memory: a product of 64 columns takes its 48 to 58 cycles to read 6 KB, of 128 columns 65 (measured alone), 24
+// of them to a slice, whose copies write 72 or 96 KB beside them; a slice takes 3 200 cycles.
+// Error against 64 bits, 2-norm, before / now: 1 830 x 256 1.90e-7 / 1.70e-7, 261 x 512 3.07e-7 / 2.16e-7, 2 855 x 128 1.16e-7 /
+// 1.08e-7, 40 000 x 64 1.76e-7 / 1.04e-7; with contiguous shares of a cluster's CTAs 2.11e-7, 3.56e-7, 1.21e-7.
+constexpr int CT_BF16 = 0, CT_PIECES = 1, CT_PARTS = 2;
+
+template <int BN, int STAGES, int NI, bool SPLIT, int FORM>
 __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                const ConvTcArgs a)
 {
+    constexpr bool F32 = FORM != CT_BF16;
     static_assert(SPLIT || F32, "whole bf16 tiles: conv_stream.cu");
+    static_assert(FORM != CT_PARTS || NI == 1, "one warp meets the three stages of a slice");
     constexpr int KC = CT_KC, ROWB = KC * 2;        // bytes per staged row: one swizzle span
     constexpr int A_BYTES = CT_TM * ROWB, B_BYTES = BN * ROWB, STAGE_BYTES = A_BYTES + B_BYTES;
     constexpr int CT_THREADS = (CT_GATHER_WARPS + NI) * 32;
@@ -84,7 +96,9 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
     // consumed by the same issuer (STAGES a multiple of NI): an issuer that met a slot whose previous use
     // another, slower issuer had not consumed yet would take the parity of that older phase for its own.
     // fp32: SPLIT_ACCS accumulators each (split_f32.cuh)
-    constexpr int ACCS = F32 ? SPLIT_ACCS : 1;
+    // ... parts: as many as tensor memory holds, three of four for the leading products (the more sums, the less is lost
+    // where the tensor core truncates, and a product into an accumulator waits for the one before it)
+    constexpr int ACCS = FORM == CT_PARTS ? 512 / BN : F32 ? SPLIT_ACCS : 1, LEADS = ACCS / 4 * 3;
     constexpr int TM_COLS = NI * ACCS * BN;
     static_assert(TM_COLS >= 32 && TM_COLS <= 512 && (TM_COLS & (TM_COLS - 1)) == 0, "tensor memory");
     static_assert(STAGES % NI == 0, "issuers and accumulators");
@@ -195,14 +209,21 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
     if (a.planned) pdl_wait();
     const uint32_t tmem_base = *tmem_slot;
     const int n_act = act[0];
-    const int kchunks = a.cin / KC;
+    // stages of an offset; parts: three to a slice of KC channels, which stay together
+    constexpr int UNIT = FORM == CT_PARTS ? 3 : 1;
+    const int kchunks = FORM == CT_PARTS ? a.cin / 6 / KC * UNIT : a.cin / KC;
     const int stored = F32 ? a.cin / 6 * split_stored(a.cin / 6) : a.cin;      // columns of a feature row
     // this CTA's share of the tile's stages (all of them without a cluster)
     int first = 0, nit = n_act * kchunks;
     if (SPLIT) {
-        const int total = nit, parts = (int)gridDim.z;
-        first = total * (int)blockIdx.z / parts;
-        nit = total * ((int)blockIdx.z + 1) / parts - first;
+        const int total = nit / UNIT, parts = (int)gridDim.z;
+        if (FORM == CT_PARTS) {
+            // slices in turn: a voxel's neighbours lie on few offsets, and their products then spread over all sums
+            nit = (total - (int)blockIdx.z + parts - 1) / parts * UNIT;
+        } else {
+            first = total * (int)blockIdx.z / parts;
+            nit = total * ((int)blockIdx.z + 1) / parts - first;
+        }
     }
     bool ok = true;
 
@@ -215,9 +236,18 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
         const uint32_t pitch = (uint32_t)stored * 2;
         StageCursor cur{(first + warp) / kchunks, (first + warp) % kchunks, warp % STAGES, 1};
         for (int it = warp < NGW ? warp : nit; it < nit; it += NGW) {
+            if (FORM == CT_PARTS) {
+                const int slice = (int)blockIdx.z + it / UNIT * (int)gridDim.z, per = kchunks / UNIT;
+                cur.at = slice / per;
+                cur.chunk = slice % per * UNIT + it % UNIT;
+            }
             const int o = act[1 + cur.at];
-            const int kc = F32 ? split_column_a(cur.chunk, a.cin / 6) : cur.chunk * KC;
-            const int kw = F32 ? split_column_b(cur.chunk, a.cin / 6) : cur.chunk * KC;
+            int kc = cur.chunk * KC, kw = kc;
+            if (FORM == CT_PIECES) {
+                kc = split_column_a(cur.chunk, a.cin / 6);
+                kw = split_column_b(cur.chunk, a.cin / 6);
+            }
+            if (FORM == CT_PARTS) kc = kw = cur.chunk % 3 * (a.cin / 6) + cur.chunk / 3 * KC;
             ok &= mbar_wait(empty0 + 8 * cur.slot, cur.phase, abort);
             fill_stage<KC, B_BYTES>(gather, sbase + cur.slot * STAGE_BYTES, nbr_s + o * CT_TM,
                                     reinterpret_cast<const char*>(a.feat + kc), pitch, &map_w, o * stored + kw, col0,
@@ -288,6 +318,69 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
 #pragma unroll
                 for (int i = 0; i < 8; ++i) y[i] = __uint_as_float(acc[g * 8 + i]) + bias_s[cb * 32 + g * 8 + i];
                 ct_store_f32(a, v, col0 + cb * 32 + g * 8, y);
+            }
+        }
+    } else if (FORM == CT_PARTS) {
+        // ---- the issuer, fp32 from parts: per slice of KC channels x1 w1 into the leading accumulators in turn, the five
+        // small products into the others in turn
+        constexpr uint32_t idesc = umma_idesc_bf16(CT_TM, BN);
+        const uint64_t da0 = umma_desc_kmajor(sbase, ROWB), db0 = umma_desc_kmajor(sbase + A_BYTES, ROWB);
+        constexpr uint32_t RESTS = ACCS - LEADS;
+        uint32_t used = 0;
+        int s = 0, phase = 0, lead = 0;
+        for (int it = 0; it < nit; it += 3) {
+            uint64_t da[3], db[3];
+            uint32_t slot[3];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                ok &= mbar_wait(full0 + 8 * s, phase, abort);
+                fence_after_sync();
+                da[p] = da0 + s * (STAGE_BYTES >> 4);
+                db[p] = db0 + s * (STAGE_BYTES >> 4);
+                slot[p] = empty0 + 8 * s;
+                if (elect_one()) {
+                    // (x_i w_j with i + j <= 4, as soon as its parts are here)
+                    if (p == 0) {
+#pragma unroll
+                        for (int k4 = 0; k4 < KC / 16; ++k4) {
+                            const uint32_t acc = lead + k4 < LEADS ? lead + k4 : lead + k4 - LEADS;
+                            const uint32_t before = k4 < LEADS ? used : ~0u;
+                            umma_bf16(tmem_base + acc * BN, da[0] + 2 * k4, db[0] + 2 * k4, idesc, (before >> acc) & 1);
+                        }
+                    } else {
+                        constexpr int X[2][3] = {{0, 1, 1}, {0, 2, 0}}, W[2][3] = {{1, 0, 1}, {2, 0, 0}};
+#pragma unroll
+                        for (int k4 = 0; k4 < KC / 16; ++k4)
+#pragma unroll
+                            for (int i = 0; i < (p == 1 ? 3 : 2); ++i) {
+                                const uint32_t turn = k4 * (p == 1 ? 3 : 2) + i;
+                                umma_bf16(tmem_base + (LEADS + turn % RESTS) * BN, da[X[p - 1][i]] + 2 * k4,
+                                          db[W[p - 1][i]] + 2 * k4, idesc, it > 0 || p > 1 || turn >= RESTS);
+                            }
+                    }
+                    if (p == 2) {
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) umma_commit(slot[i]);
+                        if (it + 3 >= nit) {
+                            umma_commit(accfull);
+                            uint32_t all = used;
+#pragma unroll
+                            for (int k4 = 0; k4 < KC / 16; ++k4) all |= 1u << (lead + k4 < LEADS ? lead + k4 : lead + k4 - LEADS);
+                            used_s[0] = all | ((1u << RESTS) - 1) << LEADS;
+                            mbar_arrive_one(accfull);
+                        }
+                    }
+                }
+                __syncwarp();
+                if (++s == STAGES) {
+                    s = 0;
+                    phase ^= 1;
+                }
+            }
+#pragma unroll
+            for (int k4 = 0; k4 < KC / 16; ++k4) {
+                used |= 1u << lead;
+                lead = lead + 1 < LEADS ? lead + 1 : 0;
             }
         }
     } else {
@@ -398,15 +491,16 @@ static constexpr size_t conv_tc05_smem()
            8 * (2 * STAGES + 1) + 32 + 1024;
 }
 
-template <int BN, int STAGES, int NI, bool SPLIT, bool F32>
+template <int BN, int STAGES, int NI, bool SPLIT, int FORM>
 static int launch_conv_tc05_as(const void* weight, const ConvTcArgs& a, cudaStream_t stream, int parts)
 {
+    constexpr bool F32 = FORM != CT_BF16;
     CUtensorMap mw;
     const uint64_t wcols = (uint64_t)a.kvol * (F32 ? a.cin / 6 * split_stored(a.cin / 6) : a.cin);
     const int rc = make_tensor_map_bf16(&mw, weight, (uint64_t)a.cout, wcols, wcols * 2, BN, CT_KC);
     if (rc) return rc;
     constexpr size_t smem = conv_tc05_smem<BN, STAGES>();
-    auto kern = conv_tc05_kernel<BN, STAGES, NI, SPLIT, F32>;
+    auto kern = conv_tc05_kernel<BN, STAGES, NI, SPLIT, FORM>;
     if (allow_smem(kern) != cudaSuccess)
         return check_launch("ptv3_subm_conv_fwd: shared memory attribute");
     const dim3 grid((unsigned)((a.n + CT_TM - 1) / CT_TM), a.cout / BN, parts);
@@ -416,14 +510,14 @@ static int launch_conv_tc05_as(const void* weight, const ConvTcArgs& a, cudaStre
 }
 
 // CTAs in clusters of `parts` that run at once (the driver's answer: a cluster lives in one GPC)
-template <int BN, int STAGES, int NI, bool F32>
+template <int BN, int STAGES, int NI, int FORM>
 static int conv_tc05_capacity(int parts)
 {
     static std::atomic<int> known[4];
     const int slot = parts == 2 ? 1 : parts == 4 ? 2 : 3;
     int c = known[slot].load(std::memory_order_relaxed);
     if (c == 0) {
-        auto kern = conv_tc05_kernel<BN, STAGES, NI, true, F32>;
+        auto kern = conv_tc05_kernel<BN, STAGES, NI, true, FORM>;
         if (allow_smem(kern) != cudaSuccess) return 0;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(SMS, 1, parts);
@@ -454,18 +548,25 @@ struct ConvVariant {
     int (*capacity)(int);
 };
 constexpr int CT_VARIANTS = 3;
-// fp32 output (an issuer's four accumulators of 64 columns fill the tensor memory of an SM).  Last: 32 channels.
+// fp32 output (the accumulators of 64 or 128 columns fill the tensor memory of an SM).  us, 64 wide in clusters of 1, 2, 4, 8 |
+// 128 wide: 822 x 256 94 55 37 - | 110 64 42 34, 487 x 128 54 34 26 22 | 66 41 30 26, 75 x 512 208 110 64 41 | 266 143 81 51.
 static const ConvVariant g_variants_f32[CT_VARIANTS] = {
-    {64, 6.5, 0, 0.20, launch_conv_tc05_as<64, 8, 2, false, true>, launch_conv_tc05_as<64, 8, 2, true, true>,
-     conv_tc05_capacity<64, 8, 2, true>},
-    {32, 6.5, 0, 0.18, launch_conv_tc05_as<32, 8, 2, false, true>, launch_conv_tc05_as<32, 8, 2, true, true>,
-     conv_tc05_capacity<32, 8, 2, true>},
+    {64, 6.5, 0, 0.56, launch_conv_tc05_as<64, 8, 1, false, CT_PARTS>, launch_conv_tc05_as<64, 8, 1, true, CT_PARTS>,
+     conv_tc05_capacity<64, 8, 1, CT_PARTS>},
+    {128, 9.5, 0, 0.63, launch_conv_tc05_as<128, 6, 1, false, CT_PARTS>, launch_conv_tc05_as<128, 6, 1, true, CT_PARTS>,
+     conv_tc05_capacity<128, 6, 1, CT_PARTS>},
+    {1 << 20, 0, 0, 0, nullptr, nullptr, nullptr}};
+// ... of 32 channels
+static const ConvVariant g_variants_f32_32[CT_VARIANTS] = {
+    {32, 6.5, 0, 0.18, launch_conv_tc05_as<32, 8, 2, false, CT_PIECES>, launch_conv_tc05_as<32, 8, 2, true, CT_PIECES>,
+     conv_tc05_capacity<32, 8, 2, CT_PIECES>},
+    {1 << 20, 0, 0, 0, nullptr, nullptr, nullptr},
     {1 << 20, 0, 0, 0, nullptr, nullptr, nullptr}};
 // bf16: clusters here, whole tiles in conv_stream.cu
 static const ConvVariant g_variants[CT_VARIANTS] = {
-    {64, 6.9, 1.6, 0.19, nullptr, launch_conv_tc05_as<64, 8, 2, true, false>, conv_tc05_capacity<64, 8, 2, false>},
-    {128, 8.7, 1.6, 0.26, nullptr, launch_conv_tc05_as<128, 6, 2, true, false>, conv_tc05_capacity<128, 6, 2, false>},
-    {256, 12., 1.6, 0.37, nullptr, launch_conv_tc05_as<256, 4, 2, true, false>, conv_tc05_capacity<256, 4, 2, false>}};
+    {64, 6.9, 1.6, 0.19, nullptr, launch_conv_tc05_as<64, 8, 2, true, CT_BF16>, conv_tc05_capacity<64, 8, 2, CT_BF16>},
+    {128, 8.7, 1.6, 0.26, nullptr, launch_conv_tc05_as<128, 6, 2, true, CT_BF16>, conv_tc05_capacity<128, 6, 2, CT_BF16>},
+    {256, 12., 1.6, 0.37, nullptr, launch_conv_tc05_as<256, 4, 2, true, CT_BF16>, conv_tc05_capacity<256, 4, 2, CT_BF16>}};
 
 // The cluster size and tile width with the shortest estimated time: waves of CTAs, each taking a
 // fixed time (prologue, epilogue) and its stages.  Wide tiles gather a row once for more output
@@ -577,8 +678,10 @@ int launch_conv_split(const void* feat, const int32_t* nbr, const void* weight, 
     a.kvol = kvol;
     a.status = status;
     int v, parts = 1;
-    conv_cluster_cost(g_variants_f32, a, (double)a.kvol * (a.cin / 64), &v, &parts);
-    return (parts > 1 ? g_variants_f32[v].split : g_variants_f32[v].plain)(weight, a, stream, parts);
+    // (half of the offsets in use; of 32 channels all, 64-column chunks of the six pieces)
+    const ConvVariant* variants = c_in == 32 ? g_variants_f32_32 : g_variants_f32;
+    conv_cluster_cost(variants, a, c_in == 32 ? (double)a.kvol * (a.cin / 64) : 0.5 * a.kvol * (c_in / 64) * 3, &v, &parts);
+    return (parts > 1 ? variants[v].split : variants[v].plain)(weight, a, stream, parts);
 }
 
 }  // namespace ptv3

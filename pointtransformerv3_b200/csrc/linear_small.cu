@@ -24,6 +24,13 @@ using namespace tc05;
 constexpr int LS_BM = 128, LS_BN = 64, LS_BK = 64;
 constexpr int LS_A_BYTES = LS_BM * LS_BK * 2, LS_B_BYTES = LS_BN * LS_BK * 2, LS_STAGE = LS_A_BYTES + LS_B_BYTES;
 constexpr int LS_MAX_STAGES = 8;
+// fp32 (split_f32.cuh): a stage is a slice of 32 columns, its three parts of x and of W beside one another, and gives all
+// six products.  (A stage for every product of 64 columns moved each part twice in the mean.  us, before / now: 40 000 x 64 ->
+// 192 37.4 / 31.1, 40 000 x 256 -> 64 41.3 / 29.3, 2 800 x 128 -> 128 10.5 / 7.6, 820 x 256 -> 768 17.0 / 10.9, 260 x 512 ->
+// 2 048 27.6 / 15.3, 260 x 2 048 -> 512 28.4 / 17.3, 27 x 2 048 -> 512 16.4 / 10.4.  Errors against 64 bits as before or,
+// with K shared by a cluster, smaller: 820 x 256 -> 768 7.0e-8 / 5.5e-8, 260 x 2 048 -> 512 3.7e-7 / 1.0e-7.)
+constexpr int LS_SLICE = 32;
+constexpr int LS_A_PART = LS_BM * LS_SLICE * 2, LS_B_PART = LS_BN * LS_SLICE * 2, LS_SPLIT_STAGE = 3 * (LS_A_PART + LS_B_PART);
 constexpr int LS_EPI_WARPS = 8, LS_THREADS = 64 + 32 * LS_EPI_WARPS;
 constexpr int LS_PITCH = LS_BN + 4;                    // floats of a row of partial sums
 constexpr int LS_PLAIN = 0, LS_GELU = 1, LS_RESIDUAL = 2, LS_F32 = 8;
@@ -39,14 +46,15 @@ struct LinearSmallArgs {
 };
 
 // bytes of the ring; a split layer's partial sums (128 x 68 floats) lie over it
-__host__ __device__ constexpr int ls_ring_bytes(int stages)
+__host__ __device__ constexpr int ls_ring_bytes(int stages, bool split)
 {
-    return stages * LS_STAGE > LS_BM * LS_PITCH * 4 ? stages * LS_STAGE : (LS_BM * LS_PITCH * 4 + 1023) / 1024 * 1024;
+    const int ring = stages * (split ? LS_SPLIT_STAGE : LS_STAGE);
+    return ring > LS_BM * LS_PITCH * 4 ? ring : (LS_BM * LS_PITCH * 4 + 1023) / 1024 * 1024;
 }
 constexpr int LS_PARAM_BYTES = LS_BN * 4;              // bias as floats
-static size_t ls_smem(int stages)
+static size_t ls_smem(int stages, bool split)
 {
-    return ls_ring_bytes(stages) + LS_PARAM_BYTES + 8 * (2 * LS_MAX_STAGES + 1) + 16 + 1024;
+    return ls_ring_bytes(stages, split) + LS_PARAM_BYTES + 8 * (2 * LS_MAX_STAGES + 1) + 16 + 1024;
 }
 
 // LS_F32: eight finished columns of a row, as floats or as split bf16 parts (see split_f32.cuh)
@@ -105,9 +113,11 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
     extern __shared__ unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t sbase = smem_u32_generic(smem);
+    constexpr bool SPLIT = (MODE & LS_F32) != 0;
+    constexpr int STAGE = SPLIT ? LS_SPLIT_STAGE : LS_STAGE, BK = SPLIT ? LS_SLICE : LS_BK;
     const int stages = a.stages;
-    float* params = reinterpret_cast<float*>(smem + ls_ring_bytes(stages));
-    const int off_bar = ls_ring_bytes(stages) + LS_PARAM_BYTES;
+    float* params = reinterpret_cast<float*>(smem + ls_ring_bytes(stages, SPLIT));
+    const int off_bar = ls_ring_bytes(stages, SPLIT) + LS_PARAM_BYTES;
     const uint32_t full0 = sbase + off_bar, empty0 = full0 + 8 * LS_MAX_STAGES,
                    accfull = empty0 + 8 * LS_MAX_STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + off_bar + 8 * (2 * LS_MAX_STAGES + 1));
@@ -119,17 +129,34 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
     const int col0 = blockIdx.x * LS_BN, row0 = blockIdx.y * LS_BM;
     // this CTA's chunks of K
     const int parts = (int)gridDim.z;
-    const int nk = a.k / LS_BK / parts, k0 = nk * (int)blockIdx.z * LS_BK;
+    const int nk = a.k / BK / parts, k0 = nk * (int)blockIdx.z * BK;
 
-    auto column_x = [&](int kc) { return (MODE & LS_F32) ? split_column_a(k0 / LS_BK + kc, a.k / 6) : k0 + kc * LS_BK; };
-    auto column_w = [&](int kc) { return (MODE & LS_F32) ? split_column_b(k0 / LS_BK + kc, a.k / 6) : k0 + kc * LS_BK; };
+    // chunk kc of x or of W into slot `s`; of a split layer part by part
+    auto load_x = [&](int kc, int s) {
+        const uint32_t at = sbase + s * STAGE;
+        if (SPLIT) {
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+                tma_load_2d(at + p * LS_A_PART, &map_x, split_part_a(p, a.k) + k0 + kc * BK, row0, full0 + 8 * s);
+        } else {
+            tma_load_2d(at, &map_x, k0 + kc * BK, row0, full0 + 8 * s);
+        }
+    };
+    auto load_w = [&](int kc, int s) {
+        const uint32_t at = sbase + s * STAGE;
+        mbar_expect_tx(full0 + 8 * s, STAGE);
+        if (SPLIT) {
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+                tma_load_2d(at + 3 * LS_A_PART + p * LS_B_PART, &map_w, p * a.k + k0 + kc * BK, col0, full0 + 8 * s);
+        } else {
+            tma_load_2d(at + LS_A_BYTES, &map_w, k0 + kc * BK, col0, full0 + 8 * s);
+        }
+    };
 
     // those of the first chunks: settled ones are fetched ahead of the wait below
     auto weights = [&] {
-        for (int kc = 0; kc < nk && kc < stages; ++kc) {
-            mbar_expect_tx(full0 + 8 * kc, LS_STAGE);
-            tma_load_2d(sbase + kc * LS_STAGE + LS_A_BYTES, &map_w, column_w(kc), col0, full0 + 8 * kc);
-        }
+        for (int kc = 0; kc < nk && kc < stages; ++kc) load_w(kc, kc);
     };
     if (warp == 0 && elect_one()) {
         for (int s = 0; s < stages; ++s) {
@@ -176,14 +203,10 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
         // (slots and phases are counted, not divided: a division by `stages` takes longer than the rest of a turn)
         int s = 0, phase = 1;
         for (int kc = 0; kc < nk; ++kc) {
-            const uint32_t sa = sbase + s * LS_STAGE;
             if (kc >= stages) ok &= mbar_wait(empty0 + 8 * s, phase, abort);
             if (elect_one()) {
-                if (kc >= stages) {
-                    mbar_expect_tx(full0 + 8 * s, LS_STAGE);
-                    tma_load_2d(sa + LS_A_BYTES, &map_w, column_w(kc), col0, full0 + 8 * s);
-                }
-                tma_load_2d(sa, &map_x, column_x(kc), row0, full0 + 8 * s);
+                if (kc >= stages) load_w(kc, s);
+                load_x(kc, s);
             }
             __syncwarp();
             if (++s == stages) {
@@ -193,29 +216,40 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
         }
     } else if (warp == 1) {
         constexpr uint32_t idesc = umma_idesc_bf16(LS_BM, LS_BN);
-        const uint64_t da0 = umma_desc_kmajor(sbase, 128), db0 = umma_desc_kmajor(sbase + LS_A_BYTES, 128);
+        const uint64_t da0 = umma_desc_kmajor(sbase, BK * 2),
+                       db0 = umma_desc_kmajor(sbase + (SPLIT ? 3 * LS_A_PART : LS_A_BYTES), BK * 2);
         uint32_t used = 0;
-        int s = 0, phase = 0;
+        int s = 0, phase = 0, lead = k0 / 16 % SPLIT_MAIN;
         for (int kc = 0; kc < nk; ++kc) {
             ok &= mbar_wait(full0 + 8 * s, phase, abort);
             fence_after_sync();
-            const uint64_t da = da0 + s * (LS_STAGE >> 4), db = db0 + s * (LS_STAGE >> 4);
+            const uint64_t da = da0 + s * (STAGE >> 4), db = db0 + s * (STAGE >> 4);
+            uint32_t seen = used;
             if (elect_one()) {
-                uint32_t seen = used;
 #pragma unroll
-                for (int k4 = 0; k4 < LS_BK / 16; ++k4) {
-                    uint32_t acc = 0;
-                    if (MODE & LS_F32) {
-                        const int step = (k0 + kc * LS_BK) / 16 + k4;      // of 16 columns; the first sixth is the leading piece
-                        acc = step * 96 < a.k ? step % SPLIT_MAIN : SPLIT_MAIN;
+                for (int k4 = 0; k4 < BK / 16; ++k4) {
+                    auto product = [&](int x, int w, uint32_t acc, bool add) {
+                        umma_bf16(tmem_base + acc * LS_BN, da + 2 * k4 + x * (LS_A_PART >> 4), db + 2 * k4 + w * (LS_B_PART >> 4),
+                                  idesc, add);
+                    };
+                    if (SPLIT) {
+                        // x1 w1 into the leading accumulators in turn, the others x_i w_j, i + j <= 4, into the last one
+                        const uint32_t acc = lead + k4 < SPLIT_MAIN ? lead + k4 : lead + k4 - SPLIT_MAIN;
+                        product(0, 0, acc, (seen >> acc) & 1);
+                        product(0, 1, SPLIT_MAIN, (seen >> SPLIT_MAIN) & 1);
+                        seen |= 1u << acc | 1u << SPLIT_MAIN;
+                        product(0, 2, SPLIT_MAIN, true);
+                        product(1, 0, SPLIT_MAIN, true);
+                        product(1, 1, SPLIT_MAIN, true);
+                        product(2, 0, SPLIT_MAIN, true);
+                    } else {
+                        product(0, 0, 0, kc > 0 || k4 > 0);
                     }
-                    umma_bf16(tmem_base + acc * LS_BN, da + 2 * k4, db + 2 * k4, idesc, (seen >> acc) & 1);
-                    seen |= 1u << acc;
                 }
                 if (kc + stages < nk) umma_commit(empty0 + 8 * s);
                 if (kc == nk - 1) {
                     umma_commit(accfull);
-                    if (MODE & LS_F32) {
+                    if (SPLIT) {
                         *used_s = seen;
                         mbar_arrive_one(accfull);
                     }
@@ -223,14 +257,13 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
             }
             __syncwarp();
             // (what the elected lane has seen, for every lane)
-            if (MODE & LS_F32) {
+            if (SPLIT) {
+                used |= 1u << SPLIT_MAIN;
 #pragma unroll
-                for (int k4 = 0; k4 < LS_BK / 16; ++k4) {
-                    const int step = (k0 + kc * LS_BK) / 16 + k4;
-                    used |= 1u << (step * 96 < a.k ? step % SPLIT_MAIN : SPLIT_MAIN);
+                for (int k4 = 0; k4 < BK / 16; ++k4) {
+                    used |= 1u << lead;
+                    lead = lead + 1 < SPLIT_MAIN ? lead + 1 : 0;
                 }
-            } else {
-                used = 1;
             }
             if (++s == stages) {
                 s = 0;
@@ -316,21 +349,23 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
 template <int MODE>
 static int launch_ls(const void* x, const void* w, LinearSmallArgs a, int parts, cudaStream_t stream)
 {
-    const int nk = a.k / LS_BK / parts;
+    constexpr bool split = (MODE & LS_F32) != 0;
+    constexpr int BK = split ? LS_SLICE : LS_BK;
+    const int nk = a.k / BK / parts;
     // (fp32: two CTAs share an SM, in shared memory as in tensor memory; two rooms of 20 000: 6.79 -> 6.65 ms)
-    const int most = (MODE & LS_F32) ? 4 : LS_MAX_STAGES;
+    const int most = split ? 3 : LS_MAX_STAGES;
     a.stages = nk < most ? nk : most;
     CUtensorMap mx, mw;
-    const uint64_t cols = (MODE & LS_F32) ? (uint64_t)a.k / 6 * split_stored(a.k / 6) : (uint64_t)a.k;      // stored
-    int rc = make_tensor_map_bf16(&mx, x, (uint64_t)a.n, cols, cols * 2, LS_BM, LS_BK);
+    const uint64_t cols = split ? (uint64_t)a.k * split_stored(a.k) : (uint64_t)a.k;      // stored
+    int rc = make_tensor_map_bf16(&mx, x, (uint64_t)a.n, cols, cols * 2, LS_BM, BK);
     if (rc) return rc;
-    rc = make_tensor_map_bf16(&mw, w, (uint64_t)a.n_out, cols, cols * 2, LS_BN, LS_BK);
+    rc = make_tensor_map_bf16(&mw, w, (uint64_t)a.n_out, cols, cols * 2, LS_BN, BK);
     if (rc) return rc;
     auto kern = linear_small_kernel<MODE>;
     if (allow_smem(kern) != cudaSuccess) return check_launch("short Linear: shared memory attribute");
     const dim3 grid((a.n_out + LS_BN - 1) / LS_BN, (unsigned)((a.n + LS_BM - 1) / LS_BM), parts);
     const dim3 cluster(1, 1, parts);
-    launch_dependent_cluster(kern, grid, dim3(LS_THREADS), ls_smem(a.stages), stream, cluster, mx, mw, a);
+    launch_dependent_cluster(kern, grid, dim3(LS_THREADS), ls_smem(a.stages, split), stream, cluster, mx, mw, a);
     count_launches(1);
     return check_launch("short Linear");
 }
@@ -345,6 +380,19 @@ static int ls_parts(int64_t tiles, int k)
     if (chunks >= 16)
         while (parts < 8 && tiles * parts * 2 <= LS_CLUSTER_CTAS && chunks % (parts * 2) == 0 && chunks / (parts * 2) >= 4)
             parts *= 2;
+    return parts;
+}
+// fp32: at least four slices each; pairs also where two CTAs share an SM.  us in clusters of 1, 2, 4, 8: 2 800 x 128 -> 128
+// (4 slices) 7.6 8.4 10.0, 820 x 256 -> 256 8.8 8.2 9.8 12.1, 820 x 256 -> 1 024 (224 CTAs in pairs) 12.7 11.7, 260 x 512 ->
+// 512 12.5 10.2 9.4 12.5, 2 800 x 512 -> 128 (176 in fours) 17.2 13.1 13.9, 260 x 2 048 -> 512 (192 in eights) 38.9 22.6 17.3
+// 18.4, 27 x 2 048 -> 512 34.5 20.5 13.5 10.4.
+static int ls_split_parts(int64_t tiles, int k)
+{
+    const int slices = k / LS_SLICE;
+    int parts = 1;
+    while (parts < 8 && tiles * parts * 2 <= (parts == 1 ? 2 : 1) * LS_CLUSTER_CTAS && slices % (parts * 2) == 0 &&
+           slices / (parts * 2) >= 4)
+        parts *= 2;
     return parts;
 }
 
@@ -396,11 +444,11 @@ int launch_linear_split(const void* xs, const void* ws, const float* bias, const
     a.out = out;
     a.split_out = (__nv_bfloat16*)split_out;
     a.n = n;
-    a.k = 6 * k;
+    a.k = k;
     a.n_out = n_out;
     a.settled = settled;
     a.status = status;
-    const int parts = ls_parts((n + LS_BM - 1) / LS_BM * ((n_out + LS_BN - 1) / LS_BN), a.k);
+    const int parts = ls_split_parts((n + LS_BM - 1) / LS_BM * ((n_out + LS_BN - 1) / LS_BN), k);
     switch ((gelu ? LS_GELU : 0) | (residual ? LS_RESIDUAL : 0)) {
     case LS_PLAIN: return launch_ls<LS_F32>(xs, ws, a, parts, stream);
     case LS_GELU: return launch_ls<LS_F32 | LS_GELU>(xs, ws, a, parts, stream);

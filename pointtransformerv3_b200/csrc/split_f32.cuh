@@ -37,6 +37,8 @@ __host__ __device__ __forceinline__ int split_column_b(int c, int k)
     const int piece = c * 64 / k;
     return (piece < 3 ? piece : piece < 5 ? piece - 3 : 0) * k + c * 64 % k;
 }
+// column of part p of a stored row of A; of a row of B it is p k either way
+__host__ __device__ __forceinline__ int split_part_a(int p, int k) { return (k % 64 == 0 ? p : p == 0 ? 0 : 2 * p + 1) * k; }
 
 constexpr int SPLIT_MAIN = 3, SPLIT_ACCS = SPLIT_MAIN + 1;
 

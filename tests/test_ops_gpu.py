@@ -975,6 +975,14 @@ def test_linear_on_split_floats(n, k, n_out, gelu, residual):
     assert rel_l2(got.double(), ref) < 1.5 * rel_l2(plain.double(), ref) + 1e-7
 
 
+@pytest.mark.parametrize("n,k,n_out,gelu", [(200, 96, 64, False), (128, 256, 96, True), (130, 256, 1024, True), (27, 512, 512, False),
+                                            (400, 1024, 256, False)])
+def test_linear_on_split_floats_in_slices(n, k, n_out, gelu):
+    """Slices of 32 columns: fewer than the ring holds and more, shared by clusters of one to eight, stored as parts and as
+    pieces (96 columns)."""
+    test_linear_on_split_floats(n, k, n_out, gelu, False)
+
+
 @pytest.mark.parametrize("n,cin,cout", [(1, 32, 32), (700, 32, 32), (900, 64, 64), (500, 64, 128), (400, 256, 256),
                                         (60, 512, 512), (40000, 64, 64)])
 def test_subm_conv_on_split_floats(n, cin, cout):
@@ -991,6 +999,12 @@ def test_subm_conv_on_split_floats(n, cin, cout):
     rows = torch.cat([feat.double(), feat.new_zeros(1, cin).double()])[nbr.long()]          # -1 -> the zero row
     ref = torch.einsum("onc,doc->nd", rows, w.double().reshape(cout, 27, cin)) + b.double()
     assert rel_l2(got.double(), ref) < 1.5 * rel_l2(plain.double(), ref) + 1e-7
+
+
+@pytest.mark.parametrize("n,cin,cout", [(1, 64, 64), (129, 64, 192), (2500, 128, 128), (6000, 128, 256)])
+def test_subm_conv_on_split_floats_in_slices(n, cin, cout):
+    """Three stages to a slice of 64 channels: one tile to a cluster, several tiles without one, 64 and 128 columns."""
+    test_subm_conv_on_split_floats(n, cin, cout)
 
 
 @pytest.mark.parametrize("count", [1, 48, 49, 100])
