@@ -83,30 +83,6 @@ struct AtLayout {
     }
 };
 
-// Descriptor of a no-swizzle operand: `lbo` / `sbo` are the leading / stride byte offsets of the canonical layouts
-// (K-major: lbo between the two 8-element halves of K = 16, sbo between 8-row groups; MN-major: lbo between 8-deep K
-// groups, sbo between 8-element chunks along M/N).
-__device__ __forceinline__ uint64_t umma_desc_plain(uint32_t smem_addr, uint32_t lbo, uint32_t sbo)
-{
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_addr & 0x3ffff) >> 4);
-    d |= (uint64_t)(lbo >> 4) << 16;
-    d |= (uint64_t)(sbo >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    return d;
-}
-// D[tmem] (+)= A[tmem] * B[smem]^T: A holds 128 rows (lanes) x 16 bf16 (8 columns of pairs)
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
-                                             bool accumulate)
-{
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"((uint32_t)accumulate)
-        : "memory");
-}
-
 __device__ __forceinline__ uint32_t at_scale_bf16x2(uint32_t v, float s)
 {
     const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v));
@@ -161,14 +137,6 @@ __device__ __forceinline__ void at_probabilities(const uint32_t (&s)[16], uint32
             pk[i] = pack_bf16(fast_exp2(x), fast_exp2(y));
         }
     }
-}
-__device__ __forceinline__ void tmem_ld16_fence(uint32_t (&r)[16])
-{
-    asm volatile("tcgen05.wait::ld.sync.aligned;"
-                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                   "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])
-                 :
-                 : "memory");
 }
 // chunk CH of a block of NCH: x holds it (in flight), y takes the next one
 template <int CH, int NCH>

@@ -419,10 +419,10 @@ def test_attention_with_and_without_reference_value(n, gain):
     assert rel_l2(b, a) < (5e-3 if gain < 10 else 1e-2)
 
 
-@pytest.mark.parametrize("n,K", [(1281, 128), (1290, 129), (700, 65), (1500, 1024), (330, 31)])
+@pytest.mark.parametrize("n,K", [(1281, 128), (1290, 129), (700, 65), (1500, 1024), (330, 31), (63, 64), (48, 17)])
 @pytest.mark.parametrize("gain", [0.3, 8.0])
-def test_attention_fp32_four_queries_per_thread(n, K, gain):
-    """Launches of more than two CTAs to an SM: ragged tiles, patches and chunks of keys, bounded and not, against the
+def test_attention_fp32_many_heads(n, K, gain):
+    """Several CTAs to an SM; ragged tiles, patches, blocks of 64 keys and steps of 16, scores bounded and not, against the
     one-query form (the order of 32-bit sums: a few 2^-24 per term, as in the test below)."""
     C, H = 512, 32
     g = torch.Generator().manual_seed(n)
@@ -435,6 +435,27 @@ def test_attention_fp32_four_queries_per_thread(n, K, gain):
     a = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25, algo=1)
     b = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25)
     assert bool(torch.isfinite(b).all()) and rel_l2(b, a) < 1e-5
+
+
+@pytest.mark.parametrize("where", ["q", "k", "v"])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3e38, -1e30])
+def test_attention_fp32_values_out_of_range(where, value):
+    """Infinities, NaN and values whose products leave the range, in one row of a patch: those outputs are finite that
+    plain arithmetic leaves finite, with the same values."""
+    n, C, H, K = 300, 32, 2, 150
+    g = torch.Generator().manual_seed(3)
+    qkv = torch.randn(n, 3 * C, generator=g)
+    qkv[70, "qkv".index(where) * C + 5] = value
+    qkv = qkv.cuda()
+    order = torch.arange(n).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    b = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25)
+    q, k, v = (t.reshape(2, 150, H, 16).transpose(1, 2) for t in qkv.split(C, dim=1))
+    ref = (torch.softmax((q * 0.25) @ k.transpose(2, 3), 3) @ v).transpose(1, 2).reshape(n, C)
+    assert torch.equal(torch.isfinite(b), torch.isfinite(ref))
+    ok = torch.isfinite(ref)
+    # scores of up to ~8: 8 x 2^-23 in their exponentials, sums of 150 terms
+    torch.testing.assert_close(b[ok], ref[ok], rtol=2e-5, atol=2e-6)
 
 
 @pytest.mark.parametrize("n", [1, 127, 129, 257, 1500])
