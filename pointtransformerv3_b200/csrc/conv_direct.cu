@@ -15,9 +15,9 @@
 // Epilogue: optional bias, optional BatchNorm(eval) scale/shift + exact GELU
 // (model.py:848,860 for the stem), rounding, one contiguous store per thread.
 //
-// bf16 features take the tensor-core form of the same kernel (conv_direct_mma_kernel):
+// bf16 features take the tensor-core form of the same kernel (conv_direct_tc05_kernel):
 // the staged neighbour rows of a few (dx, dy) rows of offsets are the A operand (128 voxels x K = offsets x 8
-// padded channels, zero rows where a neighbour is absent) of mma.sync against that
+// padded channels, zero rows where a neighbour is absent) of tcgen05.mma against that
 // round's slice of the weights; nothing is skipped because the products are cheap - the
 // CUDA-core form spends most of its instructions unpacking bf16 weights for the FMAs.
 #include <algorithm>
@@ -26,6 +26,7 @@
 #include "convert.cuh"
 #include "kmap.cuh"
 #include "mma_util.cuh"
+#include "tc05.cuh"
 #include "voxel_index.cuh"
 #include "plan.cuh"
 #include "vec.cuh"
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(CD_THREADS) conv_direct_kernel(
 
 constexpr int CDM_ROWS = 2;      // (dx, dy) rows of ksize offsets per round; even, so that K is a multiple of 16
 
-// What the kernel reads, once per call: the weights [cout][kvol][cin] -> [offset][8][cout], zero padded to whole
+// What the kernel reads, once per call: the weights [cout][kvol][cin] -> [offset][cout][8], zero padded to whole
 // rounds, and the features with their rows padded to 16 bytes, so that a neighbour is one aligned copy
 __global__ void __launch_bounds__(256) conv_direct_prepare_kernel(const __nv_bfloat16* __restrict__ w,
                                                                   __nv_bfloat16* __restrict__ wt, int cout, int kvol,
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(256) conv_direct_prepare_kernel(const __nv_bfl
 {
     const int64_t first = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
     for (int64_t idx = first; idx < (int64_t)kvol_pad * 8 * cout; idx += step) {
-        const int co = (int)idx % cout, ci = ((int)idx / cout) % 8, o = (int)idx / (8 * cout);
+        const int ci = (int)idx % 8, co = ((int)idx / 8) % cout, o = (int)idx / (8 * cout);
         wt[idx] = (o < kvol && ci < cin) ? w[((size_t)co * kvol + o) * cin + ci] : __float2bfloat16(0.f);
     }
     const unsigned short* f = reinterpret_cast<const unsigned short*>(feat);
@@ -207,15 +208,18 @@ __global__ void __launch_bounds__(256) conv_direct_prepare_kernel(const __nv_bfl
     }
 }
 
-// Bound by the gathers' passes through L1: a warp's 32 voxels touch 32 cell tables.  The cells of a (dx, dy) row
-// lie in at most two aligned groups of four (z runs fastest in a table), so a thread takes the row's offsets of
-// one voxel with two 16-byte loads where it took five of 4 bytes, and copies each neighbour's padded row
-// straight to shared memory.  Two rows per round and six CTAs per SM: four rows with half the CTAs, or the next
-// round's cells loaded ahead in registers, are slower on long inputs.  408 k voxels of four rooms, 6 channels:
-// 348 -> 249 us; 2.05 M of LiDAR frames, 4 channels: 2.06 -> 1.53 ms; 100 k: 99 -> 59 us.
+// The cells of a (dx, dy) row of offsets lie in at most two aligned groups of four (z runs fastest in a table), so a
+// thread takes the row's offsets of one voxel with two 16-byte loads, and copies each neighbour's padded row straight to
+// shared memory: [offset][voxel] of 16 bytes is the K-major layout of an operand without swizzle (a product takes two
+// offsets), [offset][channel] that of the weights.  One thread issues a round's products; while they run, the next
+// round's cells are on their way.  Two rows per round, six CTAs per SM.
+// us, here / with mma.sync, whose fragments (20 of 30 M shared-memory wavefronts, weights again for every 16 voxels) kept
+// that pipe 74 % busy: 6 000 voxels 15.7 / 20.7, 100 000 45.0 / 55.1, 400 000 of four rooms 142 / 179, 2.05 M of LiDAR
+// frames 599 / 817 (no GELU).  Error against 64 bits: that of rounding to bf16 in both, 0.0095 % of the results are not the
+// rounded sum in both.  What bounds it: the gathers' passes through L1, a warp's 32 voxels touch as many cell tables.
 // NT: 8-wide output channel tiles (c_out = 8 NT, NT even)
 template <int NT>
-__global__ void __launch_bounds__(CD_THREADS, NT <= 4 ? 6 : 4) conv_direct_mma_kernel(
+__global__ void __launch_bounds__(CD_THREADS, NT <= 4 ? 6 : 4) conv_direct_tc05_kernel(
     const uint4* __restrict__ feat, const int32_t* __restrict__ indices,
     const __nv_bfloat16* __restrict__ wt, const __nv_bfloat16* __restrict__ bias,
     const float* __restrict__ bn_scale, const float* __restrict__ bn_shift, int apply_gelu,
@@ -223,17 +227,27 @@ __global__ void __launch_bounds__(CD_THREADS, NT <= 4 ? 6 : 4) conv_direct_mma_k
     const unsigned long long* __restrict__ keys, const uint32_t* __restrict__ vals, uint64_t cap_mask,
     const uint32_t* __restrict__ cells, uint32_t* __restrict__ status)
 {
-    constexpr int COUT = 8 * NT;
-    constexpr int WROW = COUT * 2 + 16;   // weight row pitch: 16 bytes of padding keep ldmatrix conflict-free
-    extern __shared__ __align__(16) unsigned char smem[];
+    using namespace tc05;
+    constexpr int COUT = 8 * NT, TM_COLS = COUT <= 32 ? 32 : 64, PER = CDM_ROWS * CD_TM / CD_THREADS;
+    extern __shared__ __align__(128) unsigned char smem[];
     const int per_round = CDM_ROWS * ksize;                      // offsets
     unsigned char* x_s = smem;                                   // [per_round][128] rows of 8 channels (16 B)
-    unsigned char* w_s = smem + per_round * CD_TM * 16;          // [per_round * 8][COUT (+ padding)] of this round
+    unsigned char* w_s = smem + per_round * CD_TM * 16;          // [per_round][COUT] of this round
     __shared__ int row_s[CD_TM];
     __shared__ uint32_t block_s[8][CD_TM];
     __shared__ char2 delta_s[25];                                // (dx, dy) of a row
+    __shared__ __align__(8) uint64_t bar_s;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_s;
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const uint32_t bar = smem_u32_generic(&bar_s);
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        abort_s = 0;
+        fence_barrier_init();
+    }
+    if (warp == 0) tmem_alloc(smem_u32_generic(&tmem_slot), TM_COLS);
     const int v = tid % CD_TM, half = tid / CD_TM;
     const int64_t i = (int64_t)blockIdx.x * CD_TM + v;
     const int64_t row = i < n ? (row_order ? row_order[i] : i) : -1;
@@ -256,22 +270,17 @@ __global__ void __launch_bounds__(CD_THREADS, NT <= 4 ? 6 : 4) conv_direct_mma_k
         }
         block_s[bi][v] = id;
     }
+    fence_before_sync();
     __syncthreads();
-
-    float acc[NT][4];
-#pragma unroll
-    for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    fence_after_sync();
+    const uint32_t tm = tmem_slot;
     const uint32_t xs_base = smem_u32(x_s), ws_base = smem_u32(w_s);
 
-    for (int row0 = 0; row0 < n_rows; row0 += CDM_ROWS) {
-        // this round's weights: per_round * 8 rows of COUT
-        for (int idx = tid; idx < per_round * COUT; idx += CD_THREADS)
-            cp_async16(ws_base + (idx / NT) * WROW + (idx % NT) * 16,
-                       wt + ((size_t)row0 * ksize * 8 * COUT + (size_t)idx * 8));
-        // the neighbours of a voxel along one row
-        uint4 cell[CDM_ROWS * CD_TM / CD_THREADS][2];
+    // the neighbours of a voxel along the rows of a round
+    uint4 cell[PER][2];
+    auto load_cells = [&](int row0) {
 #pragma unroll
-        for (int k = 0; k < CDM_ROWS * CD_TM / CD_THREADS; ++k) {
+        for (int k = 0; k < PER; ++k) {
             const int row = row0 + half + k * (CD_THREADS / CD_TM);
             cell[k][0] = cell[k][1] = make_uint4(VI_NO_ROW, VI_NO_ROW, VI_NO_ROW, VI_NO_ROW);
             if (c.x >= 0 && row < n_rows) {
@@ -285,8 +294,17 @@ __global__ void __launch_bounds__(CD_THREADS, NT <= 4 ? 6 : 4) conv_direct_mma_k
                     cell[k][1] = *reinterpret_cast<const uint4*>(cells + (size_t)id1 * 64 + at);
             }
         }
+    };
+    load_cells(0);
+    bool ok = true;
+    int phase = 1;                     // of the round before
+    for (int row0 = 0; row0 < n_rows; row0 += CDM_ROWS, phase ^= 1) {
+        if (row0) ok &= mbar_wait(bar, phase, &abort_s);
+        // this round's weights: per_round planes of COUT rows
+        for (int idx = tid; idx < per_round * COUT; idx += CD_THREADS)
+            cp_async16(ws_base + idx * 16, wt + (size_t)row0 * ksize * 8 * COUT + (size_t)idx * 8);
 #pragma unroll
-        for (int k = 0; k < CDM_ROWS * CD_TM / CD_THREADS; ++k) {
+        for (int k = 0; k < PER; ++k) {
             // entry 0 becomes the cell of dz = -r
             const int s0 = (c.w - r) & 3;
             uint32_t e[8] = {cell[k][0].x, cell[k][0].y, cell[k][0].z, cell[k][0].w,
@@ -301,43 +319,42 @@ __global__ void __launch_bounds__(CD_THREADS, NT <= 4 ? 6 : 4) conv_direct_mma_k
                 if (q < ksize) cp_async16_zfill(dst + q * CD_TM * 16, feat + (e[q] != VI_NO_ROW ? e[q] : 0u), e[q] != VI_NO_ROW);
         }
         cp_async_commit();
+        if (row0 + CDM_ROWS < n_rows) load_cells(row0 + CDM_ROWS);
         cp_async_wait<0>();
+        fence_proxy_async();
         __syncthreads();
-        // out[16 voxels of this warp][COUT] += X[16][K] . W[K][COUT]
-#pragma unroll 5
-        for (int ks = 0; ks < per_round / 2; ++ks) {
-            uint32_t a[4];
-            {
-                const int mi = lane >> 3, rr = lane & 7;
-                const int vv = 16 * warp + (mi & 1) * 8 + rr, ol = 2 * ks + (mi >> 1);
-                ldmatrix_x4(a, xs_base + (ol * CD_TM + vv) * 16);
+        // out[128 voxels][COUT] += X[128][K] . W[COUT][K]^T, two offsets to a product
+        if (warp == 0) {
+            if (elect_one()) {
+                const uint64_t dx = umma_desc_plain(xs_base, CD_TM * 16, 128), dw = umma_desc_plain(ws_base, COUT * 16, 128);
+                for (int ks = 0; ks < per_round / 2; ++ks)
+                    umma_bf16(tm, dx + (uint64_t)(ks * 2 * CD_TM), dw + (uint64_t)(ks * 2 * COUT), umma_idesc_bf16(CD_TM, COUT),
+                              row0 > 0 || ks > 0);
+                umma_commit(bar);
             }
-#pragma unroll
-            for (int np = 0; np < NT / 2; ++np) {
-                uint32_t b[4];
-                const int mi = lane >> 3, rr = lane & 7;
-                const int kk = 16 * ks + (mi & 1) * 8 + rr, n0 = np * 16 + (mi >> 1) * 8;
-                ldmatrix_x4_trans(b, ws_base + kk * WROW + n0 * 2);
-                mma_bf16(acc[2 * np], a, b[0], b[1]);
-                mma_bf16(acc[2 * np + 1], a, b[2], b[3]);
-            }
+            __syncwarp();
         }
-        __syncthreads();
     }
     if (overflow) atomicOr(status, PTV3_STATUS_PROBE_LIMIT);
+    ok &= mbar_wait(bar, phase, &abort_s);
+    __syncwarp();
+    fence_after_sync();
 
-    const int g = lane >> 2, t = lane & 3;
+    // thread = voxel, half of its channels
+    const int q = warp & 3, c0 = (warp >> 2) * (COUT / 2), orow = row_s[q * 32 + lane];
+    const bool wide = ((uintptr_t)out & 15) == 0;
 #pragma unroll
-    for (int hrow = 0; hrow < 2; ++hrow) {
-        const int orow = row_s[16 * warp + g + 8 * hrow];
-        if (orow < 0) continue;
-        uint32_t* op = reinterpret_cast<uint32_t*>(out + (int64_t)orow * COUT);
+    for (int g = 0; g < NT / 2; ++g) {
+        uint32_t acc[8], packed[4];
+        __syncwarp();
+        tmem_ld8(tm + ((uint32_t)(q * 32) << 16) + c0 + 8 * g, acc);
+        tmem_ld8_fence(acc);
 #pragma unroll
-        for (int jn = 0; jn < NT; ++jn) {
-            float y[2] = {acc[jn][2 * hrow], acc[jn][2 * hrow + 1]};
+        for (int p = 0; p < 4; ++p) {
+            float y[2] = {__uint_as_float(acc[2 * p]), __uint_as_float(acc[2 * p + 1])};
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const int ch = 8 * jn + 2 * t + e;
+                const int ch = c0 + 8 * g + 2 * p + e;
                 if (bias) y[e] += __bfloat162float(bias[ch]);
                 if (bn_scale) {
                     // the convolution output is rounded to the element type first, as a
@@ -350,9 +367,27 @@ __global__ void __launch_bounds__(CD_THREADS, NT <= 4 ? 6 : 4) conv_direct_mma_k
                     y[e] = cd_gelu(y[e]);
                 }
             }
-            op[4 * jn + t] = pack_bf16(y[0], y[1]);
+            packed[p] = pack_bf16(y[0], y[1]);
+        }
+        __nv_bfloat16* op = out + (int64_t)orow * COUT + c0 + 8 * g;
+        if (orow >= 0 && wide) {
+            *reinterpret_cast<uint4*>(op) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+        } else if (orow >= 0) {
+#pragma unroll
+            for (int p = 0; p < 4; ++p) reinterpret_cast<uint32_t*>(op)[p] = packed[p];
         }
     }
+    fence_before_sync();
+    __syncthreads();
+    if (warp == 0) {
+        if (!ok) {
+            int give_up = 0;           // products that were waited for in vain: once more, with a limit
+            mbar_wait(bar, phase, &give_up);
+        }
+        fence_after_sync();
+        tmem_dealloc(tm, TM_COLS);
+    }
+    if (lane == 0 && !ok) atomicOr(status, PTV3_STATUS_WAIT_LIMIT);
 }
 
 // laid-out weights (whole rounds)
@@ -373,11 +408,11 @@ static int launch_conv_direct_mma(const void* feat, const int32_t* indices, cons
     conv_direct_prepare_kernel<<<(unsigned)std::min<int64_t>(prepare, SMS * 8), 256, 0, stream>>>(
         (const __nv_bfloat16*)weight, (__nv_bfloat16*)wt, cout, kvol, cin, rounds * per_round, (const __nv_bfloat16*)feat,
         rows, n);
-    const size_t smem = (size_t)per_round * CD_TM * 16 + (size_t)per_round * 8 * (cout * 2 + 16);
+    const size_t smem = (size_t)per_round * (CD_TM + cout) * 16;
     const unsigned blocks = (unsigned)((n + CD_TM - 1) / CD_TM);
 #define CDM_LAUNCH(NT)                                                                                      \
     do {                                                                                                    \
-        auto kern = conv_direct_mma_kernel<NT>;                                                             \
+        auto kern = conv_direct_tc05_kernel<NT>;                                                            \
         if (allow_smem(kern) != cudaSuccess)                                                \
             return check_launch("ptv3_subm_conv_direct_fwd: shared memory attribute");                      \
         kern<<<blocks, CD_THREADS, smem, stream>>>(                                                          \

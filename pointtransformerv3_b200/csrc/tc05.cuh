@@ -240,6 +240,13 @@ __device__ __forceinline__ void tmem_ld8_fence(uint32_t (&r)[8], uint32_t (&q)[8
                  :
                  : "memory");
 }
+__device__ __forceinline__ void tmem_ld8_fence(uint32_t (&r)[8])
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7])
+                 :
+                 : "memory");
+}
 __device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t* r)
 {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),
