@@ -2,39 +2,59 @@
 
 namespace ptv3 {
 
-// every voxel claims its block: the first claimant takes the next table and clears it
+// Every voxel claims its block: the first claimant takes the next table and clears it.  A block of threads counts its
+// claims and asks for their numbers at once, and a warp clears its lanes' tables one after another, a table to an
+// instruction.  (Numbers asked for one by one, additions on one address, and tables cleared by the thread that claimed
+// them, 16 bytes of 32 tables to an instruction: 2.05 M LiDAR voxels 147 us for 68, 400 000 of rooms 15.3 for 8.4, 85 000
+// 4.9 for 4.1, 6 000 3.7 for 3.2.)
 __global__ void __launch_bounds__(256) vi_block_insert_kernel(const int32_t* indices, int64_t n,
                                                               unsigned long long* keys, uint32_t* vals,
                                                               uint64_t cap_mask, uint32_t* counter, uint32_t* cells,
                                                               uint32_t* status)
 {
+    __shared__ uint32_t claims[8], base;
     pdl_launch_next();
     pdl_wait();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int4 v = reinterpret_cast<const int4*>(indices)[i];
-    uint64_t key;
-    if ((unsigned)v.y > 0xffffu || (unsigned)v.z > 0xffffu || (unsigned)v.w > 0xffffu ||
-        !vi_block_key(v.x, v.y >> 2, v.z >> 2, v.w >> 2, key)) {
-        atomicOr(status, PTV3_STATUS_BAD_INDEX);
-        return;
-    }
-    uint64_t slot = km_mix(key) & cap_mask;
-    for (uint64_t probe = 0; probe <= cap_mask; ++probe) {
-        const unsigned long long prev = atomicCAS(&keys[slot], KM_EMPTY, key);
-        if (prev == KM_EMPTY) {
-            const uint32_t id = atomicAdd(counter, 1u);
-            uint4* tab = reinterpret_cast<uint4*>(cells + (size_t)id * 64);
-#pragma unroll
-            for (int q = 0; q < 16; ++q) tab[q] = make_uint4(VI_NO_ROW, VI_NO_ROW, VI_NO_ROW, VI_NO_ROW);
-            __threadfence();
-            vals[slot] = id;
-            return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    bool claimed = false;
+    uint64_t slot = 0;
+    if (i < n) {
+        const int4 v = reinterpret_cast<const int4*>(indices)[i];
+        uint64_t key;
+        if ((unsigned)v.y > 0xffffu || (unsigned)v.z > 0xffffu || (unsigned)v.w > 0xffffu ||
+            !vi_block_key(v.x, v.y >> 2, v.z >> 2, v.w >> 2, key)) {
+            atomicOr(status, PTV3_STATUS_BAD_INDEX);
+        } else {
+            slot = km_mix(key) & cap_mask;
+            uint64_t probe = 0;
+            for (; probe <= cap_mask; ++probe) {
+                const unsigned long long prev = atomicCAS(&keys[slot], KM_EMPTY, key);
+                claimed = prev == KM_EMPTY;
+                if (claimed || prev == key) break;
+                slot = (slot + 1) & cap_mask;
+            }
+            if (probe > cap_mask) atomicOr(status, PTV3_STATUS_PROBE_LIMIT);
         }
-        if (prev == key) return;
-        slot = (slot + 1) & cap_mask;
     }
-    atomicOr(status, PTV3_STATUS_PROBE_LIMIT);
+    const uint32_t mine = __ballot_sync(0xffffffffu, claimed);
+    if (lane == 0) claims[warp] = __popc(mine);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t all = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            const uint32_t c = claims[w];
+            claims[w] = all;
+            all += c;
+        }
+        base = all ? atomicAdd(counter, all) : 0u;
+    }
+    __syncthreads();
+    const uint32_t first = base + claims[warp];
+    if (claimed) vals[slot] = first + __popc(mine & ((1u << lane) - 1));
+    uint2* tables = reinterpret_cast<uint2*>(cells + (size_t)first * 64) + lane;
+    for (int t = 0; t < __popc(mine); ++t) tables[t * 32] = make_uint2(VI_NO_ROW, VI_NO_ROW);
 }
 
 // second pass (all tables exist now): every voxel writes its row into its cell;
