@@ -174,7 +174,7 @@ static int launch_attn_fma(const void* qkv, const int64_t* order, const int64_t*
 static int attention_impl(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad,
                           const int32_t* cu_seqlens, void* out, int64_t n, int n_seq, int max_seqlen,
                           int channels, int heads, float scale, int dtype, int algo, ptv3::RpeArgs rpe,
-                          bool planned, uint32_t* status, void* stream)
+                          bool planned, uint32_t* status, void* stream, bool split = false)
 {
     using namespace ptv3;
     PTV3_REQUIRE(n >= 0 && n_seq >= 0 && max_seqlen >= 1 && channels >= 1 && heads >= 1 &&
@@ -205,15 +205,29 @@ static int attention_impl(const void* qkv, const int64_t* order, const int64_t* 
     if (mma_ok && algo != 1)
         return launch_attn_mma(qkv, order, pad, unpad, cu_seqlens, out, n_seq, max_seqlen, channels,
                                heads, scale, algo == 3, planned, status, (cudaStream_t)stream);
-    if (dtype == PTV3_DTYPE_F32 && algo == 0 && !rpe.grid_coord && channels / heads == 16 &&
-        (((uintptr_t)qkv | (uintptr_t)out) & 15) == 0)
-        return launch_attn_f32(qkv, order, pad, unpad, cu_seqlens, out, n_seq, max_seqlen, channels, heads, scale, status,
-                               (cudaStream_t)stream);
+    if (dtype == PTV3_DTYPE_F32 && !rpe.grid_coord && attention_splits(qkv, channels, heads, algo) &&
+        ((uintptr_t)out & 15) == 0)
+        return launch_attn_f32(qkv, order, pad, unpad, cu_seqlens, out, split, n_seq, max_seqlen, channels, heads, scale,
+                               status, (cudaStream_t)stream);
+    PTV3_REQUIRE(!split, PTV3_ERR_INVALID_ARGUMENT, "ptv3_attention_fwd: no split rows from this form");
     if (dtype == PTV3_DTYPE_F32)
         return launch_attn_fma<float>(qkv, order, pad, unpad, cu_seqlens, out, n_seq, max_seqlen,
                                       channels, heads, scale, rpe, status, (cudaStream_t)stream);
     return launch_attn_fma<__nv_bfloat16>(qkv, order, pad, unpad, cu_seqlens, out, n_seq, max_seqlen,
                                           channels, heads, scale, rpe, status, (cudaStream_t)stream);
+}
+
+bool ptv3::attention_splits(const void* qkv, int channels, int heads, int algo)
+{
+    return algo == 0 && channels / heads == 16 && ((uintptr_t)qkv & 15) == 0;
+}
+
+int ptv3::attention_split(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad,
+                          const int32_t* cu_seqlens, void* split_out, int64_t n, int n_seq, int max_seqlen, int channels,
+                          int heads, float scale, uint32_t* status, cudaStream_t stream)
+{
+    return attention_impl(qkv, order, pad, unpad, cu_seqlens, split_out, n, n_seq, max_seqlen, channels, heads, scale,
+                          PTV3_DTYPE_F32, 0, RpeArgs{nullptr, nullptr, 0, 0, 0}, false, status, stream, true);
 }
 
 int ptv3::attention_fwd(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad,

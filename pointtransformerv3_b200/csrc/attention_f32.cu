@@ -91,6 +91,7 @@ struct AxArgs {
     const int64_t *order, *pad, *unpad;
     const int32_t* cu;
     float* out;
+    __nv_bfloat16* split_out;        // the result as split rows instead
     int C, heads;
     float scale;
     uint32_t* status;
@@ -406,18 +407,25 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
 #pragma unroll
         for (int d = 0; d < AX_D; ++d) acc[d] *= inv;
     }
+    if (a.split_out) {
+#pragma unroll
+        for (int d = 0; d < AX_D; d += 8)
+            split_store8(a.split_out + mine * split_stored(a.C) * a.C, h * AX_D + d, a.C, acc + d);
+        return;
+    }
     float4* op = reinterpret_cast<float4*>(a.out + mine * a.C + h * AX_D);
 #pragma unroll
     for (int d = 0; d < 4; ++d) op[d] = make_float4(acc[4 * d], acc[4 * d + 1], acc[4 * d + 2], acc[4 * d + 3]);
 }
 
 int launch_attn_f32(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad, const int32_t* cu,
-                    void* out, int n_seq, int max_seqlen, int C, int H, float scale, uint32_t* status,
+                    void* out, bool split, int n_seq, int max_seqlen, int C, int H, float scale, uint32_t* status,
                     cudaStream_t stream)
 {
     const int tiles = (max_seqlen + AX_QT - 1) / AX_QT;
     launch_dependent(attn_f32_d16_kernel, dim3(H * tiles, n_seq), dim3(AX_THREADS), 0, stream,
-                     AxArgs{(const float*)qkv, order, pad, unpad, cu, (float*)out, C, H, scale, status});
+                     AxArgs{(const float*)qkv, order, pad, unpad, cu, split ? nullptr : (float*)out,
+                            split ? (__nv_bfloat16*)out : nullptr, C, H, scale, status});
     count_launches(1);
     return check_launch("ptv3_attention_fwd");
 }

@@ -22,8 +22,9 @@ int launch_attn_tc05(const void* qkv, const int64_t* order, const int64_t* pad, 
                      int heads, float scale, bool planned, uint32_t* status, cudaStream_t stream);
 
 // fp32, head dimension 16 (attention_f32.cu); rows 16-byte aligned
-int launch_attn_f32(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad,
-                    const int32_t* cu_seqlens, void* out, int n_seq, int max_seqlen, int channels, int heads,
-                    float scale, uint32_t* status, cudaStream_t stream);
+// out: fp32 rows, or with `split` bf16 ones (split_f32.cuh)
+int launch_attn_f32(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad, const int32_t* cu,
+                    void* out, bool split, int n_seq, int max_seqlen, int C, int H, float scale, uint32_t* status,
+                    cudaStream_t stream);
 
 }  // namespace ptv3

@@ -77,9 +77,10 @@ static size_t carve_block(const ptv3_block_args* a, void* base, BlockBuffers* b)
 
 // ---- fp32: the same block with every product on split operands (split_f32.cuh) -----------------------
 // Layers hand their result to the next product as split rows where nothing else reads it (convolution ->
-// Linear, fc1 -> fc2); the others are split by a kernel of their own.
+// Linear, norm -> qkv and fc1, attention -> projection, fc1 -> fc2); the block's input is split by a kernel of its own.  (All
+// but the first and last of these by kernels, 2.6 us each: two rooms of 20 000 points 4 430 us a pass, 4 333 so.)
 struct BlockBuffersF32 {
-    float *y, *f1, *a, *qkv, *att, *f2;
+    float *y, *f1, *qkv, *att, *f2;
     void *s, *sh;           // split rows of width C (at most 6C bf16) and of the hidden width
 };
 
@@ -90,7 +91,6 @@ static size_t carve_block_f32(const ptv3_block_args* a, void* base, BlockBuffers
     BlockBuffersF32 t;
     t.y = (float*)c.take<char>(row);
     t.f1 = (float*)c.take<char>(row);
-    t.a = (float*)c.take<char>(row);
     t.qkv = (float*)c.take<char>(3 * row);
     t.f2 = (float*)c.take<char>(row);
     t.att = t.y;
@@ -118,19 +118,20 @@ static int block_f32(const ptv3_block_args* a, bool settled, cudaStream_t stream
     STEP(launch_conv_split(b.sh, a->nbr, a->conv_weight, f(a->conv_bias), nullptr, b.s, a->row_order, n, C, C, 27,
                            a->status, stream));
     STEP(launch_linear_split(b.s, a->cpe_w, f(a->cpe_b), nullptr, b.y, nullptr, n, C, C, 0, settled, a->status, stream));
-    STEP(ptv3_add_layernorm_fwd(b.y, a->feat, a->cpe_ln_w, a->cpe_ln_b, a->cpe_ln_eps, b.f1, a->n1_w, a->n1_b, a->n1_eps,
-                                b.a, n, C, PTV3_DTYPE_F32, stream));
-    STEP(launch_split_f32(b.a, n, C, b.s, stream));
+    STEP(add_layernorm_split(b.y, f(a->feat), f(a->cpe_ln_w), f(a->cpe_ln_b), a->cpe_ln_eps, b.f1, f(a->n1_w), f(a->n1_b),
+                             a->n1_eps, b.s, n, C, stream));
     STEP(launch_linear_split(b.s, a->qkv_w, f(a->qkv_b), nullptr, b.qkv, nullptr, n, C, 3 * C, 0, settled, a->status,
                              stream));
-    STEP(ptv3_attention_fwd(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.att, n, a->n_seq, a->max_seqlen, C, a->heads,
-                            a->scale, PTV3_DTYPE_F32, a->attention_algo, a->status, stream));
-    STEP(launch_split_f32(b.att, n, C, b.s, stream));
-    // (b.a is free until the second norm)
+    if (attention_splits(b.qkv, C, a->heads, a->attention_algo)) {
+        STEP(attention_split(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.s, n, a->n_seq, a->max_seqlen, C, a->heads,
+                             a->scale, a->status, stream));
+    } else {
+        STEP(ptv3_attention_fwd(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.att, n, a->n_seq, a->max_seqlen, C,
+                                a->heads, a->scale, PTV3_DTYPE_F32, a->attention_algo, a->status, stream));
+        STEP(launch_split_f32(b.att, n, C, b.s, stream));
+    }
     STEP(launch_linear_split(b.s, a->proj_w, f(a->proj_b), nullptr, b.qkv, nullptr, n, C, C, 0, settled, a->status, stream));
-    STEP(ptv3_add_layernorm_fwd(b.qkv, b.f1, nullptr, nullptr, 0.f, b.f2, a->n2_w, a->n2_b, a->n2_eps, b.a, n, C,
-                                PTV3_DTYPE_F32, stream));
-    STEP(launch_split_f32(b.a, n, C, b.s, stream));
+    STEP(add_layernorm_split(b.qkv, b.f1, nullptr, nullptr, 0.f, b.f2, f(a->n2_w), f(a->n2_b), a->n2_eps, b.s, n, C, stream));
     STEP(launch_linear_split(b.s, a->fc1_w, f(a->fc1_b), nullptr, nullptr, b.sh, n, C, H, 1, settled, a->status, stream));
     STEP(launch_linear_split(b.sh, a->fc2_w, f(a->fc2_b), b.f2, (float*)a->out, nullptr, n, H, C, 0, settled, a->status,
                              stream));

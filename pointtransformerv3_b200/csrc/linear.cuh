@@ -45,6 +45,16 @@ int mlp_fwd(const void* x, const void* fc1_weight, const void* fc1_bias, const v
             const void* residual, void* out, int64_t n, int channels, int hidden, int dtype, bool settled,
             uint32_t* status, cudaStream_t stream);
 
+// ptv3_add_layernorm_fwd in fp32 whose second norm leaves as split rows (split_f32.cuh)
+int add_layernorm_split(const float* x, const float* residual, const float* ln1_weight, const float* ln1_bias, float ln1_eps,
+                        float* sum_out, const float* ln2_weight, const float* ln2_bias, float ln2_eps, void* norm_split,
+                        int64_t n, int channels, cudaStream_t stream);
+
+// ptv3_attention_fwd in fp32 whose result leaves as split rows, where attention_splits says that it can
+bool attention_splits(const void* qkv, int channels, int heads, int algo);
+int attention_split(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad,
+                    const int32_t* cu_seqlens, void* split_out, int64_t n, int n_seq, int max_seqlen, int channels, int heads,
+                    float scale, uint32_t* status, cudaStream_t stream);
 int attention_fwd(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad, const int32_t* cu_seqlens,
                   void* out, int64_t n, int n_seq, int max_seqlen, int channels, int heads, float scale, int dtype,
                   int algo, bool planned, uint32_t* status, cudaStream_t stream);

@@ -13,6 +13,7 @@
 // or written once, with 16-byte accesses; a row is owned by 4..32 lanes.
 #include "bn.cuh"
 #include "common.cuh"
+#include "split_f32.cuh"
 #include "vec.cuh"
 #include "../../include/ptv3_b200.h"
 
@@ -30,7 +31,7 @@ __device__ __forceinline__ float group_sum(float v)
 template <typename T, int LANES, int VPL>
 __global__ void __launch_bounds__(256) add_ln_kernel(
     const T* x, const T* residual, const T* g1, const T* b1, float eps1, T* sum_out, const T* g2, const T* b2,
-    float eps2, T* norm_out, int64_t n, int C)
+    float eps2, T* norm_out, __nv_bfloat16* norm_split, int64_t n, int C)
 {
     pdl_launch_next();
     pdl_wait();
@@ -91,9 +92,17 @@ __global__ void __launch_bounds__(256) add_ln_kernel(
         for (int k = 0; k < VPL; ++k)
             *reinterpret_cast<typename V::Raw*>(sum_out + row * C + ch(k)) = V::pack(v + k * V::N);
     }
-    if (norm_out) {
+    if (norm_out || norm_split) {
         layer_norm(g2, b2, eps2);
-        if (active) {
+        if constexpr (V::N == 4) {
+            // fp32: for a product on split operands (split_f32.cuh)
+            if (norm_split && active) {
+#pragma unroll
+                for (int k = 0; k < VPL; ++k)
+                    split_store4(norm_split + row * split_stored(C) * C, ch(k), C, v + k * V::N);
+            }
+        }
+        if (norm_out && active) {
 #pragma unroll
             for (int k = 0; k < VPL; ++k)
                 *reinterpret_cast<typename V::Raw*>(norm_out + row * C + ch(k)) = V::pack(v + k * V::N);
@@ -104,21 +113,21 @@ __global__ void __launch_bounds__(256) add_ln_kernel(
 template <typename T, int LANES, int VPL>
 static void launch_add_ln(const void* x, const void* residual, const void* g1, const void* b1, float eps1,
                           void* sum_out, const void* g2, const void* b2, float eps2, void* norm_out,
-                          int64_t n, int C, cudaStream_t stream)
+                          void* norm_split, int64_t n, int C, cudaStream_t stream)
 {
     const int64_t threads = n * LANES;
     launch_dependent(add_ln_kernel<T, LANES, VPL>, dim3((unsigned)((threads + 255) / 256)), dim3(256), 0, stream,
                      (const T*)x, (const T*)residual, (const T*)g1, (const T*)b1, eps1, (T*)sum_out, (const T*)g2,
-                     (const T*)b2, eps2, (T*)norm_out, n, C);
+                     (const T*)b2, eps2, (T*)norm_out, (__nv_bfloat16*)norm_split, n, C);
 }
 
 template <typename T>
 static int dispatch_add_ln(const void* x, const void* residual, const void* g1, const void* b1, float eps1,
                            void* sum_out, const void* g2, const void* b2, float eps2, void* norm_out,
-                           int64_t n, int C, cudaStream_t stream)
+                           void* norm_split, int64_t n, int C, cudaStream_t stream)
 {
     const int vectors = C / Vec<T>::N;   // per row
-#define ALN(L, V) launch_add_ln<T, L, V>(x, residual, g1, b1, eps1, sum_out, g2, b2, eps2, norm_out, n, C, stream)
+#define ALN(L, V) launch_add_ln<T, L, V>(x, residual, g1, b1, eps1, sum_out, g2, b2, eps2, norm_out, norm_split, n, C, stream)
     switch (vectors) {
         case 1: ALN(1, 1); break;
         case 2: ALN(2, 1); break;
@@ -142,6 +151,18 @@ static int dispatch_add_ln(const void* x, const void* residual, const void* g1, 
 #undef ALN
     count_launches(1);
     return check_launch("ptv3_add_layernorm_fwd");
+}
+
+int add_layernorm_split(const float* x, const float* residual, const float* ln1_weight, const float* ln1_bias, float ln1_eps,
+                        float* sum_out, const float* ln2_weight, const float* ln2_bias, float ln2_eps, void* norm_split,
+                        int64_t n, int channels, cudaStream_t stream)
+{
+    PTV3_REQUIRE(channels % 4 == 0, PTV3_ERR_UNSUPPORTED, "ptv3_add_layernorm_fwd: channels %d not a multiple of 4", channels);
+    if (n == 0) return PTV3_OK;
+    PTV3_REQUIRE(x && (ln1_weight == nullptr) == (ln1_bias == nullptr) && ln2_weight && ln2_bias && norm_split,
+                 PTV3_ERR_INVALID_ARGUMENT, "ptv3_add_layernorm_fwd: null pointer");
+    return dispatch_add_ln<float>(x, residual, ln1_weight, ln1_bias, ln1_eps, sum_out, ln2_weight, ln2_bias, ln2_eps,
+                                  nullptr, norm_split, n, channels, stream);
 }
 
 __global__ void __launch_bounds__(128) bn_affine_kernel(const __grid_constant__ BnJobs jobs) { bn_layer(jobs, blockIdx.x); }
@@ -187,9 +208,9 @@ extern "C" int ptv3_add_layernorm_fwd(const void* x, const void* residual, const
     PTV3_REQUIRE(x, PTV3_ERR_INVALID_ARGUMENT, "ptv3_add_layernorm_fwd: null input");
     if (dtype == PTV3_DTYPE_F32)
         return dispatch_add_ln<float>(x, residual, ln1_weight, ln1_bias, ln1_eps, sum_out, ln2_weight,
-                                      ln2_bias, ln2_eps, norm_out, n, channels, (cudaStream_t)stream);
+                                      ln2_bias, ln2_eps, norm_out, nullptr, n, channels, (cudaStream_t)stream);
     return dispatch_add_ln<__nv_bfloat16>(x, residual, ln1_weight, ln1_bias, ln1_eps, sum_out, ln2_weight,
-                                          ln2_bias, ln2_eps, norm_out, n, channels, (cudaStream_t)stream);
+                                          ln2_bias, ln2_eps, norm_out, nullptr, n, channels, (cudaStream_t)stream);
 }
 
 extern "C" int ptv3_bn_affine(const ptv3_bn_args* layers, int count, float* out, void* stream)

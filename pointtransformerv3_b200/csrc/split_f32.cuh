@@ -67,6 +67,23 @@ __device__ __forceinline__ void split_store8(__nv_bfloat16* row, int c, int k, c
     }
 }
 
+// four values of an A row
+__device__ __forceinline__ void split_store4(__nv_bfloat16* row, int c, int k, const float* y)
+{
+    uint2 p[3];
+    __nv_bfloat16* q = reinterpret_cast<__nv_bfloat16*>(p);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) split3(y[i], q[i], q[4 + i], q[8 + i]);
+    if (k % 64 == 0) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) *reinterpret_cast<uint2*>(row + i * k + c) = p[i];
+    } else {
+        const int part[6] = {0, 0, 0, 1, 1, 2};
+#pragma unroll
+        for (int i = 0; i < 6; ++i) *reinterpret_cast<uint2*>(row + i * k + c) = p[part[i]];
+    }
+}
+
 // rows x k floats -> rows x split_stored(k) k bf16, as A rows
 int launch_split_f32(const float* x, int64_t rows, int k, void* out, cudaStream_t stream);
 // ... as B rows, any number of weights
