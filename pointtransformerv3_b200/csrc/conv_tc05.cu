@@ -22,9 +22,11 @@
 //
 // A cluster of up to eight CTAs shares one tile.  Each takes a
 // contiguous share of the tile's stages; the partial sums meet in shared memory and every CTA adds the
-// peers' parts of its rows, in rank order, through distributed shared memory.  A tile alone walks
+// parts of its rows, which the peers have stored with it, in rank order.  A tile alone walks
 // 27 x c_in / 64 stages one after the other, 49 us at 512 channels on 27 voxels, while most SMs have nothing; in
 // clusters of eight that is 10 us.
+// Stored with the CTA that adds them, not read from the peers: us, 487 x 128 9.0 / 8.0, 178 x 256 10.1 / 9.4, 822 x 256 11.7 /
+// 11.2; fp32 822 x 256 26.7 / 23.5, 261 x 512 48.5 / 45.4.
 //
 // Replaces spconv.SubMConv3d.forward at model.py:546-552.
 // Useful work: 2 . pairs . C_in . C_out FLOP.  Every mbarrier wait is bounded and reports through
@@ -83,7 +85,7 @@ __device__ __forceinline__ void ct_store_f32(const ConvTcArgs& a, int64_t row, i
 constexpr int CT_BF16 = 0, CT_PIECES = 1, CT_PARTS = 2;
 
 template <int BN, int STAGES, int NI, bool SPLIT, int FORM>
-__global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(const __grid_constant__ CUtensorMap map_w,
+__global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32, 1) conv_tc05_kernel(const __grid_constant__ CUtensorMap map_w,
                                                                const ConvTcArgs a)
 {
     constexpr bool F32 = FORM != CT_BF16;
@@ -254,71 +256,9 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
                                     full0 + 8 * cur.slot, lane);
             cur.step<NGW, STAGES>(kchunks);
         }
-
-        // ---- epilogue: thread = voxel ----------------------------------------------------------
         if (nit > 0) {
             ok &= mbar_wait(accfull, 0, abort);
             fence_after_sync();
-        }
-        const bool read_acc = nit > 0 && __all_sync(0xffffffffu, ok);    // tcgen05.ld is warp-wide
-        const int q = warp & 3, half = warp >> 2;      // lane quarter of tensor memory, half of the columns
-        const int64_t v = rows_s[q * 32 + lane];
-        const uint32_t tm = tmem_base + ((uint32_t)(q * 32) << 16);
-        constexpr int NCB = BN / 32;                   // 32-column blocks, split between the two halves
-#pragma unroll 1
-        for (int cb = half * ((NCB + 1) / 2); cb < (half == 0 ? (NCB + 1) / 2 : NCB); ++cb) {
-            uint32_t acc[32];
-            if (F32) {
-                // from the small products to the leading ones, issuer after issuer
-#pragma unroll
-                for (int e = 0; e < 32; ++e) acc[e] = 0;
-#pragma unroll 1
-                for (int z = ACCS - 1; z >= 0; --z)
-#pragma unroll 1
-                    for (int i = 0; i < NI; ++i) {
-                        if (!read_acc || !((*reinterpret_cast<volatile uint32_t*>(used_s + i) >> z) & 1)) continue;
-                        uint32_t more[32];
-                        tmem_ld32(tm + (i * ACCS + z) * BN + cb * 32, more);
-                        tmem_ld_wait();
-                        tmem_ld_fence(more);
-#pragma unroll
-                        for (int e = 0; e < 32; ++e)
-                            acc[e] = __float_as_uint(__uint_as_float(acc[e]) + __uint_as_float(more[e]));
-                    }
-            } else if (read_acc) {
-                tmem_ld32(tm + cb * 32, acc);
-                tmem_ld_wait();
-                // the other issuers' partial sums, added in a fixed order
-#pragma unroll 1
-                for (int i = 1; i < NI && i < nit; ++i) {
-                    uint32_t more[32];
-                    tmem_ld32(tm + i * BN + cb * 32, more);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int e = 0; e < 32; ++e)
-                        acc[e] = __float_as_uint(__uint_as_float(acc[e]) + __uint_as_float(more[e]));
-                }
-            } else {
-#pragma unroll
-                for (int i = 0; i < 32; ++i) acc[i] = 0;
-            }
-            if (SPLIT) {
-                // (the ring is free: every product has completed)
-                float* prow = reinterpret_cast<float*>(smem) + (q * 32 + lane) * PART_PITCH + cb * 32;
-#pragma unroll
-                for (int g = 0; g < 8; ++g)
-                    *reinterpret_cast<uint4*>(prow + g * 4) = make_uint4(acc[g * 4], acc[g * 4 + 1], acc[g * 4 + 2],
-                                                                         acc[g * 4 + 3]);
-                continue;
-            }
-            if (v < 0) continue;
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                float y[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) y[i] = __uint_as_float(acc[g * 8 + i]) + bias_s[cb * 32 + g * 8 + i];
-                ct_store_f32(a, v, col0 + cb * 32 + g * 8, y);
-            }
         }
     } else if (FORM == CT_PARTS) {
         // ---- the issuer, fp32 from parts: per slice of KC channels x1 w1 into the leading accumulators in turn, the five
@@ -441,20 +381,96 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
             }
         }
     }
+    // until the rings of the cluster are free: partial sums go there (a gathering warp has read its first sums by then)
+    bool met = !SPLIT;
+    auto meet = [&]() {
+        __syncwarp();
+        cluster_sync();
+        met = true;
+    };
+    if (warp < CT_GATHER_WARPS) {
+        // ---- epilogue: thread = voxel ----------------------------------------------------------
+        const bool read_acc = nit > 0 && __all_sync(0xffffffffu, ok);    // tcgen05.ld is warp-wide
+        const int q = warp & 3, half = warp >> 2;      // lane quarter of tensor memory, half of the columns
+        const int64_t v = rows_s[q * 32 + lane];
+        const uint32_t tm = tmem_base + ((uint32_t)(q * 32) << 16);
+        constexpr int NCB = BN / 32;                   // 32-column blocks, split between the two halves
+#pragma unroll 1
+        for (int cb = half * ((NCB + 1) / 2); cb < (half == 0 ? (NCB + 1) / 2 : NCB); ++cb) {
+            uint32_t acc[32];
+            if (F32) {
+                // from the small products to the leading ones, issuer after issuer
+#pragma unroll
+                for (int e = 0; e < 32; ++e) acc[e] = 0;
+#pragma unroll 1
+                for (int z = ACCS - 1; z >= 0; --z)
+#pragma unroll 1
+                    for (int i = 0; i < NI; ++i) {
+                        if (!read_acc || !((*reinterpret_cast<volatile uint32_t*>(used_s + i) >> z) & 1)) continue;
+                        uint32_t more[32];
+                        tmem_ld32(tm + (i * ACCS + z) * BN + cb * 32, more);
+                        tmem_ld_wait();
+                        tmem_ld_fence(more);
+#pragma unroll
+                        for (int e = 0; e < 32; ++e)
+                            acc[e] = __float_as_uint(__uint_as_float(acc[e]) + __uint_as_float(more[e]));
+                    }
+            } else if (read_acc) {
+                tmem_ld32(tm + cb * 32, acc);
+                tmem_ld_wait();
+                // the other issuers' partial sums, added in a fixed order
+#pragma unroll 1
+                for (int i = 1; i < NI && i < nit; ++i) {
+                    uint32_t more[32];
+                    tmem_ld32(tm + i * BN + cb * 32, more);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 32; ++e)
+                        acc[e] = __float_as_uint(__uint_as_float(acc[e]) + __uint_as_float(more[e]));
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) acc[i] = 0;
+            }
+            if (SPLIT) {
+                if (!met) meet();
+                // to the CTA that finishes the row
+                const int rows = CT_TM / (int)gridDim.z, r = q * 32 + lane;
+                const uint32_t at = peer_address(
+                    sbase + (((int)cluster_rank() * rows + r % rows) * PART_PITCH + cb * 32) * 4, r / rows);
+#pragma unroll
+                for (int g = 0; g < 8; ++g)
+                    st_cluster_f4(at + g * 16, __uint_as_float(acc[g * 4]), __uint_as_float(acc[g * 4 + 1]),
+                                  __uint_as_float(acc[g * 4 + 2]), __uint_as_float(acc[g * 4 + 3]));
+                continue;
+            }
+            if (v < 0) continue;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                float y[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) y[i] = __uint_as_float(acc[g * 8 + i]) + bias_s[cb * 32 + g * 8 + i];
+                ct_store_f32(a, v, col0 + cb * 32 + g * 8, y);
+            }
+        }
+    }
+    if (!met) meet();
     if (SPLIT) {
-        // this CTA's rows: the peers' partial sums in rank order, bias, bf16
+        // this CTA's rows: the cluster's partial sums in rank order, bias, bf16
+        __syncwarp();
         cluster_sync();
         const int parts = (int)gridDim.z, rows = CT_TM / parts, r0 = rows * (int)cluster_rank();
         for (int e = tid; e < rows * (BN / 8); e += CT_THREADS) {
-            const int r = r0 + e / (BN / 8), c = e % (BN / 8) * 8;
-            const int64_t v = rows_s[r];
+            const int r = e / (BN / 8), c = e % (BN / 8) * 8;
+            const int64_t v = rows_s[r0 + r];
             if (v < 0) continue;
-            const uint32_t at = sbase + (r * PART_PITCH + c) * 4;
+            const float* sums = reinterpret_cast<const float*>(smem) + r * PART_PITCH + c;
             float y[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) y[i] = 0.f;
             for (int z = 0; z < parts; ++z) {
-                const float4 m = ld_peer_f4(at, z), w = ld_peer_f4(at + 16, z);
+                const float4* p = reinterpret_cast<const float4*>(sums + z * rows * PART_PITCH);
+                const float4 m = p[0], w = p[1];
                 y[0] += m.x; y[1] += m.y; y[2] += m.z; y[3] += m.w;
                 y[4] += w.x; y[5] += w.y; y[6] += w.z; y[7] += w.w;
             }
@@ -466,7 +482,6 @@ __global__ void __launch_bounds__((CT_GATHER_WARPS + NI) * 32) conv_tc05_kernel(
                 *reinterpret_cast<uint4*>((__nv_bfloat16*)a.out + v * a.cout + col0 + c) =
                     make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
         }
-        cluster_sync();      // a peer's shared memory outlives its readers
     }
     fence_before_sync();
     __syncthreads();

@@ -6,9 +6,10 @@
 //   * tiles are 64 columns wide, eight warps take 32 columns of a row each;
 //   * the weights of the first chunks are on their way before the preceding kernel has finished (where the
 //     caller vouches for them, see linear.cuh);
-//   * long K: a cluster of up to eight CTAs takes shares of K; the partial sums meet in distributed
-//     shared memory, every CTA finishing some of the rows (in rank order: the result is the same on
-//     every run).
+//   * long K: a cluster of up to eight CTAs takes shares of K; each stores its partial sums with the CTA that finishes
+//     their rows, which adds them in rank order (the result is the same on every run).  Read from the peers instead, one
+//     after another and with a barrier more, behind which they may end: us, 441 x 1 024 -> 256 8.7 for 6.5, 457 x 2 048 -> 512
+//     9.2 / 7.9, 75 x 2 048 -> 512 7.6 / 6.5; fp32 820 x 1 024 -> 256 14.8 / 10.4, 260 x 2 048 -> 512 17.9 / 14.5.
 // (Linear + LayerNorm stays with linear_tc05.cu, whose epilogue holds a row in registers: 1 560 x 64 5.1 us
 // against 6.5 in this form, 6 700 x 128 8.1 against 10.4.)
 #include "common.cuh"
@@ -45,16 +46,19 @@ struct LinearSmallArgs {
     uint32_t* status;
 };
 
-// bytes of the ring; a split layer's partial sums (128 x 68 floats) lie over it
-__host__ __device__ constexpr int ls_ring_bytes(int stages, bool split)
+// Shared memory: the ring; with K shared by a cluster the partial sums of this CTA's rows (128 / parts of each CTA); bias as
+// floats; barriers
+constexpr int LS_PART_BYTES = LS_BM * LS_PITCH * 4;
+static_assert(LS_PART_BYTES % 1024 == 0, "alignment of what follows");
+constexpr int LS_PARAM_BYTES = LS_BN * 4;
+__host__ __device__ constexpr int ls_part_offset(int stages, bool split) { return stages * (split ? LS_SPLIT_STAGE : LS_STAGE); }
+__host__ __device__ constexpr int ls_param_offset(int stages, bool split, int parts)
 {
-    const int ring = stages * (split ? LS_SPLIT_STAGE : LS_STAGE);
-    return ring > LS_BM * LS_PITCH * 4 ? ring : (LS_BM * LS_PITCH * 4 + 1023) / 1024 * 1024;
+    return ls_part_offset(stages, split) + (parts > 1 ? LS_PART_BYTES : 0);
 }
-constexpr int LS_PARAM_BYTES = LS_BN * 4;              // bias as floats
-static size_t ls_smem(int stages, bool split)
+static size_t ls_smem(int stages, bool split, int parts)
 {
-    return ls_ring_bytes(stages, split) + LS_PARAM_BYTES + 8 * (2 * LS_MAX_STAGES + 1) + 16 + 1024;
+    return ls_param_offset(stages, split, parts) + LS_PARAM_BYTES + 8 * (2 * LS_MAX_STAGES + 1) + 16 + 1024;
 }
 
 // LS_F32: eight finished columns of a row, as floats or as split bf16 parts (see split_f32.cuh)
@@ -115,9 +119,11 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
     const uint32_t sbase = smem_u32_generic(smem);
     constexpr bool SPLIT = (MODE & LS_F32) != 0;
     constexpr int STAGE = SPLIT ? LS_SPLIT_STAGE : LS_STAGE, BK = SPLIT ? LS_SLICE : LS_BK;
-    const int stages = a.stages;
-    float* params = reinterpret_cast<float*>(smem + ls_ring_bytes(stages, SPLIT));
-    const int off_bar = ls_ring_bytes(stages, SPLIT) + LS_PARAM_BYTES;
+    const int stages = a.stages, parts = (int)gridDim.z;
+    if (parts > 1) cluster_started_arrive();
+    const int off_part = ls_part_offset(stages, SPLIT), off_param = ls_param_offset(stages, SPLIT, parts),
+              off_bar = off_param + LS_PARAM_BYTES;
+    float* params = reinterpret_cast<float*>(smem + off_param);
     const uint32_t full0 = sbase + off_bar, empty0 = full0 + 8 * LS_MAX_STAGES,
                    accfull = empty0 + 8 * LS_MAX_STAGES;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + off_bar + 8 * (2 * LS_MAX_STAGES + 1));
@@ -128,7 +134,6 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int col0 = blockIdx.x * LS_BN, row0 = blockIdx.y * LS_BM;
     // this CTA's chunks of K
-    const int parts = (int)gridDim.z;
     const int nk = a.k / BK / parts, k0 = nk * (int)blockIdx.z * BK;
 
     // chunk kc of x or of W into slot `s`; of a split layer part by part
@@ -306,26 +311,30 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
                         ls_finish<MODE>(v + g * 8, params + c0 + g * 8, res[g]);
             }
     } else {
-        // partial sums over the ring (every product has completed); then this CTA's rows
+        // every CTA's partial sums go to the CTA that finishes their rows (beside its ring, which it may still need); one
+        // barrier, and it adds them up in rank order
+        const int rows = LS_BM / parts, rank = (int)cluster_rank();
+        __syncwarp();
+        cluster_started_wait();
         if (warp >= 2) {
-            float* prow = reinterpret_cast<float*>(smem) + r * LS_PITCH + c0;
+            const uint32_t at = peer_address(sbase + off_part + ((rank * rows + r % rows) * LS_PITCH + c0) * 4, r / rows);
 #pragma unroll
-            for (int g = 0; g < 8; ++g)
-                *reinterpret_cast<float4*>(prow + g * 4) = make_float4(v[g * 4], v[g * 4 + 1], v[g * 4 + 2], v[g * 4 + 3]);
+            for (int g = 0; g < 8; ++g) st_cluster_f4(at + g * 16, v[g * 4], v[g * 4 + 1], v[g * 4 + 2], v[g * 4 + 3]);
         }
+        __syncwarp();
         cluster_sync();
-        const int rows = LS_BM / parts, first = rows * (int)cluster_rank();
+        const float* sums = reinterpret_cast<const float*>(smem + off_part);
         for (int e = tid; e < rows * (LS_BN / 8); e += LS_THREADS) {
-            const int rr = first + e / (LS_BN / 8), c = e % (LS_BN / 8) * 8;
-            const int64_t orow = (int64_t)row0 + rr;
+            const int rr = e / (LS_BN / 8), c = e % (LS_BN / 8) * 8;
+            const int64_t orow = (int64_t)row0 + rows * rank + rr;
             if (orow >= a.n || ((MODE & LS_F32) && col0 + c >= a.n_out)) continue;
             uint4 r4 = make_uint4(0, 0, 0, 0);
             if ((MODE & LS_RESIDUAL) && !(MODE & LS_F32))
                 r4 = *reinterpret_cast<const uint4*>((const __nv_bfloat16*)a.residual + orow * a.n_out + col0 + c);
-            const uint32_t at = sbase + (rr * LS_PITCH + c) * 4;
             float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             for (int z = 0; z < parts; ++z) {
-                const float4 m = ld_peer_f4(at, z), w = ld_peer_f4(at + 16, z);
+                const float4* p = reinterpret_cast<const float4*>(sums + (z * rows + rr) * LS_PITCH + c);
+                const float4 m = p[0], w = p[1];
                 t[0] += m.x; t[1] += m.y; t[2] += m.z; t[3] += m.w;
                 t[4] += w.x; t[5] += w.y; t[6] += w.z; t[7] += w.w;
             }
@@ -335,7 +344,6 @@ __global__ void __launch_bounds__(LS_THREADS) linear_small_kernel(const __grid_c
                 *reinterpret_cast<uint4*>((__nv_bfloat16*)a.out + orow * a.n_out + col0 + c) =
                     ls_finish<MODE>(t, params + c, r4);
         }
-        cluster_sync();          // a peer's partial sums outlive their readers
     }
     fence_before_sync();
     __syncthreads();
@@ -353,7 +361,9 @@ static int launch_ls(const void* x, const void* w, LinearSmallArgs a, int parts,
     constexpr int BK = split ? LS_SLICE : LS_BK;
     const int nk = a.k / BK / parts;
     // (fp32: two CTAs share an SM, in shared memory as in tensor memory; two rooms of 20 000: 6.79 -> 6.65 ms)
-    const int most = split ? 3 : LS_MAX_STAGES;
+    const dim3 grid((a.n_out + LS_BN - 1) / LS_BN, (unsigned)((a.n + LS_BM - 1) / LS_BM), parts);
+    const int64_t ctas = (int64_t)grid.x * grid.y * parts;
+    const int most = split ? (parts > 1 && ctas > SMS ? 2 : 3) : parts > 1 ? LS_MAX_STAGES - 1 : LS_MAX_STAGES;
     a.stages = nk < most ? nk : most;
     CUtensorMap mx, mw;
     const uint64_t cols = split ? (uint64_t)a.k * split_stored(a.k) : (uint64_t)a.k;      // stored
@@ -363,9 +373,8 @@ static int launch_ls(const void* x, const void* w, LinearSmallArgs a, int parts,
     if (rc) return rc;
     auto kern = linear_small_kernel<MODE>;
     if (allow_smem(kern) != cudaSuccess) return check_launch("short Linear: shared memory attribute");
-    const dim3 grid((a.n_out + LS_BN - 1) / LS_BN, (unsigned)((a.n + LS_BM - 1) / LS_BM), parts);
     const dim3 cluster(1, 1, parts);
-    launch_dependent_cluster(kern, grid, dim3(LS_THREADS), ls_smem(a.stages, split), stream, cluster, mx, mw, a);
+    launch_dependent_cluster(kern, grid, dim3(LS_THREADS), ls_smem(a.stages, split, parts), stream, cluster, mx, mw, a);
     count_launches(1);
     return check_launch("short Linear");
 }

@@ -289,19 +289,20 @@ __device__ __forceinline__ void cluster_sync()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// four floats of a peer's shared memory at this CTA's address `addr`
-__device__ __forceinline__ float4 ld_peer_f4(uint32_t addr, uint32_t rank)
+// the two halves of a barrier that orders no memory: every CTA of the cluster has started
+__device__ __forceinline__ void cluster_started_arrive() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_started_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+// this CTA's address `addr` in the shared memory of a peer, and a store there
+__device__ __forceinline__ uint32_t peer_address(uint32_t addr, uint32_t rank)
 {
     uint32_t p;
-    float4 v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(p) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "r"(p)
-                 : "memory");
-    return v;
+    return p;
 }
-
+__device__ __forceinline__ void st_cluster_f4(uint32_t addr, float x, float y, float z, float w)
+{
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
 __device__ __forceinline__ void named_barrier(int id, int threads)
 {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
