@@ -74,8 +74,8 @@ __device__ __forceinline__ void ct_store_f32(const ConvTcArgs& a, int64_t row, i
     o[1] = make_float4(y[4], y[5], y[6], y[7]);
 }
 
-// Operands: bf16; fp32 as the six pieces of split_f32.cuh, a stage for each (32 channels); fp32 as three parts, a stage
-// for each, from which the six products are taken.  A stage for every product, the form before for all widths, moves
+// Operands: bf16; fp32 as the six pieces of split_f32.cuh, 64 of their columns to a stage (widths that are not whole slices
+// of 64 channels); fp32 as three parts, a stage for each, from which the six products are taken.  A stage for every product, the form before for all widths, moves
 // each part twice in the mean.  us, before / now (L2 flushed, ~5 us of it the timing): 1 830 x 256 73.7 / 48.1, 822 x 256
 // 41.0 / 33.8, 261 x 512 88 / 59.5, 2 855 x 128 36.9 / 29.6, 10 542 x 64 35.8 / 33.8, 100 000 x 64 122.8 / 119.8.  What is left is
 // shared memory: a product of 64 columns takes its 48 to 58 cycles to read 6 KB, of 128 columns 65 (measured alone), 24
@@ -571,11 +571,12 @@ static const ConvVariant g_variants_f32[CT_VARIANTS] = {
     {128, 9.5, 0, 0.63, launch_conv_tc05_as<128, 6, 1, false, CT_PARTS>, launch_conv_tc05_as<128, 6, 1, true, CT_PARTS>,
      conv_tc05_capacity<128, 6, 1, CT_PARTS>},
     {1 << 20, 0, 0, 0, nullptr, nullptr, nullptr}};
-// ... of 32 channels
-static const ConvVariant g_variants_f32_32[CT_VARIANTS] = {
+// ... of pieces.  us, 64 wide | 32 wide: 111 445 x 32 -> 64 118.7 | 204.7, -> 128 231.5 | 401.8
+static const ConvVariant g_variants_f32_pieces[CT_VARIANTS] = {
+    {64, 6.5, 0, 0.20, launch_conv_tc05_as<64, 8, 2, false, CT_PIECES>, launch_conv_tc05_as<64, 8, 2, true, CT_PIECES>,
+     conv_tc05_capacity<64, 8, 2, CT_PIECES>},
     {32, 6.5, 0, 0.18, launch_conv_tc05_as<32, 8, 2, false, CT_PIECES>, launch_conv_tc05_as<32, 8, 2, true, CT_PIECES>,
      conv_tc05_capacity<32, 8, 2, CT_PIECES>},
-    {1 << 20, 0, 0, 0, nullptr, nullptr, nullptr},
     {1 << 20, 0, 0, 0, nullptr, nullptr, nullptr}};
 // bf16: clusters here, whole tiles in conv_stream.cu
 static const ConvVariant g_variants[CT_VARIANTS] = {
@@ -693,9 +694,11 @@ int launch_conv_split(const void* feat, const int32_t* nbr, const void* weight, 
     a.kvol = kvol;
     a.status = status;
     int v, parts = 1;
-    // (half of the offsets in use; of 32 channels all, 64-column chunks of the six pieces)
-    const ConvVariant* variants = c_in == 32 ? g_variants_f32_32 : g_variants_f32;
-    conv_cluster_cost(variants, a, c_in == 32 ? (double)a.kvol * (a.cin / 64) : 0.5 * a.kvol * (c_in / 64) * 3, &v, &parts);
+    // A slice is 64 channels, so parts are for whole ones; other widths (odd multiples of 32, stored as six pieces) walk the
+    // pieces in 64-column chunks.  (Stages: half of the offsets in use; of pieces all.)
+    const bool whole = c_in % 64 == 0;
+    const ConvVariant* variants = whole ? g_variants_f32 : g_variants_f32_pieces;
+    conv_cluster_cost(variants, a, whole ? 0.5 * a.kvol * (c_in / 64) * 3 : (double)a.kvol * (a.cin / 64), &v, &parts);
     return (parts > 1 ? variants[v].split : variants[v].plain)(weight, a, stream, parts);
 }
 

@@ -1028,6 +1028,14 @@ def test_subm_conv_on_split_floats_in_slices(n, cin, cout):
     test_subm_conv_on_split_floats(n, cin, cout)
 
 
+@pytest.mark.parametrize("n,cin,cout", [(700, 96, 64), (129, 96, 192), (300, 160, 128), (2000, 224, 64), (40000, 96, 64),
+                                        (700, 32, 64), (900, 32, 192)])
+def test_subm_conv_on_split_floats_in_pieces(n, cin, cout):
+    """Widths that are no whole slices of 64 channels: 64-column chunks of the six pieces that they are stored as, alone and
+    shared by a cluster."""
+    test_subm_conv_on_split_floats(n, cin, cout)
+
+
 @pytest.mark.parametrize("count", [1, 48, 49, 100])
 @pytest.mark.parametrize("param,buffer,affine", [(torch.float32, torch.float32, True), (torch.bfloat16, torch.bfloat16, True),
                                                  (torch.bfloat16, torch.float32, True), (None, torch.float32, False)])
