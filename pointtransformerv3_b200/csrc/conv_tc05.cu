@@ -571,7 +571,7 @@ static const ConvVariant g_variants_f32[CT_VARIANTS] = {
     {128, 9.5, 0, 0.63, launch_conv_tc05_as<128, 6, 1, false, CT_PARTS>, launch_conv_tc05_as<128, 6, 1, true, CT_PARTS>,
      conv_tc05_capacity<128, 6, 1, CT_PARTS>},
     {1 << 20, 0, 0, 0, nullptr, nullptr, nullptr}};
-// ... of pieces.  us, 64 wide | 32 wide: 111 445 x 32 -> 64 118.7 | 204.7, -> 128 231.5 | 401.8
+// ... of pieces, and all of 32 columns.  us, 64 wide | 32 wide: 111 445 x 32 -> 64 118.7 | 204.7, -> 128 231.5 | 401.8
 static const ConvVariant g_variants_f32_pieces[CT_VARIANTS] = {
     {64, 6.5, 0, 0.20, launch_conv_tc05_as<64, 8, 2, false, CT_PIECES>, launch_conv_tc05_as<64, 8, 2, true, CT_PIECES>,
      conv_tc05_capacity<64, 8, 2, CT_PIECES>},
@@ -694,11 +694,13 @@ int launch_conv_split(const void* feat, const int32_t* nbr, const void* weight, 
     a.kvol = kvol;
     a.status = status;
     int v, parts = 1;
-    // A slice is 64 channels, so parts are for whole ones; other widths (odd multiples of 32, stored as six pieces) walk the
-    // pieces in 64-column chunks.  (Stages: half of the offsets in use; of pieces all.)
-    const bool whole = c_in % 64 == 0;
-    const ConvVariant* variants = whole ? g_variants_f32 : g_variants_f32_pieces;
-    conv_cluster_cost(variants, a, whole ? 0.5 * a.kvol * (c_in / 64) * 3 : (double)a.kvol * (a.cin / 64), &v, &parts);
+    // A slice is 64 channels, so parts are for whole ones, and their accumulators fill tensor memory with 64 columns or
+    // 128; other widths (odd multiples of 32, stored as six pieces) and 32 columns walk the pieces in 64-column chunks.
+    // (Stages: half of the offsets in use; of pieces all.)
+    const bool slices = c_in % 64 == 0 && c_out % 64 == 0;
+    const ConvVariant* variants = slices ? g_variants_f32 : g_variants_f32_pieces;
+    conv_cluster_cost(variants, a, slices ? 0.5 * a.kvol * (c_in / 64) * 3 : (double)a.kvol * (a.cin / 64), &v, &parts);
+    PTV3_REQUIRE(v >= 0, PTV3_ERR_UNSUPPORTED, "ptv3_subm_conv_split_fwd: no kernel of %d -> %d channels", c_in, c_out);
     return (parts > 1 ? variants[v].split : variants[v].plain)(weight, a, stream, parts);
 }
 

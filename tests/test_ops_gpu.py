@@ -1036,6 +1036,12 @@ def test_subm_conv_on_split_floats_in_pieces(n, cin, cout):
     test_subm_conv_on_split_floats(n, cin, cout)
 
 
+@pytest.mark.parametrize("n,cin,cout", [(1, 64, 32), (700, 64, 32), (300, 256, 32), (129, 96, 32), (40000, 64, 32)])
+def test_subm_conv_on_split_floats_to_32_columns(n, cin, cout):
+    """32 output columns, narrower than the kernels that take slices of 64 channels: pieces, whatever the input's width."""
+    test_subm_conv_on_split_floats(n, cin, cout)
+
+
 @pytest.mark.parametrize("count", [1, 48, 49, 100])
 @pytest.mark.parametrize("param,buffer,affine", [(torch.float32, torch.float32, True), (torch.bfloat16, torch.bfloat16, True),
                                                  (torch.bfloat16, torch.float32, True), (None, torch.float32, False)])
