@@ -325,11 +325,11 @@ int ptv3_subm_conv_direct_fwd(const void* feat, const int32_t* indices, const vo
  *               scene and sets PTV3_STATUS_BAD_INDEX
  *   meta        1 + n_scenes int64: m, then the number of clusters per scene
  *   meta_host   NULL, or 3 + n_scenes int64 of page-locked HOST memory that the
- *               device can address (cudaHostAlloc / a pinned torch tensor): meta, then
- *               the status word, then the value 1 are stored there as soon as the clusters
- *               are numbered, so the host can read them without a device-to-host copy,
+ *               device can address (cudaHostAlloc / a pinned torch tensor): the last
+ *               kernel stores meta, then the status word, then the value 1 there once all
+ *               rows are checked, so the host can read them without a device-to-host copy,
  *               either after waiting for the stream or by zeroing the last word before the
- *               call and polling it (pooled_order and pooled_inverse follow in stream order)
+ *               call and polling it
  */
 size_t ptv3_pool_plan_workspace_bytes(int k, int64_t n, int n_scenes);
 int ptv3_pool_plan(const int64_t* code, const int64_t* order, const int32_t* grid_coord,

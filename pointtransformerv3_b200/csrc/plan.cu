@@ -86,8 +86,9 @@ struct RowPerm {
 // points 1.6 ms, 0.49 here.)
 //   pool_count_kernel     starts of runs per tile, every row.  A run is a parent cell: the codes of a row name it alike
 //                         however the row is ordered, so all rows are counted at once, without the cluster ids.
-//   pool_clusters_kernel  row 0: cluster ids, heads and what is read at the heads; its last block reports the sizes
-//   pool_orders_kernel    every row: orders and inverses of the pooled level from the cluster ids
+//   pool_clusters_kernel  row 0: cluster ids, heads and what is read at the heads; its last block writes the sizes
+//   pool_orders_kernel    every row: orders and inverses of the pooled level from the cluster ids; its last block reports,
+//                         because only here it shows whether the rows belong together
 // A block adds up the tiles before its own by itself up to PP_OWN_TILES; beyond, a kernel of its own scans the counts.
 constexpr int PP_THREADS = 256, PP_WARPS = PP_THREADS / 32;
 // Up to this size a thread takes one element (the chip has idle threads, and a block has the shortest chain), above it
@@ -155,7 +156,7 @@ struct PoolArgs {
     RowPerm perm;
     uint32_t *tile_sums, *totals;     // k x ntiles, by source row; k
     unsigned long long* scene_count;  // B
-    uint32_t* done;                   // blocks of pool_clusters_kernel that are through
+    uint32_t* done;                   // blocks of pool_clusters_kernel and of pool_orders_kernel that are through
     int64_t *cluster, *idx_ptr, *head, *pcode, *porder, *pinverse, *pbatch, *meta, *meta_host, *offset;
     int32_t *pgrid, *indices;         // indices: (batch, x, y, z) rows of the pooled level, or NULL
     uint32_t* status;
@@ -172,7 +173,7 @@ __global__ void __launch_bounds__(PP_THREADS) pool_count_kernel(const __grid_con
     const int64_t* code = a.code + (int64_t)row * a.n;
     if (blockIdx.x == 0 && row == 0) {
         for (int b = threadIdx.x; b < a.B; b += PP_THREADS) a.scene_count[b] = 0;
-        if (threadIdx.x == 0) *a.done = 0;
+        if (threadIdx.x < 2) a.done[threadIdx.x] = 0;
     }
     const int64_t j0 = tile_element<ITEMS>();
     int64_t p[ITEMS], key[ITEMS], before = 0;
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(PP_THREADS) pool_clusters_kernel(const __grid_
     __syncthreads();
     if (!last) return;
     __threadfence();
-    // the last block reports.  Every row must have as many runs as row 0:
+    // the last block: every row must have as many runs as row 0
     for (int r = 1 + warp; r < a.k; r += PP_WARPS) {
         const uint32_t* sums = a.tile_sums + (int64_t)r * a.ntiles;
         uint32_t runs = 0;
@@ -341,21 +342,10 @@ __global__ void __launch_bounds__(PP_THREADS) pool_clusters_kernel(const __grid_
         end += __shfl_sync(0xffffffffu, upto, 31);
     }
     if (!a.meta_host) return;
-    // the same numbers and the status word, stored straight into the caller's mapped host
-    // memory: the host reads them after waiting for the stream, with no copy in between
-    // (a copy would queue behind whatever else the copy engine is busy with)
-    if (lane == 0) {
-        a.meta_host[0] = m;
-        a.meta_host[1 + a.B] = (int64_t)atomicOr(a.status, 0u);
-    }
+    // (the same numbers go straight into the caller's mapped host memory: a copy would queue behind whatever else the copy
+    // engine is busy with)
+    if (lane == 0) a.meta_host[0] = m;
     __threadfence_system();
-    __syncwarp();
-    // "everything above has been stored": a host that zeroed this word before the call may
-    // poll it instead of waiting for the stream
-    if (lane == 0) {
-        *reinterpret_cast<volatile int64_t*>(&a.meta_host[2 + a.B]) = 1;
-        __threadfence_system();
-    }
 }
 
 template <int ITEMS>
@@ -402,6 +392,19 @@ __global__ void __launch_bounds__(PP_THREADS) pool_orders_kernel(const __grid_co
                                  : (int)blockIdx.x + 1 < a.ntiles ? sums[blockIdx.x + 1] - sums[blockIdx.x]
                                                                   : a.totals[src] - sums[blockIdx.x];
         if (mine != counted) atomicOr(a.status, PTV3_STATUS_BAD_INDEX);
+        if (a.meta_host) {
+            // Whoever comes last has every check behind it, and the kernel before has stored the sizes: now the status word
+            // goes to the host, then "everything has been stored".  A host that zeroed this word before the call may poll
+            // it instead of waiting for the stream.
+            __threadfence();
+            if (atomicAdd(a.done + 1, 1u) == gridDim.x * gridDim.y - 1) {
+                __threadfence();
+                a.meta_host[1 + a.B] = (int64_t)atomicOr(a.status, 0u);
+                __threadfence_system();
+                *reinterpret_cast<volatile int64_t*>(&a.meta_host[2 + a.B]) = 1;
+                __threadfence_system();
+            }
+        }
     }
     const uint32_t below = (1u << lane) - 1;
 #pragma unroll
@@ -683,7 +686,7 @@ int ptv3::pool_plan(const int64_t* code, const int64_t* order, const int32_t* gr
     a.tile_sums = cv.take<uint32_t>((size_t)k * w.ntiles);
     a.totals = cv.take<uint32_t>(k);
     a.scene_count = cv.take<unsigned long long>(n_scenes);
-    a.done = cv.take<uint32_t>(1);
+    a.done = cv.take<uint32_t>(2);
     a.code = code;
     a.order = order;
     a.grid = grid_coord;

@@ -225,6 +225,22 @@ def test_pool_plan_reports_rows_that_do_not_belong_together():
         ops.pool_plan(code.cuda(), order.cuda(), data["grid_coord"].cuda(), batch.cuda(), 1, 1)
 
 
+@pytest.mark.parametrize("sizes", [[3000], [150], [90000, 80000]])
+def test_pool_plan_reports_rows_that_group_the_points_differently(sizes):
+    """Codes of one row shuffled among the points: as many parent cells as in every other row, of other points.  Only the
+    cluster ids along that row's order show it, and the call that was given such rows says so."""
+    data = small_batch(sizes, 3)
+    batch = O.offset_to_batch(data["offset"])
+    code, order, _, _ = O.serialization(data["grid_coord"], batch, ORDERS)
+    code, order = code.clone(), order.clone()
+    first = torch.cat([data["offset"].new_zeros(1), data["offset"]])
+    for a, b in zip(first[:-1].tolist(), first[1:].tolist()):          # (within a scene, whose number is in the codes)
+        code[2, a:b] = code[2, a:b][torch.randperm(b - a, generator=torch.Generator().manual_seed(1))]
+    order[2] = code[2].argsort()
+    with pytest.raises(_lib.Ptv3Error, match="status 0x1"):
+        ops.pool_plan(code.cuda(), order.cuda(), data["grid_coord"].cuda(), batch.cuda(), len(sizes), 1)
+
+
 @pytest.mark.parametrize("number", [2, 33, 1 << 40, -1])
 def test_pool_plan_reports_a_scene_number_without_a_scene(number):
     """Clusters are counted per scene: a number outside the scenes has no counter and is reported."""
