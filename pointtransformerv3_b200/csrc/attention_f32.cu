@@ -9,8 +9,9 @@
 // into the buffer that O has left.  Four CTAs to an SM, 128 columns of tensor memory each.
 //
 // Softmax needs no reference value where |q| max|k| bounds a block's scores (AX_BOUND, per warp); other blocks take their
-// maximum first.  A value whose square is not below AX_HUGE (infinities and NaN among them: their parts would be NaN) sends
-// the CTA to plain arithmetic over all keys.
+// maximum first.  V is scaled by AX_VSCALE, so that the last part of the smallest normal number is a normal one still.  (Q and
+// K need no scale: what their parts lose down there is nothing to a score.)  A row whose squares are not below AX_HUGE or
+// AX_HUGE_V (infinities and NaN among them: their parts would be NaN) sends the CTA to plain arithmetic over all keys.
 //
 // Before, queries were registers of a thread and keys came from shared memory, on CUDA cores; two or four queries to a thread.
 // us, before (the better of the two) / now, patches of 1 024: 90 000 x 64 672 / 296, 40 000 x 64 315 / 157, 10 500 x 64 112 / 56,
@@ -37,6 +38,7 @@ constexpr int AX_D = 16;
 // largest |score| taken without a reference value: the exponent's rounding (16 log2 e 2^-24) stays within
 // that of a score of this size
 constexpr float AX_BOUND = 16.f, AX_HUGE = 1e36f;
+constexpr float AX_VSCALE = 16777216.f, AX_HUGE_V = 1e26f;          // 2^24; sums of P V stay far inside fp32
 constexpr float AX_LOG2E = 1.4426950408889634f;
 
 // operands in shared memory, 16-byte chunks of eight values: [d half][part][row] for Q and K (K-major), [part][d half][key]
@@ -159,7 +161,11 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
     auto fetch = [&](int64_t src) { ax_row(kv + src * stride, x); };
     auto stage = [&](int buf) {
         const float norm = ax_norm(x);
-        if (!(norm < AX_HUGE)) plain_s[buf] = 1;
+        if (!(norm < (is_v ? AX_HUGE_V : AX_HUGE))) plain_s[buf] = 1;
+        if (is_v) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] = mul2(x[i], pack2(AX_VSCALE, AX_VSCALE));
+        }
         const AxParts parts(x);
         if (is_v) {
 #pragma unroll
@@ -403,7 +409,7 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
         for (int d = 0; d < AX_D; ++d) q[d] = a.qkv[mine * stride + h * AX_D + d] * a.scale;
         ax_plain(a, start, L, h, q, acc);
     } else {
-        const float inv = 1.f / l;
+        const float inv = 1.f / (l * AX_VSCALE);
 #pragma unroll
         for (int d = 0; d < AX_D; ++d) acc[d] *= inv;
     }

@@ -474,6 +474,24 @@ def test_attention_fp32_values_out_of_range(where, value):
     torch.testing.assert_close(b[ok], ref[ok], rtol=2e-5, atol=2e-6)
 
 
+@pytest.mark.parametrize("size", [1e12, 1e14, 1e-28, 1e-30, 1e-34, 1e-36])
+def test_attention_fp32_small_and_large_values(size):
+    """Values whose bf16 parts would fall below the smallest numbers keep their 24 bits, and large ones on both sides of the
+    line to plain arithmetic too.  (All of a sign, so that no result
+    cancels: a few 2^-24 for the scores, their exponentials and 150 terms.)"""
+    n, C, H, K = 300, 32, 2, 150
+    g = torch.Generator().manual_seed(3)
+    qkv = torch.randn(n, 3 * C, generator=g)
+    qkv[:, 2 * C:] = (1 + torch.rand(n, C, generator=g)) * size
+    qkv = qkv.cuda()
+    order = torch.arange(n).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    b = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25)
+    q, k, v = (t.reshape(2, 150, H, 16).transpose(1, 2) for t in qkv.double().split(C, dim=1))
+    ref = (torch.softmax((q * 0.25) @ k.transpose(2, 3), 3) @ v).transpose(1, 2).reshape(n, C)
+    assert float(((b.double() - ref) / ref).abs().max()) < 1.5e-6
+
+
 @pytest.mark.parametrize("n", [1, 127, 129, 257, 1500])
 @pytest.mark.parametrize("gain", [0.3, 2.0, 8.0])
 def test_attention_fp32_two_queries_per_thread(n, gain):
