@@ -9,7 +9,8 @@
 // into the buffer that O has left.  Four CTAs to an SM, 128 columns of tensor memory each.
 //
 // Softmax needs no reference value where |q| max|k| bounds a block's scores (AX_BOUND, per warp); other blocks take their
-// maximum first.  V is scaled by AX_VSCALE, so that the last part of the smallest normal number is a normal one still.  (Q and
+// maximum first, and the reference lies AX_LIFT below it: parts of the smallest probability above zero are normal numbers
+// then too.  V is scaled by AX_VSCALE, so that the last part of the smallest normal number is a normal one still.  (Q and
 // K need no scale: what their parts lose down there is nothing to a score.)  A row whose squares are not below AX_HUGE or
 // AX_HUGE_V (infinities and NaN among them: their parts would be NaN) sends the CTA to plain arithmetic over all keys.
 //
@@ -38,6 +39,7 @@ constexpr int AX_D = 16;
 // largest |score| taken without a reference value: the exponent's rounding (16 log2 e 2^-24) stays within
 // that of a score of this size
 constexpr float AX_BOUND = 16.f, AX_HUGE = 1e36f;
+constexpr float AX_LIFT = 24.f;              // (base 2)
 constexpr float AX_VSCALE = 16777216.f, AX_HUGE_V = 1e26f;          // 2^24; sums of P V stay far inside fp32
 constexpr float AX_LOG2E = 1.4426950408889634f;
 
@@ -305,8 +307,10 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
                 for (int i = 0; i < 8; ++i)
                     if (8 * c + i < nk) cm = fmaxf(cm, __uint_as_float(x0[i]) + __uint_as_float(x1[i]));
             }
-            // the first block sets the reference; after blocks without one (reference 0) it only rises
-            const float up = first ? cm : fmaxf(m, cm), corr = first ? 0.f : fast_exp2(m - up);
+            // The first block sets the reference.  After blocks without one (reference 0, scores up to AX_BOUND) it may
+            // once go as low as their scores are high; from then on it only rises.
+            const float up = first ? cm - AX_LIFT : fmaxf(m == 0.f ? -AX_LIFT : m, cm - AX_LIFT),
+                        corr = first ? 0.f : fast_exp2(m - up);
             l *= corr;
 #pragma unroll
             for (int d = 0; d < AX_D; ++d) acc[d] *= corr;

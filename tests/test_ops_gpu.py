@@ -492,6 +492,30 @@ def test_attention_fp32_small_and_large_values(size):
     assert float(((b.double() - ref) / ref).abs().max()) < 1.5e-6
 
 
+@pytest.mark.parametrize("gap", [60.0, 83.0, 86.5])
+@pytest.mark.parametrize("near", [0, 149])
+def test_attention_fp32_far_keys(gap, near):
+    """Keys whose probabilities are the smallest normal numbers, and that alone have values: the one near key lies in a
+    patch's first block or in its last, behind blocks that needed no reference value.  (Scores of 125 in base 2, rounded
+    a few times at 2^-18: 1e-5 each in an exponential.)"""
+    n, C, H, K = 300, 32, 2, 150
+    g = torch.Generator().manual_seed(3)
+    qkv = torch.randn(n, 3 * C, generator=g) * 0.01
+    qkv[:, 0] = qkv[:, 16] = 4.0
+    qkv[:, C] = qkv[:, C + 16] = 0.0
+    qkv[:, 2 * C:] = (1 + torch.rand(n, C, generator=g)) * 1e12
+    for row in (near, 150 + near):
+        qkv[row, C] = qkv[row, C + 16] = gap
+        qkv[row, 2 * C:] = 0.0
+    qkv = qkv.cuda()
+    order = torch.arange(n).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    b = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25)
+    q, k, v = (t.reshape(2, 150, H, 16).transpose(1, 2) for t in qkv.double().split(C, dim=1))
+    ref = (torch.softmax((q * 0.25) @ k.transpose(2, 3), 3) @ v).transpose(1, 2).reshape(n, C)
+    assert float(((b.double() - ref) / ref).abs().max()) < 3e-5
+
+
 @pytest.mark.parametrize("n", [1, 127, 129, 257, 1500])
 @pytest.mark.parametrize("gain", [0.3, 2.0, 8.0])
 def test_attention_fp32_two_queries_per_thread(n, gain):
