@@ -205,7 +205,7 @@ static int attention_impl(const void* qkv, const int64_t* order, const int64_t* 
     if (mma_ok && algo != 1)
         return launch_attn_mma(qkv, order, pad, unpad, cu_seqlens, out, n_seq, max_seqlen, channels,
                                heads, scale, algo == 3, planned, status, (cudaStream_t)stream);
-    if (dtype == PTV3_DTYPE_F32 && !rpe.grid_coord && attention_splits(qkv, channels, heads, algo) &&
+    if (dtype == PTV3_DTYPE_F32 && !rpe.grid_coord && attention_splits(qkv, n, n_seq, channels, heads, algo) &&
         ((uintptr_t)out & 15) == 0)
         return launch_attn_f32(qkv, order, pad, unpad, cu_seqlens, out, split, n_seq, max_seqlen, channels, heads, scale,
                                status, (cudaStream_t)stream);
@@ -217,9 +217,12 @@ static int attention_impl(const void* qkv, const int64_t* order, const int64_t* 
                                           channels, heads, scale, rpe, status, (cudaStream_t)stream);
 }
 
-bool ptv3::attention_splits(const void* qkv, int channels, int heads, int algo)
+// A CTA of attention_f32.cu takes ~5 us for a patch and head, however few rows it has: patches of up to 12 rows in the mean
+// stay with the kernel of this file.  us here and there, 64 channels: 90 000 points in patches of 4 283 / 701, 8 210 / 367,
+// 12 199 / 252, 16 193 / 197; 20 000 in patches of 8 48 / 66, 16 46 / 36.
+bool ptv3::attention_splits(const void* qkv, int64_t n, int n_seq, int channels, int heads, int algo)
 {
-    return algo == 0 && channels / heads == 16 && ((uintptr_t)qkv & 15) == 0;
+    return algo == 0 && channels / heads == 16 && ((uintptr_t)qkv & 15) == 0 && n > 12ll * n_seq;
 }
 
 int ptv3::attention_split(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad,

@@ -123,6 +123,9 @@ __device__ __noinline__ void ax_plain(const AxArgs& a, int64_t start, int L, int
     for (int d = 0; d < AX_D; ++d) y[d] *= inv;
 }
 
+// SHORT: patches of up to 128 rows.  Warps whose queries or keys all lie behind a patch's end leave them out (us, without /
+// with: 90 000 x 64 in patches of 20 178 / 166, of 28 134 / 125; the tests cost long patches 2 %).
+template <bool SHORT>
 __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __grid_constant__ AxArgs a)
 {
     __shared__ __align__(128) unsigned char q_s[2 * AX_Q_PLANE], k_s[2][AX_K_BYTES], v_s[2][AX_V_BYTES];
@@ -157,11 +160,17 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
     // of the block after the one in `x`
     const int key = min(tid & (AX_THREADS / 2 - 1), AX_KC - 1);
     const bool is_v = warp >= AX_THREADS / 64;
+    const int key_warp = warp % (AX_THREADS / 64) * 32;
     const float* kv = a.qkv + (is_v ? 2 : 1) * a.C + h * AX_D;
     uint64_t x[8];
     auto source = [&](int c0) { return a.order[a.pad[start + min(c0 + key, L - 1)]]; };
     auto fetch = [&](int64_t src) { ax_row(kv + src * stride, x); };
-    auto stage = [&](int buf) {
+    // c0: first key of the block
+    auto stage = [&](int buf, int c0) {
+        if (SHORT && c0 + key_warp >= L) {
+            if (!is_v && lane == 0) norm_s[buf][warp] = 0.f;
+            return;
+        }
         const float norm = ax_norm(x);
         if (!(norm < (is_v ? AX_HUGE_V : AX_HUGE))) plain_s[buf] = 1;
         if (is_v) {
@@ -188,13 +197,18 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
     };
     fetch(source(0));
     int64_t src = source(AX_KC);
-    // this thread's query
-    float qnorm;
-    {
+    // this thread's query, and the point whose result it writes: none behind the patch's end or in a row that fills the last
+    // patch, whose owner is elsewhere (points are numbered in 32 bits)
+    float qnorm = 0.f;
+    int mine = -1;
+    const bool queries = !SHORT || warp * 32 < L;          // of this warp
+    if (queries) {
         const int qi = tile * AX_QT + tid;
         uint64_t q[8];
         if (qi < L) {
-            ax_row(a.qkv + a.order[a.pad[start + qi]] * stride + h * AX_D, q);
+            const int64_t pd = a.pad[start + qi], row = a.order[pd];
+            ax_row(a.qkv + row * stride + h * AX_D, q);
+            if (a.unpad[pd] == start + qi) mine = (int)row;
         } else {
 #pragma unroll
             for (int i = 0; i < 8; ++i) q[i] = 0ull;
@@ -218,7 +232,7 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
     __syncthreads();
     fence_after_sync();
     if (!(qnorm < AX_HUGE)) plain_s[0] = 1;
-    stage(0);
+    stage(0, 0);
     fetch(src);
     src = source(2 * AX_KC);
     fence_proxy_async();
@@ -263,6 +277,7 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
         ok &= mbar_wait(bar_o, o_phase, abort);
         o_phase ^= 1;
         __syncwarp();
+        if (!queries) return;
         fence_after_sync();
         tmem_ld16(tm + AX_TM_O, o0);
         tmem_ld16(tm + AX_TM_O + 16, o1);
@@ -286,7 +301,7 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
         // O of the block before; then (its V has been read) the next block into that buffer
         if (c0) take_o();
         if (more) {
-            stage(buf ^ 1);
+            stage(buf ^ 1, c0 + AX_KC);
             fence_proxy_async();
             fetch(src);
             src = source(c0 + 3 * AX_KC);
@@ -297,7 +312,7 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
         __syncwarp();
         fence_after_sync();
         uint32_t x0[8], x1[8], y0[8], y1[8];
-        if (!bounded) {
+        if (!bounded && queries) {
             float cm = -INFINITY;
             for (int c = 0; c < 2 * chunks; ++c) {
                 tmem_ld8(tm + 8 * c, x0);
@@ -366,10 +381,12 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
                 tmem_st4(tm + AX_TM_SMALL + 8 * c + 4, w2);
             }
         };
-        if (bounded && nk == AX_KC)
-            rows(std::false_type(), AX_KC / 16);
-        else
-            rows(std::true_type(), chunks);
+        if (queries) {
+            if (bounded && nk == AX_KC)
+                rows(std::false_type(), AX_KC / 16);
+            else
+                rows(std::true_type(), chunks);
+        }
         l += hsum2(sum);
         tmem_st_wait();
         fence_before_sync();
@@ -402,11 +419,7 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
     }
     if (lane == 0 && !ok && a.status) atomicOr(a.status, PTV3_STATUS_WAIT_LIMIT);
 
-    const int qi = tile * AX_QT + tid;
-    if (qi >= L) return;
-    const int64_t pd = a.pad[start + qi];
-    if (a.unpad[pd] != start + qi) return;       // a row that fills the last patch: its owner is elsewhere
-    const int64_t mine = a.order[pd];
+    if (mine < 0) return;
     if (plain) {
         float q[AX_D];
 #pragma unroll
@@ -420,10 +433,10 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
     if (a.split_out) {
 #pragma unroll
         for (int d = 0; d < AX_D; d += 8)
-            split_store8(a.split_out + mine * split_stored(a.C) * a.C, h * AX_D + d, a.C, acc + d);
+            split_store8(a.split_out + (int64_t)mine * split_stored(a.C) * a.C, h * AX_D + d, a.C, acc + d);
         return;
     }
-    float4* op = reinterpret_cast<float4*>(a.out + mine * a.C + h * AX_D);
+    float4* op = reinterpret_cast<float4*>(a.out + (int64_t)mine * a.C + h * AX_D);
 #pragma unroll
     for (int d = 0; d < 4; ++d) op[d] = make_float4(acc[4 * d], acc[4 * d + 1], acc[4 * d + 2], acc[4 * d + 3]);
 }
@@ -433,7 +446,8 @@ int launch_attn_f32(const void* qkv, const int64_t* order, const int64_t* pad, c
                     cudaStream_t stream)
 {
     const int tiles = (max_seqlen + AX_QT - 1) / AX_QT;
-    launch_dependent(attn_f32_d16_kernel, dim3(H * tiles, n_seq), dim3(AX_THREADS), 0, stream,
+    launch_dependent(max_seqlen <= AX_QT ? attn_f32_d16_kernel<true> : attn_f32_d16_kernel<false>,
+                     dim3(H * tiles, n_seq), dim3(AX_THREADS), 0, stream,
                      AxArgs{(const float*)qkv, order, pad, unpad, cu, split ? nullptr : (float*)out,
                             split ? (__nv_bfloat16*)out : nullptr, C, H, scale, status});
     count_launches(1);

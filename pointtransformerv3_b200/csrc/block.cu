@@ -122,7 +122,7 @@ static int block_f32(const ptv3_block_args* a, bool settled, cudaStream_t stream
                              a->n1_eps, b.s, n, C, stream));
     STEP(launch_linear_split(b.s, a->qkv_w, f(a->qkv_b), nullptr, b.qkv, nullptr, n, C, 3 * C, 0, settled, a->status,
                              stream));
-    if (attention_splits(b.qkv, C, a->heads, a->attention_algo)) {
+    if (attention_splits(b.qkv, n, a->n_seq, C, a->heads, a->attention_algo)) {
         STEP(attention_split(b.qkv, a->order, a->pad, a->unpad, a->cu_seqlens, b.s, n, a->n_seq, a->max_seqlen, C, a->heads,
                              a->scale, a->status, stream));
     } else {

@@ -51,7 +51,7 @@ int add_layernorm_split(const float* x, const float* residual, const float* ln1_
                         int64_t n, int channels, cudaStream_t stream);
 
 // ptv3_attention_fwd in fp32 whose result leaves as split rows, where attention_splits says that it can
-bool attention_splits(const void* qkv, int channels, int heads, int algo);
+bool attention_splits(const void* qkv, int64_t n, int n_seq, int channels, int heads, int algo);
 int attention_split(const void* qkv, const int64_t* order, const int64_t* pad, const int64_t* unpad,
                     const int32_t* cu_seqlens, void* split_out, int64_t n, int n_seq, int max_seqlen, int channels, int heads,
                     float scale, uint32_t* status, cudaStream_t stream);

@@ -492,6 +492,27 @@ def test_attention_fp32_small_and_large_values(size):
     assert float(((b.double() - ref) / ref).abs().max()) < 1.5e-6
 
 
+@pytest.mark.parametrize("n,K,mean", [(700, 1, 1), (600, 8, 8), (600, 12, 12), (601, 12, 12), (130, 13, 13), (640, 16, 16),
+                                      (645, 31, 31), (640, 32, 32), (660, 33, 33), (5, 48, 5), (13, 48, 13), (1000, 100, 100)])
+def test_attention_fp32_short_patches(n, K, mean):
+    """Patches on both sides of the line between the two fp32 kernels (12 rows in the mean), and of fewer rows than a tile
+    has, or a warp, against float64 patch by patch (the same rule as below)."""
+    C, H = 64, 4
+    g = torch.Generator().manual_seed(n + K)
+    qkv = torch.randn(n, 3 * C, generator=g).cuda()
+    order = torch.randperm(n, generator=g).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    a = ops.attention(qkv, order, pad, unpad, cu, H, min(n, K), 0.25, algo=1)
+    b = ops.attention(qkv, order, pad, unpad, cu, H, min(n, K), 0.25)
+    assert torch.equal(a, b) == (mean <= 12)
+    q, k, v = (t.reshape(-1, H, 16) for t in qkv.double()[order[pad]].split(C, dim=1))
+    ref = torch.cat([(torch.softmax(torch.einsum("ihd,jhd->hij", q[s:e], k[s:e]) * 0.25, 2) @ v[s:e].transpose(0, 1))
+                     .transpose(0, 1).reshape(e - s, C) for s, e in zip(cu[:-1].tolist(), cu[1:].tolist())])
+    back = torch.empty_like(ref[:n])
+    back[order] = ref[unpad]
+    assert rel_l2(b.double(), back) < 1.5 * rel_l2(a.double(), back) + 1e-7
+
+
 @pytest.mark.parametrize("gap", [60.0, 83.0, 86.5])
 @pytest.mark.parametrize("near", [0, 149])
 def test_attention_fp32_far_keys(gap, near):
