@@ -21,10 +21,11 @@
 // Every mbarrier wait is bounded; a wait that runs out sets PTV3_STATUS_WAIT_LIMIT.
 //
 // Measured (C = 64, 4 heads, patches of 1 024; us here and by the mma.sync kernel, attention_mma.cu): 100 000 points
-// 100 / 121, 400 000 352 / 447, 912 000 785 / 991, 98 to 103 % of the exponential unit's rate at 1 965 MHz.  128 x 128 scores
-// take an SM 975 cycles (mma.sync 1 250): the exponential unit needs 640 of them for its ten of sixteen; a loop of the
-// same reads, arithmetic and stores without any hand-over runs at 784.  What is left is a block's way through the roles
-// (softmax -> issuing warp -> product -> softmax, ~900 cycles), which the two other groups cover only in part.
+// 103 / 121, 400 000 363 / 447, 912 000 807 / 991: 86, 97 and 99 % of the exponential unit's rate at 1 965 MHz.  128 x 128
+// scores take an SM 1 035 cycles at 400 000 points (mma.sync 1 280; without a CTA's first ~7 us in both): the exponential unit
+// needs 640 of them for its ten of sixteen; a loop of the same reads, arithmetic (degree 4) and stores without any hand-over
+// runs at 784.  What is left is a block's way through the roles (softmax -> issuing warp -> product -> softmax, ~900 cycles),
+// which the two other groups cover only in part.  Forms tried (these times with a polynomial of degree 4, 2 % less):
 //   * Blocks of 128 keys and one buffer, not 64 and two (505 us where this takes 406, 444 patches of 4 heads): a
 //     hand-over costs ~170 cycles in the issuing warp's wait and ~160 in issuing, whatever the block's size, and
 //     an issuing warp that keeps three groups waiting bounded the earlier forms of this kernel, not the products
@@ -33,11 +34,12 @@
 //   * Two groups with larger blocks (511) or four with blocks of 96 keys (418) are slower; so is handing a block over
 //     in halves (408 to 420), probabilities in registers with P V on mma.sync (583), and a patch's rows looked up
 //     ahead by the loading warps (their instructions count: 100 000 points 105 us).
-//   * AT_POLY 4, 5, 6, 7, 8: 430, 414, 406, 406, 418 us; 0 (all on the exponential unit): 510.
+//   * AT_POLY 5, 6, 7: 366, 363, 371 us at 400 000 points; 0 (all on the exponential unit) takes a quarter more.
 //   * 80 registers a thread, so that kernels of the planning stream fit beside a CTA: 377 us for 361 at 400 000
 //     points, and no pass gained (16 LiDAR frames 42.0 ms, with 96 registers 41.3).
 #include "common.cuh"
 #include "attention_mma.cuh"
+#include "exp2_poly.cuh"
 #include "mma_util.cuh"
 #include "tc05.cuh"
 
@@ -90,27 +92,29 @@ __device__ __forceinline__ uint32_t at_scale_bf16x2(uint32_t v, float s)
 }
 
 // exp2(s log2e) of a pair on the FMA pipe, |s log2e| <= AT_BOUND: n = round(s log2e) by adding 1.5 * 2^23, 2^r on
-// [-0.5, 0.5] by the degree-4 polynomial of least relative error (2.7e-6 with its coefficients in fp32), n added to
-// the exponent field.
+// [-0.5, 0.5] by a polynomial as close as the exponential unit (exp2_poly.cuh; one of degree 4, with 2.7e-6 for its 2.1e-7,
+// is 2 % faster: 400 000 points 355 us for 363), n added to the exponent field.
 struct AtPoly {
-    uint64_t log2e, magic, neg_one, c4, c3, c2, c1, c0;
+    uint64_t log2e, magic, neg_one, c5, c4, c3, c2, c1, c0;
     __device__ __forceinline__ AtPoly()
     {
         log2e = pack2(AT_LOG2E, AT_LOG2E);
         magic = pack2(12582912.f, 12582912.f);
         neg_one = pack2(-1.f, -1.f);
-        c4 = pack2(0.009570102207362652f, 0.009570102207362652f);
-        c3 = pack2(0.05591785907745361f, 0.05591785907745361f);
-        c2 = pack2(0.240247443318367f, 0.240247443318367f);
-        c1 = pack2(0.6931217908859253f, 0.6931217908859253f);
-        c0 = pack2(0.9999992847442627f, 0.9999992847442627f);
+        c5 = pack2(EXP2_C5, EXP2_C5);
+        c4 = pack2(EXP2_C4, EXP2_C4);
+        c3 = pack2(EXP2_C3, EXP2_C3);
+        c2 = pack2(EXP2_C2, EXP2_C2);
+        c1 = pack2(EXP2_C1, EXP2_C1);
+        c0 = pack2(EXP2_C0, EXP2_C0);
     }
 };
 __device__ __forceinline__ uint32_t at_exp2_poly(uint64_t s2, const AtPoly& k)
 {
     const uint64_t t2 = fma2(s2, k.log2e, k.magic);
     const uint64_t r2 = fma2(s2, k.log2e, fma2(t2, k.neg_one, k.magic));
-    uint64_t p2 = fma2(r2, k.c4, k.c3);
+    uint64_t p2 = fma2(r2, k.c5, k.c4);
+    p2 = fma2(p2, r2, k.c3);
     p2 = fma2(p2, r2, k.c2);
     p2 = fma2(p2, r2, k.c1);
     p2 = fma2(p2, r2, k.c0);
@@ -611,11 +615,11 @@ bool attn_tc05_supported(int n_seq, int channels, int heads, int max_seqlen)
 
 // Whether this kernel is faster than the mma.sync one (attention_mma.cu) on n points in n_seq patches.  Three things speak
 // against it: few blocks (a CTA starts with ~7 us of gather, and a group alone on an SM takes 1 800 cycles a block, three
-// together 975 each), short patches (a pair's gather takes the loading warps ~5 us) and rows of a tile that
+// together 1 035 each), short patches (a pair's gather takes the loading warps ~5 us) and rows of a tile that
 // the patch does not have.  us here and there, H heads of 16, blocks of 128 x 128 scores per SM:
-//   patches of 1 024: 8 192 points H 8 (28 blocks) 28.9 / 27.6, 12 288 H 8 (42) 34.7 / 37.9, 100 000 H 4 (169) 102 / 121,
-//     400 000 H 4 (676) 361 / 448;  of 800: 3 200 H 32 (38) 33.9 / 39.0;  of 640: 2 560 H 32 (22) 22.4 / 22.7
-//   of 512: 20 000 H 8 (35) 28.7 / 33.7;  of 384: 30 000 H 8 (38) 34.7 / 35.6, 200 000 H 4 (127) 91.6 / 99.5
+//   patches of 1 024: 8 192 points H 8 (28 blocks) 28.9 / 27.6, 12 288 H 8 (42) 35.2 / 37.9, 100 000 H 4 (169) 103 / 121,
+//     400 000 H 4 (676) 363 / 448;  of 800: 3 200 H 32 (38) 33.9 / 39.0;  of 640: 2 560 H 32 (22) 22.4 / 22.7
+//   of 512: 20 000 H 8 (35) 29.4 / 33.7;  of 384: 30 000 H 8 (38) 34.7 / 35.6, 200 000 H 4 (127) 91.6 / 99.5
 //   of 320: 200 000 H 4 (106) 103 / 88;  of 256: 400 000 H 4 (169) 168 / 146
 bool attn_tc05_wanted(int64_t n, int n_seq, int heads, int max_seqlen)
 {

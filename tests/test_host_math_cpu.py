@@ -45,3 +45,17 @@ def test_kernel_decode_math_inverts_encode(hostlib):
             hostlib.host_decode(code.ctypes.data, 3000, depth, hilbert, out.ctypes.data)
             assert (out == g).all(), (depth, name)
             assert (cenc.decode(code, depth, name)[0] == g).all()
+
+
+def test_exponentials_on_the_fma_pipe_are_as_close_as_the_exponential_unit(tmp_path):
+    """The polynomial for 2^r that attention mixes with ex2.approx keeps that instruction's relative error of 2^-22."""
+    so = str(tmp_path / "libexp2_poly_host.so")
+    subprocess.check_call(["g++", "-std=c++17", "-O2", "-shared", "-fPIC", "-o", so,
+                           os.path.join(ROOT, "tests", "hostmath", "exp2_poly_host.cpp")])
+    lib = ctypes.CDLL(so)
+    lib.host_exp2_poly.argtypes = [ctypes.c_void_p, ctypes.c_int64, ctypes.c_void_p]
+    r = np.linspace(-0.5, 0.5, (1 << 20) + 1).astype(np.float32)
+    out = np.empty_like(r)
+    lib.host_exp2_poly(r.ctypes.data, r.size, out.ctypes.data)
+    ref = np.exp2(r.astype(np.float64))
+    assert np.abs(out / ref - 1).max() < 2.0 ** -22
