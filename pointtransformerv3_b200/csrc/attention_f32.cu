@@ -9,8 +9,9 @@
 // into the buffer that O has left.  Four CTAs to an SM, 128 columns of tensor memory each.
 //
 // Softmax needs no reference value where |q| max|k| bounds a block's scores (AX_BOUND, per warp); other blocks take their
-// maximum first, and the reference lies AX_LIFT below it: parts of the smallest probability above zero are normal numbers
-// then too.  V is scaled by AX_VSCALE, so that the last part of the smallest normal number is a normal one still.  (Q and
+// maximum first, and their probabilities are scaled by AX_LIFT: the parts of the smallest one above zero are normal numbers
+// then too.  (A lower reference instead of the factor costs a score's last bits: error 3.6e-7 for 2.5e-7, q and k of 2 and 1.)
+// V is scaled by AX_VSCALE, so that the last part of the smallest normal number is a normal one still.  (Q and
 // K need no scale: what their parts lose down there is nothing to a score.)  A row whose squares are not below AX_HUGE or
 // AX_HUGE_V (infinities and NaN among them: their parts would be NaN) sends the CTA to plain arithmetic over all keys.
 //
@@ -39,8 +40,8 @@ constexpr int AX_D = 16;
 // largest |score| taken without a reference value: the exponent's rounding (16 log2 e 2^-24) stays within
 // that of a score of this size
 constexpr float AX_BOUND = 16.f, AX_HUGE = 1e36f;
-constexpr float AX_LIFT = 24.f;              // (base 2)
-constexpr float AX_VSCALE = 16777216.f, AX_HUGE_V = 1e26f;          // 2^24; sums of P V stay far inside fp32
+constexpr float AX_LIFT = 16777216.f, AX_VSCALE = 16777216.f;         // 2^24 both
+constexpr float AX_HUGE_V = 1e26f;                                    // (sums of P V stay far inside fp32)
 constexpr float AX_LOG2E = 1.4426950408889634f;
 
 // operands in shared memory, 16-byte chunks of eight values: [d half][part][row] for Q and K (K-major), [part][d half][key]
@@ -267,7 +268,7 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
         }
         umma_commit(bar_o);
     };
-    float acc[AX_D], l = 0.f, m = 0.f;
+    float acc[AX_D], l = 0.f, m = 0.f, lift = 1.f;
 #pragma unroll
     for (int d = 0; d < AX_D; ++d) acc[d] = 0.f;
     bool first = true, ok = true, plain = *reinterpret_cast<volatile int*>(&plain_s[0]) != 0;
@@ -306,7 +307,7 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
             fetch(src);
             src = source(c0 + 3 * AX_KC);
         }
-        const bool bounded = __all_sync(0xffffffffu, qnorm * kn <= AX_BOUND * AX_BOUND && m == 0.f);
+        const bool bounded = __all_sync(0xffffffffu, qnorm * kn <= AX_BOUND * AX_BOUND && lift == 1.f);
         ok &= mbar_wait(bar_s, s_phase, abort);
         s_phase ^= 1;
         __syncwarp();
@@ -322,10 +323,9 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
                 for (int i = 0; i < 8; ++i)
                     if (8 * c + i < nk) cm = fmaxf(cm, __uint_as_float(x0[i]) + __uint_as_float(x1[i]));
             }
-            // The first block sets the reference.  After blocks without one (reference 0, scores up to AX_BOUND) it may
-            // once go as low as their scores are high; from then on it only rises.
-            const float up = first ? cm - AX_LIFT : fmaxf(m == 0.f ? -AX_LIFT : m, cm - AX_LIFT),
-                        corr = first ? 0.f : fast_exp2(m - up);
+            // the first block sets the reference; after blocks without one (reference 0, not lifted) it only rises
+            const float up = first ? cm : fmaxf(m, cm), corr = first ? 0.f : fast_exp2(m - up) * (lift == 1.f ? AX_LIFT : 1.f);
+            lift = AX_LIFT;
             l *= corr;
 #pragma unroll
             for (int d = 0; d < AX_D; ++d) acc[d] *= corr;
@@ -349,7 +349,8 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
                     e0 = 2 * i < valid ? e0 : 0.f;
                     e1 = 2 * i + 1 < valid ? e1 : 0.f;
                 }
-                const uint64_t p = pack2(e0, e1);
+                uint64_t p = pack2(e0, e1);
+                if (ragged.value) p = mul2(p, pack2(lift, lift));
                 sum = add2(sum, p);
                 const uint64_t rest = fma2(round2(p, w0[i]), minus, p);
                 unpack2(fma2(round2(rest, w1[i]), minus, rest), e0, e1);
