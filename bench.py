@@ -686,7 +686,7 @@ def run_operator_case(args):
         out.update(config={"workload": "stem SubMConv3d 5x5x5, 6 -> 32 channels, bf16, 4 indoor scenes",
                            "voxels": n},
                    metric="stem_voxels_per_sec", unit="voxels/s", value=n / (t * 1e-3), ms=t,
-                   roofline={"kernel": "conv_direct_mma_kernel (+ voxel index build)", "bound": "hbm",
+                   roofline={"kernel": "conv_direct_tc05_kernel (+ voxel index build)", "bound": "hbm",
                              "achieved": byts / t / 1e6, "peak": hbm, "unit": "GB/s",
                              "frac": byts / t / 1e6 / hbm, "traffic": None})
     elif args.case == "voxelize":

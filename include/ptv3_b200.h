@@ -163,12 +163,15 @@ int ptv3_pad_plan(const int64_t* offset, int n_scenes, int patch, int64_t n, int
  *               head_dim 16, max_seqlen <= 1024, out 16-byte aligned, needs
  *               `status`).  "Automatic" takes 4 where it is the faster one
  *               (long patches, from about 33 blocks of 128 x 128 scores per
- *               SM), else 2, else 1
+ *               SM: all patches of the call count, so a scene's rows may differ
+ *               in a rounding to bf16 with the scenes beside it), else 2; fp32 of
+ *               head_dim 16 with 16-byte aligned rows on tcgen05 from split
+ *               operands (patches of more than 12 rows in the mean); else 1
  *   status      one uint32 or NULL.  Every path ORs PTV3_STATUS_BAD_INDEX into it
  *               when cu_seqlens holds a patch longer than max_seqlen (that patch is
- *               skipped, its output rows stay unwritten; with NULL it is skipped
- *               silently); path 4 also ORs PTV3_STATUS_WAIT_LIMIT when one of its
- *               bounded waits ran out (the output is then undefined)
+ *               skipped, or its rows beyond are: output rows stay unwritten; with NULL
+ *               silently); the tcgen05 paths also OR PTV3_STATUS_WAIT_LIMIT when one of
+ *               their bounded waits ran out (the output is then undefined)
  */
 int ptv3_attention_fwd(const void* qkv, const int64_t* order, const int64_t* pad,
                        const int64_t* unpad, const int32_t* cu_seqlens, void* out, int64_t n,

@@ -16,9 +16,10 @@
 // AX_HUGE_V (infinities and NaN among them: their parts would be NaN) sends the CTA to plain arithmetic over all keys.
 //
 // Before, queries were registers of a thread and keys came from shared memory, on CUDA cores; two or four queries to a thread.
-// us, before (the better of the two) / now, patches of 1 024: 90 000 x 64 672 / 296, 40 000 x 64 315 / 157, 10 500 x 64 112 / 56,
-// 2 800 x 128 72 / 47; patches of 410, 820 x 256 24.8 / 16.8, of 130, 260 x 512 12.5 / 8.5.  Error against 64 bits, 2-norm:
-// 3.4e-7 / 1.8e-7 (a row's sums are taken per block, and S and O lose only what four products in a row truncate).
+// us, before (the better of the two) / now, patches of 1 024: 90 000 x 64 672 / 294, 40 000 x 64 315 / 148, 10 500 x 64 112 / 55,
+// 2 800 x 128 72 / 46; patches of 410, 820 x 256 24.8 / 17.2, of 130, 260 x 512 12.5 / 8.5.  Error against 64 bits, rms of a
+// row, q and k of size 1: 2.7e-7 / 1.5e-7, of 8 and 8: 1.3e-6 / 1.1e-6 (a row's sums are taken per block, and S and O lose
+// only what four products in a row truncate).
 // What bounds it is instructions: 13 for a pair of probabilities and their parts, and the splitting of a block's keys and
 // values by each of a patch's CTAs (issue slots 67 % busy in the form before the last, at 21 instructions a key and thread).
 // Without gain: 64 keys a block with O over S (S then waits for O: 332 us where this takes 296).  Leaving out 16 of the 20
@@ -398,6 +399,7 @@ __global__ void __launch_bounds__(AX_THREADS, 4) attn_f32_d16_kernel(const __gri
         if (warp == 0) {
             if (elect_one()) {
                 fence_after_sync();
+                // (S of the next block overwrites P, which O is made from: products run in the order of issue, see umma_bf16)
                 issue_o(buf, chunks);
                 if (more && !plain) issue_s(buf ^ 1);
             }

@@ -57,8 +57,9 @@ __device__ __forceinline__ uint32_t scale_bf16x2(uint32_t v, float s)
 // halves of one row cost half of one lane per row with a half at a time.  That shortens the start of launches of a few
 // waves, where CTAs gather at the same time (us: 405 points of 8 heads 5.5 -> 5.1, 1 560 of 4 9.1 -> 8.0, 6 000 of 2
 // 10.7 -> 9.8, 1 757 of 16 16.3 -> 15.7, 4 x 560 of 32 20.8 -> 19.8, 632 CTAs of 256 points 19.7 -> 19.0); in long ones a CTA's
-// gather is hidden by the two beside it, and the loop behind it gets worse registers (6 252 CTAs of 256 points 146.5 ->
-// 148.1, 60 000 points of 2 048 174.7 -> 183).
+// gather is hidden by the two beside it, and the loop behind it gets worse registers (half rows: 16 bytes of a thread's are
+// spilled, 8 in the planned form, none in the long one; 6 252 CTAs of 256 points 146.5 -> 148.1, 60 000 points of 2 048 174.7 ->
+// 183).
 enum AmGather {
     AM_LONG,          // a row per lane
     AM_SHORT,         // half a row per lane

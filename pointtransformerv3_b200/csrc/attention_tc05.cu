@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) attn_tc05_d16_kernel(const AtAr
                 const uint64_t dq = desc_q + (k & 1) * (AT_Q_BYTES >> 4);
                 const uint64_t dk = desc_k + slot;
                 uint64_t dv = desc_v + slot;
-                // P V' of a full block, or of the tile's last one
+                // P V' of a full block, or of the tile's last one.  The S issued behind it overwrites P (order: see umma_bf16).
                 auto issue_pv = [&](bool first, int steps) {
                     if (steps == AT_BK / 16) {
 #pragma unroll

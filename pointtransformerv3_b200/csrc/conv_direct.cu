@@ -395,7 +395,7 @@ static size_t conv_direct_weight_bytes(int ksize) { return align_up((size_t)(ksi
 // ... and the padded features
 size_t conv_direct_scratch_bytes(int64_t n, int ksize) { return conv_direct_weight_bytes(ksize) + align_up((size_t)n * 16, 256); }
 
-static int launch_conv_direct_mma(const void* feat, const int32_t* indices, const void* weight, const void* bias,
+static int launch_conv_direct_tc05(const void* feat, const int32_t* indices, const void* weight, const void* bias,
                                   const float* bn_scale, const float* bn_shift, int apply_gelu, void* out,
                                   const int64_t* row_order, int64_t n, int cin, int cout, int ksize,
                                   const unsigned long long* keys, const uint32_t* vals, uint64_t cap_mask,
@@ -488,7 +488,7 @@ int conv_direct_from_index(const VoxelIndex& vi, const void* feat, const int32_t
         return launch_conv_direct<float>(feat, indices, weight, nullptr, bn_scale, bn_shift, 1, out, row_order, n, c_in,
                                          c_out, ksize, vi.keys, vi.vals, vi.cap_mask, vi.cells, status, weight_scratch,
                                          stream);
-    return launch_conv_direct_mma(feat, indices, weight, nullptr, bn_scale, bn_shift, 1, out, row_order, n, c_in, c_out,
+    return launch_conv_direct_tc05(feat, indices, weight, nullptr, bn_scale, bn_shift, 1, out, row_order, n, c_in, c_out,
                                   ksize, vi.keys, vi.vals, vi.cap_mask, vi.cells, status, weight_scratch, stream);
 }
 
@@ -540,6 +540,6 @@ extern "C" int ptv3_subm_conv_direct_fwd(const void* feat, const int32_t* indice
         return launch_conv_direct<float>(feat, indices, weight, bias, bn_scale, bn_shift, apply_gelu, out,
                                          row_order, n, c_in, c_out, ksize, keys, vals, cap_mask, cells, status,
                                          wt, stream);
-    return launch_conv_direct_mma(feat, indices, weight, bias, bn_scale, bn_shift, apply_gelu, out, row_order, n,
+    return launch_conv_direct_tc05(feat, indices, weight, bias, bn_scale, bn_shift, apply_gelu, out, row_order, n,
                                   c_in, c_out, ksize, keys, vals, cap_mask, cells, status, wt, stream);
 }

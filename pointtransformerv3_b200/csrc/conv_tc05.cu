@@ -20,8 +20,8 @@
 // What bounds it on few tiles: ~7 us before the first and after the last product, and ~370 cycles per stage of 64
 // channels, 500 of 128, 700 of 256 (see conv_stream.cu for what a stage is made of).
 //
-// A cluster of up to eight CTAs shares one tile.  Each takes a
-// contiguous share of the tile's stages; the partial sums meet in shared memory and every CTA adds the
+// A cluster of up to eight CTAs shares one tile.  Each takes a contiguous share of the tile's stages (of fp32 parts: slices
+// in turn); the partial sums meet in shared memory and every CTA adds the
 // parts of its rows, which the peers have stored with it, in rank order.  A tile alone walks
 // 27 x c_in / 64 stages one after the other, 49 us at 512 channels on 27 voxels, while most SMs have nothing; in
 // clusters of eight that is 10 us.
