@@ -446,10 +446,28 @@ def attention64(qkv, order, pad, unpad, cu, heads, scale):
     return out
 
 
+@pytest.mark.parametrize("n,K", [(1281, 128), (1290, 129), (700, 65), (1500, 1024), (330, 31), (63, 64), (48, 17)])
+@pytest.mark.parametrize("gain", [0.3, 8.0])
+def test_attention_fp32_many_heads(n, K, gain):
+    """Several CTAs to an SM; ragged tiles, patches, blocks of 64 keys and steps of 16, scores bounded and not, against the
+    one-query form (the order of 32-bit sums: a few 2^-24 per term, as in the test below)."""
+    C, H = 512, 32
+    g = torch.Generator().manual_seed(n)
+    qkv = torch.randn(n, 3 * C, generator=g)
+    qkv[n // 2:, C:2 * C] *= gain * gain
+    qkv[:, :C] *= gain
+    qkv = qkv.cuda()
+    order = torch.randperm(n, generator=g).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    a = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25, algo=1)
+    b = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25)
+    assert bool(torch.isfinite(b).all()) and rel_l2(b, a) < 1e-5
+
+
 @pytest.mark.parametrize("n,K", [(1281, 128), (1290, 129), (700, 65), (1500, 1024), (330, 31), (63, 64), (48, 17), (480, 48),
                                  (470, 47), (500, 49), (300, 96), (190, 95), (200, 97), (300, 144), (300, 145)])
 @pytest.mark.parametrize("gain", [0.3, 8.0])
-def test_attention_fp32_many_heads(n, K, gain):
+def test_attention_fp32_many_heads_against_float64(n, K, gain):
     """Several CTAs to an SM; whole and ragged tiles, patches, blocks of 48 keys and steps of 16, scores bounded and not: as
     close to float64 as the one-query form."""
     C, H = 512, 32
@@ -544,6 +562,28 @@ def test_attention_fp32_far_keys(gap, near):
     q, k, v = (t.reshape(2, 150, H, 16).transpose(1, 2) for t in qkv.double().split(C, dim=1))
     ref = (torch.softmax((q * 0.25) @ k.transpose(2, 3), 3) @ v).transpose(1, 2).reshape(n, C)
     assert float(((b.double() - ref) / ref).abs().max()) < 3e-5
+
+
+@pytest.mark.parametrize("n", [1, 127, 129, 257, 1500])
+@pytest.mark.parametrize("gain", [0.3, 2.0, 8.0])
+def test_attention_fp32_two_queries_per_thread(n, gain):
+    """The fp32 kernel (algo 0) against the one-query form (algo 1): bounded and unbounded chunks of
+    keys, both in one sequence (the second half has large keys), ragged ends."""
+    C, H, K = 32, 2, 1024
+    g = torch.Generator().manual_seed(n)
+    qkv = torch.randn(n, 3 * C, generator=g)
+    qkv[n // 2:, C:2 * C] *= gain * gain
+    qkv[:, :C] *= gain
+    qkv = qkv.cuda()
+    order = torch.randperm(n, generator=g).cuda()
+    pad, unpad, cu = ops.pad_plan(torch.tensor([n]).cuda(), [n], K)
+    a = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25, algo=1)
+    b = ops.attention(qkv, order, pad, unpad, cu, H, K, 0.25)
+    assert bool(torch.isfinite(b).all()) and rel_l2(b, a) < 1e-5
+    if n <= K:         # one patch: plain attention over all rows, here in float64
+        q, k, v = (t.reshape(n, H, C // H).transpose(0, 1) for t in qkv.double().split(C, dim=1))
+        ref = (torch.softmax(q @ k.transpose(1, 2) * 0.25, 2) @ v).transpose(0, 1).reshape(n, C)
+        assert rel_l2(b.double(), ref) < 1.5 * rel_l2(a.double(), ref) + 1e-7
 
 
 @pytest.mark.parametrize("n", [1, 47, 48, 49, 96, 97, 127, 129, 144, 145, 257, 1500])
