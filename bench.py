@@ -45,8 +45,9 @@ CPU_SAMPLE_VOXELS = 100_000
 LIDAR_SCENES = 16
 LIDAR_GRID = 0.05
 # DRAM read + write bytes per row and channel of one attention launch (ncu, dram__bytes_read.sum +
-# dram__bytes_write.sum of a single launch on 407 000 rows x 64 channels: 166.1 + 31.9 MB)
-ATTENTION_DRAM_BYTES_PER_ROW_CHANNEL = 7.60
+# dram__bytes_write.sum of a single launch on 407 000 rows x 64 channels: 233.9 + 34.5 MB on tcgen05, which the long
+# launches take; 166.1 + 31.9 MB on mma.sync)
+ATTENTION_DRAM_BYTES_PER_ROW_CHANNEL = 10.30
 
 
 def workload_config(n_gpus, gather=False):
@@ -633,7 +634,8 @@ def run_operator_case(args):
                            "patches": cu.numel() - 1, "algo": args.algo},
                    metric="attention_points_per_sec", unit="points/s", value=n / (t * 1e-3), ms=t,
                    exps_per_sec=pad.numel() * K * H / (t * 1e-3),
-                   roofline={"kernel": "attn_tc05_d16_kernel" if args.algo == 4 else "attn_mma_d16_kernel",
+                   roofline={"kernel": {0: "attention core (automatic choice)", 1: "attn_fma_kernel",
+                                        4: "attn_tc05_d16_kernel"}.get(args.algo, "attn_mma_d16_kernel"),
                              "bound": "tensor", "achieved": flops / t / 1e9,
                              "peak": tf, "unit": "TFLOP/s", "frac": flops / t / 1e9 / tf, "traffic": None})
     elif args.case == "conv":

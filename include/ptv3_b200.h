@@ -332,7 +332,8 @@ int ptv3_subm_conv_direct_fwd(const void* feat, const int32_t* indices, const vo
  *               kernel stores meta, then the status word, then the value 1 there once all
  *               rows are checked, so the host can read them without a device-to-host copy,
  *               either after waiting for the stream or by zeroing the last word before the
- *               call and polling it
+ *               call and polling it (pooled_order and pooled_inverse are complete in stream
+ *               order, like every output)
  */
 size_t ptv3_pool_plan_workspace_bytes(int k, int64_t n, int n_scenes);
 int ptv3_pool_plan(const int64_t* code, const int64_t* order, const int32_t* grid_coord,

@@ -20,8 +20,9 @@
 // 2 800 x 128 72 / 46; patches of 410, 820 x 256 24.8 / 17.2, of 130, 260 x 512 12.5 / 8.5.  Error against 64 bits, rms of a
 // row, q and k of size 1: 2.7e-7 / 1.5e-7, of 8 and 8: 1.3e-6 / 1.1e-6 (a row's sums are taken per block, and S and O lose
 // only what four products in a row truncate).
-// What bounds it is instructions: 13 for a pair of probabilities and their parts, and the splitting of a block's keys and
-// values by each of a patch's CTAs (issue slots 67 % busy in the form before the last, at 21 instructions a key and thread).
+// No unit is full: issue slots are 54 % busy (13 instructions for a pair of probabilities and their parts, and the splitting of
+// a block's keys and values by each of a patch's CTAs), the L1 data pipe 58 %, the tensor pipe 37 %; four warps to a scheduler
+// wait for tensor memory most, then at a block's two barriers (21 instructions a key and thread, the form before: 67 %).
 // Without gain: 64 keys a block with O over S (S then waits for O: 332 us where this takes 296).  Leaving out 16 of the 20
 // products of O, the splitting, the staging or the exponentials gave that form 4, 10, 8 and 4 %.
 #include "attention_mma.cuh"
